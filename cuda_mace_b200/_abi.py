@@ -14,6 +14,25 @@ _I = ctypes.c_int
 _L = ctypes.c_int64
 _D = ctypes.c_double
 
+class StepModel(ctypes.Structure):
+    """cmace_step_model of the header: constant weights of one model."""
+    _fields_ = [(k, ctypes.c_int32) for k in ("is_f64", "channels", "elements", "nbessel", "cutoff_p", "reserved")] + [
+        ("r_max", _D), ("scale", _D), ("shift", _D), ("radial", (_P * 4) * 2), ("radial_back", _P), ("fold", _P),
+        ("fold_back", _P * 8), ("linear", _P * 2), ("weff", _P * 2)] + [
+        (k, _P) for k in ("up", "up_back", "skip", "readout0", "readout1", "readout2", "atomic_energies")]
+
+
+class StepIO(ctypes.Structure):
+    """cmace_step_io of the header: one step's inputs, workspace and outputs."""
+    _fields_ = [(k, _L) for k in ("n_owned", "n_local", "nedges")] + [
+        (k, _P) for k in ("positions", "shifts", "species", "one_hot")] + [
+        ("one_hot_is_f64", ctypes.c_int32), ("launches", ctypes.c_int32)] + [
+        (k, _P) for k in ("sender", "receiver", "row_ptr", "perm", "send_ptr", "up_local", "gup_local", "gup_owned",
+                          "workspace")] + [
+        ("workspace_bytes", _L)] + [(k, _P) for k in ("status", "node_energy", "interaction", "sums", "gradient")] + [
+        ("gradient_sign", _D)]
+
+
 # name -> argument ctypes (every function returns int unless listed in _RESTYPES)
 SIGNATURES = {
     "cmace_abi_version": [],
@@ -66,6 +85,11 @@ SIGNATURES = {
     "cmace_scan_workspace_bytes": [_L],
     "cmace_exclusive_scan_i32": [_P, _L, _P, _P, _L, _P],
     "cmace_nl_fill_f64": [_P, _L, _L, _D, _D, _D, _D, _D, _D, _I, _D, _P, _P, _P, _P, _P, _P, _P, _P],
+    "cmace_symcon_effective_weights": [_P, _I, _P, _P, _P, _I, _I, _P, _P],
+    "cmace_step_workspace_bytes": [_P, _L, _L, _L],
+    "cmace_step_count": [],
+    "cmace_step_name": [_I],
+    "cmace_step_run": [_P, _P, _I, _I, _P],
     "cmace_symcon_plan_create": [_I, _P, _P, _P, _P, _P, _P, _I, _I, _I, ctypes.POINTER(_P)],
     "cmace_symcon_plan_destroy": [_P],
     "cmace_symcon_plan_nterms": [_P],
@@ -83,6 +107,8 @@ _RESTYPES = {
     "cmace_radial_hidden_saved_floats": _L,
     "cmace_nl_num_cells": _L,
     "cmace_scan_workspace_bytes": _L,
+    "cmace_step_workspace_bytes": _L,
+    "cmace_step_name": ctypes.c_char_p,
     "cmace_imp_bwd_edge_f64_noalloc_max_elems": _L,
     "cmace_symcon_plan_destroy": None,
 }
@@ -90,7 +116,7 @@ _RESTYPES = {
 _VALUE_FUNCS = {"cmace_abi_version", "cmace_sender_order_workspace_bytes", "cmace_imp_bwd_scratch_elems",
                 "cmace_gemm_packed_floats", "cmace_imp_bwd_edge_f64_noalloc_max_elems",
                 "cmace_radial_hidden_saved_floats", "cmace_nl_num_cells", "cmace_scan_workspace_bytes",
-                "cmace_imp_staged_stalled",
+                "cmace_imp_staged_stalled", "cmace_step_workspace_bytes", "cmace_step_count", "cmace_step_name",
                 "cmace_symcon_plan_destroy", "cmace_symcon_plan_nterms", "cmace_symcon_plan_nclasses",
                 "cmace_symcon_plan_is_canonical"}
 
@@ -106,7 +132,7 @@ KERNEL_LAUNCHES = {
     "cmace_imp_bwd_node": 1, "cmace_linear": 1, "cmace_symcon_fwd": 1, "cmace_symcon_bwd": 1,
     "cmace_gemm_pack_weights": 1, "cmace_gemm3x": 1, "cmace_gemm": 1, "cmace_gemm3x_gradr": 1, "cmace_bounded_wait_probe": 1, "cmace_linear_tc": 1,
     "cmace_radial_hidden_fwd": 1, "cmace_radial_hidden_bwd": 1, "cmace_imp_radial_fused_fwd": 1,
-    "cmace_nl_cell_ids": 1, "cmace_nl_count": 1, "cmace_exclusive_scan_i32": 1, "cmace_nl_fill": 1,
+    "cmace_symcon_effective_weights": 1, "cmace_nl_cell_ids": 1, "cmace_nl_count": 1, "cmace_exclusive_scan_i32": 1, "cmace_nl_fill": 1,
 }
 launch_count = 0       # kernels launched through this binding since import
 _timing = None         # list of (name, start_event, end_event) while timing is on
@@ -156,6 +182,28 @@ def call(name, *args, tag=None):
     if rc != 0:
         raise RuntimeError(f"{name} failed ({rc}): {lib.cmace_last_error().decode()}")
     return 0
+
+
+def run_steps(model, io, first, last, stream):
+    """cmace_step_run on a StepModel and a StepIO; while timing is on, every step is bracketed by events of its own."""
+    global launch_count
+    lib = _lib if _lib is not None else load()
+    before = io.launches
+    if _timing is None:
+        rc = lib.cmace_step_run(ctypes.byref(model), ctypes.byref(io), first, last, stream)
+    else:
+        import torch
+
+        rc = 0
+        for s in range(first, last):
+            ev0, ev1 = torch.cuda.Event(enable_timing=True), torch.cuda.Event(enable_timing=True)
+            ev0.record()
+            rc = rc or lib.cmace_step_run(ctypes.byref(model), ctypes.byref(io), s, s + 1, stream)
+            ev1.record()
+            _timing.append((f"step[{lib.cmace_step_name(s).decode()}]", ev0, ev1))
+    launch_count += io.launches - before
+    if rc != 0:
+        raise RuntimeError(f"cmace_step_run failed ({rc}): {lib.cmace_last_error().decode()}")
 
 
 def start_timing():

@@ -91,6 +91,7 @@ struct GemmArgs {
   int ep_tma;                   // PLAIN: 1 when the epilogue stores tiles with TMA from a staging buffer
   // GRADR: X [Ns, C] sender features, G [Nr, 16, C] gradient of the messages, Y [16, M] harmonics, edge lists [M]
   const float *gx, *gg, *gy;
+  int64_t y_m, y_e;             // strides of Y over components and edges
   const int32_t *sender, *receiver;
   int C;
   int g_stage_bytes;            // GRADR: shared memory behind the ring and the epilogue buffers for staged G rows
@@ -488,7 +489,7 @@ __global__ void __launch_bounds__((GT_PRODUCER_WARPS + 1 + EW + 1) * 32, 1)
       const float *xrow = g.gx + (int64_t)__ldg(g.sender + ee) * C + 16 * hf;
       float y[16];
 #pragma unroll
-      for (int m = 0; m < 16; m++) y[m] = in ? __ldg(g.gy + (int64_t)m * g.M + ee) : 0.f;
+      for (int m = 0; m < 16; m++) y[m] = in ? __ldg(g.gy + m * g.y_m + ee * g.y_e) : 0.f;
       const bool staged = my_recv - r_first < nstaged;
       const bool warp_staged = __all_sync(0xffffffffu, staged);
       const uint32_t gs = g_stage0 + buf * g_half + (uint32_t)((my_recv - r_first) * 16 * C + 16 * hf) * 4u;
@@ -1460,6 +1461,30 @@ static int gemm_launch(GemmArgs &g, const char *what, cudaStream_t st) {
   return check_launch(what);
 }
 
+int gemm3x_gradr(const float *X, const float *G, const float *Y, YStride ys, const int32_t *sender,
+                 const int32_t *receiver, const float *packed, int64_t nedges, int channels, int N, float *out,
+                 int32_t *status, cmace_stream_t stream) {
+  if (nedges < 0 || N < 32 || N > 128 || N % 4 != 0)
+    return fail(CMACE_ERR_UNSUPPORTED, "cmace_gemm3x_gradr: the hidden width must be a multiple of 4 in 32..128");
+  if (channels < 32 || channels > 128 || channels % 32 != 0)
+    return fail(CMACE_ERR_UNSUPPORTED, "cmace_gemm3x_gradr: channels must be 32, 64, 96 or 128");
+  if (nedges == 0) return CMACE_OK;
+  if (!X || !G || !Y || !sender || !receiver || !packed || !out)
+    return fail(CMACE_ERR_ARG, "cmace_gemm3x_gradr: null pointer");
+  if (!aligned16(X) || !aligned16(G) || !aligned16(packed) || !aligned16(out))
+    return fail(CMACE_ERR_ARG, "cmace_gemm3x_gradr: pointers must be 16-byte aligned");
+  const int K = 4 * channels;
+  const PackGeom p = pack_geom(N, K);
+  GemmArgs g{};
+  g.packed = packed; g.out = out; g.status = status;
+  g.gx = X; g.gg = G; g.gy = Y; g.sender = sender; g.receiver = receiver; g.C = channels;
+  g.y_m = ys.m; g.y_e = ys.e;
+  g.M = nedges; g.K = K; g.N = N; g.nelements = 1; g.mode = GT_MODE_GRADR; g.scale = 1.0f;
+  g.n_tiles = p.n_tiles; g.k_blocks = p.k_blocks; g.npad = p.npad;
+  g.total_tiles = (nedges + GT_TILE_M - 1) / GT_TILE_M;
+  return gemm_launch(g, "cmace_gemm3x_gradr", (cudaStream_t)stream);
+}
+
 }  // namespace cmace
 
 using namespace cmace;
@@ -1514,24 +1539,7 @@ int cmace_bounded_wait_probe(int32_t *status, int code, double limit_seconds, cm
 int cmace_gemm3x_gradr_f32(const float *X, const float *G, const float *Y, const int32_t *sender,
                            const int32_t *receiver, const float *packed, int64_t nedges, int channels, int N,
                            float *out, int32_t *status, cmace_stream_t stream) {
-  if (nedges < 0 || N < 32 || N > 128 || N % 4 != 0)
-    return fail(CMACE_ERR_UNSUPPORTED, "cmace_gemm3x_gradr: the hidden width must be a multiple of 4 in 32..128");
-  if (channels < 32 || channels > 128 || channels % 32 != 0)
-    return fail(CMACE_ERR_UNSUPPORTED, "cmace_gemm3x_gradr: channels must be 32, 64, 96 or 128");
-  if (nedges == 0) return CMACE_OK;
-  if (!X || !G || !Y || !sender || !receiver || !packed || !out)
-    return fail(CMACE_ERR_ARG, "cmace_gemm3x_gradr: null pointer");
-  if (!aligned16(X) || !aligned16(G) || !aligned16(packed) || !aligned16(out))
-    return fail(CMACE_ERR_ARG, "cmace_gemm3x_gradr: pointers must be 16-byte aligned");
-  const int K = 4 * channels;
-  const PackGeom p = pack_geom(N, K);
-  GemmArgs g{};
-  g.packed = packed; g.out = out; g.status = status;
-  g.gx = X; g.gg = G; g.gy = Y; g.sender = sender; g.receiver = receiver; g.C = channels;
-  g.M = nedges; g.K = K; g.N = N; g.nelements = 1; g.mode = GT_MODE_GRADR; g.scale = 1.0f;
-  g.n_tiles = p.n_tiles; g.k_blocks = p.k_blocks; g.npad = p.npad;
-  g.total_tiles = (nedges + GT_TILE_M - 1) / GT_TILE_M;
-  return gemm_launch(g, "cmace_gemm3x_gradr", (cudaStream_t)stream);
+  return cmace::gemm3x_gradr(X, G, Y, YStride{nedges, 1}, sender, receiver, packed, nedges, channels, N, out, status, stream);
 }
 
 int cmace_linear_tc_f32(const float *X, const float *packed, const int32_t *node_order, const int32_t *elem_start,

@@ -28,7 +28,7 @@ template <typename T, int VEC>
 __global__ void __launch_bounds__(kWarpsPerBlock * 32)
     imp_fwd_kernel(const T *__restrict__ X, const T *__restrict__ Y, const T *__restrict__ R,
                    const int32_t *__restrict__ sender, const int32_t *__restrict__ row_ptr,
-                   int64_t nnodes, int64_t nedges, int C, T *__restrict__ out) {
+                   int64_t nnodes, YStride ys, int C, T *__restrict__ out) {
   const int lane = threadIdx.x & 31;
   const int64_t node = (int64_t)blockIdx.x * kWarpsPerBlock + (threadIdx.x >> 5);
   if (node >= nnodes) return;
@@ -46,7 +46,7 @@ __global__ void __launch_bounds__(kWarpsPerBlock * 32)
     // second edge of the pair: clamp to a valid edge, its harmonics are zeroed below
     const int64_t eb = (e + 1 < e1) ? e + 1 : e;
     const int64_t ey = yedge ? eb : e;
-    T yv = __ldg(Y + (int64_t)ylm * nedges + ey);
+    T yv = __ldg(Y + ylm * ys.m + ey * ys.e);
     if (yedge && e + 1 >= e1) yv = T(0);
     const int64_t sa = sender[e], sb = sender[eb];
     T xa[VEC], xb[VEC], ra[4][VEC], rb[4][VEC];
@@ -124,7 +124,7 @@ template <typename T, int VEC>
 __global__ void __launch_bounds__(kWarpsPerBlock * 32)
     imp_bwd_edge_kernel(const T *__restrict__ X, const T *__restrict__ Y, const T *__restrict__ R,
                         const T *__restrict__ G, const int32_t *__restrict__ sender,
-                        const int32_t *__restrict__ row_ptr, int64_t nnodes, int64_t nedges, int C,
+                        const int32_t *__restrict__ row_ptr, int64_t nnodes, int64_t nedges, YStride ys, int C,
                         T *__restrict__ gradR, T *__restrict__ gradY_out, T *__restrict__ Tout) {
   const int lane = threadIdx.x & 31;
   const int64_t node = (int64_t)blockIdx.x * kWarpsPerBlock + (threadIdx.x >> 5);
@@ -142,7 +142,7 @@ __global__ void __launch_bounds__(kWarpsPerBlock * 32)
   const int ylm = lane & 15, yedge = lane >> 4;
   for (int64_t e = e0; e < e1; e += 2) {
     const int64_t eb = (e + 1 < e1) ? e + 1 : e;
-    const T yv = __ldg(Y + (int64_t)ylm * nedges + (yedge ? eb : e));
+    const T yv = __ldg(Y + ylm * ys.m + (yedge ? eb : e) * ys.e);
     // loads of both edges of the pair are issued before either is consumed
     const int64_t s2[2] = {sender[e], sender[eb]};
     T xx[2][VEC], rr[2][4][VEC];
@@ -189,7 +189,7 @@ __global__ void __launch_bounds__(kWarpsPerBlock * 32)
       }
       if (Tout != nullptr) store_vec<T, VEC>(Tout + ee * C + c0, t);
       const T tot = warp_reduce16(p, lane);
-      if ((lane & 1) == 0) gy[(int64_t)(lane >> 1) * nedges + ee] = tot;
+      if ((lane & 1) == 0) gy[(lane >> 1) * ys.m + ee * ys.e] = tot;
     }
   }
 }
@@ -254,7 +254,7 @@ template <bool WANT_T, bool WANT_GR>
 __global__ void __launch_bounds__(BS_WARPS * 32, 1)
     imp_bwd_edge_staged_kernel(const float *__restrict__ X, const float *__restrict__ Y, const float *__restrict__ R,
                                const float *__restrict__ G, const int32_t *__restrict__ sender,
-                               const int32_t *__restrict__ row_ptr, int64_t nnodes, int64_t nedges,
+                               const int32_t *__restrict__ row_ptr, int64_t nnodes, int64_t nedges, YStride ys,
                                float *__restrict__ gradR, float *__restrict__ gy, float *__restrict__ Tout,
                                int *__restrict__ stalled) {
   extern __shared__ __align__(128) unsigned char bs_smem[];
@@ -308,13 +308,13 @@ __global__ void __launch_bounds__(BS_WARPS * 32, 1)
   constexpr bool WANT_U = WANT_T || WANT_GR;
   unsigned long long g2[16][2];   // G[node, m, c0 .. c0 + 3] as two register pairs
   int64_t g_node = -1;
-  float yv_next = (WANT_U && cc.e >= 0) ? __ldg(Y + (int64_t)ylm * nedges + cc.e) : 0.f;
+  float yv_next = (WANT_U && cc.e >= 0) ? __ldg(Y + ylm * ys.m + cc.e * ys.e) : 0.f;
   while (cc.e >= 0) {
     const int64_t e = cc.e, node = cc.node;
     EdgeCursor nc = cc;
     cursor_next(nc, row_ptr);
     const float yv = yv_next;
-    if (WANT_U && nc.e >= 0) yv_next = __ldg(Y + (int64_t)ylm * nedges + nc.e);
+    if (WANT_U && nc.e >= 0) yv_next = __ldg(Y + ylm * ys.m + nc.e * ys.e);
     if (node != g_node) {
       g_node = node;
 #pragma unroll
@@ -416,7 +416,7 @@ __global__ void __launch_bounds__(BS_WARPS * 32, 1)
     issue_one();
     if (WANT_T) store_vec<float, 4>(Tout + e * BS_C + c0, t);
     const float tot = warp_reduce16(p, lane);
-    if ((lane & 1) == 0) gy[(int64_t)(lane >> 1) * nedges + e] = tot;
+    if ((lane & 1) == 0) gy[(lane >> 1) * ys.m + e * ys.e] = tot;
     cc = nc;
   }
 }
@@ -486,16 +486,16 @@ static int check_common(const void *a, const void *b, const void *c, int64_t nno
 
 template <typename T, int VEC>
 static void launch_fwd(const T *X, const T *Y, const T *R, const int32_t *sender,
-                       const int32_t *row_ptr, int64_t nnodes, int64_t nedges, int C, T *out,
+                       const int32_t *row_ptr, int64_t nnodes, YStride ys, int C, T *out,
                        cudaStream_t st) {
   dim3 grid((unsigned)((nnodes + kWarpsPerBlock - 1) / kWarpsPerBlock), C / (32 * VEC));
   imp_fwd_kernel<T, VEC><<<grid, kWarpsPerBlock * 32, 0, st>>>(X, Y, R, sender, row_ptr, nnodes,
-                                                                nedges, C, out);
+                                                                ys, C, out);
 }
 
 template <typename T>
-static int imp_fwd(const T *X, const T *Y, const T *R, const int32_t *sender, const int32_t *row_ptr,
-                   int64_t nnodes, int64_t nedges, int C, T *out, cmace_stream_t stream) {
+int imp_fwd(const T *X, const T *Y, const T *R, const int32_t *sender, const int32_t *row_ptr,
+            int64_t nnodes, int64_t nedges, YStride ys, int C, T *out, cmace_stream_t stream) {
   int rc = check_common<T>(X, R, out, nnodes, nedges, C, "cmace_imp_fwd");
   if (rc) return rc;
   if (nnodes == 0) return CMACE_OK;
@@ -504,21 +504,21 @@ static int imp_fwd(const T *X, const T *Y, const T *R, const int32_t *sender, co
   cudaStream_t st = (cudaStream_t)stream;
   switch (pick_vec<T>(C)) {
     case 4:
-      if constexpr (sizeof(T) == 4) launch_fwd<T, 4>(X, Y, R, sender, row_ptr, nnodes, nedges, C, out, st);
+      if constexpr (sizeof(T) == 4) launch_fwd<T, 4>(X, Y, R, sender, row_ptr, nnodes, ys, C, out, st);
       break;
-    case 2: launch_fwd<T, 2>(X, Y, R, sender, row_ptr, nnodes, nedges, C, out, st); break;
-    default: launch_fwd<T, 1>(X, Y, R, sender, row_ptr, nnodes, nedges, C, out, st); break;
+    case 2: launch_fwd<T, 2>(X, Y, R, sender, row_ptr, nnodes, ys, C, out, st); break;
+    default: launch_fwd<T, 1>(X, Y, R, sender, row_ptr, nnodes, ys, C, out, st); break;
   }
   return check_launch("cmace_imp_fwd");
 }
 
 template <typename T, int VEC>
 static void launch_bwd_edge(const T *X, const T *Y, const T *R, const T *G, const int32_t *sender,
-                            const int32_t *row_ptr, int64_t nnodes, int64_t nedges, int C, T *gradR,
+                            const int32_t *row_ptr, int64_t nnodes, int64_t nedges, YStride ys, int C, T *gradR,
                             T *gy, T *Tout, cudaStream_t st) {
   dim3 grid((unsigned)((nnodes + kWarpsPerBlock - 1) / kWarpsPerBlock), C / (32 * VEC));
   imp_bwd_edge_kernel<T, VEC><<<grid, kWarpsPerBlock * 32, 0, st>>>(X, Y, R, G, sender, row_ptr,
-                                                                     nnodes, nedges, C, gradR, gy, Tout);
+                                                                     nnodes, nedges, ys, C, gradR, gy, Tout);
 }
 
 static __device__ int g_staged_stall;   // set when a bounded wait of the staged edge pass gave up
@@ -534,8 +534,8 @@ static int *staged_stall_flag() {
 }
 
 template <typename T>
-static int imp_bwd_edge(const T *X, const T *Y, const T *R, const T *G, const int32_t *sender,
-                        const int32_t *row_ptr, int64_t nnodes, int64_t nedges, int C, T *gradR,
+int imp_bwd_edge(const T *X, const T *Y, const T *R, const T *G, const int32_t *sender,
+                        const int32_t *row_ptr, int64_t nnodes, int64_t nedges, YStride ys, int C, T *gradR,
                         T *gradY, T *Tout, T *partial, cmace_stream_t stream) {
   int rc = check_common<T>(X, R, G, nnodes, nedges, C, "cmace_imp_bwd_edge");
   if (rc) return rc;
@@ -565,7 +565,7 @@ static int imp_bwd_edge(const T *X, const T *Y, const T *R, const T *G, const in
       auto launch = [&](auto kernel) -> int {
         cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
         if (e != cudaSuccess) return fail(CMACE_ERR_CUDA, "cmace_imp_bwd_edge: %s", cudaGetErrorString(e));
-        kernel<<<(unsigned)blocks, BS_WARPS * 32, smem, st>>>(X, Y, R, G, sender, row_ptr, nnodes, nedges, gradR, gy,
+        kernel<<<(unsigned)blocks, BS_WARPS * 32, smem, st>>>(X, Y, R, G, sender, row_ptr, nnodes, nedges, ys, gradR, gy,
                                                               Tout, staged_stall_flag());
         return check_launch("cmace_imp_bwd_edge");
       };
@@ -578,10 +578,10 @@ static int imp_bwd_edge(const T *X, const T *Y, const T *R, const T *G, const in
   switch (vec) {
     case 4:
       if constexpr (sizeof(T) == 4)
-        launch_bwd_edge<T, 4>(X, Y, R, G, sender, row_ptr, nnodes, nedges, C, gradR, gy, Tout, st);
+        launch_bwd_edge<T, 4>(X, Y, R, G, sender, row_ptr, nnodes, nedges, ys, C, gradR, gy, Tout, st);
       break;
-    case 2: launch_bwd_edge<T, 2>(X, Y, R, G, sender, row_ptr, nnodes, nedges, C, gradR, gy, Tout, st); break;
-    default: launch_bwd_edge<T, 1>(X, Y, R, G, sender, row_ptr, nnodes, nedges, C, gradR, gy, Tout, st); break;
+    case 2: launch_bwd_edge<T, 2>(X, Y, R, G, sender, row_ptr, nnodes, nedges, ys, C, gradR, gy, Tout, st); break;
+    default: launch_bwd_edge<T, 1>(X, Y, R, G, sender, row_ptr, nnodes, nedges, ys, C, gradR, gy, Tout, st); break;
   }
   rc = check_launch("cmace_imp_bwd_edge");
   if (rc) return rc;
@@ -601,7 +601,7 @@ static void launch_bwd_node(const T *Tin, const int32_t *perm, const int32_t *se
 }
 
 template <typename T>
-static int imp_bwd_node(const T *Tin, const int32_t *perm, const int32_t *send_ptr, int64_t nnodes,
+int imp_bwd_node(const T *Tin, const int32_t *perm, const int32_t *send_ptr, int64_t nnodes,
                         int C, T *gradX, cmace_stream_t stream) {
   int rc = check_common<T>(Tin, gradX, gradX, nnodes, 0, C, "cmace_imp_bwd_node");
   if (rc) return rc;
@@ -617,6 +617,14 @@ static int imp_bwd_node(const T *Tin, const int32_t *perm, const int32_t *send_p
   }
   return check_launch("cmace_imp_bwd_node");
 }
+
+#define CMACE_IMP_LAUNCHERS(T)                                                                                        \
+  template int imp_fwd<T>(const T *, const T *, const T *, const int32_t *, const int32_t *, int64_t, int64_t, YStride, \
+                          int, T *, cmace_stream_t);                                                                   \
+  template int imp_bwd_edge<T>(const T *, const T *, const T *, const T *, const int32_t *, const int32_t *, int64_t,  \
+                               int64_t, YStride, int, T *, T *, T *, T *, cmace_stream_t);
+CMACE_IMP_LAUNCHERS(float)
+CMACE_IMP_LAUNCHERS(double)
 
 // ---- variant without caller scratch -------------------------------------------------------------
 // Some callers cannot hand over scratch memory because they cannot allocate on the device at the point
@@ -668,12 +676,12 @@ int cmace_imp_staged_stalled(void) {
 int cmace_imp_fwd_f32(const float *X, const float *Y, const float *R, const int32_t *sender,
                       const int32_t *row_ptr, int64_t nnodes, int64_t nedges, int channels, float *out,
                       cmace_stream_t stream) {
-  return imp_fwd<float>(X, Y, R, sender, row_ptr, nnodes, nedges, channels, out, stream);
+  return imp_fwd<float>(X, Y, R, sender, row_ptr, nnodes, nedges, YStride{nedges, 1}, channels, out, stream);
 }
 int cmace_imp_fwd_f64(const double *X, const double *Y, const double *R, const int32_t *sender,
                       const int32_t *row_ptr, int64_t nnodes, int64_t nedges, int channels, double *out,
                       cmace_stream_t stream) {
-  return imp_fwd<double>(X, Y, R, sender, row_ptr, nnodes, nedges, channels, out, stream);
+  return imp_fwd<double>(X, Y, R, sender, row_ptr, nnodes, nedges, YStride{nedges, 1}, channels, out, stream);
 }
 int64_t cmace_imp_bwd_scratch_elems(int64_t nedges, int channels, int is_f64) {
   if (channels <= 0 || channels % 32 != 0) return 0;
@@ -685,14 +693,14 @@ int cmace_imp_bwd_edge_f32(const float *X, const float *Y, const float *R, const
                            const int32_t *sender, const int32_t *row_ptr, int64_t nnodes, int64_t nedges,
                            int channels, float *gradR, float *gradY, float *T, float *gradY_partial,
                            cmace_stream_t stream) {
-  return imp_bwd_edge<float>(X, Y, R, G, sender, row_ptr, nnodes, nedges, channels, gradR, gradY, T,
+  return imp_bwd_edge<float>(X, Y, R, G, sender, row_ptr, nnodes, nedges, YStride{nedges, 1}, channels, gradR, gradY, T,
                              gradY_partial, stream);
 }
 int cmace_imp_bwd_edge_f64(const double *X, const double *Y, const double *R, const double *G,
                            const int32_t *sender, const int32_t *row_ptr, int64_t nnodes, int64_t nedges,
                            int channels, double *gradR, double *gradY, double *T, double *gradY_partial,
                            cmace_stream_t stream) {
-  return imp_bwd_edge<double>(X, Y, R, G, sender, row_ptr, nnodes, nedges, channels, gradR, gradY, T,
+  return imp_bwd_edge<double>(X, Y, R, G, sender, row_ptr, nnodes, nedges, YStride{nedges, 1}, channels, gradR, gradY, T,
                               gradY_partial, stream);
 }
 int64_t cmace_imp_bwd_edge_f64_noalloc_max_elems(void) { return kStaticScratchElems; }
@@ -715,7 +723,7 @@ int cmace_imp_bwd_edge_f64_noalloc(const double *X, const double *Y, const doubl
     if (e != cudaSuccess)
       return fail(CMACE_ERR_CUDA, "cmace_imp_bwd_edge_f64_noalloc: %s", cudaGetErrorString(e));
   }
-  return imp_bwd_edge<double>(X, Y, R, G, sender, row_ptr, nnodes, nedges, channels, gradR, gradY, T, scratch,
+  return imp_bwd_edge<double>(X, Y, R, G, sender, row_ptr, nnodes, nedges, YStride{nedges, 1}, channels, gradR, gradY, T, scratch,
                               stream);
 }
 

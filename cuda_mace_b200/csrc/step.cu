@@ -1,0 +1,241 @@
+// The whole energy+force step of a two-layer invariant model as one sequence of launches (cmace_step_run).
+//
+//   edge_prep     unit vectors, Y [E, 16], basis and its derivative; nodes grouped by element beside it
+//   radial        both perceptrons' hidden layers h and h' = dh/dr                        (radial_tangent.cu)
+//   sums          first layer: A[i, lm, (z, k)] = sum_{e in (i, z)} Y h                   (step_edges.cu)
+//   fold          A times the element-dependent matrices that hold everything up to the layer's Linear
+//   contract0     b0
+//   mid_fwd       up = b0 Wu, q0 = b0 Wsc[z], e0 = b0 . w0                                (step_nodes.cu)
+//       -- a decomposed system fills the ghost rows of `up` here --
+//   radial_out    second layer: R = h W4 [E, 4C]
+//   messages, linear, contract1 (value, readout, energy and gradient in one kernel), linear_back
+//   edges_back    T [E, C] and grad Y of the second layer; radial_back, radial_dot: dE/dr of the second layer
+//   senders       grad up = sum of T over a sender's edges
+//       -- and returns the gradients of the ghost rows here --
+//   mid_back, contract0_back, fold_back
+//   sums_back     grad Y and dE/dr of the first layer, plus the second layer's: gradient of every edge vector
+//   forces        position gradient and energies
+//
+// Nodes of the first layer are kept in element order (slots) between `sums` and `mid_fwd` and on the way back, so the
+// element-dependent products see consecutive rows whatever the caller's order is.
+#include <cstring>
+
+#include "step_common.cuh"
+
+namespace cmace {
+
+int radial_pair_f32(const float *basis, int nb, const float *const (*w)[3], int nper, int64_t nedges, float *const *h,
+                    float *const *dh, int32_t *status, cudaStream_t st);
+int radial_pair_f64(const double *basis, int nb, const double *const (*w)[3], int nper, int64_t nedges,
+                    double *const *h, double *const *dh, cudaStream_t st);
+
+enum StepId {
+  S_EDGE_PREP, S_RADIAL, S_SUMS, S_FOLD, S_CONTRACT0, S_MID_FWD,
+  S_RADIAL_OUT, S_MESSAGES, S_LINEAR, S_CONTRACT1, S_LINEAR_BACK, S_EDGES_BACK, S_RADIAL_BACK, S_RADIAL_DOT, S_SENDERS,
+  S_MID_BACK, S_CONTRACT0_BACK, S_FOLD_BACK, S_SUMS_BACK, S_FORCES, S_COUNT
+};
+static const char *const kStepNames[S_COUNT] = {
+    "edge_prep", "radial", "sums", "fold", "contract0", "mid_fwd",
+    "radial_out", "messages", "linear", "contract1", "linear_back", "edges_back", "radial_back", "radial_dot", "senders",
+    "mid_back", "contract0_back", "fold_back", "sums_back", "forces"};
+
+// dE/dr [E] = sum_k grad h[e, k] h'[e, k]: half a warp per edge
+template <typename T>
+__global__ void __launch_bounds__(256)
+    radial_dot_kernel(const T *__restrict__ gh, const T *__restrict__ dh, int64_t nedges, T *__restrict__ dr) {
+  const int64_t e = ((int64_t)blockIdx.x * 256 + threadIdx.x) >> 4;
+  const int l16 = threadIdx.x & 15;
+  T s = T(0);
+  if (e < nedges) {
+    const Quad<T> a = reinterpret_cast<const Quad<T> *>(gh + e * ST_H)[l16];
+    const Quad<T> b = reinterpret_cast<const Quad<T> *>(dh + e * ST_H)[l16];
+    s = fma(a.x, b.x, fma(a.y, b.y, fma(a.z, b.z, a.w * b.w)));
+  }
+#pragma unroll
+  for (int off = 8; off > 0; off >>= 1) s += __shfl_xor_sync(0xffffffffu, s, off);
+  if (l16 == 0 && e < nedges) dr[e] = s;
+}
+
+template <typename T>
+struct Workspace {
+  int32_t *species, *slot_of, *node_of, *slot_type, *elem_start;
+  Quad<T> *geo;
+  T *basis, *Y, *h[2], *dh[2], *A, *m0, *b0, *up, *R, *m1, *l1, *gX1, *gm1, *T_, *gY1, *gH1, *dr1, *gup, *gb0, *gX0, *gA,
+      *gvec, *gradR, *partial;
+  double *q0, *e0, *dq;
+  int64_t bytes;
+
+  Workspace(void *base, const cmace_step_model &m, int64_t n, int64_t nl, int64_t E) {
+    char *p = static_cast<char *>(base);
+    bytes = 0;
+    auto take = [&](auto *&ptr, int64_t count) {
+      using U = typename std::remove_reference<decltype(*ptr)>::type;
+      ptr = reinterpret_cast<U *>(p + bytes);
+      bytes += (count * (int64_t)sizeof(U) + 255) / 256 * 256;
+    };
+    const int64_t C = m.channels, Z = m.elements;
+    take(species, nl);
+    take(slot_of, n);
+    take(node_of, n);
+    take(slot_type, n);
+    take(elem_start, Z + 1);
+    take(geo, E);
+    take(basis, E * 2 * m.nbessel);
+    take(Y, E * 16);
+    for (int i = 0; i < 2; i++) {
+      take(h[i], E * ST_H);
+      take(dh[i], E * ST_H);
+    }
+    take(A, n * 16 * ST_H * Z);
+    take(m0, n * 16 * C);
+    take(b0, n * C);
+    take(up, n * C);
+    take(q0, n * ST_RO);
+    take(e0, n);
+    take(R, E * 4 * C);
+    take(m1, n * 16 * C);
+    take(l1, n * 16 * C);
+    take(gX1, n * 16 * C);
+    take(dq, n * ST_RO);
+    take(T_, E * C);
+    take(gY1, E * 16);
+    take(gH1, E * ST_H);
+    take(dr1, E);
+    take(gup, nl * C);
+    take(gb0, n * C);
+    take(gX0, n * 16 * C);
+    take(gvec, E * 3);
+    take(gradR, sizeof(T) == 8 ? E * 4 * C : 0);
+    take(partial, cmace_imp_bwd_scratch_elems(E, (int)C, sizeof(T) == 8 ? 1 : 0));
+    gm1 = m1;   // the messages are not read again after the Linear
+    gA = A;     // nor the sums after their product
+  }
+};
+
+static int linear_any(const float *X, const void *W, const int32_t *start, int nel, int64_t n, int K, int N, float *out,
+                      int32_t *status, cmace_stream_t st) {
+  return cmace_linear_tc_f32(X, static_cast<const float *>(W), nullptr, start, nel, n, K, N, 1.0, out, status, st);
+}
+static int linear_any(const double *X, const void *W, const int32_t *start, int nel, int64_t n, int K, int N, double *out,
+                      int32_t *, cmace_stream_t st) {
+  return cmace_linear_f64(X, static_cast<const double *>(W), nullptr, start, nel, n, K, N, 1.0, out, st);
+}
+
+template <typename T>
+static int run_step(const cmace_step_model &m, cmace_step_io &io, const Workspace<T> &w, int step, cudaStream_t st) {
+  using K = StepKernels<T>;
+  const int64_t n = io.n_owned, nl = io.n_local, E = io.nedges;
+  const int C = m.channels, Z = m.elements;
+  const T *up = io.up_local ? static_cast<const T *>(io.up_local) : w.up;
+  T *gup = io.gup_local ? static_cast<T *>(io.gup_local) : w.gup;
+  const T *gup_owned = io.gup_owned ? static_cast<const T *>(io.gup_owned) : gup;
+  const YStride ys{1, 16};
+  const int32_t *start = Z > 1 ? w.elem_start : nullptr;
+  constexpr bool f64 = sizeof(T) == 8;
+  io.launches++;
+  switch (step) {
+    case S_EDGE_PREP:
+      return K::edge_prep(io.positions, io.sender, io.receiver, io.shifts, E, m.r_max, m.nbessel, m.cutoff_p, w.geo,
+                          w.basis, w.Y, io.species, io.one_hot, io.one_hot_is_f64, nl, n, Z, w.species, w.slot_of,
+                          w.node_of, w.slot_type, w.elem_start, st);
+    case S_RADIAL: {
+      const T *rw[2][3];
+      for (int i = 0; i < 2; i++)
+        for (int k = 0; k < 3; k++) rw[i][k] = static_cast<const T *>(m.radial[i][k]);
+      if constexpr (f64) return radial_pair_f64(w.basis, m.nbessel, rw, 2, E, w.h, w.dh, st);
+      else return radial_pair_f32(w.basis, m.nbessel, rw, 2, E, w.h, w.dh, io.status, st);
+    }
+    case S_SUMS: return K::sums(w.h[0], w.Y, io.sender, io.row_ptr, w.species, w.slot_of, n, Z, w.A, st);
+    case S_FOLD: return linear_any(w.A, m.fold, start, Z, n, ST_H * Z, C, w.m0, io.status, st);
+    case S_CONTRACT0: return K::contract_fwd(w.m0, w.slot_type, static_cast<const T *>(m.weff[0]), n, C, w.b0, st);
+    case S_MID_FWD:
+      return K::mid_fwd(w.b0, w.slot_of, w.species, static_cast<const T *>(m.up), m.skip, m.readout0, n, C,
+                        io.up_local ? static_cast<T *>(io.up_local) : w.up, w.q0, w.e0, st);
+    case S_RADIAL_OUT:
+      if constexpr (f64) return cmace_gemm_f64(w.h[1], static_cast<const double *>(m.radial[1][3]), E, ST_H, 4 * C, 1.0, w.R, st);
+      else return cmace_gemm3x_f32(w.h[1], static_cast<const float *>(m.radial[1][3]), E, ST_H, 4 * C, 1.0, w.R, io.status, st);
+    case S_MESSAGES: return imp_fwd<T>(up, w.Y, w.R, io.sender, io.row_ptr, n, E, ys, C, w.m1, st);
+    case S_LINEAR: return linear_any(w.m1, m.linear[0], nullptr, 1, n, C, C, w.l1, io.status, st);
+    case S_CONTRACT1:
+      return K::contract_readout(w.l1, w.species, static_cast<const T *>(m.weff[1]), m.readout1, m.readout2, w.q0, w.e0,
+                                 m.atomic_energies, m.scale, m.shift, n, C, w.gX1, w.dq, io.interaction, io.node_energy, st);
+    case S_LINEAR_BACK: return linear_any(w.gX1, m.linear[1], nullptr, 1, n, C, C, w.gm1, io.status, st);
+    case S_EDGES_BACK:
+      return imp_bwd_edge<T>(up, w.Y, w.R, w.gm1, io.sender, io.row_ptr, n, E, ys, C, f64 ? w.gradR : nullptr, w.gY1,
+                             w.T_, w.partial, st);
+    case S_RADIAL_BACK:
+      if constexpr (f64)
+        return cmace_gemm_f64(w.gradR, static_cast<const double *>(m.radial_back), E, 4 * C, ST_H, 1.0, w.gH1, st);
+      else
+        return gemm3x_gradr(up, w.gm1, w.Y, ys, io.sender, io.receiver, static_cast<const float *>(m.radial_back), E, C,
+                            ST_H, w.gH1, io.status, st);
+    case S_RADIAL_DOT:
+      if (E > 0) radial_dot_kernel<T><<<(unsigned)((E + 15) / 16), 256, 0, st>>>(w.gH1, w.dh[1], E, w.dr1);
+      return check_launch("cmace_step(radial_dot)");
+    case S_SENDERS:
+      if constexpr (f64) return cmace_imp_bwd_node_f64(w.T_, io.perm, io.send_ptr, nl, C, gup, st);
+      else return cmace_imp_bwd_node_f32(w.T_, io.perm, io.send_ptr, nl, C, gup, st);
+    case S_MID_BACK:
+      return K::mid_bwd(gup_owned, w.slot_of, w.species, w.dq, static_cast<const T *>(m.up_back), m.skip, m.readout0,
+                        m.scale, n, C, w.gb0, st);
+    case S_CONTRACT0_BACK:
+      return K::contract_bwd(w.m0, w.slot_type, static_cast<const T *>(m.weff[0]), w.gb0, n, C, w.gX0, st);
+    case S_FOLD_BACK:
+      for (int b = 0; 2 * b < Z; b++) {
+        if (int rc = linear_any(w.gX0, m.fold_back[b], start, Z, n, C, sums_block_width(Z, b),
+                                w.gA + (int64_t)b * n * (16 * 128), io.status, st))
+          return rc;
+        if (b) io.launches++;
+      }
+      return CMACE_OK;
+    case S_SUMS_BACK:
+      return K::sums_bwd(w.gA, w.h[0], w.dh[0], w.Y, io.sender, io.row_ptr, w.species, w.slot_of, w.gY1, w.dr1, w.geo, n,
+                         Z, w.gvec, st);
+    case S_FORCES:
+      return K::forces(w.gvec, io.row_ptr, io.perm, io.send_ptr, n, nl, io.gradient_sign, io.gradient, io.interaction,
+                       io.node_energy, io.sums, st);
+  }
+  return fail(CMACE_ERR_ARG, "cmace_step: no step %d", step);
+}
+
+template <typename T>
+static int run_steps(const cmace_step_model &m, cmace_step_io &io, int first, int last, cudaStream_t st) {
+  const Workspace<T> w(io.workspace, m, io.n_owned, io.n_local, io.nedges);
+  if (io.workspace_bytes < w.bytes)
+    return fail(CMACE_ERR_ARG, "cmace_step: workspace of %lld bytes, %lld needed", (long long)io.workspace_bytes, (long long)w.bytes);
+  for (int s = first; s < last; s++)
+    if (int rc = run_step<T>(m, io, w, s, st)) return rc;
+  return CMACE_OK;
+}
+
+}  // namespace cmace
+
+using namespace cmace;
+
+extern "C" {
+
+int64_t cmace_step_workspace_bytes(const cmace_step_model *m, int64_t n_owned, int64_t n_local, int64_t nedges) {
+  if (!m || n_owned < 0 || n_local < n_owned || nedges < 0) return 0;
+  return m->is_f64 ? Workspace<double>(nullptr, *m, n_owned, n_local, nedges).bytes
+                   : Workspace<float>(nullptr, *m, n_owned, n_local, nedges).bytes;
+}
+int cmace_step_count(void) { return S_COUNT; }
+const char *cmace_step_name(int step) { return step >= 0 && step < S_COUNT ? kStepNames[step] : ""; }
+
+int cmace_step_run(const cmace_step_model *m, cmace_step_io *io, int first, int last, cmace_stream_t stream) {
+  if (!m || !io || first < 0 || last > S_COUNT || first > last) return fail(CMACE_ERR_ARG, "cmace_step: bad argument");
+  if (m->channels % 32 != 0 || m->channels < 32 || m->channels > 128 || m->elements < 1 || m->elements > ST_MAX_Z ||
+      (m->nbessel != 8 && m->nbessel != 16))
+    return fail(CMACE_ERR_UNSUPPORTED, "cmace_step: 32, 64, 96 or 128 channels, 1..%d elements, 8 or 16 basis functions", ST_MAX_Z);
+  if (io->n_owned < 1 || io->n_local < io->n_owned || io->nedges < 0 || io->nedges > 0x7fffff00LL)
+    return fail(CMACE_ERR_ARG, "cmace_step: bad size");
+  if (!io->positions || (!io->species && !io->one_hot) || !io->row_ptr || !io->send_ptr || !io->workspace ||
+      !io->node_energy || !io->interaction || !io->sums || !io->gradient ||
+      (io->nedges > 0 && (!io->sender || !io->receiver || !io->perm)))
+    return fail(CMACE_ERR_ARG, "cmace_step: null pointer");
+  if (io->n_local != io->n_owned && (!io->up_local || !io->gup_local || !io->gup_owned))
+    return fail(CMACE_ERR_ARG, "cmace_step: ghost rows need the caller's node feature arrays");
+  cudaStream_t st = (cudaStream_t)stream;
+  return m->is_f64 ? run_steps<double>(*m, *io, first, last, st) : run_steps<float>(*m, *io, first, last, st);
+}
+}

@@ -1,0 +1,49 @@
+// Shapes and array layouts shared by the kernels of the whole energy+force step (step.cu holds the sequence).
+#pragma once
+#include "common.cuh"
+
+namespace cmace {
+
+constexpr int ST_H = 64;          // hidden width of the radial perceptron
+constexpr int ST_RO = 16;         // hidden width of the second layer's readout
+constexpr int ST_MAX_Z = 16;      // elements the step's kernels are laid out for
+constexpr int ST_NW = 13;         // effective contraction weights per (element, channel): 8 cubic, 4 quadratic, 1 linear
+
+template <typename T>
+struct alignas(4 * sizeof(T)) Quad {
+  T x, y, z, w;
+};
+
+// Gradients of the first layer's sums leave the element-dependent product in blocks of at most two elements:
+// block b is a [nodes, 16, width(b)] array, width = 64 times the elements it holds.
+__host__ __device__ inline int sums_block_width(int elements, int b) { return elements - 2 * b >= 2 ? 128 : 64; }
+
+// launchers (one per kernel; every one checks its launch)
+template <typename T>
+struct StepKernels {
+  static int edge_prep(const double *pos, const int32_t *sender, const int32_t *receiver, const double *shifts,
+                       int64_t nedges, double r_max, int nb, int p, Quad<T> *geo, T *basis, T *Y,
+                       const int32_t *species_in, const void *one_hot, int one_hot_f64, int64_t n_local, int64_t n_owned,
+                       int elements, int32_t *species, int32_t *slot_of, int32_t *node_of, int32_t *slot_type,
+                       int32_t *elem_start, cudaStream_t st);
+  static int sums(const T *h, const T *Y, const int32_t *sender, const int32_t *row_ptr, const int32_t *species,
+                  const int32_t *slot_of, int64_t nnodes, int elements, T *A, cudaStream_t st);
+  static int contract_fwd(const T *X, const int32_t *types, const T *weff, int64_t n, int C, T *b, cudaStream_t st);
+  static int contract_bwd(const T *X, const int32_t *types, const T *weff, const T *gb, int64_t n, int C, T *gX,
+                          cudaStream_t st);
+  static int contract_readout(const T *X, const int32_t *types, const T *weff, const double *wp1, const double *w2,
+                              const double *q0, const double *e0, const double *atomic_e, double scale, double shift,
+                              int64_t n, int C, T *gX, double *dq, double *inter, double *node_energy, cudaStream_t st);
+  static int mid_fwd(const T *b, const int32_t *slot_of, const int32_t *species, const T *wu, const double *wsc,
+                     const double *w0, int64_t n, int C, T *up, double *q0, double *e0, cudaStream_t st);
+  static int mid_bwd(const T *gup, const int32_t *slot_of, const int32_t *species, const double *dq, const T *wu_t,
+                     const double *wsc, const double *w0, double scale, int64_t n, int C, T *gb, cudaStream_t st);
+  static int sums_bwd(const T *gA, const T *h, const T *dh, const T *Y, const int32_t *sender, const int32_t *row_ptr,
+                      const int32_t *species, const int32_t *slot_of, const T *gY1, const T *dr1, const Quad<T> *geo,
+                      int64_t nnodes, int elements, T *gvec, cudaStream_t st);
+  static int forces(const T *gvec, const int32_t *row_ptr, const int32_t *perm, const int32_t *send_ptr, int64_t nrecv,
+                    int64_t nsend, double sign, double *out, const double *inter, const double *node_energy,
+                    double *sums, cudaStream_t st);
+};
+
+}  // namespace cmace

@@ -14,7 +14,7 @@ them as a small table plus one byte per edge instead of three float64 per edge.
 import torch
 
 from . import domain as _domain
-from . import ops
+from . import ops, step
 
 
 class EnergyForceEvaluator:
@@ -31,7 +31,7 @@ class EnergyForceEvaluator:
 
     def set_neighbor_list(self, species, edge_index, shifts):
         """Device tensors: species [n_local] int32, edge_index [2,E] int32 (receivers sorted), shifts [E,3]."""
-        self.species = species
+        self.species = species.to(torch.int32).contiguous()
         self.edge_index = edge_index
         self.shifts = shifts
         self.topology = ops.EdgeTopology(edge_index[1], edge_index[0], self.dom.n_owned, self.dom.n_local)
@@ -95,11 +95,30 @@ class EnergyForceEvaluator:
             graph.replay()
             return energy.clone(), forces.clone()
 
+        if step.takes(positions_owned, self.shifts):
+            plan = step.plan_of(self.model)
+            if plan is not None:
+                return self._evaluate_native(plan, positions_owned.detach())
+
         def node_energy(pos_local, exchange):
             return self.model.node_energies(pos_local, self.species, self.edge_index, self.shifts,
                                             topology=self.topology, exchange=exchange, n_owned=self.dom.n_owned)
 
         return _domain.distributed_energy_forces(node_energy, self.dom, self.plan, positions_owned)
+
+    def _evaluate_native(self, plan, positions_owned):
+        """Total interaction energy over all ranks and forces on the owned atoms, by the library's own sequence."""
+        many = self.dom.nranks > 1
+        pos = positions_owned
+        if many:
+            pos = self.plan.forward_fill(pos) + self.plan.ghost_shift(pos.dtype)
+        sums, _, _, forces = step.energy_forces(plan, pos, self.species, None, self.shifts, self.topology,
+                                                halo=self.plan if many else None)
+        energy = sums[1]
+        if many:
+            energy = energy.clone()
+            torch.distributed.all_reduce(energy, group=self.plan.group)
+        return energy, forces
 
     # ---- end-to-end path with host buffers ----------------------------------------------------
     def host_batch(self, pos_dtype=torch.float64):

@@ -19,7 +19,7 @@ import math
 
 import torch
 
-from . import ops
+from . import ops, step
 
 SILU_2MOM = 1.676532470331092  # 1/sqrt(E[silu(x)^2]), x ~ N(0,1)
 
@@ -232,10 +232,31 @@ class InvariantMACE(torch.nn.Module):
             return ops.matmul_f64(x, W, W_T)
         return x @ W
 
+    def _forward_native(self, plan, data, topology):
+        """Energy and forces by the library's own sequence (step.py); same dictionary as forward()."""
+        positions = data["positions"].detach()
+        n = positions.shape[0]
+        if topology is None:
+            edge_index = data["edge_index"]
+            topology = ops.topology_for(edge_index[1], edge_index[0], n, n)
+        species = one_hot = None
+        if "species" in data:
+            species = data["species"].to(torch.int32).contiguous()
+        else:
+            one_hot = data["node_attrs"].contiguous()
+            if one_hot.dtype not in (torch.float32, torch.float64) or one_hot.shape[1] != self.num_elements:
+                species, one_hot = one_hot.argmax(dim=-1).to(torch.int32), None
+        sums, _, node_energy, forces = step.energy_forces(plan, positions, species, one_hot, data["shifts"], topology)
+        return {"energy": sums[0], "node_energy": node_energy, "interaction_energy": sums[1], "forces": forces}
+
     def forward(self, data, training=False, compute_force=True, topology=None):
         """data: positions [N,3], node_attrs [N,Z] one-hot (or species [N]), edge_index [2,E], shifts [E,3].
         Returns energy (float64 scalar tensor), node_energy, interaction_energy, forces [N,3]."""
         positions = data["positions"]
+        if compute_force and not training and step.takes(positions, data["shifts"]):
+            plan = step.plan_of(self)
+            if plan is not None:
+                return self._forward_native(plan, data, topology)
         if compute_force:
             positions = positions.detach().requires_grad_(True)
         species = data["species"] if "species" in data else data["node_attrs"].argmax(dim=-1)

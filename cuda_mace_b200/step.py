@@ -1,0 +1,195 @@
+"""The whole energy+force step of an ``InvariantMACE`` on the library's own sequence of kernels (cmace_step_run).
+
+``StepPlan`` lays a model's constant weights out once: products of constant matrices that the model applies one after
+the other are multiplied in float64 (embedding, linear_up, last radial layer, Linear and skip_tp of the first layer;
+product and linear_up between the layers; product, skip connection and readout), the rest is packed for the tensor
+cores.  ``energy_forces`` then runs the step: no autograd graph, one workspace, no synchronisation.  The model's
+autograd path (``node_energies``) stays for what the sequence does not cover: ``covers`` says why.
+"""
+import ctypes
+import math
+import os
+
+import torch
+
+from . import _abi, ops
+
+SILU_2MOM = 1.676532470331092   # normalisation of the activation, 1/sqrt(E[silu(x)^2]) for x ~ N(0,1)
+_H = 64                         # hidden width of the radial perceptron
+
+
+def _pack(Bt):
+    B3 = Bt.reshape(-1, Bt.shape[-2], Bt.shape[-1]).contiguous()
+    nmat, N, K = B3.shape
+    out = torch.empty(int(_abi.call("cmace_gemm_packed_floats", nmat, N, K)), dtype=torch.float32, device=Bt.device)
+    _abi.call("cmace_gemm_pack_weights_f32", B3.data_ptr(), nmat, N, K, out.data_ptr(), ops._stream())
+    return out
+
+
+def covers(model):
+    """Whether the sequence covers a model: the standard two-layer architecture in float32 or float64."""
+    if model.radial != "exact" or len(model.layers) != 2 or model.num_elements > 16:
+        return False
+    if model.dtype not in (torch.float32, torch.float64) or model.channels not in (32, 64, 96, 128):
+        return False
+    if model.edge_basis.num_bessel not in (8, 16) or os.environ.get("CMACE_SYMCON_GENERIC", "")[:1] == "1":
+        return False
+    C, nb = model.channels, model.edge_basis.num_bessel
+    for L in model.layers:
+        if L.n_radial != 4:
+            return False
+        shapes = [tuple(getattr(L, f"W_radial{i}").shape) for i in range(4)]
+        if shapes != [(nb, _H), (_H, _H), (_H, _H), (_H, 4 * C)]:
+            return False
+    L = model.layers[1]
+    return tuple(L.W_readout1.shape) == (C, 16) and tuple(L.W_readout2.shape) == (16, 1)
+
+
+class StepPlan:
+    """Folded and packed weights of one model, and the C description that points at them."""
+
+    def __init__(self, model):
+        self.keep = []
+        # what the layout was made from: any replaced or modified buffer makes a new plan necessary
+        self.sources = [(m._buffers, k, t, t._version) for m in model.modules() for k, t in m._buffers.items()]
+        f32 = model.dtype == torch.float32
+        C, Z = model.channels, model.num_elements
+        L0, L1 = model.layers
+        d = lambda t: t.double()
+        m = _abi.StepModel()
+        m.is_f64, m.channels, m.elements = int(not f32), C, Z
+        m.nbessel, m.cutoff_p = model.edge_basis.num_bessel, model.edge_basis.p
+        m.r_max, m.scale, m.shift = model.edge_basis.r_max, model.scale, model.shift
+
+        def hold(t):
+            t = t.contiguous()
+            self.keep.append(t)
+            return t.data_ptr()
+
+        def matrix(W):   # [.., K, N] in the layout the products want
+            W = W.to(model.dtype)
+            return hold(_pack(W.transpose(-1, -2)) if f32 else W)
+
+        for t, L in enumerate((L0, L1)):
+            for i in range(4):
+                if (t, i) != (0, 3):
+                    m.radial[t][i] = matrix(getattr(L, f"W_radial{i}"))
+        m.radial_back = matrix(L1.W_radial3.t())
+        x = d(model.embedding) @ d(L0.W_up)                                  # [Z, C] sender features of the first layer
+        w4 = d(L0.W_radial3).view(_H, 4, C)
+        lin = d(L0.linear.weights) / math.sqrt(C)                            # [Z, 4, C, C]
+        fold = torch.einsum("zc,klc,rlcd->rlzkd", x, w4, lin).reshape(Z, 4, Z * _H, C)
+        m.fold = matrix(fold)
+        for b in range((Z + 1) // 2):
+            m.fold_back[b] = matrix(fold[:, :, 2 * b * _H: min(2 * b + 2, Z) * _H].transpose(-1, -2))
+        lin = d(L1.linear.weights) / math.sqrt(C)
+        m.linear[0], m.linear[1] = matrix(lin), matrix(lin.transpose(-1, -2))
+        for t, L in enumerate((L0, L1)):
+            con = L.contraction
+            if con._plan is None:
+                con._plan = ops.make_plan(con.u3_max_nonsparse, con.U3_num_nonsparse, con.U3_indices, con.U3_values,
+                                          con.U2_num_nonsparse, con.U2_indices, con.U2_values, con.W3_L0_size,
+                                          con.W2_L0_size, con.W1_L0_size)
+            weff = torch.empty(Z, 13, C, dtype=model.dtype, device=x.device)
+            _abi.call("cmace_symcon_effective_weights", con._plan.handle, int(not f32), con.weights_3.data_ptr(),
+                      con.weights_2.data_ptr(), con.weights_1.data_ptr(), Z, C, weff.data_ptr(), ops._stream())
+            m.weff[t] = hold(weff)
+        prod0, prod1, ro1 = d(L0.W_prod), d(L1.W_prod), d(L1.W_readout1)
+        up = prod0 @ d(L1.W_up)
+        m.up, m.up_back = hold(up.to(model.dtype)), hold(up.t().to(model.dtype))
+        sc = d(L1.W_sc).view(C, Z, C).permute(1, 0, 2)                       # [Z, C, C]
+        m.skip = hold(prod0 @ sc @ ro1)
+        m.readout0 = hold(prod0 @ d(L0.W_readout)[:, 0])
+        m.readout1 = hold(prod1 @ ro1)
+        m.readout2 = hold(d(L1.W_readout2)[:, 0] * SILU_2MOM)
+        m.atomic_energies = hold(model.atomic_energies)
+        self.model = m
+        self.channels, self.dtype, self.elements = C, model.dtype, Z
+        self.radial_ops = (ops.USE_TENSOR_CORES, ops.RADIAL_GRADIENT_ON_THE_FLY, ops.FUSED_RADIAL_MESSAGE_PASSING)
+
+    def current(self):
+        for d, k, t, v in self.sources:
+            if d.get(k) is not t or t._version != v:
+                return False
+        return True
+
+
+def plan_of(model):
+    """The model's plan, laid out again when a weight has changed; None when the sequence does not cover the model or
+    the module-level switches of ops select other kernels."""
+    if not ops.USE_TENSOR_CORES or ops.FUSED_RADIAL_MESSAGE_PASSING or not ops.RADIAL_GRADIENT_ON_THE_FLY:
+        return None
+    plan = model.__dict__.get("_step_plan")
+    if plan is False:
+        return None
+    if plan is not None and plan.current():
+        return plan
+    plan = None
+    if covers(model):
+        try:
+            plan = StepPlan(model)
+        except RuntimeError as e:
+            if "not the generated program" not in str(e):
+                raise
+    model.__dict__["_step_plan"] = plan if plan is not None else False
+    return plan
+
+
+def takes(positions, shifts):
+    """Inputs the sequence takes: float64 positions and shifts on the current device."""
+    return positions.is_cuda and positions.dtype == torch.float64 and shifts.is_cuda and shifts.dtype == torch.float64
+
+
+_FIRST_EXCHANGE, _SECOND_EXCHANGE, _END = 6, 15, 20
+
+
+def energy_forces(plan, positions, species, one_hot, shifts, topology, halo=None):
+    """(sums [2], interaction [n_owned], node_energy [n_owned], forces): sums = (total energy, interaction energy).
+
+    positions [n_local, 3] float64, species [n_local] int32 or one_hot [n_local, Z].  `halo` (a HaloPlan of more than
+    one rank) fills and returns the ghost rows between the ranges of steps; forces are then those of the owned atoms."""
+    ops._check_cuda(positions, shifts)
+    positions, shifts = positions.contiguous(), shifts.contiguous()
+    n, nl, E = topology.nnodes, topology.nsenders, topology.nedges
+    dev = positions.device
+    if positions.shape != (nl, 3) or shifts.shape != (E, 3):
+        raise RuntimeError(f"shape mismatch: positions {tuple(positions.shape)}, shifts {tuple(shifts.shape)} for "
+                           f"{nl} atoms and {E} edges")
+    out = torch.empty(2 + 2 * n + 3 * nl, dtype=torch.float64, device=dev)
+    m = plan.model
+    nbytes = _abi.call("cmace_step_workspace_bytes", ctypes.byref(m), n, nl, E)
+    workspace = torch.empty(nbytes, dtype=torch.uint8, device=dev)
+    perm, send_ptr = topology.sender_order()
+    p = out.data_ptr()
+    io = _abi.StepIO()
+    io.n_owned, io.n_local, io.nedges = n, nl, E
+    io.positions, io.shifts = positions.data_ptr(), shifts.data_ptr()
+    if species is not None:
+        io.species = species.data_ptr()
+    else:
+        io.one_hot, io.one_hot_is_f64 = one_hot.data_ptr(), int(one_hot.dtype == torch.float64)
+    io.sender, io.receiver, io.row_ptr = topology.sender.data_ptr(), topology.receiver.data_ptr(), topology.row_ptr.data_ptr()
+    io.perm, io.send_ptr = perm.data_ptr(), send_ptr.data_ptr()
+    io.workspace, io.workspace_bytes = workspace.data_ptr(), nbytes
+    io.status = ops._status_tensor(dev).data_ptr()
+    io.sums, io.interaction, io.node_energy, io.gradient = p, p + 16, p + 16 + 8 * n, p + 16 + 16 * n
+    io.gradient_sign = -1.0
+    st = ops._stream()
+    forces = out[2 + 2 * n:].view(nl, 3)
+    if halo is None:
+        _abi.run_steps(m, io, 0, _END, st)
+    else:
+        feats = dict(dtype=plan.dtype, device=dev)
+        up = torch.empty(n, plan.channels, **feats)
+        gup = torch.empty(nl, plan.channels, **feats)
+        # the ghost-row pointers are set before the first range: the call checks them together
+        io.up_local, io.gup_local, io.gup_owned = up.data_ptr(), gup.data_ptr(), gup.data_ptr()
+        _abi.run_steps(m, io, 0, _FIRST_EXCHANGE, st)
+        up_local = halo.forward_fill(up)
+        io.up_local = up_local.data_ptr()
+        _abi.run_steps(m, io, _FIRST_EXCHANGE, _SECOND_EXCHANGE, st)
+        gup_owned = halo.backward_reduce(gup)
+        io.gup_owned = gup_owned.data_ptr()
+        _abi.run_steps(m, io, _SECOND_EXCHANGE, _END, st)
+        forces = halo.backward_reduce(forces)
+    return out[:2], out[2:2 + n], out[2 + n:2 + 2 * n], forces

@@ -336,6 +336,61 @@ int cmace_symcon_bwd_f64(const cmace_symcon_plan *plan, const double *X, const i
                          int nelements, int64_t nnodes, int channels, double *gradX,
                          cmace_stream_t stream);
 
+/* effective weights of the generated contraction program, out [nelements][13][channels] in float32 or float64
+ * (8 cubic and 4 quadratic classes, then the linear term); CMACE_ERR_UNSUPPORTED for a plan it does not apply to */
+int cmace_symcon_effective_weights(const cmace_symcon_plan *plan, int is_f64, const void *W3, const void *W2,
+                                   const void *W1, int nelements, int channels, void *out,
+                                   cmace_stream_t stream);
+
+/* ---- whole energy+force step of a two-layer model -------------------------------------------------------
+ * What OptimizedInvariantMACE.forward does with autograd (models/InvariantMACE.py:246-379), as one sequence of
+ * kernel launches with its gradient written out: no autograd graph, no allocation, no synchronisation.  The caller
+ * owns weights, workspace and outputs.  csrc/step.cu documents the sequence; steps can be run in ranges, which is
+ * where a decomposed system exchanges node features (after "mid_fwd") and their gradients (after "senders"). */
+typedef struct cmace_step_model {
+  int32_t is_f64, channels, elements, nbessel, cutoff_p, reserved;
+  double r_max, scale, shift;
+  const void *radial[2][4];  /* float32: packed images of W1..W4 (cmace_gemm_pack_weights_f32 of the transposes);
+                                float64: W1 [nb,64], W2, W3 [64,64], W4 [64,4C]; radial[0][3] is not read */
+  const void *radial_back;   /* second layer's W4 for the gradient: float32 packed W4 itself, float64 W4^T [4C,64] */
+  const void *fold;          /* first layer: [elements][4] matrices [64 elements, C] (float32: packed) */
+  const void *fold_back[8];  /* their transposes in blocks of two elements: [elements][4] [C, 128 or 64] */
+  const void *linear[2];     /* second layer's Linear and its transpose, [4] [C, C] (float32: packed) */
+  const void *weff[2];       /* effective contraction weights of both layers [elements][13][C] */
+  const void *up, *up_back;  /* first layer's product times second layer's linear_up [C, C], and its transpose */
+  const double *skip;        /* [elements][C][16]: product, skip connection and first readout matrix */
+  const double *readout0;    /* [C]: product times the first layer's readout */
+  const double *readout1;    /* [C][16]: second layer's product times the first readout matrix */
+  const double *readout2;    /* [16] */
+  const double *atomic_energies; /* [elements] */
+} cmace_step_model;
+
+typedef struct cmace_step_io {
+  int64_t n_owned, n_local, nedges; /* receivers, sender rows (owned first), edges */
+  const double *positions;          /* [n_local, 3] */
+  const double *shifts;             /* [nedges, 3] or NULL */
+  const int32_t *species;           /* [n_local], or NULL with one_hot [n_local, elements] */
+  const void *one_hot;
+  int32_t one_hot_is_f64, launches; /* launches: kernels launched so far, added to by the call */
+  const int32_t *sender, *receiver, *row_ptr, *perm, *send_ptr;
+  void *up_local;                   /* [n_local, C]: what "mid_fwd" wrote for owned rows, ghost rows filled by the
+                                       caller; NULL when n_local == n_owned */
+  void *gup_local, *gup_owned;      /* gradient of up_local, and what the owners end up with; NULL likewise */
+  void *workspace;
+  int64_t workspace_bytes;
+  int32_t *status;                  /* written by bounded waits that give up */
+  double *node_energy, *interaction; /* [n_owned] */
+  double *sums;                     /* [2]: sum of node_energy, sum of interaction */
+  double *gradient;                 /* [n_local, 3]: gradient_sign times the position gradient */
+  double gradient_sign;
+} cmace_step_io;
+
+int64_t cmace_step_workspace_bytes(const cmace_step_model *model, int64_t n_owned, int64_t n_local, int64_t nedges);
+int cmace_step_count(void);
+const char *cmace_step_name(int step);
+/* runs steps first .. last - 1 of the sequence */
+int cmace_step_run(const cmace_step_model *model, cmace_step_io *io, int first, int last, cmace_stream_t stream);
+
 #ifdef __cplusplus
 }
 #endif

@@ -1,0 +1,62 @@
+"""The whole-step sequence (cmace_step_run) against the float64 oracle at the sizes where its kernels can go wrong."""
+import numpy as np
+import pytest
+import torch
+
+from cuda_mace_b200 import model, step, systems
+from oracle import model as omodel
+
+pytestmark = pytest.mark.gpu
+
+
+def _cluster(n, seed, stretch):
+    """n atoms without periodicity, every pair within the cutoff an edge; stretch > 1 leaves some atoms alone"""
+    rng = np.random.default_rng(seed)
+    pos = rng.random((n, 3)) * (n / 0.1) ** (1.0 / 3.0) * stretch
+    d = np.linalg.norm(pos[:, None] - pos[None], axis=-1)
+    recv, send = np.nonzero((d < 5.0) & (d > 0.0))
+    return pos, np.stack([recv, send]), np.zeros((recv.size, 3))
+
+
+# float64 1e-10 and float32 1e-5 / 1e-4 on energy / forces: the bounds the package states.  Sizes: 1 atom (no edges),
+# fewer edges than a 128-edge tile, tile remainders; elements 1, odd (half a block), 10 and the largest 16; atoms
+# without edges; every channel count.
+@pytest.mark.parametrize("dtype,tol_e,tol_f", [(torch.float64, 1e-10, 1e-10), (torch.float32, 1e-5, 1e-4)])
+@pytest.mark.parametrize("n,C,Z,stretch", [
+    (1, 32, 2, 1.0), (5, 64, 1, 1.0), (23, 96, 3, 1.0), (40, 128, 10, 1.6), (61, 32, 16, 1.3), (70, 128, 2, 1.0),
+    (33, 64, 7, 3.0)])
+def test_step_against_the_oracle(U, dtype, tol_e, tol_f, n, C, Z, stretch):
+    pos, ei, sh = _cluster(n, n, stretch)
+    species = np.random.default_rng(n + 1).integers(0, Z, n)
+    params = systems.init_params(C, Z, 7)
+    one_hot = systems.one_hot(species, Z)
+    _, e_ref, f_ref = omodel.energy_and_forces(params, U, torch.from_numpy(pos), one_hot, torch.from_numpy(ei),
+                                               torch.from_numpy(sh))
+    mace = model.InvariantMACE(params, U, dtype=dtype, device="cuda")
+    assert step.plan_of(mace) is not None
+    data = dict(positions=torch.from_numpy(pos).cuda(), node_attrs=one_hot.to(dtype).cuda(),
+                edge_index=torch.from_numpy(ei).to(torch.int32).cuda(), shifts=torch.from_numpy(sh).cuda())
+    out = mace(data)
+    assert abs(float(out["interaction_energy"]) - float(e_ref)) < tol_e * max(abs(float(e_ref)), 1e-3)
+    scale = max(float(f_ref.abs().max()), 1e-6)
+    assert float((out["forces"].cpu() - f_ref).abs().max()) < tol_f * scale
+    # the element index instead of the one-hot matrix, and a changed weight: the layout has to follow
+    data["species"] = torch.from_numpy(species).cuda()
+    assert torch.equal(mace(data)["forces"], out["forces"])
+    with torch.no_grad():
+        mace.layers[1].W_readout2.mul_(2.0)
+    assert n == 1 or not torch.equal(mace(data)["forces"], out["forces"])
+
+
+@pytest.mark.parametrize("dtype,tol", [(torch.float64, 1e-10), (torch.float32, 1e-4)])
+def test_step_with_a_wider_basis(U, dtype, tol):
+    """16 basis functions (the oracle has 8): against the model's own autograd path."""
+    pos, ei, sh = _cluster(70, 3, 1.0)
+    species = torch.from_numpy(np.random.default_rng(4).integers(0, 3, 70)).to(torch.int32).cuda()
+    mace = model.InvariantMACE(systems.init_params(64, 3, 7, num_bessel=16), U, dtype=dtype, device="cuda")
+    p = torch.from_numpy(pos).cuda()
+    edges, shifts = torch.from_numpy(ei).to(torch.int32).cuda(), torch.from_numpy(sh).cuda()
+    out = mace(dict(positions=p, species=species, edge_index=edges, shifts=shifts))
+    p.requires_grad_(True)
+    (g,) = torch.autograd.grad(mace.node_energies(p, species, edges, shifts).sum(), p)
+    assert float((out["forces"] + g).abs().max()) < tol * float(g.abs().max())
