@@ -43,8 +43,8 @@ int imp_bwd_edge(const T *X, const T *Y, const T *R, const T *G, const int32_t *
                  int64_t nnodes, int64_t nedges, YStride ys, int C, T *gradR, T *gradY, T *Tout, T *partial,
                  cmace_stream_t stream);
 int gemm3x_gradr(const float *X, const float *G, const float *Y, YStride ys, const int32_t *sender,
-                 const int32_t *receiver, const float *packed, int64_t nedges, int channels, int N, float *out,
-                 int32_t *status, cmace_stream_t stream);
+                 const int32_t *receiver, const float *packed, int64_t nedges, int channels, int N, const float *dot,
+                 float *out, int32_t *status, cmace_stream_t stream);
 
 // l of each of the 16 (l, m) components
 __host__ __device__ constexpr int l_of_lm(int lm) { return lm == 0 ? 0 : (lm < 4 ? 1 : (lm < 9 ? 2 : 3)); }

@@ -92,6 +92,7 @@ struct GemmArgs {
   // GRADR: X [Ns, C] sender features, G [Nr, 16, C] gradient of the messages, Y [16, M] harmonics, edge lists [M]
   const float *gx, *gg, *gy;
   int64_t y_m, y_e;             // strides of Y over components and edges
+  const float *dot;             // GRADR: [M, N] or null; then out [M] is the row-wise product of the result with it
   const int32_t *sender, *receiver;
   int C;
   int g_stage_bytes;            // GRADR: shared memory behind the ring and the epilogue buffers for staged G rows
@@ -1066,6 +1067,35 @@ __global__ void __launch_bounds__((GT_PRODUCER_WARPS + 1 + EW + 1) * 32, 1)
           if (lane == 0 && T.row0 + q * 32 < g.M)
             tma_store_2d(&tmap_out, n0 + c0, (int)T.row0 + q * 32, stg);
         }
+      } else if (MODE == GT_MODE_GRADR && g.dot != nullptr) {
+        // only the product of the row with another one is wanted, out[e] = sum_k D[e, k] dot[e, k] (k = 0 .. N - 1):
+        // a thread holds a row
+        float sum = 0.f;
+        for (int c0 = half * 32; c0 < ncols; c0 += 8 * EW) {
+#pragma unroll
+          for (int h16 = 0; h16 < 2; h16++) {
+            if (c0 + 16 * h16 >= ncols) break;
+            uint32_t v[16], w[16];
+            float4 d[4];
+#pragma unroll
+            for (int c = 0; c < 4; c++) {
+              d[c] = make_float4(0.f, 0.f, 0.f, 0.f);
+              if (grow >= 0 && c0 + 16 * h16 + 4 * c < ncols)
+                d[c] = __ldg(reinterpret_cast<const float4 *>(g.dot + grow * g.N + c0 + 16 * h16) + c);
+            }
+            tmem_ld16_nowait(taddr + (uint32_t)(c0 + 16 * h16), v);
+            tmem_ld16_nowait(taddr + (uint32_t)(g.npad + c0 + 16 * h16), w);
+            tmem_ld_wait();
+#pragma unroll
+            for (int c = 0; c < 4; c++) {
+              sum = fmaf(__uint_as_float(v[4 * c]) + __uint_as_float(w[4 * c]), d[c].x, sum);
+              sum = fmaf(__uint_as_float(v[4 * c + 1]) + __uint_as_float(w[4 * c + 1]), d[c].y, sum);
+              sum = fmaf(__uint_as_float(v[4 * c + 2]) + __uint_as_float(w[4 * c + 2]), d[c].z, sum);
+              sum = fmaf(__uint_as_float(v[4 * c + 3]) + __uint_as_float(w[4 * c + 3]), d[c].w, sum);
+            }
+          }
+        }
+        if (grow >= 0) g.out[grow] = sum * g.scale;
       } else if (MODE != GT_MODE_LINEAR) {
         // Straight from tensor memory to global memory, no shared-memory transpose: the 16x256b load shape hands
         // thread t two rows (t/4 and t/4 + 8 of a 16-row half) and, per 8-column block, the two columns
@@ -1462,8 +1492,8 @@ static int gemm_launch(GemmArgs &g, const char *what, cudaStream_t st) {
 }
 
 int gemm3x_gradr(const float *X, const float *G, const float *Y, YStride ys, const int32_t *sender,
-                 const int32_t *receiver, const float *packed, int64_t nedges, int channels, int N, float *out,
-                 int32_t *status, cmace_stream_t stream) {
+                 const int32_t *receiver, const float *packed, int64_t nedges, int channels, int N, const float *dot,
+                 float *out, int32_t *status, cmace_stream_t stream) {
   if (nedges < 0 || N < 32 || N > 128 || N % 4 != 0)
     return fail(CMACE_ERR_UNSUPPORTED, "cmace_gemm3x_gradr: the hidden width must be a multiple of 4 in 32..128");
   if (channels < 32 || channels > 128 || channels % 32 != 0)
@@ -1478,7 +1508,7 @@ int gemm3x_gradr(const float *X, const float *G, const float *Y, YStride ys, con
   GemmArgs g{};
   g.packed = packed; g.out = out; g.status = status;
   g.gx = X; g.gg = G; g.gy = Y; g.sender = sender; g.receiver = receiver; g.C = channels;
-  g.y_m = ys.m; g.y_e = ys.e;
+  g.y_m = ys.m; g.y_e = ys.e; g.dot = dot;
   g.M = nedges; g.K = K; g.N = N; g.nelements = 1; g.mode = GT_MODE_GRADR; g.scale = 1.0f;
   g.n_tiles = p.n_tiles; g.k_blocks = p.k_blocks; g.npad = p.npad;
   g.total_tiles = (nedges + GT_TILE_M - 1) / GT_TILE_M;
@@ -1539,7 +1569,7 @@ int cmace_bounded_wait_probe(int32_t *status, int code, double limit_seconds, cm
 int cmace_gemm3x_gradr_f32(const float *X, const float *G, const float *Y, const int32_t *sender,
                            const int32_t *receiver, const float *packed, int64_t nedges, int channels, int N,
                            float *out, int32_t *status, cmace_stream_t stream) {
-  return cmace::gemm3x_gradr(X, G, Y, YStride{nedges, 1}, sender, receiver, packed, nedges, channels, N, out, status, stream);
+  return cmace::gemm3x_gradr(X, G, Y, YStride{nedges, 1}, sender, receiver, packed, nedges, channels, N, nullptr, out, status, stream);
 }
 
 int cmace_linear_tc_f32(const float *X, const float *packed, const int32_t *node_order, const int32_t *elem_start,

@@ -5,7 +5,7 @@
 //   sums          first layer: A[i, lm, (z, k)] = sum_{e in (i, z)} Y h                   (step_edges.cu)
 //   fold          A times the element-dependent matrices that hold everything up to the layer's Linear
 //   contract0     b0
-//   mid_fwd       up = b0 Wu, q0 = b0 Wsc[z], e0 = b0 . w0                                (step_nodes.cu)
+//   mid_fwd       up = b0 Wu, q0 = b0 Wsc[z] [n, 17]                                      (step_nodes.cu)
 //       -- a decomposed system fills the ghost rows of `up` here --
 //   radial_out    second layer: R = h W4 [E, 4C]
 //   messages, linear, contract1 (value, readout, energy and gradient in one kernel), linear_back
@@ -61,8 +61,7 @@ struct Workspace {
   int32_t *species, *slot_of, *node_of, *slot_type, *elem_start;
   Quad<T> *geo;
   T *basis, *Y, *h[2], *dh[2], *A, *m0, *b0, *up, *R, *m1, *l1, *gX1, *gm1, *T_, *gY1, *gH1, *dr1, *gup, *gb0, *gX0, *gA,
-      *gvec, *gradR, *partial;
-  double *q0, *e0, *dq;
+      *gvec, *gradR, *partial, *q0, *dq;
   int64_t bytes;
 
   Workspace(void *base, const cmace_step_model &m, int64_t n, int64_t nl, int64_t E) {
@@ -90,8 +89,7 @@ struct Workspace {
     take(m0, n * 16 * C);
     take(b0, n * C);
     take(up, n * C);
-    take(q0, n * ST_RO);
-    take(e0, n);
+    take(q0, n * (ST_RO + 1));
     take(R, E * 4 * C);
     take(m1, n * 16 * C);
     take(l1, n * 16 * C);
@@ -99,7 +97,7 @@ struct Workspace {
     take(dq, n * ST_RO);
     take(T_, E * C);
     take(gY1, E * 16);
-    take(gH1, E * ST_H);
+    take(gH1, sizeof(T) == 8 ? E * ST_H : 0);
     take(dr1, E);
     take(gup, nl * C);
     take(gb0, n * C);
@@ -149,16 +147,17 @@ static int run_step(const cmace_step_model &m, cmace_step_io &io, const Workspac
     case S_FOLD: return linear_any(w.A, m.fold, start, Z, n, ST_H * Z, C, w.m0, io.status, st);
     case S_CONTRACT0: return K::contract_fwd(w.m0, w.slot_type, static_cast<const T *>(m.weff[0]), n, C, w.b0, st);
     case S_MID_FWD:
-      return K::mid_fwd(w.b0, w.slot_of, w.species, static_cast<const T *>(m.up), m.skip, m.readout0, n, C,
-                        io.up_local ? static_cast<T *>(io.up_local) : w.up, w.q0, w.e0, st);
+      return K::mid_fwd(w.b0, w.node_of, w.slot_type, static_cast<const T *>(m.up), static_cast<const T *>(m.extra), n, C,
+                        io.up_local ? static_cast<T *>(io.up_local) : w.up, w.q0, st);
     case S_RADIAL_OUT:
       if constexpr (f64) return cmace_gemm_f64(w.h[1], static_cast<const double *>(m.radial[1][3]), E, ST_H, 4 * C, 1.0, w.R, st);
       else return cmace_gemm3x_f32(w.h[1], static_cast<const float *>(m.radial[1][3]), E, ST_H, 4 * C, 1.0, w.R, io.status, st);
     case S_MESSAGES: return imp_fwd<T>(up, w.Y, w.R, io.sender, io.row_ptr, n, E, ys, C, w.m1, st);
     case S_LINEAR: return linear_any(w.m1, m.linear[0], nullptr, 1, n, C, C, w.l1, io.status, st);
     case S_CONTRACT1:
-      return K::contract_readout(w.l1, w.species, static_cast<const T *>(m.weff[1]), m.readout1, m.readout2, w.q0, w.e0,
-                                 m.atomic_energies, m.scale, m.shift, n, C, w.gX1, w.dq, io.interaction, io.node_energy, st);
+      return K::contract_readout(w.l1, w.species, static_cast<const T *>(m.weff[1]), static_cast<const T *>(m.readout1),
+                                 m.readout2, w.q0, m.atomic_energies, m.scale, m.shift, n, C, w.gX1, w.dq, io.interaction,
+                                 io.node_energy, st);
     case S_LINEAR_BACK: return linear_any(w.gX1, m.linear[1], nullptr, 1, n, C, C, w.gm1, io.status, st);
     case S_EDGES_BACK:
       return imp_bwd_edge<T>(up, w.Y, w.R, w.gm1, io.sender, io.row_ptr, n, E, ys, C, f64 ? w.gradR : nullptr, w.gY1,
@@ -168,16 +167,20 @@ static int run_step(const cmace_step_model &m, cmace_step_io &io, const Workspac
         return cmace_gemm_f64(w.gradR, static_cast<const double *>(m.radial_back), E, 4 * C, ST_H, 1.0, w.gH1, st);
       else
         return gemm3x_gradr(up, w.gm1, w.Y, ys, io.sender, io.receiver, static_cast<const float *>(m.radial_back), E, C,
-                            ST_H, w.gH1, io.status, st);
+                            ST_H, w.dh[1], w.dr1, io.status, st);
     case S_RADIAL_DOT:
+      if constexpr (!f64) {   // the float32 product above has formed it
+        io.launches--;
+        return CMACE_OK;
+      }
       if (E > 0) radial_dot_kernel<T><<<(unsigned)((E + 15) / 16), 256, 0, st>>>(w.gH1, w.dh[1], E, w.dr1);
       return check_launch("cmace_step(radial_dot)");
     case S_SENDERS:
       if constexpr (f64) return cmace_imp_bwd_node_f64(w.T_, io.perm, io.send_ptr, nl, C, gup, st);
       else return cmace_imp_bwd_node_f32(w.T_, io.perm, io.send_ptr, nl, C, gup, st);
     case S_MID_BACK:
-      return K::mid_bwd(gup_owned, w.slot_of, w.species, w.dq, static_cast<const T *>(m.up_back), m.skip, m.readout0,
-                        m.scale, n, C, w.gb0, st);
+      return K::mid_bwd(gup_owned, w.node_of, w.slot_type, w.dq, static_cast<const T *>(m.up_back),
+                        static_cast<const T *>(m.extra_back), m.scale, n, C, w.gb0, st);
     case S_CONTRACT0_BACK:
       return K::contract_bwd(w.m0, w.slot_type, static_cast<const T *>(m.weff[0]), w.gb0, n, C, w.gX0, st);
     case S_FOLD_BACK:

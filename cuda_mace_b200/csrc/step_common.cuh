@@ -31,13 +31,13 @@ struct StepKernels {
   static int contract_fwd(const T *X, const int32_t *types, const T *weff, int64_t n, int C, T *b, cudaStream_t st);
   static int contract_bwd(const T *X, const int32_t *types, const T *weff, const T *gb, int64_t n, int C, T *gX,
                           cudaStream_t st);
-  static int contract_readout(const T *X, const int32_t *types, const T *weff, const double *wp1, const double *w2,
-                              const double *q0, const double *e0, const double *atomic_e, double scale, double shift,
-                              int64_t n, int C, T *gX, double *dq, double *inter, double *node_energy, cudaStream_t st);
-  static int mid_fwd(const T *b, const int32_t *slot_of, const int32_t *species, const T *wu, const double *wsc,
-                     const double *w0, int64_t n, int C, T *up, double *q0, double *e0, cudaStream_t st);
-  static int mid_bwd(const T *gup, const int32_t *slot_of, const int32_t *species, const double *dq, const T *wu_t,
-                     const double *wsc, const double *w0, double scale, int64_t n, int C, T *gb, cudaStream_t st);
+  static int contract_readout(const T *X, const int32_t *types, const T *weff, const T *wp1, const double *w2,
+                              const T *q0, const double *atomic_e, double scale, double shift, int64_t n, int C, T *gX,
+                              T *dq, double *inter, double *node_energy, cudaStream_t st);
+  static int mid_fwd(const T *b, const int32_t *node_of, const int32_t *slot_type, const T *wu, const T *extra,
+                     int64_t n, int C, T *up, T *q0, cudaStream_t st);
+  static int mid_bwd(const T *gup, const int32_t *node_of, const int32_t *slot_type, const T *dq, const T *wu_t,
+                     const T *extra_t, double scale, int64_t n, int C, T *gb, cudaStream_t st);
   static int sums_bwd(const T *gA, const T *h, const T *dh, const T *Y, const int32_t *sender, const int32_t *row_ptr,
                       const int32_t *species, const int32_t *slot_of, const T *gY1, const T *dr1, const Quad<T> *geo,
                       int64_t nnodes, int elements, T *gvec, cudaStream_t st);

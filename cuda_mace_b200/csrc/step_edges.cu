@@ -19,7 +19,6 @@ namespace cmace {
 
 // ---- edge geometry, basis and node grouping ----------------------------------------------------------------------
 constexpr int EP_THREADS = 256;
-constexpr int EP_MAX_NB = 16;
 
 // Block 0 resolves the species and groups the owned nodes by element (stable): thread t counts and then places the
 // nodes of its own consecutive piece, so equal elements keep their order.  It runs beside the edge blocks.
@@ -92,12 +91,35 @@ __device__ void group_nodes(const int32_t *species_in, const void *one_hot, int 
   }
 }
 
-// One thread per edge: vector in float64, then unit vector and 1/r, basis and its derivative [E, 2 nb], Y [E, 16].
-template <typename T>
+// A warp's 32 rows of N values each, one row per lane, to consecutive memory: through shared memory, so that a store
+// instruction covers consecutive 16-byte pieces (row stride of one piece more than the row: no bank conflicts).
+template <typename T, int N>
+__device__ __forceinline__ void store_rows(uint4 *buf, const T (&v)[N], T *__restrict__ out, int rows, int lane) {
+  constexpr int PIECES = N * (int)sizeof(T) / 16, PER = 16 / (int)sizeof(T);
+#pragma unroll
+  for (int i = 0; i < PIECES; i++) {
+    uint4 q;
+    T *t = reinterpret_cast<T *>(&q);
+#pragma unroll
+    for (int u = 0; u < PER; u++) t[u] = v[i * PER + u];
+    buf[lane * (PIECES + 1) + i] = q;
+  }
+  __syncwarp();
+  uint4 *o = reinterpret_cast<uint4 *>(out);
+#pragma unroll
+  for (int i = 0; i < PIECES; i++) {
+    const int k = i * 32 + lane, row = k / PIECES;
+    if (row < rows) o[k] = buf[row * (PIECES + 1) + (k - row * PIECES)];
+  }
+  __syncwarp();
+}
+
+// One thread per edge: vector in float64, then unit vector and 1/r, basis and its derivative [E, 2 NB], Y [E, 16].
+template <typename T, int NB>
 __global__ void __launch_bounds__(EP_THREADS)
     edge_prep_kernel(const double *__restrict__ pos, const int32_t *__restrict__ sender,
                      const int32_t *__restrict__ receiver, const double *__restrict__ shifts, int64_t nedges, T r_max,
-                     int nb, int p, Quad<T> *__restrict__ geo, T *__restrict__ basis, T *__restrict__ Y,
+                     int p, Quad<T> *__restrict__ geo, T *__restrict__ basis, T *__restrict__ Y,
                      const int32_t *species_in, const void *one_hot, int one_hot_f64, int64_t n_local, int64_t n_owned,
                      int elements, int32_t *species, int32_t *slot_of, int32_t *node_of, int32_t *slot_type,
                      int32_t *elem_start) {
@@ -106,8 +128,14 @@ __global__ void __launch_bounds__(EP_THREADS)
                 elem_start);
     return;
   }
-  const int64_t e = (int64_t)(blockIdx.x - 1) * EP_THREADS + threadIdx.x;
-  if (e >= nedges) return;
+  extern __shared__ uint4 ep_smem[];
+  const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+  constexpr int MOST = 2 * NB > 16 ? 2 * NB : 16;
+  uint4 *buf = ep_smem + w * 32 * (MOST * (int)sizeof(T) / 16 + 1);
+  const int64_t base = (int64_t)(blockIdx.x - 1) * EP_THREADS + w * 32;
+  if (base >= nedges) return;
+  const int rows = nedges - base < 32 ? (int)(nedges - base) : 32;
+  const int64_t e = base + (lane < rows ? lane : rows - 1);
   const int64_t s = sender[e], r = receiver[e];
   T v[3];
 #pragma unroll
@@ -121,19 +149,11 @@ __global__ void __launch_bounds__(EP_THREADS)
   const T ux = v[0] * ir, uy = v[1] * ir, uz = v[2] * ir;
   T y[16];
   sph_l3<T>(uz, ux, uy, y);
-  geo[e] = Quad<T>{ux, uy, uz, ir};
-  Quad<T> *yo = reinterpret_cast<Quad<T> *>(Y + e * 16);
-#pragma unroll
-  for (int i = 0; i < 4; i++) yo[i] = Quad<T>{y[4 * i], y[4 * i + 1], y[4 * i + 2], y[4 * i + 3]};
-  if (basis != nullptr) {
-    T b[EP_MAX_NB], db[EP_MAX_NB];
-    bessel_cutoff<T>(r2 * ir, r_max, nb, p, b, db);
-    T *bo = basis + e * 2 * nb;
-    for (int n = 0; n < nb; n++) {
-      bo[n] = b[n];
-      bo[nb + n] = db[n];
-    }
-  }
+  if (lane < rows) geo[e] = Quad<T>{ux, uy, uz, ir};
+  store_rows<T, 16>(buf, y, Y + base * 16, rows, lane);
+  T b[2 * NB];
+  bessel_cutoff<T>(r2 * ir, r_max, NB, p, b, b + NB);
+  store_rows<T, 2 * NB>(buf, b, basis + base * 2 * NB, rows, lane);
 }
 
 template <typename T>
@@ -143,9 +163,13 @@ int StepKernels<T>::edge_prep(const double *pos, const int32_t *sender, const in
                               int64_t n_owned, int elements, int32_t *species, int32_t *slot_of, int32_t *node_of,
                               int32_t *slot_type, int32_t *elem_start, cudaStream_t st) {
   const int64_t blocks = 1 + (nedges + EP_THREADS - 1) / EP_THREADS;
-  edge_prep_kernel<T><<<(unsigned)blocks, EP_THREADS, 0, st>>>(
-      pos, sender, receiver, shifts, nedges, (T)r_max, nb, p, geo, basis, Y, species_in, one_hot, one_hot_f64, n_local,
-      n_owned, elements, species, slot_of, node_of, slot_type, elem_start);
+  const size_t smem = (size_t)EP_THREADS * ((nb == 16 ? 32 : 16) * sizeof(T) + 16);
+  auto kern = nb == 16 ? edge_prep_kernel<T, 16> : edge_prep_kernel<T, 8>;
+  cudaError_t err = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+  if (err != cudaSuccess) return fail(CMACE_ERR_CUDA, "cmace_step(edge_prep): %s", cudaGetErrorString(err));
+  kern<<<(unsigned)blocks, EP_THREADS, smem, st>>>(pos, sender, receiver, shifts, nedges, (T)r_max, p, geo, basis, Y,
+                                                   species_in, one_hot, one_hot_f64, n_local, n_owned, elements, species,
+                                                   slot_of, node_of, slot_type, elem_start);
   return check_launch("cmace_step(edge_prep)");
 }
 
@@ -177,15 +201,98 @@ __device__ __forceinline__ void for_edges_of_element(const int32_t *__restrict__
   if (n > 0) body(n);
 }
 
-// sums over k0 = 2 lane, 2 lane + 1; float: accumulators paired over lm, so that Y pairs come straight from memory
-template <typename T>
+// 3-term TF32 split for mma.sync m16n8k8: x = hi + lo, hi by truncation, lo rounded
+__device__ __forceinline__ void split_tf32(float x, uint32_t &hi, uint32_t &lo) {
+  hi = __float_as_uint(x) & 0xFFFFE000u;
+  asm("cvt.rna.tf32.f32 %0, %1;" : "=r"(lo) : "f"(x - __uint_as_float(hi)));
+}
+__device__ __forceinline__ void mma_tf32(float (&c)[4], const uint32_t (&a)[4], uint32_t b0, uint32_t b1) {
+  asm volatile(
+      "mma.sync.aligned.m16n8k8.row.col.f32.tf32.tf32.f32 {%0, %1, %2, %3}, {%4, %5, %6, %7}, {%8, %9}, {%0, %1, %2, %3};"
+      : "+f"(c[0]), "+f"(c[1]), "+f"(c[2]), "+f"(c[3])
+      : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b0), "r"(b1));
+}
+
+// float32: eight edges at a time on the warp-level tensor instruction.  The operands of a pair are tiny (16 x n times
+// n x 64, n about 13) and come straight from memory into fragments, which is what mma.sync is for; a tcgen05 tile of
+// 128 rows would be padding.  D = Y^T h: A fragment = Y of edges t, t + 4 (t = lane & 3) for lm = g, g + 8 (g = lane >> 2);
+// column g of tile j is k = 8 g + j, so that a lane reads 32 consecutive bytes of an edge's row and the lanes of an edge
+// its whole row, and so that what a lane holds in the end is 16 consecutive k of two rows of the sums.
+__global__ void __launch_bounds__(SU_WARPS * 32)
+    sums_tf32_kernel(const float *__restrict__ h, const float *__restrict__ Y, const int32_t *__restrict__ sender,
+                     const int32_t *__restrict__ row_ptr, const int32_t *__restrict__ species,
+                     const int32_t *__restrict__ slot_of, int64_t nnodes, int elements, float *__restrict__ A) {
+  __shared__ int32_t lists[SU_WARPS][SU_LIST];
+  const int lane = threadIdx.x & 31, w = threadIdx.x >> 5, g = lane >> 2, t = lane & 3;
+  const int64_t pair = (int64_t)blockIdx.x * SU_WARPS + w;
+  if (pair >= nnodes * elements) return;
+  const int64_t node = pair / elements;
+  const int z = (int)(pair - node * elements);
+  int32_t *list = lists[w];
+  float acc[8][4];
+#pragma unroll
+  for (int j = 0; j < 8; j++) acc[j][0] = acc[j][1] = acc[j][2] = acc[j][3] = 0.f;
+  for_edges_of_element(sender, species, row_ptr[node], row_ptr[node + 1], z, list, lane, [&](int n) {
+    float4 hv[2][2];
+    float yv[4];
+    auto load = [&](int j0) {   // edges j0 + t and j0 + t + 4; past the end: the last edge with Y = 0
+#pragma unroll
+      for (int u = 0; u < 2; u++) {
+        const int j = j0 + t + 4 * u;
+        const int64_t e = list[j < n ? j : n - 1];
+        const float4 *hp = reinterpret_cast<const float4 *>(h + e * ST_H + 8 * g);
+        hv[u][0] = __ldg(hp);
+        hv[u][1] = __ldg(hp + 1);
+        yv[2 * u] = j < n ? __ldg(Y + e * 16 + g) : 0.f;
+        yv[2 * u + 1] = j < n ? __ldg(Y + e * 16 + g + 8) : 0.f;
+      }
+    };
+    load(0);
+    for (int j0 = 0; j0 < n; j0 += 8) {
+      uint32_t ah[4], al[4], bh[2][8], bl[2][8];
+#pragma unroll
+      for (int i = 0; i < 4; i++) split_tf32(yv[i], ah[i], al[i]);
+#pragma unroll
+      for (int u = 0; u < 2; u++) {
+        split_tf32(hv[u][0].x, bh[u][0], bl[u][0]);
+        split_tf32(hv[u][0].y, bh[u][1], bl[u][1]);
+        split_tf32(hv[u][0].z, bh[u][2], bl[u][2]);
+        split_tf32(hv[u][0].w, bh[u][3], bl[u][3]);
+        split_tf32(hv[u][1].x, bh[u][4], bl[u][4]);
+        split_tf32(hv[u][1].y, bh[u][5], bl[u][5]);
+        split_tf32(hv[u][1].z, bh[u][6], bl[u][6]);
+        split_tf32(hv[u][1].w, bh[u][7], bl[u][7]);
+      }
+      if (j0 + 8 < n) load(j0 + 8);
+#pragma unroll
+      for (int j = 0; j < 8; j++) mma_tf32(acc[j], ah, bh[0][j], bh[1][j]);
+#pragma unroll
+      for (int j = 0; j < 8; j++) mma_tf32(acc[j], ah, bl[0][j], bl[1][j]);
+#pragma unroll
+      for (int j = 0; j < 8; j++) mma_tf32(acc[j], al, bh[0][j], bh[1][j]);
+    }
+  });
+  const int width = elements * ST_H;
+  float *o = A + (int64_t)slot_of[node] * 16 * width + z * ST_H + 16 * t;
+#pragma unroll
+  for (int half = 0; half < 2; half++) {   // rows lm = g and g + 8
+    float4 *row = reinterpret_cast<float4 *>(o + (int64_t)(g + 8 * half) * width);
+#pragma unroll
+    for (int u = 0; u < 2; u++) {
+      row[2 * u] = make_float4(acc[0][2 * half + u], acc[1][2 * half + u], acc[2][2 * half + u], acc[3][2 * half + u]);
+      row[2 * u + 1] = make_float4(acc[4][2 * half + u], acc[5][2 * half + u], acc[6][2 * half + u], acc[7][2 * half + u]);
+    }
+  }
+}
+
+// float64: sums over k = 2 lane, 2 lane + 1
 struct SumAcc {
-  T a[16][2];
+  double a[16][2];
   __device__ __forceinline__ void zero() {
 #pragma unroll
-    for (int m = 0; m < 16; m++) a[m][0] = a[m][1] = T(0);
+    for (int m = 0; m < 16; m++) a[m][0] = a[m][1] = 0.0;
   }
-  __device__ __forceinline__ void add(const T *__restrict__ y, T h0, T h1) {
+  __device__ __forceinline__ void add(const double *__restrict__ y, double h0, double h1) {
 #pragma unroll
     for (int i = 0; i < 8; i++) {
       const double2 v = __ldg(reinterpret_cast<const double2 *>(y) + i);
@@ -195,40 +302,12 @@ struct SumAcc {
       a[2 * i + 1][1] = fma(v.y, h1, a[2 * i + 1][1]);
     }
   }
-  __device__ __forceinline__ void get(int m, T &x0, T &x1) const { x0 = a[m][0]; x1 = a[m][1]; }
-};
-template <>
-struct SumAcc<float> {
-  unsigned long long a[8][2];
-  __device__ __forceinline__ void zero() {
-#pragma unroll
-    for (int m = 0; m < 8; m++) a[m][0] = a[m][1] = 0ull;
-  }
-  __device__ __forceinline__ void add(const float *__restrict__ y, float h0, float h1) {
-    const unsigned long long h00 = pack2(h0, h0), h11 = pack2(h1, h1);
-#pragma unroll
-    for (int i = 0; i < 4; i++) {
-      const ulonglong2 v = __ldg(reinterpret_cast<const ulonglong2 *>(y) + i);
-      a[2 * i][0] = fma2(v.x, h00, a[2 * i][0]);
-      a[2 * i][1] = fma2(v.x, h11, a[2 * i][1]);
-      a[2 * i + 1][0] = fma2(v.y, h00, a[2 * i + 1][0]);
-      a[2 * i + 1][1] = fma2(v.y, h11, a[2 * i + 1][1]);
-    }
-  }
-  __device__ __forceinline__ void get(int m, float &x0, float &x1) const {
-    float lo, hi;
-    unpack2(a[m >> 1][0], lo, hi);
-    x0 = (m & 1) ? hi : lo;
-    unpack2(a[m >> 1][1], lo, hi);
-    x1 = (m & 1) ? hi : lo;
-  }
 };
 
-template <typename T>
 __global__ void __launch_bounds__(SU_WARPS * 32)
-    sums_kernel(const T *__restrict__ h, const T *__restrict__ Y, const int32_t *__restrict__ sender,
+    sums_f64_kernel(const double *__restrict__ h, const double *__restrict__ Y, const int32_t *__restrict__ sender,
                 const int32_t *__restrict__ row_ptr, const int32_t *__restrict__ species,
-                const int32_t *__restrict__ slot_of, int64_t nnodes, int elements, T *__restrict__ A) {
+                const int32_t *__restrict__ slot_of, int64_t nnodes, int elements, double *__restrict__ A) {
   __shared__ int32_t lists[SU_WARPS][SU_LIST];
   const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
   const int64_t pair = (int64_t)blockIdx.x * SU_WARPS + w;
@@ -236,35 +315,32 @@ __global__ void __launch_bounds__(SU_WARPS * 32)
   const int64_t node = pair / elements;
   const int z = (int)(pair - node * elements);
   int32_t *list = lists[w];
-  SumAcc<T> acc;
+  SumAcc acc;
   acc.zero();
-  using V2 = typename Vec<T, 2>::type;
   for_edges_of_element(sender, species, row_ptr[node], row_ptr[node + 1], z, list, lane, [&](int n) {
     int j = 0;
     for (; j + 3 < n; j += 4) {   // four edges' rows on their way before the first is used
       int64_t e[4];
-      V2 v[4];
+      double2 v[4];
 #pragma unroll
       for (int u = 0; u < 4; u++) {
         e[u] = list[j + u];
-        v[u] = __ldg(reinterpret_cast<const V2 *>(h + e[u] * ST_H) + lane);
+        v[u] = __ldg(reinterpret_cast<const double2 *>(h + e[u] * ST_H) + lane);
       }
 #pragma unroll
       for (int u = 0; u < 4; u++) acc.add(Y + e[u] * 16, v[u].x, v[u].y);
     }
     for (; j < n; j++) {
       const int64_t e = list[j];
-      const V2 v = __ldg(reinterpret_cast<const V2 *>(h + e * ST_H) + lane);
+      const double2 v = __ldg(reinterpret_cast<const double2 *>(h + e * ST_H) + lane);
       acc.add(Y + e * 16, v.x, v.y);
     }
   });
   const int width = elements * ST_H;
-  T *o = A + (int64_t)slot_of[node] * 16 * width + z * ST_H + 2 * lane;
+  double *o = A + (int64_t)slot_of[node] * 16 * width + z * ST_H + 2 * lane;
 #pragma unroll
   for (int m = 0; m < 16; m++) {
-    V2 v;
-    acc.get(m, v.x, v.y);
-    *reinterpret_cast<V2 *>(o + (int64_t)m * width) = v;
+    *reinterpret_cast<double2 *>(o + (int64_t)m * width) = make_double2(acc.a[m][0], acc.a[m][1]);
   }
 }
 
@@ -272,14 +348,19 @@ template <typename T>
 int StepKernels<T>::sums(const T *h, const T *Y, const int32_t *sender, const int32_t *row_ptr, const int32_t *species,
                          const int32_t *slot_of, int64_t nnodes, int elements, T *A, cudaStream_t st) {
   const int64_t blocks = (nnodes * elements + SU_WARPS - 1) / SU_WARPS;
-  if (blocks > 0) sums_kernel<T><<<(unsigned)blocks, SU_WARPS * 32, 0, st>>>(h, Y, sender, row_ptr, species, slot_of, nnodes, elements, A);
+  if (blocks > 0) {
+    if constexpr (sizeof(T) == 4)
+      sums_tf32_kernel<<<(unsigned)blocks, SU_WARPS * 32, 0, st>>>(h, Y, sender, row_ptr, species, slot_of, nnodes, elements, A);
+    else
+      sums_f64_kernel<<<(unsigned)blocks, SU_WARPS * 32, 0, st>>>(h, Y, sender, row_ptr, species, slot_of, nnodes, elements, A);
+  }
   return check_launch("cmace_step(sums)");
 }
 
 // ---- backward over the edges of a (receiver, element) pair, down to the gradient of the edge vector ---------------
-// The warp holds P = grad A[i, :, z, 2 lane .. 2 lane + 1]; per edge 16 + 1 sums over k (warp transpose-reduce), which
-// wait in shared memory until 32 edges (or the list's end) are there: then lane j turns edge j's numbers, plus the
-// second layer's grad Y and dE/dr, into the gradient of its vector.
+// The warp holds P = grad A[i, :, z, :]; the 16 + 1 sums of an edge over k wait in shared memory until 32 edges (or the
+// list's end) are there: then lane j turns edge j's numbers, plus the second layer's grad Y and dE/dr, into the
+// gradient of its vector.
 template <typename T>
 __device__ __forceinline__ T reduce16(T (&p)[16], int lane) {
   T q8[8], q4[4], q2[2];
@@ -307,13 +388,144 @@ __device__ __forceinline__ T reduce16(T (&p)[16], int lane) {
   return r + __shfl_xor_sync(0xffffffffu, r, 1);   // component lane >> 1
 }
 
+// lane j of the warp: edge list[j], its 16 + 1 sums in st[j * 17 ..], to the gradient of the edge's vector
 template <typename T>
-struct PairGrad {   // P, as the accumulators above hold it
-  T p[16][2];
-  __device__ __forceinline__ void set(int m, T x0, T x1) { p[m][0] = x0; p[m][1] = x1; }
+__device__ __forceinline__ void finish_edge(const T *st, int64_t e, const T *__restrict__ gY1, const T *__restrict__ dr1,
+                                            const Quad<T> *__restrict__ geo, T *__restrict__ gvec) {
+  T g[16];
+  const Quad<T> *gy = reinterpret_cast<const Quad<T> *>(gY1 + e * 16);
+#pragma unroll
+  for (int i = 0; i < 4; i++) {
+    const Quad<T> q = gy[i];
+    g[4 * i] = st[4 * i] + q.x;
+    g[4 * i + 1] = st[4 * i + 1] + q.y;
+    g[4 * i + 2] = st[4 * i + 2] + q.z;
+    g[4 * i + 3] = st[4 * i + 3] + q.w;
+  }
+  const T dr = st[16] + dr1[e];
+  const Quad<T> q = geo[e];   // unit vector in the input's component order: harmonic axes are (z, x, y)
+  T GX, GY, GZ;
+  sph_l3_vjp<T>(q.z, q.x, q.y, g, GX, GY, GZ);
+  gvec[e * 3] = GY * q.w + dr * q.x;
+  gvec[e * 3 + 1] = GZ * q.w + dr * q.y;
+  gvec[e * 3 + 2] = GX * q.w + dr * q.z;
+}
+
+// float32: eight edges at a time on the warp-level tensor instruction, D = P h^T and P h'^T.  P [16 x 64] stays in
+// registers as A fragments (hi and lo); an edge's row is read as four 16-byte pieces per lane (lanes t of edge g cover
+// 64 consecutive bytes each time), and the k order of the fragments follows: piece q holds k = 16 q + 4 t + 0 .. 3, its
+// first two values are K step 2 q, the other two K step 2 q + 1.  No shuffles but for dE/dr (8 lanes hold its lm).
+__global__ void __launch_bounds__(SU_WARPS * 32, 3)
+    sums_bwd_tf32_kernel(const float *__restrict__ gA, const float *__restrict__ h, const float *__restrict__ dh,
+                         const float *__restrict__ Y, const int32_t *__restrict__ sender,
+                         const int32_t *__restrict__ row_ptr, const int32_t *__restrict__ species,
+                         const int32_t *__restrict__ slot_of, const float *__restrict__ gY1,
+                         const float *__restrict__ dr1, const Quad<float> *__restrict__ geo, int64_t nnodes, int elements,
+                         float *__restrict__ gvec) {
+  __shared__ int32_t lists[SU_WARPS][SU_LIST];
+  __shared__ float stage[SU_WARPS][32 * 17];
+  const int lane = threadIdx.x & 31, w = threadIdx.x >> 5, g = lane >> 2, t = lane & 3;
+  const int64_t pair = (int64_t)blockIdx.x * SU_WARPS + w;
+  if (pair >= nnodes * elements) return;
+  const int64_t node = pair / elements;
+  const int z = (int)(pair - node * elements);
+  int32_t *list = lists[w];
+  float *st = stage[w];
+  uint32_t ph[8][4], pl[8][4];   // A fragments of the 8 K steps
+  {
+    const int b = z >> 1, width = sums_block_width(elements, b);
+    const float *p = gA + (int64_t)b * nnodes * (16 * 128) + (int64_t)slot_of[node] * 16 * width + (z & 1) * ST_H + 4 * t;
+#pragma unroll
+    for (int q = 0; q < 4; q++) {
+      const float4 u = __ldg(reinterpret_cast<const float4 *>(p + g * width + 16 * q));
+      const float4 v = __ldg(reinterpret_cast<const float4 *>(p + (g + 8) * width + 16 * q));
+      split_tf32(u.x, ph[2 * q][0], pl[2 * q][0]);
+      split_tf32(v.x, ph[2 * q][1], pl[2 * q][1]);
+      split_tf32(u.y, ph[2 * q][2], pl[2 * q][2]);
+      split_tf32(v.y, ph[2 * q][3], pl[2 * q][3]);
+      split_tf32(u.z, ph[2 * q + 1][0], pl[2 * q + 1][0]);
+      split_tf32(v.z, ph[2 * q + 1][1], pl[2 * q + 1][1]);
+      split_tf32(u.w, ph[2 * q + 1][2], pl[2 * q + 1][2]);
+      split_tf32(v.w, ph[2 * q + 1][3], pl[2 * q + 1][3]);
+    }
+  }
+  for_edges_of_element(sender, species, row_ptr[node], row_ptr[node + 1], z, list, lane, [&](int n) {
+    for (int j0 = 0; j0 < n; j0 += 32) {
+      const int nj = n - j0 < 32 ? n - j0 : 32;
+      float4 hv[4], dv[4];
+      auto load = [&](int j) {   // edge j0 + j + g, or the last one
+        const int i = j0 + j + g;
+        const int64_t e = list[i < n ? i : n - 1];
+        const float4 *hp = reinterpret_cast<const float4 *>(h + e * ST_H + 4 * t);
+        const float4 *dp = reinterpret_cast<const float4 *>(dh + e * ST_H + 4 * t);
+#pragma unroll
+        for (int q = 0; q < 4; q++) {
+          hv[q] = __ldg(hp + 4 * q);
+          dv[q] = __ldg(dp + 4 * q);
+        }
+      };
+      load(0);
+      for (int j = 0; j < nj; j += 8) {
+        float ch[4] = {0.f, 0.f, 0.f, 0.f}, cd[4] = {0.f, 0.f, 0.f, 0.f};
+        const int i0 = j0 + j + 2 * t;   // this lane's result columns: edges 2 t and 2 t + 1 of the eight
+        const int64_t e0 = list[i0 < n ? i0 : n - 1], e1 = list[i0 + 1 < n ? i0 + 1 : n - 1];
+        const float y00 = __ldg(Y + e0 * 16 + g), y01 = __ldg(Y + e0 * 16 + g + 8);
+        const float y10 = __ldg(Y + e1 * 16 + g), y11 = __ldg(Y + e1 * 16 + g + 8);
+#pragma unroll
+        for (int q = 0; q < 4; q++) {
+          uint32_t h0, l0, h1, l1, g0, m0, g1, m1;
+          split_tf32(hv[q].x, h0, l0);
+          split_tf32(hv[q].y, h1, l1);
+          split_tf32(dv[q].x, g0, m0);
+          split_tf32(dv[q].y, g1, m1);
+          mma_tf32(ch, ph[2 * q], h0, h1);
+          mma_tf32(cd, ph[2 * q], g0, g1);
+          mma_tf32(ch, ph[2 * q], l0, l1);
+          mma_tf32(cd, ph[2 * q], m0, m1);
+          mma_tf32(ch, pl[2 * q], h0, h1);
+          mma_tf32(cd, pl[2 * q], g0, g1);
+          split_tf32(hv[q].z, h0, l0);
+          split_tf32(hv[q].w, h1, l1);
+          split_tf32(dv[q].z, g0, m0);
+          split_tf32(dv[q].w, g1, m1);
+          mma_tf32(ch, ph[2 * q + 1], h0, h1);
+          mma_tf32(cd, ph[2 * q + 1], g0, g1);
+          mma_tf32(ch, ph[2 * q + 1], l0, l1);
+          mma_tf32(cd, ph[2 * q + 1], m0, m1);
+          mma_tf32(ch, pl[2 * q + 1], h0, h1);
+          mma_tf32(cd, pl[2 * q + 1], g0, g1);
+        }
+        if (j + 8 < nj) load(j + 8);
+        float *s0 = st + (j + 2 * t) * 17, *s1 = s0 + 17;
+        s0[g] = ch[0];
+        s1[g] = ch[1];
+        s0[g + 8] = ch[2];
+        s1[g + 8] = ch[3];
+        float r0 = fmaf(y00, cd[0], y01 * cd[2]), r1 = fmaf(y10, cd[1], y11 * cd[3]);
+#pragma unroll
+        for (int off = 4; off < 32; off <<= 1) {
+          r0 += __shfl_xor_sync(0xffffffffu, r0, off);
+          r1 += __shfl_xor_sync(0xffffffffu, r1, off);
+        }
+        if (g == 0) {
+          s0[16] = r0;
+          s1[16] = r1;
+        }
+      }
+      __syncwarp();
+      if (lane < nj) finish_edge<float>(st + lane * 17, list[j0 + lane], gY1, dr1, geo, gvec);
+      __syncwarp();
+    }
+  });
+}
+
+// float64: a lane holds k = 2 lane, 2 lane + 1 of P
+struct PairGrad {
+  double p[16][2];
   // g[lm] = sum over this lane's k of P h; returns sum_k h'_k sum_lm Y P of this lane
-  __device__ __forceinline__ T edge(const T *__restrict__ y, T h0, T h1, T d0, T d1, T (&g)[16]) const {
-    T s0 = T(0), s1 = T(0);
+  __device__ __forceinline__ double edge(const double *__restrict__ y, double h0, double h1, double d0, double d1,
+                                         double (&g)[16]) const {
+    double s0 = 0.0, s1 = 0.0;
 #pragma unroll
     for (int i = 0; i < 8; i++) {
       const double2 v = __ldg(reinterpret_cast<const double2 *>(y) + i);
@@ -327,110 +539,60 @@ struct PairGrad {   // P, as the accumulators above hold it
     return fma(s1, d1, s0 * d0);
   }
 };
-template <>
-struct PairGrad<float> {
-  unsigned long long p[8][2];
-  __device__ __forceinline__ void set(int m, float x0, float x1) {
-    float lo, hi;
-    unpack2(p[m >> 1][0], lo, hi);
-    p[m >> 1][0] = (m & 1) ? pack2(lo, x0) : pack2(x0, hi);
-    unpack2(p[m >> 1][1], lo, hi);
-    p[m >> 1][1] = (m & 1) ? pack2(lo, x1) : pack2(x1, hi);
-  }
-  __device__ __forceinline__ float edge(const float *__restrict__ y, float h0, float h1, float d0, float d1,
-                                        float (&g)[16]) const {
-    const unsigned long long h00 = pack2(h0, h0), h11 = pack2(h1, h1);
-    unsigned long long s0 = 0ull, s1 = 0ull;
-#pragma unroll
-    for (int i = 0; i < 4; i++) {
-      const ulonglong2 v = __ldg(reinterpret_cast<const ulonglong2 *>(y) + i);
-      s0 = fma2(v.x, p[2 * i][0], s0);
-      s1 = fma2(v.x, p[2 * i][1], s1);
-      s0 = fma2(v.y, p[2 * i + 1][0], s0);
-      s1 = fma2(v.y, p[2 * i + 1][1], s1);
-    }
-#pragma unroll
-    for (int i = 0; i < 8; i++) unpack2(fma2(p[i][1], h11, mul2(p[i][0], h00)), g[2 * i], g[2 * i + 1]);
-    float a, b, c, d;
-    unpack2(s0, a, b);
-    unpack2(s1, c, d);
-    return fmaf(c + d, d1, (a + b) * d0);
-  }
-};
 
-template <typename T>
 __global__ void __launch_bounds__(SU_WARPS * 32)
-    sums_bwd_kernel(const T *__restrict__ gA, const T *__restrict__ h, const T *__restrict__ dh,
-                    const T *__restrict__ Y, const int32_t *__restrict__ sender, const int32_t *__restrict__ row_ptr,
+    sums_bwd_f64_kernel(const double *__restrict__ gA, const double *__restrict__ h, const double *__restrict__ dh,
+                    const double *__restrict__ Y, const int32_t *__restrict__ sender, const int32_t *__restrict__ row_ptr,
                     const int32_t *__restrict__ species, const int32_t *__restrict__ slot_of,
-                    const T *__restrict__ gY1, const T *__restrict__ dr1, const Quad<T> *__restrict__ geo,
-                    int64_t nnodes, int elements, T *__restrict__ gvec) {
+                    const double *__restrict__ gY1, const double *__restrict__ dr1, const Quad<double> *__restrict__ geo,
+                    int64_t nnodes, int elements, double *__restrict__ gvec) {
   __shared__ int32_t lists[SU_WARPS][SU_LIST];
-  __shared__ T stage[SU_WARPS][32 * 17];
+  __shared__ double stage[SU_WARPS][32 * 17];
   const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
   const int64_t pair = (int64_t)blockIdx.x * SU_WARPS + w;
   if (pair >= nnodes * elements) return;
   const int64_t node = pair / elements;
   const int z = (int)(pair - node * elements);
   int32_t *list = lists[w];
-  T *st = stage[w];
-  using V2 = typename Vec<T, 2>::type;
-  PairGrad<T> P;
+  double *st = stage[w];
+  PairGrad P;
   {
     const int b = z >> 1, width = sums_block_width(elements, b);
-    const T *g = gA + (int64_t)b * nnodes * (16 * 128) + (int64_t)slot_of[node] * 16 * width + (z & 1) * ST_H + 2 * lane;
+    const double *g = gA + (int64_t)b * nnodes * (16 * 128) + (int64_t)slot_of[node] * 16 * width + (z & 1) * ST_H + 2 * lane;
 #pragma unroll
     for (int m = 0; m < 16; m++) {
-      const V2 v = __ldg(reinterpret_cast<const V2 *>(g + m * width));
-      P.set(m, v.x, v.y);
+      const double2 v = __ldg(reinterpret_cast<const double2 *>(g + m * width));
+      P.p[m][0] = v.x;
+      P.p[m][1] = v.y;
     }
   }
   for_edges_of_element(sender, species, row_ptr[node], row_ptr[node + 1], z, list, lane, [&](int n) {
     for (int j0 = 0; j0 < n; j0 += 32) {
       const int nj = n - j0 < 32 ? n - j0 : 32;
-      V2 hv = V2{}, dv = V2{};
+      double2 hv = double2{}, dv = double2{};
       if (nj > 0) {
         const int64_t e = list[j0];
-        hv = __ldg(reinterpret_cast<const V2 *>(h + e * ST_H) + lane);
-        dv = __ldg(reinterpret_cast<const V2 *>(dh + e * ST_H) + lane);
+        hv = __ldg(reinterpret_cast<const double2 *>(h + e * ST_H) + lane);
+        dv = __ldg(reinterpret_cast<const double2 *>(dh + e * ST_H) + lane);
       }
       for (int j = 0; j < nj; j++) {
         const int64_t e = list[j0 + j];
-        const V2 hc = hv, dc = dv;
+        const double2 hc = hv, dc = dv;
         if (j + 1 < nj) {   // the next edge's rows
           const int64_t en = list[j0 + j + 1];
-          hv = __ldg(reinterpret_cast<const V2 *>(h + en * ST_H) + lane);
-          dv = __ldg(reinterpret_cast<const V2 *>(dh + en * ST_H) + lane);
+          hv = __ldg(reinterpret_cast<const double2 *>(h + en * ST_H) + lane);
+          dv = __ldg(reinterpret_cast<const double2 *>(dh + en * ST_H) + lane);
         }
-        T g[16];
-        T r = P.edge(Y + e * 16, hc.x, hc.y, dc.x, dc.y, g);
+        double g[16];
+        double r = P.edge(Y + e * 16, hc.x, hc.y, dc.x, dc.y, g);
 #pragma unroll
         for (int off = 16; off > 0; off >>= 1) r += __shfl_xor_sync(0xffffffffu, r, off);
-        const T tot = reduce16(g, lane);
+        const double tot = reduce16(g, lane);
         if ((lane & 1) == 0) st[j * 17 + (lane >> 1)] = tot;
         if (lane == 1) st[j * 17 + 16] = r;
       }
       __syncwarp();
-      if (lane < nj) {
-        const int64_t e = list[j0 + lane];
-        T g[16];
-        const Quad<T> *gy = reinterpret_cast<const Quad<T> *>(gY1 + e * 16);
-#pragma unroll
-        for (int i = 0; i < 4; i++) {
-          const Quad<T> q = gy[i];
-          g[4 * i] = st[lane * 17 + 4 * i] + q.x;
-          g[4 * i + 1] = st[lane * 17 + 4 * i + 1] + q.y;
-          g[4 * i + 2] = st[lane * 17 + 4 * i + 2] + q.z;
-          g[4 * i + 3] = st[lane * 17 + 4 * i + 3] + q.w;
-        }
-        const T dr = st[lane * 17 + 16] + dr1[e];
-        const Quad<T> q = geo[e];   // unit vector in the input's component order: harmonic axes are (z, x, y)
-        T GX, GY, GZ;
-        sph_l3_vjp<T>(q.z, q.x, q.y, g, GX, GY, GZ);
-        gvec[e * 3] = GY * q.w + dr * q.x;
-        gvec[e * 3 + 1] = GZ * q.w + dr * q.y;
-        gvec[e * 3 + 2] = GX * q.w + dr * q.z;
-      }
+      if (lane < nj) finish_edge<double>(st + lane * 17, list[j0 + lane], gY1, dr1, geo, gvec);
       __syncwarp();
     }
   });
@@ -441,9 +603,14 @@ int StepKernels<T>::sums_bwd(const T *gA, const T *h, const T *dh, const T *Y, c
                              const int32_t *row_ptr, const int32_t *species, const int32_t *slot_of, const T *gY1,
                              const T *dr1, const Quad<T> *geo, int64_t nnodes, int elements, T *gvec, cudaStream_t st) {
   const int64_t blocks = (nnodes * elements + SU_WARPS - 1) / SU_WARPS;
-  if (blocks > 0)
-    sums_bwd_kernel<T><<<(unsigned)blocks, SU_WARPS * 32, 0, st>>>(gA, h, dh, Y, sender, row_ptr, species, slot_of, gY1,
-                                                                   dr1, geo, nnodes, elements, gvec);
+  if (blocks > 0) {
+    if constexpr (sizeof(T) == 4)
+      sums_bwd_tf32_kernel<<<(unsigned)blocks, SU_WARPS * 32, 0, st>>>(gA, h, dh, Y, sender, row_ptr, species, slot_of,
+                                                                      gY1, dr1, geo, nnodes, elements, gvec);
+    else
+      sums_bwd_f64_kernel<<<(unsigned)blocks, SU_WARPS * 32, 0, st>>>(gA, h, dh, Y, sender, row_ptr, species, slot_of,
+                                                                     gY1, dr1, geo, nnodes, elements, gvec);
+  }
   return check_launch("cmace_step(sums_bwd)");
 }
 

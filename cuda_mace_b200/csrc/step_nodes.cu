@@ -2,8 +2,8 @@
 // channel), fused in the second layer with the readout and its own gradient, and the products between the layers.
 //
 // All weights between the first contraction's output b0 [n, C] and what the rest of the model reads from it are
-// folded when the model is laid out: up1 = b0 Wu (product and linear_up of the two layers), q0 = b0 Wsc[z] (product,
-// skip connection and first readout layer: the skip term only ever enters the second readout) and e0 = b0 . w0.
+// folded when the model is laid out: up = b0 Wu (product and linear_up of the two layers) and q0 = b0 Wsc[z] [17]: product,
+// skip connection and first readout matrix (the skip term only ever enters the second readout), and the first readout.
 #include "step_common.cuh"
 #include "symcon_canonical.inc"
 
@@ -24,7 +24,7 @@ __device__ __forceinline__ void load_weff(const T *__restrict__ weff, int z, int
 }
 
 template <typename T, bool BWD>
-__global__ void __launch_bounds__(128)
+__global__ void __launch_bounds__(128, sizeof(T) == 4 ? 5 : 3)
     step_contract_kernel(const T *__restrict__ X, const int32_t *__restrict__ types, const T *__restrict__ weff,
                          const T *__restrict__ gb, int64_t nnodes, int C, T *__restrict__ out) {
   const int c = threadIdx.x;
@@ -64,37 +64,40 @@ int StepKernels<T>::contract_bwd(const T *X, const int32_t *types, const T *weff
   return check_launch("cmace_step(contract_bwd)");
 }
 
-// Second layer: value b and gradient factors from one evaluation; q = q0 + b Wp1 (float64), the readout
-// e1 = sum_j silu(q_j) w2_j, and back: grad b = Wp1 (silu'(q) w2), grad X = grad b * dB/dx.  w2 carries the
-// activation's normalisation.  C threads per node; the 16 sums over channels go through two barriers.
+// Second layer: value b and gradient factors from one evaluation; q = q0 + b Wp1, the readout e1 = sum_j silu(q_j) w2_j
+// (float64 from the sums over a warp's channels on), and back: grad b = Wp1 (silu'(q) w2), grad X = grad b * dB/dx.
+// w2 carries the activation's normalisation.  C threads per node; the 16 sums over channels go through two barriers.
+// q0 [n][17]: 16 of the hidden layer, then the first readout.
 template <typename T>
-__global__ void __launch_bounds__(128)
+__global__ void __launch_bounds__(128, sizeof(T) == 4 ? 5 : 3)
     contract_readout_kernel(const T *__restrict__ X, const int32_t *__restrict__ types, const T *__restrict__ weff,
-                            const double *__restrict__ wp1, const double *__restrict__ w2ro,
-                            const double *__restrict__ q0, const double *__restrict__ e0,
+                            const T *__restrict__ wp1, const double *__restrict__ w2ro, const T *__restrict__ q0,
                             const double *__restrict__ atomic_e, double scale, double shift, int64_t nnodes, int C,
-                            T *__restrict__ gX, double *__restrict__ dq_out, double *__restrict__ inter,
+                            T *__restrict__ gX, T *__restrict__ dq_out, double *__restrict__ inter,
                             double *__restrict__ node_energy) {
-  __shared__ double part[4][ST_RO];
-  __shared__ double dq_s[ST_RO];
+  __shared__ T part[4][ST_RO];
+  __shared__ T dq_s[ST_RO];
   const int c = threadIdx.x, lane = c & 31, w = c >> 5, nw = C >> 5;
-  double wp[ST_RO];
+  T wp[ST_RO];
 #pragma unroll
-  for (int j = 0; j < ST_RO; j++) wp[j] = wp1[c * ST_RO + j];
+  for (int j = 0; j < ST_RO; j++) wp[j] = __ldg(wp1 + j * C + c);
   for (int64_t node = blockIdx.x; node < nnodes; node += gridDim.x) {
     T x[16], g[16], w3[canon::NCLASS3], w2[canon::NCLASS2], w1, value;
     const T *xr = X + node * 16 * C + c;
-    const int z = types[node];
 #pragma unroll
     for (int i = 0; i < 16; i++) x[i] = __ldcs(xr + i * C);
+    const int z = types[node];
     load_weff(weff, z, C, c, w3, w2, w1);
+    double qd = 0.0, e0 = 0.0;
+    if (c < ST_RO) qd = (double)q0[node * (ST_RO + 1) + c];
+    if (c == 0) e0 = (double)q0[node * (ST_RO + 1) + ST_RO];
     canon::eval<T>(x, w3, w2, w1, g, value);
-    double p[ST_RO];
+    T p[ST_RO];
 #pragma unroll
-    for (int j = 0; j < ST_RO; j++) p[j] = (double)value * wp[j];
+    for (int j = 0; j < ST_RO; j++) p[j] = value * wp[j];
     // 16 sums over the warp's lanes at once: every lane ends with component lane >> 1
     {
-      double q8[8], q4[4], q2[2];
+      T q8[8], q4[4], q2[2];
       bool up = lane & 16;
 #pragma unroll
       for (int i = 0; i < 8; i++) q8[i] = (up ? p[i + 8] : p[i]) + __shfl_xor_sync(0xffffffffu, up ? p[i] : p[i + 8], 16);
@@ -105,7 +108,7 @@ __global__ void __launch_bounds__(128)
 #pragma unroll
       for (int i = 0; i < 2; i++) q2[i] = (up ? q4[i + 2] : q4[i]) + __shfl_xor_sync(0xffffffffu, up ? q4[i] : q4[i + 2], 4);
       up = lane & 2;
-      double r = (up ? q2[1] : q2[0]) + __shfl_xor_sync(0xffffffffu, up ? q2[0] : q2[1], 2);
+      T r = (up ? q2[1] : q2[0]) + __shfl_xor_sync(0xffffffffu, up ? q2[0] : q2[1], 2);
       r += __shfl_xor_sync(0xffffffffu, r, 1);
       if ((lane & 1) == 0) part[w][lane >> 1] = r;
     }
@@ -113,28 +116,27 @@ __global__ void __launch_bounds__(128)
     if (c < 32) {
       double e1 = 0.0;
       if (c < ST_RO) {
-        double q = q0[node * ST_RO + c];
-        for (int k = 0; k < nw; k++) q += part[k][c];
+        double q = qd;
+        for (int k = 0; k < nw; k++) q += (double)part[k][c];
         const double s = 1.0 / (1.0 + exp(-q));
         const double wj = w2ro[c];
         e1 = q * s * wj;
-        const double d = scale * wj * s * (1.0 + q * (1.0 - s));
+        const T d = (T)(scale * wj * s * (1.0 + q * (1.0 - s)));
         dq_s[c] = d;
         dq_out[node * ST_RO + c] = d;
       }
 #pragma unroll
       for (int off = 8; off > 0; off >>= 1) e1 += __shfl_xor_sync(0xffffffffu, e1, off);
       if (c == 0) {
-        const double v = scale * (e0[node] + e1) + shift;
+        const double v = scale * (e0 + e1) + shift;
         inter[node] = v;
         node_energy[node] = atomic_e[z] + v;
       }
     }
     __syncthreads();
-    double gbd = 0.0;
+    T go = T(0);
 #pragma unroll
-    for (int j = 0; j < ST_RO; j++) gbd = fma(dq_s[j], wp[j], gbd);
-    const T go = (T)gbd;
+    for (int j = 0; j < ST_RO; j++) go = fma(dq_s[j], wp[j], go);
     T *o = gX + node * 16 * C + c;
 #pragma unroll
     for (int i = 0; i < 16; i++) __stcs(o + i * C, go * g[i]);
@@ -142,172 +144,182 @@ __global__ void __launch_bounds__(128)
 }
 
 template <typename T>
-int StepKernels<T>::contract_readout(const T *X, const int32_t *types, const T *weff, const double *wp1,
-                                     const double *w2, const double *q0, const double *e0, const double *atomic_e,
-                                     double scale, double shift, int64_t n, int C, T *gX, double *dq, double *inter,
-                                     double *node_energy, cudaStream_t st) {
+int StepKernels<T>::contract_readout(const T *X, const int32_t *types, const T *weff, const T *wp1, const double *w2,
+                                     const T *q0, const double *atomic_e, double scale, double shift, int64_t n, int C,
+                                     T *gX, T *dq, double *inter, double *node_energy, cudaStream_t st) {
   if (n > 0)
-    contract_readout_kernel<T><<<(unsigned)node_blocks(n, 8), C, 0, st>>>(X, types, weff, wp1, w2, q0, e0, atomic_e, scale,
-                                                                         shift, n, C, gX, dq, inter, node_energy);
+    contract_readout_kernel<T><<<(unsigned)node_blocks(n, 10), C, 0, st>>>(X, types, weff, wp1, w2, q0, atomic_e, scale,
+                                                                          shift, n, C, gX, dq, inter, node_energy);
   return check_launch("cmace_step(contract_readout)");
 }
 
 // ---- between the layers --------------------------------------------------------------------------------------------
-// One block per MID_NODES consecutive nodes, their input rows in shared memory.  Thread t owns output column t mod C of
-// every MID_GROUPS-th node; a weight is loaded once (coalesced, L1 / L2) for all of the thread's nodes and multiplies
-// values that the whole warp reads from one shared-memory address.  The float64 parts (q0, e0) are 17 short dot
-// products a node.
-constexpr int MID_THREADS = 256;
+// Products with a [C, C] matrix that stays in shared memory (64 KB float32, 128 KB float64: one fill per block, blocks
+// are persistent), plus 17 columns that depend on the element: 16 of the second readout's hidden layer and the first
+// readout.  Nodes are taken in slot order, so the nodes of a tile nearly always share the element.  2 C threads: a
+// thread owns 4 columns of NODES / 8 nodes; what bounds it is the shared-memory pipe (four 16-byte loads of weights
+// and NODES / 8 of rows per 4 k).
+constexpr int MID_EXTRA = ST_RO + 1;
 
-template <typename T, int NODES>
-__global__ void __launch_bounds__(MID_THREADS)
-    mid_fwd_kernel(const T *__restrict__ b, const int32_t *__restrict__ slot_of, const int32_t *__restrict__ species,
-                   const T *__restrict__ wu, const double *__restrict__ wsc, const double *__restrict__ w0, int64_t n,
-                   int C, T *__restrict__ up, double *__restrict__ q0, double *__restrict__ e0) {
-  __shared__ __align__(16) T rows[NODES][128];
-  const int64_t first = (int64_t)blockIdx.x * NODES;
-  const int nn = n - first < NODES ? (int)(n - first) : NODES;
-  const int tid = threadIdx.x;
-  for (int i = tid; i < NODES * C; i += MID_THREADS) {
-    const int j = i / C, c = i - j * C;
-    rows[j][c] = j < nn ? b[(int64_t)slot_of[first + j] * C + c] : T(0);
+template <typename T>
+__device__ __forceinline__ void mid_fill(T *sW, const T *__restrict__ W, int C, int tid, int nthreads) {
+  for (int i = tid; i < C * C / (16 / (int)sizeof(T)); i += nthreads) {
+    const uint32_t d = (uint32_t)__cvta_generic_to_shared(sW) + 16u * (uint32_t)i;
+    asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(d), "l"(reinterpret_cast<const char *>(W) + 16 * (int64_t)i) : "memory");
   }
-  __syncthreads();
-  const int groups = MID_THREADS / C;   // threads beyond groups * C (C = 96) only help with the dot products
-  const int c = tid % C, gidx = tid / C;
-  if (gidx < groups) {
-    constexpr int MAXN = NODES / 2;     // C = 128: two groups
-    for (int j0 = gidx * MAXN; j0 < NODES; j0 += groups * MAXN) {
-      T acc[MAXN];
+  asm volatile("cp.async.commit_group;" ::: "memory");
+}
+
+// acc[i][u] = sum_k rows[j0 + i][k] W[k][4 tx + u]
+template <typename T, int PER>
+__device__ __forceinline__ void mid_product(const T *rows, const T *sW, int C, int j0, int tx, T (&acc)[PER][4]) {
 #pragma unroll
-      for (int j = 0; j < MAXN; j++) acc[j] = T(0);
-      for (int k = 0; k < C; k += 4) {
-        T w[4];
+  for (int i = 0; i < PER; i++) acc[i][0] = acc[i][1] = acc[i][2] = acc[i][3] = T(0);
+#pragma unroll 2
+  for (int k = 0; k < C; k += 4) {
+    Quad<T> r[PER];
 #pragma unroll
-        for (int u = 0; u < 4; u++) w[u] = __ldg(wu + (k + u) * C + c);
+    for (int i = 0; i < PER; i++) r[i] = *reinterpret_cast<const Quad<T> *>(rows + (j0 + i) * C + k);
 #pragma unroll
-        for (int j = 0; j < MAXN; j++) {
-          const Quad<T> v = *reinterpret_cast<const Quad<T> *>(&rows[j0 + j][k]);
-          acc[j] = fma(v.x, w[0], acc[j]);
-          acc[j] = fma(v.y, w[1], acc[j]);
-          acc[j] = fma(v.z, w[2], acc[j]);
-          acc[j] = fma(v.w, w[3], acc[j]);
+    for (int u = 0; u < 4; u++) {
+      const Quad<T> w = *reinterpret_cast<const Quad<T> *>(sW + (k + u) * C + 4 * tx);
+#pragma unroll
+      for (int i = 0; i < PER; i++) {
+        const T v = u == 0 ? r[i].x : (u == 1 ? r[i].y : (u == 2 ? r[i].z : r[i].w));
+        acc[i][0] = fma(v, w.x, acc[i][0]);
+        acc[i][1] = fma(v, w.y, acc[i][1]);
+        acc[i][2] = fma(v, w.z, acc[i][2]);
+        acc[i][3] = fma(v, w.w, acc[i][3]);
+      }
+    }
+  }
+}
+
+// extra: [Z][C/4][17][4]
+template <typename T, int NODES>
+__global__ void __launch_bounds__(256)
+    mid_fwd_kernel(const T *__restrict__ b, const int32_t *__restrict__ node_of, const int32_t *__restrict__ slot_type,
+                   const T *__restrict__ wu, const T *__restrict__ extra, int64_t n, int C, T *__restrict__ up,
+                   T *__restrict__ q0) {
+  extern __shared__ __align__(32) unsigned char mid_smem[];
+  T *sW = reinterpret_cast<T *>(mid_smem), *rows = sW + C * C;
+  constexpr int PER = NODES / 8;
+  const int tid = threadIdx.x, nt = 2 * C, tx = tid % (C / 4), ty = tid / (C / 4);
+  mid_fill(sW, wu, C, tid, nt);
+  asm volatile("cp.async.wait_group 0;" ::: "memory");
+  for (int64_t first = (int64_t)blockIdx.x * NODES; first < n; first += (int64_t)gridDim.x * NODES) {
+    const int nn = n - first < NODES ? (int)(n - first) : NODES;
+    __syncthreads();
+    for (int i = tid; i < NODES * C; i += nt) rows[i] = i < nn * C ? b[first * C + i] : T(0);
+    __syncthreads();
+    T acc[PER][4];
+    mid_product<T, PER>(rows, sW, C, ty * PER, tx, acc);
+#pragma unroll
+    for (int i = 0; i < PER; i++)
+      if (ty * PER + i < nn)
+        *reinterpret_cast<Quad<T> *>(up + (int64_t)node_of[first + ty * PER + i] * C + 4 * tx) =
+            Quad<T>{acc[i][0], acc[i][1], acc[i][2], acc[i][3]};
+    for (int i = tid; i < nn * MID_EXTRA; i += nt) {
+      const int j = i / MID_EXTRA, col = i - j * MID_EXTRA;
+      const Quad<T> *w = reinterpret_cast<const Quad<T> *>(extra) + (int64_t)slot_type[first + j] * (C / 4) * MID_EXTRA + col;
+      T a = T(0), a2 = T(0);
+#pragma unroll 8
+      for (int k = 0; k < C / 4; k++) {
+        const Quad<T> x = w[k * MID_EXTRA], r = *reinterpret_cast<const Quad<T> *>(rows + j * C + 4 * k);
+        a = fma(r.x, x.x, a);
+        a2 = fma(r.y, x.y, a2);
+        a = fma(r.z, x.z, a);
+        a2 = fma(r.w, x.w, a2);
+      }
+      q0[(int64_t)node_of[first + j] * MID_EXTRA + col] = a + a2;
+    }
+  }
+}
+
+// grad b0 [slot order] = grad up Wu^T + (dq, scale) [17] extra_t[z] [17, C]
+template <typename T, int NODES>
+__global__ void __launch_bounds__(256)
+    mid_bwd_kernel(const T *__restrict__ gup, const int32_t *__restrict__ node_of, const int32_t *__restrict__ slot_type,
+                   const T *__restrict__ dq, const T *__restrict__ wu_t, const T *__restrict__ extra_t, T scale,
+                   int64_t n, int C, T *__restrict__ gb) {
+  extern __shared__ __align__(32) unsigned char mid_smem[];
+  T *sW = reinterpret_cast<T *>(mid_smem), *rows = sW + C * C, *sdq = rows + NODES * C;
+  constexpr int PER = NODES / 8;
+  const int tid = threadIdx.x, nt = 2 * C, tx = tid % (C / 4), ty = tid / (C / 4);
+  mid_fill(sW, wu_t, C, tid, nt);
+  asm volatile("cp.async.wait_group 0;" ::: "memory");
+  for (int64_t first = (int64_t)blockIdx.x * NODES; first < n; first += (int64_t)gridDim.x * NODES) {
+    const int nn = n - first < NODES ? (int)(n - first) : NODES;
+    __syncthreads();
+    for (int i = tid; i < NODES * C; i += nt) {
+      const int j = i / C;
+      rows[i] = j < nn ? gup[(int64_t)node_of[first + j] * C + (i - j * C)] : T(0);
+    }
+    for (int i = tid; i < nn * ST_RO; i += nt) sdq[i] = dq[(int64_t)node_of[first + i / ST_RO] * ST_RO + i % ST_RO];
+    __syncthreads();
+    T acc[PER][4];
+    mid_product<T, PER>(rows, sW, C, ty * PER, tx, acc);
+#pragma unroll
+    for (int i = 0; i < PER; i++) {
+      const int j = ty * PER + i;
+      if (j < nn) {
+        const Quad<T> *w = reinterpret_cast<const Quad<T> *>(extra_t + (int64_t)slot_type[first + j] * MID_EXTRA * C) + tx;
+#pragma unroll
+        for (int k = 0; k < MID_EXTRA; k++) {
+          const Quad<T> x = w[k * (C / 4)];
+          const T d = k < ST_RO ? sdq[j * ST_RO + k] : scale;
+          acc[i][0] = fma(d, x.x, acc[i][0]);
+          acc[i][1] = fma(d, x.y, acc[i][1]);
+          acc[i][2] = fma(d, x.z, acc[i][2]);
+          acc[i][3] = fma(d, x.w, acc[i][3]);
         }
+        *reinterpret_cast<Quad<T> *>(gb + (first + j) * C + 4 * tx) = Quad<T>{acc[i][0], acc[i][1], acc[i][2], acc[i][3]};
       }
-#pragma unroll
-      for (int j = 0; j < MAXN; j++)
-        if (j0 + j < nn) up[(first + j0 + j) * C + c] = acc[j];
-    }
-  }
-  for (int i = tid; i < nn * ST_RO; i += MID_THREADS) {
-    const int j = i / ST_RO, col = i - j * ST_RO;
-    const double *w = wsc + ((int64_t)species[first + j] * C) * ST_RO + col;
-    double a0 = 0.0, a1 = 0.0;
-    for (int k = 0; k < C; k += 2) {
-      a0 = fma((double)rows[j][k], __ldg(w + k * ST_RO), a0);
-      a1 = fma((double)rows[j][k + 1], __ldg(w + (k + 1) * ST_RO), a1);
-    }
-    q0[(first + j) * ST_RO + col] = a0 + a1;
-  }
-  const int lane = tid & 31;
-  for (int j = tid >> 5; j < nn; j += MID_THREADS / 32) {
-    double a = 0.0;
-    for (int k = lane; k < C; k += 32) a = fma((double)rows[j][k], __ldg(w0 + k), a);
-#pragma unroll
-    for (int off = 16; off > 0; off >>= 1) a += __shfl_xor_sync(0xffffffffu, a, off);
-    if (lane == 0) e0[first + j] = a;
-  }
-}
-
-// grad b0 [slot order] = grad up1 Wu^T + dq Wsc[z]^T + scale w0  (dq already carries the scale)
-template <typename T, int NODES>
-__global__ void __launch_bounds__(MID_THREADS)
-    mid_bwd_kernel(const T *__restrict__ gup, const int32_t *__restrict__ slot_of, const int32_t *__restrict__ species,
-                   const double *__restrict__ dq, const T *__restrict__ wu_t, const double *__restrict__ wsc,
-                   const double *__restrict__ w0, double scale, int64_t n, int C, T *__restrict__ gb) {
-  __shared__ __align__(16) T rows[NODES][128];
-  __shared__ double dqs[NODES][ST_RO];
-  const int64_t first = (int64_t)blockIdx.x * NODES;
-  const int nn = n - first < NODES ? (int)(n - first) : NODES;
-  const int tid = threadIdx.x;
-  for (int i = tid; i < NODES * C; i += MID_THREADS) {
-    const int j = i / C, c = i - j * C;
-    rows[j][c] = j < nn ? gup[(first + j) * C + c] : T(0);
-  }
-  for (int i = tid; i < nn * ST_RO; i += MID_THREADS) dqs[i / ST_RO][i % ST_RO] = dq[first * ST_RO + i];
-  __syncthreads();
-  const int groups = MID_THREADS / C;
-  const int c = tid % C, gidx = tid / C;
-  if (gidx >= groups) return;
-  constexpr int MAXN = NODES / 2;
-  for (int j0 = gidx * MAXN; j0 < NODES; j0 += groups * MAXN) {
-    T acc[MAXN];
-#pragma unroll
-    for (int j = 0; j < MAXN; j++) acc[j] = T(0);
-    for (int k = 0; k < C; k += 4) {
-      T w[4];
-#pragma unroll
-      for (int u = 0; u < 4; u++) w[u] = __ldg(wu_t + (k + u) * C + c);
-#pragma unroll
-      for (int j = 0; j < MAXN; j++) {
-        const Quad<T> v = *reinterpret_cast<const Quad<T> *>(&rows[j0 + j][k]);
-        acc[j] = fma(v.x, w[0], acc[j]);
-        acc[j] = fma(v.y, w[1], acc[j]);
-        acc[j] = fma(v.z, w[2], acc[j]);
-        acc[j] = fma(v.w, w[3], acc[j]);
-      }
-    }
-    const double base = scale * __ldg(w0 + c);
-#pragma unroll
-    for (int j = 0; j < MAXN; j++) {
-      if (j0 + j >= nn) break;
-      const int64_t node = first + j0 + j;
-      const double *w = wsc + ((int64_t)species[node] * C + c) * ST_RO;
-      double s = base;
-#pragma unroll
-      for (int k = 0; k < ST_RO; k++) s = fma(dqs[j0 + j][k], __ldg(w + k), s);
-      gb[(int64_t)slot_of[node] * C + c] = (T)(s + (double)acc[j]);
     }
   }
 }
 
-// 16 nodes a block until that gives every SM two blocks, then 32 (twice the reuse of a weight)
-template <typename T>
-int StepKernels<T>::mid_fwd(const T *b, const int32_t *slot_of, const int32_t *species, const T *wu, const double *wsc,
-                            const double *w0, int64_t n, int C, T *up, double *q0, double *e0, cudaStream_t st) {
-  if (n > 0) {
-    if (n < 32 * 148 * 2)
-      mid_fwd_kernel<T, 16><<<(unsigned)((n + 15) / 16), MID_THREADS, 0, st>>>(b, slot_of, species, wu, wsc, w0, n, C, up, q0, e0);
-    else
-      mid_fwd_kernel<T, 32><<<(unsigned)((n + 31) / 32), MID_THREADS, 0, st>>>(b, slot_of, species, wu, wsc, w0, n, C, up, q0, e0);
-  }
-  return check_launch("cmace_step(mid_fwd)");
+// 8 nodes a tile while that leaves SMs idle, else 32 (four times the reuse of a weight); two blocks an SM in float32
+template <typename T, typename Kernel8, typename Kernel32, typename... Args>
+static int launch_mid(const char *what, int64_t n, int C, Kernel8 k8, Kernel32 k32, cudaStream_t st, Args... args) {
+  if (n == 0) return CMACE_OK;
+  const bool small = n < 32 * 148;
+  const int nodes = small ? 8 : 32;
+  const size_t smem = sizeof(T) * ((size_t)C * C + (size_t)nodes * (C + ST_RO));
+  int64_t blocks = (n + nodes - 1) / nodes;
+  const int64_t cap = 148 * (sizeof(T) == 4 ? 2 : 1);
+  if (blocks > cap) blocks = cap;
+  cudaError_t e = small ? cudaFuncSetAttribute(k8, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem)
+                        : cudaFuncSetAttribute(k32, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+  if (e != cudaSuccess) return fail(CMACE_ERR_CUDA, "%s: %s", what, cudaGetErrorString(e));
+  if (small) k8<<<(unsigned)blocks, 2 * C, smem, st>>>(args...);
+  else k32<<<(unsigned)blocks, 2 * C, smem, st>>>(args...);
+  return check_launch(what);
 }
 template <typename T>
-int StepKernels<T>::mid_bwd(const T *gup, const int32_t *slot_of, const int32_t *species, const double *dq,
-                            const T *wu_t, const double *wsc, const double *w0, double scale, int64_t n, int C, T *gb,
-                            cudaStream_t st) {
-  if (n > 0) {
-    if (n < 32 * 148 * 2)
-      mid_bwd_kernel<T, 16><<<(unsigned)((n + 15) / 16), MID_THREADS, 0, st>>>(gup, slot_of, species, dq, wu_t, wsc, w0, scale, n, C, gb);
-    else
-      mid_bwd_kernel<T, 32><<<(unsigned)((n + 31) / 32), MID_THREADS, 0, st>>>(gup, slot_of, species, dq, wu_t, wsc, w0, scale, n, C, gb);
-  }
-  return check_launch("cmace_step(mid_bwd)");
+int StepKernels<T>::mid_fwd(const T *b, const int32_t *node_of, const int32_t *slot_type, const T *wu, const T *extra,
+                            int64_t n, int C, T *up, T *q0, cudaStream_t st) {
+  return launch_mid<T>("cmace_step(mid_fwd)", n, C, mid_fwd_kernel<T, 8>, mid_fwd_kernel<T, 32>, st, b, node_of, slot_type,
+                       wu, extra, n, C, up, q0);
+}
+template <typename T>
+int StepKernels<T>::mid_bwd(const T *gup, const int32_t *node_of, const int32_t *slot_type, const T *dq, const T *wu_t,
+                            const T *extra_t, double scale, int64_t n, int C, T *gb, cudaStream_t st) {
+  return launch_mid<T>("cmace_step(mid_bwd)", n, C, mid_bwd_kernel<T, 8>, mid_bwd_kernel<T, 32>, st, gup, node_of, slot_type,
+                       dq, wu_t, extra_t, (T)scale, n, C, gb);
 }
 
 #define CMACE_STEP_NODES(T)                                                                                          \
   template int StepKernels<T>::contract_fwd(const T *, const int32_t *, const T *, int64_t, int, T *, cudaStream_t); \
   template int StepKernels<T>::contract_bwd(const T *, const int32_t *, const T *, const T *, int64_t, int, T *,     \
                                             cudaStream_t);                                                           \
-  template int StepKernels<T>::contract_readout(const T *, const int32_t *, const T *, const double *,               \
-                                                const double *, const double *, const double *, const double *,      \
-                                                double, double, int64_t, int, T *, double *, double *, double *,     \
-                                                cudaStream_t);                                                       \
-  template int StepKernels<T>::mid_fwd(const T *, const int32_t *, const int32_t *, const T *, const double *,       \
-                                       const double *, int64_t, int, T *, double *, double *, cudaStream_t);         \
-  template int StepKernels<T>::mid_bwd(const T *, const int32_t *, const int32_t *, const double *, const T *,       \
-                                       const double *, const double *, double, int64_t, int, T *, cudaStream_t);
+  template int StepKernels<T>::contract_readout(const T *, const int32_t *, const T *, const T *, const double *,    \
+                                                const T *, const double *, double, double, int64_t, int, T *, T *,   \
+                                                double *, double *, cudaStream_t);                                   \
+  template int StepKernels<T>::mid_fwd(const T *, const int32_t *, const int32_t *, const T *, const T *, int64_t,   \
+                                       int, T *, T *, cudaStream_t);                                                 \
+  template int StepKernels<T>::mid_bwd(const T *, const int32_t *, const int32_t *, const T *, const T *, const T *, \
+                                       double, int64_t, int, T *, cudaStream_t);
 CMACE_STEP_NODES(float)
 CMACE_STEP_NODES(double)
 

@@ -85,12 +85,13 @@ class EnergyForceEvaluator:
         graph = torch.cuda.CUDAGraph()
         with torch.cuda.graph(graph):
             energy, forces = self(static_pos)
-        self._graph = (graph, static_pos, energy, forces)
+        # the recording reads the plan's weights, whatever the model lays out later
+        self._graph = (graph, static_pos, energy, forces, step.plan_of(self.model))
         return self
 
     def __call__(self, positions_owned):
         if self._graph is not None and not torch.cuda.is_current_stream_capturing():
-            graph, static_pos, energy, forces = self._graph
+            graph, static_pos, energy, forces, _ = self._graph
             static_pos.copy_(positions_owned)
             graph.replay()
             return energy.clone(), forces.clone()
