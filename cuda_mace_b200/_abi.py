@@ -17,7 +17,8 @@ _D = ctypes.c_double
 class StepModel(ctypes.Structure):
     """cmace_step_model of the header: constant weights of one model."""
     _fields_ = [(k, ctypes.c_int32) for k in ("is_f64", "channels", "elements", "nbessel", "cutoff_p", "reserved")] + [
-        ("r_max", _D), ("scale", _D), ("shift", _D), ("radial", (_P * 4) * 2), ("radial_back", _P), ("fold", _P),
+        ("r_max", _D), ("scale", _D), ("shift", _D), ("radial", (_P * 4) * 2), ("radial_half", (_P * 3) * 2),
+        ("half_scales", (ctypes.c_float * 13) * 2), ("radial_back", _P), ("fold", _P),
         ("fold_back", _P * 8), ("linear", _P * 2), ("weff", _P * 2)] + [
         (k, _P) for k in ("up", "up_back", "extra", "extra_back", "readout1", "readout2", "atomic_energies")]
 

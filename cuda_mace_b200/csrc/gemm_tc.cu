@@ -1339,6 +1339,22 @@ int encode_rows_tensor_map(CUtensorMap *tmap, const float *A, int64_t rows, int 
   return CMACE_OK;
 }
 
+// [rows, 128] fp16 as boxes of box_rows rows x 64 columns (128 bytes: one swizzle span)
+int encode_half_rows_tensor_map(CUtensorMap *tmap, const void *base, int64_t rows, int box_rows, const char *what) {
+  memset(tmap, 0, sizeof(*tmap));
+  EncodeTiledFn enc = encode_tiled_fn();
+  if (enc == nullptr) return fail(CMACE_ERR_CUDA, "%s: cuTensorMapEncodeTiled is not available", what);
+  const cuuint64_t dims[2] = {128, (cuuint64_t)rows};
+  const cuuint64_t strides[1] = {256};
+  const cuuint32_t box[2] = {64, (cuuint32_t)box_rows};
+  const cuuint32_t estr[2] = {1, 1};
+  const CUresult r = enc(tmap, CU_TENSOR_MAP_DATA_TYPE_FLOAT16, 2, const_cast<void *>(base), dims, strides, box, estr,
+                         CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_128B,
+                         CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+  if (r != CUDA_SUCCESS) return fail(CMACE_ERR_CUDA, "%s: cuTensorMapEncodeTiled (fp16 rows) failed (%d)", what, (int)r);
+  return CMACE_OK;
+}
+
 // out [rows, N] as 32-row x 32-column boxes (128 bytes per row: one swizzle span) for the epilogue's tile stores
 static int encode_out_tensor_map(CUtensorMap *tmap, float *out, int64_t rows, int N, const char *what) {
   memset(tmap, 0, sizeof(*tmap));

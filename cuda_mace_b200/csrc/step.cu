@@ -26,6 +26,14 @@ namespace cmace {
 
 int radial_pair_f32(const float *basis, int nb, const float *const (*w)[3], int nper, int64_t nedges, float *const *h,
                     float *const *dh, int32_t *status, cudaStream_t st);
+int radial_half(const float *basis, int nb, const void *const (*w)[3], const RadialScales *scales, const int *half_out,
+                int nper, int64_t nedges, void *const *h, void *const *dh, int32_t *status, cudaStream_t st);
+int step_sums_half(const void *h, const float *Y, const int32_t *sender, const int32_t *row_ptr, const int32_t *species,
+                   const int32_t *slot_of, int64_t nnodes, int elements, float out_v, float *A, cudaStream_t st);
+int step_sums_bwd_half(const float *gA, const void *h, const void *dh, const float *Y, const int32_t *sender,
+                       const int32_t *row_ptr, const int32_t *species, const int32_t *slot_of, const float *gY1,
+                       const float *dr1, const Quad<float> *geo, int64_t nnodes, int elements, float out_v, float out_t,
+                       float *gvec, cudaStream_t st);
 int radial_pair_f64(const double *basis, int nb, const double *const (*w)[3], int nper, int64_t nedges,
                     double *const *h, double *const *dh, cudaStream_t st);
 
@@ -130,6 +138,10 @@ static int run_step(const cmace_step_model &m, cmace_step_io &io, const Workspac
   const YStride ys{1, 16};
   const int32_t *start = Z > 1 ? w.elem_start : nullptr;
   constexpr bool f64 = sizeof(T) == 8;
+  // float32 with radial layers whose values are bounded inside fp16's range: h and h' of the first layer are fp16 pairs
+  static_assert(sizeof(RadialScales) == sizeof(m.half_scales[0]), "RadialScales is the header's array");
+  const bool half = !f64 && m.radial_half[0][0] != nullptr;
+  const RadialScales *scales = reinterpret_cast<const RadialScales *>(m.half_scales);
   io.launches++;
   switch (step) {
     case S_EDGE_PREP:
@@ -141,9 +153,16 @@ static int run_step(const cmace_step_model &m, cmace_step_io &io, const Workspac
       for (int i = 0; i < 2; i++)
         for (int k = 0; k < 3; k++) rw[i][k] = static_cast<const T *>(m.radial[i][k]);
       if constexpr (f64) return radial_pair_f64(w.basis, m.nbessel, rw, 2, E, w.h, w.dh, st);
-      else return radial_pair_f32(w.basis, m.nbessel, rw, 2, E, w.h, w.dh, io.status, st);
+      else if (half) {
+        const int half_out[2] = {1, 0};
+        void *const h[2] = {w.h[0], w.h[1]}, *const dh[2] = {w.dh[0], w.dh[1]};
+        return radial_half(w.basis, m.nbessel, m.radial_half, scales, half_out, 2, E, h, dh, io.status, st);
+      } else return radial_pair_f32(w.basis, m.nbessel, rw, 2, E, w.h, w.dh, io.status, st);
     }
-    case S_SUMS: return K::sums(w.h[0], w.Y, io.sender, io.row_ptr, w.species, w.slot_of, n, Z, w.A, st);
+    case S_SUMS:
+      if constexpr (!f64)
+        if (half) return step_sums_half(w.h[0], w.Y, io.sender, io.row_ptr, w.species, w.slot_of, n, Z, scales[0].out_v, w.A, st);
+      return K::sums(w.h[0], w.Y, io.sender, io.row_ptr, w.species, w.slot_of, n, Z, w.A, st);
     case S_FOLD: return linear_any(w.A, m.fold, start, Z, n, ST_H * Z, C, w.m0, io.status, st);
     case S_CONTRACT0: return K::contract_fwd(w.m0, w.slot_type, static_cast<const T *>(m.weff[0]), n, C, w.b0, st);
     case S_MID_FWD:
@@ -192,6 +211,10 @@ static int run_step(const cmace_step_model &m, cmace_step_io &io, const Workspac
       }
       return CMACE_OK;
     case S_SUMS_BACK:
+      if constexpr (!f64)
+        if (half)
+          return step_sums_bwd_half(w.gA, w.h[0], w.dh[0], w.Y, io.sender, io.row_ptr, w.species, w.slot_of, w.gY1, w.dr1,
+                                    w.geo, n, Z, scales[0].out_v, scales[0].out_t, w.gvec, st);
       return K::sums_bwd(w.gA, w.h[0], w.dh[0], w.Y, io.sender, io.row_ptr, w.species, w.slot_of, w.gY1, w.dr1, w.geo, n,
                          Z, w.gvec, st);
     case S_FORCES:

@@ -14,6 +14,7 @@
 // where h' = dh/dr came with the forward, so no gradient passes back through the perceptron.
 #include "edge_math.cuh"
 #include "step_common.cuh"
+#include "tc_ptx.cuh"
 
 namespace cmace {
 
@@ -39,10 +40,11 @@ __device__ void group_nodes(const int32_t *species_in, const void *one_hot, int 
                             int32_t *slot_type, int32_t *elem_start) {
   __shared__ int count[ST_MAX_Z][EP_THREADS + 1];
   const int t = threadIdx.x, lane = t & 31, w = t >> 5;
-  const int64_t per = (n_owned + EP_THREADS - 1) / EP_THREADS;
+  const int64_t per = (n_owned + 4 * EP_THREADS - 1) / (4 * EP_THREADS) * 4;   // pieces of whole 16-byte groups
   const int64_t lo = t * per < n_owned ? t * per : n_owned, hi = lo + per < n_owned ? lo + per : n_owned;
   for (int z = 0; z < elements; z++) count[z][t] = 0;
   // coalesced pass over the species first: the counting pass then reads what this block wrote
+#pragma unroll 4
   for (int64_t i = t; i < n_local; i += EP_THREADS) {
     int z;
     if (species_in) z = species_in[i];
@@ -51,7 +53,14 @@ __device__ void group_nodes(const int32_t *species_in, const void *one_hot, int 
     species[i] = z < 0 ? 0 : (z >= elements ? elements - 1 : z);
   }
   __syncthreads();
-  for (int64_t i = lo; i < hi; i++) count[species[i]][t]++;
+#pragma unroll 4
+  for (int64_t i = lo; i < hi; i += 4) {
+    const int4 z = *reinterpret_cast<const int4 *>(species + i);
+    count[z.x][t]++;
+    if (i + 1 < hi) count[z.y][t]++;
+    if (i + 2 < hi) count[z.z][t]++;
+    if (i + 3 < hi) count[z.w][t]++;
+  }
   __syncthreads();
   // exclusive prefix over (element, thread): warp w scans elements w, w + 8, ...
   __shared__ int total[ST_MAX_Z];
@@ -82,12 +91,19 @@ __device__ void group_nodes(const int32_t *species_in, const void *one_hot, int 
     elem_start[elements] = acc;
   }
   __syncthreads();
-  for (int64_t i = lo; i < hi; i++) {
-    const int z = species[i];
-    const int s = total[z] + count[z][t]++;
-    slot_of[i] = s;
-    node_of[s] = (int32_t)i;
-    slot_type[s] = z;
+#pragma unroll 4
+  for (int64_t i = lo; i < hi; i += 4) {
+    const int4 z4 = *reinterpret_cast<const int4 *>(species + i);
+#pragma unroll
+    for (int u = 0; u < 4; u++) {
+      const int z = u == 0 ? z4.x : (u == 1 ? z4.y : (u == 2 ? z4.z : z4.w));
+      if (i + u < hi) {
+        const int s = total[z] + count[z][t]++;
+        slot_of[i + u] = s;
+        node_of[s] = (int32_t)(i + u);
+        slot_type[s] = z;
+      }
+    }
   }
 }
 
@@ -283,6 +299,87 @@ __global__ void __launch_bounds__(SU_WARPS * 32)
       row[2 * u + 1] = make_float4(acc[4][2 * half + u], acc[5][2 * half + u], acc[6][2 * half + u], acc[7][2 * half + u]);
     }
   }
+}
+
+__device__ __forceinline__ void mma_f16(float (&c)[4], const uint32_t (&a)[4], uint32_t b0, uint32_t b1) {
+  asm volatile(
+      "mma.sync.aligned.m16n8k16.row.col.f32.f16.f16.f32 {%0, %1, %2, %3}, {%4, %5, %6, %7}, {%8, %9}, {%0, %1, %2, %3};"
+      : "+f"(c[0]), "+f"(c[1]), "+f"(c[2]), "+f"(c[3])
+      : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b0), "r"(b1));
+}
+
+// The same with h as fp16 hi / lo rows ([E][hi 64 | lo 64], scaled): sixteen edges an instruction, nothing to split but
+// Y (times 2^8: |Y| < 2.7).  Lane (g, t) reads 16 bytes of the hi and of the lo row of edges 2 t, 2 t + 1, 2 t + 8,
+// 2 t + 9; a B fragment pairs the same column of two edges (one byte permute).
+constexpr float SU_Y_SCALE = 256.f;
+
+__global__ void __launch_bounds__(SU_WARPS * 32)
+    sums_f16_kernel(const uint4 *__restrict__ h, const float *__restrict__ Y, const int32_t *__restrict__ sender,
+                    const int32_t *__restrict__ row_ptr, const int32_t *__restrict__ species,
+                    const int32_t *__restrict__ slot_of, int64_t nnodes, int elements, float factor,
+                    float *__restrict__ A) {
+  __shared__ int32_t lists[SU_WARPS][SU_LIST];
+  const int lane = threadIdx.x & 31, w = threadIdx.x >> 5, g = lane >> 2, t = lane & 3;
+  const int64_t pair = (int64_t)blockIdx.x * SU_WARPS + w;
+  if (pair >= nnodes * elements) return;
+  const int64_t node = pair / elements;
+  const int z = (int)(pair - node * elements);
+  int32_t *list = lists[w];
+  float acc[8][4];
+#pragma unroll
+  for (int j = 0; j < 8; j++) acc[j][0] = acc[j][1] = acc[j][2] = acc[j][3] = 0.f;
+  for_edges_of_element(sender, species, row_ptr[node], row_ptr[node + 1], z, list, lane, [&](int n) {
+    for (int j0 = 0; j0 < n; j0 += 16) {
+      uint4 hv[4], lv[4];
+      uint32_t ah[4], al[4];
+#pragma unroll
+      for (int u = 0; u < 2; u++) {
+        float y[2][2];
+#pragma unroll
+        for (int v = 0; v < 2; v++) {   // past the end: the last edge with Y = 0
+          const int j = j0 + 8 * u + 2 * t + v;
+          const int64_t e = list[j < n ? j : n - 1];
+          hv[2 * u + v] = __ldg(h + e * 16 + g);
+          lv[2 * u + v] = __ldg(h + e * 16 + 8 + g);
+          y[v][0] = j < n ? __ldg(Y + e * 16 + g) * SU_Y_SCALE : 0.f;
+          y[v][1] = j < n ? __ldg(Y + e * 16 + g + 8) * SU_Y_SCALE : 0.f;
+        }
+        split_half2(pack2(y[0][0], y[1][0]), ah[2 * u], al[2 * u]);
+        split_half2(pack2(y[0][1], y[1][1]), ah[2 * u + 1], al[2 * u + 1]);
+      }
+#pragma unroll
+      for (int j = 0; j < 8; j++) {
+        auto word = [&](const uint4 &x) { return (j >> 1) == 0 ? x.x : ((j >> 1) == 1 ? x.y : ((j >> 1) == 2 ? x.z : x.w)); };
+        const uint32_t sel = (j & 1) ? 0x7632u : 0x5410u;
+        const uint32_t h0 = __byte_perm(word(hv[0]), word(hv[1]), sel), h1 = __byte_perm(word(hv[2]), word(hv[3]), sel);
+        const uint32_t l0 = __byte_perm(word(lv[0]), word(lv[1]), sel), l1 = __byte_perm(word(lv[2]), word(lv[3]), sel);
+        mma_f16(acc[j], ah, h0, h1);
+        mma_f16(acc[j], ah, l0, l1);
+        mma_f16(acc[j], al, h0, h1);
+      }
+    }
+  });
+  const int width = elements * ST_H;
+  float *o = A + (int64_t)slot_of[node] * 16 * width + z * ST_H + 16 * t;
+#pragma unroll
+  for (int half = 0; half < 2; half++) {   // rows lm = g and g + 8
+    float4 *row = reinterpret_cast<float4 *>(o + (int64_t)(g + 8 * half) * width);
+#pragma unroll
+    for (int u = 0; u < 2; u++) {
+      const int c = 2 * half + u;
+      row[2 * u] = make_float4(acc[0][c] * factor, acc[1][c] * factor, acc[2][c] * factor, acc[3][c] * factor);
+      row[2 * u + 1] = make_float4(acc[4][c] * factor, acc[5][c] * factor, acc[6][c] * factor, acc[7][c] * factor);
+    }
+  }
+}
+
+int step_sums_half(const void *h, const float *Y, const int32_t *sender, const int32_t *row_ptr, const int32_t *species,
+                   const int32_t *slot_of, int64_t nnodes, int elements, float out_v, float *A, cudaStream_t st) {
+  const int64_t blocks = (nnodes * elements + SU_WARPS - 1) / SU_WARPS;
+  if (blocks > 0)
+    sums_f16_kernel<<<(unsigned)blocks, SU_WARPS * 32, 0, st>>>(static_cast<const uint4 *>(h), Y, sender, row_ptr, species,
+                                                               slot_of, nnodes, elements, out_v / SU_Y_SCALE, A);
+  return check_launch("cmace_step(sums)");
 }
 
 // float64: sums over k = 2 lane, 2 lane + 1
@@ -517,6 +614,131 @@ __global__ void __launch_bounds__(SU_WARPS * 32, 3)
       __syncwarp();
     }
   });
+}
+
+// The same with h and h' as fp16 hi / lo rows.  P is scaled by the power of two that puts its largest entry of the
+// pair just below 2^14 (its magnitude is the caller's gradient's), so its split loses nothing either.  A lane reads
+// pieces t and t + 4 of an edge's 128-byte hi or lo row: piece i holds k = 8 (t + 4 i) .. + 7 of K steps 2 i and 2 i + 1.
+__global__ void __launch_bounds__(SU_WARPS * 32, 4)
+    sums_bwd_f16_kernel(const float *__restrict__ gA, const uint4 *__restrict__ h, const uint4 *__restrict__ dh,
+                        const float *__restrict__ Y, const int32_t *__restrict__ sender,
+                        const int32_t *__restrict__ row_ptr, const int32_t *__restrict__ species,
+                        const int32_t *__restrict__ slot_of, const float *__restrict__ gY1,
+                        const float *__restrict__ dr1, const Quad<float> *__restrict__ geo, int64_t nnodes, int elements,
+                        float out_v, float out_t, float *__restrict__ gvec) {
+  __shared__ int32_t lists[SU_WARPS][SU_LIST];
+  __shared__ float stage[SU_WARPS][32 * 17];
+  const int lane = threadIdx.x & 31, w = threadIdx.x >> 5, g = lane >> 2, t = lane & 3;
+  const int64_t pair = (int64_t)blockIdx.x * SU_WARPS + w;
+  if (pair >= nnodes * elements) return;
+  const int64_t node = pair / elements;
+  const int z = (int)(pair - node * elements);
+  int32_t *list = lists[w];
+  float *st = stage[w];
+  uint32_t ph[4][4], pl[4][4];   // A fragments of the 4 K steps
+  {
+    const int b = z >> 1, width = sums_block_width(elements, b);
+    const float *p = gA + (int64_t)b * nnodes * (16 * 128) + (int64_t)slot_of[node] * 16 * width + (z & 1) * ST_H + 8 * t;
+    float4 v[2][2][2];   // [piece][row g, g + 8][half of the piece]
+    float most = 0.f;
+#pragma unroll
+    for (int i = 0; i < 2; i++)
+#pragma unroll
+      for (int r = 0; r < 2; r++)
+#pragma unroll
+        for (int u = 0; u < 2; u++) {
+          v[i][r][u] = __ldg(reinterpret_cast<const float4 *>(p + (g + 8 * r) * width + 32 * i + 4 * u));
+          most = fmaxf(most, fmaxf(fmaxf(fabsf(v[i][r][u].x), fabsf(v[i][r][u].y)), fmaxf(fabsf(v[i][r][u].z), fabsf(v[i][r][u].w))));
+        }
+#pragma unroll
+    for (int off = 16; off > 0; off >>= 1) most = fmaxf(most, __shfl_xor_sync(0xffffffffu, most, off));
+    int ex = 127 + 13 - ((int)((__float_as_uint(most) >> 23) & 255u) - 127);   // biased exponent of the scale
+    ex = ex < 1 ? 1 : (ex > 253 ? 253 : ex);
+    const float sc = __uint_as_float((uint32_t)ex << 23), inv = __uint_as_float((uint32_t)(254 - ex) << 23);
+    const unsigned long long sc2 = pack2(sc, sc);
+    out_v *= inv;
+    out_t *= inv;
+#pragma unroll
+    for (int i = 0; i < 2; i++)
+#pragma unroll
+      for (int u = 0; u < 2; u++)
+#pragma unroll
+        for (int r = 0; r < 2; r++) {
+          split_half2(mul2(pack2(v[i][r][u].x, v[i][r][u].y), sc2), ph[2 * i + u][r], pl[2 * i + u][r]);
+          split_half2(mul2(pack2(v[i][r][u].z, v[i][r][u].w), sc2), ph[2 * i + u][2 + r], pl[2 * i + u][2 + r]);
+        }
+  }
+  for_edges_of_element(sender, species, row_ptr[node], row_ptr[node + 1], z, list, lane, [&](int n) {
+    for (int j0 = 0; j0 < n; j0 += 32) {
+      const int nj = n - j0 < 32 ? n - j0 : 32;
+      uint4 hh[2], hl[2], dd[2], dl[2];
+      auto load = [&](int j) {   // edge j0 + j + g, or the last one
+        const int i = j0 + j + g;
+        const int64_t e = list[i < n ? i : n - 1];
+#pragma unroll
+        for (int q = 0; q < 2; q++) {
+          hh[q] = __ldg(h + e * 16 + t + 4 * q);
+          hl[q] = __ldg(h + e * 16 + 8 + t + 4 * q);
+          dd[q] = __ldg(dh + e * 16 + t + 4 * q);
+          dl[q] = __ldg(dh + e * 16 + 8 + t + 4 * q);
+        }
+      };
+      load(0);
+      for (int j = 0; j < nj; j += 8) {
+        float ch[4] = {0.f, 0.f, 0.f, 0.f}, cd[4] = {0.f, 0.f, 0.f, 0.f};
+        const int i0 = j0 + j + 2 * t;   // this lane's result columns: edges 2 t and 2 t + 1 of the eight
+        const int64_t e0 = list[i0 < n ? i0 : n - 1], e1 = list[i0 + 1 < n ? i0 + 1 : n - 1];
+        const float y00 = __ldg(Y + e0 * 16 + g), y01 = __ldg(Y + e0 * 16 + g + 8);
+        const float y10 = __ldg(Y + e1 * 16 + g), y11 = __ldg(Y + e1 * 16 + g + 8);
+#pragma unroll
+        for (int q = 0; q < 2; q++) {
+          mma_f16(ch, ph[2 * q], hh[q].x, hh[q].y);
+          mma_f16(cd, ph[2 * q], dd[q].x, dd[q].y);
+          mma_f16(ch, ph[2 * q], hl[q].x, hl[q].y);
+          mma_f16(cd, ph[2 * q], dl[q].x, dl[q].y);
+          mma_f16(ch, pl[2 * q], hh[q].x, hh[q].y);
+          mma_f16(cd, pl[2 * q], dd[q].x, dd[q].y);
+          mma_f16(ch, ph[2 * q + 1], hh[q].z, hh[q].w);
+          mma_f16(cd, ph[2 * q + 1], dd[q].z, dd[q].w);
+          mma_f16(ch, ph[2 * q + 1], hl[q].z, hl[q].w);
+          mma_f16(cd, ph[2 * q + 1], dl[q].z, dl[q].w);
+          mma_f16(ch, pl[2 * q + 1], hh[q].z, hh[q].w);
+          mma_f16(cd, pl[2 * q + 1], dd[q].z, dd[q].w);
+        }
+        if (j + 8 < nj) load(j + 8);
+        float *s0 = st + (j + 2 * t) * 17, *s1 = s0 + 17;
+        s0[g] = ch[0] * out_v;
+        s1[g] = ch[1] * out_v;
+        s0[g + 8] = ch[2] * out_v;
+        s1[g + 8] = ch[3] * out_v;
+        float r0 = fmaf(y00, cd[0], y01 * cd[2]), r1 = fmaf(y10, cd[1], y11 * cd[3]);
+#pragma unroll
+        for (int off = 4; off < 32; off <<= 1) {
+          r0 += __shfl_xor_sync(0xffffffffu, r0, off);
+          r1 += __shfl_xor_sync(0xffffffffu, r1, off);
+        }
+        if (g == 0) {
+          s0[16] = r0 * out_t;
+          s1[16] = r1 * out_t;
+        }
+      }
+      __syncwarp();
+      if (lane < nj) finish_edge<float>(st + lane * 17, list[j0 + lane], gY1, dr1, geo, gvec);
+      __syncwarp();
+    }
+  });
+}
+
+int step_sums_bwd_half(const float *gA, const void *h, const void *dh, const float *Y, const int32_t *sender,
+                       const int32_t *row_ptr, const int32_t *species, const int32_t *slot_of, const float *gY1,
+                       const float *dr1, const Quad<float> *geo, int64_t nnodes, int elements, float out_v, float out_t,
+                       float *gvec, cudaStream_t st) {
+  const int64_t blocks = (nnodes * elements + SU_WARPS - 1) / SU_WARPS;
+  if (blocks > 0)
+    sums_bwd_f16_kernel<<<(unsigned)blocks, SU_WARPS * 32, 0, st>>>(
+        gA, static_cast<const uint4 *>(h), static_cast<const uint4 *>(dh), Y, sender, row_ptr, species, slot_of, gY1, dr1,
+        geo, nnodes, elements, out_v, out_t, gvec);
+  return check_launch("cmace_step(sums_back)");
 }
 
 // float64: a lane holds k = 2 lane, 2 lane + 1 of P

@@ -26,6 +26,60 @@ def _pack(Bt):
     return out
 
 
+def half_images(Wt, scale):
+    """fp16 hi and lo images of Wt [N, K <= 64] * scale: rows of 64 fp16 with the tensor core's 128-byte swizzle."""
+    N, K = Wt.shape
+    w = torch.zeros(N, 64, dtype=torch.float32, device=Wt.device)
+    w[:, :K] = Wt * scale
+    hi = w.half()
+    images = torch.stack([hi, (w - hi.float()).half()]).view(2, N, 8, 8)
+    rows = torch.arange(N, device=Wt.device)[:, None]
+    chunk = torch.arange(8, device=Wt.device)[None, :]
+    out = torch.empty_like(images)
+    out[:, rows, chunk ^ (rows & 7)] = images
+    return out
+
+
+def basis_bounds(nb, r_max, p):
+    """Largest |b_n| and |db_n/dr| of the radial basis on (0, r_max): sampled on a grid far finer than the n-th wave
+    (32 points per nb = 16 half-wave), plus 5 %."""
+    r = torch.arange(1, 4097, dtype=torch.float64) * (r_max / 4096)
+    x = r / r_max
+    f = 1 - 0.5 * (p + 1) * (p + 2) * x**p + p * (p + 2) * x**(p + 1) - 0.5 * p * (p + 1) * x**(p + 2)
+    df = 0.5 * p * (p + 1) * (p + 2) * (-x**(p - 1) + 2 * x**p - x**(p + 1)) / r_max
+    w = torch.arange(1, nb + 1, dtype=torch.float64)[:, None] * math.pi / r_max
+    pref = math.sqrt(2.0 / r_max)
+    b = pref * torch.sin(w * r) / r
+    db = pref * (w * torch.cos(w * r) / r - torch.sin(w * r) / r**2)
+    return (1.05 * (b * f).abs().amax(dim=1), 1.05 * (db * f + b * df).abs().amax(dim=1))
+
+
+def half_scales(Ws, bounds):
+    """The 13 powers of two of the fp16 radial kernel and the weights' factors, or None when a bound of some layer's
+    values or derivatives exceeds 2^15.  |silu(z)| <= |z| and |silu'| < 1.1 carry the bounds from layer to layer."""
+    def power(t):   # the power of two that puts the largest entry just below 2^15
+        return 14 - math.floor(math.log2(max(float(t.max()), 1e-30)))
+
+    v, d = bounds
+    sv, sd = power(v), power(d)
+    out = [2.0**sv, 2.0**sd]
+    z, a, t, factors = [], [], [], []
+    for W in Ws:
+        w = W.double().abs().cpu()
+        sw = power(w) - 1
+        v, d = v @ w, 1.1 * (d @ w)
+        nv, nd = power(v), power(d)
+        if min(nv, nd, sv, sd) < 0:
+            return None
+        nv, nd = min(nv, 12), min(nd, 12)
+        z.append(2.0 ** -(sv + sw))
+        a.append(2.0 ** (nv - sv - sw))
+        t.append(2.0 ** (nd - sd - sw))
+        factors.append(2.0**sw)
+        sv, sd = nv, nd
+    return out + z + a + t + [2.0**-sv, 2.0**-sd], factors
+
+
 def covers(model):
     """Whether the sequence covers a model: the standard two-layer architecture in float32 or float64."""
     if model.radial != "exact" or len(model.layers) != 2 or model.num_elements > 16:
@@ -74,6 +128,19 @@ class StepPlan:
             for i in range(4):
                 if (t, i) != (0, 3):
                     m.radial[t][i] = matrix(getattr(L, f"W_radial{i}"))
+        if f32:
+            bounds = basis_bounds(m.nbessel, m.r_max, m.cutoff_p)
+            scales = [half_scales([getattr(L, f"W_radial{i}") for i in range(3)], bounds) for L in (L0, L1)]
+            if None not in scales:
+                for t, L in enumerate((L0, L1)):
+                    values, factors = scales[t]
+                    if t == 1:   # the second layer's h and h' leave as float32: undo the stored scale
+                        values[7] *= values[11]
+                        values[10] *= values[12]
+                        values[11] = values[12] = 1.0
+                    m.half_scales[t][:] = values
+                    for i in range(3):
+                        m.radial_half[t][i] = hold(half_images(getattr(L, f"W_radial{i}").t(), factors[i]))
         m.radial_back = matrix(L1.W_radial3.t())
         x = d(model.embedding) @ d(L0.W_up)                                  # [Z, C] sender features of the first layer
         w4 = d(L0.W_radial3).view(_H, 4, C)

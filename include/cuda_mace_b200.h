@@ -352,6 +352,9 @@ typedef struct cmace_step_model {
   double r_max, scale, shift;
   const void *radial[2][4];  /* float32: packed images of W1..W4 (cmace_gemm_pack_weights_f32 of the transposes);
                                 float64: W1 [nb,64], W2, W3 [64,64], W4 [64,4C]; radial[0][3] is not read */
+  const void *radial_half[2][3]; /* float32, or all NULL: fp16 images (hi, lo) of W1^T (rows padded to 64), W2^T, W3^T */
+  float half_scales[2][13];  /* their powers of two: basis, derivative, per layer pre-activation / activation /
+                                derivative, then what undoes the scale of the stored h and h' */
   const void *radial_back;   /* second layer's W4 for the gradient: float32 packed W4 itself, float64 W4^T [4C,64] */
   const void *fold;          /* first layer: [elements][4] matrices [64 elements, C] (float32: packed) */
   const void *fold_back[8];  /* their transposes in blocks of two elements: [elements][4] [C, 128 or 64] */
