@@ -18,7 +18,8 @@ class StepModel(ctypes.Structure):
     """cmace_step_model of the header: constant weights of one model."""
     _fields_ = [(k, ctypes.c_int32) for k in ("is_f64", "channels", "elements", "nbessel", "cutoff_p", "reserved")] + [
         ("r_max", _D), ("scale", _D), ("shift", _D), ("radial", (_P * 4) * 2), ("radial_half", (_P * 3) * 2),
-        ("half_scales", (ctypes.c_float * 13) * 2), ("radial_back", _P), ("fold", _P),
+        ("half_scales", (ctypes.c_float * 13) * 2), ("fused_w", _P), ("fused_scale", ctypes.c_float),
+        ("reserved2", ctypes.c_float), ("radial_back", _P), ("fold", _P),
         ("fold_back", _P * 8), ("linear", _P * 2), ("weff", _P * 2)] + [
         (k, _P) for k in ("up", "up_back", "extra", "extra_back", "readout1", "readout2", "atomic_energies")]
 
@@ -89,6 +90,7 @@ SIGNATURES = {
     "cmace_symcon_effective_weights": [_P, _I, _P, _P, _P, _I, _I, _P, _P],
     "cmace_step_workspace_bytes": [_P, _L, _L, _L],
     "cmace_step_count": [],
+    "cmace_step_struct_bytes": [_I],
     "cmace_step_name": [_I],
     "cmace_step_run": [_P, _P, _I, _I, _P],
     "cmace_symcon_plan_create": [_I, _P, _P, _P, _P, _P, _P, _I, _I, _I, ctypes.POINTER(_P)],
@@ -117,7 +119,7 @@ _RESTYPES = {
 _VALUE_FUNCS = {"cmace_abi_version", "cmace_sender_order_workspace_bytes", "cmace_imp_bwd_scratch_elems",
                 "cmace_gemm_packed_floats", "cmace_imp_bwd_edge_f64_noalloc_max_elems",
                 "cmace_radial_hidden_saved_floats", "cmace_nl_num_cells", "cmace_scan_workspace_bytes",
-                "cmace_imp_staged_stalled", "cmace_step_workspace_bytes", "cmace_step_count", "cmace_step_name",
+                "cmace_imp_staged_stalled", "cmace_step_workspace_bytes", "cmace_step_count", "cmace_step_struct_bytes", "cmace_step_name",
                 "cmace_symcon_plan_destroy", "cmace_symcon_plan_nterms", "cmace_symcon_plan_nclasses",
                 "cmace_symcon_plan_is_canonical"}
 
@@ -156,6 +158,9 @@ def load():
         fn = getattr(lib, name)
         fn.argtypes = argtypes
         fn.restype = _RESTYPES.get(name, _I)
+    for which, struct in enumerate((StepModel, StepIO)):
+        if lib.cmace_step_struct_bytes(which) != ctypes.sizeof(struct):
+            raise ImportError(f"{LIB_PATH} was built from another header: rebuild it with `python -m cuda_mace_b200.build`")
     _lib = lib
     return lib
 

@@ -7,7 +7,8 @@
 //   contract0     b0
 //   mid_fwd       up = b0 Wu, q0 = b0 Wsc[z] [n, 17]                                      (step_nodes.cu)
 //       -- a decomposed system fills the ghost rows of `up` here --
-//   radial_out    second layer: R = h W4 [E, 4C]
+//   radial_out    second layer: R = h W4 [E, 4C]  (not in float32 with 128 channels: `messages` and `edges_back` form R and
+//                 R' = h' W4 themselves, fused_messages.cu, and `radial_back`, `radial_dot` are part of `edges_back`)
 //   messages, linear, contract1 (value, readout, energy and gradient in one kernel), linear_back
 //   edges_back    T [E, C] and grad Y of the second layer; radial_back, radial_dot: dE/dr of the second layer
 //   senders       grad up = sum of T over a sender's edges
@@ -34,6 +35,12 @@ int step_sums_bwd_half(const float *gA, const void *h, const void *dh, const flo
                        const int32_t *row_ptr, const int32_t *species, const int32_t *slot_of, const float *gY1,
                        const float *dr1, const Quad<float> *geo, int64_t nnodes, int elements, float out_v, float out_t,
                        float *gvec, cudaStream_t st);
+int fused_messages(const float *X, const float *Y, const void *h, const void *W, float factor, const int32_t *sender,
+                   const int32_t *receiver, const int32_t *row_ptr, int64_t nnodes, int64_t nedges, float *out,
+                   int32_t *status, cudaStream_t st);
+int fused_messages_back(const float *X, const float *Y, const float *G, const void *h, const void *dh, const void *W,
+                        float factor_v, float factor_t, const int32_t *sender, const int32_t *receiver, int64_t nnodes,
+                        int64_t nedges, float *T, float *gY, int32_t *status, cudaStream_t st);
 int radial_pair_f64(const double *basis, int nb, const double *const (*w)[3], int nper, int64_t nedges,
                     double *const *h, double *const *dh, cudaStream_t st);
 
@@ -63,6 +70,9 @@ __global__ void __launch_bounds__(256)
   for (int off = 8; off > 0; off >>= 1) s += __shfl_xor_sync(0xffffffffu, s, off);
   if (l16 == 0 && e < nedges) dr[e] = s;
 }
+
+// second layer with the radial weights formed inside its kernels: fp16 pairs of h, 128 channels (fused_messages.cu)
+static bool is_fused(const cmace_step_model &m) { return !m.is_f64 && m.fused_w != nullptr && m.channels == 128; }
 
 template <typename T>
 struct Workspace {
@@ -98,7 +108,7 @@ struct Workspace {
     take(b0, n * C);
     take(up, n * C);
     take(q0, n * (ST_RO + 1));
-    take(R, E * 4 * C);
+    take(R, is_fused(m) ? 0 : E * 4 * C);
     take(m1, n * 16 * C);
     take(l1, n * 16 * C);
     take(gX1, n * 16 * C);
@@ -142,6 +152,8 @@ static int run_step(const cmace_step_model &m, cmace_step_io &io, const Workspac
   static_assert(sizeof(RadialScales) == sizeof(m.half_scales[0]), "RadialScales is the header's array");
   const bool half = !f64 && m.radial_half[0][0] != nullptr;
   const RadialScales *scales = reinterpret_cast<const RadialScales *>(m.half_scales);
+  const bool fused = is_fused(m);
+  if (fused && (step == S_RADIAL_OUT || step == S_RADIAL_BACK || step == S_RADIAL_DOT)) return CMACE_OK;
   io.launches++;
   switch (step) {
     case S_EDGE_PREP:
@@ -154,7 +166,7 @@ static int run_step(const cmace_step_model &m, cmace_step_io &io, const Workspac
         for (int k = 0; k < 3; k++) rw[i][k] = static_cast<const T *>(m.radial[i][k]);
       if constexpr (f64) return radial_pair_f64(w.basis, m.nbessel, rw, 2, E, w.h, w.dh, st);
       else if (half) {
-        const int half_out[2] = {1, 0};
+        const int half_out[2] = {1, fused ? 1 : 0};
         void *const h[2] = {w.h[0], w.h[1]}, *const dh[2] = {w.dh[0], w.dh[1]};
         return radial_half(w.basis, m.nbessel, m.radial_half, scales, half_out, 2, E, h, dh, io.status, st);
       } else return radial_pair_f32(w.basis, m.nbessel, rw, 2, E, w.h, w.dh, io.status, st);
@@ -171,7 +183,12 @@ static int run_step(const cmace_step_model &m, cmace_step_io &io, const Workspac
     case S_RADIAL_OUT:
       if constexpr (f64) return cmace_gemm_f64(w.h[1], static_cast<const double *>(m.radial[1][3]), E, ST_H, 4 * C, 1.0, w.R, st);
       else return cmace_gemm3x_f32(w.h[1], static_cast<const float *>(m.radial[1][3]), E, ST_H, 4 * C, 1.0, w.R, io.status, st);
-    case S_MESSAGES: return imp_fwd<T>(up, w.Y, w.R, io.sender, io.row_ptr, n, E, ys, C, w.m1, st);
+    case S_MESSAGES:
+      if constexpr (!f64)
+        if (fused)
+          return fused_messages(up, w.Y, w.h[1], m.fused_w, scales[1].out_v * m.fused_scale, io.sender, io.receiver,
+                                io.row_ptr, n, E, w.m1, io.status, st);
+      return imp_fwd<T>(up, w.Y, w.R, io.sender, io.row_ptr, n, E, ys, C, w.m1, st);
     case S_LINEAR: return linear_any(w.m1, m.linear[0], nullptr, 1, n, C, C, w.l1, io.status, st);
     case S_CONTRACT1:
       return K::contract_readout(w.l1, w.species, static_cast<const T *>(m.weff[1]), static_cast<const T *>(m.readout1),
@@ -179,6 +196,10 @@ static int run_step(const cmace_step_model &m, cmace_step_io &io, const Workspac
                                  io.node_energy, st);
     case S_LINEAR_BACK: return linear_any(w.gX1, m.linear[1], nullptr, 1, n, C, C, w.gm1, io.status, st);
     case S_EDGES_BACK:
+      if constexpr (!f64)
+        if (fused)
+          return fused_messages_back(up, w.Y, w.gm1, w.h[1], w.dh[1], m.fused_w, scales[1].out_v * m.fused_scale,
+                                     scales[1].out_t * m.fused_scale, io.sender, io.receiver, n, E, w.T_, w.gY1, io.status, st);
       return imp_bwd_edge<T>(up, w.Y, w.R, w.gm1, io.sender, io.row_ptr, n, E, ys, C, f64 ? w.gradR : nullptr, w.gY1,
                              w.T_, w.partial, st);
     case S_RADIAL_BACK:
@@ -213,8 +234,8 @@ static int run_step(const cmace_step_model &m, cmace_step_io &io, const Workspac
     case S_SUMS_BACK:
       if constexpr (!f64)
         if (half)
-          return step_sums_bwd_half(w.gA, w.h[0], w.dh[0], w.Y, io.sender, io.row_ptr, w.species, w.slot_of, w.gY1, w.dr1,
-                                    w.geo, n, Z, scales[0].out_v, scales[0].out_t, w.gvec, st);
+          return step_sums_bwd_half(w.gA, w.h[0], w.dh[0], w.Y, io.sender, io.row_ptr, w.species, w.slot_of, w.gY1,
+                                    fused ? nullptr : w.dr1, w.geo, n, Z, scales[0].out_v, scales[0].out_t, w.gvec, st);
       return K::sums_bwd(w.gA, w.h[0], w.dh[0], w.Y, io.sender, io.row_ptr, w.species, w.slot_of, w.gY1, w.dr1, w.geo, n,
                          Z, w.gvec, st);
     case S_FORCES:
@@ -246,6 +267,7 @@ int64_t cmace_step_workspace_bytes(const cmace_step_model *m, int64_t n_owned, i
                    : Workspace<float>(nullptr, *m, n_owned, n_local, nedges).bytes;
 }
 int cmace_step_count(void) { return S_COUNT; }
+int cmace_step_struct_bytes(int which) { return which == 0 ? (int)sizeof(cmace_step_model) : (int)sizeof(cmace_step_io); }
 const char *cmace_step_name(int step) { return step >= 0 && step < S_COUNT ? kStepNames[step] : ""; }
 
 int cmace_step_run(const cmace_step_model *m, cmace_step_io *io, int first, int last, cmace_stream_t stream) {

@@ -499,7 +499,8 @@ __device__ __forceinline__ void finish_edge(const T *st, int64_t e, const T *__r
     g[4 * i + 2] = st[4 * i + 2] + q.z;
     g[4 * i + 3] = st[4 * i + 3] + q.w;
   }
-  const T dr = st[16] + dr1[e];
+  // without an array of its own the second layer's dE/dr is component 0 of its grad Y (Y_00 is constant)
+  const T dr = st[16] + (dr1 != nullptr ? dr1[e] : gy[0].x);
   const Quad<T> q = geo[e];   // unit vector in the input's component order: harmonic axes are (z, x, y)
   T GX, GY, GZ;
   sph_l3_vjp<T>(q.z, q.x, q.y, g, GX, GY, GZ);

@@ -80,6 +80,13 @@ def half_scales(Ws, bounds):
     return out + z + a + t + [2.0**-sv, 2.0**-sd], factors
 
 
+def fused_rows(device):
+    """Column of W4 [64, 4 * 128] in every row of the fused message kernels' W^T (header, fused_w)."""
+    j, q, i = torch.meshgrid(torch.arange(4), torch.arange(4), torch.arange(32), indexing="ij")
+    degree = torch.where(q < 2, torch.where(j < 2, 3, 0), torch.where(j < 2, 1, 2))
+    return (degree * 128 + 64 * (q & 1) + 2 * i + (j & 1)).reshape(-1).to(device)
+
+
 def covers(model):
     """Whether the sequence covers a model: the standard two-layer architecture in float32 or float64."""
     if model.radial != "exact" or len(model.layers) != 2 or model.num_elements > 16:
@@ -134,13 +141,20 @@ class StepPlan:
             if None not in scales:
                 for t, L in enumerate((L0, L1)):
                     values, factors = scales[t]
-                    if t == 1:   # the second layer's h and h' leave as float32: undo the stored scale
+                    if t == 1 and C != 128:   # the second layer's h and h' leave as float32: undo the stored scale
                         values[7] *= values[11]
                         values[10] *= values[12]
                         values[11] = values[12] = 1.0
                     m.half_scales[t][:] = values
                     for i in range(3):
                         m.radial_half[t][i] = hold(half_images(getattr(L, f"W_radial{i}").t(), factors[i]))
+                if C == 128:
+                    w = L1.W_radial3.t()[fused_rows(L1.W_radial3.device)]   # [512, 64]
+                    scale = 2.0 ** (13 - math.floor(math.log2(max(float(w.abs().max()), 1e-30))))
+                    w = w * scale
+                    hi = w.half()
+                    m.fused_w = hold(torch.cat([hi, (w - hi.float()).half()], dim=1))
+                    m.fused_scale = 1.0 / scale
         m.radial_back = matrix(L1.W_radial3.t())
         x = d(model.embedding) @ d(L0.W_up)                                  # [Z, C] sender features of the first layer
         w4 = d(L0.W_radial3).view(_H, 4, C)

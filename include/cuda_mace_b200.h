@@ -355,6 +355,10 @@ typedef struct cmace_step_model {
   const void *radial_half[2][3]; /* float32, or all NULL: fp16 images (hi, lo) of W1^T (rows padded to 64), W2^T, W3^T */
   float half_scales[2][13];  /* their powers of two: basis, derivative, per layer pre-activation / activation /
                                 derivative, then what undoes the scale of the stored h and h' */
+  const void *fused_w;       /* float32 with 128 channels and radial_half, or NULL: second layer's W4^T as fp16 rows
+                                [512][hi 64 | lo 64], row j*128 + q*32 + i = degree (q < 2 ? (j < 2 ? 3 : 0) : (j < 2 ? 1 : 2)),
+                                channel 64 (q & 1) + 2 i + (j & 1), divided by fused_scale (a power of two) */
+  float fused_scale, reserved2;
   const void *radial_back;   /* second layer's W4 for the gradient: float32 packed W4 itself, float64 W4^T [4C,64] */
   const void *fold;          /* first layer: [elements][4] matrices [64 elements, C] (float32: packed) */
   const void *fold_back[8];  /* their transposes in blocks of two elements: [elements][4] [C, 128 or 64] */
@@ -391,6 +395,7 @@ typedef struct cmace_step_io {
 
 int64_t cmace_step_workspace_bytes(const cmace_step_model *model, int64_t n_owned, int64_t n_local, int64_t nedges);
 int cmace_step_count(void);
+int cmace_step_struct_bytes(int which); /* sizes of cmace_step_model (0) and cmace_step_io (1), for bindings to check */
 const char *cmace_step_name(int step);
 /* runs steps first .. last - 1 of the sequence */
 int cmace_step_run(const cmace_step_model *model, cmace_step_io *io, int first, int last, cmace_stream_t stream);
