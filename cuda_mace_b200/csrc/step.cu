@@ -39,8 +39,8 @@ int fused_messages(const float *X, const float *Y, const void *h, const void *W,
                    const int32_t *receiver, const int32_t *row_ptr, int64_t nnodes, int64_t nedges, float *out,
                    int32_t *status, cudaStream_t st);
 int fused_messages_back(const float *X, const float *Y, const float *G, const void *h, const void *dh, const void *W,
-                        float factor_v, float factor_t, const int32_t *sender, const int32_t *receiver, int64_t nnodes,
-                        int64_t nedges, float *T, float *gY, int32_t *status, cudaStream_t st);
+                        float factor_v, float factor_t, const int32_t *sender, const int32_t *receiver, int64_t nedges,
+                        float *T, float *gY, int32_t *status, cudaStream_t st);
 int radial_pair_f64(const double *basis, int nb, const double *const (*w)[3], int nper, int64_t nedges,
                     double *const *h, double *const *dh, cudaStream_t st);
 
@@ -198,8 +198,8 @@ static int run_step(const cmace_step_model &m, cmace_step_io &io, const Workspac
     case S_EDGES_BACK:
       if constexpr (!f64)
         if (fused)
-          return fused_messages_back(up, w.Y, w.gm1, w.h[1], w.dh[1], m.fused_w, scales[1].out_v * m.fused_scale,
-                                     scales[1].out_t * m.fused_scale, io.sender, io.receiver, n, E, w.T_, w.gY1, io.status, st);
+          return fused_messages_back(up, w.Y, w.gm1, w.h[1], w.dh[1], m.fused_w_back, scales[1].out_v * m.fused_scale,
+                                     scales[1].out_t * m.fused_scale, io.sender, io.receiver, E, w.T_, w.gY1, io.status, st);
       return imp_bwd_edge<T>(up, w.Y, w.R, w.gm1, io.sender, io.row_ptr, n, E, ys, C, f64 ? w.gradR : nullptr, w.gY1,
                              w.T_, w.partial, st);
     case S_RADIAL_BACK:
