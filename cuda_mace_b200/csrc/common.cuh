@@ -99,6 +99,18 @@ __device__ __forceinline__ void store_vec_stream(T *p, const T (&src)[VEC]) {
   __stcs(reinterpret_cast<V *>(p), v);
 }
 
+// One thread of a converged warp, always the same one (elect.sync).  What it guards (tcgen05.mma, TMA and bulk copies) takes
+// uniform-register operands: under `lane == 0` the compiler does not know that a single thread is left and wraps every such
+// instruction in a loop over the lanes (a tcgen05.mma then costs 125-190 cycles to issue; elected, M = 128 with A in
+// tensor memory runs at 9, 16, 32, 64 cycles for N = 16, 32, 64, 128, and with A in shared memory at 39, 40, 48, 64).
+__device__ __forceinline__ bool elect_one() {
+  uint32_t e;
+  asm volatile("{\n\t.reg .pred p;\n\telect.sync _|p, 0xffffffff;\n\tselp.u32 %0, 1, 0, p;\n\t}" : "=r"(e));
+  return e != 0;
+}
+// a value that is the same in every lane of the warp, known to the compiler as such
+__device__ __forceinline__ int uniform(int v) { return __shfl_sync(0xffffffffu, v, 0); }
+
 // ---- two floats in one 64-bit register, handled by one instruction (fma / mul / add / sub .f32x2) --------------
 // The kernels that use these are bound by instruction issue, not by the FMA pipe.
 __device__ __forceinline__ unsigned long long pack2(float a, float b) {

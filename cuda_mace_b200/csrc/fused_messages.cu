@@ -215,7 +215,7 @@ __global__ void __launch_bounds__(FM_THREADS, 1)
   __shared__ int64_t range_s[FM_SETS + 1];
 
   const uint32_t smem_base = (smem_u32(smem) + 1023u) & ~1023u;
-  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+  const int tid = threadIdx.x, warp = uniform(tid >> 5), lane = tid & 31;
   // warps 0-3, 4-7: consumers of sets 0, 1; 8, 9: their MMA warps; 10, 11: their loaders
   const int set = warp < 8 ? warp >> 2 : warp & 1;
   const uint32_t h_full = smem_u32(&bars[set][0]), x_full = h_full + 8u * FF_STAGES, st_free = x_full + 8u * FF_STAGES;
@@ -244,7 +244,7 @@ __global__ void __launch_bounds__(FM_THREADS, 1)
   tc_fence_before();
   __syncthreads();
   tc_fence_after();
-  const uint32_t tmem = tmem_base_slot, acc_t = tmem + 256u + 128u * (uint32_t)set;
+  const uint32_t tmem = (uint32_t)uniform((int)tmem_base_slot), acc_t = tmem + 256u + 128u * (uint32_t)set;
   if (warp < 4) load_w_tmem(g.W, tmem, warp, lane);
   tc_fence_before();
   __syncthreads();
@@ -271,7 +271,7 @@ __global__ void __launch_bounds__(FM_THREADS, 1)
       }
       const int64_t base = e0 + t * FF_TILE, e = base + lane < e1 ? base + lane : e1 - 1;
       const uint32_t sX = stages + (uint32_t)stage * FF_STAGE_BYTES, sH = sX + FF_X_BYTES, sY = sH + FF_H_BYTES;
-      if (lane == 0) {
+      if (elect_one()) {
         mbar_arrive_expect_tx(h_full + 8u * stage, FF_H_BYTES);
         tma_load_2d(sH, &h_map, 0, (int)base, h_full + 8u * stage);
         tma_load_2d(sH + FF_H_BYTES / 2, &h_map, 64, (int)base, h_full + 8u * stage);
@@ -282,7 +282,7 @@ __global__ void __launch_bounds__(FM_THREADS, 1)
       recv_s[set][stage][lane] = r;
       if (lane == 0) last_s[set][stage] = last;
       __syncwarp();
-      if (lane == 0) {
+      if (elect_one()) {
         const uint32_t bytes = (uint32_t)(e1 - base < FF_TILE ? e1 - base : FF_TILE) * 64u;
         mbar_arrive_expect_tx(x_full + 8u * stage, bytes);
         bulk_copy_g2s(sY, g.Y + base * 16, bytes, x_full + 8u * stage);
@@ -298,7 +298,7 @@ __global__ void __launch_bounds__(FM_THREADS, 1)
         if (lane == 0 && g.status) atomicCAS(g.status, 0, 42);
         break;
       }
-      if (lane == 0) {
+      if (elect_one()) {
         tc_fence_after();
         issue_tile(tmem, acc_t, stages + (uint32_t)stage * FF_STAGE_BYTES + FF_X_BYTES, FF_H_BYTES / 2);
         umma_commit(acc_full);

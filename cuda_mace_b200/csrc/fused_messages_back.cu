@@ -137,7 +137,7 @@ __global__ void __launch_bounds__(EB_THREADS, 1)
   __shared__ uint32_t tmem_base_slot;
 
   const uint32_t base_s = (smem_u32(smem) + 1023u) & ~1023u;
-  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+  const int tid = threadIdx.x, warp = uniform(tid >> 5), lane = tid & 31;
   const uint32_t w_full = smem_u32(&bars[0]), w_free = w_full + 8u * EB_W_SLOTS;
   const uint32_t x_full = w_free + 8u * EB_W_SLOTS, x_free = x_full + 8u * EB_X_SLOTS;
   const uint32_t g_full = x_free + 8u * EB_X_SLOTS, g_free = g_full + 16u, h_full = g_free + 16u;
@@ -165,7 +165,7 @@ __global__ void __launch_bounds__(EB_THREADS, 1)
   tc_fence_before();
   __syncthreads();
   tc_fence_after();
-  const uint32_t tmem = tmem_base_slot;   // h buffer b at 128 b: h hi, h lo, h' hi, h' lo (32 each); acc b at 256 + 128 b
+  const uint32_t tmem = (uint32_t)uniform((int)tmem_base_slot);   // h buffer b at 128 b: h hi, h lo, h' hi, h' lo (32 each); acc b at 256 + 128 b
   const int64_t ntiles = (g.nedges + EB_TILE - 1) / EB_TILE;
 
   if (warp < 8) {
@@ -252,7 +252,7 @@ __global__ void __launch_bounds__(EB_THREADS, 1)
           break;
         }
         tc_fence_after();
-        if (lane == 0) tma_store_wait_read();   // the previous block's T has left the piece
+        if (elect_one()) tma_store_wait_read();   // the previous block's T has left the piece
         __syncwarp();
         const uint32_t sX = base_s + EB_OFF_X + (uint32_t)xs * EB_X_BYTES;
 #pragma unroll 1
@@ -274,7 +274,7 @@ __global__ void __launch_bounds__(EB_THREADS, 1)
         tc_fence_before();
         fence_proxy_async();
         __syncwarp();
-        if (lane == 0) {
+        if (elect_one()) {
           mbar_arrive(acc_free + 8u * set);
           mbar_arrive(x_free + 8u * xs);
           if (base + 32 * q < g.nedges) tma_store_2d(&t_map, EB_BLK * blk, (int)base + 32 * q, sT);
@@ -315,7 +315,8 @@ __global__ void __launch_bounds__(EB_THREADS, 1)
       }
     }
     asm volatile("cp.async.wait_all;" ::: "memory");
-    if (lane == 0) tma_store_wait_all();
+    __syncwarp();
+    if (elect_one()) tma_store_wait_all();
   } else if (warp == 8) {
     // ---- MMA issuer
     const uint32_t idesc = umma_idesc_f16(128, 64);
@@ -328,7 +329,7 @@ __global__ void __launch_bounds__(EB_THREADS, 1)
         const uint32_t b = (uint32_t)blk & 1u, use = 4u * k + (uint32_t)(blk >> 1);
         ok = warp_wait(acc_free + 8u * b, (use & 1u) ^ 1u, lane) && warp_wait(w_full + 8u * slot, wphase, lane);
         if (!ok) break;
-        if (lane == 0) {
+        if (elect_one()) {
           tc_fence_after();
           const uint32_t sW = base_s + EB_OFF_W + (uint32_t)slot * EB_W_BYTES;
           const uint64_t b_hi = umma_desc_sw128(sW), b_lo = umma_desc_sw128(sW + EB_W_BYTES / 2);
@@ -355,7 +356,7 @@ __global__ void __launch_bounds__(EB_THREADS, 1)
     if (!ok && lane == 0 && g.status) atomicCAS(g.status, 0, 63);
   } else if (warp == 9) {
     // ---- W blocks and G rows; one thread
-    if (lane == 0) {
+    if (elect_one()) {
       int slot = 0;
       uint32_t wphase = 0, k = 0;
       bool ok = true;

@@ -299,7 +299,7 @@ __global__ void __launch_bounds__((GT_PRODUCER_WARPS + 1 + EW + 1) * 32, 1)
   const int GT_STAGES = g.stages;
   const uint32_t GT_STAGE_BYTES = (uint32_t)g.stage_bytes;
 
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int warp = uniform(threadIdx.x >> 5), lane = threadIdx.x & 31;
 
   if (threadIdx.x == 0) {
     for (int s = 0; s < GT_STAGES; s++) {
@@ -323,7 +323,7 @@ __global__ void __launch_bounds__((GT_PRODUCER_WARPS + 1 + EW + 1) * 32, 1)
   tc_fence_before();
   __syncthreads();
   tc_fence_after();
-  const uint32_t tmem_base = tmem_base_slot;
+  const uint32_t tmem_base = (uint32_t)uniform((int)tmem_base_slot);
 
   const int k_blocks = g.k_blocks;
   const uint32_t b_image = (uint32_t)g.npad * 128u;  // bytes of one B image
@@ -714,7 +714,7 @@ __global__ void __launch_bounds__((GT_PRODUCER_WARPS + 1 + EW + 1) * 32, 1)
     // stage's barrier: the TMA tile load of A (128 rows x 32 columns, 128-byte swizzle, zeros outside the
     // matrix) into the hi image, and the bulk copy of the matching pre-packed B block.  Nothing waits in
     // registers for HBM; the ring depth sets the bytes in flight.
-    if (MODE == GT_MODE_GRADR && lane == 0) {
+    if (MODE == GT_MODE_GRADR && elect_one()) {
       // Per item the B block of the producers' K block order (cb outer, l inner) into a ring of g.b_slots slots; per
       // tile one bulk copy of the G rows of the NEXT tile's receiver range (contiguous) into the buffer the producers
       // released, issued in the middle of the current tile: by then every producer warp has left the previous tile
@@ -774,7 +774,7 @@ __global__ void __launch_bounds__((GT_PRODUCER_WARPS + 1 + EW + 1) * 32, 1)
         have = have_next;
       }
     }
-    if (MODE == GT_MODE_LINEAR && TS && g.lin_tma && lane == 0) {
+    if (MODE == GT_MODE_LINEAR && TS && g.lin_tma && elect_one()) {
       // Rows by TMA: per item four box loads (one per quarter of the tile: nq whole nodes x 2l+1 components x 32
       // columns land as consecutive 128-byte rows, swizzled, at the quarter's first row) and the B block, all on the
       // slot's tma_full barrier; the converter warps then add the residual image.  Boxes that reach past the last
@@ -808,7 +808,7 @@ __global__ void __launch_bounds__((GT_PRODUCER_WARPS + 1 + EW + 1) * 32, 1)
         }
       }
     }
-    if (MODE == GT_MODE_LINEAR && TS && !g.lin_tma && lane == 0) {
+    if (MODE == GT_MODE_LINEAR && TS && !g.lin_tma && elect_one()) {
       // Per item the B block of the tile's (l, element) problem into the ring of B blocks, same slot index and
       // barriers as the A images: the copy starts as soon as the slot is released, while the producers still
       // convert the items before it.
@@ -837,7 +837,7 @@ __global__ void __launch_bounds__((GT_PRODUCER_WARPS + 1 + EW + 1) * 32, 1)
         }
       }
     }
-    if (MODE == GT_MODE_PLAIN && lane == 0) {
+    if (MODE == GT_MODE_PLAIN && elect_one()) {
       int stage = 0;
       uint32_t phase = 0;
       bool ok = true;
@@ -878,7 +878,7 @@ __global__ void __launch_bounds__((GT_PRODUCER_WARPS + 1 + EW + 1) * 32, 1)
     // ================================ MMA issuer ================================
     int stage = 0;
     uint32_t phase = 0;
-    uint32_t acc_phase[2] = {0, 0};
+    uint32_t acc_phase = 0;   // one parity bit per accumulator
     int acc = 0;
     bool ok = true;
     if (MODE == GT_MODE_PLAIN && g.b_resident) {
@@ -892,7 +892,7 @@ __global__ void __launch_bounds__((GT_PRODUCER_WARPS + 1 + EW + 1) * 32, 1)
     // One thread runs the whole loop: between two batches of MMAs there is nothing but the barrier test and a few
     // integer operations, no warp-wide shuffle or re-convergence.  Whatever sits between the batches leaves the
     // tensor core idle (the issue of an MMA blocks until the previous ones have drained, so the queue is shallow).
-    if (lane != 0) ok = false;
+    if (ok && elect_one()) {
     // low / high words of the operand descriptors (umma_desc_sw128): the low word of stage 0, its step per stage
     const uint64_t d0 = umma_desc_sw128(smem_base);
     const uint32_t desc_hi32 = (uint32_t)(d0 >> 32);
@@ -914,7 +914,7 @@ __global__ void __launch_bounds__((GT_PRODUCER_WARPS + 1 + EW + 1) * 32, 1)
       // one MMA gives Ahi*Bhi in columns [0, npad) and Ahi*Blo in columns [npad, 2 npad)
       const uint32_t idesc2 = umma_idesc_tf32(GT_TILE_M, 2 * g.npad);
       const uint32_t idesc1 = umma_idesc_tf32(GT_TILE_M, nmma);
-      if (!mbar_wait(acc_empty + 8 * acc, acc_phase[acc] ^ 1)) {
+      if (!mbar_wait(acc_empty + 8 * acc, ((acc_phase >> acc) & 1u) ^ 1u)) {
         report(g, 2);
         break;
       }
@@ -998,9 +998,11 @@ __global__ void __launch_bounds__((GT_PRODUCER_WARPS + 1 + EW + 1) * 32, 1)
           b_ring_lo32 = b_ring_first;
         }
       }
-      acc_phase[acc] ^= 1;
+      acc_phase ^= 1u << acc;
       acc ^= 1;
     }
+    }
+    __syncwarp();
   } else {
     // ================================ epilogue ================================
     // Eight warps: two per tensor-memory lane quarter (a warp may only read lanes 32*(warp%4)..+31), the two
@@ -1037,7 +1039,7 @@ __global__ void __launch_bounds__((GT_PRODUCER_WARPS + 1 + EW + 1) * 32, 1)
         // outside the matrix.
         const uint32_t stg = smem_base + GT_STAGES * GT_STAGE_BYTES + (uint32_t)(warp - (GT_PRODUCER_WARPS + 1)) * 4096u;
         for (int c0 = half * 32; c0 < ncols; c0 += 8 * EW) {
-          if (lane == 0) tma_store_wait_read();   // the previous store has left the staging buffer
+          if (elect_one()) tma_store_wait_read();   // the previous store has left the staging buffer
           __syncwarp();
 #pragma unroll
           for (int h16 = 0; h16 < 2; h16++) {
@@ -1064,7 +1066,7 @@ __global__ void __launch_bounds__((GT_PRODUCER_WARPS + 1 + EW + 1) * 32, 1)
           fence_proxy_async();
           __syncwarp();
           // a box that starts inside the matrix: the engine clips what hangs over, a start outside is never issued
-          if (lane == 0 && T.row0 + q * 32 < g.M)
+          if (T.row0 + q * 32 < g.M && elect_one())
             tma_store_2d(&tmap_out, n0 + c0, (int)T.row0 + q * 32, stg);
         }
       } else if (MODE == GT_MODE_GRADR && g.dot != nullptr) {
@@ -1176,7 +1178,7 @@ __global__ void __launch_bounds__((GT_PRODUCER_WARPS + 1 + EW + 1) * 32, 1)
               }
               continue;
             }
-            if (lane == 0) tma_store_wait_read();   // the previous store has left the staging buffer
+            if (elect_one()) tma_store_wait_read();   // the previous store has left the staging buffer
             __syncwarp();
 #pragma unroll
             for (int c = 0; c < 4; c++)
@@ -1186,7 +1188,7 @@ __global__ void __launch_bounds__((GT_PRODUCER_WARPS + 1 + EW + 1) * 32, 1)
                            : "memory");
             fence_proxy_async();
             __syncwarp();
-            if (lane == 0) tma_store_3d(&lin_maps.out[T.l], n0 + cc, T.l * T.l, node_q, stg);
+            if (elect_one()) tma_store_3d(&lin_maps.out[T.l], n0 + cc, T.l * T.l, node_q, stg);
           }
         }
       } else {
@@ -1233,7 +1235,7 @@ __global__ void __launch_bounds__((GT_PRODUCER_WARPS + 1 + EW + 1) * 32, 1)
       acc ^= 1;
     }
     // the copy engine still reads this warp's staging buffer and writes its tile: wait before the CTA retires
-    if (((MODE != GT_MODE_LINEAR && g.ep_tma) || (MODE == GT_MODE_LINEAR && g.lin_tma)) && lane == 0) tma_store_wait_all();
+    if (((MODE != GT_MODE_LINEAR && g.ep_tma) || (MODE == GT_MODE_LINEAR && g.lin_tma)) && elect_one()) tma_store_wait_all();
   }
 
   tc_fence_before();

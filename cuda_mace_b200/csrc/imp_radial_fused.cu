@@ -188,7 +188,7 @@ __global__ void __launch_bounds__(RF_THREADS, 1)
   __shared__ uint32_t tmem_base_slot;
 
   const uint32_t smem_base = (smem_u32(smem) + 1023u) & ~1023u;
-  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+  const int tid = threadIdx.x, warp = uniform(tid >> 5), lane = tid & 31;
   const int group = warp / RF_GROUP_WARPS, gw = warp % RF_GROUP_WARPS, gtid = tid & (RF_GROUP_THREADS - 1);
   const int cq = blockIdx.x % g.nq;                  // channel quarter of this CTA
   const int cta_in_cq = blockIdx.x / g.nq, ctas_per_cq = gridDim.x / g.nq;
@@ -210,7 +210,7 @@ __global__ void __launch_bounds__(RF_THREADS, 1)
   tc_fence_before();
   __syncthreads();
   tc_fence_after();
-  const uint32_t tmem_acc = tmem_base_slot + group * 128;
+  const uint32_t tmem_acc = (uint32_t)uniform((int)tmem_base_slot) + group * 128;
 
   const int64_t ntiles = (g.E + RF_TILE - 1) / RF_TILE;
   const int64_t tile_step = (int64_t)ctas_per_cq * 2;
@@ -220,12 +220,12 @@ __global__ void __launch_bounds__(RF_THREADS, 1)
     mbar_arrive_expect_tx(tma_bar, (uint32_t)k_blocks * RF_SLAB);
     for (int kb = 0; kb < k_blocks; kb++) tma_load_2d(sH + kb * 2 * RF_SLAB, &tmap, kb * 32, (int)(t * RF_TILE), tma_bar);
   };
-  if (tid == 0) {
+  if (warp == 0 && elect_one()) {
     const unsigned char *src = reinterpret_cast<const unsigned char *>(g.packed) + (size_t)cq * w_bytes;
     mbar_arrive_expect_tx(wbar, w_bytes);
     for (uint32_t off = 0; off < w_bytes; off += 8192u) bulk_copy_g2s(sW + off, src + off, 8192u, wbar);
   }
-  if (gtid == 0 && tile < ntiles) start_tile_load(tile);
+  if (gw == 0 && tile < ntiles && elect_one()) start_tile_load(tile);
   bool ok = warp_wait(wbar, 0, lane);
   if (!ok && lane == 0 && g.status) atomicCAS(g.status, 0, 21);
 
@@ -257,7 +257,7 @@ __global__ void __launch_bounds__(RF_THREADS, 1)
     tc_fence_before();
     fence_proxy_async();
     rf_group_sync(group);
-    if (gtid == 0) {
+    if (gw == 0 && elect_one()) {
       tc_fence_after();
       const uint32_t idesc = umma_idesc_tf32(128, RF_TILE);
       for (int k0 = 0, kb = 0; k0 < g.K; k0 += 32, kb++) {
@@ -295,7 +295,7 @@ __global__ void __launch_bounds__(RF_THREADS, 1)
     phase ^= 1;
     tc_fence_after();
     // the H images are free again: fetch the next tile while this one is scattered
-    if (gtid == 0 && tile + tile_step < ntiles) start_tile_load(tile + tile_step);
+    if (gw == 0 && tile + tile_step < ntiles && elect_one()) start_tile_load(tile + tile_step);
     const int col0 = slice * RF_SLICE;
     if (l == 0) rf_consume<0, C>(g, t_row, col0, e0, s_ys, s_ids, ch);
     else if (l == 1) rf_consume<1, C>(g, t_row, col0, e0, s_ys, s_ids, ch);

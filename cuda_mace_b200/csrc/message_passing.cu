@@ -287,7 +287,7 @@ __global__ void __launch_bounds__(BS_WARPS * 32, 1)
       snd = (ic.e + lane < ic.end) ? sender[ic.e + lane] : 0;
     }
     const int s = __shfl_sync(0xffffffffu, snd, (int)(ic.e - chunk_base));
-    if (lane == 0) {
+    if (elect_one()) {
       const uint32_t slot = ring + (icount % BS_SLOTS) * BS_SLOT_BYTES, bar = bar0 + 8 * (icount % BS_SLOTS);
       asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(bar), "r"(BS_SLOT_BYTES) : "memory");
       asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::"r"(slot),

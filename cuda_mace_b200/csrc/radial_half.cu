@@ -56,7 +56,7 @@ __global__ void __launch_bounds__(RQ_THREADS, 1)
   __shared__ uint32_t tmem_base_slot;
 
   const uint32_t smem_base = (smem_u32(smem) + 1023u) & ~1023u;
-  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+  const int tid = threadIdx.x, warp = uniform(tid >> 5), lane = tid & 31;
   const int group = warp >> 3, gw = warp & 7, gtid = tid & (RQ_GROUP_THREADS - 1);
   const bool second = (blockIdx.x % (unsigned)g.nper) != 0;
   const uint32_t wbar = smem_u32(&bars[0]);
@@ -71,9 +71,9 @@ __global__ void __launch_bounds__(RQ_THREADS, 1)
   tc_fence_before();
   __syncthreads();
   tc_fence_after();
-  const uint32_t tmem0 = tmem_base_slot + (uint32_t)group * 256u;   // operand o: + 128 o; hi at + 64, lo at + 96
+  const uint32_t tmem0 = (uint32_t)uniform((int)tmem_base_slot) + (uint32_t)group * 256u;   // operand o: + 128 o; hi at + 64, lo at + 96
 
-  if (tid == 0) {
+  if (warp == 0 && elect_one()) {
     mbar_arrive_expect_tx(wbar, 6u * RQ_IMAGE);
 #pragma unroll
     for (int i = 0; i < 3; i++) {
@@ -123,7 +123,7 @@ __global__ void __launch_bounds__(RQ_THREADS, 1)
     tmem_st_wait();
     tc_fence_before();
     group_sync();
-    if (gtid == 0) {
+    if (gw == 0 && elect_one()) {
       tc_fence_after();
       issue(o, layer);
     }
@@ -167,7 +167,7 @@ __global__ void __launch_bounds__(RQ_THREADS, 1)
     tc_fence_before();
     fence_proxy_async();
     group_sync();
-    if (gtid == 0) {   // rows past the end of the array are clipped
+    if (gw == 0 && elect_one()) {   // rows past the end of the array are clipped
       const uint32_t sT = sOut + (uint32_t)o * RQ_OUT;
       const CUtensorMap *map = o == 0 ? (second ? &maps.h[1] : &maps.h[0]) : (second ? &maps.dh[1] : &maps.dh[0]);
       tma_store_2d(map, 0, (int)(tile * RQ_TILE), sT);
@@ -191,9 +191,9 @@ __global__ void __launch_bounds__(RQ_THREADS, 1)
       tmem_st8(t + 96u, lo);
       tmem_st_wait();
       tc_fence_before();
-      if (tile != first && gtid == 0) tma_store_wait_read();   // the staging buffers are written again at layer 3
+      if (tile != first && gw == 0 && elect_one()) tma_store_wait_read();   // the staging buffers are written again at layer 3
       group_sync();
-      if (gtid == 0) {
+      if (gw == 0 && elect_one()) {
         tc_fence_after();
         issue(0, 0);
         issue(1, 0);
@@ -257,7 +257,7 @@ __global__ void __launch_bounds__(RQ_THREADS, 1)
       phase ^= 1;
     }
   }
-  if (gtid == 0) tma_store_wait_all();
+  if (gw == 0 && elect_one()) tma_store_wait_all();
   tc_fence_before();
   __syncthreads();
   if (warp == 0) tmem_dealloc(tmem_base_slot, 512);

@@ -143,7 +143,7 @@ __global__ void __launch_bounds__(RH_THREADS, 1)
   __shared__ uint32_t tmem_base_slot;
 
   const uint32_t smem_base = (smem_u32(smem) + 1023u) & ~1023u;
-  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+  const int tid = threadIdx.x, warp = uniform(tid >> 5), lane = tid & 31;
   const int group = warp >> 3;
   const uint32_t wbar = smem_u32(&bars[0]);
   const uint32_t done0 = wbar + 8u * (1 + 2 * group);   // + 8 * slot
@@ -160,9 +160,9 @@ __global__ void __launch_bounds__(RH_THREADS, 1)
   tc_fence_before();
   __syncthreads();
   tc_fence_after();
-  const uint32_t tmem0 = tmem_base_slot + (uint32_t)(2 * group) * RF_TMEM_SLOT;   // + slot * RF_TMEM_SLOT; residual at + 64
+  const uint32_t tmem0 = (uint32_t)uniform((int)tmem_base_slot) + (uint32_t)(2 * group) * RF_TMEM_SLOT;   // + slot * RF_TMEM_SLOT; residual at + 64
 
-  if (tid == 0) {
+  if (warp == 0 && elect_one()) {
     mbar_arrive_expect_tx(wbar, w_bytes[0] + w_bytes[1] + w_bytes[2]);
     for (int i = 0; i < 3; i++)
       for (uint32_t off = 0; off < w_bytes[i]; off += 8192u) {
@@ -207,7 +207,7 @@ __global__ void __launch_bounds__(RH_THREADS, 1)
     auto hand_over = [&](int s, int layer) {
       fence_proxy_async();
       group_sync(group);
-      if (gtid == 0) {
+      if (gw == 0 && elect_one()) {
         tc_fence_after();
         const uint32_t acc0 = tmem0 + (uint32_t)s * RF_TMEM_SLOT;
         issue_tile_layer(acc0, acc0 + 64u, sA0 + (uint32_t)s * RF_SLOT_BYTES, sW[layer], layer == 0, g.nb, RH_H);
@@ -219,7 +219,7 @@ __global__ void __launch_bounds__(RH_THREADS, 1)
       const int nslots = t0 + step < ntiles ? 2 : 1;
       if (t0 != first) {
         // the tile stores of the previous pass read the buffers that are written next
-        if (gtid == 0) tma_store_wait_read();
+        if (gw == 0 && elect_one()) tma_store_wait_read();
         group_sync(group);
       }
       // ---- first layer's operand: the basis rows, raw image in slab 0, residual image in slab 1
@@ -295,7 +295,7 @@ __global__ void __launch_bounds__(RH_THREADS, 1)
                 // h3 [128, 64] of the tile: two 32-column boxes, rows past the end of the array are clipped
                 fence_proxy_async();
                 group_sync(group);
-                if (gtid == 0) {
+                if (gw == 0 && elect_one()) {
                   const uint32_t sT = sA0 + (uint32_t)s * RF_SLOT_BYTES;
                   tma_store_2d(&out_map, 0, (int)(tile * RH_TILE), sT);
                   tma_store_2d(&out_map, 32, (int)(tile * RH_TILE), sT + RH_A_SLAB);
@@ -307,7 +307,7 @@ __global__ void __launch_bounds__(RH_THREADS, 1)
         phase ^= 1;
       }
     }
-    if (gtid == 0) tma_store_wait_all();
+    if (gw == 0 && elect_one()) tma_store_wait_all();
   }
 
   tc_fence_before();
@@ -335,7 +335,7 @@ __global__ void __launch_bounds__(RH_THREADS, 1)
   __shared__ uint32_t tmem_base_slot;
 
   const uint32_t smem_base = (smem_u32(smem) + 1023u) & ~1023u;
-  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+  const int tid = threadIdx.x, warp = uniform(tid >> 5), lane = tid & 31;
   const int group = warp >> 3, gw = warp & 7, gtid = tid & (RH_GROUP_THREADS - 1);
   const uint32_t wbar = smem_u32(&bars[0]);
   const uint32_t done0 = wbar + 8u * (1 + 2 * group);   // + 8 * slot
@@ -354,9 +354,9 @@ __global__ void __launch_bounds__(RH_THREADS, 1)
   tc_fence_before();
   __syncthreads();
   tc_fence_after();
-  const uint32_t tmem0 = tmem_base_slot + (uint32_t)(2 * group) * RF_TMEM_SLOT;
+  const uint32_t tmem0 = (uint32_t)uniform((int)tmem_base_slot) + (uint32_t)(2 * group) * RF_TMEM_SLOT;
 
-  if (tid == 0) {
+  if (warp == 0 && elect_one()) {
     mbar_arrive_expect_tx(wbar, w_bytes[0] + w_bytes[1] + w_bytes[2]);
     for (int i = 0; i < 3; i++)
       for (uint32_t off = 0; off < w_bytes[i]; off += 8192u) {
@@ -396,7 +396,7 @@ __global__ void __launch_bounds__(RH_THREADS, 1)
     tc_fence_before();
     fence_proxy_async();
     group_sync(group);
-    if (gtid == 0) {
+    if (gw == 0 && elect_one()) {
       tc_fence_after();
       const uint32_t acc = tmem0 + (uint32_t)s * RF_TMEM_SLOT;
       issue_tile_layer(acc, acc + 64u, sA0 + (uint32_t)s * RF_SLOT_BYTES, sW[layer], false, 0,
@@ -422,7 +422,7 @@ __global__ void __launch_bounds__(RH_THREADS, 1)
     tmem_st16(tmem0 + (uint32_t)s * RF_TMEM_SLOT + lane_field + 64u + 32u * h + 16u * hh, lo);
   };
 
-  if (gtid == 0) {
+  if (gw == 0 && elect_one()) {
     request_g(0, first);
     request_g(1, first + step);
   }
@@ -508,7 +508,7 @@ __global__ void __launch_bounds__(RH_THREADS, 1)
           ok = false;
         } else {
           tc_fence_after();
-          if (gtid == 0) request_g(s, tile + 2 * step);
+          if (gw == 0 && elect_one()) request_g(s, tile + 2 * step);
           const int64_t e = tile * RH_TILE + r;
           if (h == 0) {
             const uint32_t t_row = tmem0 + (uint32_t)s * RF_TMEM_SLOT + lane_field;

@@ -107,7 +107,7 @@ __global__ void __launch_bounds__(RT_THREADS, 1)
   __shared__ uint32_t tmem_base_slot;
 
   const uint32_t smem_base = (smem_u32(smem) + 1023u) & ~1023u;
-  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+  const int tid = threadIdx.x, warp = uniform(tid >> 5), lane = tid & 31;
   const int group = warp >> 3, gw = warp & 7, gtid = tid & (RT_GROUP_THREADS - 1);
   const int per = (int)(blockIdx.x % (unsigned)g.nper);
   const uint32_t wbar = smem_u32(&bars[0]);
@@ -125,9 +125,9 @@ __global__ void __launch_bounds__(RT_THREADS, 1)
   tc_fence_before();
   __syncthreads();
   tc_fence_after();
-  const uint32_t tmem0 = tmem_base_slot + (uint32_t)(2 * group) * RT_TMEM_OP;   // + operand * RT_TMEM_OP
+  const uint32_t tmem0 = (uint32_t)uniform((int)tmem_base_slot) + (uint32_t)(2 * group) * RT_TMEM_OP;   // + operand * RT_TMEM_OP
 
-  if (tid == 0) {
+  if (warp == 0 && elect_one()) {
     mbar_arrive_expect_tx(wbar, w_bytes[0] + w_bytes[1] + w_bytes[2]);
 #pragma unroll
     for (int i = 0; i < 3; i++)
@@ -162,7 +162,7 @@ __global__ void __launch_bounds__(RT_THREADS, 1)
   auto hand_over = [&](int o, int layer) {
     fence_proxy_async();
     group_sync();
-    if (gtid == 0) {
+    if (gw == 0 && elect_one()) {
       tc_fence_after();
       rt_issue(tmem0 + (uint32_t)o * RT_TMEM_OP, sA0 + (uint32_t)o * RT_BUF, layer == 1 ? sW[1] : sW[2], false, g.nb);
       umma_commit(done0 + 8u * o);
@@ -195,7 +195,7 @@ __global__ void __launch_bounds__(RT_THREADS, 1)
       tc_fence_before();
       fence_proxy_async();
       group_sync();
-      if (gtid == 0) {
+      if (gw == 0 && elect_one()) {
         const uint32_t sT = sA0 + (uint32_t)o * RT_BUF;
         const CUtensorMap *map = o == 0 ? (per ? &maps.h[1] : &maps.h[0]) : (per ? &maps.dh[1] : &maps.dh[0]);
         tma_store_2d(map, 0, (int)(tile * RT_TILE), sT);
@@ -207,7 +207,7 @@ __global__ void __launch_bounds__(RT_THREADS, 1)
   load_basis(first);
   for (int64_t tile = first; ok && tile < ntiles; tile += step) {
     if (tile != first) {
-      if (gtid == 0) tma_store_wait_read();   // the previous tile's stores read the buffers that are written next
+      if (gw == 0 && elect_one()) tma_store_wait_read();   // the previous tile's stores read the buffers that are written next
       group_sync();
     }
 #pragma unroll
@@ -220,7 +220,7 @@ __global__ void __launch_bounds__(RT_THREADS, 1)
     tc_fence_before();
     fence_proxy_async();
     group_sync();
-    if (gtid == 0) {
+    if (gw == 0 && elect_one()) {
       tc_fence_after();
 #pragma unroll
       for (int o = 0; o < 2; o++) {
@@ -270,7 +270,7 @@ __global__ void __launch_bounds__(RT_THREADS, 1)
       phase ^= 1;
     }
   }
-  if (gtid == 0) tma_store_wait_all();
+  if (gw == 0 && elect_one()) tma_store_wait_all();
   tc_fence_before();
   __syncthreads();
   if (warp == 0) tmem_dealloc(tmem_base_slot, 512);
@@ -298,7 +298,7 @@ struct RadialPairArgs64 {
 
 __global__ void __launch_bounds__(RD_WARPS * 32, 1) radial_pair_f64_kernel(const RadialPairArgs64 g) {
   extern __shared__ __align__(16) double rd_smem[];
-  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+  const int tid = threadIdx.x, warp = uniform(tid >> 5), lane = tid & 31;
   const int per = (int)(blockIdx.x % (unsigned)g.nper);
   double *const sW1 = rd_smem, *const sW2 = sW1 + 16 * RD_LD, *const sW3 = sW2 + 64 * RD_LD;
   double *const act = sW3 + 64 * RD_LD + warp * (16 * RD_LD);   // 8 rows of values, 8 of derivatives
