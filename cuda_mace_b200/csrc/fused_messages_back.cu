@@ -9,12 +9,14 @@
 // every sum above runs over that thread's own values, no shuffles.  (With channels on the lanes, as in the forward, the
 // sums over channels cost 31 shuffles per four edges and warp, and the kernel took 5.0 ms at 64 000 atoms.)
 //
-// Tile = 128 edges, taken 16 channels at a time: one accumulator buffer of 64 (R, four l) + 64 (R') columns, two buffers,
-// one per set of four consumer warps.  A operand: h and h' (hi, lo fp16), 128 columns of tensor memory, two buffers; the
-// consumers bring the next tile's rows over in quarters, one per 16 channels.  B operand: 16 KB of W per 16 channels,
-// streamed from L2 (every CTA reads the same 128 KB).  With A in tensor memory a narrow MMA is not bound by reading it.
+// Tile = 128 edges, taken 16 channels at a time by two sets of four consumer warps in turn, in steps of 8 channels: an
+// accumulator buffer holds 32 (R, four l) + 32 (R') columns, two buffers a set, so that the products of a set's next step
+// run while it works (with one buffer of 16 channels a set it waited for them: 2.35 against 2.13 ms at 64 000 atoms).
+// A operand: h and h' (hi, lo fp16), 128 columns of tensor memory, two buffers; the consumers bring the next tile's rows
+// over in quarters, one per 16 channels.  B operand: 8 KB of W per step, streamed from L2 (every CTA reads the same
+// 128 KB).  With A in tensor memory a narrow MMA runs at its own rate (16 cycles at N = 32).
 //
-//   warps 0-3, 4-7  consumers of even / odd 16-channel blocks; warp w reaches the rows 32 (w % 4) .. of the tile
+//   warps 0-3, 4-7  the two sets of consumers; warp w reaches the rows 32 (w % 4) .. of the tile
 //   warp 8          issues the MMAs
 //   warp 9          W blocks and the G rows of the next tile's receivers (contiguous: the list is sorted), bulk copies
 //   warp 10         sender rows X, 64 bytes of 128 rows per block, asynchronous copies
@@ -32,8 +34,10 @@ constexpr int EB_C = 128;
 constexpr int EB_BLK = 16;                        // channels of a block
 constexpr int EB_NBLK = EB_C / EB_BLK;
 constexpr int EB_THREADS = 384;
-constexpr int EB_W_BYTES = 2 * 64 * 128;          // hi and lo image of a block of W: 64 rows (l, channel)
-constexpr int EB_W_SLOTS = 3;
+constexpr int EB_STEP = 8;                        // channels of a step
+constexpr int EB_NSTEP = EB_C / EB_STEP;
+constexpr int EB_W_BYTES = 2 * 32 * 128;          // hi and lo image of a step's W: 32 rows (l, channel)
+constexpr int EB_W_SLOTS = 6;
 constexpr int EB_X_BYTES = EB_TILE * EB_BLK * 4;
 constexpr int EB_X_SLOTS = 5;
 constexpr int EB_G_RECV = 5;                      // receivers staged per tile; further ones are read from global memory
@@ -51,7 +55,7 @@ constexpr int EB_SMEM = EB_OFF_P + 2 * EB_PART * 4 + 1024;
 struct EdgeBackArgs {
   const float *X, *Y, *G;        // [Ns, 128], [E, 16], [nnodes, 16, 128]
   const char *h, *dh;            // [E][hi 64 | lo 64] fp16
-  const char *W;                 // [8 blocks][hi, lo][64 rows x 128 B, swizzled]
+  const char *W;                 // [16 steps][hi, lo][32 rows x 128 B, swizzled]
   const int32_t *sender, *receiver;
   int32_t *status;
   int64_t nedges;
@@ -86,13 +90,13 @@ __device__ __forceinline__ void eb_half(uint32_t ta, uint32_t gs, const float *g
   unsigned long long v2[4];
   uint32_t r[2][8], d[2][8];
   eb_ld8(ta, r[0]);
-  eb_ld8(ta + 64u, d[0]);
+  eb_ld8(ta + 32u, d[0]);
 #pragma unroll
   for (int l = 0; l < 4; l++) {
     eb_ld_wait(r[l & 1], d[l & 1]);
     if (l < 3) {   // the next degree's accumulators are on their way meanwhile
-      eb_ld8(ta + 16u * (l + 1), r[(l + 1) & 1]);
-      eb_ld8(ta + 64u + 16u * (l + 1), d[(l + 1) & 1]);
+      eb_ld8(ta + 8u * (l + 1), r[(l + 1) & 1]);
+      eb_ld8(ta + 32u + 8u * (l + 1), d[(l + 1) & 1]);
     }
     unsigned long long u2[4], p2[4], r2[4];
 #pragma unroll
@@ -133,7 +137,7 @@ __device__ __forceinline__ void eb_half(uint32_t ta, uint32_t gs, const float *g
 __global__ void __launch_bounds__(EB_THREADS, 1)
     edge_back_kernel(const EdgeBackArgs g, const __grid_constant__ CUtensorMap t_map) {
   extern __shared__ __align__(1024) unsigned char smem[];
-  __shared__ __align__(8) uint64_t bars[2 * EB_W_SLOTS + 2 * EB_X_SLOTS + 10];
+  __shared__ __align__(8) uint64_t bars[2 * EB_W_SLOTS + 2 * EB_X_SLOTS + 14];
   __shared__ uint32_t tmem_base_slot;
 
   const uint32_t base_s = (smem_u32(smem) + 1023u) & ~1023u;
@@ -141,7 +145,7 @@ __global__ void __launch_bounds__(EB_THREADS, 1)
   const uint32_t w_full = smem_u32(&bars[0]), w_free = w_full + 8u * EB_W_SLOTS;
   const uint32_t x_full = w_free + 8u * EB_W_SLOTS, x_free = x_full + 8u * EB_X_SLOTS;
   const uint32_t g_full = x_free + 8u * EB_X_SLOTS, g_free = g_full + 16u, h_full = g_free + 16u;
-  const uint32_t acc_full = h_full + 16u, acc_free = acc_full + 16u;
+  const uint32_t acc_full = h_full + 16u, acc_free = acc_full + 32u;
 
   if (tid == 0) {
     for (int s = 0; s < EB_W_SLOTS; s++) {
@@ -156,6 +160,8 @@ __global__ void __launch_bounds__(EB_THREADS, 1)
       mbar_init(g_full + 8u * b, 1);
       mbar_init(g_free + 8u * b, 8);
       mbar_init(h_full + 8u * b, 8);
+    }
+    for (int b = 0; b < 4; b++) {
       mbar_init(acc_full + 8u * b, 1);
       mbar_init(acc_free + 8u * b, 4);
     }
@@ -165,7 +171,7 @@ __global__ void __launch_bounds__(EB_THREADS, 1)
   tc_fence_before();
   __syncthreads();
   tc_fence_after();
-  const uint32_t tmem = (uint32_t)uniform((int)tmem_base_slot);   // h buffer b at 128 b: h hi, h lo, h' hi, h' lo (32 each); acc b at 256 + 128 b
+  const uint32_t tmem = (uint32_t)uniform((int)tmem_base_slot);   // h buffer b at 128 b: h hi, h lo, h' hi, h' lo (32 each); acc b at 256 + 64 b
   const int64_t ntiles = (g.nedges + EB_TILE - 1) / EB_TILE;
 
   if (warp < 8) {
@@ -200,8 +206,10 @@ __global__ void __launch_bounds__(EB_THREADS, 1)
                      : "r"(sH + (uint32_t)sw64_offset(lane, c))
                      : "memory");
       tmem_st16(tmem + lanes + 128u * (uint32_t)buf + 64u * (uint32_t)set + 16u * (uint32_t)piece, v);
-      tmem_st_wait();
-      tc_fence_before();
+      if (piece == 3) {
+        tmem_st_wait();
+        tc_fence_before();
+      }
       __syncwarp();
     };
 
@@ -244,26 +252,34 @@ __global__ void __launch_bounds__(EB_THREADS, 1)
 #pragma unroll 1
       for (int j = 0; ok && j < EB_NBLK / 2; j++) {
         const int blk = 2 * j + set;
-        if (more) h_start(tile + gridDim.x, j);
-        const uint32_t use = 4u * k + (uint32_t)j;   // uses of this set's accumulator buffer
-        if (!warp_wait(x_full + 8u * xs, xphase, lane) || !warp_wait(acc_full + 8u * set, use & 1u, lane)) {
-          if (lane == 0 && g.status) atomicCAS(g.status, 0, 62);
-          ok = false;
-          break;
+        if (more) {
+          h_start(tile + gridDim.x, j);
+          if (j == 0) {   // what the next tile starts with
+            const int64_t en = e + (int64_t)gridDim.x * EB_TILE < g.nedges ? e + (int64_t)gridDim.x * EB_TILE : g.nedges - 1;
+            asm volatile("prefetch.global.L2 [%0];" ::"l"(g.Y + en * 16));
+            if (lane == 0) asm volatile("prefetch.global.L2 [%0];" ::"l"(g.receiver + en));
+          }
         }
-        tc_fence_after();
+        const uint32_t use = 4u * k + (uint32_t)j;   // uses of each of this set's accumulator buffers
+        if (!(ok = warp_wait(x_full + 8u * xs, xphase, lane))) break;
         if (elect_one()) tma_store_wait_read();   // the previous block's T has left the piece
         __syncwarp();
         const uint32_t sX = base_s + EB_OFF_X + (uint32_t)xs * EB_X_BYTES;
 #pragma unroll 1
         for (int hf = 0; hf < 2; hf++) {
+          const uint32_t buf = 2u * (uint32_t)set + (uint32_t)hf;
+          if (!(ok = warp_wait(acc_full + 8u * buf, use & 1u, lane))) break;
+          tc_fence_after();
           unsigned long long x2[4], t2[4];
           eb_lds(sX + (uint32_t)sw64_offset(row, 2 * hf), x2[0], x2[1]);
           eb_lds(sX + (uint32_t)sw64_offset(row, 2 * hf + 1), x2[2], x2[3]);
-          const uint32_t ta = tmem + lanes + 256u + 128u * (uint32_t)set + 8u * (uint32_t)hf;
+          const uint32_t ta = tmem + lanes + 256u + 64u * buf;
           const uint32_t coff = (uint32_t)(EB_BLK * blk + 8 * hf);
           if (staged) eb_half<true>(ta, gs + 4u * coff, gg, x2, y, gy2, dr2, t2);
           else eb_half<false>(ta, gs, gg + coff, x2, y, gy2, dr2, t2);
+          tc_fence_before();
+          __syncwarp();
+          if (lane == 0) mbar_arrive(acc_free + 8u * buf);
           const unsigned long long f2 = pack2(g.factor_v, g.factor_v);
 #pragma unroll
           for (int c = 0; c < 2; c++)
@@ -271,11 +287,10 @@ __global__ void __launch_bounds__(EB_THREADS, 1)
                          "l"(mul2(t2[2 * c], f2)), "l"(mul2(t2[2 * c + 1], f2))
                          : "memory");
         }
-        tc_fence_before();
+        if (!ok) break;
         fence_proxy_async();
         __syncwarp();
         if (elect_one()) {
-          mbar_arrive(acc_free + 8u * set);
           mbar_arrive(x_free + 8u * xs);
           if (base + 32 * q < g.nedges) tma_store_2d(&t_map, EB_BLK * blk, (int)base + 32 * q, sT);
         }
@@ -289,6 +304,7 @@ __global__ void __launch_bounds__(EB_THREADS, 1)
           if (j == 3 && lane == 0) mbar_arrive(h_full + 8u * ((k + 1) & 1u));
         }
       }
+      if (!ok && lane == 0 && g.status) atomicCAS(g.status, 0, 62);
       __syncwarp();
       if (lane == 0) mbar_arrive(g_free + 8u * (k & 1u));
       // the two sets' sums of an edge: odd blocks' through shared memory (two buffers, one barrier a tile and quarter)
@@ -319,29 +335,29 @@ __global__ void __launch_bounds__(EB_THREADS, 1)
     if (elect_one()) tma_store_wait_all();
   } else if (warp == 8) {
     // ---- MMA issuer
-    const uint32_t idesc = umma_idesc_f16(128, 64);
+    const uint32_t idesc = umma_idesc_f16(128, 32);
     int slot = 0;
     uint32_t wphase = 0, k = 0;
     bool ok = true;
     for (int64_t tile = blockIdx.x; ok && tile < ntiles; tile += gridDim.x, k++) {
       ok = warp_wait(h_full + 8u * (k & 1u), (k >> 1) & 1u, lane);
-      for (int blk = 0; ok && blk < EB_NBLK; blk++) {
-        const uint32_t b = (uint32_t)blk & 1u, use = 4u * k + (uint32_t)(blk >> 1);
+      for (int n = 0; ok && n < EB_NSTEP; n++) {
+        const uint32_t b = (uint32_t)n & 3u, use = 4u * k + (uint32_t)(n >> 2);   // buffers 0, 1 are set 0's, 2, 3 set 1's
         ok = warp_wait(acc_free + 8u * b, (use & 1u) ^ 1u, lane) && warp_wait(w_full + 8u * slot, wphase, lane);
         if (!ok) break;
         if (elect_one()) {
           tc_fence_after();
           const uint32_t sW = base_s + EB_OFF_W + (uint32_t)slot * EB_W_BYTES;
           const uint64_t b_hi = umma_desc_sw128(sW), b_lo = umma_desc_sw128(sW + EB_W_BYTES / 2);
-#pragma unroll 1
-          for (int o = 0; o < 2; o++) {   // R, R'
-            const uint32_t d = tmem + 256u + 128u * b + 64u * o, a = tmem + 128u * (k & 1u) + 64u * o;
+          const uint32_t d = tmem + 256u + 64u * b, a = tmem + 128u * (k & 1u);
 #pragma unroll
-            for (int j = 0; j < 4; j++) {
-              umma_f16_ts(d, a + 8u * j, b_hi + (uint64_t)(2 * j), idesc, j != 0);
-              umma_f16_ts(d, a + 8u * j, b_lo + (uint64_t)(2 * j), idesc, 1);
-              umma_f16_ts(d, a + 32u + 8u * j, b_hi + (uint64_t)(2 * j), idesc, 1);
-            }
+          for (int j = 0; j < 4; j++) {   // R and R'
+            umma_f16_ts(d, a + 8u * j, b_hi + (uint64_t)(2 * j), idesc, j != 0);
+            umma_f16_ts(d + 32u, a + 64u + 8u * j, b_hi + (uint64_t)(2 * j), idesc, j != 0);
+            umma_f16_ts(d, a + 8u * j, b_lo + (uint64_t)(2 * j), idesc, 1);
+            umma_f16_ts(d + 32u, a + 64u + 8u * j, b_lo + (uint64_t)(2 * j), idesc, 1);
+            umma_f16_ts(d, a + 32u + 8u * j, b_hi + (uint64_t)(2 * j), idesc, 1);
+            umma_f16_ts(d + 32u, a + 96u + 8u * j, b_hi + (uint64_t)(2 * j), idesc, 1);
           }
           umma_commit(w_free + 8u * slot);
           umma_commit(acc_full + 8u * b);
@@ -374,18 +390,18 @@ __global__ void __launch_bounds__(EB_THREADS, 1)
       };
       if (blockIdx.x < ntiles) ok = load_g(blockIdx.x, 0);
       for (int64_t tile = blockIdx.x; ok && tile < ntiles; tile += gridDim.x, k++)
-        for (int blk = 0; ok && blk < EB_NBLK; blk++) {
+        for (int n = 0; ok && n < EB_NSTEP; n++) {
           ok = mbar_wait(w_free + 8u * slot, wphase ^ 1);
           if (!ok) break;
           mbar_arrive_expect_tx(w_full + 8u * slot, EB_W_BYTES);
-          bulk_copy_g2s(base_s + EB_OFF_W + (uint32_t)slot * EB_W_BYTES, g.W + (int64_t)blk * EB_W_BYTES, EB_W_BYTES,
+          bulk_copy_g2s(base_s + EB_OFF_W + (uint32_t)slot * EB_W_BYTES, g.W + (int64_t)n * EB_W_BYTES, EB_W_BYTES,
                         w_full + 8u * slot);
           if (++slot == EB_W_SLOTS) {
             slot = 0;
             wphase ^= 1;
           }
-          // the buffer was last read by the tile before this one, which the consumers have left by block 4
-          if (blk == 4 && tile + gridDim.x < ntiles) ok = load_g(tile + gridDim.x, k + 1);
+          // the buffer was last read by the tile before this one, which the consumers have left by step 8
+          if (n == 8 && tile + gridDim.x < ntiles) ok = load_g(tile + gridDim.x, k + 1);
         }
       if (!ok && g.status) atomicCAS(g.status, 0, 64);
     }

@@ -155,7 +155,7 @@ class StepPlan:
                     hi = w.half()
                     m.fused_w = hold(torch.cat([hi, (w - hi.float()).half()], dim=1))
                     m.fused_scale = 1.0 / scale
-                    wt = L1.W_radial3.t().reshape(4, 8, 16, _H).transpose(0, 1).reshape(8, 64, _H)   # [block, (l, c), k]
+                    wt = L1.W_radial3.t().reshape(4, 16, 8, _H).transpose(0, 1).reshape(16, 32, _H)   # [step, (l, c), k]
                     m.fused_w_back = hold(torch.stack([half_images(b, scale) for b in wt]))
         m.radial_back = matrix(L1.W_radial3.t())
         x = d(model.embedding) @ d(L0.W_up)                                  # [Z, C] sender features of the first layer
