@@ -13,7 +13,7 @@
 // accumulator buffer holds 32 (R, four l) + 32 (R') columns, two buffers a set, so that the products of a set's next step
 // run while it works (with one buffer of 16 channels a set it waited for them: 2.35 against 2.13 ms at 64 000 atoms).
 // A operand: h and h' (hi, lo fp16), 128 columns of tensor memory, two buffers; the consumers bring the next tile's rows
-// over in quarters, one per 16 channels.  B operand: 8 KB of W per step, streamed from L2 (every CTA reads the same
+// over in quarters during a tile's first four steps.  B operand: 8 KB of W per step, streamed from L2 (every CTA reads the same
 // 128 KB).  With A in tensor memory a narrow MMA runs at its own rate (16 cycles at N = 32).
 //
 //   warps 0-3, 4-7  the two sets of consumers; warp w reaches the rows 32 (w % 4) .. of the tile
@@ -54,7 +54,7 @@ constexpr int EB_SMEM = EB_OFF_P + 2 * EB_PART * 4 + 1024;
 
 struct EdgeBackArgs {
   const float *X, *Y, *G;        // [Ns, 128], [E, 16], [nnodes, 16, 128]
-  const char *h, *dh;            // [E][hi 64 | lo 64] fp16
+  const char *h, *dh;            // [E rounded up to a tile][hi 64 | lo 64] fp16
   const char *W;                 // [16 steps][hi, lo][32 rows x 128 B, swizzled]
   const int32_t *sender, *receiver;
   int32_t *status;
@@ -137,7 +137,7 @@ __device__ __forceinline__ void eb_half(uint32_t ta, uint32_t gs, const float *g
 __global__ void __launch_bounds__(EB_THREADS, 1)
     edge_back_kernel(const EdgeBackArgs g, const __grid_constant__ CUtensorMap t_map) {
   extern __shared__ __align__(1024) unsigned char smem[];
-  __shared__ __align__(8) uint64_t bars[2 * EB_W_SLOTS + 2 * EB_X_SLOTS + 14];
+  __shared__ __align__(8) uint64_t bars[2 * EB_W_SLOTS + 2 * EB_X_SLOTS + 18];
   __shared__ uint32_t tmem_base_slot;
 
   const uint32_t base_s = (smem_u32(smem) + 1023u) & ~1023u;
@@ -145,7 +145,7 @@ __global__ void __launch_bounds__(EB_THREADS, 1)
   const uint32_t w_full = smem_u32(&bars[0]), w_free = w_full + 8u * EB_W_SLOTS;
   const uint32_t x_full = w_free + 8u * EB_W_SLOTS, x_free = x_full + 8u * EB_X_SLOTS;
   const uint32_t g_full = x_free + 8u * EB_X_SLOTS, g_free = g_full + 16u, h_full = g_free + 16u;
-  const uint32_t acc_full = h_full + 16u, acc_free = acc_full + 32u;
+  const uint32_t acc_full = h_full + 16u, acc_free = acc_full + 32u, part_full = acc_free + 32u;
 
   if (tid == 0) {
     for (int s = 0; s < EB_W_SLOTS; s++) {
@@ -164,6 +164,7 @@ __global__ void __launch_bounds__(EB_THREADS, 1)
     for (int b = 0; b < 4; b++) {
       mbar_init(acc_full + 8u * b, 1);
       mbar_init(acc_free + 8u * b, 4);
+      mbar_init(part_full + 8u * b, 1);
     }
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
   }
@@ -181,18 +182,15 @@ __global__ void __launch_bounds__(EB_THREADS, 1)
     const uint32_t lanes = (uint32_t)(32 * q) << 16;
     const uint32_t sT = base_s + EB_OFF_T + (uint32_t)warp * EB_PIECE, sH = base_s + EB_OFF_H + (uint32_t)warp * EB_PIECE;
     float *part0 = reinterpret_cast<float *>(smem + (base_s - smem_u32(smem)) + EB_OFF_P) + row * 17;
-    const char *hsrc = set == 0 ? g.h : g.dh;
+    const char *hlane = (set == 0 ? g.h : g.dh) + (32 * q + (lane >> 2)) * 256 + 16 * (lane & 3);
+    const uint32_t hdst = sH + (uint32_t)sw64_offset(lane >> 2, lane & 3);
     bool ok = true;
 
     // 64 bytes (32 k of hi or lo) of this warp's 32 rows of a tile: started here, finished by h_put
     auto h_start = [&](int64_t tile, int piece) {
+      const char *src = hlane + tile * (EB_TILE * 256) + 64 * piece;
 #pragma unroll
-      for (int i = 0; i < 4; i++) {
-        const int r = 8 * i + (lane >> 2);
-        int64_t e = tile * EB_TILE + 32 * q + r;
-        e = e < g.nedges ? e : g.nedges - 1;
-        eb_cp16(sH + (uint32_t)sw64_offset(r, lane & 3), hsrc + e * 256 + 64 * piece + 16 * (lane & 3));
-      }
+      for (int i = 0; i < 4; i++) eb_cp16(hdst + 512u * i, src + 8 * 256 * i);   // sw64_offset(r + 8, c) = sw64_offset(r, c) + 512
       asm volatile("cp.async.commit_group;" ::: "memory");
     };
     auto h_put = [&](int buf, int piece) {
@@ -252,22 +250,19 @@ __global__ void __launch_bounds__(EB_THREADS, 1)
 #pragma unroll 1
       for (int j = 0; ok && j < EB_NBLK / 2; j++) {
         const int blk = 2 * j + set;
-        if (more) {
-          h_start(tile + gridDim.x, j);
-          if (j == 0) {   // what the next tile starts with
-            const int64_t en = e + (int64_t)gridDim.x * EB_TILE < g.nedges ? e + (int64_t)gridDim.x * EB_TILE : g.nedges - 1;
-            asm volatile("prefetch.global.L2 [%0];" ::"l"(g.Y + en * 16));
-            if (lane == 0) asm volatile("prefetch.global.L2 [%0];" ::"l"(g.receiver + en));
-          }
+        if (more && j == 2) {   // what the next tile starts with
+          const int64_t en = e + (int64_t)gridDim.x * EB_TILE < g.nedges ? e + (int64_t)gridDim.x * EB_TILE : g.nedges - 1;
+          asm volatile("prefetch.global.L2 [%0];" ::"l"(g.Y + en * 16));
+          if (lane == 0) asm volatile("prefetch.global.L2 [%0];" ::"l"(g.receiver + en));
         }
         const uint32_t use = 4u * k + (uint32_t)j;   // uses of each of this set's accumulator buffers
         if (!(ok = warp_wait(x_full + 8u * xs, xphase, lane))) break;
-        if (elect_one()) tma_store_wait_read();   // the previous block's T has left the piece
-        __syncwarp();
         const uint32_t sX = base_s + EB_OFF_X + (uint32_t)xs * EB_X_BYTES;
 #pragma unroll 1
         for (int hf = 0; hf < 2; hf++) {
           const uint32_t buf = 2u * (uint32_t)set + (uint32_t)hf;
+          const int piece = 2 * j + hf;            // of the next tile's h, in this tile's first four steps
+          if (more && piece < 4) h_start(tile + gridDim.x, piece);
           if (!(ok = warp_wait(acc_full + 8u * buf, use & 1u, lane))) break;
           tc_fence_after();
           unsigned long long x2[4], t2[4];
@@ -280,6 +275,14 @@ __global__ void __launch_bounds__(EB_THREADS, 1)
           tc_fence_before();
           __syncwarp();
           if (lane == 0) mbar_arrive(acc_free + 8u * buf);
+          if (more && piece < 4) {
+            h_put((int)((k + 1) & 1u), piece);
+            if (piece == 3 && lane == 0) mbar_arrive(h_full + 8u * ((k + 1) & 1u));
+          }
+          if (hf == 0) {
+            if (elect_one()) tma_store_wait_read();   // the previous block's T has left the piece
+            __syncwarp();
+          }
           const unsigned long long f2 = pack2(g.factor_v, g.factor_v);
 #pragma unroll
           for (int c = 0; c < 2; c++)
@@ -299,15 +302,13 @@ __global__ void __launch_bounds__(EB_THREADS, 1)
           xs -= EB_X_SLOTS;
           xphase ^= 1;
         }
-        if (more) {
-          h_put((int)((k + 1) & 1u), j);
-          if (j == 3 && lane == 0) mbar_arrive(h_full + 8u * ((k + 1) & 1u));
-        }
       }
       if (!ok && lane == 0 && g.status) atomicCAS(g.status, 0, 62);
       __syncwarp();
       if (lane == 0) mbar_arrive(g_free + 8u * (k & 1u));
-      // the two sets' sums of an edge: odd blocks' through shared memory (two buffers, one barrier a tile and quarter)
+      // The two sets' sums of an edge meet through shared memory.  Set 0 is the one ahead: it leaves its sums and goes on,
+      // set 1 adds them.  (Two buffers: the MMAs come in step order, so set 0 cannot finish a tile before set 1 has left
+      // the previous one.)
       float v[16], lo, hi;
       unpack2(dr2, lo, hi);
       v[0] = (lo + hi) * g.factor_t;
@@ -317,17 +318,23 @@ __global__ void __launch_bounds__(EB_THREADS, 1)
         v[m] = (lo + hi) * g.factor_v;
       }
       float *part = part0 + (k & 1u) * EB_PART;
-      if (set == 1) {
+      if (set == 0) {
 #pragma unroll
         for (int m = 0; m < 16; m++) part[m] = v[m];
-      }
-      asm volatile("bar.sync %0, 64;" ::"r"(1 + q) : "memory");
-      if (set == 0 && in && ok) {
+        __syncwarp();
+        if (lane == 0) mbar_arrive(part_full + 8u * q);
+      } else {
+        if (ok && !warp_wait(part_full + 8u * q, k & 1u, lane)) {
+          if (lane == 0 && g.status) atomicCAS(g.status, 0, 66);
+          ok = false;
+        }
+        if (in && ok) {
 #pragma unroll
-        for (int m = 0; m < 16; m++) v[m] += part[m];
-        float4 *o = reinterpret_cast<float4 *>(g.gY + e * 16);
+          for (int m = 0; m < 16; m++) v[m] += part[m];
+          float4 *o = reinterpret_cast<float4 *>(g.gY + e * 16);
 #pragma unroll
-        for (int i = 0; i < 4; i++) o[i] = make_float4(v[4 * i], v[4 * i + 1], v[4 * i + 2], v[4 * i + 3]);
+          for (int i = 0; i < 4; i++) o[i] = make_float4(v[4 * i], v[4 * i + 1], v[4 * i + 2], v[4 * i + 3]);
+        }
       }
     }
     asm volatile("cp.async.wait_all;" ::: "memory");

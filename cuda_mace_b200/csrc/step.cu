@@ -100,8 +100,8 @@ struct Workspace {
     take(basis, E * 2 * m.nbessel);
     take(Y, E * 16);
     for (int i = 0; i < 2; i++) {
-      take(h[i], E * ST_H);
-      take(dh[i], E * ST_H);
+      take(h[i], (E + 127) / 128 * 128 * ST_H);   // whole tiles of the kernels that read them
+      take(dh[i], (E + 127) / 128 * 128 * ST_H);
     }
     take(A, n * 16 * ST_H * Z);
     take(m0, n * 16 * C);
