@@ -109,24 +109,26 @@ __global__ void __launch_bounds__(LIN_THREADS)
 }
 
 // ---- float64 on the tensor cores (DMMA) -----------------------------------------------------------
-// Same tile bookkeeping, 128 x 128 output tile per CTA, 16 warps of 32 x 32 (4 x 4 mma.sync m8n8k4 f64 tiles,
-// 32 accumulator doubles per thread).  A rows (gathered) and W rows arrive through a 3-stage cp.async ring of
-// 16-wide K slices; the row strides (20 and 132 doubles) make the fragment loads of both operands conflict-free:
-// a fragment load touches 8 rows x 4 consecutive doubles (A) or 4 rows x 8 columns (B), and 2 * stride mod 32 = 8
-// spreads the rows of each half-warp over all 32 banks.  Fragment layout of mma.m8n8k4.f64: A[lane/4][lane%4],
-// B[lane%4][lane/4], C[lane/4][2*(lane%4) + {0,1}].
-// The operator is bound by the FP64 tensor rate at K = Nout = 128 (16 flop/B against a machine balance of ~6).
-// TN: columns of the output tile, 128 or 64 (the radial perceptron's hidden layers are 64 wide: a 128-column tile would
-// spend half of its instructions on padding); the 16 warps form a 4 x 4 grid of 32 x TN/4 pieces in both cases.
-constexpr int DM_TILE = 128, DM_K = 16, DM_THREADS = 512, DM_STAGES = 3;
+// Same tile bookkeeping, TM x TN output tile per CTA, 8 warps of 32 x (8 NJ) (4 x NJ mma.sync m8n8k4 f64 tiles).
+// A rows (gathered) and W rows arrive through a 3-stage cp.async ring of 16-wide K slices; the row strides (20 doubles
+// for A, TN + 4 for W) make the fragment loads of both operands conflict-free: a fragment load touches 8 rows x 4
+// consecutive doubles (A) or 4 rows x 8 columns (B), and 2 * stride mod 32 = 8 spreads the rows of each half-warp over all
+// 32 banks.  Fragment layout of mma.m8n8k4.f64: A[lane/4][lane%4], B[lane%4][lane/4], C[lane/4][2*(lane%4) + {0,1}].
+// The operator is bound by the FP64 rate, 128 flop a cycle and SM for DMMA in every shape (m8n8k4 .. m16n8k16 measured).
+// Two CTAs of 8 warps an SM: the products have few K slices (4 for the radial layers), so a single CTA of 16 warps
+// left the pipe idle while its ring filled and its tile was stored.  Tiles: 64 x 128, 128 x 64 for narrow outputs (a
+// 128-column tile would spend half of its instructions on padding), and smaller ones while those leave SMs without work.
+constexpr int DM_K = 16, DM_THREADS = 256, DM_STAGES = 3;
 constexpr int DM_AS = DM_K + 4;                                // row stride of the A slice in doubles
-template <int TN>
+template <int TM, int TN>
 struct DmGeom {
   static constexpr int BS = TN + 4;                            // row stride of the B slice in doubles
-  static constexpr int STAGE_DOUBLES = DM_TILE * DM_AS + DM_K * BS;
+  static constexpr int STAGE_DOUBLES = TM * DM_AS + DM_K * BS;
   static constexpr int SMEM_BYTES = DM_STAGES * STAGE_DOUBLES * 8;
-  static constexpr int B_COPIES = DM_K * TN / 2 / DM_THREADS;  // 16-byte chunks of a B slice per thread
-  static constexpr int NJ = TN / 32;                           // 8-column MMA tiles per warp
+  static constexpr int A_COPIES = TM * 8 / DM_THREADS;         // 16-byte chunks of an A slice per thread
+  static constexpr int B_COPIES = DM_K * TN / 2 / DM_THREADS;  // of a B slice
+  static constexpr int WN = 8 / (TM / 32);                     // warps along the columns
+  static constexpr int NJ = TN / WN / 8;                       // 8-column MMA tiles per warp
 };
 
 __device__ __forceinline__ void cp_async_16_zfill(void *dst, const void *src, bool valid) {
@@ -135,17 +137,17 @@ __device__ __forceinline__ void cp_async_16_zfill(void *dst, const void *src, bo
   asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(d), "l"(src), "r"(n) : "memory");
 }
 
-template <bool PLAIN, int TN>
-__global__ void __launch_bounds__(DM_THREADS, 1)
+template <bool PLAIN, int TM, int TN>
+__global__ void __launch_bounds__(DM_THREADS, 2)
     linear_dmma_kernel(const double *__restrict__ X, const double *__restrict__ W,
                        const int32_t *__restrict__ node_order, const int32_t *__restrict__ elem_start,
                        int nelements, int64_t nnodes, int K, int Nout, double scale, double *__restrict__ out) {
   extern __shared__ __align__(16) double dm_smem[];
-  __shared__ int64_t row_of[DM_TILE];
+  __shared__ int64_t row_of[TM];
 
   const int l = PLAIN ? 0 : blockIdx.y;
   const int nl = 2 * l + 1;
-  using Geo = DmGeom<TN>;
+  using Geo = DmGeom<TM, TN>;
   constexpr int DM_BS = Geo::BS, DM_STAGE_DOUBLES = Geo::STAGE_DOUBLES;
   const int n0 = blockIdx.z * TN;
 
@@ -155,7 +157,7 @@ __global__ void __launch_bounds__(DM_THREADS, 1)
     for (; z < nelements; z++) {
       seg_begin = elem_start ? elem_start[z] : 0;
       seg_count = elem_start ? (int64_t)elem_start[z + 1] - seg_begin : nnodes;
-      const int64_t tiles = (seg_count * nl + DM_TILE - 1) / DM_TILE;
+      const int64_t tiles = (seg_count * nl + TM - 1) / TM;
       if (tile < tiles) break;
       tile -= tiles;
     }
@@ -163,8 +165,8 @@ __global__ void __launch_bounds__(DM_THREADS, 1)
   }
 
   const int tid = threadIdx.x;
-  if (tid < DM_TILE) {
-    const int64_t rl = tile * DM_TILE + tid;
+  if (tid < TM) {
+    const int64_t rl = tile * TM + tid;
     int64_t grow = -1;
     if (PLAIN) {
       if (rl < nnodes) grow = rl;
@@ -178,13 +180,12 @@ __global__ void __launch_bounds__(DM_THREADS, 1)
   __syncthreads();
 
   const double *Wz = PLAIN ? W : W + ((int64_t)(z * 4 + l) * K) * Nout;
-  // copy assignments: 1024 16-byte chunks per operand and K slice, two per thread
-  int64_t a_src[2];
-  int a_dst[2], a_k[2], b_dst[Geo::B_COPIES], b_k[Geo::B_COPIES], b_c[Geo::B_COPIES];
+  int64_t a_src[Geo::A_COPIES];
+  int a_dst[Geo::A_COPIES], a_k[Geo::A_COPIES], b_dst[Geo::B_COPIES], b_k[Geo::B_COPIES], b_c[Geo::B_COPIES];
 #pragma unroll
-  for (int i = 0; i < 2; i++) {
+  for (int i = 0; i < Geo::A_COPIES; i++) {
     const int c = tid + DM_THREADS * i;
-    const int ar = c >> 3, ach = c & 7;              // A: 128 rows x 8 chunks
+    const int ar = c >> 3, ach = c & 7;              // A: TM rows x 8 chunks
     a_src[i] = row_of[ar] >= 0 ? row_of[ar] * K + ach * 2 : -1;
     a_k[i] = ach * 2;
     a_dst[i] = ar * DM_AS + ach * 2;
@@ -195,13 +196,13 @@ __global__ void __launch_bounds__(DM_THREADS, 1)
     const int bk = c / (TN / 2), bch = c % (TN / 2);   // B: 16 K rows x TN/2 chunks
     b_k[i] = bk;
     b_c[i] = n0 + bch * 2;
-    b_dst[i] = DM_TILE * DM_AS + bk * DM_BS + bch * 2;
+    b_dst[i] = TM * DM_AS + bk * DM_BS + bch * 2;
   }
   auto load_slice = [&](int kt) {
     double *st = dm_smem + (kt % DM_STAGES) * DM_STAGE_DOUBLES;
     const int k0 = kt * DM_K;
 #pragma unroll
-    for (int i = 0; i < 2; i++) {
+    for (int i = 0; i < Geo::A_COPIES; i++) {
       const bool av = a_src[i] >= 0 && k0 + a_k[i] < K;
       cp_async_16_zfill(st + a_dst[i], av ? X + a_src[i] + k0 : X, av);
     }
@@ -214,7 +215,7 @@ __global__ void __launch_bounds__(DM_THREADS, 1)
 
   const int warp = tid >> 5, lane = tid & 31;
   constexpr int NJ = Geo::NJ;
-  const int wm = (warp >> 2) * 32, wn = (warp & 3) * (TN / 4);
+  const int wm = (warp / Geo::WN) * 32, wn = (warp % Geo::WN) * (8 * NJ);
   const int fr = lane >> 2, fk = lane & 3;
   double acc[4][NJ][2];
 #pragma unroll
@@ -234,7 +235,7 @@ __global__ void __launch_bounds__(DM_THREADS, 1)
     if (kt + DM_STAGES - 1 < nk) load_slice(kt + DM_STAGES - 1);
     asm volatile("cp.async.commit_group;" ::: "memory");
     const double *As = dm_smem + (kt % DM_STAGES) * DM_STAGE_DOUBLES;
-    const double *Bs = As + DM_TILE * DM_AS;
+    const double *Bs = As + TM * DM_AS;
 #pragma unroll
     for (int kk = 0; kk < DM_K; kk += 4) {
       double a[4], b[NJ];
@@ -266,22 +267,41 @@ __global__ void __launch_bounds__(DM_THREADS, 1)
   }
 }
 
+template <bool PLAIN, int TM, int TN>
+static int dmma_launch(const double *X, const double *W, const int32_t *node_order, const int32_t *elem_start, int nelements,
+                       int64_t nnodes, int K, int Nout, double scale, double *out, cudaStream_t st, const char *what) {
+  auto kern = linear_dmma_kernel<PLAIN, TM, TN>;
+  constexpr int smem = DmGeom<TM, TN>::SMEM_BYTES;
+  cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+  if (e != cudaSuccess) return fail(CMACE_ERR_CUDA, "%s: cannot reserve shared memory", what);
+  const int64_t tiles = PLAIN ? (nnodes + TM - 1) / TM : (nnodes * 7 + TM - 1) / TM + nelements;
+  if (tiles > 0x7fffffffLL) return fail(CMACE_ERR_UNSUPPORTED, "%s: too many rows", what);
+  const dim3 grid((unsigned)tiles, PLAIN ? 1 : 4, (unsigned)((Nout + TN - 1) / TN));
+  kern<<<grid, DM_THREADS, smem, st>>>(X, W, node_order, elem_start, nelements, nnodes, K, Nout, scale, out);
+  return check_launch(what);
+}
+
+// rows: how many the problem has in all; a tile size is taken when it gives every SM its two CTAs
+template <bool PLAIN>
+static int dmma_any(const double *X, const double *W, const int32_t *node_order, const int32_t *elem_start, int nelements,
+                    int64_t nnodes, int K, int Nout, double scale, double *out, cudaStream_t st, const char *what) {
+  const int64_t rows = PLAIN ? nnodes : nnodes * 16;
+  const int64_t wide = (rows + 63) / 64 * ((Nout + 127) / 128), narrow = (rows + 127) / 128;
+  const int64_t small = (rows + 63) / 64 * ((Nout + 63) / 64);
+  if (Nout > 64 && wide >= 2 * 148)
+    return dmma_launch<PLAIN, 64, 128>(X, W, node_order, elem_start, nelements, nnodes, K, Nout, scale, out, st, what);
+  if (Nout <= 64 && narrow >= 2 * 148)
+    return dmma_launch<PLAIN, 128, 64>(X, W, node_order, elem_start, nelements, nnodes, K, Nout, scale, out, st, what);
+  if (small >= 148)
+    return dmma_launch<PLAIN, 64, 64>(X, W, node_order, elem_start, nelements, nnodes, K, Nout, scale, out, st, what);
+  return dmma_launch<PLAIN, 32, 64>(X, W, node_order, elem_start, nelements, nnodes, K, Nout, scale, out, st, what);
+}
+
 static int linear_dmma(const double *X, const double *W, const int32_t *node_order, const int32_t *elem_start,
                        int nelements, int64_t nnodes, int K, int Nout, double scale, double *out,
                        cmace_stream_t stream) {
-  static bool attr_set = false;
-  if (!attr_set) {
-    if (cudaFuncSetAttribute(linear_dmma_kernel<false, 128>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                             DmGeom<128>::SMEM_BYTES) != cudaSuccess)
-      return fail(CMACE_ERR_CUDA, "cmace_linear_f64: cannot reserve shared memory");
-    attr_set = true;
-  }
-  const int64_t max_tiles = (nnodes * 7 + DM_TILE - 1) / DM_TILE + nelements;
-  if (max_tiles > 0x7fffffffLL) return fail(CMACE_ERR_UNSUPPORTED, "cmace_linear: too many rows");
-  dim3 grid((unsigned)max_tiles, 4, (unsigned)((Nout + DM_TILE - 1) / DM_TILE));
-  linear_dmma_kernel<false, 128><<<grid, DM_THREADS, DmGeom<128>::SMEM_BYTES, (cudaStream_t)stream>>>(
-      X, W, node_order, elem_start, nelements, nnodes, K, Nout, scale, out);
-  return check_launch("cmace_linear_f64");
+  return dmma_any<false>(X, W, node_order, elem_start, nelements, nnodes, K, Nout, scale, out, (cudaStream_t)stream,
+                         "cmace_linear_f64");
 }
 
 // out[M, N] = scale * A[M, K] @ B[K, N], float64: the DMMA tile loop with the identity row map; the FMA tile kernel
@@ -291,29 +311,8 @@ static int gemm_f64(const double *A, const double *B, int64_t M, int K, int N, d
   if (M < 0 || K < 1 || N < 1) return fail(CMACE_ERR_ARG, "cmace_gemm_f64: bad size");
   if (M == 0) return CMACE_OK;
   if (!A || !B || !out) return fail(CMACE_ERR_ARG, "cmace_gemm_f64: null pointer");
-  if (K % 2 == 0 && N % 2 == 0 && aligned16(A) && aligned16(B) && aligned16(out)) {
-    static bool attr_set = false;
-    if (!attr_set) {
-      if (cudaFuncSetAttribute(linear_dmma_kernel<true, 128>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                               DmGeom<128>::SMEM_BYTES) != cudaSuccess ||
-          cudaFuncSetAttribute(linear_dmma_kernel<true, 64>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                               DmGeom<64>::SMEM_BYTES) != cudaSuccess)
-        return fail(CMACE_ERR_CUDA, "cmace_gemm_f64: cannot reserve shared memory");
-      attr_set = true;
-    }
-    const int64_t tiles = (M + DM_TILE - 1) / DM_TILE;
-    if (tiles > 0x7fffffffLL) return fail(CMACE_ERR_UNSUPPORTED, "cmace_gemm_f64: too many rows");
-    if (N <= 64) {   // narrow output: 64-column tiles
-      dim3 grid((unsigned)tiles, 1, 1);
-      linear_dmma_kernel<true, 64><<<grid, DM_THREADS, DmGeom<64>::SMEM_BYTES, (cudaStream_t)stream>>>(
-          A, B, nullptr, nullptr, 1, M, K, N, scale, out);
-    } else {
-      dim3 grid((unsigned)tiles, 1, (unsigned)((N + DM_TILE - 1) / DM_TILE));
-      linear_dmma_kernel<true, 128><<<grid, DM_THREADS, DmGeom<128>::SMEM_BYTES, (cudaStream_t)stream>>>(
-          A, B, nullptr, nullptr, 1, M, K, N, scale, out);
-    }
-    return check_launch("cmace_gemm_f64");
-  }
+  if (K % 2 == 0 && N % 2 == 0 && aligned16(A) && aligned16(B) && aligned16(out))
+    return dmma_any<true>(A, B, nullptr, nullptr, 1, M, K, N, scale, out, (cudaStream_t)stream, "cmace_gemm_f64");
   const int64_t tiles = (M + TILE_M - 1) / TILE_M;
   if (tiles > 0x7fffffffLL) return fail(CMACE_ERR_UNSUPPORTED, "cmace_gemm_f64: too many rows");
   dim3 grid((unsigned)tiles, 1, (unsigned)((N + TILE_N - 1) / TILE_N));

@@ -24,13 +24,17 @@ namespace cmace {
 
 constexpr int kWarpsPerBlock = 4;
 
-template <typename T, int VEC>
-__global__ void __launch_bounds__(kWarpsPerBlock * 32)
+// SPLIT = 1: as described above.  SPLIT = 8: a block owns one receiver (and channel chunk), its eight warps take every
+// eighth pair of edges and add up through shared memory in a fixed order: with fewer receivers than the chip holds warps
+// the walk over one receiver's edges, about 1.6 us a pair, is all there is (192 receivers, 52 edges: 43 us with one warp
+// each).
+template <typename T, int VEC, int SPLIT>
+__global__ void __launch_bounds__(SPLIT == 1 ? kWarpsPerBlock * 32 : SPLIT * 32)
     imp_fwd_kernel(const T *__restrict__ X, const T *__restrict__ Y, const T *__restrict__ R,
                    const int32_t *__restrict__ sender, const int32_t *__restrict__ row_ptr,
                    int64_t nnodes, YStride ys, int C, T *__restrict__ out) {
-  const int lane = threadIdx.x & 31;
-  const int64_t node = (int64_t)blockIdx.x * kWarpsPerBlock + (threadIdx.x >> 5);
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const int64_t node = SPLIT == 1 ? (int64_t)blockIdx.x * kWarpsPerBlock + warp : blockIdx.x;
   if (node >= nnodes) return;
   const int c0 = blockIdx.y * (32 * VEC) + lane * VEC;
   const int64_t e0 = row_ptr[node], e1 = row_ptr[node + 1];
@@ -42,7 +46,7 @@ __global__ void __launch_bounds__(kWarpsPerBlock * 32)
     for (int v = 0; v < VEC; v++) acc[m][v] = T(0);
 
   const int ylm = lane & 15, yedge = lane >> 4;
-  for (int64_t e = e0; e < e1; e += 2) {
+  for (int64_t e = e0 + (SPLIT > 1 ? 2 * warp : 0); e < e1; e += 2 * SPLIT) {
     // second edge of the pair: clamp to a valid edge, its harmonics are zeroed below
     const int64_t eb = (e + 1 < e1) ? e + 1 : e;
     const int64_t ey = yedge ? eb : e;
@@ -76,6 +80,24 @@ __global__ void __launch_bounds__(kWarpsPerBlock * 32)
     }
   }
   T *o = out + node * 16 * C + c0;
+  if constexpr (SPLIT > 1) {
+    extern __shared__ __align__(16) unsigned char imp_smem[];
+    T *part = reinterpret_cast<T *>(imp_smem);   // [SPLIT][16][32 VEC]
+#pragma unroll
+    for (int m = 0; m < 16; m++) store_vec<T, VEC>(part + ((warp * 16 + m) * 32 + lane) * VEC, acc[m]);
+    __syncthreads();
+    for (int m = warp; m < 16; m += SPLIT) {     // every warp sums two components
+      T sum[VEC];
+#pragma unroll
+      for (int v = 0; v < VEC; v++) sum[v] = T(0);
+#pragma unroll
+      for (int w = 0; w < SPLIT; w++)
+#pragma unroll
+        for (int v = 0; v < VEC; v++) sum[v] += part[((w * 16 + m) * 32 + lane) * VEC + v];
+      store_vec<T, VEC>(o + m * C, sum);
+    }
+    return;
+  }
 #pragma unroll
   for (int m = 0; m < 16; m++) store_vec<T, VEC>(o + m * C, acc[m]);
 }
@@ -125,9 +147,12 @@ __global__ void __launch_bounds__(kWarpsPerBlock * 32)
     imp_bwd_edge_kernel(const T *__restrict__ X, const T *__restrict__ Y, const T *__restrict__ R,
                         const T *__restrict__ G, const int32_t *__restrict__ sender,
                         const int32_t *__restrict__ row_ptr, int64_t nnodes, int64_t nedges, YStride ys, int C,
-                        T *__restrict__ gradR, T *__restrict__ gradY_out, T *__restrict__ Tout) {
+                        int slices, T *__restrict__ gradR, T *__restrict__ gradY_out, T *__restrict__ Tout) {
   const int lane = threadIdx.x & 31;
-  const int64_t node = (int64_t)blockIdx.x * kWarpsPerBlock + (threadIdx.x >> 5);
+  // everything written is per edge: `slices` warps share a receiver, each takes every slices-th pair of its edges
+  const int64_t item = (int64_t)blockIdx.x * kWarpsPerBlock + (threadIdx.x >> 5);
+  const int64_t node = slices == 1 ? item : item / slices;
+  const int slice = slices == 1 ? 0 : (int)(item - node * slices);
   if (node >= nnodes) return;
   const int c0 = blockIdx.y * (32 * VEC) + lane * VEC;
   const int64_t e0 = row_ptr[node], e1 = row_ptr[node + 1];
@@ -140,7 +165,7 @@ __global__ void __launch_bounds__(kWarpsPerBlock * 32)
   for (int m = 0; m < 16; m++) load_vec<T, VEC>(g[m], G + (node * 16 + m) * C + c0);
 
   const int ylm = lane & 15, yedge = lane >> 4;
-  for (int64_t e = e0; e < e1; e += 2) {
+  for (int64_t e = e0 + 2 * slice; e < e1; e += 2 * slices) {
     const int64_t eb = (e + 1 < e1) ? e + 1 : e;
     const T yv = __ldg(Y + ylm * ys.m + (yedge ? eb : e) * ys.e);
     // loads of both edges of the pair are issued before either is consumed
@@ -432,21 +457,21 @@ __global__ void sum_partials_kernel(const T *__restrict__ partial, int nchunks, 
   out[i] = s;
 }
 
-template <typename T, int VEC>
-__global__ void __launch_bounds__(kWarpsPerBlock * 32)
+template <typename T, int VEC, int SPLIT>
+__global__ void __launch_bounds__(SPLIT == 1 ? kWarpsPerBlock * 32 : SPLIT * 32)
     imp_bwd_node_kernel(const T *__restrict__ Tin, const int32_t *__restrict__ perm,
                         const int32_t *__restrict__ send_ptr, int64_t nnodes, int C,
                         T *__restrict__ gradX) {
-  const int lane = threadIdx.x & 31;
-  const int64_t node = (int64_t)blockIdx.x * kWarpsPerBlock + (threadIdx.x >> 5);
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const int64_t node = SPLIT == 1 ? (int64_t)blockIdx.x * kWarpsPerBlock + warp : blockIdx.x;
   if (node >= nnodes) return;
   const int c0 = blockIdx.y * (32 * VEC) + lane * VEC;
   const int64_t k0 = send_ptr[node], k1 = send_ptr[node + 1];
   T acc[VEC], acc2[VEC];
 #pragma unroll
   for (int v = 0; v < VEC; v++) acc[v] = acc2[v] = T(0);
-  int64_t k = k0;
-  for (; k + 1 < k1; k += 2) {
+  int64_t k = k0 + (SPLIT > 1 ? 2 * warp : 0);
+  for (; k + 1 < k1; k += 2 * SPLIT) {
     const int64_t ea = perm[k], eb = perm[k + 1];
     T a[VEC], b[VEC];
     load_vec<T, VEC>(a, Tin + ea * C + c0);
@@ -465,6 +490,17 @@ __global__ void __launch_bounds__(kWarpsPerBlock * 32)
   }
 #pragma unroll
   for (int v = 0; v < VEC; v++) acc[v] += acc2[v];
+  if constexpr (SPLIT > 1) {
+    __shared__ T part[SPLIT][32 * VEC];
+#pragma unroll
+    for (int v = 0; v < VEC; v++) part[warp][lane * VEC + v] = acc[v];
+    __syncthreads();
+    if (warp > 0) return;
+#pragma unroll
+    for (int w = 1; w < SPLIT; w++)
+#pragma unroll
+      for (int v = 0; v < VEC; v++) acc[v] += part[w][lane * VEC + v];
+  }
   store_vec<T, VEC>(gradX + node * C + c0, acc);
 }
 
@@ -484,13 +520,25 @@ static int check_common(const void *a, const void *b, const void *c, int64_t nno
   return CMACE_OK;
 }
 
+// Warps per receiver when there are few (receiver, channel chunk) pairs: up to eight pairs an SM the eight-fold split
+// is one wave of blocks and takes a quarter of the time; beyond that one warp a pair fills the chip by itself.
+constexpr int kSplit = 8;
+static bool few_nodes(int64_t pairs) { return pairs <= 148 * 8; }
+
 template <typename T, int VEC>
 static void launch_fwd(const T *X, const T *Y, const T *R, const int32_t *sender,
                        const int32_t *row_ptr, int64_t nnodes, YStride ys, int C, T *out,
                        cudaStream_t st) {
-  dim3 grid((unsigned)((nnodes + kWarpsPerBlock - 1) / kWarpsPerBlock), C / (32 * VEC));
-  imp_fwd_kernel<T, VEC><<<grid, kWarpsPerBlock * 32, 0, st>>>(X, Y, R, sender, row_ptr, nnodes,
-                                                                ys, C, out);
+  const int chunks = C / (32 * VEC);
+  if (few_nodes(nnodes * chunks)) {
+    constexpr int smem = kSplit * 16 * 32 * VEC * (int)sizeof(T);
+    cudaFuncSetAttribute(imp_fwd_kernel<T, VEC, kSplit>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+    imp_fwd_kernel<T, VEC, kSplit><<<dim3((unsigned)nnodes, chunks), kSplit * 32, smem, st>>>(X, Y, R, sender, row_ptr, nnodes,
+                                                                                              ys, C, out);
+    return;
+  }
+  dim3 grid((unsigned)((nnodes + kWarpsPerBlock - 1) / kWarpsPerBlock), chunks);
+  imp_fwd_kernel<T, VEC, 1><<<grid, kWarpsPerBlock * 32, 0, st>>>(X, Y, R, sender, row_ptr, nnodes, ys, C, out);
 }
 
 template <typename T>
@@ -516,9 +564,10 @@ template <typename T, int VEC>
 static void launch_bwd_edge(const T *X, const T *Y, const T *R, const T *G, const int32_t *sender,
                             const int32_t *row_ptr, int64_t nnodes, int64_t nedges, YStride ys, int C, T *gradR,
                             T *gy, T *Tout, cudaStream_t st) {
-  dim3 grid((unsigned)((nnodes + kWarpsPerBlock - 1) / kWarpsPerBlock), C / (32 * VEC));
+  const int slices = few_nodes(nnodes * (C / (32 * VEC))) ? kSplit : 1;
+  dim3 grid((unsigned)((nnodes * slices + kWarpsPerBlock - 1) / kWarpsPerBlock), C / (32 * VEC));
   imp_bwd_edge_kernel<T, VEC><<<grid, kWarpsPerBlock * 32, 0, st>>>(X, Y, R, G, sender, row_ptr,
-                                                                     nnodes, nedges, ys, C, gradR, gy, Tout);
+                                                                     nnodes, nedges, ys, C, slices, gradR, gy, Tout);
 }
 
 static __device__ int g_staged_stall;   // set when a bounded wait of the staged edge pass gave up
@@ -596,8 +645,14 @@ int imp_bwd_edge(const T *X, const T *Y, const T *R, const T *G, const int32_t *
 template <typename T, int VEC>
 static void launch_bwd_node(const T *Tin, const int32_t *perm, const int32_t *send_ptr, int64_t nnodes,
                             int C, T *gradX, cudaStream_t st) {
-  dim3 grid((unsigned)((nnodes + kWarpsPerBlock - 1) / kWarpsPerBlock), C / (32 * VEC));
-  imp_bwd_node_kernel<T, VEC><<<grid, kWarpsPerBlock * 32, 0, st>>>(Tin, perm, send_ptr, nnodes, C, gradX);
+  const int chunks = C / (32 * VEC);
+  if (few_nodes(nnodes * chunks)) {
+    imp_bwd_node_kernel<T, VEC, kSplit><<<dim3((unsigned)nnodes, chunks), kSplit * 32, 0, st>>>(Tin, perm, send_ptr, nnodes, C,
+                                                                                              gradX);
+    return;
+  }
+  dim3 grid((unsigned)((nnodes + kWarpsPerBlock - 1) / kWarpsPerBlock), chunks);
+  imp_bwd_node_kernel<T, VEC, 1><<<grid, kWarpsPerBlock * 32, 0, st>>>(Tin, perm, send_ptr, nnodes, C, gradX);
 }
 
 template <typename T>
