@@ -87,6 +87,8 @@ SIGNATURES = {
     "cmace_scan_workspace_bytes": [_L],
     "cmace_exclusive_scan_i32": [_P, _L, _P, _P, _L, _P],
     "cmace_nl_fill_f64": [_P, _L, _L, _D, _D, _D, _D, _D, _D, _I, _D, _P, _P, _P, _P, _P, _P, _P, _P],
+    "cmace_symcon_plan_uses_program": [_P],
+    "cmace_symcon_apply": [_I, _P, _P, _P, _P, _L, _I, _P, _P],
     "cmace_symcon_effective_weights": [_P, _I, _P, _P, _P, _I, _I, _P, _P],
     "cmace_step_workspace_bytes": [_P, _L, _L, _L],
     "cmace_step_count": [],
@@ -121,7 +123,7 @@ _VALUE_FUNCS = {"cmace_abi_version", "cmace_sender_order_workspace_bytes", "cmac
                 "cmace_radial_hidden_saved_floats", "cmace_nl_num_cells", "cmace_scan_workspace_bytes",
                 "cmace_imp_staged_stalled", "cmace_step_workspace_bytes", "cmace_step_count", "cmace_step_struct_bytes", "cmace_step_name",
                 "cmace_symcon_plan_destroy", "cmace_symcon_plan_nterms", "cmace_symcon_plan_nclasses",
-                "cmace_symcon_plan_is_canonical"}
+                "cmace_symcon_plan_is_canonical", "cmace_symcon_plan_uses_program"}
 
 _lib = None
 
@@ -135,7 +137,7 @@ KERNEL_LAUNCHES = {
     "cmace_imp_bwd_node": 1, "cmace_linear": 1, "cmace_symcon_fwd": 1, "cmace_symcon_bwd": 1,
     "cmace_gemm_pack_weights": 1, "cmace_gemm3x": 1, "cmace_gemm": 1, "cmace_gemm3x_gradr": 1, "cmace_bounded_wait_probe": 1, "cmace_linear_tc": 1,
     "cmace_radial_hidden_fwd": 1, "cmace_radial_hidden_bwd": 1, "cmace_imp_radial_fused_fwd": 1,
-    "cmace_symcon_effective_weights": 1, "cmace_nl_cell_ids": 1, "cmace_nl_count": 1, "cmace_exclusive_scan_i32": 1, "cmace_nl_fill": 1,
+    "cmace_symcon_effective_weights": 1, "cmace_symcon_apply": 1, "cmace_nl_cell_ids": 1, "cmace_nl_count": 1, "cmace_exclusive_scan_i32": 1, "cmace_nl_fill": 1,
 }
 launch_count = 0       # kernels launched through this binding since import
 _timing = None         # list of (name, start_event, end_event) while timing is on

@@ -27,7 +27,7 @@ template <typename T, bool BWD>
 __global__ void __launch_bounds__(128, sizeof(T) == 4 ? 5 : 3)
     step_contract_kernel(const T *__restrict__ X, const int32_t *__restrict__ types, const T *__restrict__ weff,
                          const T *__restrict__ gb, int64_t nnodes, int C, T *__restrict__ out) {
-  const int c = threadIdx.x;
+  const int c = blockIdx.y * blockDim.x + threadIdx.x;
   for (int64_t node = blockIdx.x; node < nnodes; node += gridDim.x) {
     T x[16], g[16], w3[canon::NCLASS3], w2[canon::NCLASS2], w1, value;
     const T *xr = X + node * 16 * C + c;
@@ -46,6 +46,14 @@ __global__ void __launch_bounds__(128, sizeof(T) == 4 ? 5 : 3)
   }
 }
 
+// threads a node: its channels, or the widest block of at most 128 that divides them
+static int channel_block(int C) {
+  if (C <= 128) return C;
+  for (int ch = 128; ch > 32; ch -= 32)
+    if (C % ch == 0) return ch;
+  return 32;
+}
+
 static int64_t node_blocks(int64_t n, int per_sm) {
   const int64_t cap = (int64_t)148 * per_sm;
   return n < cap ? n : cap;
@@ -54,13 +62,17 @@ static int64_t node_blocks(int64_t n, int per_sm) {
 template <typename T>
 int StepKernels<T>::contract_fwd(const T *X, const int32_t *types, const T *weff, int64_t n, int C, T *b,
                                  cudaStream_t st) {
-  if (n > 0) step_contract_kernel<T, false><<<(unsigned)node_blocks(n, 12), C, 0, st>>>(X, types, weff, nullptr, n, C, b);
+  const int ch = channel_block(C);
+  if (n > 0)
+    step_contract_kernel<T, false><<<dim3((unsigned)node_blocks(n, 12), C / ch), ch, 0, st>>>(X, types, weff, nullptr, n, C, b);
   return check_launch("cmace_step(contract_fwd)");
 }
 template <typename T>
 int StepKernels<T>::contract_bwd(const T *X, const int32_t *types, const T *weff, const T *gb, int64_t n, int C, T *gX,
                                  cudaStream_t st) {
-  if (n > 0) step_contract_kernel<T, true><<<(unsigned)node_blocks(n, 12), C, 0, st>>>(X, types, weff, gb, n, C, gX);
+  const int ch = channel_block(C);
+  if (n > 0)
+    step_contract_kernel<T, true><<<dim3((unsigned)node_blocks(n, 12), C / ch), ch, 0, st>>>(X, types, weff, gb, n, C, gX);
   return check_launch("cmace_step(contract_bwd)");
 }
 
@@ -324,3 +336,27 @@ CMACE_STEP_NODES(float)
 CMACE_STEP_NODES(double)
 
 }  // namespace cmace
+
+using namespace cmace;
+
+extern "C" {
+int cmace_symcon_apply(int is_f64, const void *X, const int32_t *atom_types, const void *weff, const void *gout,
+                       int64_t nnodes, int channels, void *out, cmace_stream_t stream) {
+  if (nnodes < 0) return fail(CMACE_ERR_ARG, "cmace_symcon_apply: bad size");
+  if (channels <= 0 || channels % 32 != 0)
+    return fail(CMACE_ERR_UNSUPPORTED, "cmace_symcon_apply: channels must be a multiple of 32");
+  if (nnodes == 0) return CMACE_OK;
+  if (!X || !atom_types || !weff || !out) return fail(CMACE_ERR_ARG, "cmace_symcon_apply: null pointer");
+  cudaStream_t st = (cudaStream_t)stream;
+  if (is_f64) {
+    const double *x = static_cast<const double *>(X), *w = static_cast<const double *>(weff);
+    double *o = static_cast<double *>(out);
+    return gout ? StepKernels<double>::contract_bwd(x, atom_types, w, static_cast<const double *>(gout), nnodes, channels, o, st)
+                : StepKernels<double>::contract_fwd(x, atom_types, w, nnodes, channels, o, st);
+  }
+  const float *x = static_cast<const float *>(X), *w = static_cast<const float *>(weff);
+  float *o = static_cast<float *>(out);
+  return gout ? StepKernels<float>::contract_bwd(x, atom_types, w, static_cast<const float *>(gout), nnodes, channels, o, st)
+              : StepKernels<float>::contract_fwd(x, atom_types, w, nnodes, channels, o, st);
+}
+}

@@ -197,6 +197,12 @@ __global__ void __launch_bounds__(128)
   }
 }
 
+// CMACE_SYMCON_GENERIC=1 in the environment forces the table-driven kernel (tests compare both)
+static bool force_generic() {
+  const char *e = getenv("CMACE_SYMCON_GENERIC");
+  return e != nullptr && e[0] == '1';
+}
+
 // weff [Z][13][C]: the effective class weights above, written once for kernels that read them per (element, channel)
 template <typename T>
 __global__ void effective_weights_kernel(const int32_t *__restrict__ cclass3, const int32_t *__restrict__ cclass2,
@@ -290,15 +296,12 @@ void cmace_symcon_plan_destroy(cmace_symcon_plan *plan) {
 int cmace_symcon_plan_nterms(const cmace_symcon_plan *plan) { return plan ? plan->nterms3 + plan->nterms2 : 0; }
 int cmace_symcon_plan_nclasses(const cmace_symcon_plan *plan) { return plan ? plan->nclass3 + plan->nclass2 : 0; }
 int cmace_symcon_plan_is_canonical(const cmace_symcon_plan *plan) { return plan && plan->canonical ? 1 : 0; }
+int cmace_symcon_plan_uses_program(const cmace_symcon_plan *plan) {
+  return plan && plan->canonical && !force_generic() ? 1 : 0;
+}
 }
 
 namespace cmace {
-
-// CMACE_SYMCON_GENERIC=1 in the environment forces the table-driven kernel (tests compare both)
-static bool force_generic() {
-  const char *e = getenv("CMACE_SYMCON_GENERIC");
-  return e != nullptr && e[0] == '1';
-}
 
 template <typename T, bool BWD>
 static int symcon_launch(const cmace_symcon_plan *plan, const T *X, const int32_t *atom_types, const T *W3,
@@ -400,7 +403,7 @@ int cmace_symcon_effective_weights(const cmace_symcon_plan *plan, int is_f64, co
                                    const void *W1, int nelements, int channels, void *out, cmace_stream_t stream) {
   if (!plan || !W3 || !W2 || !W1 || !out || nelements < 1 || channels < 1 || channels > 1024)
     return fail(CMACE_ERR_ARG, "cmace_symcon_effective_weights: bad argument");
-  if (!plan->canonical)
+  if (!plan->canonical || force_generic())
     return fail(CMACE_ERR_UNSUPPORTED, "cmace_symcon_effective_weights: the plan's tables are not the generated program's");
   const int32_t *ci = plan->d_ints + plan->canon_int_off;
   const dim3 grid((unsigned)nelements, canon::NCLASS3 + canon::NCLASS2 + 1);

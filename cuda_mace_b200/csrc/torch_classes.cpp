@@ -350,7 +350,36 @@ std::shared_ptr<PlanHolder> plan_for(int64_t u3_max, const Tensor &U3_num, const
 
 struct PlanBox : torch::CustomClassHolder {
   std::shared_ptr<PlanHolder> holder;
+  Tensor weff;   // effective weights of the generated program; undefined when the table-driven kernel runs
 };
+
+// Effective contraction weights [Z, 13, C] per weight set: constant buffers of a model, laid out once like the packed
+// matrices above (the entry keeps its sources alive, the version counters catch in-place edits).  Combining them inside
+// the contraction kernel cost every block a pass over all elements' paths: 42 us of a 4096-node call over 10 elements.
+struct EffectiveEntry {
+  Tensor w3, w2, w1, weff;
+  std::shared_ptr<PlanHolder> plan;
+};
+
+Tensor effective_weights(const std::shared_ptr<PlanHolder> &holder, const Tensor &w3, const Tensor &w2, const Tensor &w1) {
+  if (!cmace_symcon_plan_uses_program(holder->plan)) return Tensor();
+  static std::mutex m;
+  using Key = std::tuple<void *, void *, void *, void *, int64_t, int64_t, int64_t, int, int64_t, int64_t>;
+  static std::map<Key, EffectiveEntry> cache;
+  const Key key = std::make_tuple((void *)holder->plan, w3.data_ptr(), w2.data_ptr(), w1.data_ptr(), (int64_t)w3._version(),
+                                  (int64_t)w2._version(), (int64_t)w1._version(), (int)w3.scalar_type(), w3.size(0),
+                                  w3.size(2));
+  std::lock_guard<std::mutex> lock(m);
+  auto it = cache.find(key);
+  if (it != cache.end()) return it->second.weff;
+  if (cache.size() > 32) cache.clear();
+  Tensor weff = torch::empty({w3.size(0), 13, w3.size(2)}, w3.options());
+  check(cmace_symcon_effective_weights(holder->plan, is_f64(w3) ? 1 : 0, w3.data_ptr(), w2.data_ptr(), w1.data_ptr(),
+                                       (int)w3.size(0), (int)w3.size(2), weff.data_ptr(), stream_of(w3)),
+        "cmace_symcon_effective_weights");
+  cache.emplace(key, EffectiveEntry{w3, w2, w1, weff, holder});
+  return weff;
+}
 
 class SymConAutograd : public torch::autograd::Function<SymConAutograd> {
  public:
@@ -362,7 +391,11 @@ class SymConAutograd : public torch::autograd::Function<SymConAutograd> {
     const int64_t N = X.size(0), C = X.size(2), Z = W3.size(0);
     Tensor out = torch::empty({N, 1, C}, X.options());
     const cmace_symcon_plan *plan = box->holder->plan;
-    if (is_f64(X))
+    if (box->weff.defined())
+      check(cmace_symcon_apply(is_f64(X) ? 1 : 0, X.data_ptr(), atom_types.data_ptr<int32_t>(), box->weff.data_ptr(), nullptr,
+                               N, (int)C, out.data_ptr(), stream_of(X)),
+            "cmace_symcon_apply");
+    else if (is_f64(X))
       check(cmace_symcon_fwd_f64(plan, X.data_ptr<double>(), atom_types.data_ptr<int32_t>(), W3.data_ptr<double>(),
                                  W2.data_ptr<double>(), W1.data_ptr<double>(), (int)Z, N, (int)C,
                                  out.data_ptr<double>(), stream_of(X)),
@@ -386,7 +419,11 @@ class SymConAutograd : public torch::autograd::Function<SymConAutograd> {
     const int64_t N = X.size(0), C = X.size(2), Z = W3.size(0);
     Tensor gradX = torch::empty_like(X);
     const cmace_symcon_plan *plan = box->holder->plan;
-    if (is_f64(X))
+    if (box->weff.defined())
+      check(cmace_symcon_apply(is_f64(X) ? 1 : 0, X.data_ptr(), atom_types.data_ptr<int32_t>(), box->weff.data_ptr(),
+                               G.data_ptr(), N, (int)C, gradX.data_ptr(), stream_of(X)),
+            "cmace_symcon_apply");
+    else if (is_f64(X))
       check(cmace_symcon_bwd_f64(plan, X.data_ptr<double>(), atom_types.data_ptr<int32_t>(), W3.data_ptr<double>(),
                                  W2.data_ptr<double>(), W1.data_ptr<double>(), G.data_ptr<double>(), (int)Z, N, (int)C,
                                  gradX.data_ptr<double>(), stream_of(X)),
@@ -516,6 +553,7 @@ class SymmetricContraction : public torch::CustomClassHolder {
     TORCH_CHECK(w3.scalar_type() == X.scalar_type(), "X and the weights must have the same dtype");
     TORCH_CHECK(w3.size(1) == W3_size && w2.size(1) == W2_size && w1.size(1) == W1_size,
                 "weight buffers do not match W3_size / W2_size / W1_size");
+    box->weff = effective_weights(box->holder, w3, w2, w1);
     return SymConAutograd::apply(X, int32_contig(atom_types), w3, w2, w1, box);
   }
   std::vector<Tensor> __getstate__() { return {}; }

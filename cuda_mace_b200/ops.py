@@ -713,16 +713,40 @@ def make_plan(u3_max, U3_num_nonzero, U3_indices, U3_values, U2_num_nonzero, U2_
     return _Plan(handle)
 
 
+_effective_cache = _RefCache(16)
+
+
+def effective_weights(plan, W3, W2, W1):
+    """[Z, 13, C] weights of the generated contraction program, laid out once per weight set; None when the plan runs on
+    the table-driven kernel."""
+    if not _abi.call("cmace_symcon_plan_uses_program", plan.handle):
+        return None
+    key = _RefCache.key(W3, W2, W1) + (plan.handle.value,)
+    hit = _effective_cache.get(key)
+    if hit is not None:
+        return hit
+    Z, C = W3.shape[0], W3.shape[2]
+    weff = torch.empty(Z, 13, C, dtype=W3.dtype, device=W3.device)
+    _abi.call("cmace_symcon_effective_weights", plan.handle, int(W3.dtype == torch.float64), _ptr(W3), _ptr(W2), _ptr(W1),
+              Z, C, _ptr(weff), _stream())
+    return _effective_cache.put(key, (W3, W2, W1, plan), weff)
+
+
 class _SymConFunction(torch.autograd.Function):
     @staticmethod
     def forward(ctx, X, atom_types, W3, W2, W1, plan, nelements):
         X = X.contiguous()
         N, C = X.shape[0], X.shape[2]
         out = torch.empty(N, 1, C, dtype=X.dtype, device=X.device)
-        _abi.call("cmace_symcon_fwd_" + _suffix(X), plan.handle, _ptr(X), _ptr(atom_types), _ptr(W3), _ptr(W2),
-                  _ptr(W1), nelements, N, C, _ptr(out), _stream())
+        weff = effective_weights(plan, W3, W2, W1)
+        if weff is not None:
+            _abi.call("cmace_symcon_apply", int(X.dtype == torch.float64), _ptr(X), _ptr(atom_types), _ptr(weff), 0, N, C,
+                      _ptr(out), _stream())
+        else:
+            _abi.call("cmace_symcon_fwd_" + _suffix(X), plan.handle, _ptr(X), _ptr(atom_types), _ptr(W3), _ptr(W2),
+                      _ptr(W1), nelements, N, C, _ptr(out), _stream())
         ctx.save_for_backward(X, atom_types, W3, W2, W1)
-        ctx.plan, ctx.nelements = plan, nelements
+        ctx.plan, ctx.nelements, ctx.weff = plan, nelements, weff
         return out
 
     @staticmethod
@@ -731,8 +755,12 @@ class _SymConFunction(torch.autograd.Function):
         G = G.contiguous()
         N, C = X.shape[0], X.shape[2]
         gradX = torch.empty_like(X)
-        _abi.call("cmace_symcon_bwd_" + _suffix(X), ctx.plan.handle, _ptr(X), _ptr(atom_types), _ptr(W3),
-                  _ptr(W2), _ptr(W1), _ptr(G), ctx.nelements, N, C, _ptr(gradX), _stream())
+        if ctx.weff is not None:
+            _abi.call("cmace_symcon_apply", int(X.dtype == torch.float64), _ptr(X), _ptr(atom_types), _ptr(ctx.weff),
+                      _ptr(G), N, C, _ptr(gradX), _stream())
+        else:
+            _abi.call("cmace_symcon_bwd_" + _suffix(X), ctx.plan.handle, _ptr(X), _ptr(atom_types), _ptr(W3), _ptr(W2),
+                      _ptr(W1), _ptr(G), ctx.nelements, N, C, _ptr(gradX), _stream())
         return gradX, None, None, None, None, None, None
 
 

@@ -336,6 +336,11 @@ int cmace_symcon_bwd_f64(const cmace_symcon_plan *plan, const double *X, const i
                          int nelements, int64_t nnodes, int channels, double *gradX,
                          cmace_stream_t stream);
 
+/* 1 when the generated program applies to the plan and the environment does not force the table-driven kernel */
+int cmace_symcon_plan_uses_program(const cmace_symcon_plan *plan);
+/* the generated program on effective weights (below): out [N,C] when gout is NULL, else gradX [N,16,C] */
+int cmace_symcon_apply(int is_f64, const void *X, const int32_t *atom_types, const void *weff, const void *gout,
+                       int64_t nnodes, int channels, void *out, cmace_stream_t stream);
 /* effective weights of the generated contraction program, out [nelements][13][channels] in float32 or float64
  * (8 cubic and 4 quadratic classes, then the linear term); CMACE_ERR_UNSUPPORTED for a plan it does not apply to */
 int cmace_symcon_effective_weights(const cmace_symcon_plan *plan, int is_f64, const void *W3, const void *W2,
