@@ -30,19 +30,21 @@ inline int check_launch(const char *what) {
 }
 
 // strides of an array of 16 values per edge, over components and over edges: {E, 1} for [16, E], {1, 16} for [E, 16]
-struct YStride {
+// rows: where a receiver's row stands in the messages and in their gradient, or null for receiver order
+struct ImpLayout {
   int64_t m, e;
+  const int32_t *rows = nullptr;
 };
 
 // operator launchers that other translation units call with their own layout of Y
 template <typename T>
 int imp_fwd(const T *X, const T *Y, const T *R, const int32_t *sender, const int32_t *row_ptr, int64_t nnodes,
-            int64_t nedges, YStride ys, int C, T *out, cmace_stream_t stream);
+            int64_t nedges, ImpLayout ys, int C, T *out, cmace_stream_t stream);
 template <typename T>
 int imp_bwd_edge(const T *X, const T *Y, const T *R, const T *G, const int32_t *sender, const int32_t *row_ptr,
-                 int64_t nnodes, int64_t nedges, YStride ys, int C, T *gradR, T *gradY, T *Tout, T *partial,
+                 int64_t nnodes, int64_t nedges, ImpLayout ys, int C, T *gradR, T *gradY, T *Tout, T *partial,
                  cmace_stream_t stream);
-int gemm3x_gradr(const float *X, const float *G, const float *Y, YStride ys, const int32_t *sender,
+int gemm3x_gradr(const float *X, const float *G, const float *Y, ImpLayout ys, const int32_t *sender,
                  const int32_t *receiver, const float *packed, int64_t nedges, int channels, int N, const float *dot,
                  float *out, int32_t *status, cmace_stream_t stream);
 

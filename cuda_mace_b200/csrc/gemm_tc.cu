@@ -1525,7 +1525,7 @@ static int gemm_launch(GemmArgs &g, const char *what, cudaStream_t st) {
   return check_launch(what);
 }
 
-int gemm3x_gradr(const float *X, const float *G, const float *Y, YStride ys, const int32_t *sender,
+int gemm3x_gradr(const float *X, const float *G, const float *Y, ImpLayout ys, const int32_t *sender,
                  const int32_t *receiver, const float *packed, int64_t nedges, int channels, int N, const float *dot,
                  float *out, int32_t *status, cmace_stream_t stream) {
   if (nedges < 0 || N < 32 || N > 128 || N % 4 != 0)
@@ -1603,7 +1603,7 @@ int cmace_bounded_wait_probe(int32_t *status, int code, double limit_seconds, cm
 int cmace_gemm3x_gradr_f32(const float *X, const float *G, const float *Y, const int32_t *sender,
                            const int32_t *receiver, const float *packed, int64_t nedges, int channels, int N,
                            float *out, int32_t *status, cmace_stream_t stream) {
-  return cmace::gemm3x_gradr(X, G, Y, YStride{nedges, 1}, sender, receiver, packed, nedges, channels, N, nullptr, out, status, stream);
+  return cmace::gemm3x_gradr(X, G, Y, ImpLayout{nedges, 1}, sender, receiver, packed, nedges, channels, N, nullptr, out, status, stream);
 }
 
 int cmace_linear_tc_f32(const float *X, const float *packed, const int32_t *node_order, const int32_t *elem_start,

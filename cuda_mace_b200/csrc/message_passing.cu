@@ -32,7 +32,7 @@ template <typename T, int VEC, int SPLIT>
 __global__ void __launch_bounds__(SPLIT == 1 ? kWarpsPerBlock * 32 : SPLIT * 32)
     imp_fwd_kernel(const T *__restrict__ X, const T *__restrict__ Y, const T *__restrict__ R,
                    const int32_t *__restrict__ sender, const int32_t *__restrict__ row_ptr,
-                   int64_t nnodes, YStride ys, int C, T *__restrict__ out) {
+                   int64_t nnodes, ImpLayout ys, int C, T *__restrict__ out) {
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const int64_t node = SPLIT == 1 ? (int64_t)blockIdx.x * kWarpsPerBlock + warp : blockIdx.x;
   if (node >= nnodes) return;
@@ -79,7 +79,7 @@ __global__ void __launch_bounds__(SPLIT == 1 ? kWarpsPerBlock * 32 : SPLIT * 32)
       }
     }
   }
-  T *o = out + node * 16 * C + c0;
+  T *o = out + (ys.rows ? (int64_t)ys.rows[node] : node) * 16 * C + c0;
   if constexpr (SPLIT > 1) {
     extern __shared__ __align__(16) unsigned char imp_smem[];
     T *part = reinterpret_cast<T *>(imp_smem);   // [SPLIT][16][32 VEC]
@@ -146,7 +146,7 @@ template <typename T, int VEC>
 __global__ void __launch_bounds__(kWarpsPerBlock * 32)
     imp_bwd_edge_kernel(const T *__restrict__ X, const T *__restrict__ Y, const T *__restrict__ R,
                         const T *__restrict__ G, const int32_t *__restrict__ sender,
-                        const int32_t *__restrict__ row_ptr, int64_t nnodes, int64_t nedges, YStride ys, int C,
+                        const int32_t *__restrict__ row_ptr, int64_t nnodes, int64_t nedges, ImpLayout ys, int C,
                         int slices, T *__restrict__ gradR, T *__restrict__ gradY_out, T *__restrict__ Tout) {
   const int lane = threadIdx.x & 31;
   // everything written is per edge: `slices` warps share a receiver, each takes every slices-th pair of its edges
@@ -160,9 +160,10 @@ __global__ void __launch_bounds__(kWarpsPerBlock * 32)
   // with several channel chunks each chunk writes its own [16, E] partial of gradY
   T *gy = gradY_out + (int64_t)blockIdx.y * 16 * nedges;
 
+  const int64_t grow = ys.rows ? (int64_t)ys.rows[node] : node;
   T g[16][VEC];
 #pragma unroll
-  for (int m = 0; m < 16; m++) load_vec<T, VEC>(g[m], G + (node * 16 + m) * C + c0);
+  for (int m = 0; m < 16; m++) load_vec<T, VEC>(g[m], G + (grow * 16 + m) * C + c0);
 
   const int ylm = lane & 15, yedge = lane >> 4;
   for (int64_t e = e0 + 2 * slice; e < e1; e += 2 * slices) {
@@ -279,7 +280,7 @@ template <bool WANT_T, bool WANT_GR>
 __global__ void __launch_bounds__(BS_WARPS * 32, 1)
     imp_bwd_edge_staged_kernel(const float *__restrict__ X, const float *__restrict__ Y, const float *__restrict__ R,
                                const float *__restrict__ G, const int32_t *__restrict__ sender,
-                               const int32_t *__restrict__ row_ptr, int64_t nnodes, int64_t nedges, YStride ys,
+                               const int32_t *__restrict__ row_ptr, int64_t nnodes, int64_t nedges, ImpLayout ys,
                                float *__restrict__ gradR, float *__restrict__ gy, float *__restrict__ Tout,
                                int *__restrict__ stalled) {
   extern __shared__ __align__(128) unsigned char bs_smem[];
@@ -342,9 +343,10 @@ __global__ void __launch_bounds__(BS_WARPS * 32, 1)
     if (WANT_U && nc.e >= 0) yv_next = __ldg(Y + ylm * ys.m + nc.e * ys.e);
     if (node != g_node) {
       g_node = node;
+      const int64_t grow = ys.rows ? (int64_t)ys.rows[node] : node;
 #pragma unroll
       for (int m = 0; m < 16; m++) {
-        const ulonglong2 v = __ldg(reinterpret_cast<const ulonglong2 *>(G + (node * 16 + m) * BS_C + c0));
+        const ulonglong2 v = __ldg(reinterpret_cast<const ulonglong2 *>(G + (grow * 16 + m) * BS_C + c0));
         g2[m][0] = v.x;
         g2[m][1] = v.y;
       }
@@ -527,7 +529,7 @@ static bool few_nodes(int64_t pairs) { return pairs <= 148 * 8; }
 
 template <typename T, int VEC>
 static void launch_fwd(const T *X, const T *Y, const T *R, const int32_t *sender,
-                       const int32_t *row_ptr, int64_t nnodes, YStride ys, int C, T *out,
+                       const int32_t *row_ptr, int64_t nnodes, ImpLayout ys, int C, T *out,
                        cudaStream_t st) {
   const int chunks = C / (32 * VEC);
   if (few_nodes(nnodes * chunks)) {
@@ -543,7 +545,7 @@ static void launch_fwd(const T *X, const T *Y, const T *R, const int32_t *sender
 
 template <typename T>
 int imp_fwd(const T *X, const T *Y, const T *R, const int32_t *sender, const int32_t *row_ptr,
-            int64_t nnodes, int64_t nedges, YStride ys, int C, T *out, cmace_stream_t stream) {
+            int64_t nnodes, int64_t nedges, ImpLayout ys, int C, T *out, cmace_stream_t stream) {
   int rc = check_common<T>(X, R, out, nnodes, nedges, C, "cmace_imp_fwd");
   if (rc) return rc;
   if (nnodes == 0) return CMACE_OK;
@@ -562,7 +564,7 @@ int imp_fwd(const T *X, const T *Y, const T *R, const int32_t *sender, const int
 
 template <typename T, int VEC>
 static void launch_bwd_edge(const T *X, const T *Y, const T *R, const T *G, const int32_t *sender,
-                            const int32_t *row_ptr, int64_t nnodes, int64_t nedges, YStride ys, int C, T *gradR,
+                            const int32_t *row_ptr, int64_t nnodes, int64_t nedges, ImpLayout ys, int C, T *gradR,
                             T *gy, T *Tout, cudaStream_t st) {
   const int slices = few_nodes(nnodes * (C / (32 * VEC))) ? kSplit : 1;
   dim3 grid((unsigned)((nnodes * slices + kWarpsPerBlock - 1) / kWarpsPerBlock), C / (32 * VEC));
@@ -584,7 +586,7 @@ static int *staged_stall_flag() {
 
 template <typename T>
 int imp_bwd_edge(const T *X, const T *Y, const T *R, const T *G, const int32_t *sender,
-                        const int32_t *row_ptr, int64_t nnodes, int64_t nedges, YStride ys, int C, T *gradR,
+                        const int32_t *row_ptr, int64_t nnodes, int64_t nedges, ImpLayout ys, int C, T *gradR,
                         T *gradY, T *Tout, T *partial, cmace_stream_t stream) {
   int rc = check_common<T>(X, R, G, nnodes, nedges, C, "cmace_imp_bwd_edge");
   if (rc) return rc;
@@ -674,10 +676,10 @@ int imp_bwd_node(const T *Tin, const int32_t *perm, const int32_t *send_ptr, int
 }
 
 #define CMACE_IMP_LAUNCHERS(T)                                                                                        \
-  template int imp_fwd<T>(const T *, const T *, const T *, const int32_t *, const int32_t *, int64_t, int64_t, YStride, \
+  template int imp_fwd<T>(const T *, const T *, const T *, const int32_t *, const int32_t *, int64_t, int64_t, ImpLayout, \
                           int, T *, cmace_stream_t);                                                                   \
   template int imp_bwd_edge<T>(const T *, const T *, const T *, const T *, const int32_t *, const int32_t *, int64_t,  \
-                               int64_t, YStride, int, T *, T *, T *, T *, cmace_stream_t);
+                               int64_t, ImpLayout, int, T *, T *, T *, T *, cmace_stream_t);
 CMACE_IMP_LAUNCHERS(float)
 CMACE_IMP_LAUNCHERS(double)
 
@@ -731,12 +733,12 @@ int cmace_imp_staged_stalled(void) {
 int cmace_imp_fwd_f32(const float *X, const float *Y, const float *R, const int32_t *sender,
                       const int32_t *row_ptr, int64_t nnodes, int64_t nedges, int channels, float *out,
                       cmace_stream_t stream) {
-  return imp_fwd<float>(X, Y, R, sender, row_ptr, nnodes, nedges, YStride{nedges, 1}, channels, out, stream);
+  return imp_fwd<float>(X, Y, R, sender, row_ptr, nnodes, nedges, ImpLayout{nedges, 1}, channels, out, stream);
 }
 int cmace_imp_fwd_f64(const double *X, const double *Y, const double *R, const int32_t *sender,
                       const int32_t *row_ptr, int64_t nnodes, int64_t nedges, int channels, double *out,
                       cmace_stream_t stream) {
-  return imp_fwd<double>(X, Y, R, sender, row_ptr, nnodes, nedges, YStride{nedges, 1}, channels, out, stream);
+  return imp_fwd<double>(X, Y, R, sender, row_ptr, nnodes, nedges, ImpLayout{nedges, 1}, channels, out, stream);
 }
 int64_t cmace_imp_bwd_scratch_elems(int64_t nedges, int channels, int is_f64) {
   if (channels <= 0 || channels % 32 != 0) return 0;
@@ -748,14 +750,14 @@ int cmace_imp_bwd_edge_f32(const float *X, const float *Y, const float *R, const
                            const int32_t *sender, const int32_t *row_ptr, int64_t nnodes, int64_t nedges,
                            int channels, float *gradR, float *gradY, float *T, float *gradY_partial,
                            cmace_stream_t stream) {
-  return imp_bwd_edge<float>(X, Y, R, G, sender, row_ptr, nnodes, nedges, YStride{nedges, 1}, channels, gradR, gradY, T,
+  return imp_bwd_edge<float>(X, Y, R, G, sender, row_ptr, nnodes, nedges, ImpLayout{nedges, 1}, channels, gradR, gradY, T,
                              gradY_partial, stream);
 }
 int cmace_imp_bwd_edge_f64(const double *X, const double *Y, const double *R, const double *G,
                            const int32_t *sender, const int32_t *row_ptr, int64_t nnodes, int64_t nedges,
                            int channels, double *gradR, double *gradY, double *T, double *gradY_partial,
                            cmace_stream_t stream) {
-  return imp_bwd_edge<double>(X, Y, R, G, sender, row_ptr, nnodes, nedges, YStride{nedges, 1}, channels, gradR, gradY, T,
+  return imp_bwd_edge<double>(X, Y, R, G, sender, row_ptr, nnodes, nedges, ImpLayout{nedges, 1}, channels, gradR, gradY, T,
                               gradY_partial, stream);
 }
 int64_t cmace_imp_bwd_edge_f64_noalloc_max_elems(void) { return kStaticScratchElems; }
@@ -778,7 +780,7 @@ int cmace_imp_bwd_edge_f64_noalloc(const double *X, const double *Y, const doubl
     if (e != cudaSuccess)
       return fail(CMACE_ERR_CUDA, "cmace_imp_bwd_edge_f64_noalloc: %s", cudaGetErrorString(e));
   }
-  return imp_bwd_edge<double>(X, Y, R, G, sender, row_ptr, nnodes, nedges, YStride{nedges, 1}, channels, gradR, gradY, T, scratch,
+  return imp_bwd_edge<double>(X, Y, R, G, sender, row_ptr, nnodes, nedges, ImpLayout{nedges, 1}, channels, gradR, gradY, T, scratch,
                               stream);
 }
 

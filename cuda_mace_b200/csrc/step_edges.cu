@@ -167,9 +167,13 @@ __global__ void __launch_bounds__(EP_THREADS)
   sph_l3<T>(uz, ux, uy, y);
   if (lane < rows) geo[e] = Quad<T>{ux, uy, uz, ir};
   store_rows<T, 16>(buf, y, Y + base * 16, rows, lane);
-  T b[2 * NB];
-  bessel_cutoff<T>(r2 * ir, r_max, NB, p, b, b + NB);
-  store_rows<T, 2 * NB>(buf, b, basis + base * 2 * NB, rows, lane);
+  if constexpr (NB == 0) {   // tabulated radial weights: the length itself
+    if (lane < rows) basis[e] = r2 * ir;
+  } else {
+    T b[2 * NB];
+    bessel_cutoff<T>(r2 * ir, r_max, NB, p, b, b + NB);
+    store_rows<T, 2 * NB>(buf, b, basis + base * 2 * NB, rows, lane);
+  }
 }
 
 template <typename T>
@@ -180,7 +184,7 @@ int StepKernels<T>::edge_prep(const double *pos, const int32_t *sender, const in
                               int32_t *slot_type, int32_t *elem_start, cudaStream_t st) {
   const int64_t blocks = 1 + (nedges + EP_THREADS - 1) / EP_THREADS;
   const size_t smem = (size_t)EP_THREADS * ((nb == 16 ? 32 : 16) * sizeof(T) + 16);
-  auto kern = nb == 16 ? edge_prep_kernel<T, 16> : edge_prep_kernel<T, 8>;
+  auto kern = nb == 16 ? edge_prep_kernel<T, 16> : (nb == 8 ? edge_prep_kernel<T, 8> : edge_prep_kernel<T, 0>);
   cudaError_t err = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
   if (err != cudaSuccess) return fail(CMACE_ERR_CUDA, "cmace_step(edge_prep): %s", cudaGetErrorString(err));
   kern<<<(unsigned)blocks, EP_THREADS, smem, st>>>(pos, sender, receiver, shifts, nedges, (T)r_max, p, geo, basis, Y,
@@ -836,6 +840,51 @@ int StepKernels<T>::sums_bwd(const T *gA, const T *h, const T *dh, const T *Y, c
   }
   return check_launch("cmace_step(sums_bwd)");
 }
+
+// ---- tabulated radial weights ---------------------------------------------------------------------------------------
+// element of every edge's sender
+__global__ void __launch_bounds__(256)
+    sender_species_kernel(const int32_t *__restrict__ sender, const int32_t *__restrict__ species, int64_t nedges,
+                          int32_t *__restrict__ out) {
+  const int64_t e = (int64_t)blockIdx.x * 256 + threadIdx.x;
+  if (e < nedges) out[e] = species[sender[e]];
+}
+int step_sender_species(const int32_t *sender, const int32_t *species, int64_t nedges, int32_t *out, cudaStream_t st) {
+  if (nedges > 0) sender_species_kernel<<<(unsigned)((nedges + 255) / 256), 256, 0, st>>>(sender, species, nedges, out);
+  return check_launch("cmace_step(sums)");
+}
+
+// gradient of every edge's vector from both layers' grad Y and dE/dr
+template <typename T>
+__global__ void __launch_bounds__(256)
+    edge_finish_kernel(const T *__restrict__ gY0, const T *__restrict__ dr0, const T *__restrict__ gY1,
+                       const T *__restrict__ dr1, const Quad<T> *__restrict__ geo, int64_t nedges, T *__restrict__ gvec) {
+  const int64_t e = (int64_t)blockIdx.x * 256 + threadIdx.x;
+  if (e >= nedges) return;
+  T s[17];
+  const Quad<T> *g = reinterpret_cast<const Quad<T> *>(gY0 + e * 16);
+#pragma unroll
+  for (int i = 0; i < 4; i++) {
+    const Quad<T> q = g[i];
+    s[4 * i] = q.x;
+    s[4 * i + 1] = q.y;
+    s[4 * i + 2] = q.z;
+    s[4 * i + 3] = q.w;
+  }
+  s[16] = dr0[e];
+  finish_edge<T>(s, e, gY1, dr1, geo, gvec);
+}
+template <typename T>
+int step_edge_finish(const T *gY0, const T *dr0, const T *gY1, const T *dr1, const Quad<T> *geo, int64_t nedges, T *gvec,
+                     cudaStream_t st) {
+  if (nedges > 0)
+    edge_finish_kernel<T><<<(unsigned)((nedges + 255) / 256), 256, 0, st>>>(gY0, dr0, gY1, dr1, geo, nedges, gvec);
+  return check_launch("cmace_step(sums_back)");
+}
+template int step_edge_finish<float>(const float *, const float *, const float *, const float *, const Quad<float> *, int64_t,
+                                     float *, cudaStream_t);
+template int step_edge_finish<double>(const double *, const double *, const double *, const double *, const Quad<double> *,
+                                      int64_t, double *, cudaStream_t);
 
 // ---- forces and energies ------------------------------------------------------------------------------------------
 // One warp per atom sums its edges' gradients from both groupings (float64, fixed order, no atomics); block 0 adds up

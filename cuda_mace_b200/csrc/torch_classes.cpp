@@ -11,6 +11,7 @@
 // handles they ask for with torch.classes.<ns>.<Class>().  This file owns what the C-ABI leaves to its caller:
 // output and scratch allocation through the caching allocator, argument checks, the autograd Functions
 // (gradients for the float inputs only, as in the reference) and the current CUDA stream.
+#include <ATen/cuda/CUDAEvent.h>
 #include <c10/cuda/CUDAGuard.h>
 #include <c10/cuda/CUDAFunctions.h>
 #include <c10/cuda/CUDAStream.h>
@@ -84,7 +85,7 @@ Tensor status_peek(int dev) {
 
 // ---- edge topology: receiver CSR and, for the backward, the sender-grouped edge order --------------------
 struct Topology {
-  Tensor sender, receiver, row_ptr, perm, send_ptr;
+  Tensor sender, receiver, row_ptr, perm, send_ptr, workspace;
   int64_t nnodes = 0, nsenders = 0, nedges = 0;
 };
 
@@ -102,14 +103,16 @@ Topology make_topology(const Tensor &sender_list, const Tensor &receiver_list, i
   return t;
 }
 
-void add_sender_order(Topology &t) {
+// on `stream`; the arrays come from the current stream's pool
+void add_sender_order(Topology &t, cmace_stream_t stream) {
   const int64_t nbytes = cmace_sender_order_workspace_bytes(t.nedges);
   Tensor ws = torch::empty({std::max<int64_t>(nbytes, 1)}, t.sender.options().dtype(torch::kUInt8));
   t.perm = torch::empty({std::max<int64_t>(t.nedges, 1)}, t.sender.options());
   t.send_ptr = torch::empty({t.nsenders + 1}, t.sender.options());
   check(cmace_sender_order(t.sender.data_ptr<int32_t>(), t.nedges, t.nsenders, t.perm.data_ptr<int32_t>(),
-                           t.send_ptr.data_ptr<int32_t>(), ws.data_ptr(), nbytes, stream_of(t.sender)),
+                           t.send_ptr.data_ptr<int32_t>(), ws.data_ptr(), nbytes, stream),
         "cmace_sender_order");
+  t.workspace = ws;
 }
 
 // ---- invariant message passing ------------------------------------------------------------------------
@@ -162,8 +165,23 @@ class IMPAutograd : public torch::autograd::Function<IMPAutograd> {
     Tensor T = torch::empty({std::max<int64_t>(E, 1), C}, X.options());
     const int64_t nscratch = cmace_imp_bwd_scratch_elems(E, (int)C, f64 ? 1 : 0);
     Tensor scratch = torch::empty({std::max<int64_t>(nscratch, 1)}, X.options());
-    add_sender_order(topo);
     Tensor gradX = torch::empty_like(X);
+    // The grouping by sender (a radix sort: six small kernels, 40 us at 250 000 edges) does not depend on the edge pass
+    // and leaves most of the GPU idle: beside it on a stream of its own once the list is long enough to be worth two
+    // events.  The node pass waits for it, so everything it used is free again on this stream after that.
+    const auto main_stream = c10::cuda::getCurrentCUDAStream(X.device().index());
+    at::cuda::CUDAEvent sorted;
+    const bool beside = E >= 32768;
+    if (beside) {
+      const auto side = c10::cuda::getStreamFromPool(false, X.device().index());
+      at::cuda::CUDAEvent ready;
+      ready.record(main_stream);
+      ready.block(side);
+      add_sender_order(topo, (cmace_stream_t)side.stream());
+      sorted.record(side);
+    } else {
+      add_sender_order(topo, stream_of(X));
+    }
     if (f64) {
       check(cmace_imp_bwd_edge_f64(X.data_ptr<double>(), Y.data_ptr<double>(), radial.data_ptr<double>(),
                                    G.data_ptr<double>(), topo.sender.data_ptr<int32_t>(),
@@ -171,6 +189,7 @@ class IMPAutograd : public torch::autograd::Function<IMPAutograd> {
                                    gradY.data_ptr<double>(), T.data_ptr<double>(),
                                    nscratch > 0 ? scratch.data_ptr<double>() : nullptr, stream_of(X)),
             "cmace_imp_bwd_edge_f64");
+      if (beside) sorted.block(main_stream);
       check(cmace_imp_bwd_node_f64(T.data_ptr<double>(), topo.perm.data_ptr<int32_t>(),
                                    topo.send_ptr.data_ptr<int32_t>(), topo.nsenders, (int)C, gradX.data_ptr<double>(),
                                    stream_of(X)),
@@ -182,6 +201,7 @@ class IMPAutograd : public torch::autograd::Function<IMPAutograd> {
                                    gradY.data_ptr<float>(), T.data_ptr<float>(),
                                    nscratch > 0 ? scratch.data_ptr<float>() : nullptr, stream_of(X)),
             "cmace_imp_bwd_edge_f32");
+      if (beside) sorted.block(main_stream);
       check(cmace_imp_bwd_node_f32(T.data_ptr<float>(), topo.perm.data_ptr<int32_t>(),
                                    topo.send_ptr.data_ptr<int32_t>(), topo.nsenders, (int)C, gradX.data_ptr<float>(),
                                    stream_of(X)),

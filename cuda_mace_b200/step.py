@@ -89,14 +89,23 @@ def fused_rows(device):
 
 def covers(model):
     """Whether the sequence covers a model: the standard two-layer architecture in float32 or float64."""
-    if model.radial != "exact" or len(model.layers) != 2 or model.num_elements > 16:
+    if model.radial not in ("exact", "spline") or len(model.layers) != 2 or model.num_elements > 16:
         return False
     if model.dtype not in (torch.float32, torch.float64) or model.channels not in (32, 64, 96, 128):
         return False
-    if model.edge_basis.num_bessel not in (8, 16) or os.environ.get("CMACE_SYMCON_GENERIC", "")[:1] == "1":
+    if os.environ.get("CMACE_SYMCON_GENERIC", "")[:1] == "1":
         return False
     C, nb = model.channels, model.edge_basis.num_bessel
+    if model.radial == "exact" and nb not in (8, 16):
+        return False
     for L in model.layers:
+        if model.radial == "spline":
+            first, co = model.layers[0].spline, L.spline.coefficients
+            if co.shape != first.coefficients.shape or co.shape[1:] != (4, 4 * C) or co.dtype != model.dtype:
+                return False
+            if L.spline.h != first.h or L.spline.rmax != first.rmax:
+                return False
+            continue
         if L.n_radial != 4:
             return False
         shapes = [tuple(getattr(L, f"W_radial{i}").shape) for i in range(4)]
@@ -131,6 +140,50 @@ class StepPlan:
             W = W.to(model.dtype)
             return hold(_pack(W.transpose(-1, -2)) if f32 else W)
 
+        x = d(model.embedding) @ d(L0.W_up)                                  # [Z, C] sender features of the first layer
+        lin = d(L0.linear.weights) / math.sqrt(C)                            # [Z, 4, C, C]
+        if model.radial == "spline":
+            for t, L in enumerate((L0, L1)):
+                m.spline[t] = hold(L.spline.coefficients)
+            m.spline_knots, m.sender_table = hold(L0.spline.r_knots), hold(x.to(model.dtype))
+            m.spline_width, m.spline_rmax = L0.spline.h, L0.spline.rmax
+            m.spline_intervals = L0.spline.coefficients.shape[0]
+            m.fold, m.fold_back[0] = matrix(lin), matrix(lin.transpose(-1, -2))
+        else:
+            self._radial(model, m, hold, matrix, x, lin)
+        lin = d(L1.linear.weights) / math.sqrt(C)
+        m.linear[0], m.linear[1] = matrix(lin), matrix(lin.transpose(-1, -2))
+        for t, L in enumerate((L0, L1)):
+            con = L.contraction
+            if con._plan is None:
+                con._plan = ops.make_plan(con.u3_max_nonsparse, con.U3_num_nonsparse, con.U3_indices, con.U3_values,
+                                          con.U2_num_nonsparse, con.U2_indices, con.U2_values, con.W3_L0_size,
+                                          con.W2_L0_size, con.W1_L0_size)
+            weff = torch.empty(Z, 13, C, dtype=model.dtype, device=x.device)
+            _abi.call("cmace_symcon_effective_weights", con._plan.handle, int(not f32), con.weights_3.data_ptr(),
+                      con.weights_2.data_ptr(), con.weights_1.data_ptr(), Z, C, weff.data_ptr(), ops._stream())
+            m.weff[t] = hold(weff)
+        prod0, prod1, ro1 = d(L0.W_prod), d(L1.W_prod), d(L1.W_readout1)
+        up = prod0 @ d(L1.W_up)
+        m.up, m.up_back = hold(up.to(model.dtype)), hold(up.t().to(model.dtype))
+        sc = d(L1.W_sc).view(C, Z, C).permute(1, 0, 2)                       # [Z, C, C]
+        extra = torch.cat([prod0 @ sc @ ro1, (prod0 @ d(L0.W_readout)).expand(Z, C, 1)], dim=2)   # [Z, C, 17]
+        m.extra = hold(extra.view(Z, C // 4, 4, 17).transpose(2, 3).to(model.dtype))
+        m.extra_back = hold(extra.transpose(1, 2).to(model.dtype))
+        m.readout1 = hold((prod1 @ ro1).t().to(model.dtype))
+        m.readout2 = hold(d(L1.W_readout2)[:, 0] * SILU_2MOM)
+        m.atomic_energies = hold(model.atomic_energies)
+        self.model = m
+        self.channels, self.dtype, self.elements = C, model.dtype, Z
+        self.radial_ops = (ops.USE_TENSOR_CORES, ops.RADIAL_GRADIENT_ON_THE_FLY, ops.FUSED_RADIAL_MESSAGE_PASSING)
+
+    @staticmethod
+    def _radial(model, m, hold, matrix, x, lin):
+        """Weights of the radial perceptrons, and the first layer's element-dependent product of their hidden layers."""
+        d = lambda t: t.double()
+        f32 = model.dtype == torch.float32
+        C, Z = model.channels, model.num_elements
+        L0, L1 = model.layers
         for t, L in enumerate((L0, L1)):
             for i in range(4):
                 if (t, i) != (0, 3):
@@ -158,38 +211,11 @@ class StepPlan:
                     wt = L1.W_radial3.t().reshape(4, 16, 8, _H).transpose(0, 1).reshape(16, 32, _H)   # [step, (l, c), k]
                     m.fused_w_back = hold(torch.stack([half_images(b, scale) for b in wt]))
         m.radial_back = matrix(L1.W_radial3.t())
-        x = d(model.embedding) @ d(L0.W_up)                                  # [Z, C] sender features of the first layer
         w4 = d(L0.W_radial3).view(_H, 4, C)
-        lin = d(L0.linear.weights) / math.sqrt(C)                            # [Z, 4, C, C]
         fold = torch.einsum("zc,klc,rlcd->rlzkd", x, w4, lin).reshape(Z, 4, Z * _H, C)
         m.fold = matrix(fold)
         for b in range((Z + 1) // 2):
             m.fold_back[b] = matrix(fold[:, :, 2 * b * _H: min(2 * b + 2, Z) * _H].transpose(-1, -2))
-        lin = d(L1.linear.weights) / math.sqrt(C)
-        m.linear[0], m.linear[1] = matrix(lin), matrix(lin.transpose(-1, -2))
-        for t, L in enumerate((L0, L1)):
-            con = L.contraction
-            if con._plan is None:
-                con._plan = ops.make_plan(con.u3_max_nonsparse, con.U3_num_nonsparse, con.U3_indices, con.U3_values,
-                                          con.U2_num_nonsparse, con.U2_indices, con.U2_values, con.W3_L0_size,
-                                          con.W2_L0_size, con.W1_L0_size)
-            weff = torch.empty(Z, 13, C, dtype=model.dtype, device=x.device)
-            _abi.call("cmace_symcon_effective_weights", con._plan.handle, int(not f32), con.weights_3.data_ptr(),
-                      con.weights_2.data_ptr(), con.weights_1.data_ptr(), Z, C, weff.data_ptr(), ops._stream())
-            m.weff[t] = hold(weff)
-        prod0, prod1, ro1 = d(L0.W_prod), d(L1.W_prod), d(L1.W_readout1)
-        up = prod0 @ d(L1.W_up)
-        m.up, m.up_back = hold(up.to(model.dtype)), hold(up.t().to(model.dtype))
-        sc = d(L1.W_sc).view(C, Z, C).permute(1, 0, 2)                       # [Z, C, C]
-        extra = torch.cat([prod0 @ sc @ ro1, (prod0 @ d(L0.W_readout)).expand(Z, C, 1)], dim=2)   # [Z, C, 17]
-        m.extra = hold(extra.view(Z, C // 4, 4, 17).transpose(2, 3).to(model.dtype))
-        m.extra_back = hold(extra.transpose(1, 2).to(model.dtype))
-        m.readout1 = hold((prod1 @ ro1).t().to(model.dtype))
-        m.readout2 = hold(d(L1.W_readout2)[:, 0] * SILU_2MOM)
-        m.atomic_energies = hold(model.atomic_energies)
-        self.model = m
-        self.channels, self.dtype, self.elements = C, model.dtype, Z
-        self.radial_ops = (ops.USE_TENSOR_CORES, ops.RADIAL_GRADIENT_ON_THE_FLY, ops.FUSED_RADIAL_MESSAGE_PASSING)
 
     def current(self):
         for d, k, t, v in self.sources:

@@ -367,6 +367,13 @@ typedef struct cmace_step_model {
                                 x 128 bytes], 128-byte swizzle */
   float fused_scale, reserved2;
   const void *radial_back;   /* second layer's W4 for the gradient: float32 packed W4 itself, float64 W4^T [4C,64] */
+  const void *spline[2];     /* tabulated radial weights: coefficients [intervals][4][4C] of both layers, or NULL; then the
+                                radial weights above are not read, fold is the first layer's Linear [elements][4] [C, C]
+                                and fold_back[0] its transposes */
+  const void *spline_knots;  /* [intervals] */
+  const void *sender_table;  /* with spline: the first layer's sender features [elements, C] */
+  double spline_width, spline_rmax;
+  int32_t spline_intervals, reserved3;
   const void *fold;          /* first layer: [elements][4] matrices [64 elements, C] (float32: packed) */
   const void *fold_back[8];  /* their transposes in blocks of two elements: [elements][4] [C, 128 or 64] */
   const void *linear[2];     /* second layer's Linear and its transpose, [4] [C, C] (float32: packed) */

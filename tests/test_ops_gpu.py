@@ -620,3 +620,23 @@ def test_a_wait_that_runs_out_is_reported_and_the_context_survives(dev):
     out = ops.linear_forward(x, w, w.transpose(-1, -2).contiguous())
     assert torch.isfinite(out).all()
     ops.check_status()
+
+
+# float64 products at the sizes where the tile changes (32 and 64 rows while 64- and 128-row tiles leave SMs idle) and at
+# the remainders of each; 1e-12 is 2 K ulp of the largest sum
+@pytest.mark.parametrize("M,K,N", [(1, 16, 64), (2000, 64, 64), (148 * 64 - 1, 64, 64), (148 * 64 + 1, 128, 64),
+                                   (296 * 128 + 5, 64, 32), (2367, 64, 512), (296 * 64 + 1, 32, 128)])
+def test_float64_product_tiles(M, K, N):
+    from cuda_mace_b200 import ops
+
+    g = torch.Generator("cuda").manual_seed(M)
+    A = torch.randn(M, K, generator=g, device="cuda", dtype=torch.float64)
+    B = torch.randn(K, N, generator=g, device="cuda", dtype=torch.float64)
+    assert rel_err(ops.matmul_f64(A, B), A.cpu() @ B.cpu()) < 1e-12
+
+
+# one receiver count on each side of the rule that splits a receiver over eight warps, odd degrees and empty receivers
+@pytest.mark.parametrize("dtype", DTYPES)
+@pytest.mark.parametrize("N,deg,C", [(1184, 9, 32), (1185, 9, 32), (3, 17, 128), (592, 5, 128)])
+def test_message_passing_around_the_split(dtype, N, deg, C, dev):
+    test_message_passing(dtype, N, deg, C, None, 7, dev)

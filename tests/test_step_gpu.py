@@ -48,12 +48,20 @@ def test_step_against_the_oracle(U, dtype, tol_e, tol_f, n, C, Z, stretch):
     assert n == 1 or not torch.equal(mace(data)["forces"], out["forces"])
 
 
+# against the model's own autograd path (same bounds), what the oracle does not have: 16 basis functions, tabulated radial
+# weights (one element and several, the C = 128 and the narrower edge passes), and a list that crosses from eight warps a
+# receiver to one (1 184 receivers and channel chunks)
 @pytest.mark.parametrize("dtype,tol", [(torch.float64, 1e-10), (torch.float32, 1e-4)])
-def test_step_with_a_wider_basis(U, dtype, tol):
-    """16 basis functions (the oracle has 8): against the model's own autograd path."""
-    pos, ei, sh = _cluster(70, 3, 1.0)
-    species = torch.from_numpy(np.random.default_rng(4).integers(0, 3, 70)).to(torch.int32).cuda()
-    mace = model.InvariantMACE(systems.init_params(64, 3, 7, num_bessel=16), U, dtype=dtype, device="cuda")
+@pytest.mark.parametrize("n,C,Z,nb,radial", [(70, 64, 3, 16, "exact"), (50, 128, 3, 8, "spline"), (33, 96, 1, 8, "spline"),
+                                             (1300, 32, 2, 8, "spline")])
+def test_step_against_autograd(U, dtype, tol, n, C, Z, nb, radial):
+    pos, ei, sh = _cluster(n, 3, 1.0)
+    species = torch.from_numpy(np.random.default_rng(4).integers(0, Z, n)).to(torch.int32).cuda()
+    params = systems.init_params(C, Z, 7, num_bessel=nb)
+    if radial == "spline":
+        model.add_spline_knots(params)
+    mace = model.InvariantMACE(params, U, dtype=dtype, device="cuda", radial=radial)
+    assert step.plan_of(mace) is not None
     p = torch.from_numpy(pos).cuda()
     edges, shifts = torch.from_numpy(ei).to(torch.int32).cuda(), torch.from_numpy(sh).cuda()
     out = mace(dict(positions=p, species=species, edge_index=edges, shifts=shifts))
