@@ -101,6 +101,39 @@ __device__ __forceinline__ void store_vec_stream(T *p, const T (&src)[VEC]) {
   __stcs(reinterpret_cast<V *>(p), v);
 }
 
+// Programmatic dependent launch: a kernel launched by launch_chained() may be resident before its predecessor in the stream
+// has finished (launch latency, block scheduling and what stands before grid_wait() overlap the predecessor's last
+// blocks), so it reads and writes nothing before grid_wait(), which returns when the predecessor has completed and its
+// writes are visible.  grid_release() lets the successor's blocks come once every block of this grid has called it: a
+// kernel with tensor memory calls it after its allocation, or a successor's block could take the columns that a block of
+// this grid on the same SM still needs, and wait for that block.  Worth about 2 us a kernel in a chain of small ones.
+__device__ __forceinline__ void grid_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+__device__ __forceinline__ void grid_release() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+__device__ __forceinline__ void grid_begin() {
+  grid_wait();
+  grid_release();
+}
+// It is off unless the caller has switched it on for this thread: blocks that arrive early keep the SM's split between
+// shared memory and L1 as the predecessor had it, which costs kernels that live on L1 more than 2 us once they are long.
+inline bool &chain_launches() {
+  static thread_local bool on = false;
+  return on;
+}
+template <typename... Params, typename... Args>
+inline void launch_chained(void (*kernel)(Params...), dim3 grid, dim3 block, size_t smem, cudaStream_t st, Args &&...args) {
+  cudaLaunchAttribute attr;
+  attr.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr.val.programmaticStreamSerializationAllowed = 1;
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = grid;
+  cfg.blockDim = block;
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = st;
+  cfg.attrs = &attr;
+  cfg.numAttrs = chain_launches() ? 1 : 0;
+  cudaLaunchKernelEx(&cfg, kernel, Params(args)...);
+}
+
 // One thread of a converged warp, always the same one (elect.sync).  What it guards (tcgen05.mma, TMA and bulk copies) takes
 // uniform-register operands: under `lane == 0` the compiler does not know that a single thread is left and wraps every such
 // instruction in a loop over the lanes (a tcgen05.mma then costs 125-190 cycles to issue; elected, M = 128 with A in

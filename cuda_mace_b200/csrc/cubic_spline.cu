@@ -21,6 +21,7 @@ template <typename T, int VEC>
 __global__ void __launch_bounds__(128)
     spline_fwd_kernel(const T *__restrict__ r, const T *__restrict__ knots, const T *__restrict__ coeffs,
                       int64_t E, int nint, int nout, T h, T r_max, T *__restrict__ R) {
+  grid_begin();
   const int lane = threadIdx.x & 31;
   const int64_t e = (int64_t)blockIdx.x * 4 + (threadIdx.x >> 5);
   if (e >= E) return;
@@ -51,6 +52,7 @@ __global__ void __launch_bounds__(128)
     spline_bwd_kernel(const T *__restrict__ r, const T *__restrict__ knots, const T *__restrict__ coeffs,
                       const T *__restrict__ gR, int64_t E, int nint, int nout, T h, T r_max,
                       T *__restrict__ gr) {
+  grid_begin();
   const int lane = threadIdx.x & 31;
   const int64_t e = (int64_t)blockIdx.x * 4 + (threadIdx.x >> 5);
   if (e >= E) return;
@@ -94,9 +96,9 @@ static int spline_fwd(const T *r, const T *knots, const T *coeffs, int64_t E, in
   const unsigned grid = (unsigned)((E + 3) / 4);
   cudaStream_t st = (cudaStream_t)stream;
   if (nout % W == 0)
-    spline_fwd_kernel<T, W><<<grid, 128, 0, st>>>(r, knots, coeffs, E, nint, nout, (T)h, (T)r_max, R);
+    launch_chained(spline_fwd_kernel<T, W>, grid, 128, 0, st, r, knots, coeffs, E, nint, nout, (T)h, (T)r_max, R);
   else
-    spline_fwd_kernel<T, 1><<<grid, 128, 0, st>>>(r, knots, coeffs, E, nint, nout, (T)h, (T)r_max, R);
+    launch_chained(spline_fwd_kernel<T, 1>, grid, 128, 0, st, r, knots, coeffs, E, nint, nout, (T)h, (T)r_max, R);
   return check_launch("cmace_spline_fwd");
 }
 
@@ -111,9 +113,9 @@ static int spline_bwd(const T *r, const T *knots, const T *coeffs, const T *gR, 
   const unsigned grid = (unsigned)((E + 3) / 4);
   cudaStream_t st = (cudaStream_t)stream;
   if (nout % W == 0)
-    spline_bwd_kernel<T, W><<<grid, 128, 0, st>>>(r, knots, coeffs, gR, E, nint, nout, (T)h, (T)r_max, gr);
+    launch_chained(spline_bwd_kernel<T, W>, grid, 128, 0, st, r, knots, coeffs, gR, E, nint, nout, (T)h, (T)r_max, gr);
   else
-    spline_bwd_kernel<T, 1><<<grid, 128, 0, st>>>(r, knots, coeffs, gR, E, nint, nout, (T)h, (T)r_max, gr);
+    launch_chained(spline_bwd_kernel<T, 1>, grid, 128, 0, st, r, knots, coeffs, gR, E, nint, nout, (T)h, (T)r_max, gr);
   return check_launch("cmace_spline_bwd");
 }
 

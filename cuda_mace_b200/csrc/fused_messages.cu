@@ -235,6 +235,7 @@ __global__ void __launch_bounds__(FM_THREADS, 1)
     }
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
   }
+  grid_wait();
   if (tid <= FM_SETS) {
     const int64_t pieces = (int64_t)gridDim.x * FM_SETS, b = (int64_t)blockIdx.x * FM_SETS + tid;
     const int64_t per = (g.nedges + pieces - 1) / pieces;
@@ -244,6 +245,7 @@ __global__ void __launch_bounds__(FM_THREADS, 1)
   tc_fence_before();
   __syncthreads();
   tc_fence_after();
+  grid_release();   // after the allocation
   const uint32_t tmem = (uint32_t)uniform((int)tmem_base_slot), acc_t = tmem + 256u + 128u * (uint32_t)set;
   if (warp < 4) load_w_tmem(g.W, tmem, warp, lane);
   tc_fence_before();
@@ -366,7 +368,7 @@ int fused_messages(const float *X, const float *Y, const void *h, const void *W,
   if (e != cudaSuccess) return fail(CMACE_ERR_CUDA, "%s: %s", what, cudaGetErrorString(e));
   int64_t blocks = (nnodes + FM_SETS - 1) / FM_SETS;
   if (blocks > 148) blocks = 148;
-  fused_messages_kernel<<<(unsigned)blocks, FM_THREADS, smem, st>>>(g, map);
+  launch_chained(fused_messages_kernel, (unsigned)blocks, FM_THREADS, smem, st, g, map);
   return check_launch(what);
 }
 

@@ -168,10 +168,12 @@ __global__ void __launch_bounds__(EB_THREADS, 1)
     }
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
   }
+  grid_wait();
   if (warp == 8) tmem_alloc(smem_u32(&tmem_base_slot), 512);
   tc_fence_before();
   __syncthreads();
   tc_fence_after();
+  grid_release();   // after the allocation
   const uint32_t tmem = (uint32_t)uniform((int)tmem_base_slot);   // h buffer b at 128 b: h hi, h lo, h' hi, h' lo (32 each); acc b at 256 + 64 b
   const int64_t ntiles = (g.nedges + EB_TILE - 1) / EB_TILE;
 
@@ -466,7 +468,7 @@ int fused_messages_back(const float *X, const float *Y, const float *G, const vo
   if (int rc = encode_piece_tensor_map(&map, T, nedges, EB_C, what)) return rc;
   cudaError_t e = cudaFuncSetAttribute(edge_back_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, EB_SMEM);
   if (e != cudaSuccess) return fail(CMACE_ERR_CUDA, "%s: %s", what, cudaGetErrorString(e));
-  edge_back_kernel<<<(unsigned)(ntiles < 148 ? ntiles : 148), EB_THREADS, EB_SMEM, st>>>(g, map);
+  launch_chained(edge_back_kernel, (unsigned)(ntiles < 148 ? ntiles : 148), EB_THREADS, EB_SMEM, st, g, map);
   return check_launch(what);
 }
 

@@ -283,6 +283,7 @@ __global__ void __launch_bounds__((GT_PRODUCER_WARPS + 1 + EW + 1) * 32, 1)
   __shared__ uint32_t tmem_base_slot;
   __shared__ int32_t tab_words[MODE == GT_MODE_LINEAR ? sizeof(ProblemTable) / 4 : 1];
   const ProblemTable *tab = reinterpret_cast<const ProblemTable *>(tab_words);
+  grid_wait();
   if (MODE == GT_MODE_LINEAR) build_problem_table(g, reinterpret_cast<ProblemTable *>(tab_words));
 
   // dynamic smem base rounded up to 1024 bytes (the swizzle pattern repeats every 1024 bytes)
@@ -324,6 +325,7 @@ __global__ void __launch_bounds__((GT_PRODUCER_WARPS + 1 + EW + 1) * 32, 1)
   __syncthreads();
   tc_fence_after();
   const uint32_t tmem_base = (uint32_t)uniform((int)tmem_base_slot);
+  grid_release();   // after the allocation
 
   const int k_blocks = g.k_blocks;
   const uint32_t b_image = (uint32_t)g.npad * 128u;  // bytes of one B image
@@ -1521,7 +1523,7 @@ static int gemm_launch(GemmArgs &g, const char *what, cudaStream_t st) {
   }
   if (blocks < 1) return CMACE_OK;
   const int nthreads = g.mode == GT_MODE_GRADR ? (GT_PRODUCER_WARPS + 1 + 4 + 1) * 32 : GT_THREADS;
-  kern<<<(unsigned)blocks, nthreads, smem, st>>>(g, tmap, tmap_out, lin_maps);
+  launch_chained(kern, (unsigned)blocks, nthreads, smem, st, g, tmap, tmap_out, lin_maps);
   return check_launch(what);
 }
 

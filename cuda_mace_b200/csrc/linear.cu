@@ -20,6 +20,7 @@ __global__ void __launch_bounds__(LIN_THREADS)
     linear_tile_kernel(const T *__restrict__ X, const T *__restrict__ W,
                        const int32_t *__restrict__ node_order, const int32_t *__restrict__ elem_start,
                        int nelements, int64_t nnodes, int K, int Nout, T scale, T *__restrict__ out) {
+  grid_begin();
   __shared__ T As[KSTEP][TILE_M + 4];
   __shared__ T Bs[KSTEP][TILE_N];
   __shared__ int64_t row_of[TILE_M];
@@ -142,6 +143,7 @@ __global__ void __launch_bounds__(DM_THREADS, 2)
     linear_dmma_kernel(const double *__restrict__ X, const double *__restrict__ W,
                        const int32_t *__restrict__ node_order, const int32_t *__restrict__ elem_start,
                        int nelements, int64_t nnodes, int K, int Nout, double scale, double *__restrict__ out) {
+  grid_begin();
   extern __shared__ __align__(16) double dm_smem[];
   __shared__ int64_t row_of[TM];
 
@@ -277,7 +279,7 @@ static int dmma_launch(const double *X, const double *W, const int32_t *node_ord
   const int64_t tiles = PLAIN ? (nnodes + TM - 1) / TM : (nnodes * 7 + TM - 1) / TM + nelements;
   if (tiles > 0x7fffffffLL) return fail(CMACE_ERR_UNSUPPORTED, "%s: too many rows", what);
   const dim3 grid((unsigned)tiles, PLAIN ? 1 : 4, (unsigned)((Nout + TN - 1) / TN));
-  kern<<<grid, DM_THREADS, smem, st>>>(X, W, node_order, elem_start, nelements, nnodes, K, Nout, scale, out);
+  launch_chained(kern, grid, DM_THREADS, smem, st, X, W, node_order, elem_start, nelements, nnodes, K, Nout, scale, out);
   return check_launch(what);
 }
 
@@ -316,7 +318,7 @@ static int gemm_f64(const double *A, const double *B, int64_t M, int K, int N, d
   const int64_t tiles = (M + TILE_M - 1) / TILE_M;
   if (tiles > 0x7fffffffLL) return fail(CMACE_ERR_UNSUPPORTED, "cmace_gemm_f64: too many rows");
   dim3 grid((unsigned)tiles, 1, (unsigned)((N + TILE_N - 1) / TILE_N));
-  linear_tile_kernel<double, true><<<grid, LIN_THREADS, 0, (cudaStream_t)stream>>>(A, B, nullptr, nullptr, 1, M, K, N,
+  launch_chained(linear_tile_kernel<double, true>, grid, LIN_THREADS, 0, (cudaStream_t)stream, A, B, nullptr, nullptr, 1, M, K, N,
                                                                                    scale, out);
   return check_launch("cmace_gemm_f64");
 }
@@ -339,7 +341,7 @@ static int linear(const T *X, const T *W, const int32_t *node_order, const int32
   const int64_t max_tiles = (nnodes * 7 + TILE_M - 1) / TILE_M + nelements;
   if (max_tiles > 0x7fffffffLL) return fail(CMACE_ERR_UNSUPPORTED, "cmace_linear: too many rows");
   dim3 grid((unsigned)max_tiles, 4, (unsigned)((Nout + TILE_N - 1) / TILE_N));
-  linear_tile_kernel<T, false><<<grid, LIN_THREADS, 0, (cudaStream_t)stream>>>(
+  launch_chained(linear_tile_kernel<T, false>, grid, LIN_THREADS, 0, (cudaStream_t)stream, 
       X, W, node_order, elem_start, nelements, nnodes, K, Nout, (T)scale, out);
   return check_launch("cmace_linear");
 }

@@ -33,6 +33,7 @@ __global__ void __launch_bounds__(SPLIT == 1 ? kWarpsPerBlock * 32 : SPLIT * 32)
     imp_fwd_kernel(const T *__restrict__ X, const T *__restrict__ Y, const T *__restrict__ R,
                    const int32_t *__restrict__ sender, const int32_t *__restrict__ row_ptr,
                    int64_t nnodes, ImpLayout ys, int C, T *__restrict__ out) {
+  grid_begin();
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const int64_t node = SPLIT == 1 ? (int64_t)blockIdx.x * kWarpsPerBlock + warp : blockIdx.x;
   if (node >= nnodes) return;
@@ -148,6 +149,7 @@ __global__ void __launch_bounds__(kWarpsPerBlock * 32)
                         const T *__restrict__ G, const int32_t *__restrict__ sender,
                         const int32_t *__restrict__ row_ptr, int64_t nnodes, int64_t nedges, ImpLayout ys, int C,
                         int slices, T *__restrict__ gradR, T *__restrict__ gradY_out, T *__restrict__ Tout) {
+  grid_begin();
   const int lane = threadIdx.x & 31;
   // everything written is per edge: `slices` warps share a receiver, each takes every slices-th pair of its edges
   const int64_t item = (int64_t)blockIdx.x * kWarpsPerBlock + (threadIdx.x >> 5);
@@ -283,6 +285,7 @@ __global__ void __launch_bounds__(BS_WARPS * 32, 1)
                                const int32_t *__restrict__ row_ptr, int64_t nnodes, int64_t nedges, ImpLayout ys,
                                float *__restrict__ gradR, float *__restrict__ gy, float *__restrict__ Tout,
                                int *__restrict__ stalled) {
+  grid_begin();
   extern __shared__ __align__(128) unsigned char bs_smem[];
   __shared__ __align__(8) uint64_t bs_bars[BS_WARPS][BS_SLOTS];
   const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
@@ -452,6 +455,7 @@ __global__ void __launch_bounds__(BS_WARPS * 32, 1)
 template <typename T>
 __global__ void sum_partials_kernel(const T *__restrict__ partial, int nchunks, int64_t n,
                                     T *__restrict__ out) {
+  grid_begin();
   const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= n) return;
   T s = T(0);
@@ -464,6 +468,7 @@ __global__ void __launch_bounds__(SPLIT == 1 ? kWarpsPerBlock * 32 : SPLIT * 32)
     imp_bwd_node_kernel(const T *__restrict__ Tin, const int32_t *__restrict__ perm,
                         const int32_t *__restrict__ send_ptr, int64_t nnodes, int C,
                         T *__restrict__ gradX) {
+  grid_begin();
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const int64_t node = SPLIT == 1 ? (int64_t)blockIdx.x * kWarpsPerBlock + warp : blockIdx.x;
   if (node >= nnodes) return;
@@ -535,12 +540,12 @@ static void launch_fwd(const T *X, const T *Y, const T *R, const int32_t *sender
   if (few_nodes(nnodes * chunks)) {
     constexpr int smem = kSplit * 16 * 32 * VEC * (int)sizeof(T);
     cudaFuncSetAttribute(imp_fwd_kernel<T, VEC, kSplit>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
-    imp_fwd_kernel<T, VEC, kSplit><<<dim3((unsigned)nnodes, chunks), kSplit * 32, smem, st>>>(X, Y, R, sender, row_ptr, nnodes,
+    launch_chained(imp_fwd_kernel<T, VEC, kSplit>, dim3((unsigned)nnodes, chunks), kSplit * 32, smem, st, X, Y, R, sender, row_ptr, nnodes,
                                                                                               ys, C, out);
     return;
   }
   dim3 grid((unsigned)((nnodes + kWarpsPerBlock - 1) / kWarpsPerBlock), chunks);
-  imp_fwd_kernel<T, VEC, 1><<<grid, kWarpsPerBlock * 32, 0, st>>>(X, Y, R, sender, row_ptr, nnodes, ys, C, out);
+  launch_chained(imp_fwd_kernel<T, VEC, 1>, grid, kWarpsPerBlock * 32, 0, st, X, Y, R, sender, row_ptr, nnodes, ys, C, out);
 }
 
 template <typename T>
@@ -568,7 +573,7 @@ static void launch_bwd_edge(const T *X, const T *Y, const T *R, const T *G, cons
                             T *gy, T *Tout, cudaStream_t st) {
   const int slices = few_nodes(nnodes * (C / (32 * VEC))) ? kSplit : 1;
   dim3 grid((unsigned)((nnodes * slices + kWarpsPerBlock - 1) / kWarpsPerBlock), C / (32 * VEC));
-  imp_bwd_edge_kernel<T, VEC><<<grid, kWarpsPerBlock * 32, 0, st>>>(X, Y, R, G, sender, row_ptr,
+  launch_chained(imp_bwd_edge_kernel<T, VEC>, grid, kWarpsPerBlock * 32, 0, st, X, Y, R, G, sender, row_ptr,
                                                                      nnodes, nedges, ys, C, slices, gradR, gy, Tout);
 }
 
@@ -616,7 +621,7 @@ int imp_bwd_edge(const T *X, const T *Y, const T *R, const T *G, const int32_t *
       auto launch = [&](auto kernel) -> int {
         cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
         if (e != cudaSuccess) return fail(CMACE_ERR_CUDA, "cmace_imp_bwd_edge: %s", cudaGetErrorString(e));
-        kernel<<<(unsigned)blocks, BS_WARPS * 32, smem, st>>>(X, Y, R, G, sender, row_ptr, nnodes, nedges, ys, gradR, gy,
+        launch_chained(kernel, (unsigned)blocks, BS_WARPS * 32, smem, st, X, Y, R, G, sender, row_ptr, nnodes, nedges, ys, gradR, gy,
                                                               Tout, staged_stall_flag());
         return check_launch("cmace_imp_bwd_edge");
       };
@@ -638,7 +643,7 @@ int imp_bwd_edge(const T *X, const T *Y, const T *R, const T *G, const int32_t *
   if (rc) return rc;
   if (nchunks > 1) {
     const int64_t n = 16 * nedges;
-    sum_partials_kernel<T><<<(unsigned)((n + 255) / 256), 256, 0, st>>>(partial, nchunks, n, gradY);
+    launch_chained(sum_partials_kernel<T>, (unsigned)((n + 255) / 256), 256, 0, st, partial, nchunks, n, gradY);
     rc = check_launch("cmace_imp_bwd_edge(sum)");
   }
   return rc;
@@ -649,12 +654,12 @@ static void launch_bwd_node(const T *Tin, const int32_t *perm, const int32_t *se
                             int C, T *gradX, cudaStream_t st) {
   const int chunks = C / (32 * VEC);
   if (few_nodes(nnodes * chunks)) {
-    imp_bwd_node_kernel<T, VEC, kSplit><<<dim3((unsigned)nnodes, chunks), kSplit * 32, 0, st>>>(Tin, perm, send_ptr, nnodes, C,
+    launch_chained(imp_bwd_node_kernel<T, VEC, kSplit>, dim3((unsigned)nnodes, chunks), kSplit * 32, 0, st, Tin, perm, send_ptr, nnodes, C,
                                                                                               gradX);
     return;
   }
   dim3 grid((unsigned)((nnodes + kWarpsPerBlock - 1) / kWarpsPerBlock), chunks);
-  imp_bwd_node_kernel<T, VEC, 1><<<grid, kWarpsPerBlock * 32, 0, st>>>(Tin, perm, send_ptr, nnodes, C, gradX);
+  launch_chained(imp_bwd_node_kernel<T, VEC, 1>, grid, kWarpsPerBlock * 32, 0, st, Tin, perm, send_ptr, nnodes, C, gradX);
 }
 
 template <typename T>

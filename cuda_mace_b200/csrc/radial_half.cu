@@ -67,10 +67,12 @@ __global__ void __launch_bounds__(RQ_THREADS, 1)
     for (int i = 0; i < 5; i++) mbar_init(wbar + 8u * i, 1);
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
   }
+  grid_wait();
   if (warp == 0) tmem_alloc(smem_u32(&tmem_base_slot), 512);
   tc_fence_before();
   __syncthreads();
   tc_fence_after();
+  grid_release();   // after the allocation
   const uint32_t tmem0 = (uint32_t)uniform((int)tmem_base_slot) + (uint32_t)group * 256u;   // operand o: + 128 o; hi at + 64, lo at + 96
 
   if (warp == 0 && elect_one()) {
@@ -293,7 +295,7 @@ int radial_half(const float *basis, int nb, const void *const (*w)[3], const Rad
   if (blocks > 148 / nper) blocks = 148 / nper;
   cudaError_t e = cudaFuncSetAttribute(radial_half_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
   if (e != cudaSuccess) return fail(CMACE_ERR_CUDA, "%s: %s", what, cudaGetErrorString(e));
-  radial_half_kernel<<<(unsigned)(blocks * nper), RQ_THREADS, smem, st>>>(g, maps);
+  launch_chained(radial_half_kernel, (unsigned)(blocks * nper), RQ_THREADS, smem, st, g, maps);
   return check_launch(what);
 }
 

@@ -121,10 +121,12 @@ __global__ void __launch_bounds__(RT_THREADS, 1)
     for (int i = 0; i < 5; i++) mbar_init(wbar + 8u * i, 1);
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
   }
+  grid_wait();
   if (warp == 0) tmem_alloc(smem_u32(&tmem_base_slot), 512);
   tc_fence_before();
   __syncthreads();
   tc_fence_after();
+  grid_release();   // after the allocation
   const uint32_t tmem0 = (uint32_t)uniform((int)tmem_base_slot) + (uint32_t)(2 * group) * RT_TMEM_OP;   // + operand * RT_TMEM_OP
 
   if (warp == 0 && elect_one()) {
@@ -325,6 +327,7 @@ struct RadialPairArgs64 {
 };
 
 __global__ void __launch_bounds__(RD_WARPS * 32, 1) radial_pair_f64_kernel(const RadialPairArgs64 g) {
+  grid_begin();
   extern __shared__ __align__(16) double rd_smem[];
   __shared__ double etab[32];   // 2^(j/32)
   const int tid = threadIdx.x, warp = uniform(tid >> 5), lane = tid & 31;
@@ -414,7 +417,7 @@ int radial_pair_f32(const float *basis, int nb, const float *const (*w)[3], int 
   auto kern = nb == 8 ? radial_pair_kernel<2> : radial_pair_kernel<4>;
   cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
   if (e != cudaSuccess) return fail(CMACE_ERR_CUDA, "%s: %s", what, cudaGetErrorString(e));
-  kern<<<(unsigned)(blocks * nper), RT_THREADS, smem, st>>>(g, maps);
+  launch_chained(kern, (unsigned)(blocks * nper), RT_THREADS, smem, st, g, maps);
   return check_launch(what);
 }
 
@@ -435,7 +438,7 @@ int radial_pair_f64(const double *basis, int nb, const double *const (*w)[3], in
   if (blocks > 148 / nper) blocks = 148 / nper;
   cudaError_t e = cudaFuncSetAttribute(radial_pair_f64_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
   if (e != cudaSuccess) return fail(CMACE_ERR_CUDA, "%s: %s", what, cudaGetErrorString(e));
-  radial_pair_f64_kernel<<<(unsigned)(blocks * nper), RD_WARPS * 32, smem, st>>>(g);
+  launch_chained(radial_pair_f64_kernel, (unsigned)(blocks * nper), RD_WARPS * 32, smem, st, g);
   return check_launch(what);
 }
 

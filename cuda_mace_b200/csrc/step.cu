@@ -66,6 +66,7 @@ static const char *const kStepNames[S_COUNT] = {
 template <typename T>
 __global__ void __launch_bounds__(256)
     radial_dot_kernel(const T *__restrict__ gh, const T *__restrict__ dh, int64_t nedges, T *__restrict__ dr) {
+  grid_begin();
   const int64_t e = ((int64_t)blockIdx.x * 256 + threadIdx.x) >> 4;
   const int l16 = threadIdx.x & 15;
   T s = T(0);
@@ -289,7 +290,7 @@ static int run_step(const cmace_step_model &m, cmace_step_io &io, const Workspac
         io.launches--;
         return CMACE_OK;
       }
-      if (E > 0) radial_dot_kernel<T><<<(unsigned)((E + 15) / 16), 256, 0, st>>>(w.gH1, w.dh[1], E, w.dr1);
+      if (E > 0) launch_chained(radial_dot_kernel<T>, (unsigned)((E + 15) / 16), 256, 0, st, w.gH1, w.dh[1], E, w.dr1);
       return check_launch("cmace_step(radial_dot)");
     case S_SENDERS:
       if constexpr (f64) return cmace_imp_bwd_node_f64(w.T_, io.perm, io.send_ptr, nl, C, gup, st);
@@ -321,14 +322,21 @@ static int run_step(const cmace_step_model &m, cmace_step_io &io, const Workspac
   return fail(CMACE_ERR_ARG, "cmace_step: no step %d", step);
 }
 
+// Programmatic launches while the kernels are a few microseconds long: 163 -> 119 us a step at 5 000 edges, 277 -> 246 at
+// 52 000, 385 -> 356 at 83 000; at 156 000 a recorded step is slower with them (519 -> 532 us), and one with tabulated
+// radial weights, which live on L1, much slower (1030 -> 1145).
+constexpr int64_t kChainEdges = 98304;
+
 template <typename T>
 static int run_steps(const cmace_step_model &m, cmace_step_io &io, int first, int last, cudaStream_t st) {
   const Workspace<T> w(io.workspace, m, io.n_owned, io.n_local, io.nedges);
   if (io.workspace_bytes < w.bytes)
     return fail(CMACE_ERR_ARG, "cmace_step: workspace of %lld bytes, %lld needed", (long long)io.workspace_bytes, (long long)w.bytes);
-  for (int s = first; s < last; s++)
-    if (int rc = run_step<T>(m, io, w, s, st)) return rc;
-  return CMACE_OK;
+  chain_launches() = io.nedges <= (is_spline(m) ? kChainEdges / 2 : kChainEdges);
+  int rc = CMACE_OK;
+  for (int s = first; s < last && rc == CMACE_OK; s++) rc = run_step<T>(m, io, w, s, st);
+  chain_launches() = false;
+  return rc;
 }
 
 }  // namespace cmace

@@ -139,6 +139,7 @@ __global__ void __launch_bounds__(EP_THREADS)
                      const int32_t *species_in, const void *one_hot, int one_hot_f64, int64_t n_local, int64_t n_owned,
                      int elements, int32_t *species, int32_t *slot_of, int32_t *node_of, int32_t *slot_type,
                      int32_t *elem_start) {
+  grid_begin();
   if (blockIdx.x == 0) {
     group_nodes(species_in, one_hot, one_hot_f64, n_local, n_owned, elements, species, slot_of, node_of, slot_type,
                 elem_start);
@@ -187,7 +188,7 @@ int StepKernels<T>::edge_prep(const double *pos, const int32_t *sender, const in
   auto kern = nb == 16 ? edge_prep_kernel<T, 16> : (nb == 8 ? edge_prep_kernel<T, 8> : edge_prep_kernel<T, 0>);
   cudaError_t err = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
   if (err != cudaSuccess) return fail(CMACE_ERR_CUDA, "cmace_step(edge_prep): %s", cudaGetErrorString(err));
-  kern<<<(unsigned)blocks, EP_THREADS, smem, st>>>(pos, sender, receiver, shifts, nedges, (T)r_max, p, geo, basis, Y,
+  launch_chained(kern, (unsigned)blocks, EP_THREADS, smem, st, pos, sender, receiver, shifts, nedges, (T)r_max, p, geo, basis, Y,
                                                    species_in, one_hot, one_hot_f64, n_local, n_owned, elements, species,
                                                    slot_of, node_of, slot_type, elem_start);
   return check_launch("cmace_step(edge_prep)");
@@ -242,6 +243,7 @@ __global__ void __launch_bounds__(SU_WARPS * 32)
     sums_tf32_kernel(const float *__restrict__ h, const float *__restrict__ Y, const int32_t *__restrict__ sender,
                      const int32_t *__restrict__ row_ptr, const int32_t *__restrict__ species,
                      const int32_t *__restrict__ slot_of, int64_t nnodes, int elements, float *__restrict__ A) {
+  grid_begin();
   __shared__ int32_t lists[SU_WARPS][SU_LIST];
   const int lane = threadIdx.x & 31, w = threadIdx.x >> 5, g = lane >> 2, t = lane & 3;
   const int64_t pair = (int64_t)blockIdx.x * SU_WARPS + w;
@@ -322,6 +324,7 @@ __global__ void __launch_bounds__(SU_WARPS * 32)
                     const int32_t *__restrict__ row_ptr, const int32_t *__restrict__ species,
                     const int32_t *__restrict__ slot_of, int64_t nnodes, int elements, float factor,
                     float *__restrict__ A) {
+  grid_begin();
   __shared__ int32_t lists[SU_WARPS][SU_LIST];
   const int lane = threadIdx.x & 31, w = threadIdx.x >> 5, g = lane >> 2, t = lane & 3;
   const int64_t pair = (int64_t)blockIdx.x * SU_WARPS + w;
@@ -381,7 +384,7 @@ int step_sums_half(const void *h, const float *Y, const int32_t *sender, const i
                    const int32_t *slot_of, int64_t nnodes, int elements, float out_v, float *A, cudaStream_t st) {
   const int64_t blocks = (nnodes * elements + SU_WARPS - 1) / SU_WARPS;
   if (blocks > 0)
-    sums_f16_kernel<<<(unsigned)blocks, SU_WARPS * 32, 0, st>>>(static_cast<const uint4 *>(h), Y, sender, row_ptr, species,
+    launch_chained(sums_f16_kernel, (unsigned)blocks, SU_WARPS * 32, 0, st, static_cast<const uint4 *>(h), Y, sender, row_ptr, species,
                                                                slot_of, nnodes, elements, out_v / SU_Y_SCALE, A);
   return check_launch("cmace_step(sums)");
 }
@@ -409,6 +412,7 @@ __global__ void __launch_bounds__(SU_WARPS * 32)
     sums_f64_kernel(const double *__restrict__ h, const double *__restrict__ Y, const int32_t *__restrict__ sender,
                 const int32_t *__restrict__ row_ptr, const int32_t *__restrict__ species,
                 const int32_t *__restrict__ slot_of, int64_t nnodes, int elements, double *__restrict__ A) {
+  grid_begin();
   __shared__ int32_t lists[SU_WARPS][SU_LIST];
   const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
   const int64_t pair = (int64_t)blockIdx.x * SU_WARPS + w;
@@ -451,9 +455,9 @@ int StepKernels<T>::sums(const T *h, const T *Y, const int32_t *sender, const in
   const int64_t blocks = (nnodes * elements + SU_WARPS - 1) / SU_WARPS;
   if (blocks > 0) {
     if constexpr (sizeof(T) == 4)
-      sums_tf32_kernel<<<(unsigned)blocks, SU_WARPS * 32, 0, st>>>(h, Y, sender, row_ptr, species, slot_of, nnodes, elements, A);
+      launch_chained(sums_tf32_kernel, (unsigned)blocks, SU_WARPS * 32, 0, st, h, Y, sender, row_ptr, species, slot_of, nnodes, elements, A);
     else
-      sums_f64_kernel<<<(unsigned)blocks, SU_WARPS * 32, 0, st>>>(h, Y, sender, row_ptr, species, slot_of, nnodes, elements, A);
+      launch_chained(sums_f64_kernel, (unsigned)blocks, SU_WARPS * 32, 0, st, h, Y, sender, row_ptr, species, slot_of, nnodes, elements, A);
   }
   return check_launch("cmace_step(sums)");
 }
@@ -524,6 +528,7 @@ __global__ void __launch_bounds__(SU_WARPS * 32, 3)
                          const int32_t *__restrict__ slot_of, const float *__restrict__ gY1,
                          const float *__restrict__ dr1, const Quad<float> *__restrict__ geo, int64_t nnodes, int elements,
                          float *__restrict__ gvec) {
+  grid_begin();
   __shared__ int32_t lists[SU_WARPS][SU_LIST];
   __shared__ float stage[SU_WARPS][32 * 17];
   const int lane = threadIdx.x & 31, w = threadIdx.x >> 5, g = lane >> 2, t = lane & 3;
@@ -631,6 +636,7 @@ __global__ void __launch_bounds__(SU_WARPS * 32, 4)
                         const int32_t *__restrict__ slot_of, const float *__restrict__ gY1,
                         const float *__restrict__ dr1, const Quad<float> *__restrict__ geo, int64_t nnodes, int elements,
                         float out_v, float out_t, float *__restrict__ gvec) {
+  grid_begin();
   __shared__ int32_t lists[SU_WARPS][SU_LIST];
   __shared__ float stage[SU_WARPS][32 * 17];
   const int lane = threadIdx.x & 31, w = threadIdx.x >> 5, g = lane >> 2, t = lane & 3;
@@ -740,7 +746,7 @@ int step_sums_bwd_half(const float *gA, const void *h, const void *dh, const flo
                        float *gvec, cudaStream_t st) {
   const int64_t blocks = (nnodes * elements + SU_WARPS - 1) / SU_WARPS;
   if (blocks > 0)
-    sums_bwd_f16_kernel<<<(unsigned)blocks, SU_WARPS * 32, 0, st>>>(
+    launch_chained(sums_bwd_f16_kernel, (unsigned)blocks, SU_WARPS * 32, 0, st, 
         gA, static_cast<const uint4 *>(h), static_cast<const uint4 *>(dh), Y, sender, row_ptr, species, slot_of, gY1, dr1,
         geo, nnodes, elements, out_v, out_t, gvec);
   return check_launch("cmace_step(sums_back)");
@@ -773,6 +779,7 @@ __global__ void __launch_bounds__(SU_WARPS * 32)
                     const int32_t *__restrict__ species, const int32_t *__restrict__ slot_of,
                     const double *__restrict__ gY1, const double *__restrict__ dr1, const Quad<double> *__restrict__ geo,
                     int64_t nnodes, int elements, double *__restrict__ gvec) {
+  grid_begin();
   __shared__ int32_t lists[SU_WARPS][SU_LIST];
   __shared__ double stage[SU_WARPS][32 * 17];
   const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
@@ -832,10 +839,10 @@ int StepKernels<T>::sums_bwd(const T *gA, const T *h, const T *dh, const T *Y, c
   const int64_t blocks = (nnodes * elements + SU_WARPS - 1) / SU_WARPS;
   if (blocks > 0) {
     if constexpr (sizeof(T) == 4)
-      sums_bwd_tf32_kernel<<<(unsigned)blocks, SU_WARPS * 32, 0, st>>>(gA, h, dh, Y, sender, row_ptr, species, slot_of,
+      launch_chained(sums_bwd_tf32_kernel, (unsigned)blocks, SU_WARPS * 32, 0, st, gA, h, dh, Y, sender, row_ptr, species, slot_of,
                                                                       gY1, dr1, geo, nnodes, elements, gvec);
     else
-      sums_bwd_f64_kernel<<<(unsigned)blocks, SU_WARPS * 32, 0, st>>>(gA, h, dh, Y, sender, row_ptr, species, slot_of,
+      launch_chained(sums_bwd_f64_kernel, (unsigned)blocks, SU_WARPS * 32, 0, st, gA, h, dh, Y, sender, row_ptr, species, slot_of,
                                                                      gY1, dr1, geo, nnodes, elements, gvec);
   }
   return check_launch("cmace_step(sums_bwd)");
@@ -846,11 +853,12 @@ int StepKernels<T>::sums_bwd(const T *gA, const T *h, const T *dh, const T *Y, c
 __global__ void __launch_bounds__(256)
     sender_species_kernel(const int32_t *__restrict__ sender, const int32_t *__restrict__ species, int64_t nedges,
                           int32_t *__restrict__ out) {
+  grid_begin();
   const int64_t e = (int64_t)blockIdx.x * 256 + threadIdx.x;
   if (e < nedges) out[e] = species[sender[e]];
 }
 int step_sender_species(const int32_t *sender, const int32_t *species, int64_t nedges, int32_t *out, cudaStream_t st) {
-  if (nedges > 0) sender_species_kernel<<<(unsigned)((nedges + 255) / 256), 256, 0, st>>>(sender, species, nedges, out);
+  if (nedges > 0) launch_chained(sender_species_kernel, (unsigned)((nedges + 255) / 256), 256, 0, st, sender, species, nedges, out);
   return check_launch("cmace_step(sums)");
 }
 
@@ -859,6 +867,7 @@ template <typename T>
 __global__ void __launch_bounds__(256)
     edge_finish_kernel(const T *__restrict__ gY0, const T *__restrict__ dr0, const T *__restrict__ gY1,
                        const T *__restrict__ dr1, const Quad<T> *__restrict__ geo, int64_t nedges, T *__restrict__ gvec) {
+  grid_begin();
   const int64_t e = (int64_t)blockIdx.x * 256 + threadIdx.x;
   if (e >= nedges) return;
   T s[17];
@@ -878,7 +887,7 @@ template <typename T>
 int step_edge_finish(const T *gY0, const T *dr0, const T *gY1, const T *dr1, const Quad<T> *geo, int64_t nedges, T *gvec,
                      cudaStream_t st) {
   if (nedges > 0)
-    edge_finish_kernel<T><<<(unsigned)((nedges + 255) / 256), 256, 0, st>>>(gY0, dr0, gY1, dr1, geo, nedges, gvec);
+    launch_chained(edge_finish_kernel<T>, (unsigned)((nedges + 255) / 256), 256, 0, st, gY0, dr0, gY1, dr1, geo, nedges, gvec);
   return check_launch("cmace_step(sums_back)");
 }
 template int step_edge_finish<float>(const float *, const float *, const float *, const float *, const Quad<float> *, int64_t,
@@ -895,6 +904,7 @@ __global__ void __launch_bounds__(256)
                   const int32_t *__restrict__ send_ptr, int64_t nrecv, int64_t nsend, double sign,
                   double *__restrict__ out, const double *__restrict__ inter, const double *__restrict__ node_energy,
                   double *__restrict__ sums) {
+  grid_begin();
   const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
   if (blockIdx.x == 0) {
     __shared__ double part[2][8];
@@ -950,7 +960,7 @@ int StepKernels<T>::forces(const T *gvec, const int32_t *row_ptr, const int32_t 
                            int64_t nrecv, int64_t nsend, double sign, double *out, const double *inter,
                            const double *node_energy, double *sums, cudaStream_t st) {
   const int64_t blocks = 1 + (nsend + 7) / 8;
-  forces_kernel<T><<<(unsigned)blocks, 256, 0, st>>>(gvec, row_ptr, perm, send_ptr, nrecv, nsend, sign, out, inter,
+  launch_chained(forces_kernel<T>, (unsigned)blocks, 256, 0, st, gvec, row_ptr, perm, send_ptr, nrecv, nsend, sign, out, inter,
                                                      node_energy, sums);
   return check_launch("cmace_step(forces)");
 }

@@ -27,6 +27,7 @@ template <typename T, bool BWD>
 __global__ void __launch_bounds__(128, sizeof(T) == 4 ? 5 : 3)
     step_contract_kernel(const T *__restrict__ X, const int32_t *__restrict__ types, const T *__restrict__ weff,
                          const T *__restrict__ gb, int64_t nnodes, int C, T *__restrict__ out) {
+  grid_begin();
   const int c = blockIdx.y * blockDim.x + threadIdx.x;
   for (int64_t node = blockIdx.x; node < nnodes; node += gridDim.x) {
     T x[16], g[16], w3[canon::NCLASS3], w2[canon::NCLASS2], w1, value;
@@ -64,7 +65,7 @@ int StepKernels<T>::contract_fwd(const T *X, const int32_t *types, const T *weff
                                  cudaStream_t st) {
   const int ch = channel_block(C);
   if (n > 0)
-    step_contract_kernel<T, false><<<dim3((unsigned)node_blocks(n, 12), C / ch), ch, 0, st>>>(X, types, weff, nullptr, n, C, b);
+    launch_chained(step_contract_kernel<T, false>, dim3((unsigned)node_blocks(n, 12), C / ch), ch, 0, st, X, types, weff, nullptr, n, C, b);
   return check_launch("cmace_step(contract_fwd)");
 }
 template <typename T>
@@ -72,7 +73,7 @@ int StepKernels<T>::contract_bwd(const T *X, const int32_t *types, const T *weff
                                  cudaStream_t st) {
   const int ch = channel_block(C);
   if (n > 0)
-    step_contract_kernel<T, true><<<dim3((unsigned)node_blocks(n, 12), C / ch), ch, 0, st>>>(X, types, weff, gb, n, C, gX);
+    launch_chained(step_contract_kernel<T, true>, dim3((unsigned)node_blocks(n, 12), C / ch), ch, 0, st, X, types, weff, gb, n, C, gX);
   return check_launch("cmace_step(contract_bwd)");
 }
 
@@ -87,6 +88,7 @@ __global__ void __launch_bounds__(128, sizeof(T) == 4 ? 5 : 3)
                             const double *__restrict__ atomic_e, double scale, double shift, int64_t nnodes, int C,
                             T *__restrict__ gX, T *__restrict__ dq_out, double *__restrict__ inter,
                             double *__restrict__ node_energy) {
+  grid_begin();
   __shared__ T part[4][ST_RO];
   __shared__ T dq_s[ST_RO];
   const int c = threadIdx.x, lane = c & 31, w = c >> 5, nw = C >> 5;
@@ -160,7 +162,7 @@ int StepKernels<T>::contract_readout(const T *X, const int32_t *types, const T *
                                      const T *q0, const double *atomic_e, double scale, double shift, int64_t n, int C,
                                      T *gX, T *dq, double *inter, double *node_energy, cudaStream_t st) {
   if (n > 0)
-    contract_readout_kernel<T><<<(unsigned)node_blocks(n, 10), C, 0, st>>>(X, types, weff, wp1, w2, q0, atomic_e, scale,
+    launch_chained(contract_readout_kernel<T>, (unsigned)node_blocks(n, 10), C, 0, st, X, types, weff, wp1, w2, q0, atomic_e, scale,
                                                                           shift, n, C, gX, dq, inter, node_energy);
   return check_launch("cmace_step(contract_readout)");
 }
@@ -213,6 +215,7 @@ __global__ void __launch_bounds__(256)
     mid_fwd_kernel(const T *__restrict__ b, const int32_t *__restrict__ node_of, const int32_t *__restrict__ slot_type,
                    const T *__restrict__ wu, const T *__restrict__ extra, int64_t n, int C, T *__restrict__ up,
                    T *__restrict__ q0) {
+  grid_begin();
   extern __shared__ __align__(32) unsigned char mid_smem[];
   T *sW = reinterpret_cast<T *>(mid_smem), *rows = sW + C * C;
   constexpr int PER = NODES / 8;
@@ -254,6 +257,7 @@ __global__ void __launch_bounds__(256)
     mid_bwd_kernel(const T *__restrict__ gup, const int32_t *__restrict__ node_of, const int32_t *__restrict__ slot_type,
                    const T *__restrict__ dq, const T *__restrict__ wu_t, const T *__restrict__ extra_t, T scale,
                    int64_t n, int C, T *__restrict__ gb) {
+  grid_begin();
   extern __shared__ __align__(32) unsigned char mid_smem[];
   T *sW = reinterpret_cast<T *>(mid_smem), *rows = sW + C * C, *sdq = rows + NODES * C;
   constexpr int PER = NODES / 8;
@@ -304,8 +308,8 @@ static int launch_mid(const char *what, int64_t n, int C, Kernel8 k8, Kernel32 k
   cudaError_t e = small ? cudaFuncSetAttribute(k8, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem)
                         : cudaFuncSetAttribute(k32, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
   if (e != cudaSuccess) return fail(CMACE_ERR_CUDA, "%s: %s", what, cudaGetErrorString(e));
-  if (small) k8<<<(unsigned)blocks, 2 * C, smem, st>>>(args...);
-  else k32<<<(unsigned)blocks, 2 * C, smem, st>>>(args...);
+  if (small) launch_chained(k8, (unsigned)blocks, 2 * C, smem, st, args...);
+  else launch_chained(k32, (unsigned)blocks, 2 * C, smem, st, args...);
   return check_launch(what);
 }
 template <typename T>
