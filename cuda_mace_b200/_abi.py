@@ -28,7 +28,8 @@ class StepModel(ctypes.Structure):
 class StepIO(ctypes.Structure):
     """cmace_step_io of the header: one step's inputs, workspace and outputs."""
     _fields_ = [(k, _L) for k in ("n_owned", "n_local", "nedges")] + [
-        (k, _P) for k in ("positions", "shifts", "species", "one_hot")] + [
+        (k, _P) for k in ("positions", "shifts", "shift_index", "shift_table")] + [("shift_rows", _L), ("species", _P),
+        ("one_hot", _P)] + [
         ("one_hot_is_f64", ctypes.c_int32), ("launches", ctypes.c_int32)] + [
         (k, _P) for k in ("sender", "receiver", "row_ptr", "perm", "send_ptr", "up_local", "gup_local", "gup_owned",
                           "workspace")] + [
@@ -83,6 +84,9 @@ SIGNATURES = {
     "cmace_imp_radial_fused_fwd_f32": [_P, _P, _P, _P, _P, _P, _L, _L, _I, _I, _P, _P, _P, _P],
     "cmace_imp_staged_stalled": [],
     "cmace_nl_num_cells": [_D, _D, _D, _D],
+    "cmace_nl_workspace_bytes": [_L, _L, _D, _D, _D, _D],
+    "cmace_nl_build_f64": [_P, _L, _L, _D, _D, _D, _D, _D, _D, _I, _D, _P, _L, _P, _P],
+    "cmace_nl_emit_f64": [_P, _L, _L, _D, _D, _D, _D, _D, _D, _I, _D, _P, _P, _P, _P, _P, _P, _P],
     "cmace_nl_cell_ids_f64": [_P, _L, _D, _D, _D, _D, _D, _D, _I, _D, _P, _P],
     "cmace_nl_count_f64": [_P, _L, _L, _D, _D, _D, _D, _D, _D, _I, _D, _P, _P, _P, _P],
     "cmace_scan_workspace_bytes": [_L],
@@ -112,6 +116,7 @@ _RESTYPES = {
     "cmace_gemm_packed_floats": _L,
     "cmace_radial_hidden_saved_floats": _L,
     "cmace_nl_num_cells": _L,
+    "cmace_nl_workspace_bytes": _L,
     "cmace_scan_workspace_bytes": _L,
     "cmace_step_workspace_bytes": _L,
     "cmace_step_name": ctypes.c_char_p,
@@ -121,7 +126,7 @@ _RESTYPES = {
 # functions whose integer result is a value, not a status
 _VALUE_FUNCS = {"cmace_abi_version", "cmace_sender_order_workspace_bytes", "cmace_imp_bwd_scratch_elems",
                 "cmace_gemm_packed_floats", "cmace_imp_bwd_edge_f64_noalloc_max_elems",
-                "cmace_radial_hidden_saved_floats", "cmace_nl_num_cells", "cmace_scan_workspace_bytes",
+                "cmace_radial_hidden_saved_floats", "cmace_nl_num_cells", "cmace_nl_workspace_bytes", "cmace_scan_workspace_bytes",
                 "cmace_imp_staged_stalled", "cmace_step_workspace_bytes", "cmace_step_count", "cmace_step_struct_bytes", "cmace_step_name",
                 "cmace_symcon_plan_destroy", "cmace_symcon_plan_nterms", "cmace_symcon_plan_nclasses",
                 "cmace_symcon_plan_is_canonical", "cmace_symcon_plan_uses_program"}
@@ -138,7 +143,7 @@ KERNEL_LAUNCHES = {
     "cmace_imp_bwd_node": 1, "cmace_linear": 1, "cmace_symcon_fwd": 1, "cmace_symcon_bwd": 1,
     "cmace_gemm_pack_weights": 1, "cmace_gemm3x": 1, "cmace_gemm": 1, "cmace_gemm3x_gradr": 1, "cmace_bounded_wait_probe": 1, "cmace_linear_tc": 1,
     "cmace_radial_hidden_fwd": 1, "cmace_radial_hidden_bwd": 1, "cmace_imp_radial_fused_fwd": 1,
-    "cmace_symcon_effective_weights": 1, "cmace_symcon_apply": 1, "cmace_nl_cell_ids": 1, "cmace_nl_count": 1, "cmace_exclusive_scan_i32": 1, "cmace_nl_fill": 1,
+    "cmace_symcon_effective_weights": 1, "cmace_symcon_apply": 1, "cmace_nl_build": 4, "cmace_nl_emit": 1, "cmace_nl_cell_ids": 1, "cmace_nl_count": 1, "cmace_exclusive_scan_i32": 1, "cmace_nl_fill": 1,
 }
 launch_count = 0       # kernels launched through this binding since import
 _timing = None         # list of (name, start_event, end_event) while timing is on

@@ -578,7 +578,7 @@ static void launch_bwd_edge(const T *X, const T *Y, const T *R, const T *G, cons
 }
 
 static __device__ int g_staged_stall;   // set when a bounded wait of the staged edge pass gave up
-static int *staged_stall_flag() {
+int *staged_stall_flag() {
   static int *per_device[64] = {nullptr};
   int dev = 0;
   if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) return nullptr;

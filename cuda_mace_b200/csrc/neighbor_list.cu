@@ -68,11 +68,125 @@ __global__ void nl_cell_ids_kernel(const double *__restrict__ pos, int64_t natom
   cell_id[i] = (c[0] * g.ncell[1] + c[1]) * g.ncell[2] + c[2];
 }
 
+// An atom as the walk reads it: wrapped coordinates in cell order, so that a warp's candidates are consecutive and the
+// divisions of locate() are done once per atom instead of once per candidate.
+struct alignas(16) NlAtom {
+  double x, y, z;
+  int id, wrapped;   // wrapped: the atom lies outside the box (its lattice translations are recomputed for its edges)
+};
+
+__device__ __forceinline__ NlAtom nl_atom(const double *__restrict__ pos, const NlGeom &g, int id) {
+  NlAtom a;
+  int c, w, any = 0;
+  locate(g, 0, pos[3 * (int64_t)id], a.x, c, w);
+  any |= w;
+  locate(g, 1, pos[3 * (int64_t)id + 1], a.y, c, w);
+  any |= w;
+  locate(g, 2, pos[3 * (int64_t)id + 2], a.z, c, w);
+  any |= w;
+  a.id = id;
+  a.wrapped = any != 0;
+  return a;
+}
+
+__global__ void __launch_bounds__(256)
+    nl_atoms_kernel(const double *__restrict__ pos, int64_t natoms, const NlGeom g, const int32_t *__restrict__ perm,
+                    NlAtom *__restrict__ atoms) {
+  const int64_t k = (int64_t)blockIdx.x * 256 + threadIdx.x;
+  if (k < natoms) atoms[k] = nl_atom(pos, g, perm[k]);
+}
+
+// Binning of a small system in one block: counts, prefix sums and the atoms of every cell in index order (a cell's thread
+// sorts its few atoms: the order of atomics must not show in the edge list).
+constexpr int NL_SMALL_ATOMS = 8192, NL_SMALL_CELLS = 8192, NL_SMALL_THREADS = 1024;
+constexpr int NL_SMALL_SMEM = (NL_SMALL_ATOMS + NL_SMALL_CELLS + 33) * 4;
+
+// exclusive prefix over count[0 .. n) in shared memory, in place, by the whole block; returns the total
+__device__ int block_exclusive_scan(int32_t *count, int n, int32_t *warp_sums) {
+  const int tid = threadIdx.x, lane = tid & 31, w = tid >> 5, per = (n + NL_SMALL_THREADS - 1) / NL_SMALL_THREADS;
+  const int lo = tid * per < n ? tid * per : n, hi = lo + per < n ? lo + per : n;
+  int mine = 0;
+  for (int i = lo; i < hi; i++) mine += count[i];
+  int inc = mine;
+#pragma unroll
+  for (int off = 1; off < 32; off <<= 1) {
+    const int o = __shfl_up_sync(0xffffffffu, inc, off);
+    if (lane >= off) inc += o;
+  }
+  if (lane == 31) warp_sums[w] = inc;
+  __syncthreads();
+  if (w == 0) {
+    int v = warp_sums[lane], t = v;
+#pragma unroll
+    for (int off = 1; off < 32; off <<= 1) {
+      const int o = __shfl_up_sync(0xffffffffu, t, off);
+      if (lane >= off) t += o;
+    }
+    warp_sums[lane] = t - v;
+    if (lane == 31) warp_sums[32] = t;
+  }
+  __syncthreads();
+  int run = warp_sums[w] + inc - mine;
+  for (int i = lo; i < hi; i++) {
+    const int c = count[i];
+    count[i] = run;
+    run += c;
+  }
+  __syncthreads();
+  return warp_sums[32];
+}
+
+__global__ void __launch_bounds__(NL_SMALL_THREADS)
+    nl_bin_small_kernel(const double *__restrict__ pos, int natoms, int ncells, const NlGeom g,
+                        int32_t *__restrict__ cell_ptr, NlAtom *__restrict__ atoms) {
+  extern __shared__ int32_t nl_smem[];
+  int32_t *ids = nl_smem, *count = nl_smem + NL_SMALL_ATOMS, *sums = count + NL_SMALL_CELLS;
+  const int tid = threadIdx.x;
+  for (int c = tid; c < ncells; c += NL_SMALL_THREADS) count[c] = 0;
+  __syncthreads();
+  auto cell_of = [&](int i) {
+    int c[3], w;
+    double xw;
+    for (int d = 0; d < 3; d++) locate(g, d, pos[3 * (int64_t)i + d], xw, c[d], w);
+    return (c[0] * g.ncell[1] + c[1]) * g.ncell[2] + c[2];
+  };
+  for (int i = tid; i < natoms; i += NL_SMALL_THREADS) atomicAdd(&count[cell_of(i)], 1);
+  __syncthreads();
+  block_exclusive_scan(count, ncells, sums);
+  for (int c = tid; c <= ncells; c += NL_SMALL_THREADS) cell_ptr[c] = c < ncells ? count[c] : natoms;
+  __syncthreads();
+  for (int i = tid; i < natoms; i += NL_SMALL_THREADS) ids[atomicAdd(&count[cell_of(i)], 1)] = i;   // count: past-the-end now
+  __syncthreads();
+  for (int c = tid; c < ncells; c += NL_SMALL_THREADS) {
+    const int lo = c == 0 ? 0 : count[c - 1], hi = count[c];
+    for (int a = lo + 1; a < hi; a++) {
+      const int v = ids[a];
+      int b = a;
+      for (; b > lo && ids[b - 1] > v; b--) ids[b] = ids[b - 1];
+      ids[b] = v;
+    }
+  }
+  __syncthreads();
+  for (int k = tid; k < natoms; k += NL_SMALL_THREADS) atoms[k] = nl_atom(pos, g, ids[k]);
+}
+
+// exclusive prefix of up to a few ten thousand counts in one block, in place (n values, the last one becomes the total)
+__global__ void __launch_bounds__(NL_SMALL_THREADS) nl_scan_small_kernel(int32_t *__restrict__ v, int n) {
+  extern __shared__ int32_t nl_smem[];
+  int32_t *sums = nl_smem + n;
+  for (int i = threadIdx.x; i < n; i += NL_SMALL_THREADS) nl_smem[i] = v[i];
+  __syncthreads();
+  block_exclusive_scan(nl_smem, n, sums);
+  for (int i = threadIdx.x; i < n; i += NL_SMALL_THREADS) v[i] = nl_smem[i];
+}
+
 // One warp per receiver.  FILL = false: count[i] = number of neighbours; FILL = true: writes them at row_ptr[i].
+// The three cells along z are consecutive in cell order: one range of candidates unless the row meets the box's face.
+// atoms: in cell order, or null with perm (the caller's own sequence of calls).
 template <bool FILL>
 __global__ void __launch_bounds__(128)
-    nl_walk_kernel(const double *__restrict__ pos, int64_t nrecv, const NlGeom g, const int32_t *__restrict__ perm,
-                   const int32_t *__restrict__ cell_ptr, int32_t *__restrict__ count,
+    nl_walk_kernel(const double *__restrict__ pos, int64_t nrecv, const NlGeom g, const NlAtom *__restrict__ atoms,
+                   const int32_t *__restrict__ perm, const int32_t *__restrict__ cell_ptr, int32_t *__restrict__ count,
                    const int32_t *__restrict__ row_ptr, int32_t *__restrict__ sender, int32_t *__restrict__ receiver,
                    int8_t *__restrict__ shift_idx, double *__restrict__ shifts) {
   const int lane = threadIdx.x & 31;
@@ -83,9 +197,10 @@ __global__ void __launch_bounds__(128)
   for (int d = 0; d < 3; d++) locate(g, d, pos[3 * i + d], xi[d], ci[d], wi[d]);
   int64_t out = FILL ? (int64_t)row_ptr[i] : 0;
   int total = 0;
+  const bool inside = ci[2] > 0 && ci[2] + 1 < g.ncell[2];
   for (int dx = -1; dx <= 1; dx++)
     for (int dy = -1; dy <= 1; dy++)
-      for (int dz = -1; dz <= 1; dz++) {
+      for (int dz = inside ? 0 : -1; dz <= (inside ? 0 : 1); dz++) {
         const int dd[3] = {dx, dy, dz};
         int c[3], S[3];
         bool skip = false;
@@ -106,28 +221,32 @@ __global__ void __launch_bounds__(128)
         const int cf = (c[0] * g.ncell[1] + c[1]) * g.ncell[2] + c[2];
         const double sx = (double)S[0] * g.len[0], sy = (double)S[1] * g.len[1], sz = (double)S[2] * g.len[2];
         const bool same_image = S[0] == 0 && S[1] == 0 && S[2] == 0;
-        const int k0 = cell_ptr[cf], k1 = cell_ptr[cf + 1];
+        const int k0 = cell_ptr[inside ? cf - 1 : cf], k1 = cell_ptr[inside ? cf + 2 : cf + 1];
         for (int kb = k0; kb < k1; kb += 32) {
           const int k = kb + lane;
           bool hit = false;
-          int j = 0, wj[3] = {0, 0, 0};
+          NlAtom a;
           if (k < k1) {
-            j = perm[k];
-            double xj[3];
-            int cj;
-            for (int d = 0; d < 3; d++) locate(g, d, pos[3 * (int64_t)j + d], xj[d], cj, wj[d]);
+            a = atoms ? atoms[k] : nl_atom(pos, g, perm[k]);
             // (x_j + shift) - x_i, squared and summed in the order of the host list, without contraction
-            const double ddx = __dsub_rn(__dadd_rn(xj[0], sx), xi[0]);
-            const double ddy = __dsub_rn(__dadd_rn(xj[1], sy), xi[1]);
-            const double ddz = __dsub_rn(__dadd_rn(xj[2], sz), xi[2]);
+            const double ddx = __dsub_rn(__dadd_rn(a.x, sx), xi[0]);
+            const double ddy = __dsub_rn(__dadd_rn(a.y, sy), xi[1]);
+            const double ddz = __dsub_rn(__dadd_rn(a.z, sz), xi[2]);
             const double d2 = __dadd_rn(__dadd_rn(__dmul_rn(ddx, ddx), __dmul_rn(ddy, ddy)), __dmul_rn(ddz, ddz));
-            hit = d2 < g.rc2 && !(same_image && (int64_t)j == i);
+            hit = d2 < g.rc2 && !(same_image && (int64_t)a.id == i);
           }
           const unsigned m = __ballot_sync(0xffffffffu, hit);
           if (FILL && hit) {
             const int64_t e = out + __popc(m & ((1u << lane) - 1u));
-            sender[e] = j;
+            sender[e] = a.id;
             receiver[e] = (int32_t)i;
+            int wj[3] = {0, 0, 0};
+            if (a.wrapped)
+              for (int d = 0; d < 3; d++) {
+                double xw;
+                int cj;
+                locate(g, d, pos[3 * (int64_t)a.id + d], xw, cj, wj[d]);
+              }
             for (int d = 0; d < 3; d++) {
               const int s = S[d] - wj[d] + wi[d];
               if (shift_idx) shift_idx[3 * e + d] = (int8_t)s;
@@ -140,6 +259,12 @@ __global__ void __launch_bounds__(128)
       }
   if (!FILL && lane == 0) count[i] = total;
 }
+
+static bool nl_small(int64_t natoms, int64_t ncells) { return natoms <= NL_SMALL_ATOMS && ncells <= NL_SMALL_CELLS; }
+static int64_t nl_align(int64_t x) { return (x + 255) / 256 * 256; }
+// atoms in cell order, cell pointers, then (systems that do not fit one block) cell ids, their grouping and its workspace
+static int64_t nl_ws_atoms(int64_t n) { return nl_align(n * (int64_t)sizeof(NlAtom)); }
+static int64_t nl_ws_cells(int64_t ncells) { return nl_align((ncells + 1) * 4); }
 
 }  // namespace cmace
 
@@ -173,8 +298,74 @@ int cmace_nl_count_f64(const double *pos, int64_t natoms, int64_t nrecv, double 
   if (nrecv == 0) return CMACE_OK;
   if (!pos || !perm || !cell_ptr || !count) return fail(CMACE_ERR_ARG, "cmace_nl_count: null pointer");
   nl_walk_kernel<false><<<(unsigned)((nrecv + 3) / 4), 128, 0, (cudaStream_t)stream>>>(
-      pos, nrecv, g, perm, cell_ptr, count, nullptr, nullptr, nullptr, nullptr, nullptr);
+      pos, nrecv, g, nullptr, perm, cell_ptr, count, nullptr, nullptr, nullptr, nullptr, nullptr);
   return check_launch("cmace_nl_count");
+}
+
+int cmace_nl_fill_f64(const double *pos, int64_t natoms, int64_t nrecv, double lox, double loy, double loz, double lx,
+                      double ly, double lz, int pbc_mask, double r_cut, const int32_t *perm, const int32_t *cell_ptr,
+                      const int32_t *row_ptr, int32_t *sender, int32_t *receiver, int8_t *shift_idx, double *shifts,
+                      cmace_stream_t stream) {
+  NlGeom g;
+  if (int rc = make_geom(g, lox, loy, loz, lx, ly, lz, pbc_mask, r_cut, "cmace_nl_fill")) return rc;
+  if (natoms < 0 || nrecv < 0 || nrecv > natoms) return fail(CMACE_ERR_ARG, "cmace_nl_fill: bad size");
+  if (nrecv == 0) return CMACE_OK;
+  if (!pos || !perm || !cell_ptr || !row_ptr || !sender || !receiver)
+    return fail(CMACE_ERR_ARG, "cmace_nl_fill: null pointer");
+  nl_walk_kernel<true><<<(unsigned)((nrecv + 3) / 4), 128, 0, (cudaStream_t)stream>>>(
+      pos, nrecv, g, nullptr, perm, cell_ptr, nullptr, row_ptr, sender, receiver, shift_idx, shifts);
+  return check_launch("cmace_nl_fill");
+}
+
+int64_t cmace_nl_workspace_bytes(int64_t natoms, int64_t nrecv, double lx, double ly, double lz, double r_cut) {
+  const int64_t ncells = cmace_nl_num_cells(lx, ly, lz, r_cut);
+  if (ncells < 1 || natoms < 0 || nrecv < 0) return 0;
+  int64_t b = nl_ws_atoms(natoms) + nl_ws_cells(ncells) + nl_align(cmace_scan_workspace_bytes(nrecv + 1));
+  if (!nl_small(natoms, ncells)) b += 2 * nl_align(natoms * 4) + nl_align(cmace_sender_order_workspace_bytes(natoms));
+  return b;
+}
+
+int cmace_nl_build_f64(const double *pos, int64_t natoms, int64_t nrecv, double lox, double loy, double loz, double lx,
+                       double ly, double lz, int pbc_mask, double r_cut, void *workspace, int64_t workspace_bytes,
+                       int32_t *row_ptr, cmace_stream_t stream) {
+  NlGeom g;
+  if (int rc = make_geom(g, lox, loy, loz, lx, ly, lz, pbc_mask, r_cut, "cmace_nl_build")) return rc;
+  if (natoms < 0 || nrecv < 0 || nrecv > natoms || natoms > 0x7ffffff0LL) return fail(CMACE_ERR_ARG, "cmace_nl_build: bad size");
+  if (!workspace || !row_ptr || (natoms > 0 && !pos)) return fail(CMACE_ERR_ARG, "cmace_nl_build: null pointer");
+  if (workspace_bytes < cmace_nl_workspace_bytes(natoms, nrecv, lx, ly, lz, r_cut))
+    return fail(CMACE_ERR_ARG, "cmace_nl_build: workspace too small");
+  cudaStream_t st = (cudaStream_t)stream;
+  const int64_t ncells = (int64_t)g.ncell[0] * g.ncell[1] * g.ncell[2];
+  char *w = static_cast<char *>(workspace);
+  NlAtom *atoms = reinterpret_cast<NlAtom *>(w);
+  int32_t *cell_ptr = reinterpret_cast<int32_t *>(w + nl_ws_atoms(natoms));
+  char *scan_ws = w + nl_ws_atoms(natoms) + nl_ws_cells(ncells);
+  const int64_t scan_bytes = nl_align(cmace_scan_workspace_bytes(nrecv + 1));
+  cudaError_t e = cudaMemsetAsync(row_ptr, 0, (size_t)(nrecv + 1) * 4, st);
+  if (e != cudaSuccess) return fail(CMACE_ERR_CUDA, "cmace_nl_build: %s", cudaGetErrorString(e));
+  if (nrecv == 0) return CMACE_OK;
+  if (nl_small(natoms, ncells)) {
+    cudaFuncSetAttribute(nl_bin_small_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, NL_SMALL_SMEM);
+    nl_bin_small_kernel<<<1, NL_SMALL_THREADS, NL_SMALL_SMEM, st>>>(pos, (int)natoms, (int)ncells, g, cell_ptr, atoms);
+  } else {
+    char *more = scan_ws + scan_bytes;
+    int32_t *ids = reinterpret_cast<int32_t *>(more), *perm = reinterpret_cast<int32_t *>(more + nl_align(natoms * 4));
+    nl_cell_ids_kernel<<<(unsigned)((natoms + 255) / 256), 256, 0, st>>>(pos, natoms, g, ids);
+    if (int rc = cmace_sender_order(ids, natoms, ncells, perm, cell_ptr, more + 2 * nl_align(natoms * 4),
+                                    nl_align(cmace_sender_order_workspace_bytes(natoms)), stream))
+      return rc;
+    nl_atoms_kernel<<<(unsigned)((natoms + 255) / 256), 256, 0, st>>>(pos, natoms, g, perm, atoms);
+  }
+  nl_walk_kernel<false><<<(unsigned)((nrecv + 3) / 4), 128, 0, st>>>(pos, nrecv, g, atoms, nullptr, cell_ptr, row_ptr, nullptr,
+                                                                     nullptr, nullptr, nullptr, nullptr);
+  if (nrecv + 1 <= 16384) {   // one block; longer ones by cub's scan
+    const int smem = (int)(nrecv + 1 + 33) * 4;
+    cudaFuncSetAttribute(nl_scan_small_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (16384 + 33) * 4);
+    nl_scan_small_kernel<<<1, NL_SMALL_THREADS, smem, st>>>(row_ptr, (int)(nrecv + 1));
+    return check_launch("cmace_nl_build");
+  }
+  if (int rc = check_launch("cmace_nl_build")) return rc;
+  return cmace_exclusive_scan_i32(row_ptr, nrecv + 1, row_ptr, scan_ws, scan_bytes, stream);
 }
 
 int64_t cmace_scan_workspace_bytes(int64_t n) {
@@ -194,18 +385,19 @@ int cmace_exclusive_scan_i32(const int32_t *in, int64_t n, int32_t *out, void *w
   return check_launch("cmace_exclusive_scan");
 }
 
-int cmace_nl_fill_f64(const double *pos, int64_t natoms, int64_t nrecv, double lox, double loy, double loz, double lx,
-                      double ly, double lz, int pbc_mask, double r_cut, const int32_t *perm, const int32_t *cell_ptr,
-                      const int32_t *row_ptr, int32_t *sender, int32_t *receiver, int8_t *shift_idx, double *shifts,
-                      cmace_stream_t stream) {
+int cmace_nl_emit_f64(const double *pos, int64_t natoms, int64_t nrecv, double lox, double loy, double loz, double lx,
+                      double ly, double lz, int pbc_mask, double r_cut, const void *workspace, const int32_t *row_ptr,
+                      int32_t *sender, int32_t *receiver, int8_t *shift_idx, double *shifts, cmace_stream_t stream) {
   NlGeom g;
-  if (int rc = make_geom(g, lox, loy, loz, lx, ly, lz, pbc_mask, r_cut, "cmace_nl_fill")) return rc;
-  if (natoms < 0 || nrecv < 0 || nrecv > natoms) return fail(CMACE_ERR_ARG, "cmace_nl_fill: bad size");
+  if (int rc = make_geom(g, lox, loy, loz, lx, ly, lz, pbc_mask, r_cut, "cmace_nl_emit")) return rc;
+  if (natoms < 0 || nrecv < 0 || nrecv > natoms) return fail(CMACE_ERR_ARG, "cmace_nl_emit: bad size");
   if (nrecv == 0) return CMACE_OK;
-  if (!pos || !perm || !cell_ptr || !row_ptr || !sender || !receiver)
-    return fail(CMACE_ERR_ARG, "cmace_nl_fill: null pointer");
+  if (!pos || !workspace || !row_ptr || !sender || !receiver)
+    return fail(CMACE_ERR_ARG, "cmace_nl_emit: null pointer");
+  const char *w = static_cast<const char *>(workspace);
   nl_walk_kernel<true><<<(unsigned)((nrecv + 3) / 4), 128, 0, (cudaStream_t)stream>>>(
-      pos, nrecv, g, perm, cell_ptr, nullptr, row_ptr, sender, receiver, shift_idx, shifts);
-  return check_launch("cmace_nl_fill");
+      pos, nrecv, g, reinterpret_cast<const NlAtom *>(w), nullptr, reinterpret_cast<const int32_t *>(w + nl_ws_atoms(natoms)), nullptr,
+      row_ptr, sender, receiver, shift_idx, shifts);
+  return check_launch("cmace_nl_emit");
 }
 }

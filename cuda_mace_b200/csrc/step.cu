@@ -180,7 +180,8 @@ static int run_spline_step(const cmace_step_model &m, cmace_step_io &io, const W
   const ImpLayout slots{1, 16, w.slot_of};
   switch (step) {
     case S_EDGE_PREP:
-      return StepKernels<T>::edge_prep(io.positions, io.sender, io.receiver, io.shifts, E, m.r_max, 0, m.cutoff_p, w.geo,
+      return StepKernels<T>::edge_prep(io.positions, io.sender, io.receiver, io.shifts, io.shift_index, io.shift_table,
+                                       io.shift_rows, io.status, E, m.r_max, 0, m.cutoff_p, w.geo,
                                        w.basis, w.Y, io.species, io.one_hot, io.one_hot_is_f64, io.n_local, n, Z, w.species,
                                        w.slot_of, w.node_of, w.slot_type, w.elem_start, st);
     case S_RADIAL:
@@ -234,7 +235,8 @@ static int run_step(const cmace_step_model &m, cmace_step_io &io, const Workspac
   }
   switch (step) {
     case S_EDGE_PREP:
-      return K::edge_prep(io.positions, io.sender, io.receiver, io.shifts, E, m.r_max, m.nbessel, m.cutoff_p, w.geo,
+      return K::edge_prep(io.positions, io.sender, io.receiver, io.shifts, io.shift_index, io.shift_table,
+                                       io.shift_rows, io.status, E, m.r_max, m.nbessel, m.cutoff_p, w.geo,
                           w.basis, w.Y, io.species, io.one_hot, io.one_hot_is_f64, nl, n, Z, w.species, w.slot_of,
                           w.node_of, w.slot_type, w.elem_start, st);
     case S_RADIAL: {
@@ -317,7 +319,7 @@ static int run_step(const cmace_step_model &m, cmace_step_io &io, const Workspac
                          Z, w.gvec, st);
     case S_FORCES:
       return K::forces(w.gvec, io.row_ptr, io.perm, io.send_ptr, n, nl, io.gradient_sign, io.gradient, io.interaction,
-                       io.node_energy, io.sums, st);
+                       io.node_energy, io.status, f64 ? nullptr : staged_stall_flag(), io.sums, st);
   }
   return fail(CMACE_ERR_ARG, "cmace_step: no step %d", step);
 }
@@ -332,9 +334,12 @@ static int run_steps(const cmace_step_model &m, cmace_step_io &io, int first, in
   const Workspace<T> w(io.workspace, m, io.n_owned, io.n_local, io.nedges);
   if (io.workspace_bytes < w.bytes)
     return fail(CMACE_ERR_ARG, "cmace_step: workspace of %lld bytes, %lld needed", (long long)io.workspace_bytes, (long long)w.bytes);
-  chain_launches() = io.nedges <= (is_spline(m) ? kChainEdges / 2 : kChainEdges);
+  const bool chain = io.nedges <= (is_spline(m) ? kChainEdges / 2 : kChainEdges);
   int rc = CMACE_OK;
-  for (int s = first; s < last && rc == CMACE_OK; s++) rc = run_step<T>(m, io, w, s, st);
+  for (int s = first; s < last && rc == CMACE_OK; s++) {
+    chain_launches() = chain && (s > first || first == 0);   // a later range may follow the caller's wait for another stream
+    rc = run_step<T>(m, io, w, s, st);
+  }
   chain_launches() = false;
   return rc;
 }
@@ -363,7 +368,8 @@ int cmace_step_run(const cmace_step_model *m, cmace_step_io *io, int first, int 
     return fail(CMACE_ERR_ARG, "cmace_step: bad size");
   if (!io->positions || (!io->species && !io->one_hot) || !io->row_ptr || !io->send_ptr || !io->workspace ||
       !io->node_energy || !io->interaction || !io->sums || !io->gradient ||
-      (io->nedges > 0 && (!io->sender || !io->receiver || !io->perm)))
+      (io->nedges > 0 && (!io->sender || !io->receiver || !io->perm)) ||
+      (io->shift_index && (!io->shift_table || !io->status)))
     return fail(CMACE_ERR_ARG, "cmace_step: null pointer");
   if (io->n_local != io->n_owned && (!io->up_local || !io->gup_local || !io->gup_owned))
     return fail(CMACE_ERR_ARG, "cmace_step: ghost rows need the caller's node feature arrays");

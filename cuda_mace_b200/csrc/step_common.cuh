@@ -25,10 +25,15 @@ struct RadialScales {
   float in_v, in_t, z[3], a[3], t[3], out_v, out_t;
 };
 
+constexpr int32_t CMACE_STEP_BAD_SHIFT = 90;   // status: a row of the shift table that does not exist
+
+int *staged_stall_flag();   // message_passing.cu: device word of the staged edge pass, or null
+
 // launchers (one per kernel; every one checks its launch)
 template <typename T>
 struct StepKernels {
   static int edge_prep(const double *pos, const int32_t *sender, const int32_t *receiver, const double *shifts,
+                       const uint8_t *shift_index, const double *shift_table, int64_t shift_rows, int32_t *status,
                        int64_t nedges, double r_max, int nb, int p, Quad<T> *geo, T *basis, T *Y,
                        const int32_t *species_in, const void *one_hot, int one_hot_f64, int64_t n_local, int64_t n_owned,
                        int elements, int32_t *species, int32_t *slot_of, int32_t *node_of, int32_t *slot_type,
@@ -50,7 +55,7 @@ struct StepKernels {
                       int64_t nnodes, int elements, T *gvec, cudaStream_t st);
   static int forces(const T *gvec, const int32_t *row_ptr, const int32_t *perm, const int32_t *send_ptr, int64_t nrecv,
                     int64_t nsend, double sign, double *out, const double *inter, const double *node_energy,
-                    double *sums, cudaStream_t st);
+                    const int32_t *status, const int *stalled, double *sums, cudaStream_t st);
 };
 
 }  // namespace cmace

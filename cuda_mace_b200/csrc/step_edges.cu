@@ -134,7 +134,9 @@ __device__ __forceinline__ void store_rows(uint4 *buf, const T (&v)[N], T *__res
 template <typename T, int NB>
 __global__ void __launch_bounds__(EP_THREADS)
     edge_prep_kernel(const double *__restrict__ pos, const int32_t *__restrict__ sender,
-                     const int32_t *__restrict__ receiver, const double *__restrict__ shifts, int64_t nedges, T r_max,
+                     const int32_t *__restrict__ receiver, const double *__restrict__ shifts,
+                     const uint8_t *__restrict__ shift_index, const double *__restrict__ shift_table, int shift_rows,
+                     int32_t *status, int64_t nedges, T r_max,
                      int p, Quad<T> *__restrict__ geo, T *__restrict__ basis, T *__restrict__ Y,
                      const int32_t *species_in, const void *one_hot, int one_hot_f64, int64_t n_local, int64_t n_owned,
                      int elements, int32_t *species, int32_t *slot_of, int32_t *node_of, int32_t *slot_type,
@@ -154,11 +156,17 @@ __global__ void __launch_bounds__(EP_THREADS)
   const int rows = nedges - base < 32 ? (int)(nedges - base) : 32;
   const int64_t e = base + (lane < rows ? lane : rows - 1);
   const int64_t s = sender[e], r = receiver[e];
+  const double *sh = shifts ? shifts + e * 3 : nullptr;
+  if (shift_index) {
+    const int k = shift_index[e];
+    if (k < shift_rows) sh = shift_table + 3 * k;
+    else *status = CMACE_STEP_BAD_SHIFT;
+  }
   T v[3];
 #pragma unroll
   for (int c = 0; c < 3; c++) {
     double d = __dsub_rn(pos[s * 3 + c], pos[r * 3 + c]);
-    if (shifts) d = __dadd_rn(d, shifts[e * 3 + c]);
+    if (sh) d = __dadd_rn(d, sh[c]);
     v[c] = (T)d;
   }
   const T r2 = v[0] * v[0] + v[1] * v[1] + v[2] * v[2];
@@ -179,6 +187,7 @@ __global__ void __launch_bounds__(EP_THREADS)
 
 template <typename T>
 int StepKernels<T>::edge_prep(const double *pos, const int32_t *sender, const int32_t *receiver, const double *shifts,
+                              const uint8_t *shift_index, const double *shift_table, int64_t shift_rows, int32_t *status,
                               int64_t nedges, double r_max, int nb, int p, Quad<T> *geo, T *basis, T *Y,
                               const int32_t *species_in, const void *one_hot, int one_hot_f64, int64_t n_local,
                               int64_t n_owned, int elements, int32_t *species, int32_t *slot_of, int32_t *node_of,
@@ -188,9 +197,9 @@ int StepKernels<T>::edge_prep(const double *pos, const int32_t *sender, const in
   auto kern = nb == 16 ? edge_prep_kernel<T, 16> : (nb == 8 ? edge_prep_kernel<T, 8> : edge_prep_kernel<T, 0>);
   cudaError_t err = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
   if (err != cudaSuccess) return fail(CMACE_ERR_CUDA, "cmace_step(edge_prep): %s", cudaGetErrorString(err));
-  launch_chained(kern, (unsigned)blocks, EP_THREADS, smem, st, pos, sender, receiver, shifts, nedges, (T)r_max, p, geo, basis, Y,
-                                                   species_in, one_hot, one_hot_f64, n_local, n_owned, elements, species,
-                                                   slot_of, node_of, slot_type, elem_start);
+  launch_chained(kern, (unsigned)blocks, EP_THREADS, smem, st, pos, sender, receiver, shifts, shift_index, shift_table,
+                 (int)(shift_rows < 256 ? shift_rows : 256), status, nedges, (T)r_max, p, geo, basis, Y, species_in, one_hot,
+                 one_hot_f64, n_local, n_owned, elements, species, slot_of, node_of, slot_type, elem_start);
   return check_launch("cmace_step(edge_prep)");
 }
 
@@ -903,12 +912,13 @@ __global__ void __launch_bounds__(256)
     forces_kernel(const T *__restrict__ g, const int32_t *__restrict__ row_ptr, const int32_t *__restrict__ perm,
                   const int32_t *__restrict__ send_ptr, int64_t nrecv, int64_t nsend, double sign,
                   double *__restrict__ out, const double *__restrict__ inter, const double *__restrict__ node_energy,
-                  double *__restrict__ sums) {
+                  const int32_t *status, const int *stalled, double *__restrict__ sums) {
   grid_begin();
   const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
   if (blockIdx.x == 0) {
     __shared__ double part[2][8];
     double a = 0.0, b = 0.0;
+#pragma unroll 8   // one block: the loads in flight bound it
     for (int64_t i = threadIdx.x; i < nrecv; i += 256) {
       a += node_energy[i];
       b += inter[i];
@@ -928,6 +938,8 @@ __global__ void __launch_bounds__(256)
       for (int k = 0; k < 8; k++) s += part[threadIdx.x][k];
       sums[threadIdx.x] = s;
     }
+    // non-zero when a bounded wait of this step gave up: the caller reads it with the energies
+    if (threadIdx.x == 2) sums[2] = (double)((status ? *status : 0) | (stalled ? *stalled : 0));
     return;
   }
   const int64_t n = (int64_t)(blockIdx.x - 1) * 8 + w;
@@ -958,16 +970,17 @@ __global__ void __launch_bounds__(256)
 template <typename T>
 int StepKernels<T>::forces(const T *gvec, const int32_t *row_ptr, const int32_t *perm, const int32_t *send_ptr,
                            int64_t nrecv, int64_t nsend, double sign, double *out, const double *inter,
-                           const double *node_energy, double *sums, cudaStream_t st) {
+                           const double *node_energy, const int32_t *status, const int *stalled, double *sums,
+                           cudaStream_t st) {
   const int64_t blocks = 1 + (nsend + 7) / 8;
   launch_chained(forces_kernel<T>, (unsigned)blocks, 256, 0, st, gvec, row_ptr, perm, send_ptr, nrecv, nsend, sign, out, inter,
-                                                     node_energy, sums);
+                                                     node_energy, status, stalled, sums);
   return check_launch("cmace_step(forces)");
 }
 
 #define CMACE_STEP_EDGES(T)                                                                                         \
-  template int StepKernels<T>::edge_prep(const double *, const int32_t *, const int32_t *, const double *, int64_t, \
-                                         double, int, int, Quad<T> *, T *, T *, const int32_t *, const void *, int, \
+  template int StepKernels<T>::edge_prep(const double *, const int32_t *, const int32_t *, const double *,          \
+                                         const uint8_t *, const double *, int64_t, int32_t *, int64_t, double, int, int, Quad<T> *, T *, T *, const int32_t *, const void *, int, \
                                          int64_t, int64_t, int, int32_t *, int32_t *, int32_t *, int32_t *,         \
                                          int32_t *, cudaStream_t);                                                  \
   template int StepKernels<T>::sums(const T *, const T *, const int32_t *, const int32_t *, const int32_t *,        \
@@ -976,8 +989,8 @@ int StepKernels<T>::forces(const T *gvec, const int32_t *row_ptr, const int32_t 
                                         const int32_t *, const int32_t *, const int32_t *, const T *, const T *,    \
                                         const Quad<T> *, int64_t, int, T *, cudaStream_t);                          \
   template int StepKernels<T>::forces(const T *, const int32_t *, const int32_t *, const int32_t *, int64_t,        \
-                                      int64_t, double, double *, const double *, const double *, double *,          \
-                                      cudaStream_t);
+                                      int64_t, double, double *, const double *, const double *,                    \
+                                      const int32_t *, const int *, double *, cudaStream_t);
 CMACE_STEP_EDGES(float)
 CMACE_STEP_EDGES(double)
 

@@ -25,18 +25,32 @@ class EnergyForceEvaluator:
         self.plan = _domain.HaloPlan(dom, self.device, group).verify()
         self.species = None
         self.edge_index = None
-        self.shifts = None
+        self._shifts = None   # [E, 3], or (index, table) as a host batch carries them
         self.topology = None
         self._graph = None
 
     def set_neighbor_list(self, species, edge_index, shifts):
         """Device tensors: species [n_local] int32, edge_index [2,E] int32 (receivers sorted), shifts [E,3]."""
+        return self._set_list(species, edge_index, shifts)
+
+    def _set_list(self, species, edge_index, shifts, row_ptr=None):
         self.species = species.to(torch.int32).contiguous()
         self.edge_index = edge_index
-        self.shifts = shifts
-        self.topology = ops.EdgeTopology(edge_index[1], edge_index[0], self.dom.n_owned, self.dom.n_local)
+        self._shifts = shifts
+        self.topology = ops.EdgeTopology(edge_index[1], edge_index[0], self.dom.n_owned, self.dom.n_local, row_ptr)
         self._graph = None   # a captured step belongs to the list it was captured with
         return self
+
+    @property
+    def shifts(self):
+        if isinstance(self._shifts, tuple):
+            index, table = self._shifts
+            self._shifts = table.index_select(0, index.to(torch.int64))
+        return self._shifts
+
+    @shifts.setter
+    def shifts(self, value):
+        self._shifts = value
 
     def rebuild_neighbor_list(self, positions_owned, r_cut=None):
         """Builds the neighbour list of the current positions on the device (cell-list kernels) instead of taking
@@ -47,16 +61,18 @@ class EnergyForceEvaluator:
             raise RuntimeError("the domain does not carry its box")
         r_cut = float(self.model.r_max if r_cut is None else r_cut)
         with torch.no_grad():
-            pos_local = _domain.halo_exchange(positions_owned.detach(), self.plan) + self.plan.ghost_shift(positions_owned.dtype)
+            pos_local = positions_owned.detach()
+            if d.nranks > 1:
+                pos_local = _domain.halo_exchange(pos_local, self.plan) + self.plan.ghost_shift(pos_local.dtype)
         lo, ext = [0.0, 0.0, 0.0], [float(v) for v in d.box]
         for ax in range(3):
             if not d.pbc[ax]:
                 zmin, zmax = float(pos_local[:, ax].min()), float(pos_local[:, ax].max())
                 lo[ax], ext[ax] = zmin, max(zmax - zmin, 1e-6) * (1 + 1e-12) + 1e-9
-        edge_index, shifts, _ = ops.neighbor_list(pos_local, ext, d.pbc, r_cut, d.n_owned, lo=lo)
+        edge_index, shifts, _, row_ptr = ops.neighbor_list_rows(pos_local, ext, d.pbc, r_cut, d.n_owned, lo=lo)
         if self.species is None:
             self.species = torch.as_tensor(d.species, dtype=torch.int32, device=self.device)
-        return self.set_neighbor_list(self.species, edge_index, shifts.to(positions_owned.dtype))
+        return self._set_list(self.species, edge_index, shifts.to(positions_owned.dtype), row_ptr)
 
     def load_domain(self, pos_dtype=torch.float64):
         d = self.dom
@@ -96,10 +112,10 @@ class EnergyForceEvaluator:
             graph.replay()
             return energy.clone(), forces.clone()
 
-        if step.takes(positions_owned, self.shifts):
+        if step.takes(positions_owned, self._shifts):
             plan = step.plan_of(self.model)
             if plan is not None:
-                return self._evaluate_native(plan, positions_owned.detach())
+                return self._evaluate_native(plan, positions_owned.detach())[:2]
 
         def node_energy(pos_local, exchange):
             return self.model.node_energies(pos_local, self.species, self.edge_index, self.shifts,
@@ -108,18 +124,19 @@ class EnergyForceEvaluator:
         return _domain.distributed_energy_forces(node_energy, self.dom, self.plan, positions_owned)
 
     def _evaluate_native(self, plan, positions_owned):
-        """Total interaction energy over all ranks and forces on the owned atoms, by the library's own sequence."""
+        """Total interaction energy over all ranks, forces on the owned atoms and this rank's sums, by the library's
+        own sequence."""
         many = self.dom.nranks > 1
         pos = positions_owned
         if many:
             pos = self.plan.forward_fill(pos) + self.plan.ghost_shift(pos.dtype)
-        sums, _, _, forces = step.energy_forces(plan, pos, self.species, None, self.shifts, self.topology,
+        sums, _, _, forces = step.energy_forces(plan, pos, self.species, None, self._shifts, self.topology,
                                                 halo=self.plan if many else None)
         energy = sums[1]
         if many:
             energy = energy.clone()
             torch.distributed.all_reduce(energy, group=self.plan.group)
-        return energy, forces
+        return energy, forces, sums
 
     # ---- end-to-end path with host buffers ----------------------------------------------------
     def host_batch(self, pos_dtype=torch.float64):
@@ -148,13 +165,25 @@ class EnergyForceEvaluator:
     def evaluate_host(self, batch, out_forces=None):
         dev = self.device
         moved = {k: v.to(dev, non_blocking=True) for k, v in batch.items()}
-        shifts = moved["shifts"] if "shifts" in moved else \
-            moved["shift_table"].index_select(0, moved["shift_index"].to(torch.int64))
+        shifts = moved["shifts"] if "shifts" in moved else (moved["shift_index"], moved["shift_table"])
         self.set_neighbor_list(moved["species"], moved["edge_index"], shifts)
-        energy, forces = self(moved["positions"])
+        positions, plan, sums = moved["positions"], None, None
+        if step.takes(positions, shifts):
+            plan = step.plan_of(self.model)
+        if plan is not None:
+            energy, forces, sums = self._evaluate_native(plan, positions.detach())
+        else:
+            energy, forces = self(positions)
         if out_forces is None:
             out_forces = torch.empty(forces.shape, dtype=forces.dtype, pin_memory=torch.cuda.is_available())
         out_forces.copy_(forces, non_blocking=True)
-        e = float(energy.cpu())  # synchronises
-        ops.check_status()
-        return e, out_forces
+        if sums is None:
+            e = float(energy.cpu())  # synchronises
+            ops.check_status()
+            return e, out_forces
+        # energies and the record of failures in one copy, the step's only synchronisation
+        _, inter, failed = sums.tolist()
+        if failed:
+            ops.check_status()
+            raise RuntimeError("cuda_mace_b200: a kernel of the step recorded a failure")
+        return (inter if self.dom.nranks == 1 else float(energy)), out_forces

@@ -267,7 +267,7 @@ class EdgeTopology:
     once per neighbour list and reuse it for every layer and step.
     """
 
-    def __init__(self, sender, receiver, nnodes, nsenders=None):
+    def __init__(self, sender, receiver, nnodes, nsenders=None, row_ptr=None):
         _check_cuda(sender, receiver)
         self.sender = sender.to(torch.int32).contiguous()
         self.receiver = receiver.to(torch.int32).contiguous()
@@ -275,23 +275,38 @@ class EdgeTopology:
         # rows of the node-feature matrix the senders index; larger than nnodes when ghost atoms send
         self.nsenders = self.nnodes if nsenders is None else int(nsenders)
         self.nedges = int(self.sender.numel())
-        self.row_ptr = torch.empty(self.nnodes + 1, dtype=torch.int32, device=sender.device)
-        _abi.call("cmace_receiver_csr", _ptr(self.receiver), self.nedges, self.nnodes,
-                  _ptr(self.row_ptr), _stream())
+        self.row_ptr = row_ptr   # from the neighbour list that made it along with the edges
+        if row_ptr is None:
+            self.row_ptr = torch.empty(self.nnodes + 1, dtype=torch.int32, device=sender.device)
+            _abi.call("cmace_receiver_csr", _ptr(self.receiver), self.nedges, self.nnodes,
+                      _ptr(self.row_ptr), _stream())
         self._perm = None
         self._send_ptr = None
 
+    def _group_senders(self, stream=None):
+        dev = self.sender.device
+        nbytes = _abi.call("cmace_sender_order_workspace_bytes", self.nedges)
+        ws = torch.empty(max(int(nbytes), 1), dtype=torch.uint8, device=dev)
+        perm = torch.empty(max(self.nedges, 1), dtype=torch.int32, device=dev)
+        send_ptr = torch.empty(self.nsenders + 1, dtype=torch.int32, device=dev)
+        _abi.call("cmace_sender_order", _ptr(self.sender), self.nedges, self.nsenders, _ptr(perm),
+                  _ptr(send_ptr), _ptr(ws), int(nbytes), _stream() if stream is None else stream.cuda_stream)
+        return perm, send_ptr, ws
+
     def sender_order(self):
         if self._perm is None:
-            dev = self.sender.device
-            nbytes = _abi.call("cmace_sender_order_workspace_bytes", self.nedges)
-            ws = torch.empty(max(int(nbytes), 1), dtype=torch.uint8, device=dev)
-            perm = torch.empty(max(self.nedges, 1), dtype=torch.int32, device=dev)
-            send_ptr = torch.empty(self.nsenders + 1, dtype=torch.int32, device=dev)
-            _abi.call("cmace_sender_order", _ptr(self.sender), self.nedges, self.nsenders, _ptr(perm),
-                      _ptr(send_ptr), _ptr(ws), int(nbytes), _stream())
-            self._perm, self._send_ptr = perm, send_ptr
+            self._perm, self._send_ptr, _ = self._group_senders()
         return self._perm, self._send_ptr
+
+    def sender_order_beside(self, stream):
+        """Grouping by sender on `stream`, which follows the current one.  Returns (perm, send_ptr, workspace): the
+        caller has the current stream wait for `stream` before it reads the first two or drops any of them, and then
+        hands them to grouped()."""
+        stream.wait_stream(torch.cuda.current_stream(self.sender.device))
+        return self._group_senders(stream)
+
+    def grouped(self, perm, send_ptr):
+        self._perm, self._send_ptr = perm, send_ptr
 
 
 _topology_cache = _RefCache(8)
@@ -317,41 +332,35 @@ def neighbor_list(positions, box, pbc, r_cut, n_receivers=None, lo=(0.0, 0.0, 0.
     vector = pos[sender] - pos[receiver] + shift, and shift_index [E,3] int8 (shift = shift_index * box):
     the same list as cuda_mace_b200.systems.neighbor_list builds on the host.  One host synchronisation (the
     edge count) to size the outputs."""
+    return neighbor_list_rows(positions, box, pbc, r_cut, n_receivers, lo)[:3]
+
+
+def neighbor_list_rows(positions, box, pbc, r_cut, n_receivers=None, lo=(0.0, 0.0, 0.0)):
+    """neighbor_list() and the list's row_ptr [n_receivers + 1]."""
     _check_cuda(positions)
     pos = positions.detach().to(torch.float64).contiguous()
     dev = pos.device
     n = int(pos.shape[0])
     nrecv = n if n_receivers is None else int(n_receivers)
-    geom = [float(v) for v in lo] + [float(v) for v in box]
+    length = [float(v) for v in box]
     mask = sum(1 << d for d in range(3) if bool(pbc[d]))
+    geom = [float(v) for v in lo] + length + [mask, float(r_cut)]
     st = _stream()
-    i32 = dict(dtype=torch.int32, device=dev)
-    ncells = int(_abi.call("cmace_nl_num_cells", *geom[3:], float(r_cut)))
-    if ncells < 1:
-        raise RuntimeError("neighbor_list: bad box or cutoff")
-    cell_id = torch.empty(max(n, 1), **i32)
-    _abi.call("cmace_nl_cell_ids_f64", _ptr(pos), n, *geom, mask, float(r_cut), _ptr(cell_id), st)
-    nbytes = int(_abi.call("cmace_sender_order_workspace_bytes", n))
-    ws = torch.empty(max(nbytes, 1), dtype=torch.uint8, device=dev)
-    perm = torch.empty(max(n, 1), **i32)
-    cell_ptr = torch.empty(ncells + 1, **i32)
-    _abi.call("cmace_sender_order", _ptr(cell_id), n, ncells, _ptr(perm), _ptr(cell_ptr), _ptr(ws), nbytes, st)
-    count = torch.zeros(nrecv + 1, **i32)
-    _abi.call("cmace_nl_count_f64", _ptr(pos), n, nrecv, *geom, mask, float(r_cut), _ptr(perm), _ptr(cell_ptr),
-              _ptr(count), st)
-    row_ptr = torch.empty(nrecv + 1, **i32)
-    sbytes = int(_abi.call("cmace_scan_workspace_bytes", nrecv + 1))
-    sws = torch.empty(sbytes, dtype=torch.uint8, device=dev)
-    _abi.call("cmace_exclusive_scan_i32", _ptr(count), nrecv + 1, _ptr(row_ptr), _ptr(sws), sbytes, st)
+    nbytes = int(_abi.call("cmace_nl_workspace_bytes", n, nrecv, *length, float(r_cut)))
+    if nbytes < 1:
+        raise RuntimeError("neighbor_list: bad box, cutoff or number of receivers")
+    ws = torch.empty(nbytes, dtype=torch.uint8, device=dev)
+    row_ptr = torch.empty(nrecv + 1, dtype=torch.int32, device=dev)
+    _abi.call("cmace_nl_build_f64", _ptr(pos), n, nrecv, *geom, _ptr(ws), nbytes, _ptr(row_ptr), st)
     E = int(row_ptr[nrecv].item())
-    sender = torch.empty(E, **i32)
-    receiver = torch.empty(E, **i32)
+    edge_index = torch.empty(2, E, dtype=torch.int32, device=dev)
     shift_index = torch.empty(E, 3, dtype=torch.int8, device=dev)
     shifts = torch.empty(E, 3, dtype=torch.float64, device=dev)
     if E > 0:
-        _abi.call("cmace_nl_fill_f64", _ptr(pos), n, nrecv, *geom, mask, float(r_cut), _ptr(perm), _ptr(cell_ptr),
-                  _ptr(row_ptr), _ptr(sender), _ptr(receiver), _ptr(shift_index), _ptr(shifts), st)
-    return torch.stack([receiver, sender]), shifts, shift_index
+        p = edge_index.data_ptr()
+        _abi.call("cmace_nl_emit_f64", _ptr(pos), n, nrecv, *geom, _ptr(ws), _ptr(row_ptr), p + 4 * E, p,
+                  _ptr(shift_index), _ptr(shifts), st)
+    return edge_index, shifts, shift_index, row_ptr
 
 
 # --------------------------------------------------------------------------------------

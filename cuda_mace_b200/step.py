@@ -246,34 +246,64 @@ def plan_of(model):
 
 
 def takes(positions, shifts):
-    """Inputs the sequence takes: float64 positions and shifts on the current device."""
-    return positions.is_cuda and positions.dtype == torch.float64 and shifts.is_cuda and shifts.dtype == torch.float64
+    """Inputs the sequence takes: float64 positions (at least one) and shifts, or (index, table), on the device."""
+    if isinstance(shifts, tuple):
+        index, shifts = shifts
+        if not (index.is_cuda and index.dtype == torch.uint8):
+            return False
+    return (positions.is_cuda and positions.dtype == torch.float64 and positions.shape[0] > 0 and shifts.is_cuda
+            and shifts.dtype == torch.float64)
 
 
-_FIRST_EXCHANGE, _SECOND_EXCHANGE, _END = 6, 15, 20
+_FIRST_EXCHANGE, _SENDERS, _SECOND_EXCHANGE, _END = 6, 14, 15, 20
+_BESIDE_EDGES = 32768
+_side_streams = {}
+
+
+def _side_stream(device):
+    stream = _side_streams.get(device.index)
+    if stream is None:
+        stream = _side_streams.setdefault(device.index, torch.cuda.Stream(device=device))
+    return stream
 
 
 def energy_forces(plan, positions, species, one_hot, shifts, topology, halo=None):
-    """(sums [2], interaction [n_owned], node_energy [n_owned], forces): sums = (total energy, interaction energy).
+    """(sums [3], interaction [n_owned], node_energy [n_owned], forces): sums = (total energy, interaction energy,
+    0 unless a kernel recorded a failure: check_status() tells which).
 
-    positions [n_local, 3] float64, species [n_local] int32 or one_hot [n_local, Z].  `halo` (a HaloPlan of more than
+    shifts: [E, 3] float64, or (index [E] uint8, table [rows, 3] float64).  positions [n_local, 3] float64, species [n_local] int32 or one_hot [n_local, Z].  `halo` (a HaloPlan of more than
     one rank) fills and returns the ghost rows between the ranges of steps; forces are then those of the owned atoms."""
+    index = None
+    if isinstance(shifts, tuple):
+        index, shifts = shifts[0].contiguous(), shifts[1]
     ops._check_cuda(positions, shifts)
     positions, shifts = positions.contiguous(), shifts.contiguous()
     n, nl, E = topology.nnodes, topology.nsenders, topology.nedges
     dev = positions.device
-    if positions.shape != (nl, 3) or shifts.shape != (E, 3):
+    if positions.shape != (nl, 3) or shifts.shape[1:] != (3,) or (shifts if index is None else index).shape[0] != E:
         raise RuntimeError(f"shape mismatch: positions {tuple(positions.shape)}, shifts {tuple(shifts.shape)} for "
                            f"{nl} atoms and {E} edges")
-    out = torch.empty(2 + 2 * n + 3 * nl, dtype=torch.float64, device=dev)
+    out = torch.empty(3 + 2 * n + 3 * nl, dtype=torch.float64, device=dev)
     m = plan.model
     nbytes = _abi.call("cmace_step_workspace_bytes", ctypes.byref(m), n, nl, E)
     workspace = torch.empty(nbytes, dtype=torch.uint8, device=dev)
-    perm, send_ptr = topology.sender_order()
+    # A new list's grouping by sender is first read two thirds into the step: beside the steps before, once it takes
+    # longer (40 us at 160 000 edges) than the second stream costs the host (about 15 us).
+    beside = None
+    if topology._perm is None and E >= _BESIDE_EDGES and not torch.cuda.is_current_stream_capturing():
+        beside = _side_stream(dev)
+        grouping = topology.sender_order_beside(beside)
+        perm, send_ptr, _ = grouping
+    else:
+        perm, send_ptr = topology.sender_order()
     p = out.data_ptr()
     io = _abi.StepIO()
     io.n_owned, io.n_local, io.nedges = n, nl, E
-    io.positions, io.shifts = positions.data_ptr(), shifts.data_ptr()
+    io.positions = positions.data_ptr()
+    if index is None:
+        io.shifts = shifts.data_ptr()
+    else:
+        io.shift_index, io.shift_table, io.shift_rows = index.data_ptr(), shifts.data_ptr(), shifts.shape[0]
     if species is not None:
         io.species = species.data_ptr()
     else:
@@ -282,24 +312,48 @@ def energy_forces(plan, positions, species, one_hot, shifts, topology, halo=None
     io.perm, io.send_ptr = perm.data_ptr(), send_ptr.data_ptr()
     io.workspace, io.workspace_bytes = workspace.data_ptr(), nbytes
     io.status = ops._status_tensor(dev).data_ptr()
-    io.sums, io.interaction, io.node_energy, io.gradient = p, p + 16, p + 16 + 8 * n, p + 16 + 16 * n
+    io.sums, io.interaction, io.node_energy, io.gradient = p, p + 24, p + 24 + 8 * n, p + 24 + 16 * n
     io.gradient_sign = -1.0
     st = ops._stream()
-    forces = out[2 + 2 * n:].view(nl, 3)
+    forces = out[3 + 2 * n:].view(nl, 3)
+
+    def run(first, last):
+        nonlocal beside
+        if beside is not None and last > _SENDERS:
+            if first < _SENDERS:
+                _abi.run_steps(m, io, first, _SENDERS, st)
+                first = _SENDERS
+            join()
+        _abi.run_steps(m, io, first, last, st)
+
+    def join():
+        nonlocal beside
+        torch.cuda.current_stream(dev).wait_stream(beside)
+        beside = None
+        topology.grouped(perm, send_ptr)
+
+    try:
+        forces = _run_ranges(run, plan, n, nl, io, halo, forces)
+    finally:
+        if beside is not None:   # a failed step: the grouping still owns its memory
+            join()
+    return out[:3], out[3:3 + n], out[3 + n:3 + 2 * n], forces
+
+
+def _run_ranges(run, plan, n, nl, io, halo, forces):
     if halo is None:
-        _abi.run_steps(m, io, 0, _END, st)
-    else:
-        feats = dict(dtype=plan.dtype, device=dev)
-        up = torch.empty(n, plan.channels, **feats)
-        gup = torch.empty(nl, plan.channels, **feats)
-        # the ghost-row pointers are set before the first range: the call checks them together
-        io.up_local, io.gup_local, io.gup_owned = up.data_ptr(), gup.data_ptr(), gup.data_ptr()
-        _abi.run_steps(m, io, 0, _FIRST_EXCHANGE, st)
-        up_local = halo.forward_fill(up)
-        io.up_local = up_local.data_ptr()
-        _abi.run_steps(m, io, _FIRST_EXCHANGE, _SECOND_EXCHANGE, st)
-        gup_owned = halo.backward_reduce(gup)
-        io.gup_owned = gup_owned.data_ptr()
-        _abi.run_steps(m, io, _SECOND_EXCHANGE, _END, st)
-        forces = halo.backward_reduce(forces)
-    return out[:2], out[2:2 + n], out[2 + n:2 + 2 * n], forces
+        run(0, _END)
+        return forces
+    feats = dict(dtype=plan.dtype, device=forces.device)
+    up = torch.empty(n, plan.channels, **feats)
+    gup = torch.empty(nl, plan.channels, **feats)
+    # the ghost-row pointers are set before the first range: the call checks them together
+    io.up_local, io.gup_local, io.gup_owned = up.data_ptr(), gup.data_ptr(), gup.data_ptr()
+    run(0, _FIRST_EXCHANGE)
+    up_local = halo.forward_fill(up)
+    io.up_local = up_local.data_ptr()
+    run(_FIRST_EXCHANGE, _SECOND_EXCHANGE)
+    gup_owned = halo.backward_reduce(gup)
+    io.gup_owned = gup_owned.data_ptr()
+    run(_SECOND_EXCHANGE, _END)
+    return halo.backward_reduce(forces)

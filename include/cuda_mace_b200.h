@@ -70,6 +70,15 @@ int cmace_group_by_element(const int32_t *elem, int64_t nnodes, int nelements, i
  *   4. cmace_exclusive_scan_i32 over count[0..nrecv] (count[nrecv] = 0) -> row_ptr [nrecv+1]; E = row_ptr[nrecv]
  *   5. cmace_nl_fill_f64                -> sender [E], receiver [E], shift_idx [E,3] int8 and/or shifts [E,3]
  * row_ptr is the receiver CSR cmace_imp_* take.  The edges of a receiver come out in a fixed order. */
+/* The same in two calls with a workspace of cmace_nl_workspace_bytes: build (binning, counts, row_ptr [nrecv+1]), then,
+ * once E = row_ptr[nrecv] is known, emit. */
+int64_t cmace_nl_workspace_bytes(int64_t natoms, int64_t nrecv, double lx, double ly, double lz, double r_cut);
+int cmace_nl_build_f64(const double *pos, int64_t natoms, int64_t nrecv, double lox, double loy, double loz, double lx,
+                       double ly, double lz, int pbc_mask, double r_cut, void *workspace, int64_t workspace_bytes,
+                       int32_t *row_ptr, cmace_stream_t stream);
+int cmace_nl_emit_f64(const double *pos, int64_t natoms, int64_t nrecv, double lox, double loy, double loz, double lx,
+                      double ly, double lz, int pbc_mask, double r_cut, const void *workspace, const int32_t *row_ptr,
+                      int32_t *sender, int32_t *receiver, int8_t *shift_idx, double *shifts, cmace_stream_t stream);
 int64_t cmace_nl_num_cells(double lx, double ly, double lz, double r_cut);
 int cmace_nl_cell_ids_f64(const double *pos, int64_t natoms, double lox, double loy, double loz, double lx,
                           double ly, double lz, int pbc_mask, double r_cut, int32_t *cell_id,
@@ -390,7 +399,10 @@ typedef struct cmace_step_model {
 typedef struct cmace_step_io {
   int64_t n_owned, n_local, nedges; /* receivers, sender rows (owned first), edges */
   const double *positions;          /* [n_local, 3] */
-  const double *shifts;             /* [nedges, 3] or NULL */
+  const double *shifts;             /* [nedges, 3], or NULL: */
+  const uint8_t *shift_index;       /* [nedges] rows of shift_table [.., 3], or NULL: no shifts */
+  const double *shift_table;        /* [shift_rows, 3]; an index beyond it is recorded in *status */
+  int64_t shift_rows;
   const int32_t *species;           /* [n_local], or NULL with one_hot [n_local, elements] */
   const void *one_hot;
   int32_t one_hot_is_f64, launches; /* launches: kernels launched so far, added to by the call */
@@ -402,7 +414,7 @@ typedef struct cmace_step_io {
   int64_t workspace_bytes;
   int32_t *status;                  /* written by bounded waits that give up */
   double *node_energy, *interaction; /* [n_owned] */
-  double *sums;                     /* [2]: sum of node_energy, sum of interaction */
+  double *sums;                     /* [3]: sum of node_energy, sum of interaction, and what the status words held */
   double *gradient;                 /* [n_local, 3]: gradient_sign times the position gradient */
   double gradient_sign;
 } cmace_step_io;

@@ -564,6 +564,24 @@ def test_device_neighbor_list_equals_host_list(name, n_atoms, pbc, dev):
         assert float(v.norm(dim=1).max()) < 5.0 if v.numel() else True
 
 
+@pytest.mark.parametrize("n,side", [(1, 12.0), (8192, 95.0), (8193, 95.0), (8000, 105.0), (16383, 110.0), (16384, 110.0)])
+def test_device_neighbor_list_where_its_kernels_change(n, side, dev):
+    """Binning in one block up to 8 192 atoms and cells, the scan in one block up to 16 384 values; atoms outside the
+    box (by whole box lengths, so every distance stays what it is but for its last bits)."""
+    import numpy as np
+
+    from cuda_mace_b200 import ops, systems
+
+    rng = np.random.default_rng(n)
+    pos, box = rng.random((n, 3)) * side, np.full(3, side)
+    ei_h, sh_h = systems.neighbor_list(pos, box, (True, True, True), 5.0)
+    w = rng.integers(-1, 2, (n, 3))
+    si_h = np.rint(sh_h / box).astype(np.int64) - w[ei_h[1]] + w[ei_h[0]]
+    ei_d, _, si_d = ops.neighbor_list(torch.from_numpy(pos + w * box).to(dev), box, (True, True, True), 5.0)
+    assert bool((ei_d[0, 1:] >= ei_d[0, :-1]).all())
+    assert torch.equal(_edge_keys(ei_d, si_d), _edge_keys(torch.from_numpy(ei_h), torch.from_numpy(si_h)))
+
+
 def test_device_neighbor_list_without_atoms_or_edges(dev):
     from cuda_mace_b200 import ops
 

@@ -3,7 +3,7 @@ import numpy as np
 import pytest
 import torch
 
-from cuda_mace_b200 import model, step, systems
+from cuda_mace_b200 import domain, evaluator, model, step, systems
 from oracle import model as omodel
 
 pytestmark = pytest.mark.gpu
@@ -68,3 +68,29 @@ def test_step_against_autograd(U, dtype, tol, n, C, Z, nb, radial):
     p.requires_grad_(True)
     (g,) = torch.autograd.grad(mace.node_energies(p, species, edges, shifts).sum(), p)
     assert float((out["forces"] + g).abs().max()) < tol * float(g.abs().max())
+
+
+# below and above the 32 768 edges from which a new list's grouping by sender runs beside the step
+@pytest.mark.parametrize("n", [300, 1100])
+def test_new_list_and_host_batch(U, n):
+    side = (n / 0.1) ** (1.0 / 3.0)
+    pos, species = systems.random_box(n, np.full(3, side), 0.9, 5), np.zeros(n, dtype=np.int64)
+    dom = domain.partition_slabs(pos, species, np.full(3, side), 1, 5.0, 0)
+    mace = model.InvariantMACE(systems.init_params(64, 1, 7), U, dtype=torch.float64, device="cuda")
+    ev = evaluator.EnergyForceEvaluator(mace, dom, "cuda")
+    p = ev.load_domain()
+    assert (dom.edge_index.shape[1] >= step._BESIDE_EDGES) == (n > 1000)
+    ev.topology.sender_order()          # grouped before the step
+    e, f = ev(p)
+    batch = ev.host_batch()
+    e_host, f_host = ev.evaluate_host(batch)
+    # the same edges in the same order: the same bits
+    assert e_host == float(e) and torch.equal(f_host, f.cpu())
+    assert torch.equal(ev.shifts.cpu(), torch.from_numpy(dom.shifts))
+    ev.rebuild_neighbor_list(p)
+    e_new, f_new = ev(p)                # another order of the edges: float64 rounding over about 50 edges a node
+    assert abs(float(e_new - e)) < 1e-12 * n and float((f_new - f).abs().max()) < 1e-11 * float(f.abs().max())
+    batch["shift_table"] = batch["shift_table"][:1]
+    with pytest.raises(RuntimeError):
+        ev.evaluate_host(batch)
+    assert torch.equal(ev.rebuild_neighbor_list(p)(p)[1], f_new)   # the device goes on
