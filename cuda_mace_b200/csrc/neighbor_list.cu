@@ -50,8 +50,9 @@ static int make_geom(NlGeom &g, double lox, double loy, double loz, double lx, d
 __device__ __forceinline__ void locate(const NlGeom &g, int d, double x, double &xw, int &c, int &w) {
   w = 0;
   xw = x;
-  if (g.pbc[d]) {
-    w = (int)floor((x - g.lo[d]) / g.len[d]);
+  const double t = x - g.lo[d];
+  if (g.pbc[d] && !(t >= 0.0 && t < g.len[d])) {   // inside, the quotient rounds below one: no division needed
+    w = (int)floor(t / g.len[d]);
     if (w != 0) xw = x - (double)w * g.len[d];
   }
   int ci = (int)floor((xw - g.lo[d]) / g.cell[d]);
@@ -96,10 +97,11 @@ __global__ void __launch_bounds__(256)
   if (k < natoms) atoms[k] = nl_atom(pos, g, perm[k]);
 }
 
-// Binning of a small system in one block: counts, prefix sums and the atoms of every cell in index order (a cell's thread
-// sorts its few atoms: the order of atomics must not show in the edge list).
+// Binning of a small system in one block: counts, prefix sums and the atoms of every cell in index order (an atom counts
+// the smaller indices of its cell: the order of atomics must not show in the edge list).  Bound by the latency of its
+// phases; the grouping by radix sort that larger systems take costs five launches.
 constexpr int NL_SMALL_ATOMS = 8192, NL_SMALL_CELLS = 8192, NL_SMALL_THREADS = 1024;
-constexpr int NL_SMALL_SMEM = (NL_SMALL_ATOMS + NL_SMALL_CELLS + 33) * 4;
+constexpr int NL_SMALL_SMEM = (NL_SMALL_ATOMS + NL_SMALL_CELLS + 33) * 4 + NL_SMALL_ATOMS * 2;
 
 // exclusive prefix over count[0 .. n) in shared memory, in place, by the whole block; returns the total
 __device__ int block_exclusive_scan(int32_t *count, int n, int32_t *warp_sums) {
@@ -141,33 +143,31 @@ __global__ void __launch_bounds__(NL_SMALL_THREADS)
                         int32_t *__restrict__ cell_ptr, NlAtom *__restrict__ atoms) {
   extern __shared__ int32_t nl_smem[];
   int32_t *ids = nl_smem, *count = nl_smem + NL_SMALL_ATOMS, *sums = count + NL_SMALL_CELLS;
+  uint16_t *cells = reinterpret_cast<uint16_t *>(sums + 33);
   const int tid = threadIdx.x;
   for (int c = tid; c < ncells; c += NL_SMALL_THREADS) count[c] = 0;
   __syncthreads();
-  auto cell_of = [&](int i) {
+  for (int i = tid; i < natoms; i += NL_SMALL_THREADS) {
     int c[3], w;
     double xw;
     for (int d = 0; d < 3; d++) locate(g, d, pos[3 * (int64_t)i + d], xw, c[d], w);
-    return (c[0] * g.ncell[1] + c[1]) * g.ncell[2] + c[2];
-  };
-  for (int i = tid; i < natoms; i += NL_SMALL_THREADS) atomicAdd(&count[cell_of(i)], 1);
+    const int cell = (c[0] * g.ncell[1] + c[1]) * g.ncell[2] + c[2];
+    cells[i] = (uint16_t)cell;
+    atomicAdd(&count[cell], 1);
+  }
   __syncthreads();
   block_exclusive_scan(count, ncells, sums);
   for (int c = tid; c <= ncells; c += NL_SMALL_THREADS) cell_ptr[c] = c < ncells ? count[c] : natoms;
   __syncthreads();
-  for (int i = tid; i < natoms; i += NL_SMALL_THREADS) ids[atomicAdd(&count[cell_of(i)], 1)] = i;   // count: past-the-end now
+  for (int i = tid; i < natoms; i += NL_SMALL_THREADS) ids[atomicAdd(&count[cells[i]], 1)] = i;   // count: the cell's end now
   __syncthreads();
-  for (int c = tid; c < ncells; c += NL_SMALL_THREADS) {
-    const int lo = c == 0 ? 0 : count[c - 1], hi = count[c];
-    for (int a = lo + 1; a < hi; a++) {
-      const int v = ids[a];
-      int b = a;
-      for (; b > lo && ids[b - 1] > v; b--) ids[b] = ids[b - 1];
-      ids[b] = v;
-    }
+  for (int i = tid; i < natoms; i += NL_SMALL_THREADS) {
+    const int c = cells[i], lo = c == 0 ? 0 : count[c - 1], hi = count[c];
+    int k = lo;
+#pragma unroll 4
+    for (int a = lo; a < hi; a++) k += ids[a] < i;
+    atoms[k] = nl_atom(pos, g, i);
   }
-  __syncthreads();
-  for (int k = tid; k < natoms; k += NL_SMALL_THREADS) atoms[k] = nl_atom(pos, g, ids[k]);
 }
 
 // exclusive prefix of up to a few ten thousand counts in one block, in place (n values, the last one becomes the total)
@@ -180,83 +180,112 @@ __global__ void __launch_bounds__(NL_SMALL_THREADS) nl_scan_small_kernel(int32_t
   for (int i = threadIdx.x; i < n; i += NL_SMALL_THREADS) v[i] = nl_smem[i];
 }
 
-// One warp per receiver.  FILL = false: count[i] = number of neighbours; FILL = true: writes them at row_ptr[i].
-// The three cells along z are consecutive in cell order: one range of candidates unless the row meets the box's face.
-// atoms: in cell order, or null with perm (the caller's own sequence of calls).
+// One warp per receiver.  FILL = false: count[i] = number of neighbours; FILL = true: writes them at row_ptr[i].  Lane c
+// looks up the range of cell c of the 27; the ranges are then walked as one sequence, four candidates a lane at a time:
+// the walk is bound by the latency of its dependent loads, and 27 short loops had one load in flight each (17 and 20 us
+// at 3 000 receivers).  atoms: in cell order, or null with perm (the caller's own sequence of calls).
+constexpr int NL_AHEAD = 4;
+
 template <bool FILL>
 __global__ void __launch_bounds__(128)
     nl_walk_kernel(const double *__restrict__ pos, int64_t nrecv, const NlGeom g, const NlAtom *__restrict__ atoms,
                    const int32_t *__restrict__ perm, const int32_t *__restrict__ cell_ptr, int32_t *__restrict__ count,
                    const int32_t *__restrict__ row_ptr, int32_t *__restrict__ sender, int32_t *__restrict__ receiver,
                    int8_t *__restrict__ shift_idx, double *__restrict__ shifts) {
-  const int lane = threadIdx.x & 31;
-  const int64_t i = (int64_t)blockIdx.x * 4 + (threadIdx.x >> 5);
+  __shared__ int32_t first[4][28], base[4][28];   // position of a cell's first candidate in the sequence; its place in atoms
+  __shared__ int8_t image[4][28][4];
+  const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+  const int64_t i = (int64_t)blockIdx.x * 4 + w;
   if (i >= nrecv) return;
   double xi[3];
   int ci[3], wi[3];
   for (int d = 0; d < 3; d++) locate(g, d, pos[3 * i + d], xi[d], ci[d], wi[d]);
-  int64_t out = FILL ? (int64_t)row_ptr[i] : 0;
-  int total = 0;
-  const bool inside = ci[2] > 0 && ci[2] + 1 < g.ncell[2];
-  for (int dx = -1; dx <= 1; dx++)
-    for (int dy = -1; dy <= 1; dy++)
-      for (int dz = inside ? 0 : -1; dz <= (inside ? 0 : 1); dz++) {
-        const int dd[3] = {dx, dy, dz};
-        int c[3], S[3];
-        bool skip = false;
-        for (int d = 0; d < 3; d++) {
-          int cc = ci[d] + dd[d];
-          S[d] = 0;
-          if (cc < 0 || cc >= g.ncell[d]) {
-            if (!g.pbc[d]) {
-              skip = true;
-            } else {
-              S[d] = cc < 0 ? -1 : 1;
-              cc -= S[d] * g.ncell[d];
-            }
-          }
-          c[d] = cc;
-        }
-        if (skip) continue;
-        const int cf = (c[0] * g.ncell[1] + c[1]) * g.ncell[2] + c[2];
-        const double sx = (double)S[0] * g.len[0], sy = (double)S[1] * g.len[1], sz = (double)S[2] * g.len[2];
-        const bool same_image = S[0] == 0 && S[1] == 0 && S[2] == 0;
-        const int k0 = cell_ptr[inside ? cf - 1 : cf], k1 = cell_ptr[inside ? cf + 2 : cf + 1];
-        for (int kb = k0; kb < k1; kb += 32) {
-          const int k = kb + lane;
-          bool hit = false;
-          NlAtom a;
-          if (k < k1) {
-            a = atoms ? atoms[k] : nl_atom(pos, g, perm[k]);
-            // (x_j + shift) - x_i, squared and summed in the order of the host list, without contraction
-            const double ddx = __dsub_rn(__dadd_rn(a.x, sx), xi[0]);
-            const double ddy = __dsub_rn(__dadd_rn(a.y, sy), xi[1]);
-            const double ddz = __dsub_rn(__dadd_rn(a.z, sz), xi[2]);
-            const double d2 = __dadd_rn(__dadd_rn(__dmul_rn(ddx, ddx), __dmul_rn(ddy, ddy)), __dmul_rn(ddz, ddz));
-            hit = d2 < g.rc2 && !(same_image && (int64_t)a.id == i);
-          }
-          const unsigned m = __ballot_sync(0xffffffffu, hit);
-          if (FILL && hit) {
-            const int64_t e = out + __popc(m & ((1u << lane) - 1u));
-            sender[e] = a.id;
-            receiver[e] = (int32_t)i;
-            int wj[3] = {0, 0, 0};
-            if (a.wrapped)
-              for (int d = 0; d < 3; d++) {
-                double xw;
-                int cj;
-                locate(g, d, pos[3 * (int64_t)a.id + d], xw, cj, wj[d]);
-              }
-            for (int d = 0; d < 3; d++) {
-              const int s = S[d] - wj[d] + wi[d];
-              if (shift_idx) shift_idx[3 * e + d] = (int8_t)s;
-              if (shifts) shifts[3 * e + d] = (double)s * g.len[d];
-            }
-          }
-          out += __popc(m);
-          total += __popc(m);
+  int k0 = 0, length = 0;
+  if (lane < 27) {
+    const int dd[3] = {lane / 9 - 1, lane / 3 % 3 - 1, lane % 3 - 1};
+    int c[3];
+    bool skip = false;
+    for (int d = 0; d < 3; d++) {
+      int cc = ci[d] + dd[d], S = 0;
+      if (cc < 0 || cc >= g.ncell[d]) {
+        if (!g.pbc[d]) {
+          skip = true;
+          cc = ci[d];
+        } else {
+          S = cc < 0 ? -1 : 1;
+          cc -= S * g.ncell[d];
         }
       }
+      c[d] = cc;
+      image[w][lane][d] = (int8_t)S;
+    }
+    const int cf = (c[0] * g.ncell[1] + c[1]) * g.ncell[2] + c[2];
+    k0 = cell_ptr[cf];
+    length = skip ? 0 : cell_ptr[cf + 1] - k0;
+  }
+  int inc = length;
+#pragma unroll
+  for (int off = 1; off < 32; off <<= 1) {
+    const int o = __shfl_up_sync(0xffffffffu, inc, off);
+    if (lane >= off) inc += o;
+  }
+  if (lane < 28) {   // lane 27: the end of the sequence
+    first[w][lane] = inc - length;
+    base[w][lane] = k0;
+  }
+  __syncwarp();
+  const int all = __shfl_sync(0xffffffffu, inc, 31);
+  int64_t out = FILL ? (int64_t)row_ptr[i] : 0;
+  int total = 0, cell = 0;
+  for (int t0 = 0; t0 < all; t0 += 32 * NL_AHEAD) {
+    NlAtom a[NL_AHEAD];
+    int from[NL_AHEAD];
+#pragma unroll
+    for (int u = 0; u < NL_AHEAD; u++) {
+      const int t = t0 + u * 32 + lane;
+      from[u] = -1;
+      if (t < all) {
+        while (t >= first[w][cell + 1]) cell++;   // ends: first[27] = all
+        from[u] = cell;
+        const int k = base[w][cell] + t - first[w][cell];
+        a[u] = atoms ? atoms[k] : nl_atom(pos, g, perm[k]);
+      }
+    }
+#pragma unroll
+    for (int u = 0; u < NL_AHEAD; u++) {
+      bool hit = false;
+      int S[3] = {0, 0, 0};
+      if (from[u] >= 0) {
+        for (int d = 0; d < 3; d++) S[d] = image[w][from[u]][d];
+        // (x_j + shift) - x_i, squared and summed in the order of the host list, without contraction
+        const double ddx = __dsub_rn(__dadd_rn(a[u].x, (double)S[0] * g.len[0]), xi[0]);
+        const double ddy = __dsub_rn(__dadd_rn(a[u].y, (double)S[1] * g.len[1]), xi[1]);
+        const double ddz = __dsub_rn(__dadd_rn(a[u].z, (double)S[2] * g.len[2]), xi[2]);
+        const double d2 = __dadd_rn(__dadd_rn(__dmul_rn(ddx, ddx), __dmul_rn(ddy, ddy)), __dmul_rn(ddz, ddz));
+        hit = d2 < g.rc2 && !(S[0] == 0 && S[1] == 0 && S[2] == 0 && (int64_t)a[u].id == i);
+      }
+      const unsigned m = __ballot_sync(0xffffffffu, hit);
+      if (FILL && hit) {
+        const int64_t e = out + __popc(m & ((1u << lane) - 1u));
+        sender[e] = a[u].id;
+        receiver[e] = (int32_t)i;
+        int wj[3] = {0, 0, 0};
+        if (a[u].wrapped)
+          for (int d = 0; d < 3; d++) {
+            double xw;
+            int cj;
+            locate(g, d, pos[3 * (int64_t)a[u].id + d], xw, cj, wj[d]);
+          }
+        for (int d = 0; d < 3; d++) {
+          const int s = S[d] - wj[d] + wi[d];
+          if (shift_idx) shift_idx[3 * e + d] = (int8_t)s;
+          if (shifts) shifts[3 * e + d] = (double)s * g.len[d];
+        }
+      }
+      out += __popc(m);
+      total += __popc(m);
+    }
+  }
   if (!FILL && lane == 0) count[i] = total;
 }
 

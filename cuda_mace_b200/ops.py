@@ -283,27 +283,26 @@ class EdgeTopology:
         self._perm = None
         self._send_ptr = None
 
-    def _group_senders(self, stream=None):
+    def grouping_buffers(self):
+        """(perm, send_ptr, workspace) for group_senders()."""
         dev = self.sender.device
-        nbytes = _abi.call("cmace_sender_order_workspace_bytes", self.nedges)
-        ws = torch.empty(max(int(nbytes), 1), dtype=torch.uint8, device=dev)
+        nbytes = int(_abi.call("cmace_sender_order_workspace_bytes", self.nedges))
+        ws = torch.empty(max(nbytes, 1), dtype=torch.uint8, device=dev)
         perm = torch.empty(max(self.nedges, 1), dtype=torch.int32, device=dev)
         send_ptr = torch.empty(self.nsenders + 1, dtype=torch.int32, device=dev)
-        _abi.call("cmace_sender_order", _ptr(self.sender), self.nedges, self.nsenders, _ptr(perm),
-                  _ptr(send_ptr), _ptr(ws), int(nbytes), _stream() if stream is None else stream.cuda_stream)
         return perm, send_ptr, ws
+
+    def group_senders(self, buffers, stream):
+        perm, send_ptr, ws = buffers
+        _abi.call("cmace_sender_order", _ptr(self.sender), self.nedges, self.nsenders, _ptr(perm),
+                  _ptr(send_ptr), _ptr(ws), ws.numel(), stream)
 
     def sender_order(self):
         if self._perm is None:
-            self._perm, self._send_ptr, _ = self._group_senders()
+            buffers = self.grouping_buffers()
+            self.group_senders(buffers, _stream())
+            self.grouped(*buffers[:2])
         return self._perm, self._send_ptr
-
-    def sender_order_beside(self, stream):
-        """Grouping by sender on `stream`, which follows the current one.  Returns (perm, send_ptr, workspace): the
-        caller has the current stream wait for `stream` before it reads the first two or drops any of them, and then
-        hands them to grouped()."""
-        stream.wait_stream(torch.cuda.current_stream(self.sender.device))
-        return self._group_senders(stream)
 
     def grouped(self, perm, send_ptr):
         self._perm, self._send_ptr = perm, send_ptr

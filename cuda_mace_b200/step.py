@@ -288,12 +288,14 @@ def energy_forces(plan, positions, species, one_hot, shifts, topology, halo=None
     nbytes = _abi.call("cmace_step_workspace_bytes", ctypes.byref(m), n, nl, E)
     workspace = torch.empty(nbytes, dtype=torch.uint8, device=dev)
     # A new list's grouping by sender is first read two thirds into the step: beside the steps before, once it takes
-    # longer (40 us at 160 000 edges) than the second stream costs the host (about 15 us).
-    beside = None
+    # longer (40 us at 160 000 edges) than the second stream costs the host (about 15 us).  Its launches come after those
+    # of the first two steps, which keep the device busy meanwhile.
+    beside = buffers = ready = None
     if topology._perm is None and E >= _BESIDE_EDGES and not torch.cuda.is_current_stream_capturing():
         beside = _side_stream(dev)
-        grouping = topology.sender_order_beside(beside)
-        perm, send_ptr, _ = grouping
+        buffers = topology.grouping_buffers()
+        perm, send_ptr, _ = buffers
+        ready = torch.cuda.current_stream(dev).record_event()
     else:
         perm, send_ptr = topology.sender_order()
     p = out.data_ptr()
@@ -318,7 +320,13 @@ def energy_forces(plan, positions, species, one_hot, shifts, topology, halo=None
     forces = out[3 + 2 * n:].view(nl, 3)
 
     def run(first, last):
-        nonlocal beside
+        nonlocal ready
+        if ready is not None:
+            _abi.run_steps(m, io, first, 2, st)
+            first = 2
+            beside.wait_event(ready)
+            ready = None
+            topology.group_senders(buffers, beside.cuda_stream)
         if beside is not None and last > _SENDERS:
             if first < _SENDERS:
                 _abi.run_steps(m, io, first, _SENDERS, st)
@@ -330,7 +338,8 @@ def energy_forces(plan, positions, species, one_hot, shifts, topology, halo=None
         nonlocal beside
         torch.cuda.current_stream(dev).wait_stream(beside)
         beside = None
-        topology.grouped(perm, send_ptr)
+        if ready is None:
+            topology.grouped(perm, send_ptr)
 
     try:
         forces = _run_ranges(run, plan, n, nl, io, halo, forces)
