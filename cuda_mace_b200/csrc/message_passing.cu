@@ -103,46 +103,6 @@ __global__ void __launch_bounds__(SPLIT == 1 ? kWarpsPerBlock * 32 : SPLIT * 32)
   for (int m = 0; m < 16; m++) store_vec<T, VEC>(o + m * C, acc[m]);
 }
 
-// Sum of p[m] over the 32 lanes for all 16 m at once: after the call every lane holds the
-// total of component (lane >> 1).  16 shuffles instead of 16 * 5.
-template <typename T>
-__device__ __forceinline__ T warp_reduce16(T (&p)[16], int lane) {
-  T q8[8], q4[4], q2[2];
-  {
-    const bool up = lane & 16;
-#pragma unroll
-    for (int i = 0; i < 8; i++) {
-      const T send = up ? p[i] : p[i + 8];
-      const T keep = up ? p[i + 8] : p[i];
-      q8[i] = keep + __shfl_xor_sync(0xffffffffu, send, 16);
-    }
-  }
-  {
-    const bool up = lane & 8;
-#pragma unroll
-    for (int i = 0; i < 4; i++) {
-      const T send = up ? q8[i] : q8[i + 4];
-      const T keep = up ? q8[i + 4] : q8[i];
-      q4[i] = keep + __shfl_xor_sync(0xffffffffu, send, 8);
-    }
-  }
-  {
-    const bool up = lane & 4;
-#pragma unroll
-    for (int i = 0; i < 2; i++) {
-      const T send = up ? q4[i] : q4[i + 2];
-      const T keep = up ? q4[i + 2] : q4[i];
-      q2[i] = keep + __shfl_xor_sync(0xffffffffu, send, 4);
-    }
-  }
-  const bool up = lane & 2;
-  const T send = up ? q2[0] : q2[1];
-  const T keep = up ? q2[1] : q2[0];
-  T r = keep + __shfl_xor_sync(0xffffffffu, send, 2);
-  r += __shfl_xor_sync(0xffffffffu, r, 1);
-  return r;
-}
-
 template <typename T, int VEC>
 __global__ void __launch_bounds__(kWarpsPerBlock * 32)
     imp_bwd_edge_kernel(const T *__restrict__ X, const T *__restrict__ Y, const T *__restrict__ R,

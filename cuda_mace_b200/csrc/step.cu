@@ -17,9 +17,8 @@
 //   sums_back     grad Y and dE/dr of the first layer, plus the second layer's: gradient of every edge vector
 //   forces        position gradient and energies
 //
-// With tabulated radial weights (cubic splines) the first layer has no perceptron to sum against: `radial` evaluates both
-// layers' tables, `sums` is the plain message passing on the element's constant feature row (the edges' sender index is the
-// sender's element), `fold` the layer's element-dependent Linear, and the backward mirrors that.
+// With tabulated radial weights (cubic splines) the first layer has no perceptron to sum against: `sums` is the
+// message passing on the element's constant feature row, with the table evaluated there (spline_messages.cu), `fold` the layer's element-dependent Linear, and the backward mirrors that.
 //
 // Nodes of the first layer are kept in element order (slots) between `sums` and `mid_fwd` and on the way back, so the
 // element-dependent products see consecutive rows whatever the caller's order is.
@@ -45,9 +44,8 @@ int fused_messages(const float *X, const float *Y, const void *h, const void *W,
 int fused_messages_back(const float *X, const float *Y, const float *G, const void *h, const void *dh, const void *W,
                         float factor_v, float factor_t, const int32_t *sender, const int32_t *receiver, int64_t nedges,
                         float *T, float *gY, int32_t *status, cudaStream_t st);
-int step_sender_species(const int32_t *sender, const int32_t *species, int64_t nedges, int32_t *out, cudaStream_t st);
 template <typename T>
-int step_edge_finish(const T *gY0, const T *dr0, const T *gY1, const T *dr1, const Quad<T> *geo, int64_t nedges, T *gvec,
+int step_edge_finish(const T *gY0, const T *dr0, const T *gY1, const T *dr1, const Quad<T> *geo, int64_t nedges, int shares, T *gvec,
                      cudaStream_t st);
 int radial_pair_f64(const double *basis, int nb, const double *const (*w)[3], int nper, int64_t nedges,
                     double *const *h, double *const *dh, cudaStream_t st);
@@ -86,10 +84,10 @@ static bool is_fused(const cmace_step_model &m) { return !is_spline(m) && !m.is_
 
 template <typename T>
 struct Workspace {
-  int32_t *species, *slot_of, *node_of, *slot_type, *elem_start, *sender_species;
+  int32_t *species, *slot_of, *node_of, *slot_type, *elem_start;
   Quad<T> *geo;
   T *basis, *Y, *h[2], *dh[2], *A, *m0, *b0, *up, *R, *m1, *l1, *gX1, *gm1, *T_, *gY1, *gH1, *dr1, *gup, *gb0, *gX0, *gA,
-      *gvec, *gradR, *partial, *q0, *dq, *R0, *gY0, *dr0;
+      *gvec, *gradR, *partial, *q0, *dq, *gY0, *dr0;
   int64_t bytes;
 
   Workspace(void *base, const cmace_step_model &m, int64_t n, int64_t nl, int64_t E) {
@@ -108,11 +106,10 @@ struct Workspace {
     take(elem_start, Z + 1);
     take(geo, E);
     const bool sp = is_spline(m);
-    take(sender_species, sp ? E : 0);
-    take(basis, sp ? E : E * 2 * m.nbessel);
-    take(R0, sp ? E * 4 * C : 0);
-    take(gY0, sp ? E * 16 : 0);
-    take(dr0, sp ? E : 0);
+    take(basis, E * 2 * (sp ? 1 : m.nbessel));   // with tables: a SplinePoint an edge
+    const int64_t shares = sp ? spline_chunks<T>((int)C) : 1;
+    take(gY0, sp ? shares * E * 16 : 0);
+    take(dr0, sp ? shares * E : 0);
     take(Y, E * 16);
     for (int i = 0; i < 2; i++) {
       take(h[i], sp ? 0 : (E + 127) / 128 * 128 * ST_H);   // whole tiles of the kernels that read them
@@ -123,21 +120,21 @@ struct Workspace {
     take(b0, n * C);
     take(up, n * C);
     take(q0, n * (ST_RO + 1));
-    take(R, is_fused(m) ? 0 : E * 4 * C);
+    take(R, is_fused(m) || sp ? 0 : E * 4 * C);
     take(m1, n * 16 * C);
     take(l1, n * 16 * C);
     take(gX1, n * 16 * C);
     take(dq, n * ST_RO);
     take(T_, E * C);
-    take(gY1, E * 16);
+    take(gY1, shares * E * 16);
     take(gH1, sizeof(T) == 8 && !sp ? E * ST_H : 0);
-    take(dr1, E);
+    take(dr1, shares * E);
     take(gup, nl * C);
     take(gb0, n * C);
     take(gX0, n * 16 * C);
     take(gvec, E * 3);
-    take(gradR, sizeof(T) == 8 || sp ? E * 4 * C : 0);
-    take(partial, cmace_imp_bwd_scratch_elems(E, (int)C, sizeof(T) == 8 ? 1 : 0));
+    take(gradR, sizeof(T) == 8 && !sp ? E * 4 * C : 0);
+    take(partial, sp ? 0 : cmace_imp_bwd_scratch_elems(E, (int)C, sizeof(T) == 8 ? 1 : 0));
     gm1 = m1;   // the messages are not read again after the Linear
     gA = A;     // nor the sums after their product
   }
@@ -152,24 +149,6 @@ static int linear_any(const double *X, const void *W, const int32_t *start, int 
   return cmace_linear_f64(X, static_cast<const double *>(W), nullptr, start, nel, n, K, N, 1.0, out, st);
 }
 
-static int spline_fwd(const cmace_step_model &m, int layer, const float *r, int64_t E, float *R, cudaStream_t st) {
-  return cmace_spline_fwd_f32(r, static_cast<const float *>(m.spline_knots), static_cast<const float *>(m.spline[layer]), E,
-                              m.spline_intervals, 4 * m.channels, m.spline_width, m.spline_rmax, R, st);
-}
-static int spline_fwd(const cmace_step_model &m, int layer, const double *r, int64_t E, double *R, cudaStream_t st) {
-  return cmace_spline_fwd_f64(r, static_cast<const double *>(m.spline_knots), static_cast<const double *>(m.spline[layer]), E,
-                              m.spline_intervals, 4 * m.channels, m.spline_width, m.spline_rmax, R, st);
-}
-static int spline_bwd(const cmace_step_model &m, int layer, const float *r, const float *gR, int64_t E, float *gr, cudaStream_t st) {
-  return cmace_spline_bwd_f32(r, static_cast<const float *>(m.spline_knots), static_cast<const float *>(m.spline[layer]), gR,
-                              E, m.spline_intervals, 4 * m.channels, m.spline_width, m.spline_rmax, gr, st);
-}
-static int spline_bwd(const cmace_step_model &m, int layer, const double *r, const double *gR, int64_t E, double *gr,
-                      cudaStream_t st) {
-  return cmace_spline_bwd_f64(r, static_cast<const double *>(m.spline_knots), static_cast<const double *>(m.spline[layer]), gR,
-                              E, m.spline_intervals, 4 * m.channels, m.spline_width, m.spline_rmax, gr, st);
-}
-
 // the steps that tabulated radial weights do differently; -1 for the others
 template <typename T>
 static int run_spline_step(const cmace_step_model &m, cmace_step_io &io, const Workspace<T> &w, int step, const T *up,
@@ -177,36 +156,37 @@ static int run_spline_step(const cmace_step_model &m, cmace_step_io &io, const W
   const int64_t n = io.n_owned, E = io.nedges;
   const int C = m.channels, Z = m.elements;
   const int32_t *start = Z > 1 ? w.elem_start : nullptr;
-  const ImpLayout slots{1, 16, w.slot_of};
+  const T *senders = static_cast<const T *>(m.sender_table);
+  auto table = [&](int layer) {
+    return SplineTable<T>{static_cast<const T *>(m.spline[layer]), static_cast<const T *>(m.spline_knots), (T)m.spline_width,
+                          (T)m.spline_rmax, m.spline_intervals};
+  };
+  const SplinePoint<T> *at = reinterpret_cast<const SplinePoint<T> *>(w.basis);
   switch (step) {
     case S_EDGE_PREP:
       return StepKernels<T>::edge_prep(io.positions, io.sender, io.receiver, io.shifts, io.shift_index, io.shift_table,
-                                       io.shift_rows, io.status, E, m.r_max, 0, m.cutoff_p, w.geo,
+                                       io.shift_rows, io.status, E, m.r_max, 0, m.cutoff_p, table(0), w.geo,
                                        w.basis, w.Y, io.species, io.one_hot, io.one_hot_is_f64, io.n_local, n, Z, w.species,
                                        w.slot_of, w.node_of, w.slot_type, w.elem_start, st);
-    case S_RADIAL:
-      io.launches++;
-      if (int rc = spline_fwd(m, 0, w.basis, E, w.R0, st)) return rc;
-      return spline_fwd(m, 1, w.basis, E, w.R, st);
     case S_SUMS:
-      io.launches++;
-      if (int rc = step_sender_species(io.sender, w.species, E, w.sender_species, st)) return rc;
-      return imp_fwd<T>(static_cast<const T *>(m.sender_table), w.Y, w.R0, w.sender_species, io.row_ptr, n, E, slots, C, w.A, st);
+      return spline_messages<T>(senders, w.species, w.Y, at, table(0), io.sender, io.row_ptr, n, w.slot_of, C, w.A, st);
     case S_FOLD: return linear_any(w.A, m.fold, start, Z, n, C, C, w.m0, io.status, st);
+    case S_RADIAL:
     case S_RADIAL_OUT:
+    case S_RADIAL_BACK:
     case S_RADIAL_DOT: io.launches--; return CMACE_OK;
+    case S_MESSAGES:
+      return spline_messages<T>(up, nullptr, w.Y, at, table(1), io.sender, io.row_ptr, n, nullptr, C, w.m1, st);
     case S_EDGES_BACK:
-      return imp_bwd_edge<T>(up, w.Y, w.R, w.gm1, io.sender, io.row_ptr, n, E, ImpLayout{1, 16}, C, w.gradR, w.gY1, w.T_,
-                             w.partial, st);
-    case S_RADIAL_BACK: return spline_bwd(m, 1, w.basis, w.gradR, E, w.dr1, st);
+      return spline_edges_back<T>(up, nullptr, w.Y, at, table(1), w.gm1, nullptr, io.sender, io.row_ptr, n, E, C, w.T_,
+                                  w.gY1, w.dr1, st);
     case S_FOLD_BACK: return linear_any(w.gX0, m.fold_back[0], start, Z, n, C, C, w.gA, io.status, st);
     case S_SUMS_BACK:
-      io.launches += 2;
-      if (int rc = imp_bwd_edge<T>(static_cast<const T *>(m.sender_table), w.Y, w.R0, w.gA, w.sender_species, io.row_ptr, n,
-                                   E, slots, C, w.gradR, w.gY0, nullptr, w.partial, st))
+      io.launches++;
+      if (int rc = spline_edges_back<T>(senders, w.species, w.Y, at, table(0), w.gA, w.slot_of, io.sender, io.row_ptr, n, E,
+                                        C, nullptr, w.gY0, w.dr0, st))
         return rc;
-      if (int rc = spline_bwd(m, 0, w.basis, w.gradR, E, w.dr0, st)) return rc;
-      return step_edge_finish<T>(w.gY0, w.dr0, w.gY1, w.dr1, w.geo, E, w.gvec, st);
+      return step_edge_finish<T>(w.gY0, w.dr0, w.gY1, w.dr1, w.geo, E, spline_chunks<T>(C), w.gvec, st);
   }
   return -1;
 }
@@ -236,7 +216,7 @@ static int run_step(const cmace_step_model &m, cmace_step_io &io, const Workspac
   switch (step) {
     case S_EDGE_PREP:
       return K::edge_prep(io.positions, io.sender, io.receiver, io.shifts, io.shift_index, io.shift_table,
-                                       io.shift_rows, io.status, E, m.r_max, m.nbessel, m.cutoff_p, w.geo,
+                                       io.shift_rows, io.status, E, m.r_max, m.nbessel, m.cutoff_p, SplineTable<T>{}, w.geo,
                           w.basis, w.Y, io.species, io.one_hot, io.one_hot_is_f64, nl, n, Z, w.species, w.slot_of,
                           w.node_of, w.slot_type, w.elem_start, st);
     case S_RADIAL: {

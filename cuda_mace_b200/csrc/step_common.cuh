@@ -1,5 +1,7 @@
 // Shapes and array layouts shared by the kernels of the whole energy+force step (step.cu holds the sequence).
 #pragma once
+#include <type_traits>
+
 #include "common.cuh"
 
 namespace cmace {
@@ -25,6 +27,31 @@ struct RadialScales {
   float in_v, in_t, z[3], a[3], t[3], out_v, out_t;
 };
 
+// tabulated radial weights: coefficients [intervals, 4 powers, 4 C], knots of width apart, zero beyond r_max
+template <typename T>
+struct SplineTable {
+  const T *coeffs, *knots;
+  T width, r_max;
+  int intervals;
+};
+// where in the table an edge's length lies: distance from the interval's knot; interval -1 beyond r_max
+template <typename T>
+struct alignas(2 * sizeof(T)) SplinePoint {
+  T x;
+  typename std::conditional<sizeof(T) == 8, int64_t, int32_t>::type interval;
+};
+// spline_messages.cu; gY [spline_chunks, E, 16] and dr [spline_chunks, E] are shares to be added up
+template <typename T>
+int spline_chunks(int C);
+template <typename T>
+int spline_messages(const T *X, const int32_t *row_of, const T *Y, const SplinePoint<T> *r, const SplineTable<T> &table,
+                    const int32_t *sender, const int32_t *row_ptr, int64_t n, const int32_t *out_row, int C, T *out,
+                    cudaStream_t st);
+template <typename T>
+int spline_edges_back(const T *X, const int32_t *row_of, const T *Y, const SplinePoint<T> *r, const SplineTable<T> &table, const T *G,
+                      const int32_t *g_row, const int32_t *sender, const int32_t *row_ptr, int64_t n, int64_t E, int C,
+                      T *Tout, T *gY, T *dr, cudaStream_t st);
+
 constexpr int32_t CMACE_STEP_BAD_SHIFT = 90;   // status: a row of the shift table that does not exist
 
 int *staged_stall_flag();   // message_passing.cu: device word of the staged edge pass, or null
@@ -34,7 +61,8 @@ template <typename T>
 struct StepKernels {
   static int edge_prep(const double *pos, const int32_t *sender, const int32_t *receiver, const double *shifts,
                        const uint8_t *shift_index, const double *shift_table, int64_t shift_rows, int32_t *status,
-                       int64_t nedges, double r_max, int nb, int p, Quad<T> *geo, T *basis, T *Y,
+                       int64_t nedges, double r_max, int nb, int p, const SplineTable<T> &spline, Quad<T> *geo, T *basis,
+                       T *Y,
                        const int32_t *species_in, const void *one_hot, int one_hot_f64, int64_t n_local, int64_t n_owned,
                        int elements, int32_t *species, int32_t *slot_of, int32_t *node_of, int32_t *slot_type,
                        int32_t *elem_start, cudaStream_t st);

@@ -137,7 +137,7 @@ __global__ void __launch_bounds__(EP_THREADS)
                      const int32_t *__restrict__ receiver, const double *__restrict__ shifts,
                      const uint8_t *__restrict__ shift_index, const double *__restrict__ shift_table, int shift_rows,
                      int32_t *status, int64_t nedges, T r_max,
-                     int p, Quad<T> *__restrict__ geo, T *__restrict__ basis, T *__restrict__ Y,
+                     int p, const SplineTable<T> spline, Quad<T> *__restrict__ geo, T *__restrict__ basis, T *__restrict__ Y,
                      const int32_t *species_in, const void *one_hot, int one_hot_f64, int64_t n_local, int64_t n_owned,
                      int elements, int32_t *species, int32_t *slot_of, int32_t *node_of, int32_t *slot_type,
                      int32_t *elem_start) {
@@ -176,8 +176,17 @@ __global__ void __launch_bounds__(EP_THREADS)
   sph_l3<T>(uz, ux, uy, y);
   if (lane < rows) geo[e] = Quad<T>{ux, uy, uz, ir};
   store_rows<T, 16>(buf, y, Y + base * 16, rows, lane);
-  if constexpr (NB == 0) {   // tabulated radial weights: the length itself
-    if (lane < rows) basis[e] = r2 * ir;
+  if constexpr (NB == 0) {   // tabulated radial weights: where the length lies in the table
+    const T len = r2 * ir;
+    SplinePoint<T> at;
+    at.x = T(0);
+    at.interval = -1;
+    if (!(len > spline.r_max)) {
+      const int k = (int)(len / spline.width);
+      at.interval = k < 0 ? 0 : (k >= spline.intervals ? spline.intervals - 1 : k);
+      at.x = len - spline.knots[at.interval];
+    }
+    if (lane < rows) reinterpret_cast<SplinePoint<T> *>(basis)[e] = at;
   } else {
     T b[2 * NB];
     bessel_cutoff<T>(r2 * ir, r_max, NB, p, b, b + NB);
@@ -188,7 +197,8 @@ __global__ void __launch_bounds__(EP_THREADS)
 template <typename T>
 int StepKernels<T>::edge_prep(const double *pos, const int32_t *sender, const int32_t *receiver, const double *shifts,
                               const uint8_t *shift_index, const double *shift_table, int64_t shift_rows, int32_t *status,
-                              int64_t nedges, double r_max, int nb, int p, Quad<T> *geo, T *basis, T *Y,
+                              int64_t nedges, double r_max, int nb, int p, const SplineTable<T> &spline, Quad<T> *geo,
+                              T *basis, T *Y,
                               const int32_t *species_in, const void *one_hot, int one_hot_f64, int64_t n_local,
                               int64_t n_owned, int elements, int32_t *species, int32_t *slot_of, int32_t *node_of,
                               int32_t *slot_type, int32_t *elem_start, cudaStream_t st) {
@@ -198,7 +208,7 @@ int StepKernels<T>::edge_prep(const double *pos, const int32_t *sender, const in
   cudaError_t err = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
   if (err != cudaSuccess) return fail(CMACE_ERR_CUDA, "cmace_step(edge_prep): %s", cudaGetErrorString(err));
   launch_chained(kern, (unsigned)blocks, EP_THREADS, smem, st, pos, sender, receiver, shifts, shift_index, shift_table,
-                 (int)(shift_rows < 256 ? shift_rows : 256), status, nedges, (T)r_max, p, geo, basis, Y, species_in, one_hot,
+                 (int)(shift_rows < 256 ? shift_rows : 256), status, nedges, (T)r_max, p, spline, geo, basis, Y, species_in, one_hot,
                  one_hot_f64, n_local, n_owned, elements, species, slot_of, node_of, slot_type, elem_start);
   return check_launch("cmace_step(edge_prep)");
 }
@@ -858,51 +868,44 @@ int StepKernels<T>::sums_bwd(const T *gA, const T *h, const T *dh, const T *Y, c
 }
 
 // ---- tabulated radial weights ---------------------------------------------------------------------------------------
-// element of every edge's sender
-__global__ void __launch_bounds__(256)
-    sender_species_kernel(const int32_t *__restrict__ sender, const int32_t *__restrict__ species, int64_t nedges,
-                          int32_t *__restrict__ out) {
-  grid_begin();
-  const int64_t e = (int64_t)blockIdx.x * 256 + threadIdx.x;
-  if (e < nedges) out[e] = species[sender[e]];
-}
-int step_sender_species(const int32_t *sender, const int32_t *species, int64_t nedges, int32_t *out, cudaStream_t st) {
-  if (nedges > 0) launch_chained(sender_species_kernel, (unsigned)((nedges + 255) / 256), 256, 0, st, sender, species, nedges, out);
-  return check_launch("cmace_step(sums)");
-}
-
-// gradient of every edge's vector from both layers' grad Y and dE/dr
+// gradient of every edge's vector from both layers' grad Y and dE/dr, each in `shares` arrays to be added up
 template <typename T>
 __global__ void __launch_bounds__(256)
     edge_finish_kernel(const T *__restrict__ gY0, const T *__restrict__ dr0, const T *__restrict__ gY1,
-                       const T *__restrict__ dr1, const Quad<T> *__restrict__ geo, int64_t nedges, T *__restrict__ gvec) {
+                       const T *__restrict__ dr1, const Quad<T> *__restrict__ geo, int64_t nedges, int shares, T *__restrict__ gvec) {
   grid_begin();
   const int64_t e = (int64_t)blockIdx.x * 256 + threadIdx.x;
   if (e >= nedges) return;
   T s[17];
-  const Quad<T> *g = reinterpret_cast<const Quad<T> *>(gY0 + e * 16);
 #pragma unroll
-  for (int i = 0; i < 4; i++) {
-    const Quad<T> q = g[i];
-    s[4 * i] = q.x;
-    s[4 * i + 1] = q.y;
-    s[4 * i + 2] = q.z;
-    s[4 * i + 3] = q.w;
+  for (int i = 0; i < 17; i++) s[i] = T(0);
+  for (int k = 0; k < shares; k++) {
+    for (int layer = 0; layer < (k == 0 ? 1 : 2); layer++) {   // finish_edge adds the second layer's first share
+      const Quad<T> *g = reinterpret_cast<const Quad<T> *>((layer == 0 ? gY0 : gY1) + (k * nedges + e) * 16);
+#pragma unroll
+      for (int i = 0; i < 4; i++) {
+        const Quad<T> q = g[i];
+        s[4 * i] += q.x;
+        s[4 * i + 1] += q.y;
+        s[4 * i + 2] += q.z;
+        s[4 * i + 3] += q.w;
+      }
+      s[16] += (layer == 0 ? dr0 : dr1)[k * nedges + e];
+    }
   }
-  s[16] = dr0[e];
   finish_edge<T>(s, e, gY1, dr1, geo, gvec);
 }
 template <typename T>
-int step_edge_finish(const T *gY0, const T *dr0, const T *gY1, const T *dr1, const Quad<T> *geo, int64_t nedges, T *gvec,
-                     cudaStream_t st) {
+int step_edge_finish(const T *gY0, const T *dr0, const T *gY1, const T *dr1, const Quad<T> *geo, int64_t nedges, int shares,
+                     T *gvec, cudaStream_t st) {
   if (nedges > 0)
-    launch_chained(edge_finish_kernel<T>, (unsigned)((nedges + 255) / 256), 256, 0, st, gY0, dr0, gY1, dr1, geo, nedges, gvec);
+    launch_chained(edge_finish_kernel<T>, (unsigned)((nedges + 255) / 256), 256, 0, st, gY0, dr0, gY1, dr1, geo, nedges, shares, gvec);
   return check_launch("cmace_step(sums_back)");
 }
 template int step_edge_finish<float>(const float *, const float *, const float *, const float *, const Quad<float> *, int64_t,
-                                     float *, cudaStream_t);
+                                     int, float *, cudaStream_t);
 template int step_edge_finish<double>(const double *, const double *, const double *, const double *, const Quad<double> *,
-                                      int64_t, double *, cudaStream_t);
+                                      int64_t, int, double *, cudaStream_t);
 
 // ---- forces and energies ------------------------------------------------------------------------------------------
 // One warp per atom sums its edges' gradients from both groupings (float64, fixed order, no atomics); block 0 adds up
@@ -980,7 +983,9 @@ int StepKernels<T>::forces(const T *gvec, const int32_t *row_ptr, const int32_t 
 
 #define CMACE_STEP_EDGES(T)                                                                                         \
   template int StepKernels<T>::edge_prep(const double *, const int32_t *, const int32_t *, const double *,          \
-                                         const uint8_t *, const double *, int64_t, int32_t *, int64_t, double, int, int, Quad<T> *, T *, T *, const int32_t *, const void *, int, \
+                                         const uint8_t *, const double *, int64_t, int32_t *, int64_t, double, int, \
+                                         int, const SplineTable<T> &, Quad<T> *, T *, T *, const int32_t *,         \
+                                         const void *, int,                                                         \
                                          int64_t, int64_t, int, int32_t *, int32_t *, int32_t *, int32_t *,         \
                                          int32_t *, cudaStream_t);                                                  \
   template int StepKernels<T>::sums(const T *, const T *, const int32_t *, const int32_t *, const int32_t *,        \
