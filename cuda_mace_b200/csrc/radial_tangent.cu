@@ -284,12 +284,6 @@ __global__ void __launch_bounds__(RT_THREADS, 1)
 // Row strides of 68 doubles make the fragment loads of both operands conflict-free.
 constexpr int RD_WARPS = 16, RD_LD = 68;
 
-__device__ __forceinline__ void dmma(double (&c)[2], double a, double b) {
-  asm volatile("mma.sync.aligned.m8n8k4.row.col.f64.f64.f64.f64 {%0, %1}, {%2}, {%3}, {%0, %1};"
-               : "+d"(c[0]), "+d"(c[1])
-               : "d"(a), "d"(b));
-}
-
 // 1 / (1 + e^-z).  The elementwise phase has as many FP64 operations as the products if the library's exp and divide are
 // used (the kernel took 1.26 ms at 8 000 atoms, 0.78 of them the products' own time), so: e^x by Tang's table-driven
 // method (ACM TOMS 15, 1989): x = (32 m + j) ln2 / 32 + r with |r| <= ln2 / 64, e^x = 2^m 2^(j/32) (1 + p(r)); the

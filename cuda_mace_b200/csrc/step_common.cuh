@@ -20,6 +20,12 @@ struct alignas(4 * sizeof(T)) Quad {
 // block b is a [nodes, 16, width(b)] array, width = 64 times the elements it holds.
 __host__ __device__ inline int sums_block_width(int elements, int b) { return elements - 2 * b >= 2 ? 128 : 64; }
 
+__device__ __forceinline__ void dmma(double (&c)[2], double a, double b) {
+  asm volatile("mma.sync.aligned.m8n8k4.row.col.f64.f64.f64.f64 {%0, %1}, {%2}, {%3}, {%0, %1};"
+               : "+d"(c[0]), "+d"(c[1])
+               : "d"(a), "d"(b));
+}
+
 // Powers of two of the fp16 radial kernel.  in_v, in_t: factors of the basis and its derivative; per layer k: z scales
 // the accumulator to the pre-activation, a to the scaled activation (before the sigmoid factor), t to the scaled
 // derivative.  Activations of layer 3 leave with out_v = 1 / h and out_t = 1 / h' of the stored value.

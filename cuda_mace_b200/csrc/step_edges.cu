@@ -408,63 +408,63 @@ int step_sums_half(const void *h, const float *Y, const int32_t *sender, const i
   return check_launch("cmace_step(sums)");
 }
 
-// float64: sums over k = 2 lane, 2 lane + 1
-struct SumAcc {
-  double a[16][2];
-  __device__ __forceinline__ void zero() {
-#pragma unroll
-    for (int m = 0; m < 16; m++) a[m][0] = a[m][1] = 0.0;
-  }
-  __device__ __forceinline__ void add(const double *__restrict__ y, double h0, double h1) {
-#pragma unroll
-    for (int i = 0; i < 8; i++) {
-      const double2 v = __ldg(reinterpret_cast<const double2 *>(y) + i);
-      a[2 * i][0] = fma(v.x, h0, a[2 * i][0]);
-      a[2 * i][1] = fma(v.x, h1, a[2 * i][1]);
-      a[2 * i + 1][0] = fma(v.y, h0, a[2 * i + 1][0]);
-      a[2 * i + 1][1] = fma(v.y, h1, a[2 * i + 1][1]);
-    }
-  }
-};
-
+// float64: four edges at a time on the float64 tensor instruction (m8n8k4), laid out as in sums_tf32_kernel: row g + 8 i of
+// the sums, column g of tile j is k = 8 g + j.  With fma instructions a lane held two columns and all 16 rows, its edges
+// went one after the other through eight loads of Y each: 262 us at 8 000 atoms and 23 us at 192, where the loads and the
+// stores need 80 us at 8 000; now 179 and 10 us.
 __global__ void __launch_bounds__(SU_WARPS * 32)
     sums_f64_kernel(const double *__restrict__ h, const double *__restrict__ Y, const int32_t *__restrict__ sender,
                 const int32_t *__restrict__ row_ptr, const int32_t *__restrict__ species,
                 const int32_t *__restrict__ slot_of, int64_t nnodes, int elements, double *__restrict__ A) {
   grid_begin();
   __shared__ int32_t lists[SU_WARPS][SU_LIST];
-  const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+  const int lane = threadIdx.x & 31, w = threadIdx.x >> 5, g = lane >> 2, t = lane & 3;
   const int64_t pair = (int64_t)blockIdx.x * SU_WARPS + w;
   if (pair >= nnodes * elements) return;
   const int64_t node = pair / elements;
   const int z = (int)(pair - node * elements);
   int32_t *list = lists[w];
-  SumAcc acc;
-  acc.zero();
+  double acc[2][8][2];
+#pragma unroll
+  for (int j = 0; j < 8; j++) acc[0][j][0] = acc[0][j][1] = acc[1][j][0] = acc[1][j][1] = 0.0;
   for_edges_of_element(sender, species, row_ptr[node], row_ptr[node + 1], z, list, lane, [&](int n) {
-    int j = 0;
-    for (; j + 3 < n; j += 4) {   // four edges' rows on their way before the first is used
-      int64_t e[4];
-      double2 v[4];
+    double2 hv[4];
+    double yv[2];
+    auto load = [&](int j0) {   // edge j0 + t; past the end: the last edge with Y = 0
+      const int j = j0 + t;
+      const int64_t e = list[j < n ? j : n - 1];
+      const double2 *hp = reinterpret_cast<const double2 *>(h + e * ST_H + 8 * g);
+#pragma unroll
+      for (int u = 0; u < 4; u++) hv[u] = __ldg(hp + u);
+      yv[0] = j < n ? __ldg(Y + e * 16 + g) : 0.0;
+      yv[1] = j < n ? __ldg(Y + e * 16 + g + 8) : 0.0;
+    };
+    load(0);
+    for (int j0 = 0; j0 < n; j0 += 4) {
+      double b[8];
+      const double y0 = yv[0], y1 = yv[1];
 #pragma unroll
       for (int u = 0; u < 4; u++) {
-        e[u] = list[j + u];
-        v[u] = __ldg(reinterpret_cast<const double2 *>(h + e[u] * ST_H) + lane);
+        b[2 * u] = hv[u].x;
+        b[2 * u + 1] = hv[u].y;
       }
+      if (j0 + 4 < n) load(j0 + 4);
 #pragma unroll
-      for (int u = 0; u < 4; u++) acc.add(Y + e[u] * 16, v[u].x, v[u].y);
-    }
-    for (; j < n; j++) {
-      const int64_t e = list[j];
-      const double2 v = __ldg(reinterpret_cast<const double2 *>(h + e * ST_H) + lane);
-      acc.add(Y + e * 16, v.x, v.y);
+      for (int j = 0; j < 8; j++) {
+        dmma(acc[0][j], y0, b[j]);
+        dmma(acc[1][j], y1, b[j]);
+      }
     }
   });
   const int width = elements * ST_H;
-  double *o = A + (int64_t)slot_of[node] * 16 * width + z * ST_H + 2 * lane;
+  double *o = A + (int64_t)slot_of[node] * 16 * width + z * ST_H + 16 * t;
 #pragma unroll
-  for (int m = 0; m < 16; m++) {
-    *reinterpret_cast<double2 *>(o + (int64_t)m * width) = make_double2(acc.a[m][0], acc.a[m][1]);
+  for (int i = 0; i < 2; i++) {
+    double2 *row = reinterpret_cast<double2 *>(o + (int64_t)(g + 8 * i) * width);
+#pragma unroll
+    for (int u = 0; u < 2; u++)
+#pragma unroll
+      for (int j = 0; j < 4; j++) row[4 * u + j] = make_double2(acc[i][2 * j][u], acc[i][2 * j + 1][u]);
   }
 }
 
@@ -485,33 +485,6 @@ int StepKernels<T>::sums(const T *h, const T *Y, const int32_t *sender, const in
 // The warp holds P = grad A[i, :, z, :]; the 16 + 1 sums of an edge over k wait in shared memory until 32 edges (or the
 // list's end) are there: then lane j turns edge j's numbers, plus the second layer's grad Y and dE/dr, into the
 // gradient of its vector.
-template <typename T>
-__device__ __forceinline__ T reduce16(T (&p)[16], int lane) {
-  T q8[8], q4[4], q2[2];
-  bool up = lane & 16;
-#pragma unroll
-  for (int i = 0; i < 8; i++) {
-    const T send = up ? p[i] : p[i + 8], keep = up ? p[i + 8] : p[i];
-    q8[i] = keep + __shfl_xor_sync(0xffffffffu, send, 16);
-  }
-  up = lane & 8;
-#pragma unroll
-  for (int i = 0; i < 4; i++) {
-    const T send = up ? q8[i] : q8[i + 4], keep = up ? q8[i + 4] : q8[i];
-    q4[i] = keep + __shfl_xor_sync(0xffffffffu, send, 8);
-  }
-  up = lane & 4;
-#pragma unroll
-  for (int i = 0; i < 2; i++) {
-    const T send = up ? q4[i] : q4[i + 2], keep = up ? q4[i + 2] : q4[i];
-    q2[i] = keep + __shfl_xor_sync(0xffffffffu, send, 4);
-  }
-  up = lane & 2;
-  const T send = up ? q2[0] : q2[1], keep = up ? q2[1] : q2[0];
-  T r = keep + __shfl_xor_sync(0xffffffffu, send, 2);
-  return r + __shfl_xor_sync(0xffffffffu, r, 1);   // component lane >> 1
-}
-
 // lane j of the warp: edge list[j], its 16 + 1 sums in st[j * 17 ..], to the gradient of the edge's vector
 template <typename T>
 __device__ __forceinline__ void finish_edge(const T *st, int64_t e, const T *__restrict__ gY1, const T *__restrict__ dr1,
@@ -771,27 +744,10 @@ int step_sums_bwd_half(const float *gA, const void *h, const void *dh, const flo
   return check_launch("cmace_step(sums_back)");
 }
 
-// float64: a lane holds k = 2 lane, 2 lane + 1 of P
-struct PairGrad {
-  double p[16][2];
-  // g[lm] = sum over this lane's k of P h; returns sum_k h'_k sum_lm Y P of this lane
-  __device__ __forceinline__ double edge(const double *__restrict__ y, double h0, double h1, double d0, double d1,
-                                         double (&g)[16]) const {
-    double s0 = 0.0, s1 = 0.0;
-#pragma unroll
-    for (int i = 0; i < 8; i++) {
-      const double2 v = __ldg(reinterpret_cast<const double2 *>(y) + i);
-      s0 = fma(v.x, p[2 * i][0], s0);
-      s1 = fma(v.x, p[2 * i][1], s1);
-      s0 = fma(v.y, p[2 * i + 1][0], s0);
-      s1 = fma(v.y, p[2 * i + 1][1], s1);
-    }
-#pragma unroll
-    for (int m = 0; m < 16; m++) g[m] = fma(p[m][1], h1, p[m][0] * h0);
-    return fma(s1, d1, s0 * d0);
-  }
-};
-
+// float64: eight edges at a time on the float64 tensor instruction, D = P h^T and P h'^T.  P's A fragments stay in
+// registers; K step s of lane (g, t) is k = 16 t + s, so that a lane reads 16 consecutive values of its edge's row (and of
+// P's rows g and g + 8).  With fma instructions an edge cost 21 shuffles of two words and eight loads of Y: 404 us at
+// 8 000 atoms, 37 us at 192, where its bytes need 115 us at 8 000; now 261 and 20 us.
 __global__ void __launch_bounds__(SU_WARPS * 32)
     sums_bwd_f64_kernel(const double *__restrict__ gA, const double *__restrict__ h, const double *__restrict__ dh,
                     const double *__restrict__ Y, const int32_t *__restrict__ sender, const int32_t *__restrict__ row_ptr,
@@ -801,48 +757,67 @@ __global__ void __launch_bounds__(SU_WARPS * 32)
   grid_begin();
   __shared__ int32_t lists[SU_WARPS][SU_LIST];
   __shared__ double stage[SU_WARPS][32 * 17];
-  const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+  const int lane = threadIdx.x & 31, w = threadIdx.x >> 5, g = lane >> 2, t = lane & 3;
   const int64_t pair = (int64_t)blockIdx.x * SU_WARPS + w;
   if (pair >= nnodes * elements) return;
   const int64_t node = pair / elements;
   const int z = (int)(pair - node * elements);
   int32_t *list = lists[w];
   double *st = stage[w];
-  PairGrad P;
+  double2 P[2][8];
   {
     const int b = z >> 1, width = sums_block_width(elements, b);
-    const double *g = gA + (int64_t)b * nnodes * (16 * 128) + (int64_t)slot_of[node] * 16 * width + (z & 1) * ST_H + 2 * lane;
+    const double *p = gA + (int64_t)b * nnodes * (16 * 128) + (int64_t)slot_of[node] * 16 * width + (z & 1) * ST_H + 16 * t;
 #pragma unroll
-    for (int m = 0; m < 16; m++) {
-      const double2 v = __ldg(reinterpret_cast<const double2 *>(g + m * width));
-      P.p[m][0] = v.x;
-      P.p[m][1] = v.y;
-    }
+    for (int i = 0; i < 2; i++)
+#pragma unroll
+      for (int q = 0; q < 8; q++) P[i][q] = __ldg(reinterpret_cast<const double2 *>(p + (g + 8 * i) * width) + q);
   }
   for_edges_of_element(sender, species, row_ptr[node], row_ptr[node + 1], z, list, lane, [&](int n) {
     for (int j0 = 0; j0 < n; j0 += 32) {
       const int nj = n - j0 < 32 ? n - j0 : 32;
-      double2 hv = double2{}, dv = double2{};
-      if (nj > 0) {
-        const int64_t e = list[j0];
-        hv = __ldg(reinterpret_cast<const double2 *>(h + e * ST_H) + lane);
-        dv = __ldg(reinterpret_cast<const double2 *>(dh + e * ST_H) + lane);
-      }
-      for (int j = 0; j < nj; j++) {
-        const int64_t e = list[j0 + j];
-        const double2 hc = hv, dc = dv;
-        if (j + 1 < nj) {   // the next edge's rows
-          const int64_t en = list[j0 + j + 1];
-          hv = __ldg(reinterpret_cast<const double2 *>(h + en * ST_H) + lane);
-          dv = __ldg(reinterpret_cast<const double2 *>(dh + en * ST_H) + lane);
-        }
-        double g[16];
-        double r = P.edge(Y + e * 16, hc.x, hc.y, dc.x, dc.y, g);
+      for (int j = 0; j < nj; j += 8) {
+        const int i = j0 + j + g;   // this lane's row of h: that edge, or the last one
+        const int64_t e = list[i < n ? i : n - 1];
+        const double2 *hp = reinterpret_cast<const double2 *>(h + e * ST_H + 16 * t);
+        const double2 *dp = reinterpret_cast<const double2 *>(dh + e * ST_H + 16 * t);
+        double2 hv[8], dv[8];
 #pragma unroll
-        for (int off = 16; off > 0; off >>= 1) r += __shfl_xor_sync(0xffffffffu, r, off);
-        const double tot = reduce16(g, lane);
-        if ((lane & 1) == 0) st[j * 17 + (lane >> 1)] = tot;
-        if (lane == 1) st[j * 17 + 16] = r;
+        for (int q = 0; q < 8; q++) {
+          hv[q] = __ldg(hp + q);
+          dv[q] = __ldg(dp + q);
+        }
+        const int i0 = j0 + j + 2 * t;   // its result columns: edges 2 t and 2 t + 1 of the eight
+        const int64_t e0 = list[i0 < n ? i0 : n - 1], e1 = list[i0 + 1 < n ? i0 + 1 : n - 1];
+        const double y00 = __ldg(Y + e0 * 16 + g), y01 = __ldg(Y + e0 * 16 + g + 8);
+        const double y10 = __ldg(Y + e1 * 16 + g), y11 = __ldg(Y + e1 * 16 + g + 8);
+        double ch[2][2] = {{0.0, 0.0}, {0.0, 0.0}}, cd[2][2] = {{0.0, 0.0}, {0.0, 0.0}};
+#pragma unroll
+        for (int q = 0; q < 8; q++) {
+          dmma(ch[0], P[0][q].x, hv[q].x);
+          dmma(ch[1], P[1][q].x, hv[q].x);
+          dmma(cd[0], P[0][q].x, dv[q].x);
+          dmma(cd[1], P[1][q].x, dv[q].x);
+          dmma(ch[0], P[0][q].y, hv[q].y);
+          dmma(ch[1], P[1][q].y, hv[q].y);
+          dmma(cd[0], P[0][q].y, dv[q].y);
+          dmma(cd[1], P[1][q].y, dv[q].y);
+        }
+        double *s0 = st + (j + 2 * t) * 17, *s1 = s0 + 17;
+        s0[g] = ch[0][0];
+        s1[g] = ch[0][1];
+        s0[g + 8] = ch[1][0];
+        s1[g + 8] = ch[1][1];
+        double r0 = fma(y00, cd[0][0], y01 * cd[1][0]), r1 = fma(y10, cd[0][1], y11 * cd[1][1]);
+#pragma unroll
+        for (int off = 4; off < 32; off <<= 1) {
+          r0 += __shfl_xor_sync(0xffffffffu, r0, off);
+          r1 += __shfl_xor_sync(0xffffffffu, r1, off);
+        }
+        if (g == 0) {
+          s0[16] = r0;
+          s1[16] = r1;
+        }
       }
       __syncwarp();
       if (lane < nj) finish_edge<double>(st + lane * 17, list[j0 + lane], gY1, dr1, geo, gvec);
