@@ -84,7 +84,7 @@ static bool is_fused(const cmace_step_model &m) { return !is_spline(m) && !m.is_
 
 template <typename T>
 struct Workspace {
-  int32_t *species, *slot_of, *node_of, *slot_type, *elem_start;
+  int32_t *species, *counts, *slot_of, *node_of, *slot_type, *elem_start;
   Quad<T> *geo;
   T *basis, *Y, *h[2], *dh[2], *A, *m0, *b0, *up, *R, *m1, *l1, *gX1, *gm1, *T_, *gY1, *gH1, *dr1, *gup, *gb0, *gX0, *gA,
       *gvec, *gradR, *partial, *q0, *dq, *gY0, *dr0;
@@ -100,6 +100,7 @@ struct Workspace {
     };
     const int64_t C = m.channels, Z = m.elements;
     take(species, nl);
+    take(counts, node_blocks(nl) * ST_MAX_Z);
     take(slot_of, n);
     take(node_of, n);
     take(slot_type, n);
@@ -167,7 +168,7 @@ static int run_spline_step(const cmace_step_model &m, cmace_step_io &io, const W
       return StepKernels<T>::edge_prep(io.positions, io.sender, io.receiver, io.shifts, io.shift_index, io.shift_table,
                                        io.shift_rows, io.status, E, m.r_max, 0, m.cutoff_p, table(0), w.geo,
                                        w.basis, w.Y, io.species, io.one_hot, io.one_hot_is_f64, io.n_local, n, Z, w.species,
-                                       w.slot_of, w.node_of, w.slot_type, w.elem_start, st);
+                                       w.counts, w.slot_of, w.node_of, w.slot_type, w.elem_start, st);
     case S_SUMS:
       return spline_messages<T>(senders, w.species, w.Y, at, table(0), io.sender, io.row_ptr, n, w.slot_of, C, w.A, st);
     case S_FOLD: return linear_any(w.A, m.fold, start, Z, n, C, C, w.m0, io.status, st);
@@ -209,6 +210,7 @@ static int run_step(const cmace_step_model &m, cmace_step_io &io, const Workspac
   const bool fused = is_fused(m);
   if (fused && (step == S_RADIAL_OUT || step == S_RADIAL_BACK || step == S_RADIAL_DOT)) return CMACE_OK;
   io.launches++;
+  if (step == S_EDGE_PREP && node_blocks(io.n_local) > 1) io.launches++;
   if (is_spline(m)) {
     const int rc = run_spline_step<T>(m, io, w, step, up, st);
     if (rc >= 0) return rc;
@@ -217,8 +219,8 @@ static int run_step(const cmace_step_model &m, cmace_step_io &io, const Workspac
     case S_EDGE_PREP:
       return K::edge_prep(io.positions, io.sender, io.receiver, io.shifts, io.shift_index, io.shift_table,
                                        io.shift_rows, io.status, E, m.r_max, m.nbessel, m.cutoff_p, SplineTable<T>{}, w.geo,
-                          w.basis, w.Y, io.species, io.one_hot, io.one_hot_is_f64, nl, n, Z, w.species, w.slot_of,
-                          w.node_of, w.slot_type, w.elem_start, st);
+                          w.basis, w.Y, io.species, io.one_hot, io.one_hot_is_f64, nl, n, Z, w.species, w.counts,
+                          w.slot_of, w.node_of, w.slot_type, w.elem_start, st);
     case S_RADIAL: {
       const T *rw[2][3];
       for (int i = 0; i < 2; i++)

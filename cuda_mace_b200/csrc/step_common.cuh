@@ -62,6 +62,9 @@ constexpr int32_t CMACE_STEP_BAD_SHIFT = 90;   // status: a row of the shift tab
 
 int *staged_stall_flag();   // message_passing.cu: device word of the staged edge pass, or null
 
+constexpr int GN_NODES = 2048;   // nodes a block of edge_prep resolves; several such blocks take a second launch
+constexpr int64_t node_blocks(int64_t n_local) { return (n_local + GN_NODES - 1) / GN_NODES; }
+
 // launchers (one per kernel; every one checks its launch)
 template <typename T>
 struct StepKernels {
@@ -70,8 +73,8 @@ struct StepKernels {
                        int64_t nedges, double r_max, int nb, int p, const SplineTable<T> &spline, Quad<T> *geo, T *basis,
                        T *Y,
                        const int32_t *species_in, const void *one_hot, int one_hot_f64, int64_t n_local, int64_t n_owned,
-                       int elements, int32_t *species, int32_t *slot_of, int32_t *node_of, int32_t *slot_type,
-                       int32_t *elem_start, cudaStream_t st);
+                       int elements, int32_t *species, int32_t *counts, int32_t *slot_of, int32_t *node_of,
+                       int32_t *slot_type, int32_t *elem_start, cudaStream_t st);
   static int sums(const T *h, const T *Y, const int32_t *sender, const int32_t *row_ptr, const int32_t *species,
                   const int32_t *slot_of, int64_t nnodes, int elements, T *A, cudaStream_t st);
   static int contract_fwd(const T *X, const int32_t *types, const T *weff, int64_t n, int C, T *b, cudaStream_t st);

@@ -21,8 +21,10 @@ namespace cmace {
 // ---- edge geometry, basis and node grouping ----------------------------------------------------------------------
 constexpr int EP_THREADS = 256;
 
-// Block 0 resolves the species and groups the owned nodes by element (stable): thread t counts and then places the
-// nodes of its own consecutive piece, so equal elements keep their order.  It runs beside the edge blocks.
+// The first blocks resolve the species, GN_NODES nodes each, beside the edge blocks.  One block (the usual number in the
+// systems that are bound by launches) also groups the owned nodes by element, stable; several leave their counts per element to
+// group_nodes_kernel.  One block for all nodes was the kernel's whole time: 325 us at 64 000 nodes, 50 us at 8 000, where
+// the edges take 110 and 15; now 123 and 18.
 template <typename OH>
 __device__ int first_max(const OH *row, int n) {
   int best = 0;
@@ -35,76 +37,113 @@ __device__ int first_max(const OH *row, int n) {
   return best;
 }
 
-__device__ void group_nodes(const int32_t *species_in, const void *one_hot, int one_hot_f64, int64_t n_local,
-                            int64_t n_owned, int elements, int32_t *species, int32_t *slot_of, int32_t *node_of,
-                            int32_t *slot_type, int32_t *elem_start) {
-  __shared__ int count[ST_MAX_Z][EP_THREADS + 1];
-  const int t = threadIdx.x, lane = t & 31, w = t >> 5;
-  const int64_t per = (n_owned + 4 * EP_THREADS - 1) / (4 * EP_THREADS) * 4;   // pieces of whole 16-byte groups
-  const int64_t lo = t * per < n_owned ? t * per : n_owned, hi = lo + per < n_owned ? lo + per : n_owned;
-  for (int z = 0; z < elements; z++) count[z][t] = 0;
-  // coalesced pass over the species first: the counting pass then reads what this block wrote
-#pragma unroll 4
-  for (int64_t i = t; i < n_local; i += EP_THREADS) {
-    int z;
-    if (species_in) z = species_in[i];
-    else if (one_hot_f64) z = first_max(static_cast<const double *>(one_hot) + i * elements, elements);
-    else z = first_max(static_cast<const float *>(one_hot) + i * elements, elements);
-    species[i] = z < 0 ? 0 : (z >= elements ? elements - 1 : z);
-  }
-  __syncthreads();
-#pragma unroll 4
-  for (int64_t i = lo; i < hi; i += 4) {
-    const int4 z = *reinterpret_cast<const int4 *>(species + i);
-    count[z.x][t]++;
-    if (i + 1 < hi) count[z.y][t]++;
-    if (i + 2 < hi) count[z.z][t]++;
-    if (i + 3 < hi) count[z.w][t]++;
-  }
-  __syncthreads();
-  // exclusive prefix over (element, thread): warp w scans elements w, w + 8, ...
-  __shared__ int total[ST_MAX_Z];
-  for (int z = w; z < elements; z += EP_THREADS / 32) {
-    int run = 0;
-    for (int b = 0; b < EP_THREADS; b += 32) {
-      const int v = count[z][b + lane];
-      int inc = v;
+__device__ void resolve_nodes(const int32_t *__restrict__ species_in, const void *__restrict__ one_hot, int one_hot_f64,
+                              int64_t lo, int64_t hi, int elements, int32_t *__restrict__ species) {
+  constexpr int PER = GN_NODES / EP_THREADS;
+  int z[PER];
 #pragma unroll
-      for (int off = 1; off < 32; off <<= 1) {
-        const int o = __shfl_up_sync(0xffffffffu, inc, off);
-        if (lane >= off) inc += o;
-      }
-      count[z][b + lane] = run + inc - v;
-      run += __shfl_sync(0xffffffffu, inc, 31);
-    }
-    if (lane == 0) total[z] = run;
+  for (int u = 0; u < PER; u++) {
+    const int64_t i = lo + u * EP_THREADS + threadIdx.x;
+    z[u] = 0;
+    if (i >= hi) continue;
+    if (species_in) z[u] = species_in[i];
+    else if (one_hot_f64) z[u] = first_max(static_cast<const double *>(one_hot) + i * elements, elements);
+    else z[u] = first_max(static_cast<const float *>(one_hot) + i * elements, elements);
   }
-  __syncthreads();
-  if (t == 0) {
-    int acc = 0;
-    for (int z = 0; z < elements; z++) {
-      elem_start[z] = acc;
-      const int c = total[z];
-      total[z] = acc;
-      acc += c;
-    }
-    elem_start[elements] = acc;
-  }
-  __syncthreads();
-#pragma unroll 4
-  for (int64_t i = lo; i < hi; i += 4) {
-    const int4 z4 = *reinterpret_cast<const int4 *>(species + i);
 #pragma unroll
-    for (int u = 0; u < 4; u++) {
-      const int z = u == 0 ? z4.x : (u == 1 ? z4.y : (u == 2 ? z4.z : z4.w));
-      if (i + u < hi) {
-        const int s = total[z] + count[z][t]++;
-        slot_of[i + u] = s;
-        node_of[s] = (int32_t)(i + u);
-        slot_type[s] = z;
+  for (int u = 0; u < PER; u++) {
+    const int64_t i = lo + u * EP_THREADS + threadIdx.x;
+    if (i < hi) species[i] = z[u] < 0 ? 0 : (z[u] >= elements ? elements - 1 : z[u]);
+  }
+  __syncthreads();
+}
+
+// Groups the nodes [first, end) of one block, or counts them.  A warp takes a consecutive piece, four nodes a lane, and
+// ranks them by ballot, so that loads and stores are coalesced.  counts: [blocks, ST_MAX_Z]; with one block the start of
+// every element follows from its own counts.
+__device__ void group_nodes(int64_t first, int64_t end, int blocks, int block, bool count_only, int elements,
+                            const int32_t *species, int32_t *counts, int32_t *slot_of, int32_t *node_of, int32_t *slot_type,
+                            int32_t *elem_start) {
+  constexpr int WARPS = EP_THREADS / 32, PIECE = GN_NODES / WARPS;
+  __shared__ int count[WARPS][ST_MAX_Z];
+  const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+  const int64_t lo = first + w * PIECE < end ? first + w * PIECE : end, hi = lo + PIECE < end ? lo + PIECE : end;
+  const unsigned below = (1u << lane) - 1u;
+  int run = 0;   // lane z: first its number of nodes, then the slot of the next one
+#pragma unroll 1
+  for (int pass = 0; pass < 2; pass++) {
+#pragma unroll 1
+    for (int64_t b = lo; b < hi; b += 128) {
+      const int64_t i = b + 4 * lane;
+      int4 z = make_int4(-1, -1, -1, -1);
+      if (i < hi) z = *reinterpret_cast<const int4 *>(species + i);   // the array ends on a 256-byte boundary
+      if (i + 1 >= hi) z.y = -1;
+      if (i + 2 >= hi) z.z = -1;
+      if (i + 3 >= hi) z.w = -1;
+      int4 slot = make_int4(0, 0, 0, 0);
+#pragma unroll 1
+      for (int k = 0; k < elements; k++) {
+        const unsigned m0 = __ballot_sync(0xffffffffu, z.x == k), m1 = __ballot_sync(0xffffffffu, z.y == k);
+        const unsigned m2 = __ballot_sync(0xffffffffu, z.z == k), m3 = __ballot_sync(0xffffffffu, z.w == k);
+        int at = __shfl_sync(0xffffffffu, run, k) + __popc(m0 & below) + __popc(m1 & below) + __popc(m2 & below) + __popc(m3 & below);
+        if (z.x == k) slot.x = at++;
+        if (z.y == k) slot.y = at++;
+        if (z.z == k) slot.z = at++;
+        if (z.w == k) slot.w = at++;
+        if (lane == k) run += __popc(m0) + __popc(m1) + __popc(m2) + __popc(m3);
+      }
+      if (pass == 0) continue;
+      auto place = [&](int64_t node, int s, int zz) {
+        if (zz < 0) return;
+        slot_of[node] = s;
+        node_of[s] = (int32_t)node;
+        slot_type[s] = zz;
+      };
+      place(i, slot.x, z.x);
+      place(i + 1, slot.y, z.y);
+      place(i + 2, slot.z, z.z);
+      place(i + 3, slot.w, z.w);
+    }
+    if (pass == 1) break;
+    if (lane < ST_MAX_Z) count[w][lane] = run;
+    __syncthreads();
+    int before = 0, total = 0;   // lane z: nodes of element z before this warp's piece, and in all
+    if (lane < elements) {
+      for (int v = 0; v < WARPS; v++) {
+        before += v < w ? count[v][lane] : 0;
+        total += count[v][lane];
+      }
+      if (count_only) {
+        if (w == 0) counts[block * ST_MAX_Z + lane] = total;
+      } else if (blocks > 1) {
+        total = 0;
+#pragma unroll 4
+        for (int v = 0; v < blocks; v++) {
+          const int c = counts[v * ST_MAX_Z + lane];
+          before += v < block ? c : 0;
+          total += c;
+        }
       }
     }
+    if (count_only) return;
+    int inc = total;
+#pragma unroll
+    for (int off = 1; off < 32; off <<= 1) {
+      const int o = __shfl_up_sync(0xffffffffu, inc, off);
+      if (lane >= off) inc += o;
+    }
+    if (w == 0 && block == 0 && lane <= elements) elem_start[lane] = inc - total;   // lane `elements` has none: the end
+    run = inc - total + before;
   }
+}
+
+__global__ void __launch_bounds__(EP_THREADS)
+    group_nodes_kernel(int64_t n_owned, int elements, const int32_t *species, int32_t *counts, int32_t *slot_of,
+                       int32_t *node_of, int32_t *slot_type, int32_t *elem_start) {
+  grid_begin();
+  const int64_t first = (int64_t)blockIdx.x * GN_NODES;
+  group_nodes(first, first + GN_NODES < n_owned ? first + GN_NODES : n_owned, (int)gridDim.x, (int)blockIdx.x, false, elements,
+              species, counts, slot_of, node_of, slot_type, elem_start);
 }
 
 // A warp's 32 rows of N values each, one row per lane, to consecutive memory: through shared memory, so that a store
@@ -132,26 +171,29 @@ __device__ __forceinline__ void store_rows(uint4 *buf, const T (&v)[N], T *__res
 
 // One thread per edge: vector in float64, then unit vector and 1/r, basis and its derivative [E, 2 NB], Y [E, 16].
 template <typename T, int NB>
-__global__ void __launch_bounds__(EP_THREADS)
+__global__ void __launch_bounds__(EP_THREADS, sizeof(T) == 4 ? 5 : 3)
     edge_prep_kernel(const double *__restrict__ pos, const int32_t *__restrict__ sender,
                      const int32_t *__restrict__ receiver, const double *__restrict__ shifts,
                      const uint8_t *__restrict__ shift_index, const double *__restrict__ shift_table, int shift_rows,
                      int32_t *status, int64_t nedges, T r_max,
                      int p, const SplineTable<T> spline, Quad<T> *__restrict__ geo, T *__restrict__ basis, T *__restrict__ Y,
                      const int32_t *species_in, const void *one_hot, int one_hot_f64, int64_t n_local, int64_t n_owned,
-                     int elements, int32_t *species, int32_t *slot_of, int32_t *node_of, int32_t *slot_type,
-                     int32_t *elem_start) {
+                     int elements, int32_t *species, int32_t *counts, int32_t *slot_of, int32_t *node_of,
+                     int32_t *slot_type, int32_t *elem_start) {
   grid_begin();
-  if (blockIdx.x == 0) {
-    group_nodes(species_in, one_hot, one_hot_f64, n_local, n_owned, elements, species, slot_of, node_of, slot_type,
-                elem_start);
+  const int nblocks = (int)node_blocks(n_local);
+  if ((int)blockIdx.x < nblocks) {
+    const int64_t first = (int64_t)blockIdx.x * GN_NODES, end = first + GN_NODES;
+    resolve_nodes(species_in, one_hot, one_hot_f64, first, end < n_local ? end : n_local, elements, species);
+    group_nodes(first, end < n_owned ? end : n_owned, 1, (int)blockIdx.x, nblocks > 1, elements, species, counts, slot_of,
+                node_of, slot_type, elem_start);
     return;
   }
   extern __shared__ uint4 ep_smem[];
   const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
   constexpr int MOST = 2 * NB > 16 ? 2 * NB : 16;
   uint4 *buf = ep_smem + w * 32 * (MOST * (int)sizeof(T) / 16 + 1);
-  const int64_t base = (int64_t)(blockIdx.x - 1) * EP_THREADS + w * 32;
+  const int64_t base = ((int64_t)blockIdx.x - nblocks) * EP_THREADS + w * 32;
   if (base >= nedges) return;
   const int rows = nedges - base < 32 ? (int)(nedges - base) : 32;
   const int64_t e = base + (lane < rows ? lane : rows - 1);
@@ -200,16 +242,20 @@ int StepKernels<T>::edge_prep(const double *pos, const int32_t *sender, const in
                               int64_t nedges, double r_max, int nb, int p, const SplineTable<T> &spline, Quad<T> *geo,
                               T *basis, T *Y,
                               const int32_t *species_in, const void *one_hot, int one_hot_f64, int64_t n_local,
-                              int64_t n_owned, int elements, int32_t *species, int32_t *slot_of, int32_t *node_of,
+                              int64_t n_owned, int elements, int32_t *species, int32_t *counts, int32_t *slot_of, int32_t *node_of,
                               int32_t *slot_type, int32_t *elem_start, cudaStream_t st) {
-  const int64_t blocks = 1 + (nedges + EP_THREADS - 1) / EP_THREADS;
+  const int64_t blocks = node_blocks(n_local) + (nedges + EP_THREADS - 1) / EP_THREADS;
   const size_t smem = (size_t)EP_THREADS * ((nb == 16 ? 32 : 16) * sizeof(T) + 16);
   auto kern = nb == 16 ? edge_prep_kernel<T, 16> : (nb == 8 ? edge_prep_kernel<T, 8> : edge_prep_kernel<T, 0>);
   cudaError_t err = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
   if (err != cudaSuccess) return fail(CMACE_ERR_CUDA, "cmace_step(edge_prep): %s", cudaGetErrorString(err));
   launch_chained(kern, (unsigned)blocks, EP_THREADS, smem, st, pos, sender, receiver, shifts, shift_index, shift_table,
                  (int)(shift_rows < 256 ? shift_rows : 256), status, nedges, (T)r_max, p, spline, geo, basis, Y, species_in, one_hot,
-                 one_hot_f64, n_local, n_owned, elements, species, slot_of, node_of, slot_type, elem_start);
+                 one_hot_f64, n_local, n_owned, elements, species, counts, slot_of, node_of, slot_type,
+                 elem_start);
+  if (node_blocks(n_local) > 1)
+    launch_chained(group_nodes_kernel, (unsigned)node_blocks(n_owned), EP_THREADS, 0, st, n_owned, elements,
+                   species, counts, slot_of, node_of, slot_type, elem_start);
   return check_launch("cmace_step(edge_prep)");
 }
 
@@ -962,7 +1008,7 @@ int StepKernels<T>::forces(const T *gvec, const int32_t *row_ptr, const int32_t 
                                          int, const SplineTable<T> &, Quad<T> *, T *, T *, const int32_t *,         \
                                          const void *, int,                                                         \
                                          int64_t, int64_t, int, int32_t *, int32_t *, int32_t *, int32_t *,         \
-                                         int32_t *, cudaStream_t);                                                  \
+                                         int32_t *, int32_t *, cudaStream_t);                                                  \
   template int StepKernels<T>::sums(const T *, const T *, const int32_t *, const int32_t *, const int32_t *,        \
                                     const int32_t *, int64_t, int, T *, cudaStream_t);                              \
   template int StepKernels<T>::sums_bwd(const T *, const T *, const T *, const T *, const int32_t *,                \
