@@ -169,34 +169,39 @@ int StepKernels<T>::contract_readout(const T *X, const int32_t *types, const T *
 
 // ---- between the layers --------------------------------------------------------------------------------------------
 // Products with a [C, C] matrix that stays in shared memory (64 KB float32, 128 KB float64: one fill per block, blocks
-// are persistent), plus 17 columns that depend on the element: 16 of the second readout's hidden layer and the first
-// readout.  Nodes are taken in slot order, so the nodes of a tile nearly always share the element.  2 C threads: a
-// thread owns 4 columns of NODES / 8 nodes; what bounds it is the shared-memory pipe (four 16-byte loads of weights
-// and NODES / 8 of rows per 4 k).
-constexpr int MID_EXTRA = ST_RO + 1;
+// are persistent), plus 17 columns (padded to 20) that depend on the element: 16 of the second readout's hidden layer and
+// the first readout.  Nodes are taken in slot order, so the nodes of a tile nearly always share the element, whose part
+// of the matrix is kept beside the other (a tile where the element changes takes one after the other).  The
+// next tile's rows are copied while a tile is worked on.  2 C threads: a thread owns 4 columns of NODES / 8 nodes; what
+// bounds it then is the shared-memory pipe (four 16-byte loads of weights and NODES / 8 of rows per 4 k).  With rows
+// loaded at the head of a tile and the element's columns read from memory, forward and backward took 150 + 170 us at
+// 64 000 nodes, 22 + 20 us at 3 000; now 92 + 79 and 14 + 12.
+constexpr int MID_EXTRA = ST_RO + 1, MID_PAD = 20;
 
+__device__ __forceinline__ void copy16(void *dst, const void *src) {
+  asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"((uint32_t)__cvta_generic_to_shared(dst)), "l"(src) : "memory");
+}
+__device__ __forceinline__ void copies_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
+__device__ __forceinline__ void copies_wait() { asm volatile("cp.async.wait_group 0;" ::: "memory"); }
+
+// count values, a multiple of 16 bytes
 template <typename T>
-__device__ __forceinline__ void mid_fill(T *sW, const T *__restrict__ W, int C, int tid, int nthreads) {
-  for (int i = tid; i < C * C / (16 / (int)sizeof(T)); i += nthreads) {
-    const uint32_t d = (uint32_t)__cvta_generic_to_shared(sW) + 16u * (uint32_t)i;
-    asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(d), "l"(reinterpret_cast<const char *>(W) + 16 * (int64_t)i) : "memory");
-  }
-  asm volatile("cp.async.commit_group;" ::: "memory");
+__device__ __forceinline__ void mid_fill(T *dst, const T *__restrict__ src, int count, int tid, int nthreads) {
+  constexpr int V = 16 / (int)sizeof(T);
+  for (int i = tid; i < count / V; i += nthreads) copy16(dst + i * V, src + (int64_t)i * V);
 }
 
-// acc[i][u] = sum_k rows[j0 + i][k] W[k][4 tx + u]
-template <typename T, int PER>
-__device__ __forceinline__ void mid_product(const T *rows, const T *sW, int C, int j0, int tx, T (&acc)[PER][4]) {
-#pragma unroll
-  for (int i = 0; i < PER; i++) acc[i][0] = acc[i][1] = acc[i][2] = acc[i][3] = T(0);
+// acc[i][u] += sum_k rows[j0 + i STRIDE][k] W[k][4 tx + u], k < K (a multiple of 4)
+template <typename T, int PER, int STRIDE = 1>
+__device__ __forceinline__ void mid_product(const T *rows, int ld, const T *W, int ldw, int K, int j0, int tx, T (&acc)[PER][4]) {
 #pragma unroll 2
-  for (int k = 0; k < C; k += 4) {
+  for (int k = 0; k < K; k += 4) {
     Quad<T> r[PER];
 #pragma unroll
-    for (int i = 0; i < PER; i++) r[i] = *reinterpret_cast<const Quad<T> *>(rows + (j0 + i) * C + k);
+    for (int i = 0; i < PER; i++) r[i] = *reinterpret_cast<const Quad<T> *>(rows + (j0 + i * STRIDE) * ld + k);
 #pragma unroll
     for (int u = 0; u < 4; u++) {
-      const Quad<T> w = *reinterpret_cast<const Quad<T> *>(sW + (k + u) * C + 4 * tx);
+      const Quad<T> w = *reinterpret_cast<const Quad<T> *>(W + (k + u) * ldw + 4 * tx);
 #pragma unroll
       for (int i = 0; i < PER; i++) {
         const T v = u == 0 ? r[i].x : (u == 1 ? r[i].y : (u == 2 ? r[i].z : r[i].w));
@@ -208,120 +213,211 @@ __device__ __forceinline__ void mid_product(const T *rows, const T *sW, int C, i
     }
   }
 }
-
-// extra: [Z][C/4][17][4]
-template <typename T, int NODES>
-__global__ void __launch_bounds__(256)
-    mid_fwd_kernel(const T *__restrict__ b, const int32_t *__restrict__ node_of, const int32_t *__restrict__ slot_type,
-                   const T *__restrict__ wu, const T *__restrict__ extra, int64_t n, int C, T *__restrict__ up,
-                   T *__restrict__ q0) {
-  grid_begin();
-  extern __shared__ __align__(32) unsigned char mid_smem[];
-  T *sW = reinterpret_cast<T *>(mid_smem), *rows = sW + C * C;
-  constexpr int PER = NODES / 8;
-  const int tid = threadIdx.x, nt = 2 * C, tx = tid % (C / 4), ty = tid / (C / 4);
-  mid_fill(sW, wu, C, tid, nt);
-  asm volatile("cp.async.wait_group 0;" ::: "memory");
-  for (int64_t first = (int64_t)blockIdx.x * NODES; first < n; first += (int64_t)gridDim.x * NODES) {
-    const int nn = n - first < NODES ? (int)(n - first) : NODES;
-    __syncthreads();
-    for (int i = tid; i < NODES * C; i += nt) rows[i] = i < nn * C ? b[first * C + i] : T(0);
-    __syncthreads();
-    T acc[PER][4];
-    mid_product<T, PER>(rows, sW, C, ty * PER, tx, acc);
+template <typename T, int PER>
+__device__ __forceinline__ void mid_zero(T (&acc)[PER][4]) {
 #pragma unroll
-    for (int i = 0; i < PER; i++)
-      if (ty * PER + i < nn)
-        *reinterpret_cast<Quad<T> *>(up + (int64_t)node_of[first + ty * PER + i] * C + 4 * tx) =
-            Quad<T>{acc[i][0], acc[i][1], acc[i][2], acc[i][3]};
-    for (int i = tid; i < nn * MID_EXTRA; i += nt) {
-      const int j = i / MID_EXTRA, col = i - j * MID_EXTRA;
-      const Quad<T> *w = reinterpret_cast<const Quad<T> *>(extra) + (int64_t)slot_type[first + j] * (C / 4) * MID_EXTRA + col;
-      T a = T(0), a2 = T(0);
-#pragma unroll 8
-      for (int k = 0; k < C / 4; k++) {
-        const Quad<T> x = w[k * MID_EXTRA], r = *reinterpret_cast<const Quad<T> *>(rows + j * C + 4 * k);
-        a = fma(r.x, x.x, a);
-        a2 = fma(r.y, x.y, a2);
-        a = fma(r.z, x.z, a);
-        a2 = fma(r.w, x.w, a2);
-      }
-      q0[(int64_t)node_of[first + j] * MID_EXTRA + col] = a + a2;
+  for (int i = 0; i < PER; i++) acc[i][0] = acc[i][1] = acc[i][2] = acc[i][3] = T(0);
+}
+
+// The elements of a tile in turn: body(z) with z's part of the matrix in sE.  type: of the tile's node `lane`, -1 past the
+// end; held: the element whose part is there.  Called by all threads of the block.
+template <typename T, typename Body>
+__device__ __forceinline__ void for_elements_of_tile(int type, int nn, T *sE, const T *__restrict__ extra, int count, int tid,
+                                                     int nthreads, int &held, Body body) {
+  int z = __shfl_sync(0xffffffffu, type, 0);
+  const int last = __shfl_sync(0xffffffffu, type, nn - 1);
+  while (true) {
+    if (z != held) {
+      __syncthreads();   // the part that is there has been read
+      mid_fill(sE, extra + (int64_t)z * count, count, tid, nthreads);
+      copies_commit();
+      copies_wait();
+      __syncthreads();
+      held = z;
     }
+    body(z);
+    if (z == last) break;
+    const unsigned later = __ballot_sync(0xffffffffu, type > z);   // sorted: the next element's first node
+    z = __shfl_sync(0xffffffffu, type, __ffs(later) - 1);
   }
 }
 
-// grad b0 [slot order] = grad up Wu^T + (dq, scale) [17] extra_t[z] [17, C]
+// extra: [Z][C][20].  The block's last 64 threads own the extra columns: 5 groups of 4 times 8 groups of nodes,
+// every eighth node each; rows are 4 values longer than C, so that the 8 nodes lie in different banks.
+template <typename T, int NODES>
+__global__ void __launch_bounds__(320)
+    mid_fwd_kernel(const T *__restrict__ b, const int32_t *__restrict__ node_of, const int32_t *__restrict__ slot_type,
+                   const T *__restrict__ wu, const T *__restrict__ extra, int64_t n, int C, T *__restrict__ up,
+                   T *__restrict__ q0) {
+  extern __shared__ __align__(32) unsigned char mid_smem[];
+  T *sW = reinterpret_cast<T *>(mid_smem), *sE = sW + C * C, *buf = sE + C * MID_PAD;
+  constexpr int PER = NODES / 8, V = 16 / (int)sizeof(T);
+  const int tid = threadIdx.x, nt = 2 * C, x = tid - nt;
+  const int ld = C + 4;
+  const int tx = x < 0 ? tid % (C / 4) : x % (MID_PAD / 4), ty = x < 0 ? tid / (C / 4) : x / (MID_PAD / 4);
+  mid_fill(sW, wu, C * C, tid, nt + 64);
+  grid_begin();
+  auto fetch = [&](int64_t first, T *rows) {   // rows past the end: the last one
+    for (int i = tid; i < NODES * C / V; i += nt + 64) {
+      const int j = i / (C / V), c = (i - j * (C / V)) * V;
+      const int64_t s = first + j < n ? first + j : n - 1;
+      copy16(rows + j * ld + c, b + s * C + c);
+    }
+  };
+  int64_t first = (int64_t)blockIdx.x * NODES;
+  fetch(first, buf);
+  int held = first < n ? slot_type[first] : -1;
+  if (held >= 0) mid_fill(sE, extra + (int64_t)held * C * MID_PAD, C * MID_PAD, tid, nt + 64);
+  copies_commit();
+  for (int turn = 0; first < n; first += (int64_t)gridDim.x * NODES, turn ^= 1) {
+    T *rows = buf + turn * NODES * ld;
+    const int nn = n - first < NODES ? (int)(n - first) : NODES;
+    const int type = (tid & 31) < nn ? slot_type[first + (tid & 31)] : -1;
+    int32_t node[PER];
+#pragma unroll
+    for (int i = 0; i < PER; i++) {
+      const int j = x < 0 ? ty * PER + i : ty + 8 * i;
+      node[i] = ty < 8 && j < nn ? node_of[first + j] : 0;
+    }
+    copies_wait();
+    __syncthreads();
+    if (first + (int64_t)gridDim.x * NODES < n) {
+      fetch(first + (int64_t)gridDim.x * NODES, buf + (turn ^ 1) * NODES * ld);
+      copies_commit();
+    }
+    T acc[PER][4];
+    for_elements_of_tile<T>(type, nn, sE, extra, C * MID_PAD, tid, nt + 64, held, [&](int z) {
+      if (x < 0 || ty >= 8) return;
+      mid_zero<T, PER>(acc);
+      mid_product<T, PER, 8>(rows, ld, sE, MID_PAD, C, ty, tx, acc);
+#pragma unroll
+      for (int i = 0; i < PER; i++)
+        if (ty + 8 * i < nn && slot_type[first + ty + 8 * i] == z)
+#pragma unroll
+          for (int u = 0; u < 4; u++)
+            if (4 * tx + u < MID_EXTRA) q0[(int64_t)node[i] * MID_EXTRA + 4 * tx + u] = acc[i][u];
+    });
+    if (x >= 0) continue;
+    mid_zero<T, PER>(acc);
+    mid_product<T, PER>(rows, ld, sW, C, C, ty * PER, tx, acc);
+#pragma unroll
+    for (int i = 0; i < PER; i++)
+      if (ty * PER + i < nn)
+        *reinterpret_cast<Quad<T> *>(up + (int64_t)node[i] * C + 4 * tx) = Quad<T>{acc[i][0], acc[i][1], acc[i][2], acc[i][3]};
+  }
+}
+
+// grad b0 [slot order] = grad up Wu^T + (dq, scale, 0) [20] extra_t[z] [20, C]
 template <typename T, int NODES>
 __global__ void __launch_bounds__(256)
     mid_bwd_kernel(const T *__restrict__ gup, const int32_t *__restrict__ node_of, const int32_t *__restrict__ slot_type,
                    const T *__restrict__ dq, const T *__restrict__ wu_t, const T *__restrict__ extra_t, T scale,
                    int64_t n, int C, T *__restrict__ gb) {
-  grid_begin();
   extern __shared__ __align__(32) unsigned char mid_smem[];
-  T *sW = reinterpret_cast<T *>(mid_smem), *rows = sW + C * C, *sdq = rows + NODES * C;
-  constexpr int PER = NODES / 8;
+  T *sW = reinterpret_cast<T *>(mid_smem), *sE = sW + C * C, *buf = sE + C * MID_PAD;
+  constexpr int PER = NODES / 8, V = 16 / (int)sizeof(T);
+  T *const sdq = buf + 2 * NODES * C;
   const int tid = threadIdx.x, nt = 2 * C, tx = tid % (C / 4), ty = tid / (C / 4);
-  mid_fill(sW, wu_t, C, tid, nt);
-  asm volatile("cp.async.wait_group 0;" ::: "memory");
-  for (int64_t first = (int64_t)blockIdx.x * NODES; first < n; first += (int64_t)gridDim.x * NODES) {
-    const int nn = n - first < NODES ? (int)(n - first) : NODES;
-    __syncthreads();
-    for (int i = tid; i < NODES * C; i += nt) {
-      const int j = i / C;
-      rows[i] = j < nn ? gup[(int64_t)node_of[first + j] * C + (i - j * C)] : T(0);
+  mid_fill(sW, wu_t, C * C, tid, nt);
+  for (int i = tid; i < 2 * NODES; i += nt)
+#pragma unroll
+    for (int u = ST_RO; u < MID_PAD; u++) sdq[i * MID_PAD + u] = u == ST_RO ? scale : T(0);
+  grid_begin();
+  // a thread copies NODES sizeof(T) / 32 pieces of rows; the atoms they belong to are looked up a tile ahead
+  constexpr int PIECES = NODES * (int)sizeof(T) / 32;
+  constexpr int DQ = NODES * ST_RO / V, DQ_MOST = (DQ + 63) / 64;   // pieces of dq; at most so many a thread (C = 32)
+  int32_t at[PIECES], at_dq[DQ_MOST];
+  auto look_up = [&](int64_t first) {
+#pragma unroll
+    for (int p = 0; p < PIECES; p++) {
+      const int64_t s = first + (tid + p * nt) / (C / V);
+      at[p] = node_of[s < n ? s : n - 1];
     }
-    for (int i = tid; i < nn * ST_RO; i += nt) sdq[i] = dq[(int64_t)node_of[first + i / ST_RO] * ST_RO + i % ST_RO];
+#pragma unroll
+    for (int p = 0; p < DQ_MOST; p++) {
+      const int64_t s = first + (tid + p * nt) / (ST_RO / V);
+      at_dq[p] = node_of[s < n ? s : n - 1];
+    }
+  };
+  auto fetch = [&](int turn) {
+#pragma unroll
+    for (int p = 0; p < PIECES; p++) {
+      const int i = tid + p * nt, j = i / (C / V), c = (i - j * (C / V)) * V;
+      copy16(buf + (turn * NODES + j) * C + c, gup + (int64_t)at[p] * C + c);
+    }
+#pragma unroll
+    for (int p = 0; p < DQ_MOST; p++) {
+      const int i = tid + p * nt, j = i / (ST_RO / V), c = (i - j * (ST_RO / V)) * V;
+      if (i < DQ) copy16(sdq + (turn * NODES + j) * MID_PAD + c, dq + (int64_t)at_dq[p] * ST_RO + c);
+    }
+    copies_commit();
+  };
+  const int64_t step = (int64_t)gridDim.x * NODES;
+  int64_t first = (int64_t)blockIdx.x * NODES;
+  look_up(first);
+  int held = first < n ? slot_type[first] : -1;
+  if (held >= 0) mid_fill(sE, extra_t + (int64_t)held * C * MID_PAD, C * MID_PAD, tid, nt);
+  fetch(0);
+  if (first + step < n) look_up(first + step);
+  for (int turn = 0; first < n; first += step, turn ^= 1) {
+    const T *rows = buf + turn * NODES * C, *sd = sdq + turn * NODES * MID_PAD;
+    const int nn = n - first < NODES ? (int)(n - first) : NODES;
+    const int type = (tid & 31) < nn ? slot_type[first + (tid & 31)] : -1;
+    copies_wait();
     __syncthreads();
+    if (first + step < n) {
+      fetch(turn ^ 1);
+      if (first + 2 * step < n) look_up(first + 2 * step);
+    }
     T acc[PER][4];
-    mid_product<T, PER>(rows, sW, C, ty * PER, tx, acc);
+    mid_zero<T, PER>(acc);
+    mid_product<T, PER>(rows, C, sW, C, C, ty * PER, tx, acc);
+    for_elements_of_tile<T>(type, nn, sE, extra_t, C * MID_PAD, tid, nt, held, [&](int z) {
+      T more[PER][4];
+      mid_zero<T, PER>(more);
+      mid_product<T, PER>(sd, MID_PAD, sE, C, MID_PAD, ty * PER, tx, more);
+#pragma unroll
+      for (int i = 0; i < PER; i++)
+        if (ty * PER + i < nn && slot_type[first + ty * PER + i] == z)
+#pragma unroll
+          for (int u = 0; u < 4; u++) acc[i][u] += more[i][u];
+    });
 #pragma unroll
     for (int i = 0; i < PER; i++) {
       const int j = ty * PER + i;
-      if (j < nn) {
-        const Quad<T> *w = reinterpret_cast<const Quad<T> *>(extra_t + (int64_t)slot_type[first + j] * MID_EXTRA * C) + tx;
-#pragma unroll
-        for (int k = 0; k < MID_EXTRA; k++) {
-          const Quad<T> x = w[k * (C / 4)];
-          const T d = k < ST_RO ? sdq[j * ST_RO + k] : scale;
-          acc[i][0] = fma(d, x.x, acc[i][0]);
-          acc[i][1] = fma(d, x.y, acc[i][1]);
-          acc[i][2] = fma(d, x.z, acc[i][2]);
-          acc[i][3] = fma(d, x.w, acc[i][3]);
-        }
+      if (j < nn)
         *reinterpret_cast<Quad<T> *>(gb + (first + j) * C + 4 * tx) = Quad<T>{acc[i][0], acc[i][1], acc[i][2], acc[i][3]};
-      }
     }
   }
 }
 
 // 8 nodes a tile while that leaves SMs idle, else 32 (four times the reuse of a weight); two blocks an SM in float32
 template <typename T, typename Kernel8, typename Kernel32, typename... Args>
-static int launch_mid(const char *what, int64_t n, int C, Kernel8 k8, Kernel32 k32, cudaStream_t st, Args... args) {
+static int launch_mid(const char *what, int64_t n, int C, int threads, Kernel8 k8, Kernel32 k32, cudaStream_t st, Args... args) {
   if (n == 0) return CMACE_OK;
-  const bool small = n < 32 * 148;
+  const bool small = n <= 8 * 148;
   const int nodes = small ? 8 : 32;
-  const size_t smem = sizeof(T) * ((size_t)C * C + (size_t)nodes * (C + ST_RO));
+  const size_t smem = sizeof(T) * ((size_t)C * (C + MID_PAD) + 2 * (size_t)nodes * (C + MID_PAD));   // forward: C + 4 a row
   int64_t blocks = (n + nodes - 1) / nodes;
   const int64_t cap = 148 * (sizeof(T) == 4 ? 2 : 1);
   if (blocks > cap) blocks = cap;
   cudaError_t e = small ? cudaFuncSetAttribute(k8, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem)
                         : cudaFuncSetAttribute(k32, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
   if (e != cudaSuccess) return fail(CMACE_ERR_CUDA, "%s: %s", what, cudaGetErrorString(e));
-  if (small) launch_chained(k8, (unsigned)blocks, 2 * C, smem, st, args...);
-  else launch_chained(k32, (unsigned)blocks, 2 * C, smem, st, args...);
+  if (small) launch_chained(k8, (unsigned)blocks, threads, smem, st, args...);
+  else launch_chained(k32, (unsigned)blocks, threads, smem, st, args...);
   return check_launch(what);
 }
 template <typename T>
 int StepKernels<T>::mid_fwd(const T *b, const int32_t *node_of, const int32_t *slot_type, const T *wu, const T *extra,
                             int64_t n, int C, T *up, T *q0, cudaStream_t st) {
-  return launch_mid<T>("cmace_step(mid_fwd)", n, C, mid_fwd_kernel<T, 8>, mid_fwd_kernel<T, 32>, st, b, node_of, slot_type,
+  return launch_mid<T>("cmace_step(mid_fwd)", n, C, 2 * C + 64, mid_fwd_kernel<T, 8>, mid_fwd_kernel<T, 32>, st, b, node_of, slot_type,
                        wu, extra, n, C, up, q0);
 }
 template <typename T>
 int StepKernels<T>::mid_bwd(const T *gup, const int32_t *node_of, const int32_t *slot_type, const T *dq, const T *wu_t,
                             const T *extra_t, double scale, int64_t n, int C, T *gb, cudaStream_t st) {
-  return launch_mid<T>("cmace_step(mid_bwd)", n, C, mid_bwd_kernel<T, 8>, mid_bwd_kernel<T, 32>, st, gup, node_of, slot_type,
+  return launch_mid<T>("cmace_step(mid_bwd)", n, C, 2 * C, mid_bwd_kernel<T, 8>, mid_bwd_kernel<T, 32>, st, gup, node_of, slot_type,
                        dq, wu_t, extra_t, (T)scale, n, C, gb);
 }
 

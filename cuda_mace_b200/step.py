@@ -168,7 +168,8 @@ class StepPlan:
         m.up, m.up_back = hold(up.to(model.dtype)), hold(up.t().to(model.dtype))
         sc = d(L1.W_sc).view(C, Z, C).permute(1, 0, 2)                       # [Z, C, C]
         extra = torch.cat([prod0 @ sc @ ro1, (prod0 @ d(L0.W_readout)).expand(Z, C, 1)], dim=2)   # [Z, C, 17]
-        m.extra = hold(extra.view(Z, C // 4, 4, 17).transpose(2, 3).to(model.dtype))
+        extra = torch.nn.functional.pad(extra, (0, 3))   # whole groups of four
+        m.extra = hold(extra.to(model.dtype))
         m.extra_back = hold(extra.transpose(1, 2).to(model.dtype))
         m.readout1 = hold((prod1 @ ro1).t().to(model.dtype))
         m.readout2 = hold(d(L1.W_readout2)[:, 0] * SILU_2MOM)

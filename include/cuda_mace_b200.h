@@ -388,9 +388,9 @@ typedef struct cmace_step_model {
   const void *linear[2];     /* second layer's Linear and its transpose, [4] [C, C] (float32: packed) */
   const void *weff[2];       /* effective contraction weights of both layers [elements][13][C] */
   const void *up, *up_back;  /* first layer's product times second layer's linear_up [C, C], and its transpose */
-  const void *extra;         /* [elements][C/4][17][4]: 16 columns product x skip connection x first readout matrix,
+  const void *extra;         /* [elements][C][20]: 16 columns product x skip connection x first readout matrix,
                                 then product x first layer's readout */
-  const void *extra_back;    /* the same as [elements][17][C] */
+  const void *extra_back;    /* the same as [elements][20][C] */
   const void *readout1;      /* [16][C]: second layer's product times the first readout matrix, transposed */
   const double *readout2;    /* [16] */
   const double *atomic_energies; /* [elements] */
