@@ -433,42 +433,45 @@ __global__ void __launch_bounds__(SPLIT == 1 ? kWarpsPerBlock * 32 : SPLIT * 32)
   const int64_t node = SPLIT == 1 ? (int64_t)blockIdx.x * kWarpsPerBlock + warp : blockIdx.x;
   if (node >= nnodes) return;
   const int c0 = blockIdx.y * (32 * VEC) + lane * VEC;
-  const int64_t k0 = send_ptr[node], k1 = send_ptr[node + 1];
-  T acc[VEC], acc2[VEC];
+  const int64_t k1 = send_ptr[node + 1];
+  // 32 edges' indices in one load, then four rows in flight at a time
+  constexpr int AHEAD = 4;
+  T acc[2][VEC];
 #pragma unroll
-  for (int v = 0; v < VEC; v++) acc[v] = acc2[v] = T(0);
-  int64_t k = k0 + (SPLIT > 1 ? 2 * warp : 0);
-  for (; k + 1 < k1; k += 2 * SPLIT) {
-    const int64_t ea = perm[k], eb = perm[k + 1];
-    T a[VEC], b[VEC];
-    load_vec<T, VEC>(a, Tin + ea * C + c0);
-    load_vec<T, VEC>(b, Tin + eb * C + c0);
+  for (int v = 0; v < VEC; v++) acc[0][v] = acc[1][v] = T(0);
+  for (int64_t k = send_ptr[node] + (SPLIT > 1 ? warp : 0); k < k1; k += 32 * SPLIT) {
+    const int64_t mine = k + (int64_t)SPLIT * lane;
+    const int32_t e = mine < k1 ? perm[mine] : 0;
+    const int n = (int)((k1 - k + SPLIT - 1) / SPLIT < 32 ? (k1 - k + SPLIT - 1) / SPLIT : 32);
+    for (int j = 0; j < n; j += AHEAD) {
+      T a[AHEAD][VEC];
 #pragma unroll
-    for (int v = 0; v < VEC; v++) {
-      acc[v] += a[v];
-      acc2[v] += b[v];
+      for (int u = 0; u < AHEAD; u++) {
+        const int64_t row = __shfl_sync(0xffffffffu, e, (j + u) & 31);
+        if (j + u < n) load_vec<T, VEC>(a[u], Tin + row * C + c0);
+      }
+#pragma unroll
+      for (int u = 0; u < AHEAD; u++)
+        if (j + u < n) {
+#pragma unroll
+          for (int v = 0; v < VEC; v++) acc[u & 1][v] += a[u][v];
+        }
     }
   }
-  if (k < k1) {
-    T a[VEC];
-    load_vec<T, VEC>(a, Tin + (int64_t)perm[k] * C + c0);
 #pragma unroll
-    for (int v = 0; v < VEC; v++) acc[v] += a[v];
-  }
-#pragma unroll
-  for (int v = 0; v < VEC; v++) acc[v] += acc2[v];
+  for (int v = 0; v < VEC; v++) acc[0][v] += acc[1][v];
   if constexpr (SPLIT > 1) {
     __shared__ T part[SPLIT][32 * VEC];
 #pragma unroll
-    for (int v = 0; v < VEC; v++) part[warp][lane * VEC + v] = acc[v];
+    for (int v = 0; v < VEC; v++) part[warp][lane * VEC + v] = acc[0][v];
     __syncthreads();
     if (warp > 0) return;
 #pragma unroll
     for (int w = 1; w < SPLIT; w++)
 #pragma unroll
-      for (int v = 0; v < VEC; v++) acc[v] += part[w][lane * VEC + v];
+      for (int v = 0; v < VEC; v++) acc[0][v] += part[w][lane * VEC + v];
   }
-  store_vec<T, VEC>(gradX + node * C + c0, acc);
+  store_vec<T, VEC>(gradX + node * C + c0, acc[0]);
 }
 
 // ------------------------------------------------------------------------------------------

@@ -133,7 +133,7 @@ struct Workspace {
     take(gup, nl * C);
     take(gb0, n * C);
     take(gX0, n * 16 * C);
-    take(gvec, E * 3);
+    take(gvec, E * 4);
     take(gradR, sizeof(T) == 8 && !sp ? E * 4 * C : 0);
     take(partial, sp ? 0 : cmace_imp_bwd_scratch_elems(E, (int)C, sizeof(T) == 8 ? 1 : 0));
     gm1 = m1;   // the messages are not read again after the Linear

@@ -287,6 +287,44 @@ __device__ __forceinline__ void for_edges_of_element(const int32_t *__restrict__
   if (n > 0) body(n);
 }
 
+// 32 bytes of one lane in one store.  The lanes of a result tile hold 64 bytes of a row each: in 16-byte stores every
+// instruction half-fills 32 sectors, which L2 takes as 2.5 times the writes (10.2 million sectors for 131 MB).
+__device__ __forceinline__ void store32(float *p, float a, float b, float c, float d, float e, float f, float g, float h) {
+  asm volatile("st.global.v8.f32 [%0], {%1, %2, %3, %4, %5, %6, %7, %8};" ::"l"(p), "f"(a), "f"(b), "f"(c), "f"(d), "f"(e),
+               "f"(f), "f"(g), "f"(h)
+               : "memory");
+}
+__device__ __forceinline__ void store32(double *p, double a, double b, double c, double d) {
+  asm volatile("st.global.v4.f64 [%0], {%1, %2, %3, %4};" ::"l"(p), "d"(a), "d"(b), "d"(c), "d"(d) : "memory");
+}
+
+// and in one load
+__device__ __forceinline__ void load32(const float *p, float4 &a, float4 &b) {
+  asm("ld.global.nc.v8.f32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];"
+      : "=f"(a.x), "=f"(a.y), "=f"(a.z), "=f"(a.w), "=f"(b.x), "=f"(b.y), "=f"(b.z), "=f"(b.w)
+      : "l"(p));
+}
+__device__ __forceinline__ void load_row16(const float *p, float (&v)[16]) {
+#pragma unroll
+  for (int i = 0; i < 2; i++) {
+    float4 a, b;
+    load32(p + 8 * i, a, b);
+    v[8 * i] = a.x, v[8 * i + 1] = a.y, v[8 * i + 2] = a.z, v[8 * i + 3] = a.w;
+    v[8 * i + 4] = b.x, v[8 * i + 5] = b.y, v[8 * i + 6] = b.z, v[8 * i + 7] = b.w;
+  }
+}
+__device__ __forceinline__ void load_row16(const double *p, double (&v)[16]) {
+#pragma unroll
+  for (int i = 0; i < 4; i++)
+    asm("ld.global.nc.v4.f64 {%0, %1, %2, %3}, [%4];"
+        : "=d"(v[4 * i]), "=d"(v[4 * i + 1]), "=d"(v[4 * i + 2]), "=d"(v[4 * i + 3])
+        : "l"(p + 4 * i));
+}
+__device__ __forceinline__ void store_quad(float *p, float a, float b, float c) {
+  *reinterpret_cast<float4 *>(p) = make_float4(a, b, c, 0.f);
+}
+__device__ __forceinline__ void store_quad(double *p, double a, double b, double c) { store32(p, a, b, c, 0.0); }
+
 // 3-term TF32 split for mma.sync m16n8k8: x = hi + lo, hi by truncation, lo rounded
 __device__ __forceinline__ void split_tf32(float x, uint32_t &hi, uint32_t &lo) {
   hi = __float_as_uint(x) & 0xFFFFE000u;
@@ -363,11 +401,11 @@ __global__ void __launch_bounds__(SU_WARPS * 32)
   float *o = A + (int64_t)slot_of[node] * 16 * width + z * ST_H + 16 * t;
 #pragma unroll
   for (int half = 0; half < 2; half++) {   // rows lm = g and g + 8
-    float4 *row = reinterpret_cast<float4 *>(o + (int64_t)(g + 8 * half) * width);
+    float *row = o + (int64_t)(g + 8 * half) * width;
 #pragma unroll
     for (int u = 0; u < 2; u++) {
-      row[2 * u] = make_float4(acc[0][2 * half + u], acc[1][2 * half + u], acc[2][2 * half + u], acc[3][2 * half + u]);
-      row[2 * u + 1] = make_float4(acc[4][2 * half + u], acc[5][2 * half + u], acc[6][2 * half + u], acc[7][2 * half + u]);
+      const int c = 2 * half + u;
+      store32(row + 8 * u, acc[0][c], acc[1][c], acc[2][c], acc[3][c], acc[4][c], acc[5][c], acc[6][c], acc[7][c]);
     }
   }
 }
@@ -435,12 +473,12 @@ __global__ void __launch_bounds__(SU_WARPS * 32)
   float *o = A + (int64_t)slot_of[node] * 16 * width + z * ST_H + 16 * t;
 #pragma unroll
   for (int half = 0; half < 2; half++) {   // rows lm = g and g + 8
-    float4 *row = reinterpret_cast<float4 *>(o + (int64_t)(g + 8 * half) * width);
+    float *row = o + (int64_t)(g + 8 * half) * width;
 #pragma unroll
     for (int u = 0; u < 2; u++) {
       const int c = 2 * half + u;
-      row[2 * u] = make_float4(acc[0][c] * factor, acc[1][c] * factor, acc[2][c] * factor, acc[3][c] * factor);
-      row[2 * u + 1] = make_float4(acc[4][c] * factor, acc[5][c] * factor, acc[6][c] * factor, acc[7][c] * factor);
+      store32(row + 8 * u, acc[0][c] * factor, acc[1][c] * factor, acc[2][c] * factor, acc[3][c] * factor, acc[4][c] * factor,
+              acc[5][c] * factor, acc[6][c] * factor, acc[7][c] * factor);
     }
   }
 }
@@ -506,11 +544,12 @@ __global__ void __launch_bounds__(SU_WARPS * 32)
   double *o = A + (int64_t)slot_of[node] * 16 * width + z * ST_H + 16 * t;
 #pragma unroll
   for (int i = 0; i < 2; i++) {
-    double2 *row = reinterpret_cast<double2 *>(o + (int64_t)(g + 8 * i) * width);
+    double *row = o + (int64_t)(g + 8 * i) * width;
 #pragma unroll
     for (int u = 0; u < 2; u++)
 #pragma unroll
-      for (int j = 0; j < 4; j++) row[4 * u + j] = make_double2(acc[i][2 * j][u], acc[i][2 * j + 1][u]);
+      for (int j = 0; j < 2; j++)
+        store32(row + 8 * u + 4 * j, acc[i][4 * j][u], acc[i][4 * j + 1][u], acc[i][4 * j + 2][u], acc[i][4 * j + 3][u]);
   }
 }
 
@@ -536,23 +575,15 @@ template <typename T>
 __device__ __forceinline__ void finish_edge(const T *st, int64_t e, const T *__restrict__ gY1, const T *__restrict__ dr1,
                                             const Quad<T> *__restrict__ geo, T *__restrict__ gvec) {
   T g[16];
-  const Quad<T> *gy = reinterpret_cast<const Quad<T> *>(gY1 + e * 16);
-#pragma unroll
-  for (int i = 0; i < 4; i++) {
-    const Quad<T> q = gy[i];
-    g[4 * i] = st[4 * i] + q.x;
-    g[4 * i + 1] = st[4 * i + 1] + q.y;
-    g[4 * i + 2] = st[4 * i + 2] + q.z;
-    g[4 * i + 3] = st[4 * i + 3] + q.w;
-  }
+  load_row16(gY1 + e * 16, g);
   // without an array of its own the second layer's dE/dr is component 0 of its grad Y (Y_00 is constant)
-  const T dr = st[16] + (dr1 != nullptr ? dr1[e] : gy[0].x);
+  const T dr = st[16] + (dr1 != nullptr ? dr1[e] : g[0]);
+#pragma unroll
+  for (int i = 0; i < 16; i++) g[i] += st[i];
   const Quad<T> q = geo[e];   // unit vector in the input's component order: harmonic axes are (z, x, y)
   T GX, GY, GZ;
   sph_l3_vjp<T>(q.z, q.x, q.y, g, GX, GY, GZ);
-  gvec[e * 3] = GY * q.w + dr * q.x;
-  gvec[e * 3 + 1] = GZ * q.w + dr * q.y;
-  gvec[e * 3 + 2] = GX * q.w + dr * q.z;
+  store_quad(gvec + e * 4, GY * q.w + dr * q.x, GZ * q.w + dr * q.y, GX * q.w + dr * q.z);
 }
 
 // float32: eight edges at a time on the warp-level tensor instruction, D = P h^T and P h'^T.  P [16 x 64] stays in
@@ -696,7 +727,7 @@ __global__ void __launch_bounds__(SU_WARPS * 32, 4)
       for (int r = 0; r < 2; r++)
 #pragma unroll
         for (int u = 0; u < 2; u++) {
-          v[i][r][u] = __ldg(reinterpret_cast<const float4 *>(p + (g + 8 * r) * width + 32 * i + 4 * u));
+          if (u == 0) load32(p + (g + 8 * r) * width + 32 * i, v[i][r][0], v[i][r][1]);
           most = fmaxf(most, fmaxf(fmaxf(fabsf(v[i][r][u].x), fabsf(v[i][r][u].y)), fmaxf(fabsf(v[i][r][u].z), fabsf(v[i][r][u].w))));
         }
 #pragma unroll
@@ -971,15 +1002,17 @@ __global__ void __launch_bounds__(256)
   double ax = 0.0, ay = 0.0, az = 0.0;
   for (int k = send_ptr[n] + lane; k < send_ptr[n + 1]; k += 32) {
     const int64_t e = perm[k];
-    ax += (double)g[e * 3];
-    ay += (double)g[e * 3 + 1];
-    az += (double)g[e * 3 + 2];
+    const Quad<T> q = reinterpret_cast<const Quad<T> *>(g)[e];
+    ax += (double)q.x;
+    ay += (double)q.y;
+    az += (double)q.z;
   }
   if (n < nrecv) {
     for (int64_t e = row_ptr[n] + lane; e < row_ptr[n + 1]; e += 32) {
-      ax -= (double)g[e * 3];
-      ay -= (double)g[e * 3 + 1];
-      az -= (double)g[e * 3 + 2];
+      const Quad<T> q = reinterpret_cast<const Quad<T> *>(g)[e];
+      ax -= (double)q.x;
+      ay -= (double)q.y;
+      az -= (double)q.z;
     }
   }
 #pragma unroll
