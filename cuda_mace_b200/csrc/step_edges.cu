@@ -261,18 +261,40 @@ int StepKernels<T>::edge_prep(const double *pos, const int32_t *sender, const in
 
 // ---- the edges of one (receiver, element) pair -------------------------------------------------------------------
 // A warp owns the pair.  It lists the edges whose sender has the element, 32 candidates at a time (ballot), into a
-// per-warp buffer and calls body(list, n) whenever the buffer is full and at the end; edges come in list order.
+// per-warp buffer and calls body(list, n) whenever the buffer is full and at the end; edges come in list order.  The elements
+// of the first 64 edges' senders are two dependent loads that the caller starts before it waits for anything else
+// (SenderElements): a pair's life is a chain of such loads and little work.
 constexpr int SU_WARPS = 4;
 constexpr int SU_LIST = 64;
 
+struct SenderElements {
+  const int32_t *__restrict__ sender, *__restrict__ species;
+  int64_t e0, e1;
+  int32_t s[2];
+  int lane;
+  __device__ __forceinline__ SenderElements(const int32_t *__restrict__ sender_, const int32_t *__restrict__ species_,
+                                            int64_t e0_, int64_t e1_, int lane_)
+      : sender(sender_), species(species_), e0(e0_), e1(e1_), lane(lane_) {
+#pragma unroll
+    for (int c = 0; c < 2; c++) s[c] = e0 + 32 * c + lane < e1 ? __ldg(sender + e0 + 32 * c + lane) : -1;
+  }
+  __device__ __forceinline__ void look_up() {   // the elements in place of the senders
+#pragma unroll
+    for (int c = 0; c < 2; c++) s[c] = s[c] >= 0 ? __ldg(species + s[c]) : -1;
+  }
+};
+
 template <typename Body>
-__device__ __forceinline__ void for_edges_of_element(const int32_t *__restrict__ sender,
-                                                     const int32_t *__restrict__ species, int64_t e0, int64_t e1, int z,
-                                                     int32_t *list, int lane, Body body) {
+__device__ __forceinline__ void for_edges_of_element(const SenderElements &from, int z, int32_t *list, Body body) {
+  const int lane = from.lane;
   int n = 0;
-  for (int64_t eb = e0; eb < e1; eb += 32) {
+  for (int64_t eb = from.e0; eb < from.e1; eb += 32) {
     const int64_t e = eb + lane;
-    const bool hit = e < e1 && species[sender[e]] == z;
+    int of = -1;
+    if (eb == from.e0) of = from.s[0];
+    else if (eb == from.e0 + 32) of = from.s[1];
+    else if (e < from.e1) of = __ldg(from.species + __ldg(from.sender + e));
+    const bool hit = of == z;
     const unsigned m = __ballot_sync(0xffffffffu, hit);
     if (hit) list[n + __popc(m & ((1u << lane) - 1u))] = (int32_t)e;
     n += __popc(m);
@@ -353,11 +375,13 @@ __global__ void __launch_bounds__(SU_WARPS * 32)
   if (pair >= nnodes * elements) return;
   const int64_t node = pair / elements;
   const int z = (int)(pair - node * elements);
+  SenderElements from(sender, species, row_ptr[node], row_ptr[node + 1], lane);
   int32_t *list = lists[w];
   float acc[8][4];
 #pragma unroll
   for (int j = 0; j < 8; j++) acc[j][0] = acc[j][1] = acc[j][2] = acc[j][3] = 0.f;
-  for_edges_of_element(sender, species, row_ptr[node], row_ptr[node + 1], z, list, lane, [&](int n) {
+  from.look_up();
+  for_edges_of_element(from, z, list, [&](int n) {
     float4 hv[2][2];
     float yv[4];
     auto load = [&](int j0) {   // edges j0 + t and j0 + t + 4; past the end: the last edge with Y = 0
@@ -434,11 +458,13 @@ __global__ void __launch_bounds__(SU_WARPS * 32)
   if (pair >= nnodes * elements) return;
   const int64_t node = pair / elements;
   const int z = (int)(pair - node * elements);
+  SenderElements from(sender, species, row_ptr[node], row_ptr[node + 1], lane);
   int32_t *list = lists[w];
   float acc[8][4];
 #pragma unroll
   for (int j = 0; j < 8; j++) acc[j][0] = acc[j][1] = acc[j][2] = acc[j][3] = 0.f;
-  for_edges_of_element(sender, species, row_ptr[node], row_ptr[node + 1], z, list, lane, [&](int n) {
+  from.look_up();
+  for_edges_of_element(from, z, list, [&](int n) {
     for (int j0 = 0; j0 < n; j0 += 16) {
       uint4 hv[4], lv[4];
       uint32_t ah[4], al[4];
@@ -507,11 +533,13 @@ __global__ void __launch_bounds__(SU_WARPS * 32)
   if (pair >= nnodes * elements) return;
   const int64_t node = pair / elements;
   const int z = (int)(pair - node * elements);
+  SenderElements from(sender, species, row_ptr[node], row_ptr[node + 1], lane);
   int32_t *list = lists[w];
   double acc[2][8][2];
 #pragma unroll
   for (int j = 0; j < 8; j++) acc[0][j][0] = acc[0][j][1] = acc[1][j][0] = acc[1][j][1] = 0.0;
-  for_edges_of_element(sender, species, row_ptr[node], row_ptr[node + 1], z, list, lane, [&](int n) {
+  from.look_up();
+  for_edges_of_element(from, z, list, [&](int n) {
     double2 hv[4];
     double yv[2];
     auto load = [&](int j0) {   // edge j0 + t; past the end: the last edge with Y = 0
@@ -605,6 +633,7 @@ __global__ void __launch_bounds__(SU_WARPS * 32, 3)
   if (pair >= nnodes * elements) return;
   const int64_t node = pair / elements;
   const int z = (int)(pair - node * elements);
+  SenderElements from(sender, species, row_ptr[node], row_ptr[node + 1], lane);
   int32_t *list = lists[w];
   float *st = stage[w];
   uint32_t ph[8][4], pl[8][4];   // A fragments of the 8 K steps
@@ -625,7 +654,8 @@ __global__ void __launch_bounds__(SU_WARPS * 32, 3)
       split_tf32(v.w, ph[2 * q + 1][3], pl[2 * q + 1][3]);
     }
   }
-  for_edges_of_element(sender, species, row_ptr[node], row_ptr[node + 1], z, list, lane, [&](int n) {
+  from.look_up();
+  for_edges_of_element(from, z, list, [&](int n) {
     for (int j0 = 0; j0 < n; j0 += 32) {
       const int nj = n - j0 < 32 ? n - j0 : 32;
       float4 hv[4], dv[4];
@@ -713,6 +743,7 @@ __global__ void __launch_bounds__(SU_WARPS * 32, 4)
   if (pair >= nnodes * elements) return;
   const int64_t node = pair / elements;
   const int z = (int)(pair - node * elements);
+  SenderElements from(sender, species, row_ptr[node], row_ptr[node + 1], lane);
   int32_t *list = lists[w];
   float *st = stage[w];
   uint32_t ph[4][4], pl[4][4];   // A fragments of the 4 K steps
@@ -724,10 +755,14 @@ __global__ void __launch_bounds__(SU_WARPS * 32, 4)
 #pragma unroll
     for (int i = 0; i < 2; i++)
 #pragma unroll
+      for (int r = 0; r < 2; r++) load32(p + (g + 8 * r) * width + 32 * i, v[i][r][0], v[i][r][1]);
+    from.look_up();
+#pragma unroll
+    for (int i = 0; i < 2; i++)
+#pragma unroll
       for (int r = 0; r < 2; r++)
 #pragma unroll
         for (int u = 0; u < 2; u++) {
-          if (u == 0) load32(p + (g + 8 * r) * width + 32 * i, v[i][r][0], v[i][r][1]);
           most = fmaxf(most, fmaxf(fmaxf(fabsf(v[i][r][u].x), fabsf(v[i][r][u].y)), fmaxf(fabsf(v[i][r][u].z), fabsf(v[i][r][u].w))));
         }
 #pragma unroll
@@ -748,7 +783,7 @@ __global__ void __launch_bounds__(SU_WARPS * 32, 4)
           split_half2(mul2(pack2(v[i][r][u].z, v[i][r][u].w), sc2), ph[2 * i + u][2 + r], pl[2 * i + u][2 + r]);
         }
   }
-  for_edges_of_element(sender, species, row_ptr[node], row_ptr[node + 1], z, list, lane, [&](int n) {
+  for_edges_of_element(from, z, list, [&](int n) {
     for (int j0 = 0; j0 < n; j0 += 32) {
       const int nj = n - j0 < 32 ? n - j0 : 32;
       uint4 hh[2], hl[2], dd[2], dl[2];
@@ -839,6 +874,7 @@ __global__ void __launch_bounds__(SU_WARPS * 32)
   if (pair >= nnodes * elements) return;
   const int64_t node = pair / elements;
   const int z = (int)(pair - node * elements);
+  SenderElements from(sender, species, row_ptr[node], row_ptr[node + 1], lane);
   int32_t *list = lists[w];
   double *st = stage[w];
   double2 P[2][8];
@@ -850,7 +886,8 @@ __global__ void __launch_bounds__(SU_WARPS * 32)
 #pragma unroll
       for (int q = 0; q < 8; q++) P[i][q] = __ldg(reinterpret_cast<const double2 *>(p + (g + 8 * i) * width) + q);
   }
-  for_edges_of_element(sender, species, row_ptr[node], row_ptr[node + 1], z, list, lane, [&](int n) {
+  from.look_up();
+  for_edges_of_element(from, z, list, [&](int n) {
     for (int j0 = 0; j0 < n; j0 += 32) {
       const int nj = n - j0 < 32 ? n - j0 : 32;
       for (int j = 0; j < nj; j += 8) {
@@ -1000,19 +1037,29 @@ __global__ void __launch_bounds__(256)
   const int64_t n = (int64_t)(blockIdx.x - 1) * 8 + w;
   if (n >= nsend) return;
   double ax = 0.0, ay = 0.0, az = 0.0;
-  for (int k = send_ptr[n] + lane; k < send_ptr[n + 1]; k += 32) {
-    const int64_t e = perm[k];
-    const Quad<T> q = reinterpret_cast<const Quad<T> *>(g)[e];
-    ax += (double)q.x;
-    ay += (double)q.y;
-    az += (double)q.z;
-  }
-  if (n < nrecv) {
-    for (int64_t e = row_ptr[n] + lane; e < row_ptr[n + 1]; e += 32) {
-      const Quad<T> q = reinterpret_cast<const Quad<T> *>(g)[e];
-      ax -= (double)q.x;
-      ay -= (double)q.y;
-      az -= (double)q.z;
+  const Quad<T> *gq = reinterpret_cast<const Quad<T> *>(g);
+  const bool receives = n < nrecv;
+  const int64_t k0 = send_ptr[n], k1 = send_ptr[n + 1];
+  const int64_t r0 = receives ? row_ptr[n] : 0, r1 = receives ? row_ptr[n + 1] : 0;
+  // 64 edges of either grouping at a time: the indices of the one are on their way with the gradients of the other
+  for (int64_t b = 0; b < k1 - k0 || b < r1 - r0; b += 64) {
+    int32_t e[2];
+    Quad<T> in[2], out_q[2];
+    bool has[2], had[2];
+#pragma unroll
+    for (int u = 0; u < 2; u++) {
+      has[u] = k0 + b + 32 * u + lane < k1;
+      had[u] = r0 + b + 32 * u + lane < r1;
+      if (has[u]) e[u] = perm[k0 + b + 32 * u + lane];
+      if (had[u]) in[u] = gq[r0 + b + 32 * u + lane];
+    }
+#pragma unroll
+    for (int u = 0; u < 2; u++)
+      if (has[u]) out_q[u] = gq[e[u]];
+#pragma unroll
+    for (int u = 0; u < 2; u++) {
+      if (has[u]) ax += (double)out_q[u].x, ay += (double)out_q[u].y, az += (double)out_q[u].z;
+      if (had[u]) ax -= (double)in[u].x, ay -= (double)in[u].y, az -= (double)in[u].z;
     }
   }
 #pragma unroll
