@@ -342,6 +342,7 @@ __device__ __forceinline__ void load_row16(const double *p, double (&v)[16]) {
         : "=d"(v[4 * i]), "=d"(v[4 * i + 1]), "=d"(v[4 * i + 2]), "=d"(v[4 * i + 3])
         : "l"(p + 4 * i));
 }
+__device__ __forceinline__ void prefetch_l1(const void *p) { asm volatile("prefetch.global.L1 [%0];" ::"l"(p)); }
 __device__ __forceinline__ void store_quad(float *p, float a, float b, float c) {
   *reinterpret_cast<float4 *>(p) = make_float4(a, b, c, 0.f);
 }
@@ -658,6 +659,10 @@ __global__ void __launch_bounds__(SU_WARPS * 32, 3)
   for_edges_of_element(from, z, list, [&](int n) {
     for (int j0 = 0; j0 < n; j0 += 32) {
       const int nj = n - j0 < 32 ? n - j0 : 32;
+      if (lane < nj) {   // what finish_edge reads
+        prefetch_l1(gY1 + (int64_t)list[j0 + lane] * 16);
+        prefetch_l1(geo + list[j0 + lane]);
+      }
       float4 hv[4], dv[4];
       auto load = [&](int j) {   // edge j0 + j + g, or the last one
         const int i = j0 + j + g;
@@ -786,6 +791,10 @@ __global__ void __launch_bounds__(SU_WARPS * 32, 4)
   for_edges_of_element(from, z, list, [&](int n) {
     for (int j0 = 0; j0 < n; j0 += 32) {
       const int nj = n - j0 < 32 ? n - j0 : 32;
+      if (lane < nj) {   // what finish_edge reads
+        prefetch_l1(gY1 + (int64_t)list[j0 + lane] * 16);
+        prefetch_l1(geo + list[j0 + lane]);
+      }
       uint4 hh[2], hl[2], dd[2], dl[2];
       auto load = [&](int j) {   // edge j0 + j + g, or the last one
         const int i = j0 + j + g;
@@ -890,6 +899,10 @@ __global__ void __launch_bounds__(SU_WARPS * 32)
   for_edges_of_element(from, z, list, [&](int n) {
     for (int j0 = 0; j0 < n; j0 += 32) {
       const int nj = n - j0 < 32 ? n - j0 : 32;
+      if (lane < nj) {   // what finish_edge reads
+        prefetch_l1(gY1 + (int64_t)list[j0 + lane] * 16);
+        prefetch_l1(geo + list[j0 + lane]);
+      }
       for (int j = 0; j < nj; j += 8) {
         const int i = j0 + j + g;   // this lane's row of h: that edge, or the last one
         const int64_t e = list[i < n ? i : n - 1];
