@@ -98,6 +98,9 @@ struct GemmArgs {
   int g_stage_bytes;            // GRADR: shared memory behind the ring and the epilogue buffers for staged G rows
   int b_slots;                  // GRADR: depth of the separate ring of B blocks behind the staged G rows
   int lin_tma;                  // LINEAR: rows move by TMA through rank-3 tensor maps (nodes in storage order)
+  int lin_blocks;               // LINEAR with lin_tma: products of the same rows; block b has matrices b * 4 nelements .. and
+                                // writes [M, 16, N] behind the blocks before.  The block is the fastest tile index, so the
+                                // CTAs that read the same rows do so at the same time and all but the first find them in L2.
 };
 
 // LINEAR with lin_tma: [nodes, 16, K] in and [nodes, 16, N] out, per l a box of (columns, 2l+1 components, nodes)
@@ -114,6 +117,7 @@ struct Tile {
   int64_t seg_begin;  // LINEAR: first slot of the element in node_order
   int64_t seg_rows;   // LINEAR: rows of the problem
   int l, nl, mat, ntile;
+  int64_t block_node;  // LINEAR with lin_tma: first node of the tile's block in the output
   int64_t node0;      // LINEAR with lin_tma: first node slot of the tile; quarter q holds nodes node0 + q nq .. + nq - 1
   int64_t node_end;   //   one past the last node of the tile's (element, l) problem
   int nq;
@@ -180,6 +184,13 @@ struct TileWalker {
     ntile = 0;
     rt_step = 0;
     nt_step = 0;
+    if (MODE == GT_MODE_LINEAR) {
+      n_tiles = g.lin_blocks;
+      rt = blockIdx.x / (uint32_t)n_tiles;
+      ntile = (int)(blockIdx.x - (uint32_t)rt * (uint32_t)n_tiles);
+      rt_step = gridDim.x / (uint32_t)n_tiles;
+      nt_step = (int)(gridDim.x - (uint32_t)rt_step * (uint32_t)n_tiles);
+    }
     if (MODE != GT_MODE_LINEAR) {
       rt = blockIdx.x / (uint32_t)n_tiles;
       ntile = (int)(blockIdx.x - (uint32_t)rt * (uint32_t)n_tiles);
@@ -192,13 +203,11 @@ struct TileWalker {
   __device__ __forceinline__ bool next(Tile &T) {
     if (started) {
       t += gridDim.x;
-      if (MODE != GT_MODE_LINEAR) {
-        rt += rt_step;
-        ntile += nt_step;
-        if (ntile >= n_tiles) {
-          ntile -= n_tiles;
-          rt++;
-        }
+      rt += rt_step;
+      ntile += nt_step;
+      if (ntile >= n_tiles) {
+        ntile -= n_tiles;
+        rt++;
       }
     }
     started = true;
@@ -216,7 +225,7 @@ struct TileWalker {
       T.valid = true;
       return true;
     }
-    while (prob < nprob && t >= tab->tile_begin[prob + 1]) {
+    while (prob < nprob && rt >= tab->tile_begin[prob + 1]) {
       prob++;
       if (++z == nelements) {
         z = 0;
@@ -224,15 +233,16 @@ struct TileWalker {
       }
     }
     if (prob >= nprob) return false;
-    T.row0 = (t - tab->tile_begin[prob]) * GT_TILE_M;
+    T.row0 = (rt - tab->tile_begin[prob]) * GT_TILE_M;
     T.nq = lin_nodes_per_quarter(l);
-    T.node0 = tab->seg_begin[prob] + (t - tab->tile_begin[prob]) * 4 * T.nq;
+    T.node0 = tab->seg_begin[prob] + (rt - tab->tile_begin[prob]) * 4 * T.nq;
     T.node_end = tab->seg_begin[prob] + tab->seg_rows[prob] / (2 * l + 1);
     T.seg_begin = tab->seg_begin[prob];
     T.seg_rows = tab->seg_rows[prob];
     T.l = l;
     T.nl = 2 * l + 1;
-    T.mat = z * 4 + l;
+    T.mat = ntile * nprob + z * 4 + l;
+    T.block_node = ntile * M;
     T.ntile = 0;
     T.valid = true;
     return true;
@@ -1170,7 +1180,7 @@ __global__ void __launch_bounds__((GT_PRODUCER_WARPS + 1 + EW + 1) * 32, 1)
             if (!whole) {
               const int node = node_q + lane / T.nl, m = lane - (lane / T.nl) * T.nl;
               if (lane < T.nq * T.nl && node < T.node_end) {
-                float *o = g.out + ((int64_t)node * 16 + T.l * T.l + m) * g.N + n0 + cc;
+                float *o = g.out + ((T.block_node + node) * 16 + T.l * T.l + m) * g.N + n0 + cc;
 #pragma unroll
                 for (int c = 0; c < 4; c++)
                   if (cc + 4 * c < ncols)
@@ -1190,7 +1200,7 @@ __global__ void __launch_bounds__((GT_PRODUCER_WARPS + 1 + EW + 1) * 32, 1)
                            : "memory");
             fence_proxy_async();
             __syncwarp();
-            if (elect_one()) tma_store_3d(&lin_maps.out[T.l], n0 + cc, T.l * T.l, node_q, stg);
+            if (elect_one()) tma_store_3d(&lin_maps.out[T.l], n0 + cc, T.l * T.l, (int)T.block_node + node_q, stg);
           }
         }
       } else {
@@ -1488,11 +1498,12 @@ static int gemm_launch(GemmArgs &g, const char *what, cudaStream_t st) {
   if (g.lin_tma) {
     for (int l = 0; l < 4; l++) {
       if (int rc = encode_node_tensor_map(&lin_maps.in[l], g.A, g.M, g.K, l, GT_KBLOCK, CU_TENSOR_MAP_SWIZZLE_128B, what)) return rc;
-      if (int rc = encode_node_tensor_map(&lin_maps.out[l], g.out, g.M, g.N, l, 16, CU_TENSOR_MAP_SWIZZLE_64B, what)) return rc;
+      if (int rc = encode_node_tensor_map(&lin_maps.out[l], g.out, g.M * g.lin_blocks, g.N, l, 16, CU_TENSOR_MAP_SWIZZLE_64B, what)) return rc;
     }
     // tiles hold whole nodes: 128, 40, 24 and 16 of them for l = 0 .. 3
     g.total_tiles = 4 * (int64_t)g.nelements;
     for (int l = 0; l < 4; l++) g.total_tiles += g.M / (4 * lin_nodes_per_quarter(l)) + 1;
+    g.total_tiles *= g.lin_blocks;
   }
   CUtensorMap tmap, tmap_out;
   memset(&tmap, 0, sizeof(tmap));
@@ -1525,6 +1536,31 @@ static int gemm_launch(GemmArgs &g, const char *what, cudaStream_t st) {
   const int nthreads = g.mode == GT_MODE_GRADR ? (GT_PRODUCER_WARPS + 1 + 4 + 1) * 32 : GT_THREADS;
   launch_chained(kern, (unsigned)blocks, nthreads, smem, st, g, tmap, tmap_out, lin_maps);
   return check_launch(what);
+}
+
+// nblocks > 1: no node_order
+int linear_tc(const float *X, const float *packed, const int32_t *node_order, const int32_t *elem_start, int nelements,
+              int nblocks, int64_t nnodes, int K, int Nout, double scale, float *out, int32_t *status, cudaStream_t stream) {
+  if (nnodes < 0 || K < 1 || Nout < 1 || nelements < 1) return fail(CMACE_ERR_ARG, "cmace_linear_tc: bad size");
+  if (nnodes > 0x7fffffffLL / 16 / nblocks) return fail(CMACE_ERR_UNSUPPORTED, "cmace_linear_tc: too many nodes");
+  if (K % 8 != 0 || Nout % 4 != 0 || Nout > 128)
+    return fail(CMACE_ERR_UNSUPPORTED, "cmace_linear_tc: K multiple of 8, Nout multiple of 4 and Nout <= 128");
+  if (4 * nelements > GT_MAX_PROBLEMS)
+    return fail(CMACE_ERR_UNSUPPORTED, "cmace_linear_tc: at most %d elements", GT_MAX_PROBLEMS / 4);
+  if (nnodes == 0) return CMACE_OK;
+  if (!X || !packed || !out) return fail(CMACE_ERR_ARG, "cmace_linear_tc: null pointer");
+  if ((nelements > 1) != (elem_start != nullptr) || (node_order != nullptr && elem_start == nullptr))
+    return fail(CMACE_ERR_ARG, "cmace_linear_tc: elem_start goes with nelements > 1, node_order only with elem_start");
+  if (!aligned16(X) || !aligned16(packed) || !aligned16(out))
+    return fail(CMACE_ERR_ARG, "cmace_linear_tc: pointers must be 16-byte aligned");
+  const PackGeom p = pack_geom(Nout, K);
+  GemmArgs g{};
+  g.A = X; g.packed = packed; g.out = out; g.status = status;
+  g.node_order = node_order; g.elem_start = elem_start;
+  g.M = nnodes; g.K = K; g.N = Nout; g.nelements = nelements; g.mode = GT_MODE_LINEAR; g.lin_blocks = nblocks; g.scale = (float)scale;
+  g.n_tiles = p.n_tiles; g.k_blocks = p.k_blocks; g.npad = p.npad;
+  g.total_tiles = (nnodes * 16 + GT_TILE_M - 1) / GT_TILE_M + 4 * (int64_t)nelements;
+  return gemm_launch(g, "cmace_linear_tc", stream);
 }
 
 int gemm3x_gradr(const float *X, const float *G, const float *Y, ImpLayout ys, const int32_t *sender,
@@ -1611,25 +1647,6 @@ int cmace_gemm3x_gradr_f32(const float *X, const float *G, const float *Y, const
 int cmace_linear_tc_f32(const float *X, const float *packed, const int32_t *node_order, const int32_t *elem_start,
                         int nelements, int64_t nnodes, int K, int Nout, double scale, float *out, int32_t *status,
                         cmace_stream_t stream) {
-  if (nnodes < 0 || K < 1 || Nout < 1 || nelements < 1) return fail(CMACE_ERR_ARG, "cmace_linear_tc: bad size");
-  if (nnodes > 0x7fffffffLL / 16) return fail(CMACE_ERR_UNSUPPORTED, "cmace_linear_tc: too many nodes");
-  if (K % 8 != 0 || Nout % 4 != 0 || Nout > 128)
-    return fail(CMACE_ERR_UNSUPPORTED, "cmace_linear_tc: K multiple of 8, Nout multiple of 4 and Nout <= 128");
-  if (4 * nelements > GT_MAX_PROBLEMS)
-    return fail(CMACE_ERR_UNSUPPORTED, "cmace_linear_tc: at most %d elements", GT_MAX_PROBLEMS / 4);
-  if (nnodes == 0) return CMACE_OK;
-  if (!X || !packed || !out) return fail(CMACE_ERR_ARG, "cmace_linear_tc: null pointer");
-  if ((nelements > 1) != (elem_start != nullptr) || (node_order != nullptr && elem_start == nullptr))
-    return fail(CMACE_ERR_ARG, "cmace_linear_tc: elem_start goes with nelements > 1, node_order only with elem_start");
-  if (!aligned16(X) || !aligned16(packed) || !aligned16(out))
-    return fail(CMACE_ERR_ARG, "cmace_linear_tc: pointers must be 16-byte aligned");
-  const PackGeom p = pack_geom(Nout, K);
-  GemmArgs g{};
-  g.A = X; g.packed = packed; g.out = out; g.status = status;
-  g.node_order = node_order; g.elem_start = elem_start;
-  g.M = nnodes; g.K = K; g.N = Nout; g.nelements = nelements; g.mode = GT_MODE_LINEAR; g.scale = (float)scale;
-  g.n_tiles = p.n_tiles; g.k_blocks = p.k_blocks; g.npad = p.npad;
-  g.total_tiles = (nnodes * 16 + GT_TILE_M - 1) / GT_TILE_M + 4 * (int64_t)nelements;
-  return gemm_launch(g, "cmace_linear_tc", (cudaStream_t)stream);
+  return linear_tc(X, packed, node_order, elem_start, nelements, 1, nnodes, K, Nout, scale, out, status, (cudaStream_t)stream);
 }
 }

@@ -141,6 +141,9 @@ struct Workspace {
   }
 };
 
+int linear_tc(const float *X, const float *packed, const int32_t *node_order, const int32_t *elem_start, int nelements,
+              int nblocks, int64_t nnodes, int K, int Nout, double scale, float *out, int32_t *status, cudaStream_t stream);
+
 static int linear_any(const float *X, const void *W, const int32_t *start, int nel, int64_t n, int K, int N, float *out,
                       int32_t *status, cmace_stream_t st) {
   return cmace_linear_tc_f32(X, static_cast<const float *>(W), nullptr, start, nel, n, K, N, 1.0, out, status, st);
@@ -285,7 +288,16 @@ static int run_step(const cmace_step_model &m, cmace_step_io &io, const Workspac
     case S_CONTRACT0_BACK:
       return K::contract_bwd(w.m0, w.slot_type, static_cast<const T *>(m.weff[0]), w.gb0, n, C, w.gX0, st);
     case S_FOLD_BACK:
-      for (int b = 0; 2 * b < Z; b++) {
+      // float32: the blocks of two elements in one launch, which reads the rows from memory once
+      if constexpr (!f64) {
+        if (Z >= 4) {
+          if (int rc = linear_tc(w.gX0, static_cast<const float *>(m.fold_back[0]), nullptr, start, Z, Z / 2, n, C, 128, 1.0, w.gA,
+                                 io.status, st))
+            return rc;
+          if (Z % 2 == 0) return CMACE_OK;
+        }
+      }
+      for (int b = !f64 && Z >= 4 ? Z / 2 : 0; 2 * b < Z; b++) {
         if (int rc = linear_any(w.gX0, m.fold_back[b], start, Z, n, C, sums_block_width(Z, b),
                                 w.gA + (int64_t)b * n * (16 * 128), io.status, st))
           return rc;

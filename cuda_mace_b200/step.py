@@ -215,8 +215,14 @@ class StepPlan:
         w4 = d(L0.W_radial3).view(_H, 4, C)
         fold = torch.einsum("zc,klc,rlcd->rlzkd", x, w4, lin).reshape(Z, 4, Z * _H, C)
         m.fold = matrix(fold)
-        for b in range((Z + 1) // 2):
-            m.fold_back[b] = matrix(fold[:, :, 2 * b * _H: min(2 * b + 2, Z) * _H].transpose(-1, -2))
+        blocks = [fold[:, :, 2 * b * _H: min(2 * b + 2, Z) * _H].transpose(-1, -2) for b in range((Z + 1) // 2)]
+        if model.dtype == torch.float32 and Z >= 4:   # the blocks of two elements one after the other: one launch takes them
+            m.fold_back[0] = matrix(torch.stack(blocks[:Z // 2]))
+            first = Z // 2
+        else:
+            first = 0
+        for b in range(first, (Z + 1) // 2):
+            m.fold_back[b] = matrix(blocks[b])
 
     def current(self):
         for d, k, t, v in self.sources:

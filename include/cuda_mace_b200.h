@@ -384,7 +384,8 @@ typedef struct cmace_step_model {
   double spline_width, spline_rmax;
   int32_t spline_intervals, reserved3;
   const void *fold;          /* first layer: [elements][4] matrices [64 elements, C] (float32: packed) */
-  const void *fold_back[8];  /* their transposes in blocks of two elements: [elements][4] [C, 128 or 64] */
+  const void *fold_back[8];  /* their transposes in blocks of two elements: [elements][4] [C, 128 or 64]; float32 with at
+                                least four elements: [0] holds all whole blocks, one after the other */
   const void *linear[2];     /* second layer's Linear and its transpose, [4] [C, C] (float32: packed) */
   const void *weff[2];       /* effective contraction weights of both layers [elements][13][C] */
   const void *up, *up_back;  /* first layer's product times second layer's linear_up [C, C], and its transpose */
