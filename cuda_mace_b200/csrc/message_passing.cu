@@ -28,6 +28,26 @@ constexpr int kWarpsPerBlock = 4;
 // eighth pair of edges and add up through shared memory in a fixed order: with fewer receivers than the chip holds warps
 // the walk over one receiver's edges, about 1.6 us a pair, is all there is (192 receivers, 52 edges: 43 us with one warp
 // each).
+// The 16 harmonics of a pair of edges, lane (16 h + m) -> component m of edge h, handed to all lanes through shared memory:
+// a broadcast load gives 16 bytes, a shuffle (two of them in float64) one value.  Two buffers, so that one warp barrier a
+// pair is enough.
+template <typename T, int WARPS>
+struct PairHarmonics {
+  T v[WARPS][2][32];
+};
+template <typename T>
+__device__ __forceinline__ void take16(T (&y)[16], const T *p) {
+  constexpr int V = 16 / (int)sizeof(T);
+  using Piece = typename Vec<T, V>::type;
+#pragma unroll
+  for (int i = 0; i < 16 / V; i++) {   // p is in shared memory: no read-only load
+    const Piece q = reinterpret_cast<const Piece *>(p)[i];
+    const T *s = reinterpret_cast<const T *>(&q);
+#pragma unroll
+    for (int u = 0; u < V; u++) y[V * i + u] = s[u];
+  }
+}
+
 template <typename T, int VEC, int SPLIT>
 __global__ void __launch_bounds__(SPLIT == 1 ? kWarpsPerBlock * 32 : SPLIT * 32)
     imp_fwd_kernel(const T *__restrict__ X, const T *__restrict__ Y, const T *__restrict__ R,
@@ -46,8 +66,10 @@ __global__ void __launch_bounds__(SPLIT == 1 ? kWarpsPerBlock * 32 : SPLIT * 32)
 #pragma unroll
     for (int v = 0; v < VEC; v++) acc[m][v] = T(0);
 
+  __shared__ __align__(16) PairHarmonics<T, SPLIT == 1 ? kWarpsPerBlock : SPLIT> harmonics;
+  int turn = 0;
   const int ylm = lane & 15, yedge = lane >> 4;
-  for (int64_t e = e0 + (SPLIT > 1 ? 2 * warp : 0); e < e1; e += 2 * SPLIT) {
+  for (int64_t e = e0 + (SPLIT > 1 ? 2 * warp : 0); e < e1; e += 2 * SPLIT, turn ^= 1) {
     // second edge of the pair: clamp to a valid edge, its harmonics are zeroed below
     const int64_t eb = (e + 1 < e1) ? e + 1 : e;
     const int64_t ey = yedge ? eb : e;
@@ -69,16 +91,20 @@ __global__ void __launch_bounds__(SPLIT == 1 ? kWarpsPerBlock * 32 : SPLIT * 32)
         ra[l][v] *= xa[v];
         rb[l][v] *= xb[v];
       }
+    T *yp = harmonics.v[warp][turn];
+    yp[lane] = yv;
+    __syncwarp();
+    T y[16];
+    take16<T>(y, yp);
 #pragma unroll
-    for (int m = 0; m < 16; m++) {
-      const T ya = __shfl_sync(0xffffffffu, yv, m);
-      const T yb = __shfl_sync(0xffffffffu, yv, 16 + m);
+    for (int m = 0; m < 16; m++)
 #pragma unroll
-      for (int v = 0; v < VEC; v++) {
-        acc[m][v] = fma(ya, ra[l_of_lm(m)][v], acc[m][v]);
-        acc[m][v] = fma(yb, rb[l_of_lm(m)][v], acc[m][v]);
-      }
-    }
+      for (int v = 0; v < VEC; v++) acc[m][v] = fma(y[m], ra[l_of_lm(m)][v], acc[m][v]);
+    take16<T>(y, yp + 16);
+#pragma unroll
+    for (int m = 0; m < 16; m++)
+#pragma unroll
+      for (int v = 0; v < VEC; v++) acc[m][v] = fma(y[m], rb[l_of_lm(m)][v], acc[m][v]);
   }
   T *o = out + (ys.rows ? (int64_t)ys.rows[node] : node) * 16 * C + c0;
   if constexpr (SPLIT > 1) {
@@ -127,10 +153,13 @@ __global__ void __launch_bounds__(kWarpsPerBlock * 32)
 #pragma unroll
   for (int m = 0; m < 16; m++) load_vec<T, VEC>(g[m], G + (grow * 16 + m) * C + c0);
 
+  __shared__ __align__(16) PairHarmonics<T, kWarpsPerBlock> harmonics;
+  int turn = 0;
   const int ylm = lane & 15, yedge = lane >> 4;
-  for (int64_t e = e0 + 2 * slice; e < e1; e += 2 * slices) {
+  for (int64_t e = e0 + 2 * slice; e < e1; e += 2 * slices, turn ^= 1) {
     const int64_t eb = (e + 1 < e1) ? e + 1 : e;
     const T yv = __ldg(Y + ylm * ys.m + (yedge ? eb : e) * ys.e);
+    T *yp = harmonics.v[threadIdx.x >> 5][turn];
     // loads of both edges of the pair are issued before either is consumed
     const int64_t s2[2] = {sender[e], sender[eb]};
     T xx[2][VEC], rr[2][4][VEC];
@@ -140,20 +169,23 @@ __global__ void __launch_bounds__(kWarpsPerBlock * 32)
 #pragma unroll
       for (int l = 0; l < 4; l++) load_vec_stream<T, VEC>(rr[h][l], R + ((h ? eb : e) * 4 + l) * C + c0);
     }
+    yp[lane] = yv;
+    __syncwarp();
 #pragma unroll
     for (int h = 0; h < 2; h++) {
       const int64_t ee = h ? eb : e;
       if (h && e + 1 >= e1) break;  // warp-uniform
       T(&x)[VEC] = xx[h];
       T(&r)[4][VEC] = rr[h];
-      T u[4][VEC], p[16];
+      T u[4][VEC], p[16], yy[16];
+      take16<T>(yy, yp + 16 * h);
 #pragma unroll
       for (int l = 0; l < 4; l++)
 #pragma unroll
         for (int v = 0; v < VEC; v++) u[l][v] = T(0);
 #pragma unroll
       for (int m = 0; m < 16; m++) {
-        const T y = __shfl_sync(0xffffffffu, yv, 16 * h + m);
+        const T y = yy[m];
         T pm = T(0);
 #pragma unroll
         for (int v = 0; v < VEC; v++) {
