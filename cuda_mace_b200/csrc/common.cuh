@@ -178,6 +178,26 @@ __device__ __forceinline__ unsigned long long sub2(unsigned long long a, unsigne
 }
 
 // channels handled per lane: the widest 16-byte-or-narrower vector that tiles C in 32-lane chunks
+// The 16 harmonics of a pair of edges, lane (16 h + m) -> component m of edge h, handed to all lanes through shared memory:
+// a broadcast load gives 16 bytes, a shuffle (two of them in float64) one value.  Two buffers, so that one warp barrier a
+// pair is enough.
+template <typename T, int WARPS>
+struct PairHarmonics {
+  T v[WARPS][2][32];
+};
+template <typename T>
+__device__ __forceinline__ void take16(T (&y)[16], const T *p) {
+  constexpr int V = 16 / (int)sizeof(T);
+  using Piece = typename Vec<T, V>::type;
+#pragma unroll
+  for (int i = 0; i < 16 / V; i++) {   // p is in shared memory: no read-only load
+    const Piece q = reinterpret_cast<const Piece *>(p)[i];
+    const T *s = reinterpret_cast<const T *>(&q);
+#pragma unroll
+    for (int u = 0; u < V; u++) y[V * i + u] = s[u];
+  }
+}
+
 // Sum of p[m] over the 32 lanes for all 16 m at once: after the call every lane holds the
 // total of component (lane >> 1).  16 shuffles instead of 16 * 5.
 template <typename T>

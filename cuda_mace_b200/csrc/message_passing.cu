@@ -28,28 +28,8 @@ constexpr int kWarpsPerBlock = 4;
 // eighth pair of edges and add up through shared memory in a fixed order: with fewer receivers than the chip holds warps
 // the walk over one receiver's edges, about 1.6 us a pair, is all there is (192 receivers, 52 edges: 43 us with one warp
 // each).
-// The 16 harmonics of a pair of edges, lane (16 h + m) -> component m of edge h, handed to all lanes through shared memory:
-// a broadcast load gives 16 bytes, a shuffle (two of them in float64) one value.  Two buffers, so that one warp barrier a
-// pair is enough.
-template <typename T, int WARPS>
-struct PairHarmonics {
-  T v[WARPS][2][32];
-};
-template <typename T>
-__device__ __forceinline__ void take16(T (&y)[16], const T *p) {
-  constexpr int V = 16 / (int)sizeof(T);
-  using Piece = typename Vec<T, V>::type;
-#pragma unroll
-  for (int i = 0; i < 16 / V; i++) {   // p is in shared memory: no read-only load
-    const Piece q = reinterpret_cast<const Piece *>(p)[i];
-    const T *s = reinterpret_cast<const T *>(&q);
-#pragma unroll
-    for (int u = 0; u < V; u++) y[V * i + u] = s[u];
-  }
-}
-
 template <typename T, int VEC, int SPLIT>
-__global__ void __launch_bounds__(SPLIT == 1 ? kWarpsPerBlock * 32 : SPLIT * 32)
+__global__ void __launch_bounds__(SPLIT == 1 ? kWarpsPerBlock * 32 : SPLIT * 32, SPLIT == 1 && sizeof(T) == 4 ? 4 : 1)
     imp_fwd_kernel(const T *__restrict__ X, const T *__restrict__ Y, const T *__restrict__ R,
                    const int32_t *__restrict__ sender, const int32_t *__restrict__ row_ptr,
                    int64_t nnodes, ImpLayout ys, int C, T *__restrict__ out) {

@@ -13,7 +13,7 @@
 // a cycle and scheduler), so C is a template parameter (every offset an immediate: 282 -> 180 instructions per edge and
 // 64 channels forward) and the interval is looked up once per edge (SplinePoint).  At 157 000 edges, C = 128, float32, a
 // layer: evaluating R, storing it, reading it for the messages, and in the backward reading R, storing its gradient and
-// reading that against the derivative took 78 + 75 us and 141 + 89 us; these take 95 us and 170 us.
+// reading that against the derivative took 78 + 75 us and 141 + 89 us; these take 88 us and 163 us.
 #include "step_common.cuh"
 
 namespace cmace {
@@ -67,8 +67,10 @@ __global__ void __launch_bounds__(SPLIT == 1 ? SM_WARPS * 32 : SPLIT * 32)
       sn[h] = row_of ? row_of[s] : s;
     }
   };
+  __shared__ __align__(16) PairHarmonics<T, SPLIT == 1 ? SM_WARPS : SPLIT> harmonics;
+  int turn = 0;
   if (e0 < e1) fetch(e0);
-  for (int64_t e = e0; e < e1; e += 2 * SPLIT) {
+  for (int64_t e = e0; e < e1; e += 2 * SPLIT, turn ^= 1) {
     T cf[2][4][4][VEC], xx[2][VEC], x[2];
 #pragma unroll
     for (int h = 0; h < 2; h++) {
@@ -76,8 +78,10 @@ __global__ void __launch_bounds__(SPLIT == 1 ? SM_WARPS * 32 : SPLIT * 32)
       load_coeffs<T, VEC, C>(cf[h], table, rn[h].interval >= 0 && e + h < e1, (int)rn[h].interval, c0);
       load_vec<T, VEC>(xx[h], X + (int64_t)sn[h] * C + c0);
     }
-    const T y = yn;
+    T *yp = harmonics.v[warp][turn];
+    yp[lane] = yn;
     if (e + 2 * SPLIT < e1) fetch(e + 2 * SPLIT);
+    __syncwarp();
 #pragma unroll
     for (int h = 0; h < 2; h++) {
       T R[4][VEC];   // a missing second edge has zero weights
@@ -86,12 +90,12 @@ __global__ void __launch_bounds__(SPLIT == 1 ? SM_WARPS * 32 : SPLIT * 32)
 #pragma unroll
         for (int v = 0; v < VEC; v++)
           R[l][v] = (cf[h][0][l][v] + x[h] * (cf[h][1][l][v] + x[h] * (cf[h][2][l][v] + x[h] * cf[h][3][l][v]))) * xx[h][v];
+      T y[16];
+      take16<T>(y, yp + 16 * h);
 #pragma unroll
-      for (int m = 0; m < 16; m++) {
-        const T ym = __shfl_sync(0xffffffffu, y, h * 16 + m);
+      for (int m = 0; m < 16; m++)
 #pragma unroll
-        for (int v = 0; v < VEC; v++) acc[m][v] = fma(ym, R[l_of_lm(m)][v], acc[m][v]);
-      }
+        for (int v = 0; v < VEC; v++) acc[m][v] = fma(y[m], R[l_of_lm(m)][v], acc[m][v]);
     }
   }
   T *o = out + (out_row ? (int64_t)out_row[node] : node) * 16 * C + c0;
@@ -120,7 +124,7 @@ __global__ void __launch_bounds__(SPLIT == 1 ? SM_WARPS * 32 : SPLIT * 32)
 // Every channel chunk writes its own share of gY [chunks, E, 16] and dr [chunks, E]; the pass that turns them into the
 // gradient of the edge's vector adds them up.
 template <typename T, int VEC, int C>
-__global__ void __launch_bounds__(SM_WARPS * 32, sizeof(T) == 4 ? 4 : 1)
+__global__ void __launch_bounds__(SM_WARPS * 32, sizeof(T) == 4 ? 4 : 3)
     spline_edges_back_kernel(const T *__restrict__ X, const int32_t *__restrict__ row_of, const T *__restrict__ Y,
                              const SplinePoint<T> *__restrict__ r, const SplineTable<T> table, const T *__restrict__ G,
                              const int32_t *__restrict__ g_row, const int32_t *__restrict__ sender,
@@ -154,8 +158,10 @@ __global__ void __launch_bounds__(SM_WARPS * 32, sizeof(T) == 4 ? 4 : 1)
       sn[h] = row_of ? row_of[s] : s;
     }
   };
+  __shared__ __align__(16) PairHarmonics<T, SM_WARPS> harmonics;
+  int turn = 0;
   fetch(e0);
-  for (int64_t e = e0; e < e1; e += 2 * slices) {
+  for (int64_t e = e0; e < e1; e += 2 * slices, turn ^= 1) {
     T cf[2][4][4][VEC], xx[2][VEC], x[2], d[2] = {T(0), T(0)};
 #pragma unroll
     for (int h = 0; h < 2; h++) {
@@ -163,15 +169,16 @@ __global__ void __launch_bounds__(SM_WARPS * 32, sizeof(T) == 4 ? 4 : 1)
       load_coeffs<T, VEC, C>(cf[h], table, rn[h].interval >= 0 && e + h < e1, (int)rn[h].interval, c0);
       load_vec<T, VEC>(xx[h], X + (int64_t)sn[h] * C + c0);
     }
-    const T yv = yn;
+    T *yp = harmonics.v[threadIdx.x >> 5][turn];
+    yp[lane] = yn;
     if (e + 2 * slices < e1) fetch(e + 2 * slices);
+    __syncwarp();
 #pragma unroll
     for (int h = 0; h < 2; h++) {
       if (h && e + 1 >= e1) break;   // warp-uniform
       const int64_t ee = e + h;
       T y[16], p[16], t[VEC];
-#pragma unroll
-      for (int m = 0; m < 16; m++) y[m] = __shfl_sync(0xffffffffu, yv, h * 16 + m);
+      take16<T>(y, yp + 16 * h);
 #pragma unroll
       for (int v = 0; v < VEC; v++) t[v] = T(0);
 #pragma unroll
