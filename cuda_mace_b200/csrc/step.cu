@@ -318,17 +318,27 @@ static int run_step(const cmace_step_model &m, cmace_step_io &io, const Workspac
   return fail(CMACE_ERR_ARG, "cmace_step: no step %d", step);
 }
 
-// Programmatic launches while the kernels are a few microseconds long: 163 -> 119 us a step at 5 000 edges, 277 -> 246 at
-// 52 000, 385 -> 356 at 83 000; at 156 000 a recorded step is slower with them (519 -> 532 us), and one with tabulated
-// radial weights, which live on L1, much slower (1030 -> 1145).
-constexpr int64_t kChainEdges = 98304;
+// Programmatic launches while launch latency shows between the kernels: 163 -> 119 us a step at 5 000 edges, 277 -> 246 at
+// 52 000; float32 also 503 -> 473 at 157 000, 728 -> 700 at 261 000 and 961 -> 949 at 366 000.  A recorded step has no such
+// gaps beyond 98 304 edges and float64 kernels are long by then: 473 -> 481 us at 157 000 recorded, 2 300 -> 2 333 in
+// float64 (the kernels keep their predecessor's split between shared memory and L1).  Tabulated radial weights live on L1:
+// half the edges (516 -> 489 us at 94 000, 709 -> 700 at 157 000, the same at 261 000).
+constexpr int64_t kChainEdges = 98304, kChainEdgesLive = 393216;
+
+static bool chain_for(const cmace_step_model &m, int64_t edges, cudaStream_t st) {
+  const int64_t e = is_spline(m) ? 2 * edges : edges;
+  if (e <= kChainEdges) return true;
+  if (m.is_f64 || e > kChainEdgesLive) return false;
+  cudaStreamCaptureStatus status;
+  return cudaStreamIsCapturing(st, &status) == cudaSuccess && status == cudaStreamCaptureStatusNone;
+}
 
 template <typename T>
 static int run_steps(const cmace_step_model &m, cmace_step_io &io, int first, int last, cudaStream_t st) {
   const Workspace<T> w(io.workspace, m, io.n_owned, io.n_local, io.nedges);
   if (io.workspace_bytes < w.bytes)
     return fail(CMACE_ERR_ARG, "cmace_step: workspace of %lld bytes, %lld needed", (long long)io.workspace_bytes, (long long)w.bytes);
-  const bool chain = io.nedges <= (is_spline(m) ? kChainEdges / 2 : kChainEdges);
+  const bool chain = chain_for(m, io.nedges, st);
   int rc = CMACE_OK;
   for (int s = first; s < last && rc == CMACE_OK; s++) {
     chain_launches() = chain && (s > first || first == 0);   // a later range may follow the caller's wait for another stream
