@@ -136,68 +136,68 @@ class ClockSampler:
 
 
 def algorithmic_bytes(name, s, N, Ns, E, C, Z):
-    """Bytes each kernel has to move when every tensor is read or written once (indices 4 B)."""
-    if name.startswith("cmace_gemm3x_f32["):  # tagged with its shape: A [rows,K] in, [rows,N] out, weights
-        dims = dict(x.split("=") for x in name[name.index("[") + 1:-1].split(","))
-        rows, k, n = int(dims.get("M", E)), int(dims["K"]), int(dims["N"])   # no M: a product over the edges
-        return 4 * (rows * k + rows * n + k * n)
-    if name == "cmace_imp_bwd_edge_f32[no gradR]":   # the edge pass of radial_message_passing: R in, no gradR out
-        return s * (4 * E * C + 2 * 16 * E + Ns * C + 16 * N * C) + 8 * E
-    base = name[:-4]
+    """Bytes each step of the native sequence has to move when every tensor is read or written once (indices 4 B); the
+    float32 step at 128 channels forms the second layer's radial weights on chip, the others write them."""
+    if not name.startswith("step["):
+        return {"cmace_receiver_csr": 4 * E + 4 * N, "cmace_nl_emit_f64": 35 * E + 48 * N}.get(name)
+    row = 64 * s                              # one edge's hidden row (float32: an fp16 pair)
+    m16, sums = 16 * N * C * s, 16 * N * 64 * Z * s
+    fused = s == 4 and C == 128
+    R = 4 * C * s
     return {
-        "cmace_imp_fwd": s * (4 * E * C + 16 * E + Ns * C + 16 * N * C) + 8 * E,
-        "cmace_imp_bwd_edge": s * (2 * 4 * E * C + 2 * 16 * E + Ns * C + 16 * N * C) + 8 * E,
-        "cmace_imp_bwd_node": s * (E * C + Ns * C) + 4 * E,
-        "cmace_linear": s * (16 * N * C * 2 + 4 * Z * C * C),
-        "cmace_linear_tc": s * (16 * N * C * 2 + 4 * Z * C * C),
-        "cmace_symcon_fwd": s * (16 * N * C + N * C),
-        "cmace_symcon_bwd": s * (16 * N * C * 2 + N * C),
-        # hidden radial layers: basis in, h3 out, three saved derivative arrays (written forward, read backward)
-        "cmace_radial_hidden_fwd": 4 * E * (8 + 64 + 3 * 64),
-        "cmace_radial_hidden_bwd": 4 * E * (64 + 3 * 64 + 8),
-        "cmace_imp_radial_fused_fwd": 4 * (E * 64 + 16 * E + Ns * C + 16 * N * C + 4 * E * C) + 8 * E,
-        # grad h3 from operands formed on the fly: X, G, Y, the edge lists and the weights in, [E,64] out
-        "cmace_gemm3x_gradr": 4 * (E * 64 + 16 * E + Ns * C + 16 * N * C + 64 * 4 * C) + 8 * E,
-        # tabulated radial weights (secondary configuration): r in, R [E,4C] out / gradR in, grad r out; table in L2
-        "cmace_spline_fwd": s * (E + 4 * E * C),
-        "cmace_spline_bwd": s * (2 * E + 4 * E * C),
-        "cmace_edge_vectors_fwd": 24 * Ns + 24 * E + 8 * E + s * 3 * E,
-        "cmace_edge_vectors_bwd": 2 * s * 3 * E + 4 * E + 24 * Ns,
-        "cmace_edge_basis_fwd": s * E * (3 + 16 + 8),
-        "cmace_edge_basis_bwd": s * E * (3 + 16 + 8 + 3),
-    }.get(base)
+        "edge_prep": 24 * Ns + E * (24 + 8 + 4 * s + 16 * s + 16 * s),
+        "radial": E * (16 * s + 4 * row),
+        "sums": E * (row + 16 * s + 4) + sums,
+        "fold": sums + m16,
+        "contract0": m16 + N * C * s,
+        "mid_fwd": 2 * N * C * s,
+        "radial_out": 0 if fused else E * (row + R),
+        "messages": E * ((row if fused else R) + 16 * s + 8) + Ns * C * s + m16,
+        "linear": 2 * m16,
+        "contract1": 2 * m16,
+        "linear_back": 2 * m16,
+        "edges_back": E * ((2 * row if fused else 2 * R) + 32 * s + C * s + 8) + Ns * C * s + m16,
+        "radial_back": 0 if fused else E * (R + row),
+        "radial_dot": 0 if fused else E * (2 * row + s),
+        "senders": E * (C * s + 4) + Ns * C * s,
+        "mid_back": 2 * N * C * s,
+        "contract0_back": 2 * m16,
+        "fold_back": m16 + sums,
+        "sums_back": E * (2 * row + 32 * s + 4 * s + 4 * s + 4) + sums,
+        "forces": E * (2 * 4 * s + 4) + 24 * Ns,
+    }[name[5:-1]] or None
 
 
 # DRAM traffic per edge (dram__bytes_read.sum + dram__bytes_write.sum of one launch / edges) from the ncu capture of
-# the 8 000-atom case summarised in profiles/step_kernels_small_case_f32.txt (E = 417 248 there); the traffic of every
-# edge kernel grows in proportion to E, so a full launch moves this many bytes times its own E.
-_SRC = "profiles/step_kernels_small_case_f32.txt"
+# the 8 000-atom case (E = 417 248 there); the traffic of every edge kernel grows in proportion to E, so a full launch
+# moves this many bytes times its own E.
+_SRC = "profiles/step_sequence_8000_f32.txt"
 NCU_TRAFFIC_PER_EDGE = {
-    "cmace_imp_bwd_edge_f32[no gradR]": (2622.0, _SRC),   # mean of a step's two launches (with / without the T array)
-    "cmace_imp_fwd_f32": (2173.0, _SRC),
-    "cmace_gemm3x_gradr_f32": (402.0, _SRC),
-    "cmace_gemm3x_f32[K=64,N=512]": (2163.0, _SRC),
-    "cmace_radial_hidden_fwd_f32": (920.0, _SRC),
-    "cmace_radial_hidden_bwd_f32": (1060.0, _SRC),
+    "step[edges_back]": (1229.0, _SRC),
+    "step[messages]": (424.0, _SRC),
+    "step[radial]": (933.0, _SRC),
+    "step[sums_back]": (985.0, _SRC),
 }
 
 
-def tensor_flops(name, E, C):
-    """Tensor-core flops one launch executes, for the kernels whose binding roof is the tensor pipe: the product of
-    the radial-weight gradient with the last radial layer runs three TF32 terms of 2 * E * 4C * 64 flops each."""
-    if name == "cmace_gemm3x_gradr_f32":
-        return 3 * 2 * E * 4 * C * 64
-    return None
+def tensor_flops(name, s, E, C):
+    """Tensor-core flops one launch executes, for the steps whose binding roof is the tensor pipe: float32 runs three
+    fp16 terms of the product with the last radial layer ([E,64] x [64,4C]; the backward forms it for the derivative as
+    well) and of the hidden layers for values and derivatives of both perceptrons."""
+    if s != 4 or C != 128:
+        return None
+    return {"step[messages]": 3 * 2 * E * 4 * C * 64, "step[edges_back]": 2 * 3 * 2 * E * 4 * C * 64,
+            "step[radial]": 2 * 2 * 3 * 2 * E * (16 * 64 + 2 * 64 * 64)}.get(name)
 
 
-def tf32_peak():
-    """Dense TF32 peak = half the measured dense bf16 rate (MEASURED_PEAKS.json bf16_tflops, the burst figure of a kernel
-    timed alone); TF32 runs at half the bf16 rate on this tensor core."""
+def half_peak():
+    """Dense fp16 peak = the measured dense bf16 rate (MEASURED_PEAKS.json bf16_tflops, the burst figure of a kernel timed
+    alone)."""
     path = os.path.join(ROOT, "MEASURED_PEAKS.json")
     if os.path.isfile(path):
         with open(path) as f:
-            return float(json.load(f)["bf16_tflops"]) / 2.0, "half of the measured bf16 burst rate (MEASURED_PEAKS.json bf16_tflops)"
-    return 1590.0 / 2.0, "fallback (half of 1.59 PFLOP/s bf16)"
+            return float(json.load(f)["bf16_tflops"]), "measured bf16 burst rate (MEASURED_PEAKS.json bf16_tflops)"
+    return 1590.0, "fallback (1.59 PFLOP/s bf16)"
 
 
 def cpu_reference_run(args, steps, warmup):
@@ -529,9 +529,6 @@ def main():
     peak, peak_src = peaks()
     per_kernel = {}
     top, top_ms = None, -1.0
-    # products over the edges keep the short name [K=..,N=..]; the node products carry their row count
-    kernel_ms = {(name.replace(f"M={E},", "") if name.startswith("cmace_gemm3x_f32[") else name): v
-                 for name, v in kernel_ms.items()}
     for name, (calls, tot) in sorted(kernel_ms.items()):
         b = algorithmic_bytes(name, s_bytes, N, Ns, E, 128, sysd["n_species"])
         avg = tot / calls
@@ -545,18 +542,18 @@ def main():
         per_edge = NCU_TRAFFIC_PER_EDGE.get(top)
         traffic = per_edge[0] * E if per_edge else None
         traffic_src = f"ncu capture of a smaller case scaled by edges, {per_edge[1]}" if per_edge else None
-        flops = tensor_flops(top, E, 128)
+        flops = tensor_flops(top, s_bytes, E, 128)
         if flops:
             # not HBM-bound (its operands are formed on chip): the tensor pipe is the roof that binds it
-            tpeak, tsrc = tf32_peak()
+            tpeak, tsrc = half_peak()
             ach = flops / (per_kernel[top]["avg_ms"] * 1e-3) / 1e12
             roofline = {"kernel": top, "bound": "tensor", "achieved": ach, "peak": tpeak, "unit": "TFLOP/s",
                         "frac": ach / tpeak, "traffic": traffic, "traffic_source": traffic_src, "peak_source": tsrc,
                         "algorithmic_flops_per_launch": flops, "avg_launch_ms": per_kernel[top]["avg_ms"],
                         "hbm_gbs_of_algorithmic_bytes": per_kernel[top]["achieved_gbs"],
-                        "note": "of the two roofs this schema knows the tensor pipe is the nearer one; the unit that "
-                                "binds the kernel is the SM's load/store data pipe (about 80 % busy in the ncu "
-                                "capture named in traffic_source): the operand is formed from shared-memory reads"}
+                        "note": "of the two roofs this schema knows the tensor pipe is the nearer one; what binds the "
+                                "kernel is the arithmetic between its products, on 4 warps a scheduler (issue slots "
+                                "46 % used in the ncu capture named in traffic_source)"}
         else:
             ach = per_kernel[top]["achieved_gbs"]
             roofline = {"kernel": top, "bound": "hbm", "achieved": ach, "peak": peak, "unit": "GB/s",
@@ -564,7 +561,7 @@ def main():
                         "algorithmic_bytes_per_launch": algorithmic_bytes(top, s_bytes, N, Ns, E, 128, sysd["n_species"]),
                         "avg_launch_ms": per_kernel[top]["avg_ms"]}
         # the largest HBM-bound kernel beside it, for the fraction of the copy peak the streaming kernels reach
-        hbm = [(v["share_of_step"], k) for k, v in per_kernel.items() if v["achieved_gbs"] and not tensor_flops(k, E, 128)]
+        hbm = [(v["share_of_step"], k) for k, v in per_kernel.items() if v["achieved_gbs"] and not tensor_flops(k, s_bytes, E, 128)]
         if hbm:
             k = max(hbm)[1]
             roofline["largest_hbm_bound_kernel"] = {"kernel": k, "achieved": per_kernel[k]["achieved_gbs"], "peak": peak,
