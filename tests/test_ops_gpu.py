@@ -582,6 +582,35 @@ def test_device_neighbor_list_where_its_kernels_change(n, side, dev):
     assert torch.equal(_edge_keys(ei_d, si_d), _edge_keys(torch.from_numpy(ei_h), torch.from_numpy(si_h)))
 
 
+def test_device_neighbor_list_in_single_steps(dev):
+    """The C entry points one by one give the list that the two calls give, edge for edge."""
+    from cuda_mace_b200 import _abi, ops
+
+    n, side, rc = 700, 21.0, 5.0
+    pos = torch.rand(n, 3, generator=torch.Generator().manual_seed(2), dtype=torch.float64).to(dev) * side
+    ei, sh, si = ops.neighbor_list(pos, (side,) * 3, (True, True, False), rc)
+    box, mask, st = [0.0] * 3 + [side] * 3, 3, ops._stream()
+    i32 = dict(dtype=torch.int32, device=dev)
+    ncells = _abi.call("cmace_nl_num_cells", side, side, side, rc)
+    ids, perm, cells, count = (torch.zeros(k, **i32) for k in (n, n, ncells + 1, n + 1))
+    _abi.call("cmace_nl_cell_ids_f64", pos.data_ptr(), n, *box, mask, rc, ids.data_ptr(), st)
+    nbytes = _abi.call("cmace_sender_order_workspace_bytes", n)
+    ws = torch.empty(nbytes, dtype=torch.uint8, device=dev)
+    _abi.call("cmace_sender_order", ids.data_ptr(), n, ncells, perm.data_ptr(), cells.data_ptr(), ws.data_ptr(), nbytes, st)
+    _abi.call("cmace_nl_count_f64", pos.data_ptr(), n, n, *box, mask, rc, perm.data_ptr(), cells.data_ptr(),
+              count.data_ptr(), st)
+    rows = torch.empty(n + 1, **i32)
+    nbytes = _abi.call("cmace_scan_workspace_bytes", n + 1)
+    ws = torch.empty(nbytes, dtype=torch.uint8, device=dev)
+    _abi.call("cmace_exclusive_scan_i32", count.data_ptr(), n + 1, rows.data_ptr(), ws.data_ptr(), nbytes, st)
+    E = int(rows[-1])
+    out = torch.empty(2, E, **i32)
+    index, shifts = torch.empty(E, 3, dtype=torch.int8, device=dev), torch.empty(E, 3, dtype=torch.float64, device=dev)
+    _abi.call("cmace_nl_fill_f64", pos.data_ptr(), n, n, *box, mask, rc, perm.data_ptr(), cells.data_ptr(),
+              rows.data_ptr(), out[1].data_ptr(), out[0].data_ptr(), index.data_ptr(), shifts.data_ptr(), st)
+    assert torch.equal(out, ei) and torch.equal(index, si) and torch.equal(shifts, sh)
+
+
 def test_device_neighbor_list_without_atoms_or_edges(dev):
     from cuda_mace_b200 import ops
 
