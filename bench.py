@@ -157,8 +157,7 @@ def algorithmic_bytes(name, s, N, Ns, E, C, Z):
         "contract1": 2 * m16,
         "linear_back": 2 * m16,
         "edges_back": E * ((2 * row if fused else 2 * R) + 32 * s + C * s + 8) + Ns * C * s + m16,
-        "radial_back": 0 if fused else E * (R + row),
-        "radial_dot": 0 if fused else E * (2 * row + s),
+        "radial_back": 0 if fused else E * (R + row + s),
         "senders": E * (C * s + 4) + Ns * C * s,
         "mid_back": 2 * N * C * s,
         "contract0_back": 2 * m16,

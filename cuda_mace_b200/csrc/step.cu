@@ -8,9 +8,9 @@
 //   mid_fwd       up = b0 Wu, q0 = b0 Wsc[z] [n, 17]                                      (step_nodes.cu)
 //       -- a decomposed system fills the ghost rows of `up` here --
 //   radial_out    second layer: R = h W4 [E, 4C]  (not in float32 with 128 channels: `messages` and `edges_back` form R and
-//                 R' = h' W4 themselves, fused_messages.cu, and `radial_back`, `radial_dot` are part of `edges_back`)
+//                 R' = h' W4 themselves, fused_messages.cu, and `radial_back` is part of `edges_back`)
 //   messages, linear, contract1 (value, readout, energy and gradient in one kernel), linear_back
-//   edges_back    T [E, C] and grad Y of the second layer; radial_back, radial_dot: dE/dr of the second layer
+//   edges_back    T [E, C] and grad Y of the second layer; radial_back: dE/dr of the second layer
 //   senders       grad up = sum of T over a sender's edges
 //       -- and returns the gradients of the ghost rows here --
 //   mid_back, contract0_back, fold_back
@@ -47,36 +47,19 @@ int fused_messages_back(const float *X, const float *Y, const float *G, const vo
 template <typename T>
 int step_edge_finish(const T *gY0, const T *dr0, const T *gY1, const T *dr1, const Quad<T> *geo, int64_t nedges, int shares, T *gvec,
                      cudaStream_t st);
+int gemm_dot_f64(const double *A, const double *B, const double *dot, int64_t M, int K, int N, double *out, cudaStream_t st);
 int radial_pair_f64(const double *basis, int nb, const double *const (*w)[3], int nper, int64_t nedges,
                     double *const *h, double *const *dh, cudaStream_t st);
 
 enum StepId {
   S_EDGE_PREP, S_RADIAL, S_SUMS, S_FOLD, S_CONTRACT0, S_MID_FWD,
-  S_RADIAL_OUT, S_MESSAGES, S_LINEAR, S_CONTRACT1, S_LINEAR_BACK, S_EDGES_BACK, S_RADIAL_BACK, S_RADIAL_DOT, S_SENDERS,
+  S_RADIAL_OUT, S_MESSAGES, S_LINEAR, S_CONTRACT1, S_LINEAR_BACK, S_EDGES_BACK, S_RADIAL_BACK, S_SENDERS,
   S_MID_BACK, S_CONTRACT0_BACK, S_FOLD_BACK, S_SUMS_BACK, S_FORCES, S_COUNT
 };
 static const char *const kStepNames[S_COUNT] = {
     "edge_prep", "radial", "sums", "fold", "contract0", "mid_fwd",
-    "radial_out", "messages", "linear", "contract1", "linear_back", "edges_back", "radial_back", "radial_dot", "senders",
+    "radial_out", "messages", "linear", "contract1", "linear_back", "edges_back", "radial_back", "senders",
     "mid_back", "contract0_back", "fold_back", "sums_back", "forces"};
-
-// dE/dr [E] = sum_k grad h[e, k] h'[e, k]: half a warp per edge
-template <typename T>
-__global__ void __launch_bounds__(256)
-    radial_dot_kernel(const T *__restrict__ gh, const T *__restrict__ dh, int64_t nedges, T *__restrict__ dr) {
-  grid_begin();
-  const int64_t e = ((int64_t)blockIdx.x * 256 + threadIdx.x) >> 4;
-  const int l16 = threadIdx.x & 15;
-  T s = T(0);
-  if (e < nedges) {
-    const Quad<T> a = reinterpret_cast<const Quad<T> *>(gh + e * ST_H)[l16];
-    const Quad<T> b = reinterpret_cast<const Quad<T> *>(dh + e * ST_H)[l16];
-    s = fma(a.x, b.x, fma(a.y, b.y, fma(a.z, b.z, a.w * b.w)));
-  }
-#pragma unroll
-  for (int off = 8; off > 0; off >>= 1) s += __shfl_xor_sync(0xffffffffu, s, off);
-  if (l16 == 0 && e < nedges) dr[e] = s;
-}
 
 // second layer with the radial weights formed inside its kernels: fp16 pairs of h, 128 channels (fused_messages.cu)
 static bool is_spline(const cmace_step_model &m) { return m.spline[0] != nullptr; }
@@ -86,7 +69,7 @@ template <typename T>
 struct Workspace {
   int32_t *species, *counts, *slot_of, *node_of, *slot_type, *elem_start;
   Quad<T> *geo;
-  T *basis, *Y, *h[2], *dh[2], *A, *m0, *b0, *up, *R, *m1, *l1, *gX1, *gm1, *T_, *gY1, *gH1, *dr1, *gup, *gb0, *gX0, *gA,
+  T *basis, *Y, *h[2], *dh[2], *A, *m0, *b0, *up, *R, *m1, *l1, *gX1, *gm1, *T_, *gY1, *dr1, *gup, *gb0, *gX0, *gA,
       *gvec, *gradR, *partial, *q0, *dq, *gY0, *dr0;
   int64_t bytes;
 
@@ -128,7 +111,6 @@ struct Workspace {
     take(dq, n * ST_RO);
     take(T_, E * C);
     take(gY1, shares * E * 16);
-    take(gH1, sizeof(T) == 8 && !sp ? E * ST_H : 0);
     take(dr1, shares * E);
     take(gup, nl * C);
     take(gb0, n * C);
@@ -177,8 +159,7 @@ static int run_spline_step(const cmace_step_model &m, cmace_step_io &io, const W
     case S_FOLD: return linear_any(w.A, m.fold, start, Z, n, C, C, w.m0, io.status, st);
     case S_RADIAL:
     case S_RADIAL_OUT:
-    case S_RADIAL_BACK:
-    case S_RADIAL_DOT: io.launches--; return CMACE_OK;
+    case S_RADIAL_BACK: io.launches--; return CMACE_OK;
     case S_MESSAGES:
       return spline_messages<T>(up, nullptr, w.Y, at, table(1), io.sender, io.row_ptr, n, nullptr, C, w.m1, st);
     case S_EDGES_BACK:
@@ -211,7 +192,7 @@ static int run_step(const cmace_step_model &m, cmace_step_io &io, const Workspac
   const bool half = !f64 && m.radial_half[0][0] != nullptr;
   const RadialScales *scales = reinterpret_cast<const RadialScales *>(m.half_scales);
   const bool fused = is_fused(m);
-  if (fused && (step == S_RADIAL_OUT || step == S_RADIAL_BACK || step == S_RADIAL_DOT)) return CMACE_OK;
+  if (fused && (step == S_RADIAL_OUT || step == S_RADIAL_BACK)) return CMACE_OK;
   io.launches++;
   if (step == S_EDGE_PREP && node_blocks(io.n_local) > 1) io.launches++;
   if (is_spline(m)) {
@@ -268,17 +249,10 @@ static int run_step(const cmace_step_model &m, cmace_step_io &io, const Workspac
                              w.T_, w.partial, st);
     case S_RADIAL_BACK:
       if constexpr (f64)
-        return cmace_gemm_f64(w.gradR, static_cast<const double *>(m.radial_back), E, 4 * C, ST_H, 1.0, w.gH1, st);
+        return gemm_dot_f64(w.gradR, static_cast<const double *>(m.radial_back), w.dh[1], E, 4 * C, ST_H, w.dr1, st);
       else
         return gemm3x_gradr(up, w.gm1, w.Y, ys, io.sender, io.receiver, static_cast<const float *>(m.radial_back), E, C,
                             ST_H, w.dh[1], w.dr1, io.status, st);
-    case S_RADIAL_DOT:
-      if constexpr (!f64) {   // the float32 product above has formed it
-        io.launches--;
-        return CMACE_OK;
-      }
-      if (E > 0) launch_chained(radial_dot_kernel<T>, (unsigned)((E + 15) / 16), 256, 0, st, w.gH1, w.dh[1], E, w.dr1);
-      return check_launch("cmace_step(radial_dot)");
     case S_SENDERS:
       if constexpr (f64) return cmace_imp_bwd_node_f64(w.T_, io.perm, io.send_ptr, nl, C, gup, st);
       else return cmace_imp_bwd_node_f32(w.T_, io.perm, io.send_ptr, nl, C, gup, st);

@@ -262,7 +262,7 @@ def takes(positions, shifts):
             and shifts.dtype == torch.float64)
 
 
-_FIRST_EXCHANGE, _SENDERS, _SECOND_EXCHANGE, _END = 6, 14, 15, 20
+_FIRST_EXCHANGE, _SENDERS, _SECOND_EXCHANGE, _END = 6, 13, 14, 19
 _BESIDE_EDGES = 32768
 _side_streams = {}
 

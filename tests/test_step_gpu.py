@@ -50,11 +50,12 @@ def test_step_against_the_oracle(U, dtype, tol_e, tol_f, n, C, Z, stretch):
 
 # against the model's own autograd path (same bounds), what the oracle does not have: 16 basis functions, tabulated radial
 # weights (one element and several, the C = 128 and the narrower edge passes), and a list that crosses from eight warps a
-# receiver to one (1 184 receivers and channel chunks); grouping by element in one block (up to 2 048 nodes) and in several
+# receiver to one (1 184 receivers and channel chunks); grouping by element in one block (up to 2 048 nodes) and in several;
+# float64 products with a row-wise epilogue in tiles of 32 (70 atoms), 64 (400) and 128 rows
 @pytest.mark.parametrize("dtype,tol", [(torch.float64, 1e-10), (torch.float32, 1e-4)])
 @pytest.mark.parametrize("n,C,Z,nb,radial", [(70, 64, 3, 16, "exact"), (50, 128, 3, 8, "spline"), (33, 96, 1, 8, "spline"),
                                              (1300, 32, 2, 8, "spline"), (2048, 32, 3, 8, "exact"),
-                                             (4100, 64, 5, 8, "exact")])
+                                             (4100, 64, 5, 8, "exact"), (400, 32, 2, 8, "exact")])
 def test_step_against_autograd(U, dtype, tol, n, C, Z, nb, radial):
     pos, ei, sh = _cluster(n, 3, 1.0)
     species = torch.from_numpy(np.random.default_rng(4).integers(0, Z, n)).to(torch.int32).cuda()
