@@ -241,10 +241,10 @@ class InvariantMACE(torch.nn.Module):
             topology = ops.topology_for(edge_index[1], edge_index[0], n, n)
         species = one_hot = None
         if "species" in data:
-            species = data["species"].to(torch.int32).contiguous()
+            species = data["species"].to(torch.int32)
         else:
-            one_hot = data["node_attrs"].contiguous()
-            if one_hot.dtype not in (torch.float32, torch.float64) or one_hot.shape[1] != self.num_elements:
+            one_hot = data["node_attrs"]
+            if one_hot.dtype not in (torch.float32, torch.float64) or one_hot.shape[-1] != self.num_elements:
                 species, one_hot = one_hot.argmax(dim=-1).to(torch.int32), None
         sums, _, node_energy, forces = step.energy_forces(plan, positions, species, one_hot, data["shifts"], topology)
         return {"energy": sums[0], "node_energy": node_energy, "interaction_energy": sums[1], "forces": forces}

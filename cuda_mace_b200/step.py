@@ -87,32 +87,49 @@ def fused_rows(device):
     return (degree * 128 + 64 * (q & 1) + 2 * i + (j & 1)).reshape(-1).to(device)
 
 
+def _expected_buffers(model):
+    """(tensor, shape, dtype) of every buffer that a plan of `model` reads."""
+    C, Z, T, D = model.channels, model.num_elements, model.dtype, torch.float64
+    L0, L1 = model.layers
+    out = [(model.atomic_energies, (Z,), D), (model.embedding, (Z, C), T), (L0.linear.weights, (Z, 4, C, C), T),
+           (L0.W_readout, (C, 1), D), (L1.linear.weights, (4, C, C), T), (L1.W_sc, (C, Z * C), T),
+           (L1.W_readout1, (C, 16), D), (L1.W_readout2, (16, 1), D)]
+    for L in model.layers:
+        con = L.contraction
+        out += [(L.W_up, (C, C), T), (L.W_prod, (C, C), T), (con.weights_3, (1, Z, con.W3_L0_size, C), T),
+                (con.weights_2, (1, Z, con.W2_L0_size, C), T), (con.weights_1, (1, Z, con.W1_L0_size, C), T)]
+        if model.radial == "spline":
+            intervals = model.layers[0].spline.coefficients.shape[0]
+            out += [(L.spline.coefficients, (intervals, 4, 4 * C), T), (L.spline.r_knots, (intervals + 1,), T)]
+        else:
+            nb = model.edge_basis.num_bessel
+            widths = (nb, _H, _H, _H, 4 * C)
+            out += [(getattr(L, f"W_radial{i}"), widths[i:i + 2], T) for i in range(4)]
+    return out
+
+
 def covers(model):
-    """Whether the sequence covers a model: the standard two-layer architecture in float32 or float64."""
+    """Whether the sequence covers a model: the standard two-layer architecture in float32 or float64, every buffer with
+    the shape and type it was built with, on one device (kernels get plain pointers: a model that was converted or
+    replaced in part afterwards is left to the operators and their checks)."""
     if model.radial not in ("exact", "spline") or len(model.layers) != 2 or model.num_elements > 16:
         return False
     if model.dtype not in (torch.float32, torch.float64) or model.channels not in (32, 64, 96, 128):
         return False
     if os.environ.get("CMACE_SYMCON_GENERIC", "")[:1] == "1":
         return False
-    C, nb = model.channels, model.edge_basis.num_bessel
-    if model.radial == "exact" and nb not in (8, 16):
+    if model.radial == "exact" and model.edge_basis.num_bessel not in (8, 16):
         return False
     for L in model.layers:
         if model.radial == "spline":
-            first, co = model.layers[0].spline, L.spline.coefficients
-            if co.shape != first.coefficients.shape or co.shape[1:] != (4, 4 * C) or co.dtype != model.dtype:
-                return False
+            first = model.layers[0].spline
             if L.spline.h != first.h or L.spline.rmax != first.rmax:
                 return False
-            continue
-        if L.n_radial != 4:
+        elif L.n_radial != 4:
             return False
-        shapes = [tuple(getattr(L, f"W_radial{i}").shape) for i in range(4)]
-        if shapes != [(nb, _H), (_H, _H), (_H, _H), (_H, 4 * C)]:
-            return False
-    L = model.layers[1]
-    return tuple(L.W_readout1.shape) == (C, 16) and tuple(L.W_readout2.shape) == (16, 1)
+    dev = model.embedding.device
+    return all(t.device == dev and t.dtype == dtype and tuple(t.shape) == shape
+               for t, shape, dtype in _expected_buffers(model))
 
 
 class StepPlan:
@@ -126,6 +143,7 @@ class StepPlan:
         C, Z = model.channels, model.num_elements
         L0, L1 = model.layers
         d = lambda t: t.double()
+        self.device = model.embedding.device
         m = _abi.StepModel()
         m.is_f64, m.channels, m.elements = int(not f32), C, Z
         m.nbessel, m.cutoff_p = model.edge_basis.num_bessel, model.edge_basis.p
@@ -160,8 +178,9 @@ class StepPlan:
                                           con.U2_num_nonsparse, con.U2_indices, con.U2_values, con.W3_L0_size,
                                           con.W2_L0_size, con.W1_L0_size)
             weff = torch.empty(Z, 13, C, dtype=model.dtype, device=x.device)
-            _abi.call("cmace_symcon_effective_weights", con._plan.handle, int(not f32), con.weights_3.data_ptr(),
-                      con.weights_2.data_ptr(), con.weights_1.data_ptr(), Z, C, weff.data_ptr(), ops._stream())
+            weights = [w.contiguous() for w in (con.weights_3, con.weights_2, con.weights_1)]
+            _abi.call("cmace_symcon_effective_weights", con._plan.handle, int(not f32), *[w.data_ptr() for w in weights],
+                      Z, C, weff.data_ptr(), ops._stream())
             m.weff[t] = hold(weff)
         prod0, prod1, ro1 = d(L0.W_prod), d(L1.W_prod), d(L1.W_readout1)
         up = prod0 @ d(L1.W_up)
@@ -241,6 +260,9 @@ def plan_of(model):
         return None
     if plan is not None and plan.current():
         return plan
+    dev = model.embedding.device
+    if dev.type != "cuda" or dev.index != torch.cuda.current_device():
+        return None   # the operators refuse such a call
     plan = None
     if covers(model):
         try:
@@ -278,15 +300,29 @@ def energy_forces(plan, positions, species, one_hot, shifts, topology, halo=None
     """(sums [3], interaction [n_owned], node_energy [n_owned], forces): sums = (total energy, interaction energy,
     0 unless a kernel recorded a failure: check_status() tells which).
 
-    shifts: [E, 3] float64, or (index [E] uint8, table [rows, 3] float64).  positions [n_local, 3] float64, species [n_local] int32 or one_hot [n_local, Z].  `halo` (a HaloPlan of more than
-    one rank) fills and returns the ghost rows between the ranges of steps; forces are then those of the owned atoms."""
+    shifts: [E, 3] float64, or (index [E] uint8, table [rows, 3] float64).  positions [n_local, 3] float64, species
+    [n_local] int32 or one_hot [n_local, Z] float32 or float64.  `halo` (a HaloPlan of more than one rank) fills and
+    returns the ghost rows between the ranges of steps; forces are then those of the owned atoms.
+
+    The kernels get plain pointers, so devices, sizes and types are checked here, before the first launch."""
     index = None
     if isinstance(shifts, tuple):
         index, shifts = shifts[0].contiguous(), shifts[1]
-    ops._check_cuda(positions, shifts)
+    ops._check_cuda(positions, shifts, index, species, one_hot, topology.sender)
     positions, shifts = positions.contiguous(), shifts.contiguous()
     n, nl, E = topology.nnodes, topology.nsenders, topology.nedges
     dev = positions.device
+    if plan.device != dev:
+        raise RuntimeError(f"the model is on {plan.device}, the positions are on {dev}")
+    if species is not None:
+        species = species.contiguous()
+        if species.dtype != torch.int32 or species.shape != (nl,):
+            raise RuntimeError(f"species must be int32 [{nl}], got {species.dtype} {tuple(species.shape)}")
+    else:
+        one_hot = one_hot.contiguous()
+        if one_hot.dtype not in (torch.float32, torch.float64) or one_hot.shape != (nl, plan.elements):
+            raise RuntimeError(f"node attributes must be float32 or float64 [{nl}, {plan.elements}], got "
+                               f"{one_hot.dtype} {tuple(one_hot.shape)}")
     if positions.shape != (nl, 3) or shifts.shape[1:] != (3,) or (shifts if index is None else index).shape[0] != E:
         raise RuntimeError(f"shape mismatch: positions {tuple(positions.shape)}, shifts {tuple(shifts.shape)} for "
                            f"{nl} atoms and {E} edges")

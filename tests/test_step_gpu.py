@@ -96,3 +96,40 @@ def test_new_list_and_host_batch(U, n):
     with pytest.raises(RuntimeError):
         ev.evaluate_host(batch)
     assert torch.equal(ev.rebuild_neighbor_list(p)(p)[1], f_new)   # the device goes on
+
+
+def _small(U, dtype=torch.float64, n=12, C=32, Z=3, **more):
+    pos, ei, sh = _cluster(n, 3, 1.0)
+    mace = model.InvariantMACE(systems.init_params(C, Z, 7, **more), U, dtype=dtype, device="cuda")
+    species = torch.arange(n, dtype=torch.int32) % Z
+    data = dict(positions=torch.from_numpy(pos).cuda(), species=species.cuda(),
+                edge_index=torch.from_numpy(ei).to(torch.int32).cuda(), shifts=torch.from_numpy(sh).cuda())
+    return mace, data
+
+
+# nothing of these calls is launched: the checks come first
+@pytest.mark.parametrize("species,node_attrs", [
+    (torch.zeros(12, dtype=torch.int32), None), (torch.zeros(11, dtype=torch.int32, device="meta"), None),
+    (torch.zeros(12, 1, dtype=torch.int32, device="meta"), None), (None, torch.eye(3)[torch.zeros(12, dtype=torch.long)]),
+    (None, torch.zeros(11, 3, device="meta")), (None, torch.zeros(13, 3, device="meta"))])
+def test_elements_that_do_not_fit_the_atoms_are_refused(U, species, node_attrs):
+    mace, data = _small(U)
+    del data["species"]
+    for name, t in (("species", species), ("node_attrs", node_attrs)):
+        if t is not None:   # "meta" stands for the GPU: the parameters are made where there may be none
+            data[name] = torch.zeros(t.shape, dtype=t.dtype, device="cuda") if t.is_meta else t
+    with pytest.raises(RuntimeError):
+        mace(data)
+
+
+def test_a_model_on_another_device_or_of_another_type_is_refused(U):
+    mace, data = _small(U)
+    mace(data)
+    mace.float()
+    with pytest.raises((RuntimeError, TypeError)):
+        mace(data)
+    mace, data = _small(U)
+    mace(data)
+    mace.cpu()
+    with pytest.raises(RuntimeError):
+        mace(data)
