@@ -1,6 +1,7 @@
 // Shared helpers of the C-ABI library: status codes, error text, launch checks.
 #pragma once
 #include <cuda_runtime.h>
+#include <math_constants.h>
 #include <stdint.h>
 
 #include <cstdarg>

@@ -58,7 +58,9 @@ int spline_edges_back(const T *X, const int32_t *row_of, const T *Y, const Splin
                       const int32_t *g_row, const int32_t *sender, const int32_t *row_ptr, int64_t n, int64_t E, int C,
                       T *Tout, T *gY, T *dr, cudaStream_t st);
 
-constexpr int32_t CMACE_STEP_BAD_SHIFT = 90;   // status: a row of the shift table that does not exist
+// status words of inputs that only a kernel sees; what such an input enters comes out as NaN
+constexpr int32_t CMACE_STEP_BAD_SHIFT = 90;     // a row of the shift table that does not exist
+constexpr int32_t CMACE_STEP_BAD_ELEMENT = 91;   // an element index outside 0 .. elements - 1
 
 int *staged_stall_flag();   // message_passing.cu: device word of the staged edge pass, or null
 
@@ -81,8 +83,9 @@ struct StepKernels {
   static int contract_bwd(const T *X, const int32_t *types, const T *weff, const T *gb, int64_t n, int C, T *gX,
                           cudaStream_t st);
   static int contract_readout(const T *X, const int32_t *types, const T *weff, const T *wp1, const double *w2,
-                              const T *q0, const double *atomic_e, double scale, double shift, int64_t n, int C, T *gX,
-                              T *dq, double *inter, double *node_energy, cudaStream_t st);
+                              const T *q0, const double *atomic_e, const int32_t *species_in, int elements, double scale,
+                              double shift, int64_t n, int C, T *gX, T *dq, double *inter, double *node_energy,
+                              cudaStream_t st);
   static int mid_fwd(const T *b, const int32_t *node_of, const int32_t *slot_type, const T *wu, const T *extra,
                      int64_t n, int C, T *up, T *q0, cudaStream_t st);
   static int mid_bwd(const T *gup, const int32_t *node_of, const int32_t *slot_type, const T *dq, const T *wu_t,

@@ -38,7 +38,7 @@ __device__ int first_max(const OH *row, int n) {
 }
 
 __device__ void resolve_nodes(const int32_t *__restrict__ species_in, const void *__restrict__ one_hot, int one_hot_f64,
-                              int64_t lo, int64_t hi, int elements, int32_t *__restrict__ species) {
+                              int64_t lo, int64_t hi, int elements, int32_t *__restrict__ species, int32_t *status) {
   constexpr int PER = GN_NODES / EP_THREADS;
   int z[PER];
 #pragma unroll
@@ -53,7 +53,10 @@ __device__ void resolve_nodes(const int32_t *__restrict__ species_in, const void
 #pragma unroll
   for (int u = 0; u < PER; u++) {
     const int64_t i = lo + u * EP_THREADS + threadIdx.x;
-    if (i < hi) species[i] = z[u] < 0 ? 0 : (z[u] >= elements ? elements - 1 : z[u]);
+    if (i >= hi) continue;
+    const bool known = z[u] >= 0 && z[u] < elements;
+    species[i] = known ? z[u] : 0;   // the tables are read with it; the readout gives such a node no energy
+    if (!known && status) *status = CMACE_STEP_BAD_ELEMENT;
   }
   __syncthreads();
 }
@@ -184,7 +187,7 @@ __global__ void __launch_bounds__(EP_THREADS, sizeof(T) == 4 ? 5 : 3)
   const int nblocks = (int)node_blocks(n_local);
   if ((int)blockIdx.x < nblocks) {
     const int64_t first = (int64_t)blockIdx.x * GN_NODES, end = first + GN_NODES;
-    resolve_nodes(species_in, one_hot, one_hot_f64, first, end < n_local ? end : n_local, elements, species);
+    resolve_nodes(species_in, one_hot, one_hot_f64, first, end < n_local ? end : n_local, elements, species, status);
     group_nodes(first, end < n_owned ? end : n_owned, 1, (int)blockIdx.x, nblocks > 1, elements, species, counts, slot_of,
                 node_of, slot_type, elem_start);
     return;
@@ -199,9 +202,11 @@ __global__ void __launch_bounds__(EP_THREADS, sizeof(T) == 4 ? 5 : 3)
   const int64_t e = base + (lane < rows ? lane : rows - 1);
   const int64_t s = sender[e], r = receiver[e];
   const double *sh = shifts ? shifts + e * 3 : nullptr;
+  bool known = true;
   if (shift_index) {
     const int k = shift_index[e];
-    if (k < shift_rows) sh = shift_table + 3 * k;
+    known = k < shift_rows;
+    if (known) sh = shift_table + 3 * k;
     else *status = CMACE_STEP_BAD_SHIFT;
   }
   T v[3];
@@ -209,7 +214,7 @@ __global__ void __launch_bounds__(EP_THREADS, sizeof(T) == 4 ? 5 : 3)
   for (int c = 0; c < 3; c++) {
     double d = __dsub_rn(pos[s * 3 + c], pos[r * 3 + c]);
     if (sh) d = __dadd_rn(d, sh[c]);
-    v[c] = (T)d;
+    v[c] = known ? (T)d : (T)CUDART_NAN;
   }
   const T r2 = v[0] * v[0] + v[1] * v[1] + v[2] * v[2];
   const T ir = inv_sqrt(r2);

@@ -97,6 +97,11 @@ FUSED_RADIAL_MESSAGE_PASSING = False
 RADIAL_GRADIENT_ON_THE_FLY = True
 
 
+# codes of the status word that a wrong input of the energy+force step leaves (csrc/step_common.cuh)
+_STATUS_INPUTS = {90: "an edge's shift index is beyond the shift table",
+                  91: "an atom's element index is outside the model's elements"}
+
+
 def _status_tensor(device):
     idx = device.index if device.index is not None else torch.cuda.current_device()
     if idx not in _status:
@@ -105,14 +110,16 @@ def _status_tensor(device):
 
 
 def check_status():
-    """Raises if any tensor-core kernel reported a timed-out wait since the last check (synchronises)."""
+    """Raises if a kernel reported a timed-out wait, or an index that does not exist, since the last check
+    (synchronises)."""
     if _abi.call("cmace_imp_staged_stalled") != 0:
         raise RuntimeError("cuda_mace_b200: the message-passing backward gave up waiting for a bulk copy")
     for idx, t in _status.items():
         code = int(t.item())
         if code != 0:
             t.zero_()
-            raise RuntimeError(f"cuda_mace_b200: a tensor-core kernel on cuda:{idx} gave up waiting (code {code})")
+            what = _STATUS_INPUTS.get(code, f"a tensor-core kernel gave up waiting (code {code})")
+            raise RuntimeError(f"cuda_mace_b200: {what} (cuda:{idx})")
 
 
 def probe_bounded_wait(device, code=77, limit_seconds=0.05):

@@ -402,9 +402,10 @@ typedef struct cmace_step_io {
   const double *positions;          /* [n_local, 3] */
   const double *shifts;             /* [nedges, 3], or NULL: */
   const uint8_t *shift_index;       /* [nedges] rows of shift_table [.., 3], or NULL: no shifts */
-  const double *shift_table;        /* [shift_rows, 3]; an index beyond it is recorded in *status */
+  const double *shift_table;        /* [shift_rows, 3]; an index beyond it is recorded in *status and makes the edge NaN */
   int64_t shift_rows;
-  const int32_t *species;           /* [n_local], or NULL with one_hot [n_local, elements] */
+  const int32_t *species;           /* [n_local], or NULL with one_hot [n_local, elements]; an index outside the elements
+                                       is recorded in *status and gives that node's energy as NaN */
   const void *one_hot;
   int32_t one_hot_is_f64, launches; /* launches: kernels launched so far, added to by the call */
   const int32_t *sender, *receiver, *row_ptr, *perm, *send_ptr;
@@ -413,7 +414,7 @@ typedef struct cmace_step_io {
   void *gup_local, *gup_owned;      /* gradient of up_local, and what the owners end up with; NULL likewise */
   void *workspace;
   int64_t workspace_bytes;
-  int32_t *status;                  /* written by bounded waits that give up */
+  int32_t *status;                  /* written by bounded waits that give up and by the checks of indices above */
   double *node_energy, *interaction; /* [n_owned] */
   double *sums;                     /* [3]: sum of node_energy, sum of interaction, and what the status words held */
   double *gradient;                 /* [n_local, 3]: gradient_sign times the position gradient */

@@ -3,7 +3,7 @@ import numpy as np
 import pytest
 import torch
 
-from cuda_mace_b200 import domain, evaluator, model, step, systems
+from cuda_mace_b200 import domain, evaluator, model, ops, step, systems
 from oracle import model as omodel
 
 pytestmark = pytest.mark.gpu
@@ -93,8 +93,11 @@ def test_new_list_and_host_batch(U, n):
     e_new, f_new = ev(p)                # another order of the edges: float64 rounding over about 50 edges a node
     assert abs(float(e_new - e)) < 1e-12 * n and float((f_new - f).abs().max()) < 1e-11 * float(f.abs().max())
     batch["shift_table"] = batch["shift_table"][:1]
-    with pytest.raises(RuntimeError):
+    with pytest.raises(RuntimeError, match="shift"):
         ev.evaluate_host(batch)
+    assert bool(ev(p)[0].isnan())
+    with pytest.raises(RuntimeError, match="shift"):
+        ops.check_status()
     assert torch.equal(ev.rebuild_neighbor_list(p)(p)[1], f_new)   # the device goes on
 
 
@@ -133,3 +136,21 @@ def test_a_model_on_another_device_or_of_another_type_is_refused(U):
     mace.cpu()
     with pytest.raises(RuntimeError):
         mace(data)
+
+
+# one block of nodes and several
+@pytest.mark.parametrize("dtype,index,at,n", [(torch.float64, 3, 0, 12), (torch.float32, -1, 11, 12),
+                                              (torch.float32, 2**31 - 1, 2100, 2200)])
+def test_an_element_index_that_does_not_exist_is_reported(U, dtype, index, at, n):
+    mace, data = _small(U, dtype, n)
+    good = mace(data)
+    data["species"] = data["species"].clone()
+    data["species"][at] = index
+    bad = mace(data)
+    assert bool(bad["energy"].isnan()) and bool(bad["interaction_energy"].isnan())
+    assert bad["node_energy"].isnan().nonzero().flatten().tolist() == [at]
+    with pytest.raises(RuntimeError, match="element"):
+        ops.check_status()
+    data["species"][at] = at % 3
+    assert torch.equal(mace(data)["forces"], good["forces"])
+    ops.check_status()
