@@ -26,6 +26,7 @@ class EnergyForceEvaluator:
         self.species = None
         self.edge_index = None
         self._shifts = None   # [E, 3], or (index, table) as a host batch carries them
+        self._shift_rows = None   # [E, 3] of an (index, table), made when somebody asks
         self.topology = None
         self._graph = None
 
@@ -36,21 +37,24 @@ class EnergyForceEvaluator:
     def _set_list(self, species, edge_index, shifts, row_ptr=None):
         self.species = species.to(torch.int32).contiguous()
         self.edge_index = edge_index
-        self._shifts = shifts
+        self._shifts, self._shift_rows = shifts, None
         self.topology = ops.EdgeTopology(edge_index[1], edge_index[0], self.dom.n_owned, self.dom.n_local, row_ptr)
         self._graph = None   # a captured step belongs to the list it was captured with
         return self
 
     @property
     def shifts(self):
-        if isinstance(self._shifts, tuple):
+        if not isinstance(self._shifts, tuple):
+            return self._shifts
+        if self._shift_rows is None:   # beside the pair, not in its place: a recorded step reads the pair
             index, table = self._shifts
-            self._shifts = table.index_select(0, index.to(torch.int64))
-        return self._shifts
+            self._shift_rows = table.index_select(0, index.to(torch.int64))
+        return self._shift_rows
 
     @shifts.setter
     def shifts(self, value):
-        self._shifts = value
+        self._shifts, self._shift_rows = value, None
+        self._graph = None
 
     def rebuild_neighbor_list(self, positions_owned, r_cut=None):
         """Builds the neighbour list of the current positions on the device (cell-list kernels) instead of taking
@@ -101,8 +105,10 @@ class EnergyForceEvaluator:
         graph = torch.cuda.CUDAGraph()
         with torch.cuda.graph(graph):
             energy, forces = self(static_pos)
-        # the recording reads the plan's weights, whatever the model lays out later
-        self._graph = (graph, static_pos, energy, forces, step.plan_of(self.model))
+        # what the recording reads by address stays alive with it, whatever the attributes become: the list, the plan's
+        # weights
+        reads = (step.plan_of(self.model), self.species, self.edge_index, self._shifts, self.topology)
+        self._graph = (graph, static_pos, energy, forces, reads)
         return self
 
     def __call__(self, positions_owned):

@@ -154,3 +154,23 @@ def test_an_element_index_that_does_not_exist_is_reported(U, dtype, index, at, n
     data["species"][at] = at % 3
     assert torch.equal(mace(data)["forces"], good["forces"])
     ops.check_status()
+
+
+def test_a_recorded_step_of_a_host_batch_keeps_its_inputs(U):
+    n = 300
+    side = (n / 0.1) ** (1.0 / 3.0)
+    pos, species = systems.random_box(n, np.full(3, side), 0.9, 5), np.zeros(n, dtype=np.int64)
+    dom = domain.partition_slabs(pos, species, np.full(3, side), 1, 5.0, 0)
+    mace = model.InvariantMACE(systems.init_params(64, 1, 7), U, dtype=torch.float32, device="cuda")
+    ev = evaluator.EnergyForceEvaluator(mace, dom, "cuda")
+    e, f = ev.evaluate_host(ev.host_batch())
+    p = torch.from_numpy(dom.positions[:n]).cuda()
+    ev.capture(p)
+    pair = ev._shifts
+    rows = ev.shifts                               # as rows: the recording goes on reading the pair
+    assert torch.equal(rows.cpu(), torch.from_numpy(dom.shifts)) and ev._shifts is pair and ev.shifts is rows
+    assert any(x is pair for x in ev._graph[4])
+    assert torch.equal(ev(p)[1].cpu(), f)
+    ev.shifts = torch.zeros_like(rows)             # another list: no replay of the recorded one
+    assert ev._graph is None
+    assert not torch.equal(ev(p)[1].cpu(), f)
