@@ -89,8 +89,8 @@ class EnergyForceEvaluator:
     def capture(self, positions_owned):
         """Records the whole energy+force step for the current neighbour list as a CUDA graph; later calls copy
         the positions into the graph's input and replay it, which removes the per-launch cost that dominates
-        small systems (about a hundred launches per step).  Single-rank domains only: the halo exchange of a
-        multi-rank step is host-driven.  A new neighbour list drops the recording."""
+        small systems.  Single-rank domains only: the halo exchange of a multi-rank step is host-driven.  A new
+        neighbour list drops the recording, and so does a changed model."""
         if self.dom.nranks != 1:
             raise RuntimeError("capture() needs a single-rank domain")
         self._graph = None
@@ -113,10 +113,12 @@ class EnergyForceEvaluator:
 
     def __call__(self, positions_owned):
         if self._graph is not None and not torch.cuda.is_current_stream_capturing():
-            graph, static_pos, energy, forces, _ = self._graph
-            static_pos.copy_(positions_owned)
-            graph.replay()
-            return energy.clone(), forces.clone()
+            graph, static_pos, energy, forces, (plan, *_) = self._graph
+            if plan is None or plan.current():
+                static_pos.copy_(positions_owned)
+                graph.replay()
+                return energy.clone(), forces.clone()
+            self._graph = None   # the model has changed: the recording has the old weights laid out
 
         if step.takes(positions_owned, self._shifts):
             plan = step.plan_of(self.model)

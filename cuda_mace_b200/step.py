@@ -108,6 +108,56 @@ def _expected_buffers(model):
     return out
 
 
+# what no plan reads: the tables that a contraction's own plan is made from once, transposes that only autograd uses
+_UNREAD = ("U1_", "U2_", "U3_", "weights_transposed")
+
+
+class _Stamp:
+    """What a plan was made from: the tensors, submodules and plain attributes of a model, by identity, version or value.
+    (Edits that autograd's version counter does not see, such as those through ``.data``, are not seen here either.)"""
+
+    def __init__(self, model):
+        modules = list(model.modules())
+        self.tensors = [(d, k, t, t._version) for m in modules for d in (m._buffers, m._parameters)
+                        for k, t in d.items() if t is not None and not k.endswith("_T") and not k.startswith(_UNREAD)]
+        self.children = [(m._modules, tuple(m._modules.values())) for m in modules]
+        self.plain = [(m.__dict__, k, v) for m in modules for k, v in m.__dict__.items()
+                      if k[0] != "_" and k != "training" and isinstance(v, (bool, int, float, str, torch.dtype))]
+        # hooks of the parts would not run: the model's own run around forward()
+        self.hooks = [h for m in modules[1:] for h in (m._forward_hooks, m._forward_pre_hooks, m._backward_hooks,
+                                                       m._backward_pre_hooks)]
+        self.hooked = any(self.hooks)
+
+    def current(self):
+        for d, k, t, v in self.tensors:
+            if d.get(k) is not t or t._version != v:
+                return False
+        for d, v in self.children:
+            if tuple(d.values()) != v:
+                return False
+        for d, k, v in self.plain:
+            if d.get(k) != v:
+                return False
+        return any(self.hooks) == self.hooked
+
+
+_PARTS = ("node_energies", "_messages", "_radial_weights", "_mm")   # what forward() is made of
+
+
+def _is_standard(model):
+    """Whether the model's parts are the package's own: a subclass or a replaced module computes something else."""
+    from .model import InvariantMACE
+
+    L0, L1 = model.layers
+    parts = [(model.edge_basis, ops.EdgeBasis), (model.spherical_harmonics, ops.SphericalHarmonics),
+             (model.tp, ops.InvariantMessagePassingTP), (L0.linear, ops.ElementalLinear), (L1.linear, ops.Linear)]
+    parts += [(L.contraction, ops.SymmetricContraction) for L in model.layers]
+    if model.radial == "spline":
+        parts += [(L.spline, ops.CubicSpline) for L in model.layers]
+    return (all(type(m) is kind for m, kind in parts)
+            and all(getattr(type(model), k) is getattr(InvariantMACE, k) and k not in model.__dict__ for k in _PARTS))
+
+
 def covers(model):
     """Whether the sequence covers a model: the standard two-layer architecture in float32 or float64, every buffer with
     the shape and type it was built with, on one device (kernels get plain pointers: a model that was converted or
@@ -116,7 +166,7 @@ def covers(model):
         return False
     if model.dtype not in (torch.float32, torch.float64) or model.channels not in (32, 64, 96, 128):
         return False
-    if os.environ.get("CMACE_SYMCON_GENERIC", "")[:1] == "1":
+    if not _is_standard(model):
         return False
     if model.radial == "exact" and model.edge_basis.num_bessel not in (8, 16):
         return False
@@ -137,8 +187,7 @@ class StepPlan:
 
     def __init__(self, model):
         self.keep = []
-        # what the layout was made from: any replaced or modified buffer makes a new plan necessary
-        self.sources = [(m._buffers, k, t, t._version) for m in model.modules() for k, t in m._buffers.items()]
+        self.stamp = _Stamp(model)
         f32 = model.dtype == torch.float32
         C, Z = model.channels, model.num_elements
         L0, L1 = model.layers
@@ -244,33 +293,33 @@ class StepPlan:
             m.fold_back[b] = matrix(blocks[b])
 
     def current(self):
-        for d, k, t, v in self.sources:
-            if d.get(k) is not t or t._version != v:
-                return False
-        return True
+        return self.stamp.current()
 
 
 def plan_of(model):
-    """The model's plan, laid out again when a weight has changed; None when the sequence does not cover the model or
-    the module-level switches of ops select other kernels."""
+    """The model's plan, laid out again when the model has changed; None when the sequence does not cover the model, or
+    the module-level switches of ops or the environment select other kernels."""
     if not ops.USE_TENSOR_CORES or ops.FUSED_RADIAL_MESSAGE_PASSING or not ops.RADIAL_GRADIENT_ON_THE_FLY:
         return None
-    plan = model.__dict__.get("_step_plan")
-    if plan is False:
+    if os.environ.get("CMACE_SYMCON_GENERIC", "")[:1] == "1":
         return None
-    if plan is not None and plan.current():
+    stamp, plan = model.__dict__.get("_step_plan", (None, None))
+    if stamp is not None and stamp.current():
         return plan
     dev = model.embedding.device
     if dev.type != "cuda" or dev.index != torch.cuda.current_device():
         return None   # the operators refuse such a call
     plan = None
-    if covers(model):
+    stamp = _Stamp(model)
+    if not stamp.hooked and covers(model):
         try:
-            plan = StepPlan(model)
+            with torch.no_grad():
+                plan = StepPlan(model)
+            stamp = plan.stamp
         except RuntimeError as e:
             if "not the generated program" not in str(e):
                 raise
-    model.__dict__["_step_plan"] = plan if plan is not None else False
+    model.__dict__["_step_plan"] = (stamp, plan)
     return plan
 
 

@@ -174,3 +174,53 @@ def test_a_recorded_step_of_a_host_batch_keeps_its_inputs(U):
     ev.shifts = torch.zeros_like(rows)             # another list: no replay of the recorded one
     assert ev._graph is None
     assert not torch.equal(ev(p)[1].cpu(), f)
+
+
+@pytest.mark.parametrize("how", ["model", "captured"])
+def test_a_changed_model_changes_the_step(U, how):
+    """scale, shift and r_max like the weights: the step agrees with node_energies() after every change, recorded or not;
+    a model that the sequence has refused is taken again once it is what it was."""
+    n = 300
+    side = (n / 0.1) ** (1.0 / 3.0)
+    pos, species = systems.random_box(n, np.full(3, side), 0.9, 5), np.zeros(n, dtype=np.int64)
+    dom = domain.partition_slabs(pos, species, np.full(3, side), 1, 5.0, 0)
+    mace = model.InvariantMACE(systems.init_params(32, 1, 7), U, dtype=torch.float64, device="cuda")
+    ev = evaluator.EnergyForceEvaluator(mace, dom, "cuda")
+    p = ev.load_domain()
+
+    def agrees():
+        q = p.clone().requires_grad_(True)
+        e = mace.node_energies(q, ev.species, ev.edge_index, ev.shifts).sum()
+        (g,), e = torch.autograd.grad(e, q), e.detach()
+        if how == "captured":
+            got = ev(p)
+        else:
+            out = mace(dict(positions=p, species=ev.species, edge_index=ev.edge_index, shifts=ev.shifts))
+            got = out["interaction_energy"], out["forces"]
+        assert abs(float(got[0] - e)) < 1e-10 * abs(float(e))
+        assert float((got[1] + g).abs().max()) < 1e-10 * float(g.abs().max())
+
+    def scale():
+        mace.scale = 1.7
+
+    def shift():
+        mace.shift = -0.25
+
+    def radius():
+        mace.edge_basis.r_max = 4.5
+
+    def weight():
+        for W in (mace.layers[1].W_readout2, mace.layers[1].W_readout2_T):
+            W.mul_(0.5)
+
+    for change in (scale, shift, radius, weight):
+        if how == "captured":
+            ev.capture(p)
+        agrees()
+        change()
+        agrees()
+    assert step.plan_of(mace) is not None
+    hook = mace.layers[1].linear.register_forward_hook(lambda *a: None)
+    assert step.plan_of(mace) is None
+    hook.remove()
+    assert step.plan_of(mace) is not None
