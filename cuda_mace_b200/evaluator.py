@@ -102,12 +102,16 @@ class EnergyForceEvaluator:
                 self(static_pos)
         torch.cuda.current_stream(self.device).wait_stream(side)
         ops.check_status()
+        plan = step.plan_of(self.model) if step.takes(static_pos, self._shifts) else None
+        others = plan is not None and plan.recorded
         graph = torch.cuda.CUDAGraph()
         with torch.cuda.graph(graph):
             energy, forces = self(static_pos)
+        if plan is not None:
+            plan.recorded = others   # kept below, by this object
         # what the recording reads by address stays alive with it, whatever the attributes become: the list, the plan's
         # weights
-        reads = (step.plan_of(self.model), self.species, self.edge_index, self._shifts, self.topology)
+        reads = (plan, self.species, self.edge_index, self._shifts, self.topology)
         self._graph = (graph, static_pos, energy, forces, reads)
         return self
 

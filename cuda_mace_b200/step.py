@@ -187,6 +187,7 @@ class StepPlan:
 
     def __init__(self, model):
         self.keep = []
+        self.recorded = False   # a graph that somebody else keeps reads this plan by address
         self.stamp = _Stamp(model)
         f32 = model.dtype == torch.float32
         C, Z = model.channels, model.num_elements
@@ -298,7 +299,11 @@ class StepPlan:
 
 def plan_of(model):
     """The model's plan, laid out again when the model has changed; None when the sequence does not cover the model, or
-    the module-level switches of ops or the environment select other kernels."""
+    the module-level switches of ops or the environment select other kernels.
+
+    A plan is finished before anybody sees it and goes when nobody reads it any more, so that any stream may use it without
+    an event: one synchronisation per set of weights.  While a stream
+    is captured nothing is laid out (the kernels would be recorded, not run): such a step takes the operators."""
     if not ops.USE_TENSOR_CORES or ops.FUSED_RADIAL_MESSAGE_PASSING or not ops.RADIAL_GRADIENT_ON_THE_FLY:
         return None
     if os.environ.get("CMACE_SYMCON_GENERIC", "")[:1] == "1":
@@ -309,17 +314,25 @@ def plan_of(model):
     dev = model.embedding.device
     if dev.type != "cuda" or dev.index != torch.cuda.current_device():
         return None   # the operators refuse such a call
-    plan = None
+    if torch.cuda.is_current_stream_capturing():
+        return None
+    before, plan = plan, None
     stamp = _Stamp(model)
     if not stamp.hooked and covers(model):
         try:
             with torch.no_grad():
                 plan = StepPlan(model)
             stamp = plan.stamp
+            torch.cuda.current_stream(dev).synchronize()
         except RuntimeError as e:
             if "not the generated program" not in str(e):
                 raise
     model.__dict__["_step_plan"] = (stamp, plan)
+    if before is not None:
+        if before.recorded:
+            model.__dict__.setdefault("_step_recorded", []).append(before)
+        else:
+            torch.cuda.synchronize(dev)   # steps on other streams may still read it
     return plan
 
 
@@ -375,6 +388,8 @@ def energy_forces(plan, positions, species, one_hot, shifts, topology, halo=None
     if positions.shape != (nl, 3) or shifts.shape[1:] != (3,) or (shifts if index is None else index).shape[0] != E:
         raise RuntimeError(f"shape mismatch: positions {tuple(positions.shape)}, shifts {tuple(shifts.shape)} for "
                            f"{nl} atoms and {E} edges")
+    capturing = torch.cuda.is_current_stream_capturing()
+    plan.recorded = plan.recorded or capturing
     out = torch.empty(3 + 2 * n + 3 * nl, dtype=torch.float64, device=dev)
     m = plan.model
     nbytes = _abi.call("cmace_step_workspace_bytes", ctypes.byref(m), n, nl, E)
@@ -383,7 +398,7 @@ def energy_forces(plan, positions, species, one_hot, shifts, topology, halo=None
     # longer (40 us at 160 000 edges) than the second stream costs the host (about 15 us).  Its launches come after those
     # of the first two steps, which keep the device busy meanwhile.
     beside = buffers = ready = None
-    if topology._perm is None and E >= _BESIDE_EDGES and not torch.cuda.is_current_stream_capturing():
+    if topology._perm is None and E >= _BESIDE_EDGES and not capturing:
         beside = _side_stream(dev)
         buffers = topology.grouping_buffers()
         perm, send_ptr, _ = buffers

@@ -224,3 +224,56 @@ def test_a_changed_model_changes_the_step(U, how):
     assert step.plan_of(mace) is None
     hook.remove()
     assert step.plan_of(mace) is not None
+
+
+# what a plan is made of has to be there for every stream, and to stay for whoever still reads it
+def test_a_plan_laid_out_on_one_stream_serves_another(U):
+    mace, data = _small(U, torch.float32)
+    want = mace(data)["forces"]
+    first, second = torch.cuda.Stream(), torch.cuda.Stream()
+    for _ in range(3):
+        mace.layers[1].W_readout2.mul_(1.0)          # another version: laid out again
+        torch.cuda.synchronize()
+        with torch.cuda.stream(first):
+            torch.cuda._sleep(20_000_000)            # some 10 ms before the layout's kernels
+            a = mace(data)["forces"]
+        with torch.cuda.stream(second):
+            b = mace(data)["forces"]
+        torch.cuda.synchronize()
+        assert torch.equal(a, want) and torch.equal(b, want)
+
+
+def _record(mace, data):
+    side, graph = torch.cuda.Stream(), torch.cuda.CUDAGraph()
+    side.wait_stream(torch.cuda.current_stream())
+    with torch.cuda.graph(graph, stream=side):
+        out = mace(data)
+    return graph, out
+
+
+def test_a_graph_of_the_caller_keeps_the_weights_it_reads(U):
+    mace, data = _small(U, torch.float32)
+    want = mace(data)["forces"].clone()
+    graph, out = _record(mace, data)
+    old = step.plan_of(mace)
+    sizes = [t.numel() * t.element_size() for t in old.keep]
+    mace.layers[1].W_readout2.mul_(2.0)
+    changed = mace(data)["forces"].clone()
+    assert step.plan_of(mace) is not old and not torch.equal(changed, want)
+    del old
+    junk = [torch.full((s,), 255, dtype=torch.uint8, device="cuda") for s in sizes for _ in range(4)]
+    graph.replay()
+    assert torch.equal(out["forces"], want) and len(junk) > 0
+
+
+@pytest.mark.parametrize("dtype,tol", [(torch.float64, 1e-10), (torch.float32, 1e-4)])
+def test_no_layout_while_a_graph_is_recorded(U, dtype, tol):
+    mace, data = _small(U, dtype)
+    mace(data)
+    mace.node_energies(data["positions"], data["species"], data["edge_index"], data["shifts"])
+    for W in (mace.layers[1].W_readout2, mace.layers[1].W_readout2_T):
+        W.mul_(2.0)
+    graph, out = _record(mace, data)
+    eager = mace(data)["forces"]
+    graph.replay()
+    assert float((out["forces"] - eager).abs().max()) < tol * float(eager.abs().max())
