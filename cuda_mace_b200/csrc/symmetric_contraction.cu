@@ -203,18 +203,22 @@ static bool force_generic() {
   return e != nullptr && e[0] == '1';
 }
 
-// weff [Z][13][C]: the effective class weights above, written once for kernels that read them per (element, channel)
+// weff [Z][13][C]: the effective class weights above, written out for kernels that read them per (element, channel)
 template <typename T>
 __global__ void effective_weights_kernel(const int32_t *__restrict__ cclass3, const int32_t *__restrict__ cclass2,
                                          const T *__restrict__ cscale3, const T *__restrict__ cscale2, int w3, int w2,
                                          int w1, const T *__restrict__ W3, const T *__restrict__ W2,
                                          const T *__restrict__ W1, int C, T *__restrict__ weff) {
   constexpr int NW = canon::NCLASS3 + canon::NCLASS2 + 1;
-  const int c = threadIdx.x, z = blockIdx.x, q = blockIdx.y;
+  const int c = blockIdx.z * blockDim.x + threadIdx.x, z = blockIdx.x, q = blockIdx.y;
+  if (c >= C) return;
   T acc = T(0);
   if (q < canon::NCLASS3) {
-    for (int p = 0; p < w3; p++)
-      if (cclass3[p] == q) acc += cscale3[p] * W3[((int64_t)z * w3 + p) * C + c];
+#pragma unroll 8   // the loads of several paths on their way, the class's or not
+    for (int p = 0; p < w3; p++) {
+      const T w = W3[((int64_t)z * w3 + p) * C + c];
+      if (cclass3[p] == q) acc = fma(cscale3[p], w, acc);
+    }
   } else if (q < NW - 1) {
     for (int p = 0; p < w2; p++)
       if (cclass2[p] == q - canon::NCLASS3) acc += cscale2[p] * W2[((int64_t)z * w2 + p) * C + c];
@@ -401,21 +405,22 @@ int cmace_symcon_bwd_f64(const cmace_symcon_plan *plan, const double *X, const i
 
 int cmace_symcon_effective_weights(const cmace_symcon_plan *plan, int is_f64, const void *W3, const void *W2,
                                    const void *W1, int nelements, int channels, void *out, cmace_stream_t stream) {
-  if (!plan || !W3 || !W2 || !W1 || !out || nelements < 1 || channels < 1 || channels > 1024)
+  if (!plan || !W3 || !W2 || !W1 || !out || nelements < 1 || channels < 1)
     return fail(CMACE_ERR_ARG, "cmace_symcon_effective_weights: bad argument");
   if (!plan->canonical || force_generic())
     return fail(CMACE_ERR_UNSUPPORTED, "cmace_symcon_effective_weights: the plan's tables are not the generated program's");
   const int32_t *ci = plan->d_ints + plan->canon_int_off;
-  const dim3 grid((unsigned)nelements, canon::NCLASS3 + canon::NCLASS2 + 1);
+  const int threads = channels < 128 ? channels : 128;
+  const dim3 grid((unsigned)nelements, canon::NCLASS3 + canon::NCLASS2 + 1, (unsigned)((channels + threads - 1) / threads));
   cudaStream_t st = (cudaStream_t)stream;
   if (is_f64) {
     const double *cr = plan->d_f64 + plan->canon_real_off;
-    effective_weights_kernel<double><<<grid, channels, 0, st>>>(
+    effective_weights_kernel<double><<<grid, threads, 0, st>>>(
         ci, ci + plan->w3, cr, cr + plan->w3, plan->w3, plan->w2, plan->w1, static_cast<const double *>(W3),
         static_cast<const double *>(W2), static_cast<const double *>(W1), channels, static_cast<double *>(out));
   } else {
     const float *cr = plan->d_f32 + plan->canon_real_off;
-    effective_weights_kernel<float><<<grid, channels, 0, st>>>(
+    effective_weights_kernel<float><<<grid, threads, 0, st>>>(
         ci, ci + plan->w3, cr, cr + plan->w3, plan->w3, plan->w2, plan->w1, static_cast<const float *>(W3),
         static_cast<const float *>(W2), static_cast<const float *>(W1), channels, static_cast<float *>(out));
   }

@@ -370,37 +370,39 @@ std::shared_ptr<PlanHolder> plan_for(int64_t u3_max, const Tensor &U3_num, const
 
 struct PlanBox : torch::CustomClassHolder {
   std::shared_ptr<PlanHolder> holder;
-  Tensor weff;   // effective weights of the generated program; undefined when the table-driven kernel runs
 };
 
-// Effective contraction weights [Z, 13, C] per weight set: constant buffers of a model, laid out once like the packed
-// matrices above (the entry keeps its sources alive, the version counters catch in-place edits).  Combining them inside
-// the contraction kernel cost every block a pass over all elements' paths: 42 us of a 4096-node call over 10 elements.
-struct EffectiveEntry {
-  Tensor w3, w2, w1, weff;
-  std::shared_ptr<PlanHolder> plan;
+// The generated program on effective weights [Z, 13, C].  They are laid out by every call, in a launch of its own: the
+// weights are inputs of the operator, and nothing but reading them shows whether they are the last call's.  (Combining them
+// inside the contraction kernel costs every block a pass over all elements' paths.)
+class SymConProgramAutograd : public torch::autograd::Function<SymConProgramAutograd> {
+ public:
+  static Tensor forward(AutogradContext *ctx, Tensor X, Tensor atom_types, Tensor weff) {
+    Range nvtx("cuda_mace_b200::symmetric_contraction::forward");
+    X = X.contiguous();
+    const int64_t N = X.size(0), C = X.size(2);
+    Tensor out = torch::empty({N, 1, C}, X.options());
+    check(cmace_symcon_apply(is_f64(X) ? 1 : 0, X.data_ptr(), atom_types.data_ptr<int32_t>(), weff.data_ptr(), nullptr, N,
+                             (int)C, out.data_ptr(), stream_of(X)),
+          "cmace_symcon_apply");
+    ctx->save_for_backward({X, atom_types, weff});
+    return out;
+  }
+  static variable_list backward(AutogradContext *ctx, variable_list grads) {
+    Range nvtx("cuda_mace_b200::symmetric_contraction::backward");
+    auto s = ctx->get_saved_variables();
+    const Tensor &X = s[0];
+    c10::cuda::CUDAGuard guard(X.device());
+    Tensor G = grads[0].contiguous();
+    Tensor gradX = torch::empty_like(X);
+    check(cmace_symcon_apply(is_f64(X) ? 1 : 0, X.data_ptr(), s[1].data_ptr<int32_t>(), s[2].data_ptr(), G.data_ptr(),
+                             X.size(0), (int)X.size(2), gradX.data_ptr(), stream_of(X)),
+          "cmace_symcon_apply");
+    return {gradX, Tensor(), Tensor()};
+  }
 };
 
-Tensor effective_weights(const std::shared_ptr<PlanHolder> &holder, const Tensor &w3, const Tensor &w2, const Tensor &w1) {
-  if (!cmace_symcon_plan_uses_program(holder->plan)) return Tensor();
-  static std::mutex m;
-  using Key = std::tuple<void *, void *, void *, void *, int64_t, int64_t, int64_t, int, int64_t, int64_t>;
-  static std::map<Key, EffectiveEntry> cache;
-  const Key key = std::make_tuple((void *)holder->plan, w3.data_ptr(), w2.data_ptr(), w1.data_ptr(), (int64_t)w3._version(),
-                                  (int64_t)w2._version(), (int64_t)w1._version(), (int)w3.scalar_type(), w3.size(0),
-                                  w3.size(2));
-  std::lock_guard<std::mutex> lock(m);
-  auto it = cache.find(key);
-  if (it != cache.end()) return it->second.weff;
-  if (cache.size() > 32) cache.clear();
-  Tensor weff = torch::empty({w3.size(0), 13, w3.size(2)}, w3.options());
-  check(cmace_symcon_effective_weights(holder->plan, is_f64(w3) ? 1 : 0, w3.data_ptr(), w2.data_ptr(), w1.data_ptr(),
-                                       (int)w3.size(0), (int)w3.size(2), weff.data_ptr(), stream_of(w3)),
-        "cmace_symcon_effective_weights");
-  cache.emplace(key, EffectiveEntry{w3, w2, w1, weff, holder});
-  return weff;
-}
-
+// the table-driven kernel: tables that the generated program does not know
 class SymConAutograd : public torch::autograd::Function<SymConAutograd> {
  public:
   static Tensor forward(AutogradContext *ctx, Tensor X, Tensor atom_types, Tensor W3, Tensor W2, Tensor W1,
@@ -411,11 +413,7 @@ class SymConAutograd : public torch::autograd::Function<SymConAutograd> {
     const int64_t N = X.size(0), C = X.size(2), Z = W3.size(0);
     Tensor out = torch::empty({N, 1, C}, X.options());
     const cmace_symcon_plan *plan = box->holder->plan;
-    if (box->weff.defined())
-      check(cmace_symcon_apply(is_f64(X) ? 1 : 0, X.data_ptr(), atom_types.data_ptr<int32_t>(), box->weff.data_ptr(), nullptr,
-                               N, (int)C, out.data_ptr(), stream_of(X)),
-            "cmace_symcon_apply");
-    else if (is_f64(X))
+    if (is_f64(X))
       check(cmace_symcon_fwd_f64(plan, X.data_ptr<double>(), atom_types.data_ptr<int32_t>(), W3.data_ptr<double>(),
                                  W2.data_ptr<double>(), W1.data_ptr<double>(), (int)Z, N, (int)C,
                                  out.data_ptr<double>(), stream_of(X)),
@@ -439,11 +437,7 @@ class SymConAutograd : public torch::autograd::Function<SymConAutograd> {
     const int64_t N = X.size(0), C = X.size(2), Z = W3.size(0);
     Tensor gradX = torch::empty_like(X);
     const cmace_symcon_plan *plan = box->holder->plan;
-    if (box->weff.defined())
-      check(cmace_symcon_apply(is_f64(X) ? 1 : 0, X.data_ptr(), atom_types.data_ptr<int32_t>(), box->weff.data_ptr(),
-                               G.data_ptr(), N, (int)C, gradX.data_ptr(), stream_of(X)),
-            "cmace_symcon_apply");
-    else if (is_f64(X))
+    if (is_f64(X))
       check(cmace_symcon_bwd_f64(plan, X.data_ptr<double>(), atom_types.data_ptr<int32_t>(), W3.data_ptr<double>(),
                                  W2.data_ptr<double>(), W1.data_ptr<double>(), G.data_ptr<double>(), (int)Z, N, (int)C,
                                  gradX.data_ptr<double>(), stream_of(X)),
@@ -564,17 +558,31 @@ class SymmetricContraction : public torch::CustomClassHolder {
     c10::cuda::CUDAGuard guard(X.device());
     (void)U1_num_nonzero;  // accepted for signature compatibility; the reference kernel does not read them either
     (void)U1_index;        // (symmetric_contraction_impl.cu:115-117)
+    const auto holder = plan_for(U3_max_nonsparse, U3_num_nonzero, U3_indices, U3_values, U2_num_nonzero, U2_indices,
+                                 U2_values, W3_size, W2_size, W1_size, (int)X.device().index());
+    TORCH_CHECK(X.dim() == 3 && X.size(1) == 16, "X must be [nnodes, 16, C]");
+    const Tensor w[3] = {W3.contiguous(), W2.contiguous(), W1.contiguous()};
+    const int64_t paths[3] = {W3_size, W2_size, W1_size};
+    for (int k = 0; k < 3; k++) {
+      // the reference's buffers are [nlout, Z, w, C]; output irrep 0, the first, is the one it contracts (impl.cu:64-76)
+      TORCH_CHECK((w[k].dim() == 3 || w[k].dim() == 4) && w[k].numel() > 0, "weights must be [nlout, Z, w, C] or [Z, w, C]");
+      TORCH_CHECK(w[k].scalar_type() == X.scalar_type(), "X and the weights must have the same dtype");
+      TORCH_CHECK(w[k].device() == X.device(), "X and the weights must be on the same device");
+      TORCH_CHECK(w[k].size(-2) == paths[k], "weight buffers do not match W3_size / W2_size / W1_size");
+      TORCH_CHECK(w[k].size(-3) >= w[0].size(-3) && w[k].size(-1) == X.size(2), "weights do not match in elements or channels");
+    }
+    if (cmace_symcon_plan_uses_program(holder->plan)) {
+      Tensor weff = torch::empty({w[0].size(-3), 13, X.size(2)}, w[0].options());
+      check(cmace_symcon_effective_weights(holder->plan, is_f64(X) ? 1 : 0, w[0].data_ptr(), w[1].data_ptr(),
+                                           w[2].data_ptr(), (int)weff.size(0), (int)weff.size(2), weff.data_ptr(),
+                                           stream_of(X)),
+            "cmace_symcon_effective_weights");
+      return SymConProgramAutograd::apply(X, int32_contig(atom_types), weff);
+    }
     auto box = c10::make_intrusive<PlanBox>();
-    box->holder = plan_for(U3_max_nonsparse, U3_num_nonzero, U3_indices, U3_values, U2_num_nonzero, U2_indices,
-                           U2_values, W3_size, W2_size, W1_size, (int)X.device().index());
-    // the reference's buffers are [nlout, Z, w, C]; output irrep 0 is the one it contracts (impl.cu:64-76)
-    auto first = [](const Tensor &w) { return (w.dim() == 4 ? w.select(0, 0) : w).contiguous(); };
-    Tensor w3 = first(W3), w2 = first(W2), w1 = first(W1);
-    TORCH_CHECK(w3.scalar_type() == X.scalar_type(), "X and the weights must have the same dtype");
-    TORCH_CHECK(w3.size(1) == W3_size && w2.size(1) == W2_size && w1.size(1) == W1_size,
-                "weight buffers do not match W3_size / W2_size / W1_size");
-    box->weff = effective_weights(box->holder, w3, w2, w1);
-    return SymConAutograd::apply(X, int32_contig(atom_types), w3, w2, w1, box);
+    box->holder = holder;
+    auto first = [](const Tensor &t) { return t.dim() == 4 ? t.select(0, 0) : t; };
+    return SymConAutograd::apply(X, int32_contig(atom_types), first(w[0]), first(w[1]), first(w[2]), box);
   }
   std::vector<Tensor> __getstate__() { return {}; }
   void __setstate__(const std::vector<Tensor> &) {}

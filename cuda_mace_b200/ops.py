@@ -728,23 +728,16 @@ def make_plan(u3_max, U3_num_nonzero, U3_indices, U3_values, U2_num_nonzero, U2_
     return _Plan(handle)
 
 
-_effective_cache = _RefCache(16)
-
-
 def effective_weights(plan, W3, W2, W1):
-    """[Z, 13, C] weights of the generated contraction program, laid out once per weight set; None when the plan runs on
-    the table-driven kernel."""
+    """[Z, 13, C] weights of the generated contraction program, laid out anew for every call (they are inputs of the
+    operator); None when the plan runs on the table-driven kernel."""
     if not _abi.call("cmace_symcon_plan_uses_program", plan.handle):
         return None
-    key = _RefCache.key(W3, W2, W1) + (plan.handle.value,)
-    hit = _effective_cache.get(key)
-    if hit is not None:
-        return hit
     Z, C = W3.shape[0], W3.shape[2]
     weff = torch.empty(Z, 13, C, dtype=W3.dtype, device=W3.device)
     _abi.call("cmace_symcon_effective_weights", plan.handle, int(W3.dtype == torch.float64), _ptr(W3), _ptr(W2), _ptr(W1),
               Z, C, _ptr(weff), _stream())
-    return _effective_cache.put(key, (W3, W2, W1, plan), weff)
+    return weff
 
 
 class _SymConFunction(torch.autograd.Function):
@@ -800,7 +793,7 @@ def symmetric_contraction_forward(X, atom_types, U3_max_nonsparse, U3_num_nonzer
                 make_plan(U3_max_nonsparse, U3_num_nonzero, U3_indices, U3_values, U2_num_nonzero, U2_indices,
                           U2_values, W3_size, W2_size, W1_size))
     W3, W2, W1 = [w[0] if w.dim() == 4 else w for w in (W3, W2, W1)]
-    if W3.dtype != X.dtype:
+    if not W3.dtype == W2.dtype == W1.dtype == X.dtype:
         raise TypeError("X and the weights must have the same dtype")
     if W3.shape[1] != W3_size or W2.shape[1] != W2_size or W1.shape[1] != W1_size:
         raise RuntimeError("weight buffers do not match W3_size/W2_size/W1_size")

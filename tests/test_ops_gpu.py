@@ -180,6 +180,7 @@ def test_elemental_linear_on_nodes_stored_grouped_by_element(dtype, N, Z, K, dev
 
 @pytest.mark.parametrize("dtype", DTYPES)
 @pytest.mark.parametrize("N,C,Z", [(256, 128, 10), (19, 32, 1), (64, 64, 4),
+                                   (7, 1056, 2),       # more channels than a block has threads
                                    (4096, 128, 10)])   # last: the benchmark spec's configuration at full size
 def test_symmetric_contraction(dtype, N, C, Z, dev, U):
     from cuda_mace_b200 import ops
@@ -199,6 +200,43 @@ def test_symmetric_contraction(dtype, N, C, Z, dev, U):
     (out ** 2).sum().backward()
     assert rel_err(out, ref) < TOL[dtype]["out"]
     assert rel_err(Xg.grad, Xo.grad) < TOL[dtype]["grad"]
+
+
+def test_symmetric_contraction_needs_one_type(dev, U):
+    from cuda_mace_b200 import ops
+
+    W = [torch.randn(2, n, 32) for n in (23, 4, 1)]
+    for k in range(3):
+        mod = ops.SymmetricContraction(*U, *[w.double() if i == k else w for i, w in enumerate(W)]).to(dev)
+        with pytest.raises(TypeError):
+            mod(torch.randn(5, 16, 32, device=dev), torch.zeros(5, dtype=torch.int32, device=dev))
+
+
+@pytest.mark.parametrize("dtype", DTYPES)
+@pytest.mark.parametrize("N,C,Z", [(19, 32, 1), (300, 128, 10), (40, 256, 3), (33, 96, 40)])
+def test_symmetric_contraction_c_entry_points(dtype, N, C, Z, dev, U):
+    """cmace_symcon_fwd / _bwd, which combine the weights themselves; 40 elements: their table does not fit in shared
+    memory and the table-driven kernel runs."""
+    from cuda_mace_b200 import _abi, ops
+    from oracle import ops as oops
+
+    g = torch.Generator().manual_seed(N + C)
+    X = torch.randn(N, 16, C, generator=g, dtype=torch.float64).to(dtype)
+    at = torch.randint(0, Z, (N,), generator=g, dtype=torch.int32)
+    W = [torch.randn(Z, n, C, generator=g, dtype=torch.float64).to(dtype) / n for n in (23, 4, 1)]
+    G = torch.randn(N, 1, C, generator=g, dtype=torch.float64).to(dtype)
+    Xo = X.double().clone().requires_grad_(True)
+    ref = oops.symmetric_contraction_chunked(Xo, at, *U, *[w.double() for w in W])
+    ref.backward(G.double())
+    mod = ops.SymmetricContraction(*U, *W).to(dev)
+    Xg, atg, Gg, Wg = X.to(dev), at.to(dev), G.to(dev), [w.to(dev) for w in W]
+    mod(Xg, atg)   # makes the plan
+    out, grad = torch.empty(N, 1, C, dtype=dtype, device=dev), torch.empty_like(Xg)
+    head = (mod._plan.handle, Xg.data_ptr(), atg.data_ptr(), *[w.data_ptr() for w in Wg])
+    tail = (Z, N, C)
+    _abi.call("cmace_symcon_fwd_" + ops._suffix(Xg), *head, *tail, out.data_ptr(), ops._stream())
+    _abi.call("cmace_symcon_bwd_" + ops._suffix(Xg), *head, Gg.data_ptr(), *tail, grad.data_ptr(), ops._stream())
+    assert rel_err(out, ref) < TOL[dtype]["out"] and rel_err(grad, Xo.grad) < TOL[dtype]["grad"]
 
 
 def test_symmetric_contraction_reference_argument_list(dev, U):

@@ -95,6 +95,36 @@ def test_linear_classes(classes, dtype):
 
 
 @pytest.mark.gpu
+def test_contraction_reads_its_weights_in_every_call(classes, U):
+    """The weights are inputs: edits that no version counter sees count, tensors without one are taken, each of them has to
+    have X's type."""
+    from oracle import ops as oops
+
+    d = lambda t: t.cuda()
+    maxnz, *tables = oops.pack_sparse_u(*U)
+    tables = [d(t) for t in tables]
+    g = torch.Generator().manual_seed(1)
+    N, C, Z = 24, 32, 2
+    X, at = torch.randn(N, 16, C, generator=g), torch.randint(0, Z, (N,), generator=g, dtype=torch.int32)
+    W = [torch.randn(1, Z, n, C, generator=g) / n for n in (23, 4, 1)]
+    op = classes.symm_contract.SymmetricContraction()
+    run = lambda W: op.forward(d(X), d(at), maxnz, *tables, *W, 23, 4, 1)
+    Wg = [d(w) for w in W]
+    out = run(Wg)
+    assert rel_err(out, oops.symmetric_contraction(X.double(), at, *U, *[w[0].double() for w in W])) < 1e-5
+    for w in Wg:
+        w.data.mul_(2.0)
+    assert torch.equal(run(Wg), 2.0 * out)
+    with torch.inference_mode():
+        made = [d(w) for w in W]
+    assert torch.equal(run(made), out)
+    for k in range(3):
+        other = [w.double() if i == k else w for i, w in enumerate(Wg)]
+        with pytest.raises(RuntimeError):
+            run(other)
+
+
+@pytest.mark.gpu
 def test_contraction_harmonics_and_spline_classes(classes, U):
     from oracle import ops as oops
     from oracle import sh as osh
