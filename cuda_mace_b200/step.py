@@ -56,7 +56,11 @@ def basis_bounds(nb, r_max, p):
 
 def half_scales(Ws, bounds):
     """The 13 powers of two of the fp16 radial kernel and the weights' factors, or None when a bound of some layer's
-    values or derivatives exceeds 2^15.  |silu(z)| <= |z| and |silu'| < 1.1 carry the bounds from layer to layer."""
+    values or derivatives exceeds 2^15 or a weight is not finite.  |silu(z)| <= |z| and |silu'| < 1.1 carry the bounds from
+    layer to layer."""
+    if not all(bool(W.isfinite().all()) for W in Ws):
+        return None
+
     def power(t):   # the power of two that puts the largest entry just below 2^15
         return 14 - math.floor(math.log2(max(float(t.max()), 1e-30)))
 
@@ -261,7 +265,7 @@ class StepPlan:
         if f32:
             bounds = basis_bounds(m.nbessel, m.r_max, m.cutoff_p)
             scales = [half_scales([getattr(L, f"W_radial{i}") for i in range(3)], bounds) for L in (L0, L1)]
-            if None not in scales:
+            if None not in scales and bool(L1.W_radial3.isfinite().all()):
                 for t, L in enumerate((L0, L1)):
                     values, factors = scales[t]
                     if t == 1 and C != 128:   # the second layer's h and h' leave as float32: undo the stored scale

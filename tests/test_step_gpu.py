@@ -277,3 +277,14 @@ def test_no_layout_while_a_graph_is_recorded(U, dtype, tol):
     eager = mace(data)["forces"]
     graph.replay()
     assert float((out["forces"] - eager).abs().max()) < tol * float(eager.abs().max())
+
+
+# a diverged model: NaN comes out, as from the operators, instead of an error from the layout
+@pytest.mark.parametrize("dtype,C", [(torch.float32, 128), (torch.float32, 32), (torch.float64, 32)])
+@pytest.mark.parametrize("layer,which", [(0, 0), (1, 2), (1, 3)])
+def test_weights_that_are_not_finite(U, dtype, C, layer, which):
+    mace, data = _small(U, dtype, C=C)
+    getattr(mace.layers[layer], f"W_radial{which}")[1, 2] = float("nan")
+    out = mace(data)
+    assert bool(out["energy"].isnan()) and bool(out["forces"].isnan().any())
+    ops.check_status()

@@ -70,3 +70,15 @@ def test_a_model_with_parts_of_its_own_is_not_covered(U):
 
     mace.layers[1].linear = Doubled(mace.layers[1].linear.weights)
     assert not step.covers(mace)
+
+
+@pytest.mark.parametrize("value", [float("nan"), float("inf")])
+def test_no_fp16_range_for_weights_that_are_not_finite(value):
+    Ws = [torch.full((8, 64), 0.1), torch.full((64, 64), 0.1), torch.full((64, 64), 0.1)]
+    bounds = step.basis_bounds(8, 5.0, 5)
+    assert step.half_scales(Ws, bounds) is not None
+    for W in Ws:
+        old = float(W[3, 5])
+        W[3, 5] = value
+        assert step.half_scales(Ws, bounds) is None
+        W[3, 5] = old
