@@ -75,7 +75,8 @@ def half_scales(Ws, bounds):
         nv, nd = power(v), power(d)
         if min(nv, nd, sv, sd) < 0:
             return None
-        nv, nd = min(nv, 12), min(nd, 12)
+        # the split's absolute error, 2^-25, has to stay small beside small values too; 2^60 is far from float32's end
+        nv, nd = min(nv, 60), min(nd, 60)
         z.append(2.0 ** -(sv + sw))
         a.append(2.0 ** (nv - sv - sw))
         t.append(2.0 ** (nd - sd - sw))

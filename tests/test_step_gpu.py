@@ -288,3 +288,22 @@ def test_weights_that_are_not_finite(U, dtype, C, layer, which):
     out = mace(data)
     assert bool(out["energy"].isnan()) and bool(out["forces"].isnan().any())
     ops.check_status()
+
+
+# Layers whose values are small everywhere: silu is linear there, so factors of two layers that cancel leave the model nearly
+# as it is.  Against the same weights in float64; 1e-5 and 1e-4 are the package's float32 bounds.
+@pytest.mark.parametrize("C", [32, 128])
+@pytest.mark.parametrize("small,back", [(0, 1), (1, 2), (2, 3)])
+def test_small_hidden_values_keep_their_digits(U, C, small, back):
+    out = {}
+    for dtype in (torch.float64, torch.float32):
+        mace, data = _small(U, dtype, n=40, C=C)
+        for L in mace.layers:
+            for k, factor in ((small, 2.0**-30), (back, 2.0**30)):
+                for name in (f"W_radial{k}", f"W_radial{k}_T"):
+                    getattr(L, name).mul_(factor)
+        assert step.plan_of(mace).model.radial_half[0][0] or dtype == torch.float64
+        out[dtype] = mace(data)
+    ref, got = out[torch.float64], out[torch.float32]
+    assert abs(float(got["interaction_energy"] / ref["interaction_energy"]) - 1.0) < 1e-5
+    assert float((got["forces"] - ref["forces"]).abs().max()) < 1e-4 * float(ref["forces"].abs().max())
