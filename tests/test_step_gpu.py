@@ -307,3 +307,48 @@ def test_small_hidden_values_keep_their_digits(U, C, small, back):
     ref, got = out[torch.float64], out[torch.float32]
     assert abs(float(got["interaction_energy"] / ref["interaction_energy"]) - 1.0) < 1e-5
     assert float((got["forces"] - ref["forces"]).abs().max()) < 1e-4 * float(ref["forces"].abs().max())
+
+
+def _with_hidden_weights_times(params, factor):
+    for P in params["layers"]:
+        P["W_radial"] = [W * factor if i < 3 else W / factor**3 for i, W in enumerate(P["W_radial"])]   # R stays as large
+    return params
+
+
+def _largest_factor(C, Z, nb):
+    """Largest power of 2^(1/8) of the initial hidden weights whose bounds still fit fp16, seed 7"""
+    bounds, k = step.basis_bounds(nb, 5.0, 5), 0
+    while True:
+        params = _with_hidden_weights_times(systems.init_params(C, Z, 7, num_bessel=nb), 2.0 ** ((k + 1) / 8))
+        for P in params["layers"]:
+            Ws = [W / W.shape[0] ** 0.5 * (model.SILU_2MOM if i else 1.0) for i, W in enumerate(P["W_radial"][:3])]
+            if step.half_scales(Ws, bounds) is None:
+                return 2.0 ** (k / 8)
+        k += 1
+
+
+# float32 on both sides of the rule that gives a model the fp16 kernels: just below the largest hidden weights that fit, and
+# well beyond, where radial_pair, sums_tf32, sums_bwd_tf32 and, at 128 channels, the passes over [E, 4, C] run.  Edges around
+# the kernels' tiles of 128, odd numbers of elements; the package's bounds of 1e-5 and 1e-4 on energy and forces.
+@pytest.mark.parametrize("nb", [8, 16])
+@pytest.mark.parametrize("C,Z,edges", [(64, 3, 127), (128, 5, 128), (96, 1, 129), (128, 2, 385), (32, 7, 1), (128, 3, 5000)])
+@pytest.mark.parametrize("fits", [True, False])
+def test_hidden_weights_around_the_limit_of_fp16(U, nb, C, Z, edges, fits):
+    n = 180 if edges > 1000 else 40
+    pos, ei, sh = _cluster(n, 3, 1.0)
+    ei, sh = ei[:, :edges], sh[:edges]
+    assert ei.shape[1] == edges
+    factor = _largest_factor(C, Z, nb) * (1.0 if fits else 2.0)
+    params = _with_hidden_weights_times(systems.init_params(C, Z, 7, num_bessel=nb), factor)
+    species = torch.from_numpy(np.random.default_rng(4).integers(0, Z, n)).to(torch.int32).cuda()
+    edge_index, shifts = torch.from_numpy(ei).to(torch.int32).cuda(), torch.from_numpy(sh).cuda()
+    p = torch.from_numpy(pos).cuda().requires_grad_(True)
+    ref = model.InvariantMACE(params, U, dtype=torch.float64, device="cuda")
+    e = ref.node_energies(p, species, edge_index, shifts).sum()
+    (g,), e = torch.autograd.grad(e, p), e.detach()
+    mace = model.InvariantMACE(params, U, dtype=torch.float32, device="cuda")
+    assert bool(step.plan_of(mace).model.radial_half[0][0]) == fits
+    out = mace(dict(positions=p, species=species, edge_index=edge_index, shifts=shifts))
+    assert abs(float(out["interaction_energy"] - e)) < 1e-5 * abs(float(e))
+    assert float((out["forces"] + g).abs().max()) < 1e-4 * float(g.abs().max())
+    ops.check_status()
