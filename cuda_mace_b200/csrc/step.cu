@@ -237,8 +237,8 @@ static int run_step(const cmace_step_model &m, cmace_step_io &io, const Workspac
     case S_LINEAR: return linear_any(w.m1, m.linear[0], nullptr, 1, n, C, C, w.l1, io.status, st);
     case S_CONTRACT1:
       return K::contract_readout(w.l1, w.species, static_cast<const T *>(m.weff[1]), static_cast<const T *>(m.readout1),
-                                 m.readout2, w.q0, m.atomic_energies, io.species, Z, m.scale, m.shift, n, C, w.gX1, w.dq,
-                                 io.interaction, io.node_energy, st);
+                                 m.readout2, w.q0, m.atomic_energies, m.scale, m.shift, n, C, w.gX1, w.dq, io.interaction,
+                                 io.node_energy, st);
     case S_LINEAR_BACK: return linear_any(w.gX1, m.linear[1], nullptr, 1, n, C, C, w.gm1, io.status, st);
     case S_EDGES_BACK:
       if constexpr (!f64)
@@ -286,8 +286,8 @@ static int run_step(const cmace_step_model &m, cmace_step_io &io, const Workspac
       return K::sums_bwd(w.gA, w.h[0], w.dh[0], w.Y, io.sender, io.row_ptr, w.species, w.slot_of, w.gY1, w.dr1, w.geo, n,
                          Z, w.gvec, st);
     case S_FORCES:
-      return K::forces(w.gvec, io.row_ptr, io.perm, io.send_ptr, n, nl, io.gradient_sign, io.gradient, io.interaction,
-                       io.node_energy, io.status, f64 ? nullptr : staged_stall_flag(), io.sums, st);
+      return K::forces(w.gvec, io.row_ptr, io.perm, io.send_ptr, n, nl, io.gradient_sign, io.gradient, io.species, Z,
+                       io.interaction, io.node_energy, io.status, f64 ? nullptr : staged_stall_flag(), io.sums, st);
   }
   return fail(CMACE_ERR_ARG, "cmace_step: no step %d", step);
 }

@@ -83,9 +83,8 @@ struct StepKernels {
   static int contract_bwd(const T *X, const int32_t *types, const T *weff, const T *gb, int64_t n, int C, T *gX,
                           cudaStream_t st);
   static int contract_readout(const T *X, const int32_t *types, const T *weff, const T *wp1, const double *w2,
-                              const T *q0, const double *atomic_e, const int32_t *species_in, int elements, double scale,
-                              double shift, int64_t n, int C, T *gX, T *dq, double *inter, double *node_energy,
-                              cudaStream_t st);
+                              const T *q0, const double *atomic_e, double scale, double shift, int64_t n, int C, T *gX,
+                              T *dq, double *inter, double *node_energy, cudaStream_t st);
   static int mid_fwd(const T *b, const int32_t *node_of, const int32_t *slot_type, const T *wu, const T *extra,
                      int64_t n, int C, T *up, T *q0, cudaStream_t st);
   static int mid_bwd(const T *gup, const int32_t *node_of, const int32_t *slot_type, const T *dq, const T *wu_t,
@@ -94,8 +93,8 @@ struct StepKernels {
                       const int32_t *species, const int32_t *slot_of, const T *gY1, const T *dr1, const Quad<T> *geo,
                       int64_t nnodes, int elements, T *gvec, cudaStream_t st);
   static int forces(const T *gvec, const int32_t *row_ptr, const int32_t *perm, const int32_t *send_ptr, int64_t nrecv,
-                    int64_t nsend, double sign, double *out, const double *inter, const double *node_energy,
-                    const int32_t *status, const int *stalled, double *sums, cudaStream_t st);
+                    int64_t nsend, double sign, double *out, const int32_t *species_in, int elements, double *inter,
+                    double *node_energy, const int32_t *status, const int *stalled, double *sums, cudaStream_t st);
 };
 
 }  // namespace cmace

@@ -55,7 +55,7 @@ __device__ void resolve_nodes(const int32_t *__restrict__ species_in, const void
     const int64_t i = lo + u * EP_THREADS + threadIdx.x;
     if (i >= hi) continue;
     const bool known = z[u] >= 0 && z[u] < elements;
-    species[i] = known ? z[u] : 0;   // the tables are read with it; the readout gives such a node no energy
+    species[i] = known ? z[u] : 0;   // the tables are read with it; forces_kernel takes such a node's energy away
     if (!known && status) *status = CMACE_STEP_BAD_ELEMENT;
   }
   __syncthreads();
@@ -1021,13 +1021,17 @@ template <typename T>
 __global__ void __launch_bounds__(256)
     forces_kernel(const T *__restrict__ g, const int32_t *__restrict__ row_ptr, const int32_t *__restrict__ perm,
                   const int32_t *__restrict__ send_ptr, int64_t nrecv, int64_t nsend, double sign,
-                  double *__restrict__ out, const double *__restrict__ inter, const double *__restrict__ node_energy,
-                  const int32_t *status, const int *stalled, double *__restrict__ sums) {
+                  double *__restrict__ out, const int32_t *__restrict__ species_in, int elements,
+                  double *__restrict__ inter, double *__restrict__ node_energy, const int32_t *status, const int *stalled,
+                  double *__restrict__ sums) {
   grid_begin();
   const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
   if (blockIdx.x == 0) {
     __shared__ double part[2][8];
     double a = 0.0, b = 0.0;
+    if (species_in && status && *status != 0)   // this call's edge_prep, or one before it, met an index that does not exist
+      for (int64_t i = threadIdx.x; i < nrecv; i += 256)
+        if (species_in[i] < 0 || species_in[i] >= elements) inter[i] = node_energy[i] = CUDART_NAN;
 #pragma unroll 8   // one block: the loads in flight bound it
     for (int64_t i = threadIdx.x; i < nrecv; i += 256) {
       a += node_energy[i];
@@ -1091,12 +1095,12 @@ __global__ void __launch_bounds__(256)
 
 template <typename T>
 int StepKernels<T>::forces(const T *gvec, const int32_t *row_ptr, const int32_t *perm, const int32_t *send_ptr,
-                           int64_t nrecv, int64_t nsend, double sign, double *out, const double *inter,
-                           const double *node_energy, const int32_t *status, const int *stalled, double *sums,
-                           cudaStream_t st) {
+                           int64_t nrecv, int64_t nsend, double sign, double *out, const int32_t *species_in,
+                           int elements, double *inter, double *node_energy, const int32_t *status, const int *stalled,
+                           double *sums, cudaStream_t st) {
   const int64_t blocks = 1 + (nsend + 7) / 8;
-  launch_chained(forces_kernel<T>, (unsigned)blocks, 256, 0, st, gvec, row_ptr, perm, send_ptr, nrecv, nsend, sign, out, inter,
-                                                     node_energy, status, stalled, sums);
+  launch_chained(forces_kernel<T>, (unsigned)blocks, 256, 0, st, gvec, row_ptr, perm, send_ptr, nrecv, nsend, sign, out,
+                 species_in, elements, inter, node_energy, status, stalled, sums);
   return check_launch("cmace_step(forces)");
 }
 
@@ -1113,7 +1117,7 @@ int StepKernels<T>::forces(const T *gvec, const int32_t *row_ptr, const int32_t 
                                         const int32_t *, const int32_t *, const int32_t *, const T *, const T *,    \
                                         const Quad<T> *, int64_t, int, T *, cudaStream_t);                          \
   template int StepKernels<T>::forces(const T *, const int32_t *, const int32_t *, const int32_t *, int64_t,        \
-                                      int64_t, double, double *, const double *, const double *,                    \
+                                      int64_t, double, double *, const int32_t *, int, double *, double *,          \
                                       const int32_t *, const int *, double *, cudaStream_t);
 CMACE_STEP_EDGES(float)
 CMACE_STEP_EDGES(double)

@@ -85,8 +85,7 @@ template <typename T>
 __global__ void __launch_bounds__(128, sizeof(T) == 4 ? 5 : 3)
     contract_readout_kernel(const T *__restrict__ X, const int32_t *__restrict__ types, const T *__restrict__ weff,
                             const T *__restrict__ wp1, const double *__restrict__ w2ro, const T *__restrict__ q0,
-                            const double *__restrict__ atomic_e, const int32_t *__restrict__ species_in, int elements,
-                            double scale, double shift, int64_t nnodes, int C,
+                            const double *__restrict__ atomic_e, double scale, double shift, int64_t nnodes, int C,
                             T *__restrict__ gX, T *__restrict__ dq_out, double *__restrict__ inter,
                             double *__restrict__ node_energy) {
   grid_begin();
@@ -104,12 +103,8 @@ __global__ void __launch_bounds__(128, sizeof(T) == 4 ? 5 : 3)
     const int z = types[node];
     load_weff(weff, z, C, c, w3, w2, w1);
     double qd = 0.0, e0 = 0.0;
-    bool known = true;
     if (c < ST_RO) qd = (double)q0[node * (ST_RO + 1) + c];
-    if (c == 0) {
-      e0 = (double)q0[node * (ST_RO + 1) + ST_RO];
-      if (species_in) known = species_in[node] >= 0 && species_in[node] < elements;
-    }
+    if (c == 0) e0 = (double)q0[node * (ST_RO + 1) + ST_RO];
     canon::eval<T>(x, w3, w2, w1, g, value);
     T p[ST_RO];
 #pragma unroll
@@ -147,7 +142,7 @@ __global__ void __launch_bounds__(128, sizeof(T) == 4 ? 5 : 3)
 #pragma unroll
       for (int off = 8; off > 0; off >>= 1) e1 += __shfl_xor_sync(0xffffffffu, e1, off);
       if (c == 0) {
-        const double v = known ? scale * (e0 + e1) + shift : CUDART_NAN;
+        const double v = scale * (e0 + e1) + shift;
         inter[node] = v;
         node_energy[node] = atomic_e[z] + v;
       }
@@ -164,12 +159,11 @@ __global__ void __launch_bounds__(128, sizeof(T) == 4 ? 5 : 3)
 
 template <typename T>
 int StepKernels<T>::contract_readout(const T *X, const int32_t *types, const T *weff, const T *wp1, const double *w2,
-                                     const T *q0, const double *atomic_e, const int32_t *species_in, int elements,
-                                     double scale, double shift, int64_t n, int C, T *gX, T *dq, double *inter,
-                                     double *node_energy, cudaStream_t st) {
+                                     const T *q0, const double *atomic_e, double scale, double shift, int64_t n, int C,
+                                     T *gX, T *dq, double *inter, double *node_energy, cudaStream_t st) {
   if (n > 0)
-    launch_chained(contract_readout_kernel<T>, (unsigned)node_blocks(n, 10), C, 0, st, X, types, weff, wp1, w2, q0, atomic_e,
-                   species_in, elements, scale, shift, n, C, gX, dq, inter, node_energy);
+    launch_chained(contract_readout_kernel<T>, (unsigned)node_blocks(n, 10), C, 0, st, X, types, weff, wp1, w2, q0, atomic_e, scale,
+                                                                          shift, n, C, gX, dq, inter, node_energy);
   return check_launch("cmace_step(contract_readout)");
 }
 
@@ -432,8 +426,8 @@ int StepKernels<T>::mid_bwd(const T *gup, const int32_t *node_of, const int32_t 
   template int StepKernels<T>::contract_bwd(const T *, const int32_t *, const T *, const T *, int64_t, int, T *,     \
                                             cudaStream_t);                                                           \
   template int StepKernels<T>::contract_readout(const T *, const int32_t *, const T *, const T *, const double *,    \
-                                                const T *, const double *, const int32_t *, int, double, double,     \
-                                                int64_t, int, T *, T *, double *, double *, cudaStream_t);           \
+                                                const T *, const double *, double, double, int64_t, int, T *, T *,   \
+                                                double *, double *, cudaStream_t);                                   \
   template int StepKernels<T>::mid_fwd(const T *, const int32_t *, const int32_t *, const T *, const T *, int64_t,   \
                                        int, T *, T *, cudaStream_t);                                                 \
   template int StepKernels<T>::mid_bwd(const T *, const int32_t *, const int32_t *, const T *, const T *, const T *, \
