@@ -325,11 +325,11 @@ __device__ __forceinline__ void store32(double *p, double a, double b, double c,
   asm volatile("st.global.v4.f64 [%0], {%1, %2, %3, %4};" ::"l"(p), "d"(a), "d"(b), "d"(c), "d"(d) : "memory");
 }
 
-// and in one load
+// and in one load; volatile, like the wait for the kernel before that wrote these rows, so that it stays behind it
 __device__ __forceinline__ void load32(const float *p, float4 &a, float4 &b) {
-  asm("ld.global.nc.v8.f32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];"
-      : "=f"(a.x), "=f"(a.y), "=f"(a.z), "=f"(a.w), "=f"(b.x), "=f"(b.y), "=f"(b.z), "=f"(b.w)
-      : "l"(p));
+  asm volatile("ld.global.nc.v8.f32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];"
+               : "=f"(a.x), "=f"(a.y), "=f"(a.z), "=f"(a.w), "=f"(b.x), "=f"(b.y), "=f"(b.z), "=f"(b.w)
+               : "l"(p));
 }
 __device__ __forceinline__ void load_row16(const float *p, float (&v)[16]) {
 #pragma unroll
@@ -343,9 +343,9 @@ __device__ __forceinline__ void load_row16(const float *p, float (&v)[16]) {
 __device__ __forceinline__ void load_row16(const double *p, double (&v)[16]) {
 #pragma unroll
   for (int i = 0; i < 4; i++)
-    asm("ld.global.nc.v4.f64 {%0, %1, %2, %3}, [%4];"
-        : "=d"(v[4 * i]), "=d"(v[4 * i + 1]), "=d"(v[4 * i + 2]), "=d"(v[4 * i + 3])
-        : "l"(p + 4 * i));
+    asm volatile("ld.global.nc.v4.f64 {%0, %1, %2, %3}, [%4];"
+                 : "=d"(v[4 * i]), "=d"(v[4 * i + 1]), "=d"(v[4 * i + 2]), "=d"(v[4 * i + 3])
+                 : "l"(p + 4 * i));
 }
 __device__ __forceinline__ void prefetch_l1(const void *p) { asm volatile("prefetch.global.L1 [%0];" ::"l"(p)); }
 __device__ __forceinline__ void store_quad(float *p, float a, float b, float c) {
