@@ -312,12 +312,11 @@ static int run_steps(const cmace_step_model &m, cmace_step_io &io, int first, in
   const Workspace<T> w(io.workspace, m, io.n_owned, io.n_local, io.nedges);
   if (io.workspace_bytes < w.bytes)
     return fail(CMACE_ERR_ARG, "cmace_step: workspace of %lld bytes, %lld needed", (long long)io.workspace_bytes, (long long)w.bytes);
-  const bool chain = chain_for(m, io.nedges, st);
+  // The first kernel of a range as well: the attribute relaxes the order after the kernel before it and nothing else, so a
+  // wait for another stream or a copy that the caller has put between still comes first.
+  chain_launches() = chain_for(m, io.nedges, st);
   int rc = CMACE_OK;
-  for (int s = first; s < last && rc == CMACE_OK; s++) {
-    chain_launches() = chain && (s > first || first == 0);   // a later range may follow the caller's wait for another stream
-    rc = run_step<T>(m, io, w, s, st);
-  }
+  for (int s = first; s < last && rc == CMACE_OK; s++) rc = run_step<T>(m, io, w, s, st);
   chain_launches() = false;
   return rc;
 }

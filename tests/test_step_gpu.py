@@ -352,3 +352,56 @@ def test_hidden_weights_around_the_limit_of_fp16(U, nb, C, Z, edges, fits):
     assert abs(float(out["interaction_energy"] - e)) < 1e-5 * abs(float(e))
     assert float((out["forces"] + g).abs().max()) < 1e-4 * float(g.abs().max())
     ops.check_status()
+
+
+def _periodic(U, n, dtype, C=64):
+    side = (n / 0.1) ** (1.0 / 3.0)
+    pos, species = systems.random_box(n, np.full(3, side), 0.9, 5), np.zeros(n, dtype=np.int64)
+    dom = domain.partition_slabs(pos, species, np.full(3, side), 1, 5.0, 0)
+    mace = model.InvariantMACE(systems.init_params(C, 1, 7), U, dtype=dtype, device="cuda")
+    ev = evaluator.EnergyForceEvaluator(mace, dom, "cuda")
+    return ev, ev.load_domain()
+
+
+# Programmatic launches overlap the kernel before them, not what the stream waits for: positions that another stream writes
+# late, and a grouping by sender that is late, both before the first kernel of a range.  (All buffers hold valid values before.)
+def test_a_wait_between_launches_is_kept(U, monkeypatch):
+    ev, p = _periodic(U, 300, torch.float32)
+    moved = p + 0.01
+    moved[0] += 0.2
+    old, want = ev(p)[1].clone(), ev(moved)[1].clone()
+    assert not torch.equal(old, want)
+    other = torch.cuda.Stream()
+    buffer = p.clone()
+    for _ in range(5):
+        buffer.copy_(p)
+        other.wait_stream(torch.cuda.current_stream())
+        ev(buffer)                                    # its last kernel lets the next one come early
+        with torch.cuda.stream(other):
+            torch.cuda._sleep(2_000_000)
+            buffer.copy_(moved, non_blocking=True)
+            written = other.record_event()
+        torch.cuda.current_stream().wait_event(written)
+        assert torch.equal(ev(buffer)[1], want)
+
+
+def test_a_late_grouping_is_waited_for(U, monkeypatch):
+    ev, p = _periodic(U, 1100, torch.float32)
+    assert step._BESIDE_EDGES <= ev.topology.nedges <= 98304   # beside the step, launches chained
+    ev.topology.sender_order()
+    want = ev(p)[1].clone()
+    buffers, group = ops.EdgeTopology.grouping_buffers, ops.EdgeTopology.group_senders
+
+    def zeros(self):
+        return tuple(t.zero_() for t in buffers(self))
+
+    def late(self, b, stream):
+        with torch.cuda.stream(torch.cuda.ExternalStream(stream)):
+            torch.cuda._sleep(2_000_000)
+        group(self, b, stream)
+
+    monkeypatch.setattr(ops.EdgeTopology, "grouping_buffers", zeros)
+    monkeypatch.setattr(ops.EdgeTopology, "group_senders", late)
+    for _ in range(5):
+        ev.set_neighbor_list(ev.species, ev.edge_index, ev.shifts)
+        assert torch.equal(ev(p)[1], want)
