@@ -118,7 +118,7 @@ class EnergyForceEvaluator:
     def __call__(self, positions_owned):
         if self._graph is not None and not torch.cuda.is_current_stream_capturing():
             graph, static_pos, energy, forces, (plan, *_) = self._graph
-            if plan is None or plan.current():
+            if plan is None or plan.current(self.model):
                 static_pos.copy_(positions_owned)
                 graph.replay()
                 return energy.clone(), forces.clone()

@@ -119,21 +119,24 @@ _UNREAD = ("U1_", "U2_", "U3_", "weights_transposed")
 
 class _Stamp:
     """What a plan was made from: the tensors, submodules and plain attributes of a model, by identity, version or value.
-    (Edits that autograd's version counter does not see, such as those through ``.data``, are not seen here either.)"""
+    (Edits that autograd's version counter does not see, such as those through ``.data``, are not seen here either.)
+    It holds the parts, not the model, which holds it: no cycle that would keep a model's memory until it is collected."""
 
     def __init__(self, model):
         modules = list(model.modules())
         self.tensors = [(d, k, t, t._version) for m in modules for d in (m._buffers, m._parameters)
                         for k, t in d.items() if t is not None and not k.endswith("_T") and not k.startswith(_UNREAD)]
         self.children = [(m._modules, tuple(m._modules.values())) for m in modules]
-        self.plain = [(m.__dict__, k, v) for m in modules for k, v in m.__dict__.items()
-                      if k[0] != "_" and k != "training" and isinstance(v, (bool, int, float, str, torch.dtype))]
+        plain = [(m.__dict__, k, v) for m in modules for k, v in m.__dict__.items()
+                 if k[0] != "_" and k != "training" and isinstance(v, (bool, int, float, str, torch.dtype))]
+        self.plain = [p for p in plain if p[0] is not model.__dict__]
+        self.own = [p[1:] for p in plain if p[0] is model.__dict__]
         # hooks of the parts would not run: the model's own run around forward()
         self.hooks = [h for m in modules[1:] for h in (m._forward_hooks, m._forward_pre_hooks, m._backward_hooks,
                                                        m._backward_pre_hooks)]
         self.hooked = any(self.hooks)
 
-    def current(self):
+    def current(self, model):
         for d, k, t, v in self.tensors:
             if d.get(k) is not t or t._version != v:
                 return False
@@ -141,6 +144,10 @@ class _Stamp:
             if tuple(d.values()) != v:
                 return False
         for d, k, v in self.plain:
+            if d.get(k) != v:
+                return False
+        d = model.__dict__
+        for k, v in self.own:
             if d.get(k) != v:
                 return False
         return any(self.hooks) == self.hooked
@@ -298,8 +305,8 @@ class StepPlan:
         for b in range(first, (Z + 1) // 2):
             m.fold_back[b] = matrix(blocks[b])
 
-    def current(self):
-        return self.stamp.current()
+    def current(self, model):
+        return self.stamp.current(model)
 
 
 def plan_of(model):
@@ -314,7 +321,7 @@ def plan_of(model):
     if os.environ.get("CMACE_SYMCON_GENERIC", "")[:1] == "1":
         return None
     stamp, plan = model.__dict__.get("_step_plan", (None, None))
-    if stamp is not None and stamp.current():
+    if stamp is not None and stamp.current(model):
         return plan
     dev = model.embedding.device
     if dev.type != "cuda" or dev.index != torch.cuda.current_device():

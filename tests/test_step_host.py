@@ -1,4 +1,7 @@
 """Host-side rules of the whole-step sequence: which models it covers, before any kernel is launched."""
+import gc
+import weakref
+
 import pytest
 import torch
 
@@ -43,9 +46,9 @@ def test_what_a_plan_is_made_from(U, radial):
     for change in changes:
         mace = _model(U, radial=radial)
         stamp = step._Stamp(mace)
-        assert stamp.current() and not stamp.hooked
+        assert stamp.current(mace) and not stamp.hooked
         change(mace)
-        assert not stamp.current()
+        assert not stamp.current(mace)
     mace = _model(U)     # a weight that became a parameter is followed like a buffer
     W = mace.layers[1].W_readout2
     del mace.layers[1].W_readout2
@@ -53,7 +56,20 @@ def test_what_a_plan_is_made_from(U, radial):
     stamp = step._Stamp(mace)
     with torch.no_grad():
         W.mul_(2.0)
-    assert not stamp.current()
+    assert not stamp.current(mace)
+
+
+def test_a_stamp_does_not_keep_its_model(U):
+    mace = _model(U)
+    mace.__dict__["_step_plan"] = (step._Stamp(mace), None)
+    gone = weakref.ref(mace)
+    gc.collect()
+    gc.disable()
+    try:
+        del mace
+        assert gone() is None
+    finally:
+        gc.enable()
 
 
 def test_a_model_with_parts_of_its_own_is_not_covered(U):
