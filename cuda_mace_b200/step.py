@@ -402,7 +402,9 @@ def energy_forces(plan, positions, species, one_hot, shifts, topology, halo=None
                            f"{nl} atoms and {E} edges")
     capturing = torch.cuda.is_current_stream_capturing()
     plan.recorded = plan.recorded or capturing
-    out = torch.empty(3 + 2 * n + 3 * nl, dtype=torch.float64, device=dev)
+    # results of their own: a program that keeps an energy or saves the forces does not keep the rest with them
+    new = dict(dtype=torch.float64, device=dev)
+    sums, interaction, node_energy, forces = (torch.empty(k, **new) for k in (3, n, n, (nl, 3)))
     m = plan.model
     nbytes = _abi.call("cmace_step_workspace_bytes", ctypes.byref(m), n, nl, E)
     workspace = torch.empty(nbytes, dtype=torch.uint8, device=dev)
@@ -417,7 +419,6 @@ def energy_forces(plan, positions, species, one_hot, shifts, topology, halo=None
         ready = torch.cuda.current_stream(dev).record_event()
     else:
         perm, send_ptr = topology.sender_order()
-    p = out.data_ptr()
     io = _abi.StepIO()
     io.n_owned, io.n_local, io.nedges = n, nl, E
     io.positions = positions.data_ptr()
@@ -433,10 +434,9 @@ def energy_forces(plan, positions, species, one_hot, shifts, topology, halo=None
     io.perm, io.send_ptr = perm.data_ptr(), send_ptr.data_ptr()
     io.workspace, io.workspace_bytes = workspace.data_ptr(), nbytes
     io.status = ops._status_tensor(dev).data_ptr()
-    io.sums, io.interaction, io.node_energy, io.gradient = p, p + 24, p + 24 + 8 * n, p + 24 + 16 * n
+    io.sums, io.interaction, io.node_energy, io.gradient = [t.data_ptr() for t in (sums, interaction, node_energy, forces)]
     io.gradient_sign = -1.0
     st = ops._stream()
-    forces = out[3 + 2 * n:].view(nl, 3)
 
     def run(first, last):
         nonlocal ready
@@ -465,7 +465,7 @@ def energy_forces(plan, positions, species, one_hot, shifts, topology, halo=None
     finally:
         if beside is not None:   # a failed step: the grouping still owns its memory
             join()
-    return out[:3], out[3:3 + n], out[3 + n:3 + 2 * n], forces
+    return sums, interaction, node_energy, forces
 
 
 def _run_ranges(run, plan, n, nl, io, halo, forces):

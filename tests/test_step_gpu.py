@@ -405,3 +405,15 @@ def test_a_late_grouping_is_waited_for(U, monkeypatch):
     for _ in range(5):
         ev.set_neighbor_list(ev.species, ev.edge_index, ev.shifts)
         assert torch.equal(ev(p)[1], want)
+
+
+def test_results_do_not_share_memory(U):
+    """An energy that is kept keeps three values, the forces their own rows."""
+    mace, data = _small(U)
+    out = mace(data)
+    size = {k: t.untyped_storage().nbytes() for k, t in out.items()}
+    assert size["energy"] <= 24 and size["interaction_energy"] <= 24
+    assert size["node_energy"] == 12 * 8 and size["forces"] == 12 * 3 * 8
+    ev, p = _periodic(U, 300, torch.float32)
+    energy, forces = ev(p)
+    assert energy.untyped_storage().nbytes() <= 24 and forces.untyped_storage().nbytes() == 300 * 3 * 8
