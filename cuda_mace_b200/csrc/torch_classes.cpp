@@ -22,6 +22,7 @@
 
 #include <map>
 #include <mutex>
+#include <optional>
 #include <tuple>
 #include <vector>
 
@@ -109,11 +110,37 @@ void add_sender_order(Topology &t, cmace_stream_t stream) {
   Tensor ws = torch::empty({std::max<int64_t>(nbytes, 1)}, t.sender.options().dtype(torch::kUInt8));
   t.perm = torch::empty({std::max<int64_t>(t.nedges, 1)}, t.sender.options());
   t.send_ptr = torch::empty({t.nsenders + 1}, t.sender.options());
+  t.workspace = ws;
   check(cmace_sender_order(t.sender.data_ptr<int32_t>(), t.nedges, t.nsenders, t.perm.data_ptr<int32_t>(),
                            t.send_ptr.data_ptr<int32_t>(), ws.data_ptr(), nbytes, stream),
         "cmace_sender_order");
-  t.workspace = ws;
 }
+
+// Work on a second stream that the main one has to wait for before what it uses is free again, also when a check between
+// throws: declared after the memory, so that it goes first.
+struct Beside {
+  c10::cuda::CUDAStream main, side;
+  bool open = true;
+  explicit Beside(c10::cuda::CUDAStream stream)
+      : main(stream), side(c10::cuda::getStreamFromPool(false, stream.device_index())) {
+    at::cuda::CUDAEvent ready;
+    ready.record(main);
+    ready.block(side);
+  }
+  void join() {
+    open = false;
+    at::cuda::CUDAEvent done;
+    done.record(side);
+    done.block(main);
+  }
+  ~Beside() {
+    if (!open) return;
+    try {
+      join();
+    } catch (...) {
+    }
+  }
+};
 
 // ---- invariant message passing ------------------------------------------------------------------------
 class IMPAutograd : public torch::autograd::Function<IMPAutograd> {
@@ -170,15 +197,10 @@ class IMPAutograd : public torch::autograd::Function<IMPAutograd> {
     // and leaves most of the GPU idle: beside it on a stream of its own once the list is long enough to be worth two
     // events.  The node pass waits for it, so everything it used is free again on this stream after that.
     const auto main_stream = c10::cuda::getCurrentCUDAStream(X.device().index());
-    at::cuda::CUDAEvent sorted;
-    const bool beside = E >= 32768;
-    if (beside) {
-      const auto side = c10::cuda::getStreamFromPool(false, X.device().index());
-      at::cuda::CUDAEvent ready;
-      ready.record(main_stream);
-      ready.block(side);
-      add_sender_order(topo, (cmace_stream_t)side.stream());
-      sorted.record(side);
+    std::optional<Beside> beside;
+    if (E >= 32768) {
+      beside.emplace(main_stream);
+      add_sender_order(topo, (cmace_stream_t)beside->side.stream());
     } else {
       add_sender_order(topo, stream_of(X));
     }
@@ -189,7 +211,7 @@ class IMPAutograd : public torch::autograd::Function<IMPAutograd> {
                                    gradY.data_ptr<double>(), T.data_ptr<double>(),
                                    nscratch > 0 ? scratch.data_ptr<double>() : nullptr, stream_of(X)),
             "cmace_imp_bwd_edge_f64");
-      if (beside) sorted.block(main_stream);
+      if (beside) beside->join();
       check(cmace_imp_bwd_node_f64(T.data_ptr<double>(), topo.perm.data_ptr<int32_t>(),
                                    topo.send_ptr.data_ptr<int32_t>(), topo.nsenders, (int)C, gradX.data_ptr<double>(),
                                    stream_of(X)),
@@ -201,7 +223,7 @@ class IMPAutograd : public torch::autograd::Function<IMPAutograd> {
                                    gradY.data_ptr<float>(), T.data_ptr<float>(),
                                    nscratch > 0 ? scratch.data_ptr<float>() : nullptr, stream_of(X)),
             "cmace_imp_bwd_edge_f32");
-      if (beside) sorted.block(main_stream);
+      if (beside) beside->join();
       check(cmace_imp_bwd_node_f32(T.data_ptr<float>(), topo.perm.data_ptr<int32_t>(),
                                    topo.send_ptr.data_ptr<int32_t>(), topo.nsenders, (int)C, gradX.data_ptr<float>(),
                                    stream_of(X)),

@@ -95,6 +95,26 @@ def test_linear_classes(classes, dtype):
 
 
 @pytest.mark.gpu
+def test_a_refused_gradient_leaves_the_second_stream_joined(classes):
+    """From 32 768 edges the backward groups the edges beside its edge pass.  A gradient that the edge pass refuses (not on a
+    16-byte boundary; checked on the host) throws between the two; the memory is used again at once."""
+    g = torch.Generator("cuda").manual_seed(3)
+    N, C, E = 600, 64, 40000
+    receiver = torch.randint(0, N, (E,), generator=g, device="cuda", dtype=torch.int32).sort()[0]
+    sender = torch.randint(0, N, (E,), generator=g, device="cuda", dtype=torch.int32)
+    X, Y, R, G = (torch.randn(*s, generator=g, device="cuda").requires_grad_(k < 3)
+                  for k, s in enumerate(((N, C), (16, E), (E, 4, C), (N, 16, C))))
+    op = classes.inv_message_passing.InvariantMessagePassingTP()
+    want = torch.autograd.grad(op.forward(X, Y, R, sender, receiver, N), (X, Y, R), G)
+    odd = torch.empty(G.numel() + 1, device="cuda")[1:].view(G.shape).copy_(G)
+    for _ in range(3):
+        with pytest.raises(RuntimeError, match="aligned"):
+            torch.autograd.grad(op.forward(X, Y, R, sender, receiver, N), (X, Y, R), odd)
+        got = torch.autograd.grad(op.forward(X, Y, R, sender, receiver, N), (X, Y, R), G)
+        assert all(torch.equal(a, b) for a, b in zip(got, want))
+
+
+@pytest.mark.gpu
 def test_contraction_reads_its_weights_in_every_call(classes, U):
     """The weights are inputs: edits that no version counter sees count, tensors without one are taken, each of them has to
     have X's type."""
