@@ -14,6 +14,7 @@
 // values' products of the next layer run while the derivatives' elementwise phase does, and the groups overlap each
 // other.  Tensor memory holds per group 64 accumulator + 64 residual columns for each operand: all 512.
 #include "common.cuh"
+#include "sigmoid64.cuh"
 #include "step_common.cuh"
 #include "tc_ptx.cuh"
 
@@ -284,34 +285,6 @@ __global__ void __launch_bounds__(RT_THREADS, 1)
 // Row strides of 68 doubles make the fragment loads of both operands conflict-free.
 constexpr int RD_WARPS = 16, RD_LD = 68;
 
-// 1 / (1 + e^-z).  The elementwise phase has as many FP64 operations as the products if the library's exp and divide are
-// used (the kernel took 1.26 ms at 8 000 atoms, 0.78 of them the products' own time), so: e^x by Tang's table-driven
-// method (ACM TOMS 15, 1989): x = (32 m + j) ln2 / 32 + r with |r| <= ln2 / 64, e^x = 2^m 2^(j/32) (1 + p(r)); the
-// remainder of the exponential series after r^6 is below 4e-18.  The reciprocal starts from the hardware's 20-bit
-// approximation and one step of third order, 1/d = y (1 + e + e^2), e = 1 - d y: e^3 < 2^-57.
-// |z| beyond 700 saturates the exponent (the result is 0 or 1 to 300 digits).
-__device__ __forceinline__ double rd_sigmoid(double z, const double *etab) {
-  const double x = fmin(fmax(-z, -700.0), 700.0);
-  const double kd = __fma_rn(x, 46.16624130844683, 6755399441055744.0);   // 32 / ln 2; 1.5 * 2^52 rounds to an integer
-  const int k = __double2loint(kd);
-  const double n = kd - 6755399441055744.0;
-  double r = __fma_rn(n, -0.021660849391992087, x);                           // ln2 / 32 in two parts, the first 35 bits long
-  r = __fma_rn(n, -5.062034433330175e-13, r);
-  double p = __fma_rn(r, 1.0 / 720.0, 1.0 / 120.0);
-  p = __fma_rn(p, r, 1.0 / 24.0);
-  p = __fma_rn(p, r, 1.0 / 6.0);
-  p = __fma_rn(p, r, 0.5);
-  p = __fma_rn(p, r * r, r);
-  const double t = etab[k & 31];
-  const double e0 = __fma_rn(t, p, t);
-  const double e = __hiloint2double(__double2hiint(e0) + ((k >> 5) << 20), __double2loint(e0));
-  const double d = 1.0 + e;
-  double y;
-  asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(d));
-  const double c = __fma_rn(-d, y, 1.0);
-  return __fma_rn(y, __fma_rn(c, c, c), y);
-}
-
 struct RadialPairArgs64 {
   const double *basis;
   const double *w[2][3];   // [nb, 64], [64, 64], [64, 64]
@@ -371,7 +344,7 @@ __global__ void __launch_bounds__(RD_WARPS * 32, 1) radial_pair_f64_kernel(const
         double a[2], da[2];
 #pragma unroll
         for (int u = 0; u < 2; u++) {
-          const double z = acc[0][n][u], s = rd_sigmoid(z, etab);
+          const double z = acc[0][n][u], s = table_sigmoid(z, etab);
           a[u] = z * s;
           da[u] = s * (1.0 + z * (1.0 - s)) * acc[1][n][u];
         }

@@ -3,11 +3,17 @@
 // device entry points (xyz [E,3], Y [16,E], B [E,nb]).
 #include <cstdint>
 
+#include "sigmoid64.cuh"
 #include "edge_math.cuh"   // found through -I cuda_mace_b200/csrc (tests/conftest.py builds this file)
 
 using namespace cmace;
 
 extern "C" {
+void hc_sigmoid_f64(const double *z, int64_t n, double *s) {
+  double etab[32];
+  for (int j = 0; j < 32; j++) etab[j] = std::exp2(j / 32.0);
+  for (int64_t i = 0; i < n; i++) s[i] = table_sigmoid(z[i], etab);
+}
 void hc_edge_basis_fwd_f64(const double *xyz, int64_t E, double r_max, int nb, int p, double *Y, double *B) {
   for (int64_t e = 0; e < E; e++) {
     double y[16], b[16];

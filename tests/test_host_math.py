@@ -27,6 +27,25 @@ def edges(seed, n):
     return v * rng.uniform(0.6, 5.4, size=(n, 1))  # a few beyond the 5.0 cutoff
 
 
+def test_table_sigmoid_f64(hc):
+    """The float64 logistic function of the radial kernel against long double: every interval of its table, both ends of
+    the exponent's range, zero, and values beyond.  Bound: half an ulp of 1 + e and of the result each, the exponential's
+    own 2 ulp where it dominates: 2^-53 (1 + 1 + 2) = 4.5e-16."""
+    rng = np.random.default_rng(5)
+    edges_of_table = (np.arange(-2000, 2001) + 0.5) * np.log(2.0) / 32
+    z = np.concatenate([rng.uniform(-40, 40, 200000), rng.uniform(-700, 700, 50000), rng.normal(size=50000) * 1e-3,
+                        edges_of_table, np.nextafter(edges_of_table, 100.0), [0.0, -0.0, 700.0, -700.0]])
+    s = np.zeros_like(z)
+    hc.hc_sigmoid_f64(P(z), ctypes.c_int64(z.size), P(s))
+    zl = z.astype(np.longdouble)
+    ref = 1.0 / (1.0 + np.exp(-zl))
+    assert float(np.abs((s - ref) / ref).max()) < 4.5e-16
+    beyond = np.array([1e4, np.inf, -1e4, -np.inf])
+    s = np.zeros(4)
+    hc.hc_sigmoid_f64(P(beyond), ctypes.c_int64(4), P(s))
+    assert s[0] == s[1] == 1.0 and 0.0 <= s[2] < 1e-300 and 0.0 <= s[3] < 1e-300
+
+
 def test_edge_basis_forward_f64(hc):
     xyz = edges(0, 1500)
     E = xyz.shape[0]
