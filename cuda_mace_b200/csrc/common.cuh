@@ -31,10 +31,8 @@ inline int check_launch(const char *what) {
 }
 
 // strides of an array of 16 values per edge, over components and over edges: {E, 1} for [16, E], {1, 16} for [E, 16]
-// rows: where a receiver's row stands in the messages and in their gradient, or null for receiver order
 struct ImpLayout {
   int64_t m, e;
-  const int32_t *rows = nullptr;
 };
 
 // operator launchers that other translation units call with their own layout of Y

@@ -86,7 +86,7 @@ __global__ void __launch_bounds__(SPLIT == 1 ? kWarpsPerBlock * 32 : SPLIT * 32,
 #pragma unroll
       for (int v = 0; v < VEC; v++) acc[m][v] = fma(y[m], rb[l_of_lm(m)][v], acc[m][v]);
   }
-  T *o = out + (ys.rows ? (int64_t)ys.rows[node] : node) * 16 * C + c0;
+  T *o = out + node * 16 * C + c0;
   if constexpr (SPLIT > 1) {
     extern __shared__ __align__(16) unsigned char imp_smem[];
     T *part = reinterpret_cast<T *>(imp_smem);   // [SPLIT][16][32 VEC]
@@ -128,10 +128,9 @@ __global__ void __launch_bounds__(kWarpsPerBlock * 32)
   // with several channel chunks each chunk writes its own [16, E] partial of gradY
   T *gy = gradY_out + (int64_t)blockIdx.y * 16 * nedges;
 
-  const int64_t grow = ys.rows ? (int64_t)ys.rows[node] : node;
   T g[16][VEC];
 #pragma unroll
-  for (int m = 0; m < 16; m++) load_vec<T, VEC>(g[m], G + (grow * 16 + m) * C + c0);
+  for (int m = 0; m < 16; m++) load_vec<T, VEC>(g[m], G + (node * 16 + m) * C + c0);
 
   __shared__ __align__(16) PairHarmonics<T, kWarpsPerBlock> harmonics;
   int turn = 0;
@@ -318,10 +317,9 @@ __global__ void __launch_bounds__(BS_WARPS * 32, 1)
     if (WANT_U && nc.e >= 0) yv_next = __ldg(Y + ylm * ys.m + nc.e * ys.e);
     if (node != g_node) {
       g_node = node;
-      const int64_t grow = ys.rows ? (int64_t)ys.rows[node] : node;
-#pragma unroll
+    #pragma unroll
       for (int m = 0; m < 16; m++) {
-        const ulonglong2 v = __ldg(reinterpret_cast<const ulonglong2 *>(G + (grow * 16 + m) * BS_C + c0));
+        const ulonglong2 v = __ldg(reinterpret_cast<const ulonglong2 *>(G + (node * 16 + m) * BS_C + c0));
         g2[m][0] = v.x;
         g2[m][1] = v.y;
       }

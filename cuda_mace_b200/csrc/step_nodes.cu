@@ -109,23 +109,8 @@ __global__ void __launch_bounds__(128, sizeof(T) == 4 ? 5 : 3)
     T p[ST_RO];
 #pragma unroll
     for (int j = 0; j < ST_RO; j++) p[j] = value * wp[j];
-    // 16 sums over the warp's lanes at once: every lane ends with component lane >> 1
-    {
-      T q8[8], q4[4], q2[2];
-      bool up = lane & 16;
-#pragma unroll
-      for (int i = 0; i < 8; i++) q8[i] = (up ? p[i + 8] : p[i]) + __shfl_xor_sync(0xffffffffu, up ? p[i] : p[i + 8], 16);
-      up = lane & 8;
-#pragma unroll
-      for (int i = 0; i < 4; i++) q4[i] = (up ? q8[i + 4] : q8[i]) + __shfl_xor_sync(0xffffffffu, up ? q8[i] : q8[i + 4], 8);
-      up = lane & 4;
-#pragma unroll
-      for (int i = 0; i < 2; i++) q2[i] = (up ? q4[i + 2] : q4[i]) + __shfl_xor_sync(0xffffffffu, up ? q4[i] : q4[i + 2], 4);
-      up = lane & 2;
-      T r = (up ? q2[1] : q2[0]) + __shfl_xor_sync(0xffffffffu, up ? q2[0] : q2[1], 2);
-      r += __shfl_xor_sync(0xffffffffu, r, 1);
-      if ((lane & 1) == 0) part[w][lane >> 1] = r;
-    }
+    const T r = warp_reduce16(p, lane);
+    if ((lane & 1) == 0) part[w][lane >> 1] = r;
     __syncthreads();
     if (c < 32) {
       double e1 = 0.0;

@@ -257,7 +257,6 @@ class StepPlan:
         m.atomic_energies = hold(model.atomic_energies)
         self.model = m
         self.channels, self.dtype, self.elements = C, model.dtype, Z
-        self.radial_ops = (ops.USE_TENSOR_CORES, ops.RADIAL_GRADIENT_ON_THE_FLY, ops.FUSED_RADIAL_MESSAGE_PASSING)
 
     @staticmethod
     def _radial(model, m, hold, matrix, x, lin):
