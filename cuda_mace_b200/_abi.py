@@ -69,6 +69,7 @@ SIGNATURES = {
     "cmace_imp_bwd_edge_f64_noalloc": [_P, _P, _P, _P, _P, _P, _L, _L, _I, _P, _P, _P, _P],
     "cmace_imp_bwd_node_f32": [_P, _P, _P, _L, _I, _P, _P],
     "cmace_imp_bwd_node_f64": [_P, _P, _P, _L, _I, _P, _P],
+    "cmace_imp_bwd_node_edges": [_I, _P, _P, _P, _L, _L, _I, _P, _P],
     "cmace_linear_f32": [_P, _P, _P, _P, _I, _L, _I, _I, _D, _P, _P],
     "cmace_linear_f64": [_P, _P, _P, _P, _I, _L, _I, _I, _D, _P, _P],
     "cmace_gemm_f64": [_P, _P, _L, _I, _I, _D, _P, _P],
@@ -140,7 +141,7 @@ KERNEL_LAUNCHES = {
     "cmace_sph_fwd": 1, "cmace_sph_bwd": 1, "cmace_edge_basis_fwd": 1, "cmace_edge_basis_bwd": 1,
     "cmace_edge_vectors_fwd": 1, "cmace_edge_vectors_bwd": 1,
     "cmace_spline_fwd": 1, "cmace_spline_bwd": 1, "cmace_imp_fwd": 1, "cmace_imp_bwd_edge": 1, "cmace_imp_bwd_edge_f64_noalloc": 2,
-    "cmace_imp_bwd_node": 1, "cmace_linear": 1, "cmace_symcon_fwd": 1, "cmace_symcon_bwd": 1,
+    "cmace_imp_bwd_node": 1, "cmace_imp_bwd_node_edges": 1, "cmace_linear": 1, "cmace_symcon_fwd": 1, "cmace_symcon_bwd": 1,
     "cmace_gemm_pack_weights": 1, "cmace_gemm3x": 1, "cmace_gemm": 1, "cmace_gemm3x_gradr": 1, "cmace_bounded_wait_probe": 1, "cmace_linear_tc": 1,
     "cmace_radial_hidden_fwd": 1, "cmace_radial_hidden_bwd": 1, "cmace_imp_radial_fused_fwd": 1,
     "cmace_symcon_effective_weights": 1, "cmace_symcon_apply": 1, "cmace_nl_build": 4, "cmace_nl_emit": 1, "cmace_nl_cell_ids": 1, "cmace_nl_count": 1, "cmace_exclusive_scan_i32": 1, "cmace_nl_fill": 1,

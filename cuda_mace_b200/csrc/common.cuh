@@ -43,6 +43,9 @@ template <typename T>
 int imp_bwd_edge(const T *X, const T *Y, const T *R, const T *G, const int32_t *sender, const int32_t *row_ptr,
                  int64_t nnodes, int64_t nedges, ImpLayout ys, int C, T *gradR, T *gradY, T *Tout, T *partial,
                  cmace_stream_t stream);
+template <typename T>   // nedges < 0: not known
+int imp_bwd_node(const T *Tin, const int32_t *perm, const int32_t *send_ptr, int64_t nnodes, int64_t nedges, int C, T *gradX,
+                 cmace_stream_t stream);
 int gemm3x_gradr(const float *X, const float *G, const float *Y, ImpLayout ys, const int32_t *sender,
                  const int32_t *receiver, const float *packed, int64_t nedges, int channels, int N, const float *dot,
                  float *out, int32_t *status, cmace_stream_t stream);

@@ -623,12 +623,15 @@ int imp_bwd_edge(const T *X, const T *Y, const T *R, const T *G, const int32_t *
 }
 
 template <typename T, int VEC>
-static void launch_bwd_node(const T *Tin, const int32_t *perm, const int32_t *send_ptr, int64_t nnodes,
+static void launch_bwd_node(const T *Tin, const int32_t *perm, const int32_t *send_ptr, int64_t nnodes, int64_t nedges,
                             int C, T *gradX, cudaStream_t st) {
   const int chunks = C / (32 * VEC);
-  // float32: eight warps a sender while all its rows come from L2 (35 -> 23 us at 3 000 nodes and 157 000 edges, 62 -> 55 at
-  // 8 000); one beyond (320 against 355 us at 64 000).  float64 rows leave L2 earlier (84 against 130 us at 8 000).
-  if (sizeof(T) == 4 ? nnodes * chunks <= 148 * 64 : few_nodes(nnodes * chunks)) {
+  // float32: eight warps a sender (one; eight), us at 128 channels: 36.9; 23.4 at 3 000 nodes of 52 edges, 53.3; 47.1 at
+  // 8 192 of 40, 69.6; 62.3 at 9 500 of 52, but 45.2; 43.0 at 8 192 of 32, 30.6; 32.9 of 20 and 16.0; 27.0 of 8: a warp
+  // with fewer than four rows has its loads' latency and the sum through shared memory to pay for.  98.3; 96.3 at 16 000 of
+  // 52 and 170.0; 176.3 at 32 000: one warp a sender fills the chip.  float64: 84 against 130 at 8 000 of 52.
+  const bool dense = nedges < 0 || nedges >= 36 * nnodes;   // unknown: as in a condensed system
+  if (sizeof(T) == 4 ? dense && nnodes * chunks <= 148 * 64 : few_nodes(nnodes * chunks)) {
     launch_chained(imp_bwd_node_kernel<T, VEC, kSplit>, dim3((unsigned)nnodes, chunks), kSplit * 32, 0, st, Tin, perm, send_ptr, nnodes, C,
                                                                                               gradX);
     return;
@@ -638,8 +641,8 @@ static void launch_bwd_node(const T *Tin, const int32_t *perm, const int32_t *se
 }
 
 template <typename T>
-int imp_bwd_node(const T *Tin, const int32_t *perm, const int32_t *send_ptr, int64_t nnodes,
-                        int C, T *gradX, cmace_stream_t stream) {
+int imp_bwd_node(const T *Tin, const int32_t *perm, const int32_t *send_ptr, int64_t nnodes, int64_t nedges, int C,
+                 T *gradX, cmace_stream_t stream) {
   int rc = check_common<T>(Tin, gradX, gradX, nnodes, 0, C, "cmace_imp_bwd_node");
   if (rc) return rc;
   if (nnodes == 0) return CMACE_OK;
@@ -647,10 +650,10 @@ int imp_bwd_node(const T *Tin, const int32_t *perm, const int32_t *send_ptr, int
   cudaStream_t st = (cudaStream_t)stream;
   switch (pick_vec<T>(C)) {
     case 4:
-      if constexpr (sizeof(T) == 4) launch_bwd_node<T, 4>(Tin, perm, send_ptr, nnodes, C, gradX, st);
+      if constexpr (sizeof(T) == 4) launch_bwd_node<T, 4>(Tin, perm, send_ptr, nnodes, nedges, C, gradX, st);
       break;
-    case 2: launch_bwd_node<T, 2>(Tin, perm, send_ptr, nnodes, C, gradX, st); break;
-    default: launch_bwd_node<T, 1>(Tin, perm, send_ptr, nnodes, C, gradX, st); break;
+    case 2: launch_bwd_node<T, 2>(Tin, perm, send_ptr, nnodes, nedges, C, gradX, st); break;
+    default: launch_bwd_node<T, 1>(Tin, perm, send_ptr, nnodes, nedges, C, gradX, st); break;
   }
   return check_launch("cmace_imp_bwd_node");
 }
@@ -659,7 +662,8 @@ int imp_bwd_node(const T *Tin, const int32_t *perm, const int32_t *send_ptr, int
   template int imp_fwd<T>(const T *, const T *, const T *, const int32_t *, const int32_t *, int64_t, int64_t, ImpLayout, \
                           int, T *, cmace_stream_t);                                                                   \
   template int imp_bwd_edge<T>(const T *, const T *, const T *, const T *, const int32_t *, const int32_t *, int64_t,  \
-                               int64_t, ImpLayout, int, T *, T *, T *, T *, cmace_stream_t);
+                               int64_t, ImpLayout, int, T *, T *, T *, T *, cmace_stream_t);                           \
+  template int imp_bwd_node<T>(const T *, const int32_t *, const int32_t *, int64_t, int64_t, int, T *, cmace_stream_t);
 CMACE_IMP_LAUNCHERS(float)
 CMACE_IMP_LAUNCHERS(double)
 
@@ -766,10 +770,18 @@ int cmace_imp_bwd_edge_f64_noalloc(const double *X, const double *Y, const doubl
 
 int cmace_imp_bwd_node_f32(const float *T, const int32_t *perm, const int32_t *send_ptr, int64_t nnodes,
                            int channels, float *gradX, cmace_stream_t stream) {
-  return imp_bwd_node<float>(T, perm, send_ptr, nnodes, channels, gradX, stream);
+  return imp_bwd_node<float>(T, perm, send_ptr, nnodes, -1, channels, gradX, stream);
 }
 int cmace_imp_bwd_node_f64(const double *T, const int32_t *perm, const int32_t *send_ptr, int64_t nnodes,
                            int channels, double *gradX, cmace_stream_t stream) {
-  return imp_bwd_node<double>(T, perm, send_ptr, nnodes, channels, gradX, stream);
+  return imp_bwd_node<double>(T, perm, send_ptr, nnodes, -1, channels, gradX, stream);
+}
+int cmace_imp_bwd_node_edges(int is_f64, const void *T, const int32_t *perm, const int32_t *send_ptr, int64_t nnodes,
+                             int64_t nedges, int channels, void *gradX, cmace_stream_t stream) {
+  if (is_f64)
+    return imp_bwd_node<double>(static_cast<const double *>(T), perm, send_ptr, nnodes, nedges, channels,
+                                static_cast<double *>(gradX), stream);
+  return imp_bwd_node<float>(static_cast<const float *>(T), perm, send_ptr, nnodes, nedges, channels,
+                             static_cast<float *>(gradX), stream);
 }
 }

@@ -254,8 +254,7 @@ static int run_step(const cmace_step_model &m, cmace_step_io &io, const Workspac
         return gemm3x_gradr(up, w.gm1, w.Y, ys, io.sender, io.receiver, static_cast<const float *>(m.radial_back), E, C,
                             ST_H, w.dh[1], w.dr1, io.status, st);
     case S_SENDERS:
-      if constexpr (f64) return cmace_imp_bwd_node_f64(w.T_, io.perm, io.send_ptr, nl, C, gup, st);
-      else return cmace_imp_bwd_node_f32(w.T_, io.perm, io.send_ptr, nl, C, gup, st);
+      return imp_bwd_node<T>(w.T_, io.perm, io.send_ptr, nl, E, C, gup, st);
     case S_MID_BACK:
       return K::mid_bwd(gup_owned, w.node_of, w.slot_type, w.dq, static_cast<const T *>(m.up_back),
                         static_cast<const T *>(m.extra_back), m.scale, n, C, w.gb0, st);

@@ -211,11 +211,6 @@ class IMPAutograd : public torch::autograd::Function<IMPAutograd> {
                                    gradY.data_ptr<double>(), T.data_ptr<double>(),
                                    nscratch > 0 ? scratch.data_ptr<double>() : nullptr, stream_of(X)),
             "cmace_imp_bwd_edge_f64");
-      if (beside) beside->join();
-      check(cmace_imp_bwd_node_f64(T.data_ptr<double>(), topo.perm.data_ptr<int32_t>(),
-                                   topo.send_ptr.data_ptr<int32_t>(), topo.nsenders, (int)C, gradX.data_ptr<double>(),
-                                   stream_of(X)),
-            "cmace_imp_bwd_node_f64");
     } else {
       check(cmace_imp_bwd_edge_f32(X.data_ptr<float>(), Y.data_ptr<float>(), radial.data_ptr<float>(),
                                    G.data_ptr<float>(), topo.sender.data_ptr<int32_t>(),
@@ -223,12 +218,11 @@ class IMPAutograd : public torch::autograd::Function<IMPAutograd> {
                                    gradY.data_ptr<float>(), T.data_ptr<float>(),
                                    nscratch > 0 ? scratch.data_ptr<float>() : nullptr, stream_of(X)),
             "cmace_imp_bwd_edge_f32");
-      if (beside) beside->join();
-      check(cmace_imp_bwd_node_f32(T.data_ptr<float>(), topo.perm.data_ptr<int32_t>(),
-                                   topo.send_ptr.data_ptr<int32_t>(), topo.nsenders, (int)C, gradX.data_ptr<float>(),
-                                   stream_of(X)),
-            "cmace_imp_bwd_node_f32");
     }
+    if (beside) beside->join();
+    check(cmace_imp_bwd_node_edges(f64 ? 1 : 0, T.data_ptr(), topo.perm.data_ptr<int32_t>(), topo.send_ptr.data_ptr<int32_t>(),
+                                   topo.nsenders, E, (int)C, gradX.data_ptr(), stream_of(X)),
+          "cmace_imp_bwd_node");
     return {gradX, gradY, gradR, Tensor(), Tensor(), Tensor()};
   }
 };

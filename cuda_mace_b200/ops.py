@@ -409,8 +409,8 @@ class _IMPFunction(torch.autograd.Function):
         if need_x:
             perm, send_ptr = topo.sender_order()
             gradX = torch.empty(topo.nsenders, C, dtype=X.dtype, device=X.device)
-            _abi.call("cmace_imp_bwd_node_" + _suffix(X), _ptr(T), _ptr(perm), _ptr(send_ptr), topo.nsenders, C,
-                      _ptr(gradX), _stream())
+            _abi.call("cmace_imp_bwd_node_edges", int(X.dtype == torch.float64), _ptr(T), _ptr(perm), _ptr(send_ptr),
+                      topo.nsenders, topo.nedges, C, _ptr(gradX), _stream())
         return gradX, gradY, gradR, None
 
 
@@ -453,8 +453,8 @@ class _RadialIMPFunction(torch.autograd.Function):
         if need_x:
             perm, send_ptr = topo.sender_order()
             gradX = torch.empty(topo.nsenders, C, dtype=X.dtype, device=X.device)
-            _abi.call("cmace_imp_bwd_node_f32", _ptr(T), _ptr(perm), _ptr(send_ptr), topo.nsenders, C, _ptr(gradX),
-                      _stream())
+            _abi.call("cmace_imp_bwd_node_edges", 0, _ptr(T), _ptr(perm), _ptr(send_ptr), topo.nsenders, topo.nedges, C,
+                      _ptr(gradX), _stream())
         gradH = radial_gradient_product(X, G, Y, W, topo) if ctx.needs_input_grad[2] else None
         return gradX, gradY, gradH, None, None, None
 
@@ -545,8 +545,8 @@ class _FusedRadialIMPFunction(torch.autograd.Function):
         if need_x:
             perm, send_ptr = topo.sender_order()
             gradX = torch.empty(topo.nsenders, C, dtype=X.dtype, device=X.device)
-            _abi.call("cmace_imp_bwd_node_f32", _ptr(T), _ptr(perm), _ptr(send_ptr), topo.nsenders, C, _ptr(gradX),
-                      _stream())
+            _abi.call("cmace_imp_bwd_node_edges", 0, _ptr(T), _ptr(perm), _ptr(send_ptr), topo.nsenders, topo.nedges, C,
+                      _ptr(gradX), _stream())
         gradH = _gemm3x(gradR.view(E, 4 * C), W) if ctx.needs_input_grad[2] else None
         return gradX, gradY, gradH, None, None, None
 

@@ -208,6 +208,9 @@ int cmace_imp_bwd_node_f32(const float *T, const int32_t *perm, const int32_t *s
                            int64_t nnodes, int channels, float *gradX, cmace_stream_t stream);
 int cmace_imp_bwd_node_f64(const double *T, const int32_t *perm, const int32_t *send_ptr,
                            int64_t nnodes, int channels, double *gradX, cmace_stream_t stream);
+/* the same node pass when the number of edges is known: it chooses the split of a sender's rows */
+int cmace_imp_bwd_node_edges(int is_f64, const void *T, const int32_t *perm, const int32_t *send_ptr, int64_t nnodes,
+                             int64_t nedges, int channels, void *gradX, cmace_stream_t stream);
 
 /* ---- Linear / ElementalLinear -------------------------------------------------------------
  * Replace jit_linear and jit_elemental_linear (jit_wrappers/src/linear_wrapper.cpp:23-191, kernels

@@ -720,8 +720,10 @@ def test_float64_product_tiles(M, K, N):
     assert rel_err(ops.matmul_f64(A, B), A.cpu() @ B.cpu()) < 1e-12
 
 
-# one receiver count on each side of the rule that splits a receiver over eight warps, odd degrees and empty receivers
+# one receiver count on each side of the rule that splits a receiver over eight warps, odd degrees and empty receivers; the
+# sums over a sender's edges are split from 36 edges a sender on, up to 9 472 senders and channel chunks (three at C = 96)
 @pytest.mark.parametrize("dtype", DTYPES)
-@pytest.mark.parametrize("N,deg,C", [(1184, 9, 32), (1185, 9, 32), (3, 17, 128), (592, 5, 128)])
+@pytest.mark.parametrize("N,deg,C", [(1184, 9, 32), (1185, 9, 32), (3, 17, 128), (592, 5, 128),
+                                     (40, 34, 128), (40, 45, 128), (3157, 45, 96), (3158, 45, 96)])
 def test_message_passing_around_the_split(dtype, N, deg, C, dev):
     test_message_passing(dtype, N, deg, C, None, 7, dev)
