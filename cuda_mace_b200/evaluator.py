@@ -125,7 +125,7 @@ class EnergyForceEvaluator:
             self._graph = None   # the model has changed: the recording has the old weights laid out
 
         if step.takes(positions_owned, self._shifts):
-            plan = step.plan_of(self.model)
+            plan = self._plan()
             if plan is not None:
                 return self._evaluate_native(plan, positions_owned.detach())[:2]
 
@@ -134,6 +134,13 @@ class EnergyForceEvaluator:
                                             topology=self.topology, exchange=exchange, n_owned=self.dom.n_owned)
 
         return _domain.distributed_energy_forces(node_energy, self.dom, self.plan, positions_owned)
+
+    def _plan(self):
+        """The model's plan for the current list, or None for the operators; every rank of a decomposition decides alike."""
+        plan = step.plan_of(self.model)
+        if plan is None or self.dom.nranks > 1 or step.pays(plan, self.dom.n_owned, self.topology.nedges):
+            return plan
+        return None
 
     def _evaluate_native(self, plan, positions_owned):
         """Total interaction energy over all ranks, forces on the owned atoms and this rank's sums, by the library's
@@ -181,7 +188,7 @@ class EnergyForceEvaluator:
         self.set_neighbor_list(moved["species"], moved["edge_index"], shifts)
         positions, plan, sums = moved["positions"], None, None
         if step.takes(positions, shifts):
-            plan = step.plan_of(self.model)
+            plan = self._plan()
         if plan is not None:
             energy, forces, sums = self._evaluate_native(plan, positions.detach())
         else:

@@ -255,7 +255,7 @@ class InvariantMACE(torch.nn.Module):
         positions = data["positions"]
         if compute_force and not training and step.takes(positions, data["shifts"]):
             plan = step.plan_of(self)
-            if plan is not None:
+            if plan is not None and step.pays(plan, positions.shape[0], data["shifts"].shape[0]):
                 return self._forward_native(plan, data, topology)
         if compute_force:
             positions = positions.detach().requires_grad_(True)

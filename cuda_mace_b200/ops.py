@@ -51,8 +51,8 @@ def _check_cuda(*tensors):
             raise RuntimeError("cuda_mace_b200 operators need CUDA tensors (there is no CPU path)")
         if cur is None:
             cur = torch.cuda.current_device()
-        if t.device.index != cur:
-            raise RuntimeError(f"operand on cuda:{t.device.index} while cuda:{cur} is the current device")
+        if t.get_device() != cur:
+            raise RuntimeError(f"operand on cuda:{t.get_device()} while cuda:{cur} is the current device")
 
 
 class _RefCache:

@@ -347,6 +347,33 @@ def plan_of(model):
     return plan
 
 
+# Z beyond a + b edges / atom: the operators are faster, {is_f64: {channels: (a, b)}}
+_MANY_ELEMENTS = {False: {32: (2.4, 0.255), 64: (2.3, 0.385), 96: (3.0, 0.65), 128: (8.0, 0.475)},
+                  True: {32: (1.7, 0.345), 64: (2.3, 0.405), 96: (3.0, 0.48), 128: (4.2, 0.42)}}
+
+
+def pays(plan, atoms, edges):
+    """Whether the sequence is the faster way for a system of this size.
+
+    The first layer's sums and the products on them take 64 Z columns an atom whatever its edges are, the operators 4 C
+    radial weights an edge.  Native against operators, ms, one B200: 100 000 atoms of 10 edges, float32, 64 channels: 5.4; 6.4
+    at 4 elements, 6.8; 6.5 at 7, 8.1; 6.5 at 10, 10.8; 6.6 at 16; of 21 edges 10.2; 10.2 at 10; of 31 edges 13.7; 14.2 at
+    13; float64, 30 000 atoms of 10 edges, 128 channels: 8.4; 11.0 at 4, 10.5; 11.2 at 7, 12.6; 11.5 at 10.  The lines are
+    where both take the same; a condensed system (52 edges) stays native up to 15 elements.  The operators' launches take the
+    host 2.1 ms, which small systems never need natively (20 000 atoms of 10 edges, 16 elements, float32, 32 channels: 1.98;
+    2.07); recorded, both take the same at 3 000 atoms of 16 elements in float32 (0.39; 0.40) and 1 000 in float64."""
+    m = plan.model
+    if plan.elements <= 4 or m.spline[0]:
+        return True
+    a, b = _MANY_ELEMENTS[bool(m.is_f64)][plan.channels]
+    if plan.elements <= a + b * edges / atoms:
+        return True
+    least = 100_000 if m.is_f64 else 320_000
+    if torch.cuda.is_current_stream_capturing():
+        least //= 6
+    return atoms * plan.elements < least
+
+
 def takes(positions, shifts):
     """Inputs the sequence takes: float64 positions (at least one) and shifts, or (index, table), on the device."""
     if isinstance(shifts, tuple):

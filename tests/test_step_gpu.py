@@ -417,3 +417,19 @@ def test_results_do_not_share_memory(U):
     ev, p = _periodic(U, 300, torch.float32)
     energy, forces = ev(p)
     assert energy.untyped_storage().nbytes() <= 24 and forces.untyped_storage().nbytes() == 300 * 3 * 8
+
+
+# around the line beyond which a system of few edges and many elements takes the operators: the same energies either way
+@pytest.mark.parametrize("dtype,tol", [(torch.float64, 1e-10), (torch.float32, 1e-4)])
+def test_few_edges_and_many_elements(U, dtype, tol, monkeypatch):
+    mace, data = _small(U, dtype, n=40, C=32, Z=10)
+    plan = step.plan_of(mace)
+    big = 400_000 // 10
+    assert step.pays(plan, big, 52 * big) and not step.pays(plan, big, 8 * big) and step.pays(plan, 400, 8 * 400)
+    assert step.pays(step.plan_of(_small(U, dtype, Z=4)[0]), 10 * big, 0)
+    native = mace(data)
+    monkeypatch.setattr(step, "pays", lambda *a: False)
+    monkeypatch.setattr(step, "energy_forces", None)
+    operators = mace(data)
+    assert abs(float(native["energy"] / operators["energy"]) - 1.0) < tol
+    assert float((native["forces"] - operators["forces"]).abs().max()) < tol * float(native["forces"].abs().max())
