@@ -179,6 +179,11 @@ NCU_TRAFFIC_PER_EDGE = {
 }
 
 
+# warps a scheduler and issue slots used while active, from the same capture
+ISSUE_NOTE = {step: f", on {warps} warps a scheduler (issue slots {slots} % used in the ncu capture {_SRC})"
+              for step, warps, slots in (("step[edges_back]", 3, 46), ("step[messages]", 3, 42), ("step[radial]", 4, 51))}
+
+
 def tensor_flops(name, s, E, C):
     """Tensor-core flops one launch executes, for the steps whose binding roof is the tensor pipe: float32 runs three
     fp16 terms of the product with the last radial layer ([E,64] x [64,4C]; the backward forms it for the derivative as
@@ -551,8 +556,7 @@ def main():
                         "algorithmic_flops_per_launch": flops, "avg_launch_ms": per_kernel[top]["avg_ms"],
                         "hbm_gbs_of_algorithmic_bytes": per_kernel[top]["achieved_gbs"],
                         "note": "of the two roofs this schema knows the tensor pipe is the nearer one; what binds the "
-                                "kernel is the arithmetic between its products, on 4 warps a scheduler (issue slots "
-                                "46 % used in the ncu capture named in traffic_source)"}
+                                "kernel is the arithmetic between its products" + ISSUE_NOTE.get(top, "")}
         else:
             ach = per_kernel[top]["achieved_gbs"]
             roofline = {"kernel": top, "bound": "hbm", "achieved": ach, "peak": peak, "unit": "GB/s",

@@ -40,7 +40,9 @@ constexpr int EB_W_BYTES = 2 * 32 * 128;          // hi and lo image of a step's
 constexpr int EB_W_SLOTS = 6;
 constexpr int EB_X_BYTES = EB_TILE * EB_BLK * 4;
 constexpr int EB_X_SLOTS = 5;
-constexpr int EB_G_RECV = 5;                      // receivers staged per tile; further ones are read from global memory
+// Receivers staged per tile; a warp with a further one reads G from global memory.  Five hold a tile of a condensed system: 0.57
+// ns an edge at 52 edges a receiver, 0.68 at 31, 0.96 at 21, 1.07 at 10 (832 000 edges).  Two buffers of more do not fit.
+constexpr int EB_G_RECV = 5;
 constexpr int EB_G_BYTES = EB_G_RECV * 16 * EB_C * 4;
 constexpr int EB_PIECE = 2048;                    // 32 rows x 64 bytes
 constexpr int EB_PART = EB_TILE * 17;             // floats of a buffer of partial sums

@@ -55,6 +55,7 @@ static int channel_block(int C) {
   return 32;
 }
 
+// blocks, sized for 128 channels (four warps a block): at 32 channels 10 to 12 blocks are as many warps an SM
 static int64_t node_blocks(int64_t n, int per_sm) {
   const int64_t cap = (int64_t)148 * per_sm;
   return n < cap ? n : cap;

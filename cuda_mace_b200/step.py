@@ -41,7 +41,7 @@ def half_images(Wt, scale):
 
 
 def basis_bounds(nb, r_max, p):
-    """Largest |b_n| and |db_n/dr| of the radial basis on (0, r_max): sampled on a grid far finer than the n-th wave
+    """Estimates of the largest |b_n| and |db_n/dr| of the radial basis on (0, r_max): sampled on a grid far finer than the n-th wave
     (32 points per nb = 16 half-wave), plus 5 %."""
     r = torch.arange(1, 4097, dtype=torch.float64) * (r_max / 4096)
     x = r / r_max
@@ -313,8 +313,8 @@ def plan_of(model):
     the module-level switches of ops or the environment select other kernels.
 
     A plan is finished before anybody sees it and goes when nobody reads it any more, so that any stream may use it without
-    an event: one synchronisation per set of weights.  While a stream
-    is captured nothing is laid out (the kernels would be recorded, not run): such a step takes the operators."""
+    an event: one synchronisation per set of weights.  While a stream is captured nothing is laid out (the kernels would be
+    recorded, not run): such a step takes the operators."""
     if not ops.USE_TENSOR_CORES or ops.FUSED_RADIAL_MESSAGE_PASSING or not ops.RADIAL_GRADIENT_ON_THE_FLY:
         return None
     if os.environ.get("CMACE_SYMCON_GENERIC", "")[:1] == "1":
