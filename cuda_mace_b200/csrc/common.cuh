@@ -121,6 +121,12 @@ inline bool &chain_launches() {
   static thread_local bool on = false;
   return on;
 }
+// on for a scope: the layout of the contraction's weights and the program that reads it
+struct ChainScope {
+  const bool before = chain_launches();
+  ChainScope() { chain_launches() = true; }
+  ~ChainScope() { chain_launches() = before; }
+};
 template <typename... Params, typename... Args>
 inline void launch_chained(void (*kernel)(Params...), dim3 grid, dim3 block, size_t smem, cudaStream_t st, Args &&...args) {
   cudaLaunchAttribute attr;

@@ -434,6 +434,7 @@ int cmace_symcon_apply(int is_f64, const void *X, const int32_t *atom_types, con
   if (nnodes == 0) return CMACE_OK;
   if (!X || !atom_types || !weff || !out) return fail(CMACE_ERR_ARG, "cmace_symcon_apply: null pointer");
   cudaStream_t st = (cudaStream_t)stream;
+  const ChainScope chained;
   if (is_f64) {
     const double *x = static_cast<const double *>(X), *w = static_cast<const double *>(weff);
     double *o = static_cast<double *>(out);

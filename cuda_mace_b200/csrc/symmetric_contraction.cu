@@ -17,6 +17,7 @@
 // with warp-uniform addresses.  No atomics; every output element has one writer.
 #include <cmath>
 #include <cstdlib>
+#include <cstring>
 #include <string>
 #include <vector>
 
@@ -210,6 +211,7 @@ __global__ void effective_weights_kernel(const int32_t *__restrict__ cclass3, co
                                          int w1, const T *__restrict__ W3, const T *__restrict__ W2,
                                          const T *__restrict__ W1, int C, T *__restrict__ weff) {
   constexpr int NW = canon::NCLASS3 + canon::NCLASS2 + 1;
+  grid_begin();
   const int c = blockIdx.z * blockDim.x + threadIdx.x, z = blockIdx.x, q = blockIdx.y;
   if (c >= C) return;
   T acc = T(0);
@@ -275,12 +277,18 @@ int cmace_symcon_plan_create(int maxnz, const int16_t *u3_num, const int32_t *u3
   plan->ints_total = (int)ints.size();
   plan->reals_total = (int)reals.size();
 
-  cudaError_t e = cudaMalloc(&plan->d_ints, ints.size() * sizeof(int32_t));
-  if (e == cudaSuccess) e = cudaMalloc(&plan->d_f64, reals.size() * sizeof(double));
-  if (e == cudaSuccess) e = cudaMalloc(&plan->d_f32, reals.size() * sizeof(float));
-  if (e == cudaSuccess) e = cudaMemcpy(plan->d_ints, ints.data(), ints.size() * sizeof(int32_t), cudaMemcpyHostToDevice);
-  if (e == cudaSuccess) e = cudaMemcpy(plan->d_f64, reals.data(), reals.size() * sizeof(double), cudaMemcpyHostToDevice);
-  if (e == cudaSuccess) e = cudaMemcpy(plan->d_f32, reals32.data(), reals32.size() * sizeof(float), cudaMemcpyHostToDevice);
+  // one allocation and one copy, doubles first: a first call on new tables waits for both, and for the release of old plans
+  const size_t b64 = reals.size() * sizeof(double), b32 = reals.size() * sizeof(float), bi = ints.size() * sizeof(int32_t);
+  std::vector<char> image(b64 + b32 + bi);
+  memcpy(image.data(), reals.data(), b64);
+  memcpy(image.data() + b64, reals32.data(), b32);
+  memcpy(image.data() + b64 + b32, ints.data(), bi);
+  char *base = nullptr;
+  cudaError_t e = cudaMalloc(&base, image.size());
+  plan->d_f64 = reinterpret_cast<double *>(base);
+  plan->d_f32 = reinterpret_cast<float *>(base + b64);
+  plan->d_ints = reinterpret_cast<int32_t *>(base + b64 + b32);
+  if (e == cudaSuccess) e = cudaMemcpy(base, image.data(), image.size(), cudaMemcpyHostToDevice);
   if (e != cudaSuccess) {
     cmace_symcon_plan_destroy(plan);
     return fail(CMACE_ERR_CUDA, "cmace_symcon_plan_create: %s", cudaGetErrorString(e));
@@ -291,9 +299,7 @@ int cmace_symcon_plan_create(int maxnz, const int16_t *u3_num, const int32_t *u3
 
 void cmace_symcon_plan_destroy(cmace_symcon_plan *plan) {
   if (!plan) return;
-  cudaFree(plan->d_ints);
-  cudaFree(plan->d_f64);
-  cudaFree(plan->d_f32);
+  cudaFree(plan->d_f64);   // the allocation's start
   delete plan;
 }
 
@@ -413,15 +419,16 @@ int cmace_symcon_effective_weights(const cmace_symcon_plan *plan, int is_f64, co
   const int threads = channels < 128 ? channels : 128;
   const dim3 grid((unsigned)nelements, canon::NCLASS3 + canon::NCLASS2 + 1, (unsigned)((channels + threads - 1) / threads));
   cudaStream_t st = (cudaStream_t)stream;
+  const ChainScope chained;
   if (is_f64) {
     const double *cr = plan->d_f64 + plan->canon_real_off;
-    effective_weights_kernel<double><<<grid, threads, 0, st>>>(
-        ci, ci + plan->w3, cr, cr + plan->w3, plan->w3, plan->w2, plan->w1, static_cast<const double *>(W3),
+    launch_chained(
+        effective_weights_kernel<double>, grid, threads, 0, st, ci, ci + plan->w3, cr, cr + plan->w3, plan->w3, plan->w2, plan->w1, static_cast<const double *>(W3),
         static_cast<const double *>(W2), static_cast<const double *>(W1), channels, static_cast<double *>(out));
   } else {
     const float *cr = plan->d_f32 + plan->canon_real_off;
-    effective_weights_kernel<float><<<grid, threads, 0, st>>>(
-        ci, ci + plan->w3, cr, cr + plan->w3, plan->w3, plan->w2, plan->w1, static_cast<const float *>(W3),
+    launch_chained(
+        effective_weights_kernel<float>, grid, threads, 0, st, ci, ci + plan->w3, cr, cr + plan->w3, plan->w3, plan->w2, plan->w1, static_cast<const float *>(W3),
         static_cast<const float *>(W2), static_cast<const float *>(W1), channels, static_cast<float *>(out));
   }
   return check_launch("cmace_symcon_effective_weights");
