@@ -168,17 +168,15 @@ def algorithmic_bytes(name, s, N, Ns, E, C, Z):
 
 
 # DRAM traffic per edge (dram__bytes_read.sum + dram__bytes_write.sum of one launch / edges) from the ncu capture of
-# the 8 000-atom case (E = 417 248 there); the traffic of every edge kernel grows in proportion to E, so a full launch
+# the 8 000-atom case (E = 416 510 there); the traffic of every edge kernel grows in proportion to E, so a full launch
 # moves this many bytes times its own E.
 _SRC = "profiles/step_sequence_8000_f32.txt"
 NCU_TRAFFIC_PER_EDGE = {
-    "step[edges_back]": (1229.0, _SRC),
-    "step[messages]": (424.0, _SRC),
-    "step[radial]": (933.0, _SRC),
-    "step[sums_back]": (985.0, _SRC),
+    "step[edges_back]": (1232.0, _SRC),
+    "step[messages]": (426.0, _SRC),
+    "step[radial]": (937.0, _SRC),
+    "step[sums_back]": (988.0, _SRC),
 }
-
-
 # warps a scheduler and issue slots used while active, from the same capture
 ISSUE_NOTE = {step: f", on {warps} warps a scheduler (issue slots {slots} % used in the ncu capture {_SRC})"
               for step, warps, slots in (("step[edges_back]", 3, 46), ("step[messages]", 3, 42), ("step[radial]", 4, 51))}
