@@ -29,6 +29,7 @@ class EnergyForceEvaluator:
         self._shift_rows = None   # [E, 3] of an (index, table), made when somebody asks
         self.topology = None
         self._graph = None
+        self._recording = False
 
     def set_neighbor_list(self, species, edge_index, shifts):
         """Device tensors: species [n_local] int32, edge_index [2,E] int32 (receivers sorted), shifts [E,3]."""
@@ -93,7 +94,13 @@ class EnergyForceEvaluator:
         neighbour list drops the recording, and so does a changed model."""
         if self.dom.nranks != 1:
             raise RuntimeError("capture() needs a single-rank domain")
-        self._graph = None
+        self._graph, self._recording = None, True   # the warm-up takes the way that will be recorded
+        try:
+            return self._capture(positions_owned)
+        finally:
+            self._recording = False
+
+    def _capture(self, positions_owned):
         static_pos = positions_owned.detach().clone()
         side = torch.cuda.Stream(device=self.device)
         side.wait_stream(torch.cuda.current_stream(self.device))
@@ -138,7 +145,8 @@ class EnergyForceEvaluator:
     def _plan(self):
         """The model's plan for the current list, or None for the operators; every rank of a decomposition decides alike."""
         plan = step.plan_of(self.model)
-        if plan is None or self.dom.nranks > 1 or step.pays(plan, self.dom.n_owned, self.topology.nedges):
+        if plan is None or self.dom.nranks > 1 or step.pays(plan, self.dom.n_owned, self.topology.nedges,
+                                                                   self._recording):
             return plan
         return None
 

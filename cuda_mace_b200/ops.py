@@ -63,6 +63,7 @@ class _RefCache:
     def __init__(self, size=8):
         self.size = size
         self.entries = OrderedDict()
+        self.recorded = []
 
     @staticmethod
     def key(*tensors):
@@ -76,6 +77,12 @@ class _RefCache:
         return None
 
     def put(self, key, tensors, value):
+        if torch.cuda.is_current_stream_capturing():
+            # Its kernels are recorded, not run: nobody outside the graph may find it.  Kept until the recording is over,
+            # since callers pass on the address only.
+            self.recorded.append(value)
+            return value
+        self.recorded.clear()
         self.entries[key] = (tensors, value)
         while len(self.entries) > self.size:
             self.entries.popitem(last=False)
@@ -308,6 +315,8 @@ class EdgeTopology:
         if self._perm is None:
             buffers = self.grouping_buffers()
             self.group_senders(buffers, _stream())
+            if torch.cuda.is_current_stream_capturing():
+                return buffers[:2]   # recorded, not run
             self.grouped(*buffers[:2])
         return self._perm, self._send_ptr
 

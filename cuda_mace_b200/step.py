@@ -352,8 +352,8 @@ _MANY_ELEMENTS = {False: {32: (2.4, 0.255), 64: (2.3, 0.385), 96: (3.0, 0.65), 1
                   True: {32: (1.7, 0.345), 64: (2.3, 0.405), 96: (3.0, 0.48), 128: (4.2, 0.42)}}
 
 
-def pays(plan, atoms, edges):
-    """Whether the sequence is the faster way for a system of this size.
+def pays(plan, atoms, edges, recorded=False):
+    """Whether the sequence is the faster way for a system of this size; `recorded`: in a replayed graph.
 
     The first layer's sums and the products on them take 64 Z columns an atom whatever its edges are, the operators 4 C
     radial weights an edge.  Native against operators, ms, one B200: 100 000 atoms of 10 edges, float32, 64 channels: 5.4; 6.4
@@ -369,7 +369,7 @@ def pays(plan, atoms, edges):
     if plan.elements <= a + b * edges / atoms:
         return True
     least = 100_000 if m.is_f64 else 320_000
-    if torch.cuda.is_current_stream_capturing():
+    if recorded:
         least //= 6
     return atoms * plan.elements < least
 

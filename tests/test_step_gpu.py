@@ -433,3 +433,35 @@ def test_few_edges_and_many_elements(U, dtype, tol, monkeypatch):
     operators = mace(data)
     assert abs(float(native["energy"] / operators["energy"]) - 1.0) < tol
     assert float((native["forces"] - operators["forces"]).abs().max()) < tol * float(native["forces"].abs().max())
+
+
+# A recording of operators that nothing has warmed up leaves nothing behind: their packed weights, groupings and edge orders are
+# filled by a replay only, so no call outside the graph may find them.  (Without that the second call would read them unwritten.)
+@pytest.mark.parametrize("dtype,tol", [(torch.float64, 1e-10), (torch.float32, 1e-4)])
+def test_a_recording_leaves_no_cached_results_behind(U, dtype, tol, monkeypatch):
+    mace, data = _small(U, dtype, n=40, C=64, Z=3)
+    want = mace(data)["forces"]                       # native: makes the plans of the contractions
+    data = {k: t.clone() for k, t in data.items()}    # tensors that no cache knows
+    for L in mace.layers:
+        for name, b in list(L.named_buffers()):
+            b.mul_(1)                                 # nor these versions
+    caches = (ops._packed_cache, ops._topology_cache, ops._grouping_cache, ops._onehot_cache)
+    sizes = [set(c.entries) for c in caches]
+    graph, out = _record(mace, data)                  # no layout while recording: the operators
+    assert [set(c.entries) for c in caches] == sizes
+    graph.replay()
+    assert float((out["forces"] - want).abs().max()) < tol * float(want.abs().max())
+    monkeypatch.setattr(step, "pays", lambda *a: False)
+    assert float((mace(data)["forces"] - want).abs().max()) < tol * float(want.abs().max())
+
+
+def test_a_recorded_step_that_takes_the_operators(U, monkeypatch):
+    ev, p = _periodic(U, 300, torch.float64, C=32)
+    e, f = ev(p)
+    asked = []
+    monkeypatch.setattr(step, "pays", lambda plan, atoms, edges, recorded=False: asked.append(recorded) or not recorded)
+    ev.capture(p)
+    assert set(asked) == {True} and len(asked) == 3   # twice to warm up, once recorded
+    assert torch.equal(ev(p)[1], ev(p)[1]) and float((ev(p)[1] - f).abs().max()) < 1e-10 * float(f.abs().max())
+    ev.shifts = ev.shifts                             # live again
+    assert torch.equal(ev(p)[1], f) and asked[-1] is False
