@@ -9,20 +9,30 @@
 // every sum above runs over that thread's own values, no shuffles.  (With channels on the lanes, as in the forward, the
 // sums over channels cost 31 shuffles per four edges and warp, and the kernel took 5.0 ms at 64 000 atoms.)
 //
-// Tile = 128 edges, taken 16 channels at a time by two sets of four consumer warps in turn, in steps of 8 channels: an
-// accumulator buffer holds 32 (R, four l) + 32 (R') columns, two buffers a set, so that the products of a set's next step
-// run while it works (with one buffer of 16 channels a set it waited for them: 2.35 against 2.13 ms at 64 000 atoms).
-// A operand: h and h' (hi, lo fp16), 128 columns of tensor memory, two buffers; the consumers bring the next tile's rows
-// over in quarters during a tile's first four steps.  B operand: 8 KB of W per step, streamed from L2 (every CTA reads the same
-// 128 KB).  With A in tensor memory a narrow MMA runs at its own rate (16 cycles at N = 32).
+// Tile = 128 edges in steps of 16 channels.  A operand: h and h' (hi, lo fp16), 128 columns of tensor memory, two buffers.
+// B operand: 16 KB of W per step, streamed from L2 (every CTA reads the same 128 KB).  An accumulator buffer holds 64 (R,
+// four l) + 64 (R') columns; two buffers, so that the next step's products run while a step is worked on.
 //
-//   warps 0-3, 4-7  the two sets of consumers; warp w reaches the rows 32 (w % 4) .. of the tile
-//   warp 8          issues the MMAs
-//   warp 9          W blocks and the G rows of the next tile's receivers (contiguous: the list is sorted), bulk copies
-//   warp 10         sender rows X, 64 bytes of 128 rows per block, asynchronous copies
+// A consumer warp has 16 edges and all channels: lane (g, t) holds two edges and four channels of a step, which is what
+// tcgen05.ld.16x256b hands out (column 8 j + 2 t + i of a degree is channel 4 t + 2 j + i of the step).  Every word of G
+// that a lane reads serves two edges; with an edge a lane and eight channels a step the same sums read twice the words, and
+// shared memory's 2 048 words an edge bound the kernel (128 bytes a cycle: 64 of 120 cycles an edge).
 //
-// What bounds it: the bytes that shared memory delivers to registers: a thread needs G[lm, c] of its receiver, 2048 words
-// an edge, as warp-wide broadcasts (64 wavefronts an edge), next to the B operand (24), X, T and W (24).
+//   warps 0-7    consumers: warp w the rows 32 (w % 4) + 16 (w / 4) .. of the tile
+//   warp 8       issues the MMAs
+//   warp 9       W blocks, bulk copies
+//   warps 10, 11 sender rows X, 64 bytes of 64 rows per step each, asynchronous copies
+//   warps 12-15  the next tile: Y and receivers to shared memory, h and h' through shared memory to tensor memory, and the
+//                G rows of its receivers (contiguous: the list is sorted), bulk copies by warp 12
+//
+// The consumers' 184 registers leave the other eight warps 72 (setmaxnreg); with 168 or 192 one side spills, 420 -> 465 us.
+//
+// What the consumers do besides the sums is kept short, since two warps a scheduler hide little of it: h, h', Y and G are
+// brought by other warps (consumers doing it themselves: 150 of 890 thousand cycles at 16 000 atoms), T goes out in 64-byte
+// pieces from registers instead of through shared memory, a step's barriers are asked for while the step before it is worked
+// on, the MMA issuer is one thread that does the same.  16 000 atoms (832 000 edges): 485 -> 417 us, 64 000: 2 040 -> 1 700,
+// 3 000: 102 -> 88.  What bounds it: instruction issue (59 %) and the latency of a step's chain, accumulators to registers,
+// G, sums, with two warps a scheduler; without the sums 312 us are left, without the products as well 257.
 #include "common.cuh"
 #include "step_common.cuh"
 #include "tc_ptx.cuh"
@@ -31,42 +41,48 @@ namespace cmace {
 
 constexpr int EB_TILE = 128;
 constexpr int EB_C = 128;
-constexpr int EB_BLK = 16;                        // channels of a block
-constexpr int EB_NBLK = EB_C / EB_BLK;
-constexpr int EB_THREADS = 384;
-constexpr int EB_STEP = 8;                        // channels of a step
+constexpr int EB_STEP = 16;                       // channels of a step
 constexpr int EB_NSTEP = EB_C / EB_STEP;
-constexpr int EB_W_BYTES = 2 * 32 * 128;          // hi and lo image of a step's W: 32 rows (l, channel)
-constexpr int EB_W_SLOTS = 6;
-constexpr int EB_X_BYTES = EB_TILE * EB_BLK * 4;
+constexpr int EB_THREADS = 512;
+constexpr int EB_REGS = 184, EB_REGS_OTHER = 72;   // (184 + 72) * 256 = 128 * 512: what the block is launched with
+constexpr int EB_W_BYTES = 2 * 64 * 128;          // hi and lo image of a step's W: 64 rows (l, channel)
+constexpr int EB_W_SLOTS = 3;
+constexpr int EB_X_BYTES = EB_TILE * EB_STEP * 4;
 constexpr int EB_X_SLOTS = 5;
-// Receivers staged per tile; a warp with a further one reads G from global memory.  Five hold a tile of a condensed system: 0.57
-// ns an edge at 52 edges a receiver, 0.68 at 31, 0.96 at 21, 1.07 at 10 (832 000 edges).  Two buffers of more do not fit.
-constexpr int EB_G_RECV = 5;
+// Receivers staged per tile; a warp with a further one reads G from global memory.  Six hold a tile of a condensed system: 0.50
+// ns an edge at 52 edges a receiver, 0.52 at 31, 0.88 at 21, 1.00 at 10 (416 000 edges; 0.59, 0.68, 0.97 and 1.14 with an
+// edge a lane and five).  Two buffers of more do not fit.
+constexpr int EB_G_RECV = 6;
 constexpr int EB_G_BYTES = EB_G_RECV * 16 * EB_C * 4;
 constexpr int EB_PIECE = 2048;                    // 32 rows x 64 bytes
-constexpr int EB_PART = EB_TILE * 17;             // floats of a buffer of partial sums
 constexpr int EB_OFF_W = 0;
 constexpr int EB_OFF_X = EB_OFF_W + EB_W_SLOTS * EB_W_BYTES;
 constexpr int EB_OFF_G = EB_OFF_X + EB_X_SLOTS * EB_X_BYTES;
-constexpr int EB_OFF_T = EB_OFF_G + 2 * EB_G_BYTES;        // eight pieces: T of a warp on its way out
-constexpr int EB_OFF_H = EB_OFF_T + 8 * EB_PIECE;          // eight pieces: h of the next tile on its way in
-constexpr int EB_OFF_P = EB_OFF_H + 8 * EB_PIECE;
-constexpr int EB_SMEM = EB_OFF_P + 2 * EB_PART * 4 + 1024;
+constexpr int EB_OFF_H = EB_OFF_G + 2 * EB_G_BYTES;        // eight pieces: h of the next tile on its way in, two a warp
+constexpr int EB_OFF_Y = EB_OFF_H + 8 * EB_PIECE;          // Y of the next tile, then its receivers
+constexpr int EB_SMEM = EB_OFF_Y + EB_TILE * 64 + EB_TILE * 4 + 1024;
+static_assert(EB_SMEM <= 226 * 1024, "shared memory of a block");
+
+// Which edge of the tile a row of tensor memory and shared memory holds: rows r and r + 8 of 16 are two edges in a row, so
+// that few lanes have edges of two receivers (8 of 52 places for a receiver's end in a condensed system, 15 otherwise).
+__device__ __forceinline__ int eb_edge(int row) { return (row & ~15) + 2 * (row & 7) + ((row >> 3) & 1); }
 
 struct EdgeBackArgs {
   const float *X, *Y, *G;        // [Ns, 128], [E, 16], [nnodes, 16, 128]
   const char *h, *dh;            // [E rounded up to a tile][hi 64 | lo 64] fp16
-  const char *W;                 // [16 steps][hi, lo][32 rows x 128 B, swizzled]
+  const char *W;                 // [8 steps][hi, lo][64 rows x 128 B, swizzled]
   const int32_t *sender, *receiver;
   int32_t *status;
   int64_t nedges;
   float factor_v, factor_t;      // undo the powers of two of h W and h' W
+  float *T;                      // [E, 128]
   float *gY;                     // [E, 16]; component 0 is dE/dr (Y_00 is constant)
 };
 
-__device__ __forceinline__ void eb_ld8(uint32_t taddr, uint32_t (&r)[8]) {
-  asm volatile("tcgen05.ld.sync.aligned.32x32b.x8.b32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];"
+// 16 lanes x 16 columns: thread (g, t) gets, for j = 0, 1, r[4 j], r[4 j + 1] = lane g, columns 8 j + 2 t, + 1 and r[4 j + 2],
+// r[4 j + 3] = lane g + 8, the same columns
+__device__ __forceinline__ void eb_ld(uint32_t taddr, uint32_t (&r)[8]) {
+  asm volatile("tcgen05.ld.sync.aligned.16x256b.x2.b32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];"
                : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7])
                : "r"(taddr)
                : "memory");
@@ -77,77 +93,114 @@ __device__ __forceinline__ void eb_ld_wait(uint32_t (&r)[8], uint32_t (&d)[8]) {
                : "+r"(r[0]), "+r"(r[1]), "+r"(r[2]), "+r"(r[3]), "+r"(r[4]), "+r"(r[5]), "+r"(r[6]), "+r"(r[7]), "+r"(d[0]),
                  "+r"(d[1]), "+r"(d[2]), "+r"(d[3]), "+r"(d[4]), "+r"(d[5]), "+r"(d[6]), "+r"(d[7])::"memory");
 }
-__device__ __forceinline__ void eb_lds(uint32_t a, unsigned long long &x, unsigned long long &y) {
-  asm volatile("ld.shared.v2.b64 {%0, %1}, [%2];" : "=l"(x), "=l"(y) : "r"(a) : "memory");
+__device__ __forceinline__ void eb_lds(uint32_t a, unsigned long long (&x)[2]) {
+  asm volatile("ld.shared.v2.b64 {%0, %1}, [%2];" : "=l"(x[0]), "=l"(x[1]) : "r"(a) : "memory");
 }
 __device__ __forceinline__ void eb_cp16(uint32_t dst, const void *src) {
   asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(dst), "l"(src) : "memory");
 }
 
-// eight channels of one edge: sums into gy2 (pairs of channels per component), dr2; returns T in t2
-template <bool STAGED>
-__device__ __forceinline__ void eb_half(uint32_t ta, uint32_t gs, const float *gg, const unsigned long long (&x2)[4],
-                                        const float (&y)[16], unsigned long long (&gy2)[16], unsigned long long &dr2,
-                                        unsigned long long (&t2)[4]) {
-  unsigned long long v2[4];
+__device__ __forceinline__ void eb_cp4(uint32_t dst, const void *src) {
+  asm volatile("cp.async.ca.shared.global [%0], [%1], 4;" ::"r"(dst), "l"(src) : "memory");
+}
+__device__ __forceinline__ void eb_cp_arrive(uint32_t bar) {
+  asm volatile("cp.async.mbarrier.arrive.noinc.shared::cta.b64 [%0];" ::"r"(bar) : "memory");
+}
+
+// Four channels (two pairs) of two edges: sums into gy (per edge and component) and dr2; T in t2.
+// SAME: both edges have the same receiver.  The accumulators are given back as soon as the last of them is in registers;
+// ready says whether the next step's accumulators and sender rows were there at that time.
+template <bool STAGED, bool SAME>
+__device__ __forceinline__ void eb_step(uint32_t ta, uint32_t acc_free, uint32_t next_acc, uint32_t next_acc_phase,
+                                        uint32_t next_x, uint32_t next_x_phase, bool &ready, int lane, const uint32_t (&gs)[2],
+                                        const float *const (&gg)[2], const unsigned long long (&x2)[2][2],
+                                        const float (&y)[2][16], float (&gy)[2][16],
+                                        unsigned long long (&dr2)[2], unsigned long long (&t2)[2][2]) {
+  unsigned long long v2[2][2];
   uint32_t r[2][8], d[2][8];
-  eb_ld8(ta, r[0]);
-  eb_ld8(ta + 32u, d[0]);
+  eb_ld(ta, r[0]);
+  eb_ld(ta + 64u, d[0]);
 #pragma unroll
   for (int l = 0; l < 4; l++) {
     eb_ld_wait(r[l & 1], d[l & 1]);
     if (l < 3) {   // the next degree's accumulators are on their way meanwhile
-      eb_ld8(ta + 8u * (l + 1), r[(l + 1) & 1]);
-      eb_ld8(ta + 32u + 8u * (l + 1), d[(l + 1) & 1]);
+      eb_ld(ta + 16u * (l + 1), r[(l + 1) & 1]);
+      eb_ld(ta + 64u + 16u * (l + 1), d[(l + 1) & 1]);
+    } else {
+      tc_fence_before();
+      __syncwarp();
+      if (lane == 0) mbar_arrive(acc_free);
+      ready = mbar_test(next_acc, next_acc_phase) && mbar_test(next_x, next_x_phase);
     }
-    unsigned long long u2[4], p2[4], r2[4];
+    unsigned long long r2[2][2], u2[2][2];
+    float p[2][4], u[2][4];
 #pragma unroll
-    for (int c = 0; c < 4; c++) {
-      r2[c] = pack2(__uint_as_float(r[l & 1][2 * c]), __uint_as_float(r[l & 1][2 * c + 1]));
-      if (l > 0) p2[c] = mul2(r2[c], x2[c]);
-    }
+    for (int e = 0; e < 2; e++)
+#pragma unroll
+      for (int c = 0; c < 2; c++) {
+        r2[e][c] = pack2(__uint_as_float(r[l & 1][4 * c + 2 * e]), __uint_as_float(r[l & 1][4 * c + 2 * e + 1]));
+        if (l > 0) unpack2(mul2(r2[e][c], x2[e][c]), p[e][2 * c], p[e][2 * c + 1]);
+      }
 #pragma unroll
     for (int m = l * l; m < (l + 1) * (l + 1); m++) {
-      unsigned long long g2[4];
-      if (STAGED) {
-        eb_lds(gs + (uint32_t)(m * EB_C * 4), g2[0], g2[1]);
-        eb_lds(gs + (uint32_t)(m * EB_C * 4) + 16u, g2[2], g2[3]);
-      } else {
-        const ulonglong2 a = __ldg(reinterpret_cast<const ulonglong2 *>(gg + m * EB_C));
-        const ulonglong2 b = __ldg(reinterpret_cast<const ulonglong2 *>(gg + m * EB_C) + 1);
-        g2[0] = a.x; g2[1] = a.y; g2[2] = b.x; g2[3] = b.y;
-      }
-      const unsigned long long yy = pack2(y[m], y[m]);
+      unsigned long long w[2][2];
 #pragma unroll
-      for (int c = 0; c < 4; c++) {
-        if (l == 0) u2[c] = g2[c];                       // Y_00 = 1
-        else u2[c] = m == l * l ? mul2(yy, g2[c]) : fma2(yy, g2[c], u2[c]);
-        if (l > 0) gy2[m] = fma2(p2[c], g2[c], gy2[m]);
+      for (int e = 0; e < 2; e++) {
+        if (e == 1 && SAME) {
+          w[1][0] = w[0][0];
+          w[1][1] = w[0][1];
+        } else if (STAGED) {
+          eb_lds(gs[e] + (uint32_t)(m * EB_C * 4), w[e]);
+        } else {
+          const ulonglong2 q = __ldg(reinterpret_cast<const ulonglong2 *>(gg[e] + m * EB_C));
+          w[e][0] = q.x;
+          w[e][1] = q.y;
+        }
       }
+#pragma unroll
+      for (int e = 0; e < 2; e++)
+#pragma unroll
+          for (int c = 0; c < 2; c++) {
+            float wa, wb;
+            unpack2(w[e][c], wa, wb);
+            if (l == 0) {                       // Y_00 = 1
+              u[e][2 * c] = wa;
+              u[e][2 * c + 1] = wb;
+            } else {
+              u[e][2 * c] = m == l * l ? y[e][m] * wa : fmaf(y[e][m], wa, u[e][2 * c]);
+              u[e][2 * c + 1] = m == l * l ? y[e][m] * wb : fmaf(y[e][m], wb, u[e][2 * c + 1]);
+              gy[e][m] = fmaf(p[e][2 * c + 1], wb, fmaf(p[e][2 * c], wa, gy[e][m]));
+            }
+          }
     }
 #pragma unroll
-    for (int c = 0; c < 4; c++) {
-      const unsigned long long d2 = pack2(__uint_as_float(d[l & 1][2 * c]), __uint_as_float(d[l & 1][2 * c + 1]));
-      t2[c] = l == 0 ? mul2(r2[c], u2[c]) : fma2(r2[c], u2[c], t2[c]);
-      v2[c] = l == 0 ? mul2(d2, u2[c]) : fma2(d2, u2[c], v2[c]);
-    }
+    for (int e = 0; e < 2; e++)
+#pragma unroll
+      for (int c = 0; c < 2; c++) {
+        u2[e][c] = pack2(u[e][2 * c], u[e][2 * c + 1]);
+        const unsigned long long d2 = pack2(__uint_as_float(d[l & 1][4 * c + 2 * e]), __uint_as_float(d[l & 1][4 * c + 2 * e + 1]));
+        t2[e][c] = l == 0 ? mul2(r2[e][c], u2[e][c]) : fma2(r2[e][c], u2[e][c], t2[e][c]);
+        v2[e][c] = l == 0 ? mul2(d2, u2[e][c]) : fma2(d2, u2[e][c], v2[e][c]);
+      }
   }
 #pragma unroll
-  for (int c = 0; c < 4; c++) dr2 = fma2(x2[c], v2[c], dr2);
+  for (int e = 0; e < 2; e++)
+#pragma unroll
+    for (int c = 0; c < 2; c++) dr2[e] = fma2(x2[e][c], v2[e][c], dr2[e]);
 }
 
 __global__ void __launch_bounds__(EB_THREADS, 1)
-    edge_back_kernel(const EdgeBackArgs g, const __grid_constant__ CUtensorMap t_map) {
+    edge_back_kernel(const EdgeBackArgs g) {
   extern __shared__ __align__(1024) unsigned char smem[];
-  __shared__ __align__(8) uint64_t bars[2 * EB_W_SLOTS + 2 * EB_X_SLOTS + 18];
+  __shared__ __align__(8) uint64_t bars[2 * EB_W_SLOTS + 2 * EB_X_SLOTS + 10];
   __shared__ uint32_t tmem_base_slot;
 
   const uint32_t base_s = (smem_u32(smem) + 1023u) & ~1023u;
   const int tid = threadIdx.x, warp = uniform(tid >> 5), lane = tid & 31;
   const uint32_t w_full = smem_u32(&bars[0]), w_free = w_full + 8u * EB_W_SLOTS;
   const uint32_t x_full = w_free + 8u * EB_W_SLOTS, x_free = x_full + 8u * EB_X_SLOTS;
-  const uint32_t g_full = x_free + 8u * EB_X_SLOTS, g_free = g_full + 16u, h_full = g_free + 16u;
-  const uint32_t acc_full = h_full + 16u, acc_free = acc_full + 32u, part_full = acc_free + 32u;
+  const uint32_t g_full = x_free + 8u * EB_X_SLOTS, h_full = g_full + 16u, acc_full = h_full + 16u, acc_free = acc_full + 16u;
+  const uint32_t y_full = acc_free + 16u, y_free = y_full + 8u;
 
   if (tid == 0) {
     for (int s = 0; s < EB_W_SLOTS; s++) {
@@ -155,19 +208,17 @@ __global__ void __launch_bounds__(EB_THREADS, 1)
       mbar_init(w_free + 8u * s, 1);     // the commit of the MMAs that read the slot
     }
     for (int s = 0; s < EB_X_SLOTS; s++) {
-      mbar_init(x_full + 8u * s, 32);
-      mbar_init(x_free + 8u * s, 4);
+      mbar_init(x_full + 8u * s, 64);
+      mbar_init(x_free + 8u * s, 8);
     }
     for (int b = 0; b < 2; b++) {
       mbar_init(g_full + 8u * b, 1);
-      mbar_init(g_free + 8u * b, 8);
-      mbar_init(h_full + 8u * b, 8);
-    }
-    for (int b = 0; b < 4; b++) {
+      mbar_init(h_full + 8u * b, 4);
       mbar_init(acc_full + 8u * b, 1);
-      mbar_init(acc_free + 8u * b, 4);
-      mbar_init(part_full + 8u * b, 1);
+      mbar_init(acc_free + 8u * b, 8);
     }
+    mbar_init(y_full, 128);
+    mbar_init(y_free, 8);
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
   }
   grid_wait();
@@ -176,286 +227,291 @@ __global__ void __launch_bounds__(EB_THREADS, 1)
   __syncthreads();
   tc_fence_after();
   grid_release();   // after the allocation
-  const uint32_t tmem = (uint32_t)uniform((int)tmem_base_slot);   // h buffer b at 128 b: h hi, h lo, h' hi, h' lo (32 each); acc b at 256 + 64 b
+  // h buffer b at 128 b: h, h', hi and lo 32 each; acc b at 256 + 128 b
+  const uint32_t tmem = (uint32_t)uniform((int)tmem_base_slot);
   const int64_t ntiles = (g.nedges + EB_TILE - 1) / EB_TILE;
 
   if (warp < 8) {
     // ---- consumers
-    const int q = warp & 3, set = warp >> 2;
-    const int row = 32 * q + lane;
-    const uint32_t lanes = (uint32_t)(32 * q) << 16;
-    const uint32_t sT = base_s + EB_OFF_T + (uint32_t)warp * EB_PIECE, sH = base_s + EB_OFF_H + (uint32_t)warp * EB_PIECE;
-    float *part0 = reinterpret_cast<float *>(smem + (base_s - smem_u32(smem)) + EB_OFF_P) + row * 17;
-    const char *hlane = (set == 0 ? g.h : g.dh) + (32 * q + (lane >> 2)) * 256 + 16 * (lane & 3);
-    const uint32_t hdst = sH + (uint32_t)sw64_offset(lane >> 2, lane & 3);
+    asm volatile("setmaxnreg.inc.sync.aligned.u32 %0;" ::"n"(EB_REGS));   // by whole warpgroups
+    const int row0 = 32 * (warp & 3) + 16 * (warp >> 2), rg = row0 + (lane >> 2), t = lane & 3;   // rows rg, rg + 8 of the tile
+    const uint32_t sY = base_s + EB_OFF_Y;
+    const uint32_t acc0 = tmem + ((uint32_t)row0 << 16) + 256u;
     bool ok = true;
-
-    // 64 bytes (32 k of hi or lo) of this warp's 32 rows of a tile: started here, finished by h_put
-    auto h_start = [&](int64_t tile, int piece) {
-      const char *src = hlane + tile * (EB_TILE * 256) + 64 * piece;
-#pragma unroll
-      for (int i = 0; i < 4; i++) eb_cp16(hdst + 512u * i, src + 8 * 256 * i);   // sw64_offset(r + 8, c) = sw64_offset(r, c) + 512
-      asm volatile("cp.async.commit_group;" ::: "memory");
-    };
-    auto h_put = [&](int buf, int piece) {
-      asm volatile("cp.async.wait_group 0;" ::: "memory");
-      __syncwarp();
-      uint32_t v[16];
-#pragma unroll
-      for (int c = 0; c < 4; c++)
-        asm volatile("ld.shared.v4.b32 {%0, %1, %2, %3}, [%4];"
-                     : "=r"(v[4 * c]), "=r"(v[4 * c + 1]), "=r"(v[4 * c + 2]), "=r"(v[4 * c + 3])
-                     : "r"(sH + (uint32_t)sw64_offset(lane, c))
-                     : "memory");
-      tmem_st16(tmem + lanes + 128u * (uint32_t)buf + 64u * (uint32_t)set + 16u * (uint32_t)piece, v);
-      if (piece == 3) {
-        tmem_st_wait();
-        tc_fence_before();
-      }
-      __syncwarp();
-    };
-
-    if (blockIdx.x < ntiles)
-      for (int p = 0; p < 4; p++) {
-        h_start(blockIdx.x, p);
-        h_put(0, p);
-      }
-    if (lane == 0) mbar_arrive(h_full);
-
     uint32_t k = 0;   // tiles done
-    int xs = set;     // X slot of this set's next block: blocks are numbered through the tiles, this set takes every other
+    int xs = 0;
     uint32_t xphase = 0;
     for (int64_t tile = blockIdx.x; tile < ntiles; tile += gridDim.x, k++) {
-      const int64_t base = tile * EB_TILE, e = base + row;
-      const bool in = e < g.nedges;
-      const int64_t ec = in ? e : g.nedges - 1;
-      const int r_first = __ldg(g.receiver + base);
-      const int my = __ldg(g.receiver + ec);
-      float y[16];
-      {
-        const float4 *yp = reinterpret_cast<const float4 *>(g.Y + ec * 16);
-#pragma unroll
-        for (int i = 0; i < 4; i++) {
-          const float4 v = __ldg(yp + i);
-          y[4 * i] = v.x; y[4 * i + 1] = v.y; y[4 * i + 2] = v.z; y[4 * i + 3] = v.w;
-        }
-      }
-      const bool staged = __all_sync(0xffffffffu, my - r_first < EB_G_RECV);
-      const uint32_t gs = base_s + EB_OFF_G + (k & 1u) * EB_G_BYTES + (uint32_t)(my - r_first) * (16 * EB_C * 4);
-      const float *gg = g.G + (int64_t)my * (16 * EB_C);
-      if (ok && !warp_wait(g_full + 8u * (k & 1u), (k >> 1) & 1u, lane)) {
+      const int64_t e0 = tile * EB_TILE + row0 + 2 * (lane >> 2), e1 = e0 + 1;   // eb_edge()
+      if (ok && !warp_wait_all(y_full, k & 1u, lane)) {
         if (lane == 0 && g.status) atomicCAS(g.status, 0, 61);
         ok = false;
       }
-      const bool more = tile + gridDim.x < ntiles;
-      unsigned long long gy2[16], dr2 = 0ull;
+      float y[2][16];
+      int my[2], r_first;
 #pragma unroll
-      for (int m = 0; m < 16; m++) gy2[m] = 0ull;
-#pragma unroll 1
-      for (int j = 0; ok && j < EB_NBLK / 2; j++) {
-        const int blk = 2 * j + set;
-        if (more && j == 2) {   // what the next tile starts with
-          const int64_t en = e + (int64_t)gridDim.x * EB_TILE < g.nedges ? e + (int64_t)gridDim.x * EB_TILE : g.nedges - 1;
-          asm volatile("prefetch.global.L2 [%0];" ::"l"(g.Y + en * 16));
-          if (lane == 0) asm volatile("prefetch.global.L2 [%0];" ::"l"(g.receiver + en));
-        }
-        const uint32_t use = 4u * k + (uint32_t)j;   // uses of each of this set's accumulator buffers
-        if (!(ok = warp_wait(x_full + 8u * xs, xphase, lane))) break;
-        const uint32_t sX = base_s + EB_OFF_X + (uint32_t)xs * EB_X_BYTES;
-#pragma unroll 1
-        for (int hf = 0; hf < 2; hf++) {
-          const uint32_t buf = 2u * (uint32_t)set + (uint32_t)hf;
-          const int piece = 2 * j + hf;            // of the next tile's h, in this tile's first four steps
-          if (more && piece < 4) h_start(tile + gridDim.x, piece);
-          if (!(ok = warp_wait(acc_full + 8u * buf, use & 1u, lane))) break;
-          tc_fence_after();
-          unsigned long long x2[4], t2[4];
-          eb_lds(sX + (uint32_t)sw64_offset(row, 2 * hf), x2[0], x2[1]);
-          eb_lds(sX + (uint32_t)sw64_offset(row, 2 * hf + 1), x2[2], x2[3]);
-          const uint32_t ta = tmem + lanes + 256u + 64u * buf;
-          const uint32_t coff = (uint32_t)(EB_BLK * blk + 8 * hf);
-          if (staged) eb_half<true>(ta, gs + 4u * coff, gg, x2, y, gy2, dr2, t2);
-          else eb_half<false>(ta, gs, gg + coff, x2, y, gy2, dr2, t2);
-          tc_fence_before();
-          __syncwarp();
-          if (lane == 0) mbar_arrive(acc_free + 8u * buf);
-          if (more && piece < 4) {
-            h_put((int)((k + 1) & 1u), piece);
-            if (piece == 3 && lane == 0) mbar_arrive(h_full + 8u * ((k + 1) & 1u));
-          }
-          if (hf == 0) {
-            if (elect_one()) tma_store_wait_read();   // the previous block's T has left the piece
-            __syncwarp();
-          }
-          const unsigned long long f2 = pack2(g.factor_v, g.factor_v);
+      for (int e = 0; e < 2; e++) {
 #pragma unroll
-          for (int c = 0; c < 2; c++)
-            asm volatile("st.shared.v2.b64 [%0], {%1, %2};" ::"r"(sT + (uint32_t)sw64_offset(lane, 2 * hf + c)),
-                         "l"(mul2(t2[2 * c], f2)), "l"(mul2(t2[2 * c + 1], f2))
-                         : "memory");
+        for (int i = 0; i < 4; i++) {
+          asm volatile("ld.shared.v4.f32 {%0, %1, %2, %3}, [%4];"
+                       : "=f"(y[e][4 * i]), "=f"(y[e][4 * i + 1]), "=f"(y[e][4 * i + 2]), "=f"(y[e][4 * i + 3])
+                       : "r"(sY + (uint32_t)sw64_offset(rg + 8 * e, i))
+                       : "memory");
         }
-        if (!ok) break;
-        fence_proxy_async();
-        __syncwarp();
-        if (elect_one()) {
-          mbar_arrive(x_free + 8u * xs);
-          if (base + 32 * q < g.nedges) tma_store_2d(&t_map, EB_BLK * blk, (int)base + 32 * q, sT);
+        asm volatile("ld.shared.b32 %0, [%1];" : "=r"(my[e]) : "r"(sY + EB_TILE * 64 + 4u * (uint32_t)(rg + 8 * e)) : "memory");
+      }
+      asm volatile("ld.shared.b32 %0, [%1];" : "=r"(r_first) : "r"(sY + EB_TILE * 64) : "memory");
+      __syncwarp();
+      // Y is in registers, and this warp has left the tile before: its G and h buffers are free
+      if (lane == 0) mbar_arrive(y_free);
+      const bool same = __all_sync(0xffffffffu, my[0] == my[1]);
+      const bool staged = __all_sync(0xffffffffu, my[1] - r_first < EB_G_RECV);   // the list is sorted
+      if (ok && !warp_wait_all(g_full + 8u * (k & 1u), (k >> 1) & 1u, lane)) {
+        if (lane == 0 && g.status) atomicCAS(g.status, 0, 62);
+        ok = false;
+      }
+      const uint32_t sG = base_s + EB_OFF_G + (k & 1u) * EB_G_BYTES + 16u * t;
+      float gy[2][16];
+      unsigned long long dr2[2] = {0ull, 0ull};
+#pragma unroll
+      for (int m = 0; m < 16; m++) gy[0][m] = gy[1][m] = 0.f;
+      bool ready = false;
+#pragma unroll 1
+      for (int n = 0; ok && n < EB_NSTEP; n++) {
+        // use number 4 k + n / 2 of accumulator buffer b
+        const uint32_t b = (uint32_t)n & 1u, next_phase = ((uint32_t)(n + 1) >> 1) & 1u;
+        if (!__all_sync(0xffffffffu, ready)) {
+          ok = warp_wait(x_full + 8u * xs, xphase, lane) && warp_wait(acc_full + 8u * b, ((uint32_t)n >> 1) & 1u, lane);
+          if (!ok) break;
         }
-        xs += 2;
-        if (xs >= EB_X_SLOTS) {
-          xs -= EB_X_SLOTS;
+        tc_fence_after();
+        const uint32_t sX = base_s + EB_OFF_X + (uint32_t)xs * EB_X_BYTES, x_done = x_free + 8u * xs;
+        unsigned long long x2[2][2], t2[2][2];
+        eb_lds(sX + (uint32_t)sw64_offset(rg, t), x2[0]);
+        eb_lds(sX + (uint32_t)sw64_offset(rg + 8, t), x2[1]);
+        if (++xs == EB_X_SLOTS) {
+          xs = 0;
           xphase ^= 1;
         }
+        const int c0 = EB_STEP * n + 4 * t;
+        const uint32_t gs[2] = {sG + (uint32_t)(my[0] - r_first) * (16 * EB_C * 4) + 4u * EB_STEP * (uint32_t)n,
+                                sG + (uint32_t)(my[1] - r_first) * (16 * EB_C * 4) + 4u * EB_STEP * (uint32_t)n};
+        const float *const gg[2] = {g.G + (int64_t)my[0] * (16 * EB_C) + c0, g.G + (int64_t)my[1] * (16 * EB_C) + c0};
+        auto step = [&](auto in_smem, auto one) {
+          eb_step<decltype(in_smem)::value, decltype(one)::value>(
+              acc0 + 128u * b, acc_free + 8u * b, acc_full + 8u * (b ^ 1u), next_phase, x_full + 8u * xs, xphase, ready, lane,
+              gs, gg, x2, y, gy, dr2, t2);
+        };
+        if (staged && same) step(std::true_type{}, std::true_type{});
+        else if (staged) step(std::true_type{}, std::false_type{});
+        else step(std::false_type{}, std::false_type{});
+        if (lane == 0) mbar_arrive(x_done);   // the accumulators went back after every lane had read its X
+        const unsigned long long f2 = pack2(g.factor_v, g.factor_v);
+        ulonglong2 *out = reinterpret_cast<ulonglong2 *>(g.T + e0 * EB_C + c0);
+        if (e0 < g.nedges) out[0] = make_ulonglong2(mul2(t2[0][0], f2), mul2(t2[0][1], f2));
+        if (e1 < g.nedges) out[EB_C / 4] = make_ulonglong2(mul2(t2[1][0], f2), mul2(t2[1][1], f2));
       }
-      if (!ok && lane == 0 && g.status) atomicCAS(g.status, 0, 62);
+      if (!ok) {
+        if (lane == 0 && g.status) atomicCAS(g.status, 0, 66);
+        break;
+      }
+      // the four lanes of an edge hold its sums over their channels; lane t ends up with the components 4 t .. 4 t + 3
+#pragma unroll
+      for (int e = 0; e < 2; e++) {
+        float h8[8], o[4], lo, hi;
+        unpack2(dr2[e], lo, hi);
+        gy[e][0] = lo + hi;
+        const bool up = (t & 2) != 0, odd = (t & 1) != 0;
+#pragma unroll
+        for (int i = 0; i < 8; i++) {
+          const float send = up ? gy[e][i] : gy[e][i + 8], keep = up ? gy[e][i + 8] : gy[e][i];
+          h8[i] = keep + __shfl_xor_sync(0xffffffffu, send, 2);
+        }
+#pragma unroll
+        for (int i = 0; i < 4; i++) {
+          const float send = odd ? h8[i] : h8[i + 4], keep = odd ? h8[i + 4] : h8[i];
+          o[i] = (keep + __shfl_xor_sync(0xffffffffu, send, 1)) * (i == 0 && t == 0 ? g.factor_t : g.factor_v);
+        }
+        const int64_t ee = e ? e1 : e0;
+        if (ee < g.nedges) *reinterpret_cast<float4 *>(g.gY + ee * 16 + 4 * t) = make_float4(o[0], o[1], o[2], o[3]);
+      }
+    }
+  } else {
+    asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(EB_REGS_OTHER));
+    if (warp == 8) {
+      // ---- MMA issuer, one thread: what a step waits for is asked for while the step before it is still being issued
+      if (elect_one()) {
+        const uint32_t idesc = umma_idesc_f16(128, 64);
+        int slot = 0;
+        uint32_t wphase = 0, k = 0;
+        bool ok = true;
+        for (int64_t tile = blockIdx.x; ok && tile < ntiles; tile += gridDim.x, k++) {
+          ok = mbar_wait(h_full + 8u * (k & 1u), (k >> 1) & 1u);
+          bool ready = false;
+          for (int n = 0; ok && n < EB_NSTEP; n++) {
+            const uint32_t b = (uint32_t)n & 1u;
+            if (!ready) ok = mbar_wait(acc_free + 8u * b, (((uint32_t)n >> 1) & 1u) ^ 1u) && mbar_wait(w_full + 8u * slot, wphase);
+            if (!ok) break;
+            tc_fence_after();
+            const uint32_t sW = base_s + EB_OFF_W + (uint32_t)slot * EB_W_BYTES;
+            const uint64_t b_hi = umma_desc_sw128(sW), b_lo = umma_desc_sw128(sW + EB_W_BYTES / 2);
+            const uint32_t d = tmem + 256u + 128u * b, a = tmem + 128u * (k & 1u);
+            const uint32_t done = w_free + 8u * slot;
+            if (++slot == EB_W_SLOTS) {
+              slot = 0;
+              wphase ^= 1;
+            }
+#pragma unroll
+            for (int j = 0; j < 4; j++) {   // R and R'
+              if (j == 3)
+                ready = n + 1 < EB_NSTEP && mbar_test(acc_free + 8u * (b ^ 1u), (((uint32_t)(n + 1) >> 1) & 1u) ^ 1u) &&
+                        mbar_test(w_full + 8u * slot, wphase);
+              umma_f16_ts(d, a + 8u * j, b_hi + (uint64_t)(2 * j), idesc, j != 0);
+              umma_f16_ts(d + 64u, a + 64u + 8u * j, b_hi + (uint64_t)(2 * j), idesc, j != 0);
+              umma_f16_ts(d, a + 8u * j, b_lo + (uint64_t)(2 * j), idesc, 1);
+              umma_f16_ts(d + 64u, a + 64u + 8u * j, b_lo + (uint64_t)(2 * j), idesc, 1);
+              umma_f16_ts(d, a + 32u + 8u * j, b_hi + (uint64_t)(2 * j), idesc, 1);
+              umma_f16_ts(d + 64u, a + 96u + 8u * j, b_hi + (uint64_t)(2 * j), idesc, 1);
+            }
+            umma_commit(done);
+            umma_commit(acc_full + 8u * b);
+          }
+        }
+        if (!ok && g.status) atomicCAS(g.status, 0, 63);
+      }
       __syncwarp();
-      if (lane == 0) mbar_arrive(g_free + 8u * (k & 1u));
-      // The two sets' sums of an edge meet through shared memory.  Set 0 is the one ahead: it leaves its sums and goes on,
-      // set 1 adds them.  (Two buffers: the MMAs come in step order, so set 0 cannot finish a tile before set 1 has left
-      // the previous one.)
-      float v[16], lo, hi;
-      unpack2(dr2, lo, hi);
-      v[0] = (lo + hi) * g.factor_t;
-#pragma unroll
-      for (int m = 1; m < 16; m++) {
-        unpack2(gy2[m], lo, hi);
-        v[m] = (lo + hi) * g.factor_v;
-      }
-      float *part = part0 + (k & 1u) * EB_PART;
-      if (set == 0) {
-#pragma unroll
-        for (int m = 0; m < 16; m++) part[m] = v[m];
-        __syncwarp();
-        if (lane == 0) mbar_arrive(part_full + 8u * q);
-      } else {
-        if (ok && !warp_wait(part_full + 8u * q, k & 1u, lane)) {
-          if (lane == 0 && g.status) atomicCAS(g.status, 0, 66);
-          ok = false;
-        }
-        if (in && ok) {
-#pragma unroll
-          for (int m = 0; m < 16; m++) v[m] += part[m];
-          float4 *o = reinterpret_cast<float4 *>(g.gY + e * 16);
-#pragma unroll
-          for (int i = 0; i < 4; i++) o[i] = make_float4(v[4 * i], v[4 * i + 1], v[4 * i + 2], v[4 * i + 3]);
-        }
-      }
-    }
-    asm volatile("cp.async.wait_all;" ::: "memory");
-    __syncwarp();
-    if (elect_one()) tma_store_wait_all();
-  } else if (warp == 8) {
-    // ---- MMA issuer
-    const uint32_t idesc = umma_idesc_f16(128, 32);
-    int slot = 0;
-    uint32_t wphase = 0, k = 0;
-    bool ok = true;
-    for (int64_t tile = blockIdx.x; ok && tile < ntiles; tile += gridDim.x, k++) {
-      ok = warp_wait(h_full + 8u * (k & 1u), (k >> 1) & 1u, lane);
-      for (int n = 0; ok && n < EB_NSTEP; n++) {
-        const uint32_t b = (uint32_t)n & 3u, use = 4u * k + (uint32_t)(n >> 2);   // buffers 0, 1 are set 0's, 2, 3 set 1's
-        ok = warp_wait(acc_free + 8u * b, (use & 1u) ^ 1u, lane) && warp_wait(w_full + 8u * slot, wphase, lane);
-        if (!ok) break;
-        if (elect_one()) {
-          tc_fence_after();
-          const uint32_t sW = base_s + EB_OFF_W + (uint32_t)slot * EB_W_BYTES;
-          const uint64_t b_hi = umma_desc_sw128(sW), b_lo = umma_desc_sw128(sW + EB_W_BYTES / 2);
-          const uint32_t d = tmem + 256u + 64u * b, a = tmem + 128u * (k & 1u);
-#pragma unroll
-          for (int j = 0; j < 4; j++) {   // R and R'
-            umma_f16_ts(d, a + 8u * j, b_hi + (uint64_t)(2 * j), idesc, j != 0);
-            umma_f16_ts(d + 32u, a + 64u + 8u * j, b_hi + (uint64_t)(2 * j), idesc, j != 0);
-            umma_f16_ts(d, a + 8u * j, b_lo + (uint64_t)(2 * j), idesc, 1);
-            umma_f16_ts(d + 32u, a + 64u + 8u * j, b_lo + (uint64_t)(2 * j), idesc, 1);
-            umma_f16_ts(d, a + 32u + 8u * j, b_hi + (uint64_t)(2 * j), idesc, 1);
-            umma_f16_ts(d + 32u, a + 96u + 8u * j, b_hi + (uint64_t)(2 * j), idesc, 1);
+    } else if (warp == 9) {
+      // ---- W blocks; one thread
+      if (elect_one()) {
+        int slot = 0;
+        uint32_t wphase = 0;
+        bool ok = true;
+        for (int64_t tile = blockIdx.x; ok && tile < ntiles; tile += gridDim.x)
+          for (int n = 0; ok && n < EB_NSTEP; n++) {
+            ok = mbar_wait(w_free + 8u * slot, wphase ^ 1);
+            if (!ok) break;
+            mbar_arrive_expect_tx(w_full + 8u * slot, EB_W_BYTES);
+            bulk_copy_g2s(base_s + EB_OFF_W + (uint32_t)slot * EB_W_BYTES, g.W + (int64_t)n * EB_W_BYTES, EB_W_BYTES,
+                          w_full + 8u * slot);
+            if (++slot == EB_W_SLOTS) {
+              slot = 0;
+              wphase ^= 1;
+            }
           }
-          umma_commit(w_free + 8u * slot);
-          umma_commit(acc_full + 8u * b);
-        }
-        __syncwarp();
-        if (++slot == EB_W_SLOTS) {
-          slot = 0;
-          wphase ^= 1;
-        }
+        if (!ok && g.status) atomicCAS(g.status, 0, 64);
       }
-    }
-    if (!ok && lane == 0 && g.status) atomicCAS(g.status, 0, 63);
-  } else if (warp == 9) {
-    // ---- W blocks and G rows; one thread
-    if (elect_one()) {
+      __syncwarp();
+    } else if (warp < 12) {
+      // ---- sender rows: warp 10 the first 64 of a tile, warp 11 the others
+      const int r0 = 64 * (warp - 10) + (lane >> 2);
       int slot = 0;
-      uint32_t wphase = 0, k = 0;
+      uint32_t phase = 0;
       bool ok = true;
-      auto load_g = [&](int64_t tile, uint32_t n) -> bool {   // n: how many tiles of this CTA came before
-        const int64_t base = tile * EB_TILE, last = base + EB_TILE - 1 < g.nedges ? base + EB_TILE - 1 : g.nedges - 1;
-        const int r0 = __ldg(g.receiver + base);
-        int count = __ldg(g.receiver + last) - r0 + 1;
-        count = count < EB_G_RECV ? count : EB_G_RECV;
-        if (!mbar_wait(g_free + 8u * (n & 1u), ((n >> 1) & 1u) ^ 1u)) return false;
-        const uint32_t bar = g_full + 8u * (n & 1u), dst = base_s + EB_OFF_G + (n & 1u) * EB_G_BYTES;
-        mbar_arrive_expect_tx(bar, (uint32_t)count * (16 * EB_C * 4));
-        for (int i = 0; i < count; i++)
-          bulk_copy_g2s(dst + (uint32_t)i * (16 * EB_C * 4), g.G + (int64_t)(r0 + i) * (16 * EB_C), 16 * EB_C * 4, bar);
-        return true;
+      int next[8];
+      auto load_senders = [&](int64_t tile) {
+#pragma unroll
+        for (int i = 0; i < 8; i++) {
+          const int64_t e = tile * EB_TILE + eb_edge(8 * i + r0);
+          next[i] = __ldg(g.sender + (e < g.nedges ? e : g.nedges - 1));
+        }
       };
-      if (blockIdx.x < ntiles) ok = load_g(blockIdx.x, 0);
-      for (int64_t tile = blockIdx.x; ok && tile < ntiles; tile += gridDim.x, k++)
-        for (int n = 0; ok && n < EB_NSTEP; n++) {
-          ok = mbar_wait(w_free + 8u * slot, wphase ^ 1);
-          if (!ok) break;
-          mbar_arrive_expect_tx(w_full + 8u * slot, EB_W_BYTES);
-          bulk_copy_g2s(base_s + EB_OFF_W + (uint32_t)slot * EB_W_BYTES, g.W + (int64_t)n * EB_W_BYTES, EB_W_BYTES,
-                        w_full + 8u * slot);
-          if (++slot == EB_W_SLOTS) {
-            slot = 0;
-            wphase ^= 1;
-          }
-          // the buffer was last read by the tile before this one, which the consumers have left by step 8
-          if (n == 8 && tile + gridDim.x < ntiles) ok = load_g(tile + gridDim.x, k + 1);
-        }
-      if (!ok && g.status) atomicCAS(g.status, 0, 64);
-    }
-    __syncwarp();
-  } else if (warp == 10) {
-    // ---- sender rows
-    int slot = 0;
-    uint32_t phase = 0;
-    bool ok = true;
-    for (int64_t tile = blockIdx.x; ok && tile < ntiles; tile += gridDim.x) {
-      int s[16];
+      if (blockIdx.x < ntiles) load_senders(blockIdx.x);
+      for (int64_t tile = blockIdx.x; ok && tile < ntiles; tile += gridDim.x) {
+        const float *src[8];
 #pragma unroll
-      for (int i = 0; i < 16; i++) {
-        int64_t e = tile * EB_TILE + 8 * i + (lane >> 2);
-        e = e < g.nedges ? e : g.nedges - 1;
-        s[i] = __ldg(g.sender + e);
-      }
+        for (int i = 0; i < 8; i++) src[i] = g.X + (int64_t)next[i] * EB_C + 4 * (lane & 3);
+        if (tile + gridDim.x < ntiles) load_senders(tile + gridDim.x);
 #pragma unroll 1
-      for (int blk = 0; blk < EB_NBLK; blk++) {
-        ok = warp_wait(x_free + 8u * slot, phase ^ 1, lane);
-        if (!ok) break;
-        const uint32_t dst = base_s + EB_OFF_X + (uint32_t)slot * EB_X_BYTES;
-        const float *src = g.X + EB_BLK * blk + 4 * (lane & 3);
+        for (int n = 0; n < EB_NSTEP; n++) {
+          ok = warp_wait_all(x_free + 8u * slot, phase ^ 1, lane);
+          if (!ok) break;
+          const uint32_t dst = base_s + EB_OFF_X + (uint32_t)slot * EB_X_BYTES;
 #pragma unroll
-        for (int i = 0; i < 16; i++)
-          eb_cp16(dst + (uint32_t)sw64_offset(8 * i + (lane >> 2), lane & 3), src + (int64_t)s[i] * EB_C);
-        asm volatile("cp.async.mbarrier.arrive.noinc.shared::cta.b64 [%0];" ::"r"(x_full + 8u * slot) : "memory");
-        if (++slot == EB_X_SLOTS) {
-          slot = 0;
-          phase ^= 1;
+          for (int i = 0; i < 8; i++) eb_cp16(dst + (uint32_t)sw64_offset(8 * i + r0, lane & 3), src[i] + EB_STEP * n);
+          eb_cp_arrive(x_full + 8u * slot);
+          if (++slot == EB_X_SLOTS) {
+            slot = 0;
+            phase ^= 1;
+          }
         }
       }
+      if (!ok && lane == 0 && g.status) atomicCAS(g.status, 0, 65);
+      asm volatile("cp.async.wait_all;" ::: "memory");
+    } else {
+      // ---- the next tile's rows; warp 12 + q the rows 32 q ..
+      const int q = warp & 3;
+      const uint32_t sH = base_s + EB_OFF_H + (uint32_t)(2 * q) * EB_PIECE, sY = base_s + EB_OFF_Y;
+      const uint32_t lanes = (uint32_t)(32 * q) << 16;
+      const int r0 = 32 * q + (lane >> 2);
+      const uint32_t hdst = sH + (uint32_t)sw64_offset(lane >> 2, lane & 3);
+      bool ok = true;
+      uint32_t k = 0;
+      for (int64_t tile = blockIdx.x; ok && tile < ntiles; tile += gridDim.x, k++) {
+        const int64_t base = tile * EB_TILE;
+        if (k && !warp_wait_all(y_free, (k & 1u) ^ 1u, lane)) {   // the consumers have begun the tile before this one
+          if (lane == 0 && g.status) atomicCAS(g.status, 0, 67);
+          ok = false;
+          break;
+        }
+        tc_fence_after();
+#pragma unroll
+        for (int i = 0; i < 4; i++) {
+          const int64_t r = base + eb_edge(r0 + 8 * i), e = r < g.nedges ? r : g.nedges - 1;
+          eb_cp16(sY + (uint32_t)sw64_offset(r0 + 8 * i, lane & 3), g.Y + e * 16 + 4 * (lane & 3));
+        }
+        const int64_t rr = base + eb_edge(32 * q + lane), er = rr < g.nedges ? rr : g.nedges - 1;
+        eb_cp4(sY + EB_TILE * 64 + 4u * (uint32_t)(32 * q + lane), g.receiver + er);
+        eb_cp_arrive(y_full);
+        // 64 bytes (32 k of hi or lo) of 32 rows: pieces 0-3 of h, 4-7 of h'
+        auto start = [&](int piece) {
+          if (piece < 8) {
+            const char *src = (piece < 4 ? g.h : g.dh) + base * 256 + 64 * (piece & 3) + 16 * (lane & 3);
+#pragma unroll
+            for (int i = 0; i < 4; i++)   // sw64_offset(r + 8, c) = sw64_offset(r, c) + 512
+              eb_cp16(hdst + (uint32_t)((piece & 1) * EB_PIECE) + 512u * i, src + 256 * eb_edge(r0 + 8 * i));
+          }
+          asm volatile("cp.async.commit_group;" ::: "memory");
+        };
+        start(0);
+        start(1);
+        if (warp == 12 && elect_one()) {
+          const int64_t last = base + EB_TILE - 1 < g.nedges ? base + EB_TILE - 1 : g.nedges - 1;
+          const int first = __ldg(g.receiver + base);
+          int count = __ldg(g.receiver + last) - first + 1;
+          count = count < EB_G_RECV ? count : EB_G_RECV;
+          const uint32_t bar = g_full + 8u * (k & 1u), dst = base_s + EB_OFF_G + (k & 1u) * EB_G_BYTES;
+          mbar_arrive_expect_tx(bar, (uint32_t)count * (16 * EB_C * 4));
+          for (int i = 0; i < count; i++)
+            bulk_copy_g2s(dst + (uint32_t)i * (16 * EB_C * 4), g.G + (int64_t)(first + i) * (16 * EB_C), 16 * EB_C * 4, bar);
+        }
+        __syncwarp();
+#pragma unroll 1
+        for (int piece = 0; piece < 8; piece++) {
+          asm volatile("cp.async.wait_group 1;" ::: "memory");
+          __syncwarp();
+          uint32_t v[16];
+#pragma unroll
+          for (int c = 0; c < 4; c++)
+            asm volatile("ld.shared.v4.b32 {%0, %1, %2, %3}, [%4];"
+                         : "=r"(v[4 * c]), "=r"(v[4 * c + 1]), "=r"(v[4 * c + 2]), "=r"(v[4 * c + 3])
+                         : "r"(sH + (uint32_t)((piece & 1) * EB_PIECE) + (uint32_t)sw64_offset(lane, c))
+                         : "memory");
+          tmem_st16(tmem + lanes + 128u * (k & 1u) + 16u * (uint32_t)piece, v);
+          __syncwarp();
+          start(piece + 2);
+        }
+        tmem_st_wait();
+        tc_fence_before();
+        __syncwarp();
+        if (lane == 0) mbar_arrive(h_full + 8u * (k & 1u));
+      }
+      asm volatile("cp.async.wait_all;" ::: "memory");
     }
-    if (!ok && lane == 0 && g.status) atomicCAS(g.status, 0, 65);
-    asm volatile("cp.async.wait_all;" ::: "memory");
   }
   tc_fence_before();
   __syncthreads();
   if (warp == 8) tmem_dealloc(tmem, 512);
 }
-
-// [rows, 128] float32 as boxes of 32 rows x 16 columns with the 64-byte swizzle
-int encode_piece_tensor_map(CUtensorMap *tmap, float *base, int64_t rows, int cols, const char *what);
 
 int fused_messages_back(const float *X, const float *Y, const float *G, const void *h, const void *dh, const void *W,
                         float factor_v, float factor_t, const int32_t *sender, const int32_t *receiver, int64_t nedges,
@@ -465,12 +521,10 @@ int fused_messages_back(const float *X, const float *Y, const float *G, const vo
   const int64_t ntiles = (nedges + EB_TILE - 1) / EB_TILE;
   if (ntiles * EB_TILE > 0x7fffffffLL) return fail(CMACE_ERR_UNSUPPORTED, "%s: too many edges", what);
   const EdgeBackArgs g{X, Y, G, static_cast<const char *>(h), static_cast<const char *>(dh), static_cast<const char *>(W),
-                       sender, receiver, status, nedges, factor_v, factor_t, gY};
-  CUtensorMap map;
-  if (int rc = encode_piece_tensor_map(&map, T, nedges, EB_C, what)) return rc;
+                       sender, receiver, status, nedges, factor_v, factor_t, T, gY};
   cudaError_t e = cudaFuncSetAttribute(edge_back_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, EB_SMEM);
   if (e != cudaSuccess) return fail(CMACE_ERR_CUDA, "%s: %s", what, cudaGetErrorString(e));
-  launch_chained(edge_back_kernel, (unsigned)(ntiles < 148 ? ntiles : 148), EB_THREADS, EB_SMEM, st, g, map);
+  launch_chained(edge_back_kernel, (unsigned)(ntiles < 148 ? ntiles : 148), EB_THREADS, EB_SMEM, st, g);
   return check_launch(what);
 }
 

@@ -1369,22 +1369,6 @@ int encode_half_rows_tensor_map(CUtensorMap *tmap, const void *base, int64_t row
   return CMACE_OK;
 }
 
-// [rows, cols] float32 as boxes of 32 rows x 16 columns with the 64-byte swizzle
-int encode_piece_tensor_map(CUtensorMap *tmap, float *base, int64_t rows, int cols, const char *what) {
-  memset(tmap, 0, sizeof(*tmap));
-  EncodeTiledFn enc = encode_tiled_fn();
-  if (enc == nullptr) return fail(CMACE_ERR_CUDA, "%s: cuTensorMapEncodeTiled is not available", what);
-  const cuuint64_t dims[2] = {(cuuint64_t)cols, (cuuint64_t)rows};
-  const cuuint64_t strides[1] = {(cuuint64_t)cols * 4};
-  const cuuint32_t box[2] = {16, 32};
-  const cuuint32_t estr[2] = {1, 1};
-  const CUresult r = enc(tmap, CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 2, base, dims, strides, box, estr,
-                         CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_64B, CU_TENSOR_MAP_L2_PROMOTION_NONE,
-                         CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
-  if (r != CUDA_SUCCESS) return fail(CMACE_ERR_CUDA, "%s: cuTensorMapEncodeTiled (pieces) failed (%d)", what, (int)r);
-  return CMACE_OK;
-}
-
 // out [rows, N] as 32-row x 32-column boxes (128 bytes per row: one swizzle span) for the epilogue's tile stores
 static int encode_out_tensor_map(CUtensorMap *tmap, float *out, int64_t rows, int N, const char *what) {
   memset(tmap, 0, sizeof(*tmap));

@@ -33,6 +33,18 @@ __device__ __forceinline__ bool mbar_try_wait(uint32_t bar, uint32_t parity) {
       : "memory");
   return ok != 0;
 }
+// asks without waiting (try_wait may suspend the thread for a while)
+__device__ __forceinline__ bool mbar_test(uint32_t bar, uint32_t parity) {
+  uint32_t ok;
+  asm volatile(
+      "{\n\t.reg .pred p;\n\t"
+      "mbarrier.test_wait.parity.shared::cta.b64 p, [%1], %2;\n\t"
+      "selp.u32 %0, 1, 0, p;\n\t}"
+      : "=r"(ok)
+      : "r"(bar), "r"(parity)
+      : "memory");
+  return ok != 0;
+}
 // bounded wait: false after GT_TIMEOUT_CYCLES
 __device__ __forceinline__ bool mbar_wait(uint32_t bar, uint32_t parity) {
   if (mbar_try_wait(bar, parity)) return true;
@@ -265,6 +277,12 @@ __device__ __forceinline__ bool warp_wait(uint32_t bar, uint32_t parity, int lan
   uint32_t got = 1;
   if (lane == 0) got = mbar_wait(bar, parity) ? 1u : 0u;
   return __shfl_sync(0xffffffffu, got, 0) != 0;
+}
+
+// every lane asks once, which is enough when the barrier is there already (no lane waits for another's answer to be handed on)
+__device__ __forceinline__ bool warp_wait_all(uint32_t bar, uint32_t parity, int lane) {
+  if (__all_sync(0xffffffffu, mbar_try_wait(bar, parity))) return true;
+  return warp_wait(bar, parity, lane);
 }
 
 // host side (gemm_tc.cu): tensor map for 128-row x 32-column tile loads of a row-major float32 matrix [rows, K]

@@ -375,8 +375,8 @@ typedef struct cmace_step_model {
   const void *fused_w;       /* float32 with 128 channels and radial_half, or NULL: second layer's W4^T as fp16 rows
                                 [512][hi 64 | lo 64], row j*128 + q*32 + i = degree (q < 2 ? (j < 2 ? 3 : 0) : (j < 2 ? 1 : 2)),
                                 channel 64 (q & 1) + 2 i + (j & 1), divided by fused_scale (a power of two) */
-  const void *fused_w_back;  /* the same W4^T for the backward: [16 steps of 8 channels][hi, lo][32 rows (degree, channel)
-                                x 128 bytes], 128-byte swizzle */
+  const void *fused_w_back;  /* the same W4^T for the backward: [8 steps of 16 channels][hi, lo][64 rows x 128 bytes], 128-byte
+                                swizzle; row 16 l + 8 j + 2 t + i is degree l, channel 4 t + 2 j + i of the step */
   float fused_scale, reserved2;
   const void *radial_back;   /* second layer's W4 for the gradient: float32 packed W4 itself, float64 W4^T [4C,64] */
   const void *spline[2];     /* tabulated radial weights: coefficients [intervals][4][4C] of both layers, or NULL; then the

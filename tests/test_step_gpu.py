@@ -72,6 +72,32 @@ def test_step_against_autograd(U, dtype, tol, n, C, Z, nb, radial):
     assert float((out["forces"] + g).abs().max()) < tol * float(g.abs().max())
 
 
+# the second layer's fused kernels at the edges of their tiles (32 and 128 edges) and of their pairs and groups of edges (2, 8,
+# 16): lists of so many edges with so many a receiver, and receivers without any; 40 a receiver is more than a tile of the
+# forward holds, 1 more receivers than the backward stages.  The model's own autograd path is the reference.
+@pytest.mark.parametrize("edges", [1, 9, 127, 128, 129, 300])
+@pytest.mark.parametrize("degree", [1, 2, 3, 17, 40])
+def test_second_layer_at_tile_edges(U, edges, degree):
+    rng = np.random.default_rng(edges * 50 + degree)
+    n = -(-edges // degree) + 2
+    receiver = np.minimum(np.arange(edges) // degree, n - 1)
+    receiver[receiver > 0] += 1          # receiver 1 and the last one have no edges
+    sender = rng.integers(0, n, edges)
+    pos, shifts = rng.normal(size=(n, 3)), rng.normal(size=(edges, 3))   # a shift an edge: any distance up to the cutoff
+    length = rng.uniform(0.9, 4.9, edges)[:, None]
+    shifts = shifts / np.linalg.norm(shifts, axis=1, keepdims=True) * length - (pos[sender] - pos[receiver])
+    mace = model.InvariantMACE(systems.init_params(128, 3, 7), U, dtype=torch.float32, device="cuda")
+    p, species = torch.from_numpy(pos).cuda(), torch.from_numpy(rng.integers(0, 3, n).astype(np.int32)).cuda()
+    ei, sh = torch.from_numpy(np.stack([receiver, sender]).astype(np.int32)).cuda(), torch.from_numpy(shifts).cuda()
+    out = mace(dict(positions=p, species=species, edge_index=ei, shifts=sh))
+    assert step.plan_of(mace) is not None
+    p.requires_grad_(True)
+    energies = mace.node_energies(p, species, ei, sh)
+    (g,) = torch.autograd.grad(energies.sum(), p)
+    assert abs(float(out["interaction_energy"].double() - energies.sum())) < 1e-5 * max(float(energies.abs().sum()), 1e-3)
+    assert float((out["forces"] + g).abs().max()) < 1e-4 * max(float(g.abs().max()), 1e-6)
+
+
 # below and above the 32 768 edges from which a new list's grouping by sender runs beside the step
 @pytest.mark.parametrize("n", [300, 1100])
 def test_new_list_and_host_batch(U, n):
