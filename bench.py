@@ -179,7 +179,7 @@ NCU_TRAFFIC_PER_EDGE = {
 }
 # warps a scheduler and issue slots used while active, from the same capture
 ISSUE_NOTE = {step: f", on {warps} warps a scheduler (issue slots {slots} % used in the ncu capture {_SRC})"
-              for step, warps, slots in (("step[edges_back]", 3, 46), ("step[messages]", 3, 42), ("step[radial]", 4, 51))}
+              for step, warps, slots in (("step[edges_back]", 4, 59), ("step[messages]", 3, 42), ("step[radial]", 4, 51))}
 
 
 def tensor_flops(name, s, E, C):
