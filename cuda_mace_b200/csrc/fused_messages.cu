@@ -15,6 +15,11 @@
 // and 1 hold l = 3 and l = 0, quarters 2 and 3 hold l = 1 and l = 2, two channels a lane, blocks (l, even), (l, odd),
 // (l', even), (l', odd).  Every quarter then works for eight components of two channels a lane: an edge costs 32 + 2
 // wavefronts of Y instead of 64.
+//
+// A set's loader has to keep up with four consumer warps: its part of the list is in registers a tile ahead, a lane's rows are
+// its own (a shuffle per row: 112 cycles a copy instead of about 30), and the MMAs come from one thread that asks its barriers
+// itself.  340 -> 258 us at 16 000 atoms (832 000 edges), 1 355 -> 1 011 at 64 000, 78 -> 64 at 3 000.  What bounds it now: a
+// set's products and sums take turns on one accumulator buffer (250 us remain without the products, measured before).
 #include "common.cuh"
 #include "step_common.cuh"
 #include "tc_ptx.cuh"
@@ -93,20 +98,6 @@ __device__ __forceinline__ void issue_tile(uint32_t tmem, uint32_t acc, uint32_t
       umma_f16_ts(d, a + 32u + 8u * k, b_hi + (uint64_t)(2 * k), idesc, 1);
     }
   }
-}
-
-// a row of X (512 bytes) for every lane's sender index s, rows i = 0 .. N - 1: one 16-byte asynchronous copy a lane each;
-// the 32 lanes' arrivals on bar follow their copies
-template <int N>
-__device__ __forceinline__ void copy_sender_rows(const float *__restrict__ X, int s, uint32_t dst, uint32_t bar, int lane) {
-#pragma unroll 8
-  for (int i = 0; i < N; i++) {
-    const int64_t row = __shfl_sync(0xffffffffu, s, i);
-    asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(dst + (uint32_t)i * 512u + 16u * lane),
-                 "l"(X + row * FM_C + 4 * lane)
-                 : "memory");
-  }
-  asm volatile("cp.async.mbarrier.arrive.noinc.shared::cta.b64 [%0];" ::"r"(bar) : "memory");
 }
 
 // ---- forward --------------------------------------------------------------------------------------------------------
@@ -265,23 +256,38 @@ __global__ void __launch_bounds__(FM_THREADS, 1)
   };
 
   if (warp >= 10) {
-    // ---- loader: h rows by TMA, Y rows as one bulk copy, sender rows by asynchronous copies
+    // ---- loader: h rows by TMA, Y rows as one bulk copy, sender rows by asynchronous copies (lane: rows lane / 4 + 8 i, of
+    // every 64 bytes the 16 at lane % 4); the next tile's part of the list is on its way meanwhile
+    const int rr = lane >> 2;
+    int send[4], r = 0, rn = 0;
+    auto load_list = [&](int64_t t) {
+      const int64_t base = e0 + t * FF_TILE;
+      auto at = [&](int64_t e) { return e < e1 ? e : e1 - 1; };
+#pragma unroll
+      for (int i = 0; i < 4; i++) send[i] = __ldg(g.sender + at(base + rr + 8 * i));
+      r = __ldg(g.receiver + at(base + lane));
+      rn = base + lane + 1 < e1 ? __ldg(g.receiver + base + lane + 1) : -1;
+    };
+    if (ntiles > 0) load_list(0);
     for (int64_t t = 0; t < ntiles; t++) {
-      if (!warp_wait(st_free + 8u * stage, phase ^ 1, lane)) {
+      const int64_t base = e0 + t * FF_TILE;
+      const unsigned last = __ballot_sync(0xffffffffu, base + lane < e1 && rn != r);
+      const int receiver = r;
+      const float *src[4];
+#pragma unroll
+      for (int i = 0; i < 4; i++) src[i] = g.X + (int64_t)send[i] * FM_C + 4 * (lane & 3);
+      if (t + 1 < ntiles) load_list(t + 1);
+      if (!warp_wait_all(st_free + 8u * stage, phase ^ 1, lane)) {
         if (lane == 0 && g.status) atomicCAS(g.status, 0, 41);
         break;
       }
-      const int64_t base = e0 + t * FF_TILE, e = base + lane < e1 ? base + lane : e1 - 1;
       const uint32_t sX = stages + (uint32_t)stage * FF_STAGE_BYTES, sH = sX + FF_X_BYTES, sY = sH + FF_H_BYTES;
       if (elect_one()) {
         mbar_arrive_expect_tx(h_full + 8u * stage, FF_H_BYTES);
         tma_load_2d(sH, &h_map, 0, (int)base, h_full + 8u * stage);
         tma_load_2d(sH + FF_H_BYTES / 2, &h_map, 64, (int)base, h_full + 8u * stage);
       }
-      const int s = g.sender[e], r = g.receiver[e];
-      const int rn = base + lane + 1 < e1 ? g.receiver[base + lane + 1] : -1;
-      const unsigned last = __ballot_sync(0xffffffffu, base + lane < e1 && rn != r);
-      recv_s[set][stage][lane] = r;
+      recv_s[set][stage][lane] = receiver;
       if (lane == 0) last_s[set][stage] = last;
       __syncwarp();
       if (elect_one()) {
@@ -289,25 +295,31 @@ __global__ void __launch_bounds__(FM_THREADS, 1)
         mbar_arrive_expect_tx(x_full + 8u * stage, bytes);
         bulk_copy_g2s(sY, g.Y + base * 16, bytes, x_full + 8u * stage);
       }
-      copy_sender_rows<FF_TILE>(g.X, s, sX, x_full + 8u * stage, lane);
+      const uint32_t dst = sX + 512u * (uint32_t)rr + 16u * (uint32_t)(lane & 3);
+#pragma unroll
+      for (int k = 0; k < 8; k++)
+#pragma unroll
+        for (int i = 0; i < 4; i++)
+          asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(dst + 4096u * i + 64u * k), "l"(src[i] + 16 * k) : "memory");
+      asm volatile("cp.async.mbarrier.arrive.noinc.shared::cta.b64 [%0];" ::"r"(x_full + 8u * stage) : "memory");
       advance();
     }
     asm volatile("cp.async.wait_all;" ::: "memory");
   } else if (warp >= 8) {
-    // ---- MMA issuer
-    for (int64_t t = 0; t < ntiles; t++) {
-      if (!warp_wait(acc_free, ((uint32_t)t & 1u) ^ 1u, lane) || !warp_wait(h_full + 8u * stage, phase, lane)) {
-        if (lane == 0 && g.status) atomicCAS(g.status, 0, 42);
-        break;
-      }
-      if (elect_one()) {
+    // ---- MMA issuer, one thread
+    if (elect_one()) {
+      bool ok = true;
+      for (int64_t t = 0; t < ntiles; t++) {
+        ok = mbar_wait(h_full + 8u * stage, phase) && mbar_wait(acc_free, ((uint32_t)t & 1u) ^ 1u);
+        if (!ok) break;
         tc_fence_after();
         issue_tile(tmem, acc_t, stages + (uint32_t)stage * FF_STAGE_BYTES + FF_X_BYTES, FF_H_BYTES / 2);
         umma_commit(acc_full);
+        advance();
       }
-      __syncwarp();
-      advance();
+      if (!ok && g.status) atomicCAS(g.status, 0, 42);
     }
+    __syncwarp();
   } else {
     // ---- consumers
     const int q = warp & 3;
@@ -325,7 +337,7 @@ __global__ void __launch_bounds__(FM_THREADS, 1)
 #pragma unroll
     for (int m = 0; m < 16; m++) acc[m] = 0.f;
     for (int64_t t = 0; t < ntiles; t++) {
-      if (!warp_wait(x_full + 8u * stage, phase, lane) || !warp_wait(acc_full, (uint32_t)t & 1u, lane)) {
+      if (!warp_wait_all(x_full + 8u * stage, phase, lane) || !warp_wait_all(acc_full, (uint32_t)t & 1u, lane)) {
         if (lane == 0 && g.status) atomicCAS(g.status, 0, 43);
         break;
       }
