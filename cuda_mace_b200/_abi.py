@@ -14,12 +14,15 @@ _I = ctypes.c_int
 _L = ctypes.c_int64
 _D = ctypes.c_double
 
+FUSED_LAYOUT = 2   # CMACE_FUSED_LAYOUT of the header
+
+
 class StepModel(ctypes.Structure):
     """cmace_step_model of the header: constant weights of one model."""
     _fields_ = [(k, ctypes.c_int32) for k in ("is_f64", "channels", "elements", "nbessel", "cutoff_p", "reserved")] + [
         ("r_max", _D), ("scale", _D), ("shift", _D), ("radial", (_P * 4) * 2), ("radial_half", (_P * 3) * 2),
         ("half_scales", (ctypes.c_float * 13) * 2), ("fused_w", _P), ("fused_w_back", _P), ("fused_scale", ctypes.c_float),
-        ("reserved2", ctypes.c_float), ("radial_back", _P), ("spline", _P * 2), ("spline_knots", _P), ("sender_table", _P), ("spline_width", _D),
+        ("fused_layout", ctypes.c_int32), ("radial_back", _P), ("spline", _P * 2), ("spline_knots", _P), ("sender_table", _P), ("spline_width", _D),
         ("spline_rmax", _D), ("spline_intervals", ctypes.c_int32), ("reserved3", ctypes.c_int32), ("fold", _P),
         ("fold_back", _P * 8), ("linear", _P * 2), ("weff", _P * 2)] + [
         (k, _P) for k in ("up", "up_back", "extra", "extra_back", "readout1", "readout2", "atomic_energies")]

@@ -61,9 +61,11 @@ static const char *const kStepNames[S_COUNT] = {
     "radial_out", "messages", "linear", "contract1", "linear_back", "edges_back", "radial_back", "senders",
     "mid_back", "contract0_back", "fold_back", "sums_back", "forces"};
 
-// second layer with the radial weights formed inside its kernels: fp16 pairs of h, 128 channels (fused_messages.cu)
 static bool is_spline(const cmace_step_model &m) { return m.spline[0] != nullptr; }
-static bool is_fused(const cmace_step_model &m) { return !is_spline(m) && !m.is_f64 && m.fused_w != nullptr && m.channels == 128; }
+// second layer with the radial weights formed inside its kernels: fp16 pairs of h, 128 channels (fused_messages.cu)
+static bool is_fused(const cmace_step_model &m) {
+  return !is_spline(m) && !m.is_f64 && m.fused_w != nullptr && m.fused_layout == CMACE_FUSED_LAYOUT && m.channels == 128;
+}
 
 template <typename T>
 struct Workspace {
@@ -190,8 +192,15 @@ static int run_step(const cmace_step_model &m, cmace_step_io &io, const Workspac
   // float32 with radial layers whose values are bounded inside fp16's range: h and h' of the first layer are fp16 pairs
   static_assert(sizeof(RadialScales) == sizeof(m.half_scales[0]), "RadialScales is the header's array");
   const bool half = !f64 && m.radial_half[0][0] != nullptr;
-  const RadialScales *scales = reinterpret_cast<const RadialScales *>(m.half_scales);
   const bool fused = is_fused(m);
+  RadialScales scales[2];
+  memcpy(scales, m.half_scales, sizeof(scales));
+  if (!fused) {   // the second layer's h and h' leave as float32, without the scale of the pairs
+    RadialScales &s = scales[1];
+    s.a[2] *= s.out_v;
+    s.t[2] *= s.out_t;
+    s.out_v = s.out_t = 1.f;
+  }
   if (fused && (step == S_RADIAL_OUT || step == S_RADIAL_BACK)) return CMACE_OK;
   io.launches++;
   if (step == S_EDGE_PREP && node_blocks(io.n_local) > 1) io.launches++;

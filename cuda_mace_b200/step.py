@@ -288,7 +288,7 @@ class StepPlan:
                     w = w * scale
                     hi = w.half()
                     m.fused_w = hold(torch.cat([hi, (w - hi.float()).half()], dim=1))
-                    m.fused_scale = 1.0 / scale
+                    m.fused_scale, m.fused_layout = 1.0 / scale, _abi.FUSED_LAYOUT
                     # [step of 16 channels, (l, j, t, i), k]: row 8 j + 2 t + i of a degree is channel 4 t + 2 j + i of the step
                     wt = L1.W_radial3.t().reshape(4, 8, 4, 2, 2, _H).permute(1, 0, 3, 2, 4, 5).reshape(8, 64, _H)
                     m.fused_w_back = hold(torch.stack([half_images(b, scale) for b in wt]))

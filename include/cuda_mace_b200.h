@@ -364,6 +364,7 @@ int cmace_symcon_effective_weights(const cmace_symcon_plan *plan, int is_f64, co
  * kernel launches with its gradient written out: no autograd graph, no allocation, no synchronisation.  The caller
  * owns weights, workspace and outputs.  csrc/step.cu documents the sequence; steps can be run in ranges, which is
  * where a decomposed system exchanges node features (after "mid_fwd") and their gradients (after "senders"). */
+#define CMACE_FUSED_LAYOUT 2 /* names the layouts of fused_w and fused_w_back below; changes with them */
 typedef struct cmace_step_model {
   int32_t is_f64, channels, elements, nbessel, cutoff_p, reserved;
   double r_max, scale, shift;
@@ -377,7 +378,10 @@ typedef struct cmace_step_model {
                                 channel 64 (q & 1) + 2 i + (j & 1), divided by fused_scale (a power of two) */
   const void *fused_w_back;  /* the same W4^T for the backward: [8 steps of 16 channels][hi, lo][64 rows x 128 bytes], 128-byte
                                 swizzle; row 16 l + 8 j + 2 t + i is degree l, channel 4 t + 2 j + i of the step */
-  float fused_scale, reserved2;
+  float fused_scale;
+  int32_t fused_layout;      /* CMACE_FUSED_LAYOUT.  With any other value, such as the 0 of a caller that lays fused_w_back out as
+                                earlier libraries read it (steps of 8 channels), neither array is read and the second layer's
+                                radial weights are written, as for other numbers of channels */
   const void *radial_back;   /* second layer's W4 for the gradient: float32 packed W4 itself, float64 W4^T [4C,64] */
   const void *spline[2];     /* tabulated radial weights: coefficients [intervals][4][4C] of both layers, or NULL; then the
                                 radial weights above are not read, fold is the first layer's Linear [elements][4] [C, C]

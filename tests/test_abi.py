@@ -35,6 +35,19 @@ def test_version_and_queries_need_no_gpu(built_library):
     assert _abi.call("cmace_imp_bwd_scratch_elems", 1000, 96, 0) == 3 * 16 * 1000   # f32, three 32-channel chunks
 
 
+def test_fused_layout_of_earlier_callers_is_not_read(built_library):
+    """A caller that lays fused_w_back out as earlier libraries read it leaves the word after fused_scale 0: its second layer
+    writes the radial weights, which the workspace then has room for."""
+    header = open(os.path.join(ROOT, "include", "cuda_mace_b200.h")).read()
+    assert int(re.search(r"#define CMACE_FUSED_LAYOUT (\d+)", header).group(1)) == _abi.FUSED_LAYOUT
+    m = _abi.StepModel(channels=128, elements=2, nbessel=8, fused_w=1, fused_w_back=1, fused_layout=_abi.FUSED_LAYOUT)
+    E = 1024
+    size = lambda: _abi.call("cmace_step_workspace_bytes", ctypes.byref(m), 10, 10, E)
+    fused = size()
+    m.fused_layout = 0
+    assert size() == fused + E * 4 * 128 * 4
+
+
 def test_argument_errors_are_reported_not_raised(built_library):
     lib = _abi.load()
     rc = lib.cmace_imp_fwd_f32(None, None, None, None, None, 4, 4, 33, None, None)

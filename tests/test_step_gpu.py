@@ -138,6 +138,23 @@ def _small(U, dtype=torch.float64, n=12, C=32, Z=3, **more):
     return mace, data
 
 
+# a caller of the C interface that lays fused_w_back out as earlier libraries read it, steps of 8 channels, without the word
+# that names the layout: right forces, from the radial weights in memory.  Bounds of a float32 step
+def test_a_layout_of_earlier_callers_gives_the_same_forces(U):
+    mace, data = _small(U, torch.float32, n=70, C=128)
+    ref = mace(data)
+    plan = step.plan_of(mace)
+    w = mace.layers[1].W_radial3.t()
+    old = w.reshape(4, 16, 8, 64).transpose(0, 1).reshape(16, 32, 64)
+    old = torch.stack([step.half_images(b, 1.0 / plan.model.fused_scale) for b in old]).contiguous()
+    plan.model.fused_w_back, plan.model.fused_layout = old.data_ptr(), 0
+    out = mace(data)
+    assert mace.__dict__["_step_plan"][1] is plan
+    scale = float(ref["forces"].abs().max())
+    assert float((out["forces"] - ref["forces"]).abs().max()) < 1e-4 * scale
+    assert abs(float(out["interaction_energy"] - ref["interaction_energy"])) < 1e-5 * abs(float(ref["interaction_energy"]))
+
+
 # nothing of these calls is launched: the checks come first
 @pytest.mark.parametrize("species,node_attrs", [
     (torch.zeros(12, dtype=torch.int32), None), (torch.zeros(11, dtype=torch.int32, device="meta"), None),
