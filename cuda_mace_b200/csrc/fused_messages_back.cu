@@ -33,7 +33,10 @@
 // on, the MMA issuer is one thread that does the same.  16 000 atoms (832 000 edges): 485 -> 417 us, 64 000: 2 040 -> 1 700,
 // 3 000: 102 -> 88.  What bounds it: instruction issue (59 %) and the latency of a step's chain, accumulators to registers,
 // G, sums, with two warps a scheduler; without the sums 312 us are left, without the products as well 257.
+#include <atomic>
+
 #include "common.cuh"
+#include "register_split.hpp"
 #include "step_common.cuh"
 #include "tc_ptx.cuh"
 
@@ -44,7 +47,10 @@ constexpr int EB_C = 128;
 constexpr int EB_STEP = 16;                       // channels of a step
 constexpr int EB_NSTEP = EB_C / EB_STEP;
 constexpr int EB_THREADS = 512;
-constexpr int EB_REGS = 184, EB_REGS_OTHER = 72;   // (184 + 72) * 256 = 128 * 512: what the block is launched with
+constexpr int EB_REGS = 184, EB_REGS_OTHER = 72;
+// 128 registers are the most that 512 threads can have, and what ptxas gives a kernel with these bounds and setmaxnreg (also
+// without optimisation and under -maxrregcount); the launch asks, since a block that started with fewer would wait for good
+static_assert(register_split_fits(65536 / EB_THREADS, EB_THREADS, EB_REGS, EB_REGS_OTHER), "register split");
 constexpr int EB_W_BYTES = 2 * 64 * 128;          // hi and lo image of a step's W: 64 rows (l, channel)
 constexpr int EB_W_SLOTS = 3;
 constexpr int EB_X_BYTES = EB_TILE * EB_STEP * 4;
@@ -522,7 +528,18 @@ int fused_messages_back(const float *X, const float *Y, const float *G, const vo
   if (ntiles * EB_TILE > 0x7fffffffLL) return fail(CMACE_ERR_UNSUPPORTED, "%s: too many edges", what);
   const EdgeBackArgs g{X, Y, G, static_cast<const char *>(h), static_cast<const char *>(dh), static_cast<const char *>(W),
                        sender, receiver, status, nedges, factor_v, factor_t, T, gY};
-  cudaError_t e = cudaFuncSetAttribute(edge_back_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, EB_SMEM);
+  static std::atomic<int> compiled_regs{0};   // a property of the binary
+  int regs = compiled_regs.load(std::memory_order_relaxed);
+  cudaError_t e = cudaSuccess;
+  if (regs == 0) {
+    cudaFuncAttributes attr;
+    e = cudaFuncGetAttributes(&attr, edge_back_kernel);
+    if (e != cudaSuccess) return fail(CMACE_ERR_CUDA, "%s: %s", what, cudaGetErrorString(e));
+    compiled_regs.store(regs = attr.numRegs, std::memory_order_relaxed);
+  }
+  if (!register_split_fits(regs, EB_THREADS, EB_REGS, EB_REGS_OTHER))
+    return fail(CMACE_ERR_UNSUPPORTED, "%s: compiled with %d registers a thread, too few for its register split", what, regs);
+  e = cudaFuncSetAttribute(edge_back_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, EB_SMEM);
   if (e != cudaSuccess) return fail(CMACE_ERR_CUDA, "%s: %s", what, cudaGetErrorString(e));
   launch_chained(edge_back_kernel, (unsigned)(ntiles < 148 ? ntiles : 148), EB_THREADS, EB_SMEM, st, g);
   return check_launch(what);

@@ -4,6 +4,7 @@
 #include <cstdint>
 
 #include "sigmoid64.cuh"
+#include "register_split.hpp"
 #include "edge_math.cuh"   // found through -I cuda_mace_b200/csrc (tests/conftest.py builds this file)
 
 using namespace cmace;
@@ -13,6 +14,9 @@ void hc_sigmoid_f64(const double *z, int64_t n, double *s) {
   double etab[32];
   for (int j = 0; j < 32; j++) etab[j] = std::exp2(j / 32.0);
   for (int64_t i = 0; i < n; i++) s[i] = table_sigmoid(z[i], etab);
+}
+int hc_register_split_fits(int regs, int threads, int first_half, int second_half) {
+  return register_split_fits(regs, threads, first_half, second_half);
 }
 void hc_edge_basis_fwd_f64(const double *xyz, int64_t E, double r_max, int nb, int p, double *Y, double *B) {
   for (int64_t e = 0; e < E; e++) {

@@ -27,6 +27,12 @@ def edges(seed, n):
     return v * rng.uniform(0.6, 5.4, size=(n, 1))  # a few beyond the 5.0 cutoff
 
 
+# the split of the backward of the fused messages: what 512 threads have at most, one register less, a smaller first half
+@pytest.mark.parametrize("regs,first,second,fits", [(128, 184, 72, 1), (127, 184, 72, 0), (128, 192, 72, 0), (127, 176, 72, 1)])
+def test_register_split_needs_what_the_block_starts_with(hc, regs, first, second, fits):
+    assert hc.hc_register_split_fits(regs, 512, first, second) == fits
+
+
 def test_table_sigmoid_f64(hc):
     """The float64 logistic function of the radial kernel against long double: every interval of its table, both ends of
     the exponent's range, zero, and values beyond.  Bound: half an ulp of 1 + e and of the result each, the exponential's
