@@ -55,10 +55,10 @@ constexpr int EB_W_BYTES = 2 * 64 * 128;          // hi and lo image of a step's
 constexpr int EB_W_SLOTS = 3;
 constexpr int EB_X_BYTES = EB_TILE * EB_STEP * 4;
 constexpr int EB_X_SLOTS = 5;
-// Receivers staged per tile; a warp with a further one reads G from global memory.  Six hold a tile of a condensed system: 0.50
-// ns an edge at 52 edges a receiver, 0.52 at 31, 0.88 at 21, 1.00 at 10 (416 000 edges; 0.59, 0.68, 0.97 and 1.14 with an
-// edge a lane and five).  Two buffers of more do not fit.
-constexpr int EB_G_RECV = 6;
+// Receivers staged per tile, as many as two buffers hold; a warp with a further one reads G from global memory.  Nanoseconds an
+// edge with seven and six, 413 000 edges: 0.55 and 0.55 at 52 edges a receiver, 0.52 and 0.52 at 31, 0.70 and 0.89 at 21,
+// 0.96 and 0.96 at 10, 1.05 and 1.05 at 5.
+constexpr int EB_G_RECV = 7;
 constexpr int EB_G_BYTES = EB_G_RECV * 16 * EB_C * 4;
 constexpr int EB_PIECE = 2048;                    // 32 rows x 64 bytes
 constexpr int EB_OFF_W = 0;
@@ -67,7 +67,8 @@ constexpr int EB_OFF_G = EB_OFF_X + EB_X_SLOTS * EB_X_BYTES;
 constexpr int EB_OFF_H = EB_OFF_G + 2 * EB_G_BYTES;        // eight pieces: h of the next tile on its way in, two a warp
 constexpr int EB_OFF_Y = EB_OFF_H + 8 * EB_PIECE;          // Y of the next tile, then its receivers
 constexpr int EB_SMEM = EB_OFF_Y + EB_TILE * 64 + EB_TILE * 4 + 1024;
-static_assert(EB_SMEM <= 226 * 1024, "shared memory of a block");
+constexpr int EB_SMEM_MOST = 226 * 1024;          // a block's 227 KB less its static part
+static_assert(EB_SMEM <= EB_SMEM_MOST && EB_SMEM + 2 * EB_G_BYTES / EB_G_RECV > EB_SMEM_MOST, "receivers staged: as many as fit");
 
 // Which edge of the tile a row of tensor memory and shared memory holds: rows r and r + 8 of 16 are two edges in a row, so
 // that few lanes have edges of two receivers (8 of 52 places for a receiver's end in a condensed system, 15 otherwise).
