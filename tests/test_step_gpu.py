@@ -72,32 +72,62 @@ def test_step_against_autograd(U, dtype, tol, n, C, Z, nb, radial):
     assert float((out["forces"] + g).abs().max()) < tol * float(g.abs().max())
 
 
+def _list_of(receiver, n, seed):
+    """A float32 model of 128 channels and a list with these receivers; a shift an edge gives any distance up to the cutoff."""
+    rng = np.random.default_rng(seed)
+    edges = receiver.size
+    sender = rng.integers(0, n, edges)
+    pos, shifts = rng.normal(size=(n, 3)), rng.normal(size=(edges, 3))
+    length = rng.uniform(0.9, 4.9, edges)[:, None]
+    shifts = shifts / np.linalg.norm(shifts, axis=1, keepdims=True) * length - (pos[sender] - pos[receiver])
+    return systems.init_params(128, 3, 7), pos, np.stack([receiver, sender]), shifts, rng.integers(0, 3, n)
+
+
+def _step_of(U, params, pos, ei, sh, species):
+    mace = model.InvariantMACE(params, U, dtype=torch.float32, device="cuda")
+    out = mace(dict(positions=torch.from_numpy(pos).cuda(), species=torch.from_numpy(species.astype(np.int32)).cuda(),
+                    edge_index=torch.from_numpy(ei.astype(np.int32)).cuda(), shifts=torch.from_numpy(sh).cuda()))
+    assert step.plan_of(mace).model.fused_w   # the kernels meant here
+    return out
+
+
 # the second layer's fused kernels at the edges of their tiles (32 and 128 edges) and of their pairs and groups of edges (2, 8,
 # 16): lists of so many edges with so many a receiver, and receivers without any; 40 a receiver is more than a tile of the
-# forward holds, 1 more receivers than the backward stages.  The model's own autograd path is the reference, the bounds are
-# those of the whole step above.
-@pytest.mark.parametrize("edges", [1, 9, 127, 128, 129, 300])
-@pytest.mark.parametrize("degree", [1, 2, 3, 17, 40])
+# forward holds, 1 more receivers than the backward stages.  Energy and forces against the oracle, with the bounds of the
+# whole step above; a list shorter than its degree is that of any larger one.
+@pytest.mark.parametrize("edges,degree", [(1, 1)] + [(9, d) for d in (1, 2, 3, 17)] +
+                         [(e, d) for e in (127, 128, 129, 300) for d in (1, 2, 3, 17, 40)])
 def test_second_layer_at_tile_edges(U, edges, degree):
-    rng = np.random.default_rng(edges * 50 + degree)
     n = -(-edges // degree) + 2
     receiver = np.minimum(np.arange(edges) // degree, n - 1)
     receiver[receiver > 0] += 1          # receiver 1 and the last one have no edges
-    sender = rng.integers(0, n, edges)
-    pos, shifts = rng.normal(size=(n, 3)), rng.normal(size=(edges, 3))   # a shift an edge: any distance up to the cutoff
-    length = rng.uniform(0.9, 4.9, edges)[:, None]
-    shifts = shifts / np.linalg.norm(shifts, axis=1, keepdims=True) * length - (pos[sender] - pos[receiver])
-    mace = model.InvariantMACE(systems.init_params(128, 3, 7), U, dtype=torch.float32, device="cuda")
-    p, species = torch.from_numpy(pos).cuda(), torch.from_numpy(rng.integers(0, 3, n).astype(np.int32)).cuda()
-    ei, sh = torch.from_numpy(np.stack([receiver, sender]).astype(np.int32)).cuda(), torch.from_numpy(shifts).cuda()
-    out = mace(dict(positions=p, species=species, edge_index=ei, shifts=sh))
-    assert step.plan_of(mace) is not None
-    p.requires_grad_(True)
-    energies = mace.node_energies(p, species, ei, sh)
+    params, pos, ei, sh, species = _list_of(receiver, n, edges * 50 + degree)
+    out = _step_of(U, params, pos, ei, sh, species)
+    _, e_ref, f_ref = omodel.energy_and_forces(params, U, torch.from_numpy(pos), systems.one_hot(species, 3),
+                                               torch.from_numpy(ei), torch.from_numpy(sh))
+    assert abs(float(out["interaction_energy"]) - float(e_ref)) < 1e-5 * max(abs(float(e_ref)), 1e-3)
+    assert float((out["forces"].cpu() - f_ref).abs().max()) < 1e-4 * max(float(f_ref.abs().max()), 1e-6)
+
+
+# Four and five tiles of the backward a block on 148 blocks, eight and nine of the forward a set: every buffer and barrier is
+# used again, its phase wraps.  Receivers of so many edges in turn: few (warps whose receivers are not staged beside those
+# whose are), and a long one before many short ones.  Against the operators in float64 (the oracle's contraction of so many
+# nodes takes 60 GB), same bounds.
+@pytest.mark.parametrize("degrees", [(3,), (10,), (70,) + (1,) * 40])
+def test_second_layer_over_many_tiles(U, degrees):
+    edges = 80_001
+    receiver = np.repeat(np.arange(edges), np.resize(degrees, edges))[:edges]
+    n = int(receiver[-1]) + 1
+    params, pos, ei, sh, species = _list_of(receiver, n, len(degrees))
+    out = _step_of(U, params, pos, ei, sh, species)
+    mace = model.InvariantMACE(params, U, dtype=torch.float64, device="cuda")
+    p = torch.from_numpy(pos).cuda().requires_grad_(True)
+    energies = mace.node_energies(p, torch.from_numpy(species.astype(np.int32)).cuda(),
+                                  torch.from_numpy(ei.astype(np.int32)).cuda(), torch.from_numpy(sh).cuda())
     (g,) = torch.autograd.grad(energies.sum(), p)
     energies = energies.detach()
-    assert abs(float(out["interaction_energy"].double() - energies.sum())) < 1e-5 * max(float(energies.abs().sum()), 1e-3)
-    assert float((out["forces"] + g).abs().max()) < 1e-4 * max(float(g.abs().max()), 1e-6)
+    assert abs(float(out["interaction_energy"] - energies.sum())) < 1e-5 * float(energies.abs().sum())
+    assert float((out["forces"] + g).abs().max()) < 1e-4 * float(g.abs().max())
 
 
 # below and above the 32 768 edges from which a new list's grouping by sender runs beside the step
