@@ -185,17 +185,6 @@ __device__ __forceinline__ unsigned long long sub2(unsigned long long a, unsigne
   return r;
 }
 
-// 32 bytes of one lane in one store.  The lanes of a result tile hold 64 bytes of a row each: in 16-byte stores every
-// instruction half-fills 32 sectors, which L2 takes as 2.5 times the writes (10.2 million sectors for 131 MB).
-__device__ __forceinline__ void store32(float *p, float a, float b, float c, float d, float e, float f, float g, float h) {
-  asm volatile("st.global.v8.f32 [%0], {%1, %2, %3, %4, %5, %6, %7, %8};" ::"l"(p), "f"(a), "f"(b), "f"(c), "f"(d), "f"(e),
-               "f"(f), "f"(g), "f"(h)
-               : "memory");
-}
-__device__ __forceinline__ void store32(double *p, double a, double b, double c, double d) {
-  asm volatile("st.global.v4.f64 [%0], {%1, %2, %3, %4};" ::"l"(p), "d"(a), "d"(b), "d"(c), "d"(d) : "memory");
-}
-
 // channels handled per lane: the widest 16-byte-or-narrower vector that tiles C in 32-lane chunks
 // The 16 harmonics of a pair of edges, lane (16 h + m) -> component m of edge h, handed to all lanes through shared memory:
 // a broadcast load gives 16 bytes, a shuffle (two of them in float64) one value.  Two buffers, so that one warp barrier a
