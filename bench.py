@@ -172,14 +172,14 @@ def algorithmic_bytes(name, s, N, Ns, E, C, Z):
 # moves this many bytes times its own E.
 _SRC = "profiles/step_sequence_8000_f32.txt"
 NCU_TRAFFIC_PER_EDGE = {
-    "step[edges_back]": (1232.0, _SRC),
-    "step[messages]": (426.0, _SRC),
-    "step[radial]": (937.0, _SRC),
-    "step[sums_back]": (988.0, _SRC),
+    "step[edges_back]": (1240.0, _SRC),
+    "step[messages]": (434.0, _SRC),
+    "step[radial]": (943.0, _SRC),
+    "step[sums_back]": (996.0, _SRC),
 }
 # warps a scheduler and issue slots used while active, from the same capture
 ISSUE_NOTE = {step: f", on {warps} warps a scheduler (issue slots {slots} % used in the ncu capture {_SRC})"
-              for step, warps, slots in (("step[edges_back]", 4, 59), ("step[messages]", 3, 42), ("step[radial]", 4, 51))}
+              for step, warps, slots in (("step[edges_back]", 4, 59), ("step[messages]", 3, 43), ("step[radial]", 4, 51))}
 
 
 def tensor_flops(name, s, E, C):
