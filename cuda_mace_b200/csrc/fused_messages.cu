@@ -18,8 +18,13 @@
 //
 // A set's loader has to keep up with four consumer warps: its part of the list is in registers a tile ahead, a lane's rows are
 // its own (a shuffle per row: 112 cycles a copy instead of about 30), and the MMAs come from one thread that asks its barriers
-// itself.  340 -> 258 us at 16 000 atoms (832 000 edges), 1 355 -> 1 011 at 64 000, 78 -> 64 at 3 000.  What bounds it now: a
-// set's products and sums take turns on one accumulator buffer (250 us remain without the products, measured before).
+// itself.  317 -> 254 us at 16 000 atoms (833 000 edges), 1 320 -> 1 046 at 64 000, 80 -> 66 at 3 000, 264 -> 240 for 412 000
+// edges of 4 a receiver, 294 -> 300 of 3 (events around the kernel, both in one run).  One copy instruction writes 64 bytes of
+// eight rows, all on the same 16 banks, eight wavefronts instead of four; without that conflict (128 bytes of four rows) the
+// kernel takes the same at 16 000 atoms, with the 64 bytes rotated by the row 259 us.
+//
+// What bounds it now: a set's products and sums take turns on one accumulator buffer.  Of 254 us at 16 000 atoms 182 remain
+// without the products, 125 without the sums, 86 without both; of 1 046 at 64 000 744, 500 and 297.
 #include "common.cuh"
 #include "step_common.cuh"
 #include "tc_ptx.cuh"

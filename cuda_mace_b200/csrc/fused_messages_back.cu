@@ -15,8 +15,8 @@
 //
 // A consumer warp has 16 edges and all channels: lane (g, t) holds two edges and four channels of a step, which is what
 // tcgen05.ld.16x256b hands out (column 8 j + 2 t + i of a degree is channel 4 t + 2 j + i of the step).  Every word of G
-// that a lane reads serves two edges; with an edge a lane and eight channels a step the same sums read twice the words, and
-// shared memory's 2 048 words an edge bound the kernel (128 bytes a cycle: 64 of 120 cycles an edge).
+// that a lane reads serves two edges; with an edge a lane and eight channels a step the same sums read twice the words, 2 048 an
+// edge (128 bytes a cycle: 64 of the 158 cycles an edge took).
 //
 //   warps 0-7    consumers: warp w the rows 32 (w % 4) + 16 (w / 4) .. of the tile
 //   warp 8       issues the MMAs
@@ -30,9 +30,10 @@
 // What the consumers do besides the sums is kept short, since two warps a scheduler hide little of it: h, h', Y and G are
 // brought by other warps (consumers doing it themselves: 150 of 890 thousand cycles at 16 000 atoms), T goes out in 64-byte
 // pieces from registers instead of through shared memory, a step's barriers are asked for while the step before it is worked
-// on, the MMA issuer is one thread that does the same.  16 000 atoms (832 000 edges): 485 -> 417 us, 64 000: 2 040 -> 1 700,
-// 3 000: 102 -> 88.  What bounds it: instruction issue (59 %) and the latency of a step's chain, accumulators to registers,
-// G, sums, with two warps a scheduler; without the sums 312 us are left, without the products as well 257.
+// on, the MMA issuer is one thread that does the same.  With the words of G halved 16 000 atoms (833 000 edges) take 471 -> 411 us,
+// 64 000 2 000 -> 1 700, 3 000 107 -> 92 (events around the kernel, both in one run).  What bounds it: instruction issue (59 %) and
+// the latency of a step's chain, accumulators to registers, G, sums, with two warps a scheduler; of 417 us 312 are left without
+// the sums, 257 without the products as well.
 #include <atomic>
 
 #include "common.cuh"

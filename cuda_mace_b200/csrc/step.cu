@@ -300,11 +300,12 @@ static int run_step(const cmace_step_model &m, cmace_step_io &io, const Workspac
   return fail(CMACE_ERR_ARG, "cmace_step: no step %d", step);
 }
 
-// Programmatic launches while launch latency shows between the kernels: 163 -> 119 us a step at 5 000 edges, 277 -> 246 at
-// 52 000; float32 also 503 -> 473 at 157 000, 728 -> 700 at 261 000 and 961 -> 949 at 366 000.  A recorded step has no such
-// gaps beyond 98 304 edges and float64 kernels are long by then: 473 -> 481 us at 157 000 recorded, 2 300 -> 2 333 in
-// float64 (the kernels keep their predecessor's split between shared memory and L1).  Tabulated radial weights live on L1:
-// half the edges (516 -> 489 us at 94 000, 709 -> 700 at 157 000, the same at 261 000).
+// Programmatic launches while launch latency shows between the kernels, us a float32 step of 128 channels without and with them:
+// 150 -> 117 at 4 700 edges, 241 -> 213 at 52 000, 477 -> 456 at 156 000, 684 -> 670 at 260 000, 903 -> 897 at 364 000, the same
+// at 417 000, 1 265 -> 1 297 at 521 000.  A recorded step has smaller gaps: 130 -> 121 at 4 700, the same at 52 000, 300 -> 305 at
+// 78 000, 336 -> 344 at 99 000, 451 -> 462 at 156 000; its line is float64's, whose kernels are long by then (2 300 -> 2 333 at
+// 156 000), because chained kernels keep their predecessor's split between shared memory and L1.  Tabulated radial weights
+// live on L1: half the edges (516 -> 489 us at 94 000, 709 -> 700 at 157 000, the same at 261 000).
 constexpr int64_t kChainEdges = 98304, kChainEdgesLive = 393216;
 
 static bool chain_for(const cmace_step_model &m, int64_t edges, cudaStream_t st) {

@@ -359,7 +359,8 @@ def pays(plan, atoms, edges, recorded=False):
     The first layer's sums and the products on them take 64 Z columns an atom whatever its edges are, the operators 4 C
     radial weights an edge.  Native against operators, ms, one B200: 100 000 atoms of 10 edges, float32, 64 channels: 5.4; 6.4
     at 4 elements, 6.8; 6.5 at 7, 8.1; 6.5 at 10, 10.8; 6.6 at 16; of 21 edges 10.2; 10.2 at 10; of 31 edges 13.7; 14.2 at
-    13; float64, 30 000 atoms of 10 edges, 128 channels: 8.4; 11.0 at 4, 10.5; 11.2 at 7, 12.6; 11.5 at 10.  The lines are
+    13; 128 channels, of 10 edges 11.65; 11.76 at 13, 12.05; 11.77
+    at 14; float64, 30 000 atoms of 10 edges, 128 channels: 8.4; 11.0 at 4, 10.5; 11.2 at 7, 12.6; 11.5 at 10.  The lines are
     where both take the same; a condensed system (52 edges) stays native up to 15 elements.  The operators' launches take the
     host 2.1 ms, which small systems never need natively (20 000 atoms of 10 edges, 16 elements, float32, 32 channels: 1.98;
     2.07); recorded, both take the same at 3 000 atoms of 16 elements in float32 (0.39; 0.40) and 1 000 in float64."""
