@@ -14,7 +14,7 @@ _I = ctypes.c_int
 _L = ctypes.c_int64
 _D = ctypes.c_double
 
-FUSED_LAYOUT = 2   # CMACE_FUSED_LAYOUT of the header
+FUSED_LAYOUT, FUSED_LAYOUT_NARROW = 2, 3   # CMACE_FUSED_LAYOUT and CMACE_FUSED_LAYOUT_NARROW of the header
 
 
 class StepModel(ctypes.Structure):

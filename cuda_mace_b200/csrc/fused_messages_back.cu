@@ -1,5 +1,5 @@
-// Backward of the second layer's message passing with the radial weights formed where they are used (float32, 128
-// channels; forward in fused_messages.cu).  With u_l[e, c] = sum_m Y[lm, e] G[i, lm, c] (G the gradient of the messages,
+// Backward of the second layer's message passing with the radial weights formed where they are used (float32; forward in
+// fused_messages.cu).  With u_l[e, c] = sum_m Y[lm, e] G[i, lm, c] (G the gradient of the messages,
 // i the receiver of edge e) an edge's results are
 //
 //   T[e, c] = sum_l R_l u_l,   grad Y[lm, e] = sum_c X R_l G[lm],   dE/dr = sum_c X sum_l R'_l u_l,
@@ -10,7 +10,7 @@
 // sums over channels cost 31 shuffles per four edges and warp, and the kernel took 5.0 ms at 64 000 atoms.)
 //
 // Tile = 128 edges in steps of 16 channels.  A operand: h and h' (hi, lo fp16), 128 columns of tensor memory, two buffers.
-// B operand: 16 KB of W per step, streamed from L2 (every CTA reads the same 128 KB).  An accumulator buffer holds 64 (R,
+// B operand: 16 KB of W per step, streamed from L2 (every CTA reads the same C KB).  An accumulator buffer holds 64 (R,
 // four l) + 64 (R') columns; two buffers, so that the next step's products run while a step is worked on.
 //
 // A consumer warp has 16 edges and all channels: lane (g, t) holds two edges and four channels of a step, which is what
@@ -34,6 +34,9 @@
 // 64 000 2 000 -> 1 700, 3 000 107 -> 92 (events around the kernel, both in one run).  What bounds it: instruction issue (59 %) and
 // the latency of a step's chain, accumulators to registers, G, sums, with two warps a scheduler; of 417 us 312 are left without
 // the sums, 257 without the products as well.
+//
+// Fewer channels are fewer steps a tile.  Edge pass on written weights and the product for dE/dr together -> this kernel, us at
+// 16 000 atoms: 564 -> 199 at 32 channels, 722 -> 244 at 64, 1 446 -> 330 at 96; 3 000 atoms: 148 -> 46, 178 -> 58, 315 -> 74.
 #include <atomic>
 
 #include "common.cuh"
@@ -44,9 +47,7 @@
 namespace cmace {
 
 constexpr int EB_TILE = 128;
-constexpr int EB_C = 128;
 constexpr int EB_STEP = 16;                       // channels of a step
-constexpr int EB_NSTEP = EB_C / EB_STEP;
 constexpr int EB_THREADS = 512;
 constexpr int EB_REGS = 184, EB_REGS_OTHER = 72;
 // 128 registers are the most that 512 threads can have, and what ptxas gives a kernel with these bounds and setmaxnreg (also
@@ -56,34 +57,41 @@ constexpr int EB_W_BYTES = 2 * 64 * 128;          // hi and lo image of a step's
 constexpr int EB_W_SLOTS = 3;
 constexpr int EB_X_BYTES = EB_TILE * EB_STEP * 4;
 constexpr int EB_X_SLOTS = 5;
-// Receivers staged per tile, as many as two buffers hold; a warp with a further one reads G from global memory.  Nanoseconds an
-// edge with seven and six, 413 000 edges: 0.55 and 0.55 at 52 edges a receiver, 0.52 and 0.52 at 31, 0.70 and 0.89 at 21,
-// 0.96 and 0.96 at 10, 1.05 and 1.05 at 5.
-constexpr int EB_G_RECV = 7;
-constexpr int EB_G_BYTES = EB_G_RECV * 16 * EB_C * 4;
 constexpr int EB_PIECE = 2048;                    // 32 rows x 64 bytes
-constexpr int EB_OFF_W = 0;
-constexpr int EB_OFF_X = EB_OFF_W + EB_W_SLOTS * EB_W_BYTES;
-constexpr int EB_OFF_G = EB_OFF_X + EB_X_SLOTS * EB_X_BYTES;
-constexpr int EB_OFF_H = EB_OFF_G + 2 * EB_G_BYTES;        // eight pieces: h of the next tile on its way in, two a warp
-constexpr int EB_OFF_Y = EB_OFF_H + 8 * EB_PIECE;          // Y of the next tile, then its receivers
-constexpr int EB_SMEM = EB_OFF_Y + EB_TILE * 64 + EB_TILE * 4 + 1024;
 constexpr int EB_SMEM_MOST = 226 * 1024;          // a block's 227 KB less its static part
-static_assert(EB_SMEM <= EB_SMEM_MOST && EB_SMEM + 2 * EB_G_BYTES / EB_G_RECV > EB_SMEM_MOST, "receivers staged: as many as fit");
+
+template <int C>
+struct EdgeBackShape {
+  static constexpr int NSTEP = C / EB_STEP;
+  static constexpr int G_ROW = 16 * C * 4;        // gradient of a receiver's messages
+  static constexpr int OFF_W = 0;
+  static constexpr int OFF_X = OFF_W + EB_W_SLOTS * EB_W_BYTES;
+  static constexpr int OFF_H = OFF_X + EB_X_SLOTS * EB_X_BYTES;   // eight pieces: h of the next tile on its way in, two a warp
+  static constexpr int OFF_Y = OFF_H + 8 * EB_PIECE;              // Y of the next tile, then its receivers
+  static constexpr int OFF_G = OFF_Y + EB_TILE * 64 + EB_TILE * 4;
+  // Receivers staged per tile, as many as two buffers hold; a warp with a further one reads G from global memory.  Nanoseconds
+  // an edge with seven and six, 413 000 edges, 128 channels: 0.55 and 0.55 at 52 edges a receiver, 0.52 and 0.52 at 31, 0.70 and
+  // 0.89 at 21, 0.96 and 0.96 at 10, 1.05 and 1.05 at 5.
+  static constexpr int RECV = (EB_SMEM_MOST - 1024 - OFF_G) / (2 * G_ROW);
+  static constexpr int G_BYTES = RECV * G_ROW;
+  static constexpr int SMEM = OFF_G + 2 * G_BYTES + 1024;
+  static_assert(SMEM <= EB_SMEM_MOST && RECV >= 7, "receivers staged: as many as fit");
+  static_assert(OFF_G % 16 == 0, "bulk copies");
+};
 
 // Which edge of the tile a row of tensor memory and shared memory holds: rows r and r + 8 of 16 are two edges in a row, so
 // that few lanes have edges of two receivers (8 of 52 places for a receiver's end in a condensed system, 15 otherwise).
 __device__ __forceinline__ int eb_edge(int row) { return (row & ~15) + 2 * (row & 7) + ((row >> 3) & 1); }
 
 struct EdgeBackArgs {
-  const float *X, *Y, *G;        // [Ns, 128], [E, 16], [nnodes, 16, 128]
+  const float *X, *Y, *G;        // [Ns, C], [E, 16], [nnodes, 16, C]
   const char *h, *dh;            // [E rounded up to a tile][hi 64 | lo 64] fp16
-  const char *W;                 // [8 steps][hi, lo][64 rows x 128 B, swizzled]
+  const char *W;                 // [C / 16 steps][hi, lo][64 rows x 128 B, swizzled]
   const int32_t *sender, *receiver;
   int32_t *status;
   int64_t nedges;
   float factor_v, factor_t;      // undo the powers of two of h W and h' W
-  float *T;                      // [E, 128]
+  float *T;                      // [E, C]
   float *gY;                     // [E, 16]; component 0 is dE/dr (Y_00 is constant)
 };
 
@@ -118,7 +126,7 @@ __device__ __forceinline__ void eb_cp_arrive(uint32_t bar) {
 // Four channels (two pairs) of two edges: sums into gy (per edge and component) and dr2; T in t2.
 // SAME: both edges have the same receiver.  The accumulators are given back as soon as the last of them is in registers;
 // ready says whether the next step's accumulators and sender rows were there at that time.
-template <bool STAGED, bool SAME>
+template <int C, bool STAGED, bool SAME>
 __device__ __forceinline__ void eb_step(uint32_t ta, uint32_t acc_free, uint32_t next_acc, uint32_t next_acc_phase,
                                         uint32_t next_x, uint32_t next_x_phase, bool &ready, int lane, const uint32_t (&gs)[2],
                                         const float *const (&gg)[2], const unsigned long long (&x2)[2][2],
@@ -158,9 +166,9 @@ __device__ __forceinline__ void eb_step(uint32_t ta, uint32_t acc_free, uint32_t
           w[1][0] = w[0][0];
           w[1][1] = w[0][1];
         } else if (STAGED) {
-          eb_lds(gs[e] + (uint32_t)(m * EB_C * 4), w[e]);
+          eb_lds(gs[e] + (uint32_t)(m * C * 4), w[e]);
         } else {
-          const ulonglong2 q = __ldg(reinterpret_cast<const ulonglong2 *>(gg[e] + m * EB_C));
+          const ulonglong2 q = __ldg(reinterpret_cast<const ulonglong2 *>(gg[e] + m * C));
           w[e][0] = q.x;
           w[e][1] = q.y;
         }
@@ -197,8 +205,10 @@ __device__ __forceinline__ void eb_step(uint32_t ta, uint32_t acc_free, uint32_t
     for (int c = 0; c < 2; c++) dr2[e] = fma2(x2[e][c], v2[e][c], dr2[e]);
 }
 
+template <int C>
 __global__ void __launch_bounds__(EB_THREADS, 1)
     edge_back_kernel(const EdgeBackArgs g) {
+  using S = EdgeBackShape<C>;
   extern __shared__ __align__(1024) unsigned char smem[];
   __shared__ __align__(8) uint64_t bars[2 * EB_W_SLOTS + 2 * EB_X_SLOTS + 10];
   __shared__ uint32_t tmem_base_slot;
@@ -243,7 +253,7 @@ __global__ void __launch_bounds__(EB_THREADS, 1)
     // ---- consumers
     asm volatile("setmaxnreg.inc.sync.aligned.u32 %0;" ::"n"(EB_REGS));   // by whole warpgroups
     const int row0 = 32 * (warp & 3) + 16 * (warp >> 2), rg = row0 + (lane >> 2), t = lane & 3;   // rows rg, rg + 8 of the tile
-    const uint32_t sY = base_s + EB_OFF_Y;
+    const uint32_t sY = base_s + S::OFF_Y;
     const uint32_t acc0 = tmem + ((uint32_t)row0 << 16) + 256u;
     bool ok = true;
     uint32_t k = 0;   // tiles done
@@ -273,27 +283,27 @@ __global__ void __launch_bounds__(EB_THREADS, 1)
       // Y is in registers, and this warp has left the tile before: its G and h buffers are free
       if (lane == 0) mbar_arrive(y_free);
       const bool same = __all_sync(0xffffffffu, my[0] == my[1]);
-      const bool staged = __all_sync(0xffffffffu, my[1] - r_first < EB_G_RECV);   // the list is sorted
+      const bool staged = __all_sync(0xffffffffu, my[1] - r_first < S::RECV);   // the list is sorted
       if (ok && !warp_wait_all(g_full + 8u * (k & 1u), (k >> 1) & 1u, lane)) {
         if (lane == 0 && g.status) atomicCAS(g.status, 0, 62);
         ok = false;
       }
-      const uint32_t sG = base_s + EB_OFF_G + (k & 1u) * EB_G_BYTES + 16u * t;
+      const uint32_t sG = base_s + S::OFF_G + (k & 1u) * S::G_BYTES + 16u * t;
       float gy[2][16];
       unsigned long long dr2[2] = {0ull, 0ull};
 #pragma unroll
       for (int m = 0; m < 16; m++) gy[0][m] = gy[1][m] = 0.f;
       bool ready = false;
 #pragma unroll 1
-      for (int n = 0; ok && n < EB_NSTEP; n++) {
-        // use number 4 k + n / 2 of accumulator buffer b
-        const uint32_t b = (uint32_t)n & 1u, next_phase = ((uint32_t)(n + 1) >> 1) & 1u;
+      for (int n = 0; ok && n < S::NSTEP; n++) {
+        // use number k NSTEP / 2 + n / 2 of accumulator buffer b
+        const uint32_t use = k * (S::NSTEP / 2), b = (uint32_t)n & 1u, next_phase = (use + ((uint32_t)(n + 1) >> 1)) & 1u;
         if (!__all_sync(0xffffffffu, ready)) {
-          ok = warp_wait(x_full + 8u * xs, xphase, lane) && warp_wait(acc_full + 8u * b, ((uint32_t)n >> 1) & 1u, lane);
+          ok = warp_wait(x_full + 8u * xs, xphase, lane) && warp_wait(acc_full + 8u * b, (use + ((uint32_t)n >> 1)) & 1u, lane);
           if (!ok) break;
         }
         tc_fence_after();
-        const uint32_t sX = base_s + EB_OFF_X + (uint32_t)xs * EB_X_BYTES, x_done = x_free + 8u * xs;
+        const uint32_t sX = base_s + S::OFF_X + (uint32_t)xs * EB_X_BYTES, x_done = x_free + 8u * xs;
         unsigned long long x2[2][2], t2[2][2];
         eb_lds(sX + (uint32_t)sw64_offset(rg, t), x2[0]);
         eb_lds(sX + (uint32_t)sw64_offset(rg + 8, t), x2[1]);
@@ -302,11 +312,11 @@ __global__ void __launch_bounds__(EB_THREADS, 1)
           xphase ^= 1;
         }
         const int c0 = EB_STEP * n + 4 * t;
-        const uint32_t gs[2] = {sG + (uint32_t)(my[0] - r_first) * (16 * EB_C * 4) + 4u * EB_STEP * (uint32_t)n,
-                                sG + (uint32_t)(my[1] - r_first) * (16 * EB_C * 4) + 4u * EB_STEP * (uint32_t)n};
-        const float *const gg[2] = {g.G + (int64_t)my[0] * (16 * EB_C) + c0, g.G + (int64_t)my[1] * (16 * EB_C) + c0};
+        const uint32_t gs[2] = {sG + (uint32_t)(my[0] - r_first) * S::G_ROW + 4u * EB_STEP * (uint32_t)n,
+                                sG + (uint32_t)(my[1] - r_first) * S::G_ROW + 4u * EB_STEP * (uint32_t)n};
+        const float *const gg[2] = {g.G + (int64_t)my[0] * (16 * C) + c0, g.G + (int64_t)my[1] * (16 * C) + c0};
         auto step = [&](auto in_smem, auto one) {
-          eb_step<decltype(in_smem)::value, decltype(one)::value>(
+          eb_step<C, decltype(in_smem)::value, decltype(one)::value>(
               acc0 + 128u * b, acc_free + 8u * b, acc_full + 8u * (b ^ 1u), next_phase, x_full + 8u * xs, xphase, ready, lane,
               gs, gg, x2, y, gy, dr2, t2);
         };
@@ -315,9 +325,9 @@ __global__ void __launch_bounds__(EB_THREADS, 1)
         else step(std::false_type{}, std::false_type{});
         if (lane == 0) mbar_arrive(x_done);   // the accumulators went back after every lane had read its X
         const unsigned long long f2 = pack2(g.factor_v, g.factor_v);
-        ulonglong2 *out = reinterpret_cast<ulonglong2 *>(g.T + e0 * EB_C + c0);
+        ulonglong2 *out = reinterpret_cast<ulonglong2 *>(g.T + e0 * C + c0);
         if (e0 < g.nedges) out[0] = make_ulonglong2(mul2(t2[0][0], f2), mul2(t2[0][1], f2));
-        if (e1 < g.nedges) out[EB_C / 4] = make_ulonglong2(mul2(t2[1][0], f2), mul2(t2[1][1], f2));
+        if (e1 < g.nedges) out[C / 4] = make_ulonglong2(mul2(t2[1][0], f2), mul2(t2[1][1], f2));
       }
       if (!ok) {
         if (lane == 0 && g.status) atomicCAS(g.status, 0, 66);
@@ -356,12 +366,13 @@ __global__ void __launch_bounds__(EB_THREADS, 1)
         for (int64_t tile = blockIdx.x; ok && tile < ntiles; tile += gridDim.x, k++) {
           ok = mbar_wait(h_full + 8u * (k & 1u), (k >> 1) & 1u);
           bool ready = false;
-          for (int n = 0; ok && n < EB_NSTEP; n++) {
+          const uint32_t use = k * (S::NSTEP / 2);
+          for (int n = 0; ok && n < S::NSTEP; n++) {
             const uint32_t b = (uint32_t)n & 1u;
-            if (!ready) ok = mbar_wait(acc_free + 8u * b, (((uint32_t)n >> 1) & 1u) ^ 1u) && mbar_wait(w_full + 8u * slot, wphase);
+            if (!ready) ok = mbar_wait(acc_free + 8u * b, ((use + ((uint32_t)n >> 1)) & 1u) ^ 1u) && mbar_wait(w_full + 8u * slot, wphase);
             if (!ok) break;
             tc_fence_after();
-            const uint32_t sW = base_s + EB_OFF_W + (uint32_t)slot * EB_W_BYTES;
+            const uint32_t sW = base_s + S::OFF_W + (uint32_t)slot * EB_W_BYTES;
             const uint64_t b_hi = umma_desc_sw128(sW), b_lo = umma_desc_sw128(sW + EB_W_BYTES / 2);
             const uint32_t d = tmem + 256u + 128u * b, a = tmem + 128u * (k & 1u);
             const uint32_t done = w_free + 8u * slot;
@@ -372,7 +383,7 @@ __global__ void __launch_bounds__(EB_THREADS, 1)
 #pragma unroll
             for (int j = 0; j < 4; j++) {   // R and R'
               if (j == 3)
-                ready = n + 1 < EB_NSTEP && mbar_test(acc_free + 8u * (b ^ 1u), (((uint32_t)(n + 1) >> 1) & 1u) ^ 1u) &&
+                ready = n + 1 < S::NSTEP && mbar_test(acc_free + 8u * (b ^ 1u), ((use + ((uint32_t)(n + 1) >> 1)) & 1u) ^ 1u) &&
                         mbar_test(w_full + 8u * slot, wphase);
               umma_f16_ts(d, a + 8u * j, b_hi + (uint64_t)(2 * j), idesc, j != 0);
               umma_f16_ts(d + 64u, a + 64u + 8u * j, b_hi + (uint64_t)(2 * j), idesc, j != 0);
@@ -395,11 +406,11 @@ __global__ void __launch_bounds__(EB_THREADS, 1)
         uint32_t wphase = 0;
         bool ok = true;
         for (int64_t tile = blockIdx.x; ok && tile < ntiles; tile += gridDim.x)
-          for (int n = 0; ok && n < EB_NSTEP; n++) {
+          for (int n = 0; ok && n < S::NSTEP; n++) {
             ok = mbar_wait(w_free + 8u * slot, wphase ^ 1);
             if (!ok) break;
             mbar_arrive_expect_tx(w_full + 8u * slot, EB_W_BYTES);
-            bulk_copy_g2s(base_s + EB_OFF_W + (uint32_t)slot * EB_W_BYTES, g.W + (int64_t)n * EB_W_BYTES, EB_W_BYTES,
+            bulk_copy_g2s(base_s + S::OFF_W + (uint32_t)slot * EB_W_BYTES, g.W + (int64_t)n * EB_W_BYTES, EB_W_BYTES,
                           w_full + 8u * slot);
             if (++slot == EB_W_SLOTS) {
               slot = 0;
@@ -427,13 +438,13 @@ __global__ void __launch_bounds__(EB_THREADS, 1)
       for (int64_t tile = blockIdx.x; ok && tile < ntiles; tile += gridDim.x) {
         const float *src[8];
 #pragma unroll
-        for (int i = 0; i < 8; i++) src[i] = g.X + (int64_t)next[i] * EB_C + 4 * (lane & 3);
+        for (int i = 0; i < 8; i++) src[i] = g.X + (int64_t)next[i] * C + 4 * (lane & 3);
         if (tile + gridDim.x < ntiles) load_senders(tile + gridDim.x);
 #pragma unroll 1
-        for (int n = 0; n < EB_NSTEP; n++) {
+        for (int n = 0; n < S::NSTEP; n++) {
           ok = warp_wait_all(x_free + 8u * slot, phase ^ 1, lane);
           if (!ok) break;
-          const uint32_t dst = base_s + EB_OFF_X + (uint32_t)slot * EB_X_BYTES;
+          const uint32_t dst = base_s + S::OFF_X + (uint32_t)slot * EB_X_BYTES;
 #pragma unroll
           for (int i = 0; i < 8; i++) eb_cp16(dst + (uint32_t)sw64_offset(8 * i + r0, lane & 3), src[i] + EB_STEP * n);
           eb_cp_arrive(x_full + 8u * slot);
@@ -448,7 +459,7 @@ __global__ void __launch_bounds__(EB_THREADS, 1)
     } else {
       // ---- the next tile's rows; warp 12 + q the rows 32 q ..
       const int q = warp & 3;
-      const uint32_t sH = base_s + EB_OFF_H + (uint32_t)(2 * q) * EB_PIECE, sY = base_s + EB_OFF_Y;
+      const uint32_t sH = base_s + S::OFF_H + (uint32_t)(2 * q) * EB_PIECE, sY = base_s + S::OFF_Y;
       const uint32_t lanes = (uint32_t)(32 * q) << 16;
       const int r0 = 32 * q + (lane >> 2);
       const uint32_t hdst = sH + (uint32_t)sw64_offset(lane >> 2, lane & 3);
@@ -486,11 +497,11 @@ __global__ void __launch_bounds__(EB_THREADS, 1)
           const int64_t last = base + EB_TILE - 1 < g.nedges ? base + EB_TILE - 1 : g.nedges - 1;
           const int first = __ldg(g.receiver + base);
           int count = __ldg(g.receiver + last) - first + 1;
-          count = count < EB_G_RECV ? count : EB_G_RECV;
-          const uint32_t bar = g_full + 8u * (k & 1u), dst = base_s + EB_OFF_G + (k & 1u) * EB_G_BYTES;
-          mbar_arrive_expect_tx(bar, (uint32_t)count * (16 * EB_C * 4));
+          count = count < S::RECV ? count : S::RECV;
+          const uint32_t bar = g_full + 8u * (k & 1u), dst = base_s + S::OFF_G + (k & 1u) * S::G_BYTES;
+          mbar_arrive_expect_tx(bar, (uint32_t)count * S::G_ROW);
           for (int i = 0; i < count; i++)
-            bulk_copy_g2s(dst + (uint32_t)i * (16 * EB_C * 4), g.G + (int64_t)(first + i) * (16 * EB_C), 16 * EB_C * 4, bar);
+            bulk_copy_g2s(dst + (uint32_t)i * S::G_ROW, g.G + (int64_t)(first + i) * (16 * C), S::G_ROW, bar);
         }
         __syncwarp();
 #pragma unroll 1
@@ -521,8 +532,29 @@ __global__ void __launch_bounds__(EB_THREADS, 1)
   if (warp == 8) tmem_dealloc(tmem, 512);
 }
 
+template <int C>
+static int launch_edge_back(const EdgeBackArgs &g, const char *what, cudaStream_t st) {
+  using S = EdgeBackShape<C>;
+  static std::atomic<int> compiled_regs{0};   // a property of the binary
+  int regs = compiled_regs.load(std::memory_order_relaxed);
+  cudaError_t e = cudaSuccess;
+  if (regs == 0) {
+    cudaFuncAttributes attr;
+    e = cudaFuncGetAttributes(&attr, edge_back_kernel<C>);
+    if (e != cudaSuccess) return fail(CMACE_ERR_CUDA, "%s: %s", what, cudaGetErrorString(e));
+    compiled_regs.store(regs = attr.numRegs, std::memory_order_relaxed);
+  }
+  if (!register_split_fits(regs, EB_THREADS, EB_REGS, EB_REGS_OTHER))
+    return fail(CMACE_ERR_UNSUPPORTED, "%s: compiled with %d registers a thread, too few for its register split", what, regs);
+  e = cudaFuncSetAttribute(edge_back_kernel<C>, cudaFuncAttributeMaxDynamicSharedMemorySize, S::SMEM);
+  if (e != cudaSuccess) return fail(CMACE_ERR_CUDA, "%s: %s", what, cudaGetErrorString(e));
+  const int64_t ntiles = (g.nedges + EB_TILE - 1) / EB_TILE;
+  launch_chained(edge_back_kernel<C>, (unsigned)(ntiles < 148 ? ntiles : 148), EB_THREADS, S::SMEM, st, g);
+  return check_launch(what);
+}
+
 int fused_messages_back(const float *X, const float *Y, const float *G, const void *h, const void *dh, const void *W,
-                        float factor_v, float factor_t, const int32_t *sender, const int32_t *receiver, int64_t nedges,
+                        float factor_v, float factor_t, const int32_t *sender, const int32_t *receiver, int64_t nedges, int C,
                         float *T, float *gY, int32_t *status, cudaStream_t st) {
   const char *what = "cmace_step(edges_back)";
   if (nedges == 0) return CMACE_OK;
@@ -530,21 +562,13 @@ int fused_messages_back(const float *X, const float *Y, const float *G, const vo
   if (ntiles * EB_TILE > 0x7fffffffLL) return fail(CMACE_ERR_UNSUPPORTED, "%s: too many edges", what);
   const EdgeBackArgs g{X, Y, G, static_cast<const char *>(h), static_cast<const char *>(dh), static_cast<const char *>(W),
                        sender, receiver, status, nedges, factor_v, factor_t, T, gY};
-  static std::atomic<int> compiled_regs{0};   // a property of the binary
-  int regs = compiled_regs.load(std::memory_order_relaxed);
-  cudaError_t e = cudaSuccess;
-  if (regs == 0) {
-    cudaFuncAttributes attr;
-    e = cudaFuncGetAttributes(&attr, edge_back_kernel);
-    if (e != cudaSuccess) return fail(CMACE_ERR_CUDA, "%s: %s", what, cudaGetErrorString(e));
-    compiled_regs.store(regs = attr.numRegs, std::memory_order_relaxed);
+  switch (C) {
+    case 32: return launch_edge_back<32>(g, what, st);
+    case 64: return launch_edge_back<64>(g, what, st);
+    case 96: return launch_edge_back<96>(g, what, st);
+    case 128: return launch_edge_back<128>(g, what, st);
   }
-  if (!register_split_fits(regs, EB_THREADS, EB_REGS, EB_REGS_OTHER))
-    return fail(CMACE_ERR_UNSUPPORTED, "%s: compiled with %d registers a thread, too few for its register split", what, regs);
-  e = cudaFuncSetAttribute(edge_back_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, EB_SMEM);
-  if (e != cudaSuccess) return fail(CMACE_ERR_CUDA, "%s: %s", what, cudaGetErrorString(e));
-  launch_chained(edge_back_kernel, (unsigned)(ntiles < 148 ? ntiles : 148), EB_THREADS, EB_SMEM, st, g);
-  return check_launch(what);
+  return fail(CMACE_ERR_UNSUPPORTED, "%s: no kernel for %d channels", what, C);
 }
 
 }  // namespace cmace

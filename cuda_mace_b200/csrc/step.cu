@@ -7,7 +7,7 @@
 //   contract0     b0
 //   mid_fwd       up = b0 Wu, q0 = b0 Wsc[z] [n, 17]                                      (step_nodes.cu)
 //       -- a decomposed system fills the ghost rows of `up` here --
-//   radial_out    second layer: R = h W4 [E, 4C]  (not in float32 with 128 channels: `messages` and `edges_back` form R and
+//   radial_out    second layer: R = h W4 [E, 4C]  (not in float32 with fp16 pairs: `messages` and `edges_back` form R and
 //                 R' = h' W4 themselves, fused_messages.cu, and `radial_back` is part of `edges_back`)
 //   messages, linear, contract1 (value, readout, energy and gradient in one kernel), linear_back
 //   edges_back    T [E, C] and grad Y of the second layer; radial_back: dE/dr of the second layer
@@ -39,10 +39,10 @@ int step_sums_bwd_half(const float *gA, const void *h, const void *dh, const flo
                        const float *dr1, const Quad<float> *geo, int64_t nnodes, int elements, float out_v, float out_t,
                        float *gvec, cudaStream_t st);
 int fused_messages(const float *X, const float *Y, const void *h, const void *W, float factor, const int32_t *sender,
-                   const int32_t *receiver, const int32_t *row_ptr, int64_t nnodes, int64_t nedges, float *out,
+                   const int32_t *receiver, const int32_t *row_ptr, int64_t nnodes, int64_t nedges, int C, float *out,
                    int32_t *status, cudaStream_t st);
 int fused_messages_back(const float *X, const float *Y, const float *G, const void *h, const void *dh, const void *W,
-                        float factor_v, float factor_t, const int32_t *sender, const int32_t *receiver, int64_t nedges,
+                        float factor_v, float factor_t, const int32_t *sender, const int32_t *receiver, int64_t nedges, int C,
                         float *T, float *gY, int32_t *status, cudaStream_t st);
 template <typename T>
 int step_edge_finish(const T *gY0, const T *dr0, const T *gY1, const T *dr1, const Quad<T> *geo, int64_t nedges, int shares, T *gvec,
@@ -62,9 +62,10 @@ static const char *const kStepNames[S_COUNT] = {
     "mid_back", "contract0_back", "fold_back", "sums_back", "forces"};
 
 static bool is_spline(const cmace_step_model &m) { return m.spline[0] != nullptr; }
-// second layer with the radial weights formed inside its kernels: fp16 pairs of h, 128 channels (fused_messages.cu)
+// second layer with the radial weights formed inside its kernels: fp16 pairs of h (fused_messages.cu)
 static bool is_fused(const cmace_step_model &m) {
-  return !is_spline(m) && !m.is_f64 && m.fused_w != nullptr && m.fused_layout == CMACE_FUSED_LAYOUT && m.channels == 128;
+  return !is_spline(m) && !m.is_f64 && m.fused_w != nullptr &&
+         m.fused_layout == (m.channels == 128 ? CMACE_FUSED_LAYOUT : CMACE_FUSED_LAYOUT_NARROW);
 }
 
 template <typename T>
@@ -241,7 +242,7 @@ static int run_step(const cmace_step_model &m, cmace_step_io &io, const Workspac
       if constexpr (!f64)
         if (fused)
           return fused_messages(up, w.Y, w.h[1], m.fused_w, scales[1].out_v * m.fused_scale, io.sender, io.receiver,
-                                io.row_ptr, n, E, w.m1, io.status, st);
+                                io.row_ptr, n, E, C, w.m1, io.status, st);
       return imp_fwd<T>(up, w.Y, w.R, io.sender, io.row_ptr, n, E, ys, C, w.m1, st);
     case S_LINEAR: return linear_any(w.m1, m.linear[0], nullptr, 1, n, C, C, w.l1, io.status, st);
     case S_CONTRACT1:
@@ -253,7 +254,8 @@ static int run_step(const cmace_step_model &m, cmace_step_io &io, const Workspac
       if constexpr (!f64)
         if (fused)
           return fused_messages_back(up, w.Y, w.gm1, w.h[1], w.dh[1], m.fused_w_back, scales[1].out_v * m.fused_scale,
-                                     scales[1].out_t * m.fused_scale, io.sender, io.receiver, E, w.T_, w.gY1, io.status, st);
+                                     scales[1].out_t * m.fused_scale, io.sender, io.receiver, E, C, w.T_, w.gY1, io.status,
+                                     st);
       return imp_bwd_edge<T>(up, w.Y, w.R, w.gm1, io.sender, io.row_ptr, n, E, ys, C, f64 ? w.gradR : nullptr, w.gY1,
                              w.T_, w.partial, st);
     case S_RADIAL_BACK:

@@ -85,11 +85,16 @@ def half_scales(Ws, bounds):
     return out + z + a + t + [2.0**-sv, 2.0**-sd], factors
 
 
-def fused_rows(device):
-    """Column of W4 [64, 4 * 128] in every row of the fused message kernels' W^T (header, fused_w)."""
-    j, q, i = torch.meshgrid(torch.arange(4), torch.arange(4), torch.arange(32), indexing="ij")
-    degree = torch.where(q < 2, torch.where(j < 2, 3, 0), torch.where(j < 2, 1, 2))
-    return (degree * 128 + 64 * (q & 1) + 2 * i + (j & 1)).reshape(-1).to(device)
+def fused_rows(C):
+    """Column of W4 [64, 4 C] in every row of the fused message kernel's W^T (header, fused_w), -1 for a row of zeros."""
+    blocks = {32: 1, 64: 2, 96: 4, 128: 4}[C]
+    j, q, i = torch.meshgrid(torch.arange(blocks), torch.arange(4), torch.arange(32), indexing="ij")
+    if C == 32:
+        degree, channel = 3 - q, i
+    else:
+        degree = torch.where(q < 2, torch.where(2 * j < blocks, 3, 0), torch.where(2 * j < blocks, 1, 2))
+        channel = 32 * (q & 1) + i if C == 64 else 64 * (q & 1) + 2 * i + (j & 1)
+    return torch.where(channel < C, degree * C + channel, -1).reshape(-1)
 
 
 def _expected_buffers(model):
@@ -275,23 +280,21 @@ class StepPlan:
             if None not in scales and bool(L1.W_radial3.isfinite().all()):
                 for t, L in enumerate((L0, L1)):
                     values, factors = scales[t]
-                    if t == 1 and C != 128:   # the second layer's h and h' leave as float32: undo the stored scale
-                        values[7] *= values[11]
-                        values[10] *= values[12]
-                        values[11] = values[12] = 1.0
                     m.half_scales[t][:] = values
                     for i in range(3):
                         m.radial_half[t][i] = hold(half_images(getattr(L, f"W_radial{i}").t(), factors[i]))
-                if C == 128:
-                    w = L1.W_radial3.t()[fused_rows(L1.W_radial3.device)]   # [512, 64]
-                    scale = 2.0 ** (13 - math.floor(math.log2(max(float(w.abs().max()), 1e-30))))
-                    w = w * scale
-                    hi = w.half()
-                    m.fused_w = hold(torch.cat([hi, (w - hi.float()).half()], dim=1))
-                    m.fused_scale, m.fused_layout = 1.0 / scale, _abi.FUSED_LAYOUT
-                    # [step of 16 channels, (l, j, t, i), k]: row 8 j + 2 t + i of a degree is channel 4 t + 2 j + i of the step
-                    wt = L1.W_radial3.t().reshape(4, 8, 4, 2, 2, _H).permute(1, 0, 3, 2, 4, 5).reshape(8, 64, _H)
-                    m.fused_w_back = hold(torch.stack([half_images(b, scale) for b in wt]))
+                w4 = torch.nn.functional.pad(L1.W_radial3.t(), (0, 0, 0, 1))   # row -1: zeros
+                w = w4[fused_rows(C).to(w4.device)]
+                scale = 2.0 ** (13 - math.floor(math.log2(max(float(w.abs().max()), 1e-30))))
+                w = w * scale
+                hi = w.half()
+                m.fused_w = hold(torch.cat([hi, (w - hi.float()).half()], dim=1))
+                m.fused_scale = 1.0 / scale
+                m.fused_layout = _abi.FUSED_LAYOUT if C == 128 else _abi.FUSED_LAYOUT_NARROW
+                # [step of 16 channels, (l, j, t, i), k]: row 8 j + 2 t + i of a degree is channel 4 t + 2 j + i of the step
+                steps = C // 16
+                wt = L1.W_radial3.t().reshape(4, steps, 4, 2, 2, _H).permute(1, 0, 3, 2, 4, 5).reshape(steps, 64, _H)
+                m.fused_w_back = hold(torch.stack([half_images(b, scale) for b in wt]))
         m.radial_back = matrix(L1.W_radial3.t())
         w4 = d(L0.W_radial3).view(_H, 4, C)
         fold = torch.einsum("zc,klc,rlcd->rlzkd", x, w4, lin).reshape(Z, 4, Z * _H, C)

@@ -364,7 +364,8 @@ int cmace_symcon_effective_weights(const cmace_symcon_plan *plan, int is_f64, co
  * kernel launches with its gradient written out: no autograd graph, no allocation, no synchronisation.  The caller
  * owns weights, workspace and outputs.  csrc/step.cu documents the sequence; steps can be run in ranges, which is
  * where a decomposed system exchanges node features (after "mid_fwd") and their gradients (after "senders"). */
-#define CMACE_FUSED_LAYOUT 2 /* names the layouts of fused_w and fused_w_back below; changes with them */
+#define CMACE_FUSED_LAYOUT 2 /* names the layouts of fused_w and fused_w_back below for 128 channels; changes with them */
+#define CMACE_FUSED_LAYOUT_NARROW 3 /* and those for 32, 64 and 96 channels */
 typedef struct cmace_step_model {
   int32_t is_f64, channels, elements, nbessel, cutoff_p, reserved;
   double r_max, scale, shift;
@@ -373,15 +374,17 @@ typedef struct cmace_step_model {
   const void *radial_half[2][3]; /* float32, or all NULL: fp16 images (hi, lo) of W1^T (rows padded to 64), W2^T, W3^T */
   float half_scales[2][13];  /* their powers of two: basis, derivative, per layer pre-activation / activation /
                                 derivative, then what undoes the scale of the stored h and h' */
-  const void *fused_w;       /* float32 with 128 channels and radial_half, or NULL: second layer's W4^T as fp16 rows
-                                [512][hi 64 | lo 64], row j*128 + q*32 + i = degree (q < 2 ? (j < 2 ? 3 : 0) : (j < 2 ? 1 : 2)),
-                                channel 64 (q & 1) + 2 i + (j & 1), divided by fused_scale (a power of two) */
-  const void *fused_w_back;  /* the same W4^T for the backward: [8 steps of 16 channels][hi, lo][64 rows x 128 bytes], 128-byte
+  const void *fused_w;       /* float32 with radial_half, or NULL: second layer's W4^T as fp16 rows [128 blocks][hi 64 | lo 64]
+                                divided by fused_scale (a power of two).  Row j*128 + q*32 + i, 128 and 96 channels (4 blocks):
+                                degree (q < 2 ? (j < 2 ? 3 : 0) : (j < 2 ? 1 : 2)), channel 64 (q & 1) + 2 i + (j & 1), zeros
+                                where there is none; 64 (2 blocks): degree (q < 2 ? (j < 1 ? 3 : 0) : (j < 1 ? 1 : 2)),
+                                channel 32 (q & 1) + i; 32 (1 block): degree 3 - q, channel i */
+  const void *fused_w_back;  /* the same W4^T for the backward: [steps of 16 channels][hi, lo][64 rows x 128 bytes], 128-byte
                                 swizzle; row 16 l + 8 j + 2 t + i is degree l, channel 4 t + 2 j + i of the step */
   float fused_scale;
-  int32_t fused_layout;      /* CMACE_FUSED_LAYOUT.  With any other value, such as the 0 of a caller that lays fused_w_back out as
-                                earlier libraries read it (steps of 8 channels), neither array is read and the second layer's
-                                radial weights are written, as for other numbers of channels */
+  int32_t fused_layout;      /* 128 channels: CMACE_FUSED_LAYOUT, fewer: CMACE_FUSED_LAYOUT_NARROW.  With any other value, such as
+                                the 0 of a caller that lays fused_w_back out as earlier libraries read it (steps of 8 channels),
+                                neither array is read and the second layer's radial weights are written */
   const void *radial_back;   /* second layer's W4 for the gradient: float32 packed W4 itself, float64 W4^T [4C,64] */
   const void *spline[2];     /* tabulated radial weights: coefficients [intervals][4][4C] of both layers, or NULL; then the
                                 radial weights above are not read, fold is the first layer's Linear [elements][4] [C, C]

@@ -72,15 +72,15 @@ def test_step_against_autograd(U, dtype, tol, n, C, Z, nb, radial):
     assert float((out["forces"] + g).abs().max()) < tol * float(g.abs().max())
 
 
-def _list_of(receiver, n, seed):
-    """A float32 model of 128 channels and a list with these receivers; a shift an edge gives any distance up to the cutoff."""
+def _list_of(receiver, n, seed, channels=128):
+    """A model's weights and a list with these receivers; a shift an edge gives any distance up to the cutoff."""
     rng = np.random.default_rng(seed)
     edges = receiver.size
     sender = rng.integers(0, n, edges)
     pos, shifts = rng.normal(size=(n, 3)), rng.normal(size=(edges, 3))
     length = rng.uniform(0.9, 4.9, edges)[:, None]
     shifts = shifts / np.linalg.norm(shifts, axis=1, keepdims=True) * length - (pos[sender] - pos[receiver])
-    return systems.init_params(128, 3, 7), pos, np.stack([receiver, sender]), shifts, rng.integers(0, 3, n)
+    return systems.init_params(channels, 3, 7), pos, np.stack([receiver, sender]), shifts, rng.integers(0, 3, n)
 
 
 def _step_of(U, params, pos, ei, sh, species):
@@ -109,16 +109,34 @@ def test_second_layer_at_tile_edges(U, edges, degree):
     assert float((out["forces"].cpu() - f_ref).abs().max()) < 1e-4 * max(float(f_ref.abs().max()), 1e-6)
 
 
+# the same kernels for fewer channels, whose rows, tiles and steps are laid out differently: an odd number of steps a tile (96
+# channels) and a single one (32), one and two words of last edges, lanes without a channel; 300 edges of 1 a receiver are more
+# receivers than any of them stages.  Bounds as above
+@pytest.mark.parametrize("channels", [32, 64, 96])
+@pytest.mark.parametrize("edges,degree", [(1, 1), (9, 2), (63, 40), (65, 3), (128, 1), (129, 17), (300, 1), (300, 40)])
+def test_narrow_second_layer_at_tile_edges(U, channels, edges, degree):
+    n = -(-edges // degree) + 2
+    receiver = np.minimum(np.arange(edges) // degree, n - 1)
+    receiver[receiver > 0] += 1
+    params, pos, ei, sh, species = _list_of(receiver, n, edges * 50 + degree, channels)
+    out = _step_of(U, params, pos, ei, sh, species)
+    _, e_ref, f_ref = omodel.energy_and_forces(params, U, torch.from_numpy(pos), systems.one_hot(species, 3),
+                                               torch.from_numpy(ei), torch.from_numpy(sh))
+    assert abs(float(out["interaction_energy"]) - float(e_ref)) < 1e-5 * max(abs(float(e_ref)), 1e-3)
+    assert float((out["forces"].cpu() - f_ref).abs().max()) < 1e-4 * max(float(f_ref.abs().max()), 1e-6)
+
+
 # Four and five tiles of the backward a block on 148 blocks, eight and nine of the forward a set: every buffer and barrier is
 # used again, its phase wraps.  Receivers of so many edges in turn: few (warps whose receivers are not staged beside those
 # whose are), and a long one before many short ones.  Against the operators in float64 (the oracle's contraction of so many
 # nodes takes 60 GB), same bounds.
-@pytest.mark.parametrize("degrees", [(3,), (10,), (70,) + (1,) * 40])
-def test_second_layer_over_many_tiles(U, degrees):
+@pytest.mark.parametrize("channels,degrees", [(128, (3,)), (128, (10,)), (128, (70,) + (1,) * 40), (32, (3,)), (64, (70,) + (1,) * 40),
+                                              (96, (10,))])
+def test_second_layer_over_many_tiles(U, channels, degrees):
     edges = 80_001
     receiver = np.repeat(np.arange(edges), np.resize(degrees, edges))[:edges]
     n = int(receiver[-1]) + 1
-    params, pos, ei, sh, species = _list_of(receiver, n, len(degrees))
+    params, pos, ei, sh, species = _list_of(receiver, n, len(degrees), channels)
     out = _step_of(U, params, pos, ei, sh, species)
     mace = model.InvariantMACE(params, U, dtype=torch.float64, device="cuda")
     p = torch.from_numpy(pos).cuda().requires_grad_(True)
