@@ -138,14 +138,11 @@ __device__ __forceinline__ void cp_async_16_zfill(void *dst, const void *src, bo
   asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(d), "l"(src), "r"(n) : "memory");
 }
 
-// DOT (PLAIN, at most TN columns): out [rows] is the product of every row of the result with the row of `dot` [rows, Nout];
-// a pass of its own wrote and read the result again (64 us at 418 000 rows of 64).
-template <bool PLAIN, int TM, int TN, bool DOT = false>
+template <bool PLAIN, int TM, int TN>
 __global__ void __launch_bounds__(DM_THREADS, 2)
     linear_dmma_kernel(const double *__restrict__ X, const double *__restrict__ W,
                        const int32_t *__restrict__ node_order, const int32_t *__restrict__ elem_start,
-                       int nelements, int64_t nnodes, int K, int Nout, double scale, const double *__restrict__ dot,
-                       double *__restrict__ out) {
+                       int nelements, int64_t nnodes, int K, int Nout, double scale, double *__restrict__ out) {
   grid_begin();
   extern __shared__ __align__(16) double dm_smem[];
   __shared__ int64_t row_of[TM];
@@ -259,32 +256,6 @@ __global__ void __launch_bounds__(DM_THREADS, 2)
   }
   asm volatile("cp.async.wait_group 0;" ::: "memory");
 
-  if constexpr (DOT) {
-    __shared__ double part[TM * Geo::WN];   // [row][warp along the columns]
-#pragma unroll
-    for (int i = 0; i < 4; i++) {
-      const int64_t grow = row_of[wm + i * 8 + fr];
-      double s = 0.0;
-#pragma unroll
-      for (int j = 0; j < NJ; j++) {
-        const int c = n0 + wn + j * 8 + 2 * fk;
-        if (grow >= 0 && c < Nout) {
-          const double2 d = __ldg(reinterpret_cast<const double2 *>(dot + grow * Nout + c));
-          s = fma(acc[i][j][0], d.x, fma(acc[i][j][1], d.y, s));
-        }
-      }
-      s += __shfl_xor_sync(0xffffffffu, s, 1);
-      s += __shfl_xor_sync(0xffffffffu, s, 2);
-      if (fk == 0) part[(wm + i * 8 + fr) * Geo::WN + warp % Geo::WN] = s;
-    }
-    __syncthreads();
-    if (tid < TM && row_of[tid] >= 0) {
-      double s = 0.0;
-      for (int k = 0; k < Geo::WN; k++) s += part[tid * Geo::WN + k];
-      out[row_of[tid]] = s * scale;
-    }
-    return;
-  }
 #pragma unroll
   for (int i = 0; i < 4; i++) {
     const int64_t grow = row_of[wm + i * 8 + fr];
@@ -298,18 +269,17 @@ __global__ void __launch_bounds__(DM_THREADS, 2)
   }
 }
 
-template <bool PLAIN, int TM, int TN, bool DOT = false>
+template <bool PLAIN, int TM, int TN>
 static int dmma_launch(const double *X, const double *W, const int32_t *node_order, const int32_t *elem_start, int nelements,
-                       int64_t nnodes, int K, int Nout, double scale, double *out, cudaStream_t st, const char *what,
-                       const double *dot = nullptr) {
-  auto kern = linear_dmma_kernel<PLAIN, TM, TN, DOT>;
+                       int64_t nnodes, int K, int Nout, double scale, double *out, cudaStream_t st, const char *what) {
+  auto kern = linear_dmma_kernel<PLAIN, TM, TN>;
   constexpr int smem = DmGeom<TM, TN>::SMEM_BYTES;
   cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
   if (e != cudaSuccess) return fail(CMACE_ERR_CUDA, "%s: cannot reserve shared memory", what);
   const int64_t tiles = PLAIN ? (nnodes + TM - 1) / TM : (nnodes * 7 + TM - 1) / TM + nelements;
   if (tiles > 0x7fffffffLL) return fail(CMACE_ERR_UNSUPPORTED, "%s: too many rows", what);
   const dim3 grid((unsigned)tiles, PLAIN ? 1 : 4, (unsigned)((Nout + TN - 1) / TN));
-  launch_chained(kern, grid, DM_THREADS, smem, st, X, W, node_order, elem_start, nelements, nnodes, K, Nout, scale, dot, out);
+  launch_chained(kern, grid, DM_THREADS, smem, st, X, W, node_order, elem_start, nelements, nnodes, K, Nout, scale, out);
   return check_launch(what);
 }
 
@@ -327,16 +297,6 @@ static int dmma_any(const double *X, const double *W, const int32_t *node_order,
   if (small >= 148)
     return dmma_launch<PLAIN, 64, 64>(X, W, node_order, elem_start, nelements, nnodes, K, Nout, scale, out, st, what);
   return dmma_launch<PLAIN, 32, 64>(X, W, node_order, elem_start, nelements, nnodes, K, Nout, scale, out, st, what);
-}
-
-// out [M] = row-wise product of A [M, K] B [K, N] with dot [M, N], N <= 64 (the tile sizes of dmma_any)
-int gemm_dot_f64(const double *A, const double *B, const double *dot, int64_t M, int K, int N, double *out, cudaStream_t st) {
-  const char *what = "cmace_step(radial_back)";
-  if (M == 0) return CMACE_OK;
-  if (N > 64 || K % 2 != 0 || N % 2 != 0) return fail(CMACE_ERR_ARG, "%s: bad size", what);
-  if ((M + 127) / 128 >= 2 * 148) return dmma_launch<true, 128, 64, true>(A, B, nullptr, nullptr, 1, M, K, N, 1.0, out, st, what, dot);
-  if ((M + 63) / 64 >= 148) return dmma_launch<true, 64, 64, true>(A, B, nullptr, nullptr, 1, M, K, N, 1.0, out, st, what, dot);
-  return dmma_launch<true, 32, 64, true>(A, B, nullptr, nullptr, 1, M, K, N, 1.0, out, st, what, dot);
 }
 
 static int linear_dmma(const double *X, const double *W, const int32_t *node_order, const int32_t *elem_start,

@@ -19,6 +19,7 @@
 #include <cstdlib>
 
 #include "common.cuh"
+#include "step_common.cuh"
 
 namespace cmace {
 
@@ -28,10 +29,12 @@ constexpr int kWarpsPerBlock = 4;
 // eighth pair of edges and add up through shared memory in a fixed order: with fewer receivers than the chip holds warps
 // the walk over one receiver's edges, about 1.6 us a pair, is all there is (192 receivers, 52 edges: 43 us with one warp
 // each).
-template <typename T, int VEC, int SPLIT>
+// ROWS: edge e reads row row_of[e] of R, which another edge may read as well; rows and senders are looked up a pair ahead (420 ->
+// 338 us at 8 000 atoms in float64, the same as from a row of its own).
+template <typename T, int VEC, int SPLIT, bool ROWS = false>
 __global__ void __launch_bounds__(SPLIT == 1 ? kWarpsPerBlock * 32 : SPLIT * 32, SPLIT == 1 && sizeof(T) == 4 ? 4 : 1)
     imp_fwd_kernel(const T *__restrict__ X, const T *__restrict__ Y, const T *__restrict__ R,
-                   const int32_t *__restrict__ sender, const int32_t *__restrict__ row_ptr,
+                   const int32_t *__restrict__ row_of, const int32_t *__restrict__ sender, const int32_t *__restrict__ row_ptr,
                    int64_t nnodes, ImpLayout ys, int C, T *__restrict__ out) {
   grid_begin();
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
@@ -49,20 +52,33 @@ __global__ void __launch_bounds__(SPLIT == 1 ? kWarpsPerBlock * 32 : SPLIT * 32,
   __shared__ __align__(16) PairHarmonics<T, SPLIT == 1 ? kWarpsPerBlock : SPLIT> harmonics;
   int turn = 0;
   const int ylm = lane & 15, yedge = lane >> 4;
+  int32_t next[4];   // ROWS: senders and rows of the next pair, or the row of R would wait for its number
+  auto look_up = [&](int64_t e) {
+    const int64_t a = e < e1 ? e : e1 - 1, b = e + 1 < e1 ? e + 1 : e1 - 1;
+    next[0] = __ldg(sender + a), next[1] = __ldg(sender + b), next[2] = __ldg(row_of + a), next[3] = __ldg(row_of + b);
+  };
+  if (ROWS && e0 < e1) look_up(e0 + (SPLIT > 1 ? 2 * warp : 0));
   for (int64_t e = e0 + (SPLIT > 1 ? 2 * warp : 0); e < e1; e += 2 * SPLIT, turn ^= 1) {
     // second edge of the pair: clamp to a valid edge, its harmonics are zeroed below
     const int64_t eb = (e + 1 < e1) ? e + 1 : e;
     const int64_t ey = yedge ? eb : e;
     T yv = __ldg(Y + ylm * ys.m + ey * ys.e);
     if (yedge && e + 1 >= e1) yv = T(0);
-    const int64_t sa = sender[e], sb = sender[eb];
+    const int64_t sa = ROWS ? next[0] : sender[e], sb = ROWS ? next[1] : sender[eb];
+    const int64_t ea = ROWS ? next[2] : e, ec = ROWS ? next[3] : eb;
+    if (ROWS) look_up(e + 2 * SPLIT);
     T xa[VEC], xb[VEC], ra[4][VEC], rb[4][VEC];
     load_vec<T, VEC>(xa, X + sa * C + c0);
     load_vec<T, VEC>(xb, X + sb * C + c0);
 #pragma unroll
     for (int l = 0; l < 4; l++) {
-      load_vec_stream<T, VEC>(ra[l], R + (e * 4 + l) * C + c0);
-      load_vec_stream<T, VEC>(rb[l], R + (eb * 4 + l) * C + c0);
+      if constexpr (ROWS) {
+        load_vec<T, VEC>(ra[l], R + (ea * 4 + l) * C + c0);
+        load_vec<T, VEC>(rb[l], R + (ec * 4 + l) * C + c0);
+      } else {
+        load_vec_stream<T, VEC>(ra[l], R + (ea * 4 + l) * C + c0);
+        load_vec_stream<T, VEC>(rb[l], R + (ec * 4 + l) * C + c0);
+      }
     }
 #pragma unroll
     for (int l = 0; l < 4; l++)
@@ -189,6 +205,95 @@ __global__ void __launch_bounds__(kWarpsPerBlock * 32)
       if (Tout != nullptr) store_vec<T, VEC>(Tout + ee * C + c0, t);
       const T tot = warp_reduce16(p, lane);
       if ((lane & 1) == 0) gy[(lane >> 1) * ys.m + ee * ys.e] = tot;
+    }
+  }
+}
+
+// The edge pass of a float64 step, with dE/dr from the radial weights' derivative instead of a gradient of the weights that a
+// product would read again:  T and grad Y as above, dE/dr = sum_c X sum_l R'_l u_l in the place of grad Y_00 (Y_00 is constant).
+// Edge e reads rows row_of[e] (null: e) of R and R', whose numbers are asked for a pair of edges ahead.  Each channel chunk has its
+// own gY [E, 16].  Bound by bytes, as the pass that wrote the gradient: 848 -> 678 us at 8 000 atoms and 128 channels (805 with
+// 220 registers, two blocks an SM), 406 -> 363 at 64.
+template <int VEC>
+__global__ void __launch_bounds__(kWarpsPerBlock * 32, VEC == 1 ? 4 : 3)
+    imp_bwd_edge_pair_kernel(const double *__restrict__ X, const double *__restrict__ Y, const double *__restrict__ R,
+                             const double *__restrict__ dR, const int32_t *__restrict__ row_of, const double *__restrict__ G,
+                             const int32_t *__restrict__ sender, const int32_t *__restrict__ row_ptr, int64_t nnodes,
+                             int64_t nedges, int C, int slices, double *__restrict__ gY, double *__restrict__ Tout) {
+  grid_begin();
+  const int lane = threadIdx.x & 31;
+  const int64_t item = (int64_t)blockIdx.x * kWarpsPerBlock + (threadIdx.x >> 5);
+  const int64_t node = slices == 1 ? item : item / slices;
+  const int slice = slices == 1 ? 0 : (int)(item - node * slices);
+  if (node >= nnodes) return;
+  const int c0 = blockIdx.y * (32 * VEC) + lane * VEC;
+  const int64_t e0 = row_ptr[node], e1 = row_ptr[node + 1];
+  if (e0 + 2 * slice >= e1) return;
+  double *gy = gY + (int64_t)blockIdx.y * 16 * nedges;
+  double g[16][VEC];
+#pragma unroll
+  for (int m = 0; m < 16; m++) load_vec<double, VEC>(g[m], G + (node * 16 + m) * C + c0);
+  __shared__ __align__(16) PairHarmonics<double, kWarpsPerBlock> harmonics;
+  int turn = 0;
+  const int ylm = lane & 15, yedge = lane >> 4;
+  int32_t next[4];   // senders and rows of the next pair of edges
+  auto look_up = [&](int64_t e) {
+    const int64_t a = e < e1 ? e : e1 - 1, b = e + 1 < e1 ? e + 1 : e1 - 1;
+    next[0] = __ldg(sender + a), next[1] = __ldg(sender + b);
+    next[2] = row_of ? __ldg(row_of + a) : (int32_t)a, next[3] = row_of ? __ldg(row_of + b) : (int32_t)b;
+  };
+  look_up(e0 + 2 * slice);
+  for (int64_t e = e0 + 2 * slice; e < e1; e += 2 * slices, turn ^= 1) {
+    const int64_t eb = e + 1 < e1 ? e + 1 : e;
+    const double yv = __ldg(Y + ylm + (yedge ? eb : e) * 16);
+    double *yp = harmonics.v[threadIdx.x >> 5][turn];
+    const int64_t s2[2] = {next[0], next[1]}, row[2] = {next[2], next[3]};
+    look_up(e + 2 * slices);
+    double xx[2][VEC], rr[2][4][VEC], dd[2][4][VEC];
+#pragma unroll
+    for (int h = 0; h < 2; h++) {
+      load_vec<double, VEC>(xx[h], X + s2[h] * C + c0);
+#pragma unroll
+      for (int l = 0; l < 4; l++) {
+        load_vec<double, VEC>(rr[h][l], R + (row[h] * 4 + l) * C + c0);
+        load_vec<double, VEC>(dd[h][l], dR + (row[h] * 4 + l) * C + c0);
+      }
+    }
+    yp[lane] = yv;
+    __syncwarp();
+#pragma unroll
+    for (int h = 0; h < 2; h++) {
+      const int64_t ee = h ? eb : e;
+      if (h && e + 1 >= e1) break;  // warp-uniform
+      double(&x)[VEC] = xx[h], p[16], yy[16], t[VEC], v[VEC];
+      take16<double>(yy, yp + 16 * h);
+#pragma unroll
+      for (int l = 0; l < 4; l++) {
+        double u[VEC], rx[VEC];
+#pragma unroll
+        for (int c = 0; c < VEC; c++) rx[c] = rr[h][l][c] * x[c];
+#pragma unroll
+        for (int m = l * l; m < (l + 1) * (l + 1); m++) {
+          double pm = 0.0;
+#pragma unroll
+          for (int c = 0; c < VEC; c++) {
+            u[c] = m == l * l ? yy[m] * g[m][c] : fma(yy[m], g[m][c], u[c]);
+            pm = fma(g[m][c], rx[c], pm);
+          }
+          p[m] = pm;
+        }
+#pragma unroll
+        for (int c = 0; c < VEC; c++) {
+          t[c] = l == 0 ? u[c] * rr[h][l][c] : fma(u[c], rr[h][l][c], t[c]);
+          v[c] = l == 0 ? u[c] * dd[h][l][c] : fma(u[c], dd[h][l][c], v[c]);
+        }
+      }
+      p[0] = 0.0;
+#pragma unroll
+      for (int c = 0; c < VEC; c++) p[0] = fma(x[c], v[c], p[0]);
+      store_vec<double, VEC>(Tout + ee * C + c0, t);
+      const double tot = warp_reduce16(p, lane);
+      if ((lane & 1) == 0) gy[(lane >> 1) + ee * 16] = tot;
     }
   }
 }
@@ -505,20 +610,21 @@ static int check_common(const void *a, const void *b, const void *c, int64_t nno
 constexpr int kSplit = 8;
 static bool few_nodes(int64_t pairs) { return pairs <= 148 * 8; }
 
-template <typename T, int VEC>
-static void launch_fwd(const T *X, const T *Y, const T *R, const int32_t *sender,
+template <typename T, int VEC, bool ROWS = false>
+static void launch_fwd(const T *X, const T *Y, const T *R, const int32_t *row_of, const int32_t *sender,
                        const int32_t *row_ptr, int64_t nnodes, ImpLayout ys, int C, T *out,
                        cudaStream_t st) {
   const int chunks = C / (32 * VEC);
   if (few_nodes(nnodes * chunks)) {
     constexpr int smem = kSplit * 16 * 32 * VEC * (int)sizeof(T);
-    cudaFuncSetAttribute(imp_fwd_kernel<T, VEC, kSplit>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
-    launch_chained(imp_fwd_kernel<T, VEC, kSplit>, dim3((unsigned)nnodes, chunks), kSplit * 32, smem, st, X, Y, R, sender, row_ptr, nnodes,
-                                                                                              ys, C, out);
+    cudaFuncSetAttribute(imp_fwd_kernel<T, VEC, kSplit, ROWS>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+    launch_chained(imp_fwd_kernel<T, VEC, kSplit, ROWS>, dim3((unsigned)nnodes, chunks), kSplit * 32, smem, st, X, Y, R, row_of, sender,
+                   row_ptr, nnodes, ys, C, out);
     return;
   }
   dim3 grid((unsigned)((nnodes + kWarpsPerBlock - 1) / kWarpsPerBlock), chunks);
-  launch_chained(imp_fwd_kernel<T, VEC, 1>, grid, kWarpsPerBlock * 32, 0, st, X, Y, R, sender, row_ptr, nnodes, ys, C, out);
+  launch_chained(imp_fwd_kernel<T, VEC, 1, ROWS>, grid, kWarpsPerBlock * 32, 0, st, X, Y, R, row_of, sender, row_ptr, nnodes, ys, C,
+                 out);
 }
 
 template <typename T>
@@ -532,10 +638,10 @@ int imp_fwd(const T *X, const T *Y, const T *R, const int32_t *sender, const int
   cudaStream_t st = (cudaStream_t)stream;
   switch (pick_vec<T>(C)) {
     case 4:
-      if constexpr (sizeof(T) == 4) launch_fwd<T, 4>(X, Y, R, sender, row_ptr, nnodes, ys, C, out, st);
+      if constexpr (sizeof(T) == 4) launch_fwd<T, 4>(X, Y, R, nullptr, sender, row_ptr, nnodes, ys, C, out, st);
       break;
-    case 2: launch_fwd<T, 2>(X, Y, R, sender, row_ptr, nnodes, ys, C, out, st); break;
-    default: launch_fwd<T, 1>(X, Y, R, sender, row_ptr, nnodes, ys, C, out, st); break;
+    case 2: launch_fwd<T, 2>(X, Y, R, nullptr, sender, row_ptr, nnodes, ys, C, out, st); break;
+    default: launch_fwd<T, 1>(X, Y, R, nullptr, sender, row_ptr, nnodes, ys, C, out, st); break;
   }
   return check_launch("cmace_imp_fwd");
 }
@@ -548,6 +654,28 @@ static void launch_bwd_edge(const T *X, const T *Y, const T *R, const T *G, cons
   dim3 grid((unsigned)((nnodes * slices + kWarpsPerBlock - 1) / kWarpsPerBlock), C / (32 * VEC));
   launch_chained(imp_bwd_edge_kernel<T, VEC>, grid, kWarpsPerBlock * 32, 0, st, X, Y, R, G, sender, row_ptr,
                                                                      nnodes, nedges, ys, C, slices, gradR, gy, Tout);
+}
+
+int imp_bwd_edge_pair_f64(const double *X, const double *Y, const double *R, const double *dR, const int32_t *row_of,
+                          const double *G, const int32_t *sender, const int32_t *row_ptr, int64_t nnodes, int64_t nedges, int C,
+                          double *gY, double *T, cudaStream_t st) {
+  if (nnodes == 0 || nedges == 0) return CMACE_OK;
+  auto launch = [&](auto kernel, int chunks) {
+    const int slices = few_nodes(nnodes * chunks) ? kSplit : 1;
+    const dim3 grid((unsigned)((nnodes * slices + kWarpsPerBlock - 1) / kWarpsPerBlock), (unsigned)chunks);
+    launch_chained(kernel, grid, kWarpsPerBlock * 32, 0, st, X, Y, R, dR, row_of, G, sender, row_ptr, nnodes, nedges, C, slices, gY, T);
+  };
+  if (C % 64 == 0) launch(imp_bwd_edge_pair_kernel<2>, C / 64);
+  else launch(imp_bwd_edge_pair_kernel<1>, C / 32);
+  return check_launch("cmace_step(edges_back)");
+}
+int imp_fwd_rows_f64(const double *X, const double *Y, const double *R, const int32_t *row_of, const int32_t *sender,
+                     const int32_t *row_ptr, int64_t nnodes, int64_t nedges, int C, double *out, cudaStream_t st) {
+  if (nnodes == 0) return CMACE_OK;
+  const ImpLayout ys{1, 16};
+  if (C % 64 == 0) launch_fwd<double, 2, true>(X, Y, R, row_of, sender, row_ptr, nnodes, ys, C, out, st);
+  else launch_fwd<double, 1, true>(X, Y, R, row_of, sender, row_ptr, nnodes, ys, C, out, st);
+  return check_launch("cmace_step(messages)");
 }
 
 static __device__ int g_staged_stall;   // set when a bounded wait of the staged edge pass gave up

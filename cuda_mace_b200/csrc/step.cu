@@ -10,7 +10,8 @@
 //   radial_out    second layer: R = h W4 [E, 4C]  (not in float32 with fp16 pairs: `messages` and `edges_back` form R and
 //                 R' = h' W4 themselves, fused_messages.cu, and `radial_back` is part of `edges_back`)
 //   messages, linear, contract1 (value, readout, energy and gradient in one kernel), linear_back
-//   edges_back    T [E, C] and grad Y of the second layer; radial_back: dE/dr of the second layer
+//   edges_back    T [E, C] and grad Y of the second layer; radial_back: dE/dr of the second layer (float64: part of edges_back,
+//                 from R' = h' W4 that radial_out forms beside R, a row a pair of edges)
 //   senders       grad up = sum of T over a sender's edges
 //       -- and returns the gradients of the ghost rows here --
 //   mid_back, contract0_back, fold_back
@@ -47,8 +48,7 @@ int fused_messages_back(const float *X, const float *Y, const float *G, const vo
 template <typename T>
 int step_edge_finish(const T *gY0, const T *dr0, const T *gY1, const T *dr1, const Quad<T> *geo, int64_t nedges, int shares, T *gvec,
                      cudaStream_t st);
-int gemm_dot_f64(const double *A, const double *B, const double *dot, int64_t M, int K, int N, double *out, cudaStream_t st);
-int radial_pair_f64(const double *basis, int nb, const double *const (*w)[3], int nper, int64_t nedges,
+int radial_pair_f64(const double *basis, int nb, const double *const (*w)[3], int nper, const EdgeRows &rows, int64_t nedges,
                     double *const *h, double *const *dh, cudaStream_t st);
 
 enum StepId {
@@ -68,13 +68,20 @@ static bool is_fused(const cmace_step_model &m) {
          m.fused_layout == (m.channels == 128 ? CMACE_FUSED_LAYOUT : CMACE_FUSED_LAYOUT_NARROW);
 }
 
+// Whether the edges of a pair share a row of h and h' (find_pairs), float64: once the radial kernel needs more than one round of
+// its warps without it.  The search takes 8 us there, the second round 30.
+constexpr int64_t kPairEdges64 = 74 * 16 * 8;
+static bool has_pairs(const cmace_step_model &m, int64_t edges) { return m.is_f64 && !is_spline(m) && edges > kPairEdges64; }
+
 template <typename T>
 struct Workspace {
   int32_t *species, *counts, *slot_of, *node_of, *slot_type, *elem_start;
+  EdgeRows rows;
   Quad<T> *geo;
   T *basis, *Y, *h[2], *dh[2], *A, *m0, *b0, *up, *R, *m1, *l1, *gX1, *gm1, *T_, *gY1, *dr1, *gup, *gb0, *gX0, *gA,
-      *gvec, *gradR, *partial, *q0, *dq, *gY0, *dr0;
+      *gvec, *dR, *partial, *q0, *dq, *gY0, *dr0;
   int64_t bytes;
+  int shares;   // of grad Y of the second layer, to be added up
 
   Workspace(void *base, const cmace_step_model &m, int64_t n, int64_t nl, int64_t E) {
     char *p = static_cast<char *>(base);
@@ -94,7 +101,12 @@ struct Workspace {
     take(geo, E);
     const bool sp = is_spline(m);
     take(basis, E * 2 * (sp ? 1 : m.nbessel));   // with tables: a SplinePoint an edge
-    const int64_t shares = sp ? spline_chunks<T>((int)C) : 1;
+    const bool f64 = sizeof(T) == 8, pairs = has_pairs(m, E);
+    take(rows.row_of, pairs ? E : 0);
+    take(rows.leaders, pairs ? E : 0);
+    take(rows.count, pairs ? 1 : 0);
+    if (!pairs) rows = EdgeRows{};
+    shares = sp ? spline_chunks<T>((int)C) : (f64 ? (int)C / (32 * pick_vec<T>((int)C)) : 1);
     take(gY0, sp ? shares * E * 16 : 0);
     take(dr0, sp ? shares * E : 0);
     take(Y, E * 16);
@@ -119,8 +131,8 @@ struct Workspace {
     take(gb0, n * C);
     take(gX0, n * 16 * C);
     take(gvec, E * 4);
-    take(gradR, sizeof(T) == 8 && !sp ? E * 4 * C : 0);
-    take(partial, sp ? 0 : cmace_imp_bwd_scratch_elems(E, (int)C, sizeof(T) == 8 ? 1 : 0));
+    take(dR, f64 && !sp ? E * 4 * C : 0);
+    take(partial, f64 || sp || is_fused(m) ? 0 : cmace_imp_bwd_scratch_elems(E, (int)C, 0));
     gm1 = m1;   // the messages are not read again after the Linear
     gA = A;     // nor the sums after their product
   }
@@ -156,7 +168,7 @@ static int run_spline_step(const cmace_step_model &m, cmace_step_io &io, const W
       return StepKernels<T>::edge_prep(io.positions, io.sender, io.receiver, io.shifts, io.shift_index, io.shift_table,
                                        io.shift_rows, io.status, E, m.r_max, 0, m.cutoff_p, table(0), w.geo,
                                        w.basis, w.Y, io.species, io.one_hot, io.one_hot_is_f64, io.n_local, n, Z, w.species,
-                                       w.counts, w.slot_of, w.node_of, w.slot_type, w.elem_start, st);
+                                       w.counts, w.slot_of, w.node_of, w.slot_type, w.elem_start, io.row_ptr, w.rows, st);
     case S_SUMS:
       return spline_messages<T>(senders, w.species, w.Y, at, table(0), io.sender, io.row_ptr, n, w.slot_of, C, w.A, st);
     case S_FOLD: return linear_any(w.A, m.fold, start, Z, n, C, C, w.m0, io.status, st);
@@ -203,8 +215,9 @@ static int run_step(const cmace_step_model &m, cmace_step_io &io, const Workspac
     s.out_v = s.out_t = 1.f;
   }
   if (fused && (step == S_RADIAL_OUT || step == S_RADIAL_BACK)) return CMACE_OK;
+  if (f64 && !is_spline(m) && step == S_RADIAL_BACK) return CMACE_OK;   // part of edges_back
   io.launches++;
-  if (step == S_EDGE_PREP && node_blocks(io.n_local) > 1) io.launches++;
+  if (step == S_EDGE_PREP && (node_blocks(io.n_local) > 1 || w.rows.count)) io.launches++;
   if (is_spline(m)) {
     const int rc = run_spline_step<T>(m, io, w, step, up, st);
     if (rc >= 0) return rc;
@@ -214,12 +227,12 @@ static int run_step(const cmace_step_model &m, cmace_step_io &io, const Workspac
       return K::edge_prep(io.positions, io.sender, io.receiver, io.shifts, io.shift_index, io.shift_table,
                                        io.shift_rows, io.status, E, m.r_max, m.nbessel, m.cutoff_p, SplineTable<T>{}, w.geo,
                           w.basis, w.Y, io.species, io.one_hot, io.one_hot_is_f64, nl, n, Z, w.species, w.counts,
-                          w.slot_of, w.node_of, w.slot_type, w.elem_start, st);
+                          w.slot_of, w.node_of, w.slot_type, w.elem_start, io.row_ptr, w.rows, st);
     case S_RADIAL: {
       const T *rw[2][3];
       for (int i = 0; i < 2; i++)
         for (int k = 0; k < 3; k++) rw[i][k] = static_cast<const T *>(m.radial[i][k]);
-      if constexpr (f64) return radial_pair_f64(w.basis, m.nbessel, rw, 2, E, w.h, w.dh, st);
+      if constexpr (f64) return radial_pair_f64(w.basis, m.nbessel, rw, 2, w.rows, E, w.h, w.dh, st);
       else if (half) {
         const int half_out[2] = {1, fused ? 1 : 0};
         void *const h[2] = {w.h[0], w.h[1]}, *const dh[2] = {w.dh[0], w.dh[1]};
@@ -229,20 +242,23 @@ static int run_step(const cmace_step_model &m, cmace_step_io &io, const Workspac
     case S_SUMS:
       if constexpr (!f64)
         if (half) return step_sums_half(w.h[0], w.Y, io.sender, io.row_ptr, w.species, w.slot_of, n, Z, scales[0].out_v, w.A, st);
-      return K::sums(w.h[0], w.Y, io.sender, io.row_ptr, w.species, w.slot_of, n, Z, w.A, st);
+      return K::sums(w.h[0], w.Y, io.sender, io.row_ptr, w.species, w.slot_of, w.rows.row_of, n, Z, w.A, st);
     case S_FOLD: return linear_any(w.A, m.fold, start, Z, n, ST_H * Z, C, w.m0, io.status, st);
     case S_CONTRACT0: return K::contract_fwd(w.m0, w.slot_type, static_cast<const T *>(m.weff[0]), n, C, w.b0, st);
     case S_MID_FWD:
       return K::mid_fwd(w.b0, w.node_of, w.slot_type, static_cast<const T *>(m.up), static_cast<const T *>(m.extra), n, C,
                         io.up_local ? static_cast<T *>(io.up_local) : w.up, w.q0, st);
     case S_RADIAL_OUT:
-      if constexpr (f64) return cmace_gemm_f64(w.h[1], static_cast<const double *>(m.radial[1][3]), E, ST_H, 4 * C, 1.0, w.R, st);
+      if constexpr (f64)
+        return radial_out_f64(w.h[1], w.dh[1], static_cast<const double *>(m.radial[1][3]), w.rows, E, 4 * C, w.R, w.dR, st);
       else return cmace_gemm3x_f32(w.h[1], static_cast<const float *>(m.radial[1][3]), E, ST_H, 4 * C, 1.0, w.R, io.status, st);
     case S_MESSAGES:
       if constexpr (!f64)
         if (fused)
           return fused_messages(up, w.Y, w.h[1], m.fused_w, scales[1].out_v * m.fused_scale, io.sender, io.receiver,
                                 io.row_ptr, n, E, C, w.m1, io.status, st);
+      if constexpr (f64)
+        if (w.rows.count) return imp_fwd_rows_f64(up, w.Y, w.R, w.rows.row_of, io.sender, io.row_ptr, n, E, C, w.m1, st);
       return imp_fwd<T>(up, w.Y, w.R, io.sender, io.row_ptr, n, E, ys, C, w.m1, st);
     case S_LINEAR: return linear_any(w.m1, m.linear[0], nullptr, 1, n, C, C, w.l1, io.status, st);
     case S_CONTRACT1:
@@ -256,11 +272,12 @@ static int run_step(const cmace_step_model &m, cmace_step_io &io, const Workspac
           return fused_messages_back(up, w.Y, w.gm1, w.h[1], w.dh[1], m.fused_w_back, scales[1].out_v * m.fused_scale,
                                      scales[1].out_t * m.fused_scale, io.sender, io.receiver, E, C, w.T_, w.gY1, io.status,
                                      st);
-      return imp_bwd_edge<T>(up, w.Y, w.R, w.gm1, io.sender, io.row_ptr, n, E, ys, C, f64 ? w.gradR : nullptr, w.gY1,
-                             w.T_, w.partial, st);
-    case S_RADIAL_BACK:
       if constexpr (f64)
-        return gemm_dot_f64(w.gradR, static_cast<const double *>(m.radial_back), w.dh[1], E, 4 * C, ST_H, w.dr1, st);
+        return imp_bwd_edge_pair_f64(up, w.Y, w.R, w.dR, w.rows.row_of, w.gm1, io.sender, io.row_ptr, n, E, C, w.gY1, w.T_, st);
+      else
+        return imp_bwd_edge<T>(up, w.Y, w.R, w.gm1, io.sender, io.row_ptr, n, E, ys, C, nullptr, w.gY1, w.T_, w.partial, st);
+    case S_RADIAL_BACK:
+      if constexpr (f64) return CMACE_OK;   // not reached
       else
         return gemm3x_gradr(up, w.gm1, w.Y, ys, io.sender, io.receiver, static_cast<const float *>(m.radial_back), E, C,
                             ST_H, w.dh[1], w.dr1, io.status, st);
@@ -293,8 +310,8 @@ static int run_step(const cmace_step_model &m, cmace_step_io &io, const Workspac
         if (half)
           return step_sums_bwd_half(w.gA, w.h[0], w.dh[0], w.Y, io.sender, io.row_ptr, w.species, w.slot_of, w.gY1,
                                     fused ? nullptr : w.dr1, w.geo, n, Z, scales[0].out_v, scales[0].out_t, w.gvec, st);
-      return K::sums_bwd(w.gA, w.h[0], w.dh[0], w.Y, io.sender, io.row_ptr, w.species, w.slot_of, w.gY1, w.dr1, w.geo, n,
-                         Z, w.gvec, st);
+      return K::sums_bwd(w.gA, w.h[0], w.dh[0], w.Y, io.sender, io.row_ptr, w.species, w.slot_of, w.rows.row_of, w.gY1, w.shares,
+                         w.dr1, w.geo, n, E, Z, w.gvec, st);
     case S_FORCES:
       return K::forces(w.gvec, io.row_ptr, io.perm, io.send_ptr, n, nl, io.gradient_sign, io.gradient, io.species, Z,
                        io.interaction, io.node_energy, io.status, f64 ? nullptr : staged_stall_flag(), io.sums, st);

@@ -58,6 +58,34 @@ int spline_edges_back(const T *X, const int32_t *row_of, const T *Y, const Splin
                       const int32_t *g_row, const int32_t *sender, const int32_t *row_ptr, int64_t n, int64_t E, int C,
                       T *Tout, T *gY, T *dr, cudaStream_t st);
 
+// Rows of the perceptrons' h and h' shared by edges of one length (step_edges.cu): count of them on the device, the edge that
+// row k belongs to, an edge's row; all null: an edge has a row of its own.  Radial kernels go through the rows and look up
+// what find_pairs left open.
+struct EdgeRows {
+  int32_t *row_of, *leaders, *count;
+};
+#ifdef __CUDACC__
+__device__ __forceinline__ int64_t count_rows(const EdgeRows &rows, int64_t nedges) { return rows.count ? (int64_t)*rows.count : nedges; }
+// the row of the other edge of a pair, in place of its leader; a share of the edges a thread
+__device__ __forceinline__ void resolve_rows(const EdgeRows &rows, int64_t nedges, int64_t thread, int64_t nthreads) {
+  if (!rows.count) return;
+  for (int64_t e = thread; e < nedges; e += nthreads) {
+    const int32_t r = rows.row_of[e];
+    if (r < 0) rows.row_of[e] = rows.row_of[~r];   // a leader's row, which nobody writes here
+  }
+}
+#endif
+
+// radial_out64.cu: R = h W, dR = dh W, float64, for the rows of EdgeRows; W [64, N]
+int radial_out_f64(const double *h, const double *dh, const double *W, const EdgeRows &rows, int64_t nedges, int N, double *R,
+                   double *dR, cudaStream_t st);
+// message_passing.cu: the edge pass with dE/dr from R' in component 0 of gY [chunks, E, 16]; R, dR rows by row_of (or null)
+int imp_bwd_edge_pair_f64(const double *X, const double *Y, const double *R, const double *dR, const int32_t *row_of,
+                          const double *G, const int32_t *sender, const int32_t *row_ptr, int64_t nnodes, int64_t nedges, int C,
+                          double *gY, double *T, cudaStream_t st);
+int imp_fwd_rows_f64(const double *X, const double *Y, const double *R, const int32_t *row_of, const int32_t *sender,
+                     const int32_t *row_ptr, int64_t nnodes, int64_t nedges, int C, double *out, cudaStream_t st);
+
 // status words of inputs that only a kernel sees; what such an input enters comes out as NaN
 constexpr int32_t CMACE_STEP_BAD_SHIFT = 90;     // a row of the shift table that does not exist
 constexpr int32_t CMACE_STEP_BAD_ELEMENT = 91;   // an element index outside 0 .. elements - 1
@@ -76,9 +104,9 @@ struct StepKernels {
                        T *Y,
                        const int32_t *species_in, const void *one_hot, int one_hot_f64, int64_t n_local, int64_t n_owned,
                        int elements, int32_t *species, int32_t *counts, int32_t *slot_of, int32_t *node_of,
-                       int32_t *slot_type, int32_t *elem_start, cudaStream_t st);
+                       int32_t *slot_type, int32_t *elem_start, const int32_t *row_ptr, const EdgeRows &rows, cudaStream_t st);
   static int sums(const T *h, const T *Y, const int32_t *sender, const int32_t *row_ptr, const int32_t *species,
-                  const int32_t *slot_of, int64_t nnodes, int elements, T *A, cudaStream_t st);
+                  const int32_t *slot_of, const int32_t *row_of, int64_t nnodes, int elements, T *A, cudaStream_t st);
   static int contract_fwd(const T *X, const int32_t *types, const T *weff, int64_t n, int C, T *b, cudaStream_t st);
   static int contract_bwd(const T *X, const int32_t *types, const T *weff, const T *gb, int64_t n, int C, T *gX,
                           cudaStream_t st);
@@ -90,8 +118,8 @@ struct StepKernels {
   static int mid_bwd(const T *gup, const int32_t *node_of, const int32_t *slot_type, const T *dq, const T *wu_t,
                      const T *extra_t, double scale, int64_t n, int C, T *gb, cudaStream_t st);
   static int sums_bwd(const T *gA, const T *h, const T *dh, const T *Y, const int32_t *sender, const int32_t *row_ptr,
-                      const int32_t *species, const int32_t *slot_of, const T *gY1, const T *dr1, const Quad<T> *geo,
-                      int64_t nnodes, int elements, T *gvec, cudaStream_t st);
+                      const int32_t *species, const int32_t *slot_of, const int32_t *row_of, const T *gY1, int shares, const T *dr1,
+                      const Quad<T> *geo, int64_t nnodes, int64_t nedges, int elements, T *gvec, cudaStream_t st);
   static int forces(const T *gvec, const int32_t *row_ptr, const int32_t *perm, const int32_t *send_ptr, int64_t nrecv,
                     int64_t nsend, double sign, double *out, const int32_t *species_in, int elements, double *inter,
                     double *node_energy, const int32_t *status, const int *stalled, double *sums, cudaStream_t st);

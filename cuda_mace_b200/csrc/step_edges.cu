@@ -140,13 +140,105 @@ __device__ void group_nodes(int64_t first, int64_t end, int blocks, int block, b
   }
 }
 
+// ---- edges that share a length ------------------------------------------------------------------------------------
+// An edge j -> i and its reverse i -> j have the same length bit for bit (their vectors are exact negatives), so both
+// perceptrons' rows h and h' are the same: they are formed once a pair.  In a complete list that is half of the radial work; an
+// edge whose reverse is missing (an incomplete list, a ghost sender) keeps a row of its own, and no row is shared on anything but
+// the equality of the vectors of this call.
+//
+// Of a pair the edge with the lower receiver leads; the other looks for it in its sender's row of the list: a warp asks the rows
+// of eight of its edges at a time, lanes beside one another, the first edge that matches is the leader.  Leaders are numbered as
+// they come, a block at a time (rows do not depend on one another, so their places need not be the same in every call):
+// leaders[k] is the edge of row k, row_of[e] the row of a leader, and ~leader for the other edge of a pair until the radial kernel
+// looks its row up (resolve_rows).  The search is a chain of four dependent loads and a ballot an edge: 14 us for 416 000 edges, 8
+// for 9 900; with the vectors compared for four edges one after the other it took 39 and 20.
+template <typename T>
+__device__ __forceinline__ void find_pairs(int64_t first, const int32_t *__restrict__ sender, const int32_t *__restrict__ receiver,
+                                           const int32_t *__restrict__ row_ptr, const Quad<T> *__restrict__ geo, int64_t nedges,
+                                           int32_t *__restrict__ row_of, int32_t *__restrict__ leaders, int32_t *count) {
+  __shared__ int32_t found[EP_THREADS / 32], start;
+  const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+  const int64_t e = first + threadIdx.x;
+  const bool valid = e < nedges;
+  int s = 0, r = 0, k0 = 0, k1 = 0, leader = -1;
+  Quad<T> q{};
+  if (valid) {
+    s = sender[e];
+    r = receiver[e];
+    q = geo[e];
+  }
+  const bool looks = valid && s < r;   // then the sender receives too
+  if (looks) {
+    k0 = row_ptr[s];
+    k1 = row_ptr[s + 1];
+  }
+  unsigned open = __ballot_sync(0xffffffffu, looks);
+  for (int at = 0; open != 0; at += 64) {
+    unsigned hits[2] = {0, 0};   // candidates at .. at + 63 with the right sender, of this lane's edge
+    for (unsigned todo = open; todo != 0;) {
+      constexpr int AT = 8;      // rows on their way together
+      int src[AT], cand[AT][2];
+#pragma unroll
+      for (int u = 0; u < AT; u++) {
+        src[u] = todo ? __ffs(todo) - 1 : -1;
+        todo &= todo - 1;
+        const int c = __shfl_sync(0xffffffffu, k0, src[u] & 31) + at + lane, hi = __shfl_sync(0xffffffffu, k1, src[u] & 31);
+        cand[u][0] = src[u] >= 0 && c < hi ? __ldg(sender + c) : -1;
+        cand[u][1] = src[u] >= 0 && c + 32 < hi ? __ldg(sender + c + 32) : -1;
+      }
+#pragma unroll
+      for (int u = 0; u < AT; u++) {
+        if (src[u] < 0) break;
+        const int want = __shfl_sync(0xffffffffu, r, src[u]);
+        const unsigned m0 = __ballot_sync(0xffffffffu, cand[u][0] == want), m1 = __ballot_sync(0xffffffffu, cand[u][1] == want);
+        if (lane == src[u]) {
+          hits[0] = m0;
+          hits[1] = m1;
+        }
+      }
+    }
+    // every lane for itself: nearly always one candidate, several where images of an atom are neighbours
+#pragma unroll
+    for (int h = 0; h < 2; h++)
+      while (leader < 0 && hits[h] != 0) {
+        const int c = k0 + at + 32 * h + __ffs(hits[h]) - 1;
+        hits[h] &= hits[h] - 1;
+        const Quad<T> v = geo[c];
+        if (v.x == -q.x && v.y == -q.y && v.z == -q.z && v.w == q.w) leader = c;
+      }
+    __syncwarp();
+    open = __ballot_sync(0xffffffffu, looks && leader < 0 && k0 + at + 64 < k1);
+  }
+  const bool leads = valid && leader < 0;
+  const unsigned mine = __ballot_sync(0xffffffffu, leads);
+  if (lane == 0) found[w] = __popc(mine);
+  __syncthreads();
+  if (threadIdx.x == 0) {
+    int n = 0;
+    for (int k = 0; k < EP_THREADS / 32; k++) n += found[k];
+    start = atomicAdd(count, n);
+  }
+  __syncthreads();
+  int row = start + __popc(mine & ((1u << lane) - 1u));
+  for (int k = 0; k < w; k++) row += found[k];
+  if (leads) leaders[row] = (int32_t)e;
+  if (valid) row_of[e] = leads ? row : ~leader;
+}
+
+// What has to wait for edge_prep's counts and vectors: with several node blocks the grouping of the nodes, and the pairs
+template <typename T>
 __global__ void __launch_bounds__(EP_THREADS)
-    group_nodes_kernel(int64_t n_owned, int elements, const int32_t *species, int32_t *counts, int32_t *slot_of,
-                       int32_t *node_of, int32_t *slot_type, int32_t *elem_start) {
+    group_kernel(int64_t n_owned, int grouping, int elements, const int32_t *species, int32_t *counts, int32_t *slot_of,
+                 int32_t *node_of, int32_t *slot_type, int32_t *elem_start, const int32_t *sender, const int32_t *receiver,
+                 const int32_t *row_ptr, const Quad<T> *geo, int64_t nedges, int32_t *row_of, int32_t *leaders, int32_t *count) {
   grid_begin();
-  const int64_t first = (int64_t)blockIdx.x * GN_NODES;
-  group_nodes(first, first + GN_NODES < n_owned ? first + GN_NODES : n_owned, (int)gridDim.x, (int)blockIdx.x, false, elements,
-              species, counts, slot_of, node_of, slot_type, elem_start);
+  if ((int)blockIdx.x < grouping) {
+    const int64_t first = (int64_t)blockIdx.x * GN_NODES;
+    group_nodes(first, first + GN_NODES < n_owned ? first + GN_NODES : n_owned, grouping, (int)blockIdx.x, false, elements,
+                species, counts, slot_of, node_of, slot_type, elem_start);
+    return;
+  }
+  find_pairs<T>(((int64_t)blockIdx.x - grouping) * EP_THREADS, sender, receiver, row_ptr, geo, nedges, row_of, leaders, count);
 }
 
 // A warp's 32 rows of N values each, one row per lane, to consecutive memory: through shared memory, so that a store
@@ -182,8 +274,9 @@ __global__ void __launch_bounds__(EP_THREADS, sizeof(T) == 4 ? 5 : 3)
                      int p, const SplineTable<T> spline, Quad<T> *__restrict__ geo, T *__restrict__ basis, T *__restrict__ Y,
                      const int32_t *species_in, const void *one_hot, int one_hot_f64, int64_t n_local, int64_t n_owned,
                      int elements, int32_t *species, int32_t *counts, int32_t *slot_of, int32_t *node_of,
-                     int32_t *slot_type, int32_t *elem_start) {
+                     int32_t *slot_type, int32_t *elem_start, int32_t *pair_count) {
   grid_begin();
+  if (pair_count && blockIdx.x == 0 && threadIdx.x == 0) *pair_count = 0;
   const int nblocks = (int)node_blocks(n_local);
   if ((int)blockIdx.x < nblocks) {
     const int64_t first = (int64_t)blockIdx.x * GN_NODES, end = first + GN_NODES;
@@ -248,7 +341,8 @@ int StepKernels<T>::edge_prep(const double *pos, const int32_t *sender, const in
                               T *basis, T *Y,
                               const int32_t *species_in, const void *one_hot, int one_hot_f64, int64_t n_local,
                               int64_t n_owned, int elements, int32_t *species, int32_t *counts, int32_t *slot_of, int32_t *node_of,
-                              int32_t *slot_type, int32_t *elem_start, cudaStream_t st) {
+                              int32_t *slot_type, int32_t *elem_start, const int32_t *row_ptr, const EdgeRows &rows,
+                              cudaStream_t st) {
   const int64_t blocks = node_blocks(n_local) + (nedges + EP_THREADS - 1) / EP_THREADS;
   const size_t smem = (size_t)EP_THREADS * ((nb == 16 ? 32 : 16) * sizeof(T) + 16);
   auto kern = nb == 16 ? edge_prep_kernel<T, 16> : (nb == 8 ? edge_prep_kernel<T, 8> : edge_prep_kernel<T, 0>);
@@ -257,10 +351,13 @@ int StepKernels<T>::edge_prep(const double *pos, const int32_t *sender, const in
   launch_chained(kern, (unsigned)blocks, EP_THREADS, smem, st, pos, sender, receiver, shifts, shift_index, shift_table,
                  (int)(shift_rows < 256 ? shift_rows : 256), status, nedges, (T)r_max, p, spline, geo, basis, Y, species_in, one_hot,
                  one_hot_f64, n_local, n_owned, elements, species, counts, slot_of, node_of, slot_type,
-                 elem_start);
-  if (node_blocks(n_local) > 1)
-    launch_chained(group_nodes_kernel, (unsigned)node_blocks(n_owned), EP_THREADS, 0, st, n_owned, elements,
-                   species, counts, slot_of, node_of, slot_type, elem_start);
+                 elem_start, rows.count);
+  const int64_t grouping = node_blocks(n_local) > 1 ? node_blocks(n_owned) : 0;
+  const int64_t pairs = rows.count ? (nedges + EP_THREADS - 1) / EP_THREADS : 0;
+  if (grouping + pairs > 0)
+    launch_chained(group_kernel<T>, (unsigned)(grouping + pairs), EP_THREADS, 0, st, n_owned, (int)grouping, elements, species, counts,
+                   slot_of, node_of, slot_type, elem_start, sender, receiver, row_ptr, geo, nedges, rows.row_of, rows.leaders,
+                   rows.count);
   return check_launch("cmace_step(edge_prep)");
 }
 
@@ -313,6 +410,34 @@ __device__ __forceinline__ void for_edges_of_element(const SenderElements &from,
   __syncwarp();
   if (n > 0) body(n);
 }
+
+// Rows of h and h' of a receiver's edges (EdgeRows; null: an edge's own).  Those of the first 64 wait in shared memory, where
+// asynchronous copies bring them: in registers they cost these kernels a block an SM.
+struct SharedRows {
+  const int32_t *__restrict__ row_of;
+  int32_t *first;
+  int32_t e0;
+  __device__ __forceinline__ SharedRows(const int32_t *__restrict__ row_of_, int32_t *first_, const SenderElements &from)
+      : row_of(row_of_), first(first_), e0((int32_t)from.e0) {
+#pragma unroll
+    for (int i = 0; i < 64; i += 32)
+      if (from.e0 + i + from.lane < from.e1) {
+        if (row_of)
+          asm volatile("cp.async.ca.shared.global [%0], [%1], 4;" ::"r"(smem_u32(first + i + from.lane)),
+                       "l"(row_of + from.e0 + i + from.lane)
+                       : "memory");
+        else
+          first[i + from.lane] = e0 + i + from.lane;
+      }
+  }
+  __device__ __forceinline__ void wait() const {
+    asm volatile("cp.async.wait_all;" ::: "memory");
+    __syncwarp();
+  }
+  __device__ __forceinline__ int64_t operator[](int32_t e) const {
+    return e - e0 < 64 ? first[e - e0] : (row_of ? __ldg(row_of + e) : e);
+  }
+};
 
 // 32 bytes of one lane in one store.  The lanes of a result tile hold 64 bytes of a row each: in 16-byte stores every
 // instruction half-fills 32 sectors, which L2 takes as 2.5 times the writes (10.2 million sectors for 131 MB).
@@ -531,27 +656,30 @@ int step_sums_half(const void *h, const float *Y, const int32_t *sender, const i
 __global__ void __launch_bounds__(SU_WARPS * 32)
     sums_f64_kernel(const double *__restrict__ h, const double *__restrict__ Y, const int32_t *__restrict__ sender,
                 const int32_t *__restrict__ row_ptr, const int32_t *__restrict__ species,
-                const int32_t *__restrict__ slot_of, int64_t nnodes, int elements, double *__restrict__ A) {
+                const int32_t *__restrict__ slot_of, const int32_t *__restrict__ row_of, int64_t nnodes, int elements,
+                double *__restrict__ A) {
   grid_begin();
-  __shared__ int32_t lists[SU_WARPS][SU_LIST];
+  __shared__ int32_t lists[SU_WARPS][SU_LIST], first_rows[SU_WARPS][64];
   const int lane = threadIdx.x & 31, w = threadIdx.x >> 5, g = lane >> 2, t = lane & 3;
   const int64_t pair = (int64_t)blockIdx.x * SU_WARPS + w;
   if (pair >= nnodes * elements) return;
   const int64_t node = pair / elements;
   const int z = (int)(pair - node * elements);
   SenderElements from(sender, species, row_ptr[node], row_ptr[node + 1], lane);
+  const SharedRows rows(row_of, first_rows[w], from);
   int32_t *list = lists[w];
   double acc[2][8][2];
 #pragma unroll
   for (int j = 0; j < 8; j++) acc[0][j][0] = acc[0][j][1] = acc[1][j][0] = acc[1][j][1] = 0.0;
   from.look_up();
+  rows.wait();
   for_edges_of_element(from, z, list, [&](int n) {
     double2 hv[4];
     double yv[2];
     auto load = [&](int j0) {   // edge j0 + t; past the end: the last edge with Y = 0
       const int j = j0 + t;
       const int64_t e = list[j < n ? j : n - 1];
-      const double2 *hp = reinterpret_cast<const double2 *>(h + e * ST_H + 8 * g);
+      const double2 *hp = reinterpret_cast<const double2 *>(h + rows[e] * ST_H + 8 * g);
 #pragma unroll
       for (int u = 0; u < 4; u++) hv[u] = __ldg(hp + u);
       yv[0] = j < n ? __ldg(Y + e * 16 + g) : 0.0;
@@ -589,13 +717,14 @@ __global__ void __launch_bounds__(SU_WARPS * 32)
 
 template <typename T>
 int StepKernels<T>::sums(const T *h, const T *Y, const int32_t *sender, const int32_t *row_ptr, const int32_t *species,
-                         const int32_t *slot_of, int64_t nnodes, int elements, T *A, cudaStream_t st) {
+                         const int32_t *slot_of, const int32_t *row_of, int64_t nnodes, int elements, T *A, cudaStream_t st) {
   const int64_t blocks = (nnodes * elements + SU_WARPS - 1) / SU_WARPS;
   if (blocks > 0) {
     if constexpr (sizeof(T) == 4)
       launch_chained(sums_tf32_kernel, (unsigned)blocks, SU_WARPS * 32, 0, st, h, Y, sender, row_ptr, species, slot_of, nnodes, elements, A);
     else
-      launch_chained(sums_f64_kernel, (unsigned)blocks, SU_WARPS * 32, 0, st, h, Y, sender, row_ptr, species, slot_of, nnodes, elements, A);
+      launch_chained(sums_f64_kernel, (unsigned)blocks, SU_WARPS * 32, 0, st, h, Y, sender, row_ptr, species, slot_of, row_of, nnodes,
+                     elements, A);
   }
   return check_launch("cmace_step(sums)");
 }
@@ -607,9 +736,17 @@ int StepKernels<T>::sums(const T *h, const T *Y, const int32_t *sender, const in
 // lane j of the warp: edge list[j], its 16 + 1 sums in st[j * 17 ..], to the gradient of the edge's vector
 template <typename T>
 __device__ __forceinline__ void finish_edge(const T *st, int64_t e, const T *__restrict__ gY1, const T *__restrict__ dr1,
-                                            const Quad<T> *__restrict__ geo, T *__restrict__ gvec) {
+                                            const Quad<T> *__restrict__ geo, T *__restrict__ gvec, int shares = 1,
+                                            int64_t nedges = 0) {
   T g[16];
   load_row16(gY1 + e * 16, g);
+  for (int k = 1; k < shares; k++) {   // gY1 [shares, E, 16]
+#pragma unroll
+    for (int i = 0; i < 4; i++) {
+      const Quad<T> more = reinterpret_cast<const Quad<T> *>(gY1 + (k * nedges + e) * 16)[i];
+      g[4 * i] += more.x, g[4 * i + 1] += more.y, g[4 * i + 2] += more.z, g[4 * i + 3] += more.w;
+    }
+  }
   // without an array of its own the second layer's dE/dr is component 0 of its grad Y (Y_00 is constant)
   const T dr = st[16] + (dr1 != nullptr ? dr1[e] : g[0]);
 #pragma unroll
@@ -874,14 +1011,15 @@ int step_sums_bwd_half(const float *gA, const void *h, const void *dh, const flo
 // registers; K step s of lane (g, t) is k = 16 t + s, so that a lane reads 16 consecutive values of its edge's row (and of
 // P's rows g and g + 8).  With fma instructions an edge cost 21 shuffles of two words and eight loads of Y: 404 us at
 // 8 000 atoms, 37 us at 192, where its bytes need 115 us at 8 000; now 261 and 20 us.
-__global__ void __launch_bounds__(SU_WARPS * 32)
+__global__ void __launch_bounds__(SU_WARPS * 32, 3)
     sums_bwd_f64_kernel(const double *__restrict__ gA, const double *__restrict__ h, const double *__restrict__ dh,
                     const double *__restrict__ Y, const int32_t *__restrict__ sender, const int32_t *__restrict__ row_ptr,
                     const int32_t *__restrict__ species, const int32_t *__restrict__ slot_of,
-                    const double *__restrict__ gY1, const double *__restrict__ dr1, const Quad<double> *__restrict__ geo,
-                    int64_t nnodes, int elements, double *__restrict__ gvec) {
+                    const int32_t *__restrict__ row_of, const double *__restrict__ gY1, int shares,
+                    const Quad<double> *__restrict__ geo, int64_t nnodes, int64_t nedges, int elements,
+                    double *__restrict__ gvec) {
   grid_begin();
-  __shared__ int32_t lists[SU_WARPS][SU_LIST];
+  __shared__ int32_t lists[SU_WARPS][SU_LIST], first_rows[SU_WARPS][64];
   __shared__ double stage[SU_WARPS][32 * 17];
   const int lane = threadIdx.x & 31, w = threadIdx.x >> 5, g = lane >> 2, t = lane & 3;
   const int64_t pair = (int64_t)blockIdx.x * SU_WARPS + w;
@@ -889,6 +1027,7 @@ __global__ void __launch_bounds__(SU_WARPS * 32)
   const int64_t node = pair / elements;
   const int z = (int)(pair - node * elements);
   SenderElements from(sender, species, row_ptr[node], row_ptr[node + 1], lane);
+  const SharedRows rows(row_of, first_rows[w], from);
   int32_t *list = lists[w];
   double *st = stage[w];
   double2 P[2][8];
@@ -901,16 +1040,17 @@ __global__ void __launch_bounds__(SU_WARPS * 32)
       for (int q = 0; q < 8; q++) P[i][q] = __ldg(reinterpret_cast<const double2 *>(p + (g + 8 * i) * width) + q);
   }
   from.look_up();
+  rows.wait();
   for_edges_of_element(from, z, list, [&](int n) {
     for (int j0 = 0; j0 < n; j0 += 32) {
       const int nj = n - j0 < 32 ? n - j0 : 32;
       if (lane < nj) {   // what finish_edge reads
-        prefetch_l1(gY1 + (int64_t)list[j0 + lane] * 16);
+        for (int k = 0; k < shares; k++) prefetch_l1(gY1 + (k * nedges + list[j0 + lane]) * 16);
         prefetch_l1(geo + list[j0 + lane]);
       }
       for (int j = 0; j < nj; j += 8) {
         const int i = j0 + j + g;   // this lane's row of h: that edge, or the last one
-        const int64_t e = list[i < n ? i : n - 1];
+        const int64_t e = rows[list[i < n ? i : n - 1]];
         const double2 *hp = reinterpret_cast<const double2 *>(h + e * ST_H + 16 * t);
         const double2 *dp = reinterpret_cast<const double2 *>(dh + e * ST_H + 16 * t);
         double2 hv[8], dv[8];
@@ -952,7 +1092,7 @@ __global__ void __launch_bounds__(SU_WARPS * 32)
         }
       }
       __syncwarp();
-      if (lane < nj) finish_edge<double>(st + lane * 17, list[j0 + lane], gY1, dr1, geo, gvec);
+      if (lane < nj) finish_edge<double>(st + lane * 17, list[j0 + lane], gY1, nullptr, geo, gvec, shares, nedges);
       __syncwarp();
     }
   });
@@ -960,8 +1100,9 @@ __global__ void __launch_bounds__(SU_WARPS * 32)
 
 template <typename T>
 int StepKernels<T>::sums_bwd(const T *gA, const T *h, const T *dh, const T *Y, const int32_t *sender,
-                             const int32_t *row_ptr, const int32_t *species, const int32_t *slot_of, const T *gY1,
-                             const T *dr1, const Quad<T> *geo, int64_t nnodes, int elements, T *gvec, cudaStream_t st) {
+                             const int32_t *row_ptr, const int32_t *species, const int32_t *slot_of, const int32_t *row_of,
+                             const T *gY1, int shares, const T *dr1, const Quad<T> *geo, int64_t nnodes, int64_t nedges, int elements,
+                             T *gvec, cudaStream_t st) {
   const int64_t blocks = (nnodes * elements + SU_WARPS - 1) / SU_WARPS;
   if (blocks > 0) {
     if constexpr (sizeof(T) == 4)
@@ -969,7 +1110,7 @@ int StepKernels<T>::sums_bwd(const T *gA, const T *h, const T *dh, const T *Y, c
                                                                       gY1, dr1, geo, nnodes, elements, gvec);
     else
       launch_chained(sums_bwd_f64_kernel, (unsigned)blocks, SU_WARPS * 32, 0, st, gA, h, dh, Y, sender, row_ptr, species, slot_of,
-                                                                     gY1, dr1, geo, nnodes, elements, gvec);
+                     row_of, gY1, shares, geo, nnodes, nedges, elements, gvec);
   }
   return check_launch("cmace_step(sums_bwd)");
 }
@@ -1110,12 +1251,13 @@ int StepKernels<T>::forces(const T *gvec, const int32_t *row_ptr, const int32_t 
                                          int, const SplineTable<T> &, Quad<T> *, T *, T *, const int32_t *,         \
                                          const void *, int,                                                         \
                                          int64_t, int64_t, int, int32_t *, int32_t *, int32_t *, int32_t *,         \
-                                         int32_t *, int32_t *, cudaStream_t);                                                  \
+                                         int32_t *, int32_t *, const int32_t *, const EdgeRows &, cudaStream_t);    \
   template int StepKernels<T>::sums(const T *, const T *, const int32_t *, const int32_t *, const int32_t *,        \
-                                    const int32_t *, int64_t, int, T *, cudaStream_t);                              \
+                                    const int32_t *, const int32_t *, int64_t, int, T *, cudaStream_t);             \
   template int StepKernels<T>::sums_bwd(const T *, const T *, const T *, const T *, const int32_t *,                \
-                                        const int32_t *, const int32_t *, const int32_t *, const T *, const T *,    \
-                                        const Quad<T> *, int64_t, int, T *, cudaStream_t);                          \
+                                        const int32_t *, const int32_t *, const int32_t *, const int32_t *,         \
+                                        const T *, int, const T *, const Quad<T> *, int64_t, int64_t, int, T *,     \
+                                        cudaStream_t);                                                              \
   template int StepKernels<T>::forces(const T *, const int32_t *, const int32_t *, const int32_t *, int64_t,        \
                                       int64_t, double, double *, const int32_t *, int, double *, double *,          \
                                       const int32_t *, const int *, double *, cudaStream_t);

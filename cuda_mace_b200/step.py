@@ -295,7 +295,7 @@ class StepPlan:
                 steps = C // 16
                 wt = L1.W_radial3.t().reshape(4, steps, 4, 2, 2, _H).permute(1, 0, 3, 2, 4, 5).reshape(steps, 64, _H)
                 m.fused_w_back = hold(torch.stack([half_images(b, scale) for b in wt]))
-        m.radial_back = matrix(L1.W_radial3.t())
+            m.radial_back = matrix(L1.W_radial3.t())
         w4 = d(L0.W_radial3).view(_H, 4, C)
         fold = torch.einsum("zc,klc,rlcd->rlzkd", x, w4, lin).reshape(Z, 4, Z * _H, C)
         m.fold = matrix(fold)

@@ -385,7 +385,7 @@ typedef struct cmace_step_model {
   int32_t fused_layout;      /* 128 channels: CMACE_FUSED_LAYOUT, fewer: CMACE_FUSED_LAYOUT_NARROW.  With any other value, such as
                                 the 0 of a caller that lays fused_w_back out as earlier libraries read it (steps of 8 channels),
                                 neither array is read and the second layer's radial weights are written */
-  const void *radial_back;   /* second layer's W4 for the gradient: float32 packed W4 itself, float64 W4^T [4C,64] */
+  const void *radial_back;   /* float32: second layer's W4 for the gradient, packed; not read in float64 */
   const void *spline[2];     /* tabulated radial weights: coefficients [intervals][4][4C] of both layers, or NULL; then the
                                 radial weights above are not read, fold is the first layer's Linear [elements][4] [C, C]
                                 and fold_back[0] its transposes */

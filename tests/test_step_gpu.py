@@ -148,6 +148,52 @@ def test_second_layer_over_many_tiles(U, channels, degrees):
     assert float((out["forces"] + g).abs().max()) < 1e-4 * float(g.abs().max())
 
 
+def _images(n, side, seed):
+    """Every edge of n atoms in a cell that is hardly longer than the cutoff: several images of a neighbour in a receiver's row,
+    atoms that are their own neighbours, rows of many more than 64 edges."""
+    pos = np.random.default_rng(seed).uniform(0, side, (n, 3))
+    cells = np.stack(np.meshgrid(*[np.arange(-2, 3)] * 3, indexing="ij"), -1).reshape(-1, 3) * side
+    recv, send, shift = [], [], []
+    for i in range(n):
+        d = pos[None] + cells[:, None] - pos[i]
+        r = np.linalg.norm(d, axis=-1)
+        k, j = np.nonzero((r > 1e-9) & (r < 5.0))
+        recv.append(np.full(j.size, i)), send.append(j), shift.append(cells[k])
+    return pos, np.stack([np.concatenate(recv), np.concatenate(send)]), np.concatenate(shift)
+
+
+# An edge and its reverse share the rows of the radial perceptrons where both are in the list: a complete list, one with every
+# third edge missing (a reverse that is not there), one with edges twice and a row shuffled, one with ghost-like one-way edges.
+# Against the operators in float64, which know of no pairs: rounding over the chain, as in the tests above.
+@pytest.mark.parametrize("kind", ["complete", "missing", "twice", "one way"])
+@pytest.mark.parametrize("channels", [32, 64, 96])
+def test_edges_that_share_a_length(U, kind, channels):
+    pos, ei, sh = _images(130, 7.0, 3)
+    rng = np.random.default_rng(4)
+    keep = np.arange(ei.shape[1])
+    if kind == "missing":
+        keep = keep[rng.random(keep.size) > 0.33]
+    elif kind == "one way":
+        keep = keep[ei[0] <= ei[1]]
+    elif kind == "twice":
+        keep = np.concatenate([keep, rng.choice(keep, 2000)])
+        keep = rng.permutation(keep)
+    keep = keep[np.argsort(ei[0][keep], kind="stable")]
+    ei, sh = torch.from_numpy(ei[:, keep].astype(np.int32)).cuda(), torch.from_numpy(sh[keep]).cuda()
+    assert ei.shape[1] > 74 * 16 * 8
+    mace = model.InvariantMACE(systems.init_params(channels, 3, 7), U, dtype=torch.float64, device="cuda")
+    p = torch.from_numpy(pos).cuda()
+    species = torch.from_numpy(rng.integers(0, 3, pos.shape[0]).astype(np.int32)).cuda()
+    out = mace(dict(positions=p, species=species, edge_index=ei, shifts=sh))
+    assert step.plan_of(mace) is not None
+    p.requires_grad_(True)
+    energies = mace.node_energies(p, species, ei, sh)
+    (g,) = torch.autograd.grad(energies.sum(), p)
+    energies = energies.detach()
+    assert abs(float(out["interaction_energy"] - energies.sum())) < 1e-12 * float(energies.abs().sum())
+    assert float((out["forces"] + g).abs().max()) < 1e-11 * float(g.abs().max())
+
+
 # below and above the 32 768 edges from which a new list's grouping by sender runs beside the step
 @pytest.mark.parametrize("n", [300, 1100])
 def test_new_list_and_host_batch(U, n):
