@@ -16,6 +16,10 @@
 // (l', even), (l', odd).  Every quarter then works for eight components of two channels a lane: an edge costs 32 + 2
 // wavefronts of Y instead of 64.
 //
+// Rows of h that two edges share (EdgeRows) come by the loader's asynchronous copies into the swizzled images, as fast as boxes
+// of consecutive rows (256 and 254 us at 16 000 atoms; four rows an instruction by TMA, from a warp of its own, 281; at 32 channels
+// 177 against 113).  The lanes' copies and the tensor core's reads are ordered by a proxy fence of the thread that issues the MMAs.
+//
 // A set's loader has to keep up with four consumer warps: its part of the list is in registers a tile ahead, a lane's rows are
 // its own (a shuffle per row: 112 cycles a copy instead of about 30), and the MMAs come from one thread that asks its barriers
 // itself.  317 -> 254 us at 16 000 atoms (833 000 edges), 1 320 -> 1 046 at 64 000, 80 -> 66 at 3 000, 264 -> 240 for 412 000
@@ -138,8 +142,9 @@ __device__ __forceinline__ void issue_tile(uint32_t tmem, uint32_t acc, uint32_t
 // A set owns a contiguous range of receivers, so no sum is split and none is atomic; its warps keep up to 16 sums a lane.
 struct FusedMessagesArgs {
   const float *X, *Y;            // [Ns, C], [E, 16]
+  const char *h;                 // rows of [hi 64 | lo 64] fp16
   const uint4 *W;                // permuted W^T
-  const int32_t *sender, *receiver, *row_ptr;
+  const int32_t *sender, *receiver, *row_ptr, *row_of;   // row_of: an edge's row of h; null: its own
   int32_t *status;
   int64_t nnodes, nedges;
   float factor;                  // undoes the powers of two of h and W
@@ -289,7 +294,7 @@ __global__ void __launch_bounds__(FusedShape<C>::THREADS, 1)
   const int tid = threadIdx.x, warp = uniform(tid >> 5), lane = tid & 31;
   // warps 0-3, 4-7, ..: consumers of sets 0, 1, ..; then the sets' MMA warps, then their loaders
   constexpr int MMA0 = 4 * SETS, LOADER0 = 5 * SETS;
-  const int set = warp < MMA0 ? warp >> 2 : (warp < LOADER0 ? warp - MMA0 : warp - LOADER0);
+  const int set = warp < MMA0 ? warp >> 2 : (warp - MMA0) % SETS;
   const uint32_t h_full = smem_u32(&bars[set][0]), x_full = h_full + 8u * STAGES, st_free = x_full + 8u * STAGES;
   const uint32_t acc_full = st_free + 8u * STAGES, acc_free = acc_full + 8u * ACCS;
   const uint32_t stages = smem_base + (uint32_t)(set * STAGES) * S::STAGE_BYTES;
@@ -298,7 +303,7 @@ __global__ void __launch_bounds__(FusedShape<C>::THREADS, 1)
     for (int k = 0; k < SETS; k++) {
       const uint32_t b = smem_u32(&bars[k][0]);
       for (int s = 0; s < STAGES; s++) {
-        mbar_init(b + 8u * s, 1);
+        mbar_init(b + 8u * s, g.row_of ? 32 : 1);      // h: the loader's lanes, or its expect_tx
         mbar_init(b + 8u * (STAGES + s), 33);          // the loader's 32 lanes and its expect_tx
         mbar_init(b + 8u * (2 * STAGES + s), 4);
       }
@@ -343,16 +348,21 @@ __global__ void __launch_bounds__(FusedShape<C>::THREADS, 1)
   };
 
   if (warp >= LOADER0) {
-    // ---- loader: h rows by TMA, Y rows as one bulk copy, sender rows by asynchronous copies (lane: rows lane / 4 + 8 i, of
-    // every 64 bytes the 16 at lane % 4); the next tile's part of the list is on its way meanwhile
+    // ---- loader: Y rows as one bulk copy, sender rows by asynchronous copies (lane: rows lane / 4 + 8 i, of every 64 bytes
+    // the 16 at lane % 4); rows of h the same way into the swizzled images, or as two boxes where an edge has a row of its own;
+    // the next tile's part of the list is on its way meanwhile
     const int rr = lane >> 2;
     constexpr int ROWS = TILE / 8, WORDS = TILE / 32;
-    int send[ROWS], r[WORDS], rn[WORDS];
+    int send[ROWS], hrow[ROWS], r[WORDS], rn[WORDS];
     auto load_list = [&](int64_t t) {
       const int64_t base = e0 + t * TILE;
       auto at = [&](int64_t e) { return e < e1 ? e : e1 - 1; };
 #pragma unroll
       for (int i = 0; i < ROWS; i++) send[i] = __ldg(g.sender + at(base + rr + 8 * i));
+      if (g.row_of) {
+#pragma unroll
+        for (int i = 0; i < ROWS; i++) hrow[i] = __ldg(g.row_of + at(base + rr + 8 * i));
+      }
 #pragma unroll
       for (int k = 0; k < WORDS; k++) {
         const int64_t e = base + 32 * k + lane;
@@ -371,15 +381,29 @@ __global__ void __launch_bounds__(FusedShape<C>::THREADS, 1)
         receiver[k] = r[k];
       }
       const float *src[ROWS];
+      const char *hsrc[ROWS];
 #pragma unroll
-      for (int i = 0; i < ROWS; i++) src[i] = g.X + (int64_t)send[i] * C + 4 * (lane & 3);
+      for (int i = 0; i < ROWS; i++) {
+        src[i] = g.X + (int64_t)send[i] * C + 4 * (lane & 3);
+        hsrc[i] = g.h + (int64_t)hrow[i] * 256 + 16 * (lane & 3);
+      }
       if (t + 1 < ntiles) load_list(t + 1);
       if (!warp_wait_all(st_free + 8u * stage, phase ^ 1, lane)) {
         if (lane == 0 && g.status) atomicCAS(g.status, 0, 41);
         break;
       }
       const uint32_t sX = stages + (uint32_t)stage * S::STAGE_BYTES, sH = sX + S::X_BYTES, sY = sH + S::H_BYTES;
-      if (elect_one()) {
+      if (g.row_of) {
+#pragma unroll
+        for (int k = 0; k < 4; k++)   // 64 bytes of hi, 64 more, the same of lo
+#pragma unroll
+          for (int i = 0; i < ROWS; i++)
+            asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(sH + (k >> 1) * (S::H_BYTES / 2) +
+                                                                          (uint32_t)sw128_offset(rr + 8 * i, (lane & 3) + 4 * (k & 1))),
+                         "l"(hsrc[i] + 64 * k)
+                         : "memory");
+        asm volatile("cp.async.mbarrier.arrive.noinc.shared::cta.b64 [%0];" ::"r"(h_full + 8u * stage) : "memory");
+      } else if (elect_one()) {
         mbar_arrive_expect_tx(h_full + 8u * stage, S::H_BYTES);
         tma_load_2d(sH, &h_map, 0, (int)base, h_full + 8u * stage);
         tma_load_2d(sH + S::H_BYTES / 2, &h_map, 64, (int)base, h_full + 8u * stage);
@@ -410,7 +434,9 @@ __global__ void __launch_bounds__(FusedShape<C>::THREADS, 1)
     if (elect_one()) {
       bool ok = true;
       for (int64_t t = 0; t < ntiles; t++) {
-        ok = mbar_wait(h_full + 8u * stage, phase) && mbar_wait(acc_free + 8u * at_acc, acc_phase ^ 1u);
+        ok = mbar_wait(h_full + 8u * stage, phase);
+        if (g.row_of) fence_proxy_async();   // rows copied by the loader's lanes, read by the tensor core
+        ok = ok && mbar_wait(acc_free + 8u * at_acc, acc_phase ^ 1u);
         if (!ok) break;
         tc_fence_after();
         issue_tile<S::BLOCKS, TILE>(tmem, acc_t + (uint32_t)(at_acc * S::BLOCKS * TILE),
@@ -482,10 +508,10 @@ __global__ void __launch_bounds__(FusedShape<C>::THREADS, 1)
 int encode_half_rows_tensor_map(CUtensorMap *tmap, const void *base, int64_t rows, int box_rows, const char *what);
 
 template <int C>
-static int launch_fused_messages(const FusedMessagesArgs &g, const void *h, const char *what, cudaStream_t st) {
+static int launch_fused_messages(const FusedMessagesArgs &g, const char *what, cudaStream_t st) {
   using S = FusedShape<C>;
   CUtensorMap map;
-  if (int rc = encode_half_rows_tensor_map(&map, h, g.nedges, S::TILE, what)) return rc;
+  if (int rc = encode_half_rows_tensor_map(&map, g.h, g.nedges, S::TILE, what)) return rc;
   cudaError_t e = cudaFuncSetAttribute(fused_messages_kernel<C>, cudaFuncAttributeMaxDynamicSharedMemorySize, S::SMEM);
   if (e != cudaSuccess) return fail(CMACE_ERR_CUDA, "%s: %s", what, cudaGetErrorString(e));
   int64_t blocks = (g.nnodes + S::SETS - 1) / S::SETS;
@@ -495,20 +521,20 @@ static int launch_fused_messages(const FusedMessagesArgs &g, const void *h, cons
 }
 
 int fused_messages(const float *X, const float *Y, const void *h, const void *W, float factor, const int32_t *sender,
-                   const int32_t *receiver, const int32_t *row_ptr, int64_t nnodes, int64_t nedges, int C, float *out,
-                   int32_t *status, cudaStream_t st) {
+                   const int32_t *receiver, const int32_t *row_ptr, const int32_t *row_of, int64_t nnodes, int64_t nedges, int C,
+                   float *out, int32_t *status, cudaStream_t st) {
   const char *what = "cmace_step(messages)";
   if (nnodes == 0) return CMACE_OK;
   if (nedges == 0) {
     cudaError_t e = cudaMemsetAsync(out, 0, (size_t)nnodes * 16 * C * sizeof(float), st);
     return e == cudaSuccess ? CMACE_OK : fail(CMACE_ERR_CUDA, "%s: %s", what, cudaGetErrorString(e));
   }
-  const FusedMessagesArgs g{X, Y, static_cast<const uint4 *>(W), sender, receiver, row_ptr, status, nnodes, nedges, factor, out};
+  const FusedMessagesArgs g{X, Y, static_cast<const char *>(h), static_cast<const uint4 *>(W), sender, receiver, row_ptr, row_of, status, nnodes, nedges, factor, out};
   switch (C) {
-    case 32: return launch_fused_messages<32>(g, h, what, st);
-    case 64: return launch_fused_messages<64>(g, h, what, st);
-    case 96: return launch_fused_messages<96>(g, h, what, st);
-    case 128: return launch_fused_messages<128>(g, h, what, st);
+    case 32: return launch_fused_messages<32>(g, what, st);
+    case 64: return launch_fused_messages<64>(g, what, st);
+    case 96: return launch_fused_messages<96>(g, what, st);
+    case 128: return launch_fused_messages<128>(g, what, st);
   }
   return fail(CMACE_ERR_UNSUPPORTED, "%s: no kernel for %d channels", what, C);
 }

@@ -85,9 +85,9 @@ __device__ __forceinline__ int eb_edge(int row) { return (row & ~15) + 2 * (row 
 
 struct EdgeBackArgs {
   const float *X, *Y, *G;        // [Ns, C], [E, 16], [nnodes, 16, C]
-  const char *h, *dh;            // [E rounded up to a tile][hi 64 | lo 64] fp16
+  const char *h, *dh;            // rows of [hi 64 | lo 64] fp16
   const char *W;                 // [C / 16 steps][hi, lo][64 rows x 128 B, swizzled]
-  const int32_t *sender, *receiver;
+  const int32_t *sender, *receiver, *row_of;   // row_of: an edge's row of h and h'; null: its own
   int32_t *status;
   int64_t nedges;
   float factor_v, factor_t;      // undo the powers of two of h W and h' W
@@ -465,8 +465,21 @@ __global__ void __launch_bounds__(EB_THREADS, 1)
       const uint32_t hdst = sH + (uint32_t)sw64_offset(lane >> 2, lane & 3);
       bool ok = true;
       uint32_t k = 0;
+      int next[4];   // rows of h of this lane's edges in the next tile
+      auto load_rows = [&](int64_t tile) {
+#pragma unroll
+        for (int i = 0; i < 4; i++) {
+          const int64_t e = tile * EB_TILE + eb_edge(r0 + 8 * i), c = e < g.nedges ? e : g.nedges - 1;
+          next[i] = g.row_of ? __ldg(g.row_of + c) : (int)c;
+        }
+      };
+      if (blockIdx.x < ntiles) load_rows(blockIdx.x);
       for (int64_t tile = blockIdx.x; ok && tile < ntiles; tile += gridDim.x, k++) {
         const int64_t base = tile * EB_TILE;
+        int row[4];
+#pragma unroll
+        for (int i = 0; i < 4; i++) row[i] = next[i];
+        if (tile + gridDim.x < ntiles) load_rows(tile + gridDim.x);
         if (k && !warp_wait_all(y_free, (k & 1u) ^ 1u, lane)) {   // the consumers have begun the tile before this one
           if (lane == 0 && g.status) atomicCAS(g.status, 0, 67);
           ok = false;
@@ -484,10 +497,10 @@ __global__ void __launch_bounds__(EB_THREADS, 1)
         // 64 bytes (32 k of hi or lo) of 32 rows: pieces 0-3 of h, 4-7 of h'
         auto start = [&](int piece) {
           if (piece < 8) {
-            const char *src = (piece < 4 ? g.h : g.dh) + base * 256 + 64 * (piece & 3) + 16 * (lane & 3);
+            const char *src = (piece < 4 ? g.h : g.dh) + 64 * (piece & 3) + 16 * (lane & 3);
 #pragma unroll
             for (int i = 0; i < 4; i++)   // sw64_offset(r + 8, c) = sw64_offset(r, c) + 512
-              eb_cp16(hdst + (uint32_t)((piece & 1) * EB_PIECE) + 512u * i, src + 256 * eb_edge(r0 + 8 * i));
+              eb_cp16(hdst + (uint32_t)((piece & 1) * EB_PIECE) + 512u * i, src + (int64_t)row[i] * 256);
           }
           asm volatile("cp.async.commit_group;" ::: "memory");
         };
@@ -554,14 +567,14 @@ static int launch_edge_back(const EdgeBackArgs &g, const char *what, cudaStream_
 }
 
 int fused_messages_back(const float *X, const float *Y, const float *G, const void *h, const void *dh, const void *W,
-                        float factor_v, float factor_t, const int32_t *sender, const int32_t *receiver, int64_t nedges, int C,
-                        float *T, float *gY, int32_t *status, cudaStream_t st) {
+                        float factor_v, float factor_t, const int32_t *sender, const int32_t *receiver, const int32_t *row_of,
+                        int64_t nedges, int C, float *T, float *gY, int32_t *status, cudaStream_t st) {
   const char *what = "cmace_step(edges_back)";
   if (nedges == 0) return CMACE_OK;
   const int64_t ntiles = (nedges + EB_TILE - 1) / EB_TILE;
   if (ntiles * EB_TILE > 0x7fffffffLL) return fail(CMACE_ERR_UNSUPPORTED, "%s: too many edges", what);
   const EdgeBackArgs g{X, Y, G, static_cast<const char *>(h), static_cast<const char *>(dh), static_cast<const char *>(W),
-                       sender, receiver, status, nedges, factor_v, factor_t, T, gY};
+                       sender, receiver, row_of, status, nedges, factor_v, factor_t, T, gY};
   switch (C) {
     case 32: return launch_edge_back<32>(g, what, st);
     case 64: return launch_edge_back<64>(g, what, st);

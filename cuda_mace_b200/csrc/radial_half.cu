@@ -11,6 +11,9 @@
 // tcgen05.mma with its A operand in shared memory is bound by reading 4 KB of it, 48 cycles at N = 64 instead of 32.
 // Tensor memory per group of eight warps, for values and derivatives each: 64 accumulator columns, 32 + 32 of hi and lo.
 //
+// A pair of edges shares a row (EdgeRows): 322 -> 182 us at 16 000 atoms, 1 375 -> 745 at 64 000, 79 -> 52 at 3 000, 30 -> 22 at
+// 400, the look-up of the other edges' rows included.
+//
 // Output rows: HALF: [E][hi 64 | lo 64] fp16 of the value times a power of two, what the products and sums of the step
 // read; otherwise [E, 64] float32.
 #include "common.cuh"
@@ -29,6 +32,7 @@ struct RadialHalfArgs {
   const float *basis;           // [E, 2 nb]
   const void *w[2][3];          // per layer: hi image, lo image (128-byte swizzle), zero rows beyond nb in the first
   RadialScales s[2];
+  EdgeRows rows;
   int32_t *status;
   int64_t E;
   int nb, nper;
@@ -54,6 +58,7 @@ __global__ void __launch_bounds__(RQ_THREADS, 1)
   extern __shared__ __align__(1024) unsigned char smem[];
   __shared__ __align__(8) uint64_t bars[5];   // weights; done[group][operand]
   __shared__ uint32_t tmem_base_slot;
+  __shared__ int32_t edge_s[RQ_THREADS];      // a thread's own: the edge of its next row
 
   const uint32_t smem_base = (smem_u32(smem) + 1023u) & ~1023u;
   const int tid = threadIdx.x, warp = uniform(tid >> 5), lane = tid & 31;
@@ -87,7 +92,8 @@ __global__ void __launch_bounds__(RQ_THREADS, 1)
   bool ok = warp_wait(wbar, 0, lane);
   if (!ok && lane == 0 && g.status) atomicCAS(g.status, 0, 31);
 
-  const int64_t ntiles = (g.E + RQ_TILE - 1) / RQ_TILE;
+  resolve_rows(g.rows, g.E, (int64_t)blockIdx.x * RQ_THREADS + tid, (int64_t)gridDim.x * RQ_THREADS);
+  const int64_t nrows = count_rows(g.rows, g.E), ntiles = (nrows + RQ_TILE - 1) / RQ_TILE;
   const int64_t step = (int64_t)(gridDim.x / (unsigned)g.nper) * 2;
   const int64_t first = (int64_t)(blockIdx.x / (unsigned)g.nper) * 2 + group;
   const int q = gw & 3, h = gw >> 2;      // lane quarter; column half (first operand: 0 values, 1 derivatives)
@@ -97,14 +103,27 @@ __global__ void __launch_bounds__(RQ_THREADS, 1)
   uint32_t phase = 0;
 
   float4 pre[4];
+  // whose basis this thread's row of tile t has, brought by an asynchronous copy (a register more is one too many: it would be
+  // spilled, and the spill would wait for the load)
+  auto load_edge = [&](int64_t t) {
+    const int64_t k = t * RQ_TILE + r;
+    if (g.rows.count && k < nrows)
+      asm volatile("cp.async.ca.shared.global [%0], [%1], 4;" ::"r"(smem_u32(edge_s + tid)), "l"(g.rows.leaders + k) : "memory");
+  };
   auto load_basis = [&](int64_t t) {
-    const int64_t e = t * RQ_TILE + r;
+    const int64_t k = t * RQ_TILE + r;
+    int64_t e = k;
+    if (g.rows.count) {
+      asm volatile("cp.async.wait_all;" ::: "memory");
+      e = k < nrows ? *static_cast<volatile int32_t *>(edge_s + tid) : 0;
+    }
     const float4 *b = reinterpret_cast<const float4 *>(g.basis + e * 2 * g.nb + h * g.nb);
 #pragma unroll
     for (int i = 0; i < 4; i++) {
       pre[i] = make_float4(0.f, 0.f, 0.f, 0.f);
-      if (4 * i < g.nb && t < ntiles && e < g.E) pre[i] = __ldg(b + i);
+      if (4 * i < g.nb && k < nrows) pre[i] = __ldg(b + i);
     }
+    load_edge(t + step);
   };
   auto group_sync = [&]() { asm volatile("bar.sync %0, %1;" ::"r"(group + 1), "r"(RQ_GROUP_THREADS) : "memory"); };
   auto issue = [&](int o, int layer) {
@@ -177,6 +196,7 @@ __global__ void __launch_bounds__(RQ_THREADS, 1)
     }
   };
 
+  load_edge(first);
   load_basis(first);
   for (int64_t tile = first; ok && tile < ntiles; tile += step) {
     {
@@ -269,13 +289,13 @@ __global__ void __launch_bounds__(RQ_THREADS, 1)
 int encode_half_rows_tensor_map(CUtensorMap *tmap, const void *base, int64_t rows, int box_rows, const char *what);
 
 int radial_half(const float *basis, int nb, const void *const (*w)[3], const RadialScales *scales, const int *half_out,
-                int nper, int64_t nedges, void *const *h, void *const *dh, int32_t *status, cudaStream_t st) {
+                int nper, const EdgeRows &rows, int64_t nedges, void *const *h, void *const *dh, int32_t *status, cudaStream_t st) {
   const char *what = "cmace_step(radial)";
   if (nedges == 0) return CMACE_OK;
   if (nb != 8 && nb != 16) return fail(CMACE_ERR_UNSUPPORTED, "%s: the basis size must be 8 or 16", what);
   RadialHalfArgs g{};
   RadialHalfMaps maps;
-  g.basis = basis; g.status = status; g.E = nedges; g.nb = nb; g.nper = nper;
+  g.basis = basis; g.rows = rows; g.status = status; g.E = nedges; g.nb = nb; g.nper = nper;
   for (int i = 0; i < nper; i++) {
     for (int k = 0; k < 3; k++) g.w[i][k] = w[i][k];
     g.s[i] = scales[i];

@@ -32,19 +32,21 @@ namespace cmace {
 int radial_pair_f32(const float *basis, int nb, const float *const (*w)[3], int nper, int64_t nedges, float *const *h,
                     float *const *dh, int32_t *status, cudaStream_t st);
 int radial_half(const float *basis, int nb, const void *const (*w)[3], const RadialScales *scales, const int *half_out,
-                int nper, int64_t nedges, void *const *h, void *const *dh, int32_t *status, cudaStream_t st);
+                int nper, const EdgeRows &rows, int64_t nedges, void *const *h, void *const *dh, int32_t *status,
+                cudaStream_t st);
 int step_sums_half(const void *h, const float *Y, const int32_t *sender, const int32_t *row_ptr, const int32_t *species,
-                   const int32_t *slot_of, int64_t nnodes, int elements, float out_v, float *A, cudaStream_t st);
+                   const int32_t *slot_of, const int32_t *row_of, int64_t nnodes, int elements, float out_v, float *A,
+                   cudaStream_t st);
 int step_sums_bwd_half(const float *gA, const void *h, const void *dh, const float *Y, const int32_t *sender,
-                       const int32_t *row_ptr, const int32_t *species, const int32_t *slot_of, const float *gY1,
-                       const float *dr1, const Quad<float> *geo, int64_t nnodes, int elements, float out_v, float out_t,
-                       float *gvec, cudaStream_t st);
+                       const int32_t *row_ptr, const int32_t *species, const int32_t *slot_of, const int32_t *row_of,
+                       const float *gY1, const float *dr1, const Quad<float> *geo, int64_t nnodes, int elements, float out_v,
+                       float out_t, float *gvec, cudaStream_t st);
 int fused_messages(const float *X, const float *Y, const void *h, const void *W, float factor, const int32_t *sender,
-                   const int32_t *receiver, const int32_t *row_ptr, int64_t nnodes, int64_t nedges, int C, float *out,
-                   int32_t *status, cudaStream_t st);
+                   const int32_t *receiver, const int32_t *row_ptr, const int32_t *row_of, int64_t nnodes, int64_t nedges, int C,
+                   float *out, int32_t *status, cudaStream_t st);
 int fused_messages_back(const float *X, const float *Y, const float *G, const void *h, const void *dh, const void *W,
-                        float factor_v, float factor_t, const int32_t *sender, const int32_t *receiver, int64_t nedges, int C,
-                        float *T, float *gY, int32_t *status, cudaStream_t st);
+                        float factor_v, float factor_t, const int32_t *sender, const int32_t *receiver, const int32_t *row_of,
+                        int64_t nedges, int C, float *T, float *gY, int32_t *status, cudaStream_t st);
 template <typename T>
 int step_edge_finish(const T *gY0, const T *dr0, const T *gY1, const T *dr1, const Quad<T> *geo, int64_t nedges, int shares, T *gvec,
                      cudaStream_t st);
@@ -68,10 +70,14 @@ static bool is_fused(const cmace_step_model &m) {
          m.fused_layout == (m.channels == 128 ? CMACE_FUSED_LAYOUT : CMACE_FUSED_LAYOUT_NARROW);
 }
 
-// Whether the edges of a pair share a row of h and h' (find_pairs), float64: once the radial kernel needs more than one round of
-// its warps without it.  The search takes 8 us there, the second round 30.
-constexpr int64_t kPairEdges64 = 74 * 16 * 8;
-static bool has_pairs(const cmace_step_model &m, int64_t edges) { return m.is_f64 && !is_spline(m) && edges > kPairEdges64; }
+// Whether the edges of a pair share a row of h and h' (find_pairs): once the radial kernel needs more than one round of its warps
+// (float64: eight edges each) or groups (float32: 128 edges) without it.  The search takes 8 us there, the second round 30 and 10:
+// float32, 64 channels, 127 -> 125 us a step at 20 900 edges, 136 -> 132 at 26 200, 150 -> 145 at 36 700, 226 -> 211 at 73 000; at
+// 15 500, in one round, 112 -> 121.
+constexpr int64_t kPairEdges64 = 74 * 16 * 8, kPairEdges32 = 74 * 2 * 128;
+static bool has_pairs(const cmace_step_model &m, int64_t edges) {
+  return m.is_f64 ? !is_spline(m) && edges > kPairEdges64 : is_fused(m) && edges > kPairEdges32;
+}
 
 template <typename T>
 struct Workspace {
@@ -236,12 +242,13 @@ static int run_step(const cmace_step_model &m, cmace_step_io &io, const Workspac
       else if (half) {
         const int half_out[2] = {1, fused ? 1 : 0};
         void *const h[2] = {w.h[0], w.h[1]}, *const dh[2] = {w.dh[0], w.dh[1]};
-        return radial_half(w.basis, m.nbessel, m.radial_half, scales, half_out, 2, E, h, dh, io.status, st);
+        return radial_half(w.basis, m.nbessel, m.radial_half, scales, half_out, 2, w.rows, E, h, dh, io.status, st);
       } else return radial_pair_f32(w.basis, m.nbessel, rw, 2, E, w.h, w.dh, io.status, st);
     }
     case S_SUMS:
       if constexpr (!f64)
-        if (half) return step_sums_half(w.h[0], w.Y, io.sender, io.row_ptr, w.species, w.slot_of, n, Z, scales[0].out_v, w.A, st);
+        if (half) return step_sums_half(w.h[0], w.Y, io.sender, io.row_ptr, w.species, w.slot_of, w.rows.row_of, n, Z, scales[0].out_v, w.A,
+                                        st);
       return K::sums(w.h[0], w.Y, io.sender, io.row_ptr, w.species, w.slot_of, w.rows.row_of, n, Z, w.A, st);
     case S_FOLD: return linear_any(w.A, m.fold, start, Z, n, ST_H * Z, C, w.m0, io.status, st);
     case S_CONTRACT0: return K::contract_fwd(w.m0, w.slot_type, static_cast<const T *>(m.weff[0]), n, C, w.b0, st);
@@ -256,7 +263,7 @@ static int run_step(const cmace_step_model &m, cmace_step_io &io, const Workspac
       if constexpr (!f64)
         if (fused)
           return fused_messages(up, w.Y, w.h[1], m.fused_w, scales[1].out_v * m.fused_scale, io.sender, io.receiver,
-                                io.row_ptr, n, E, C, w.m1, io.status, st);
+                                io.row_ptr, w.rows.row_of, n, E, C, w.m1, io.status, st);
       if constexpr (f64)
         if (w.rows.count) return imp_fwd_rows_f64(up, w.Y, w.R, w.rows.row_of, io.sender, io.row_ptr, n, E, C, w.m1, st);
       return imp_fwd<T>(up, w.Y, w.R, io.sender, io.row_ptr, n, E, ys, C, w.m1, st);
@@ -270,8 +277,8 @@ static int run_step(const cmace_step_model &m, cmace_step_io &io, const Workspac
       if constexpr (!f64)
         if (fused)
           return fused_messages_back(up, w.Y, w.gm1, w.h[1], w.dh[1], m.fused_w_back, scales[1].out_v * m.fused_scale,
-                                     scales[1].out_t * m.fused_scale, io.sender, io.receiver, E, C, w.T_, w.gY1, io.status,
-                                     st);
+                                     scales[1].out_t * m.fused_scale, io.sender, io.receiver, w.rows.row_of, E, C, w.T_, w.gY1,
+                                     io.status, st);
       if constexpr (f64)
         return imp_bwd_edge_pair_f64(up, w.Y, w.R, w.dR, w.rows.row_of, w.gm1, io.sender, io.row_ptr, n, E, C, w.gY1, w.T_, st);
       else
@@ -308,7 +315,7 @@ static int run_step(const cmace_step_model &m, cmace_step_io &io, const Workspac
     case S_SUMS_BACK:
       if constexpr (!f64)
         if (half)
-          return step_sums_bwd_half(w.gA, w.h[0], w.dh[0], w.Y, io.sender, io.row_ptr, w.species, w.slot_of, w.gY1,
+          return step_sums_bwd_half(w.gA, w.h[0], w.dh[0], w.Y, io.sender, io.row_ptr, w.species, w.slot_of, w.rows.row_of, w.gY1,
                                     fused ? nullptr : w.dr1, w.geo, n, Z, scales[0].out_v, scales[0].out_t, w.gvec, st);
       return K::sums_bwd(w.gA, w.h[0], w.dh[0], w.Y, io.sender, io.row_ptr, w.species, w.slot_of, w.rows.row_of, w.gY1, w.shares,
                          w.dr1, w.geo, n, E, Z, w.gvec, st);

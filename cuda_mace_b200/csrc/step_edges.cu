@@ -150,8 +150,9 @@ __device__ void group_nodes(int64_t first, int64_t end, int blocks, int block, b
 // of eight of its edges at a time, lanes beside one another, the first edge that matches is the leader.  Leaders are numbered as
 // they come, a block at a time (rows do not depend on one another, so their places need not be the same in every call):
 // leaders[k] is the edge of row k, row_of[e] the row of a leader, and ~leader for the other edge of a pair until the radial kernel
-// looks its row up (resolve_rows).  The search is a chain of four dependent loads and a ballot an edge: 14 us for 416 000 edges, 8
-// for 9 900; with the vectors compared for four edges one after the other it took 39 and 20.
+// looks its row up (resolve_rows).  The search is a chain of four dependent loads in short lists and instruction issue in long ones:
+// 8 us for 9 900 edges, 14 for 416 000 in float64, 22 for 833 000 and 100 for 3.3 million in float32 (a quarter of the blocks'
+// additions to the counter: the same); with the vectors compared for four edges one after the other 20 and 39 in float64.
 template <typename T>
 __device__ __forceinline__ void find_pairs(int64_t first, const int32_t *__restrict__ sender, const int32_t *__restrict__ receiver,
                                            const int32_t *__restrict__ row_ptr, const Quad<T> *__restrict__ geo, int64_t nedges,
@@ -386,8 +387,40 @@ struct SenderElements {
   }
 };
 
-template <typename Body>
-__device__ __forceinline__ void for_edges_of_element(const SenderElements &from, int z, int32_t *list, Body body) {
+// Rows of h and h' of a receiver's edges (EdgeRows; null: an edge's own), listed beside the edges.  Those of the first 64 wait in
+// shared memory, where asynchronous copies bring them: in registers they cost these kernels a block an SM, from L1, prefetched, the
+// sums of 16 000 atoms take 158 us instead of 137 in float32, of 8 000 156 instead of 127 in float64.
+struct SharedRows {
+  const int32_t *__restrict__ row_of;
+  int32_t *first, *list;
+  __device__ __forceinline__ SharedRows(const int32_t *__restrict__ row_of_, int32_t (&buf)[64 + SU_LIST], const SenderElements &from)
+      : row_of(row_of_), first(buf), list(buf + 64) {
+#pragma unroll
+    for (int i = 0; i < 64; i += 32)
+      if (from.e0 + i + from.lane < from.e1) {
+        if (row_of)
+          asm volatile("cp.async.ca.shared.global [%0], [%1], 4;" ::"r"(smem_u32(first + i + from.lane)),
+                       "l"(row_of + from.e0 + i + from.lane)
+                       : "memory");
+        else
+          first[i + from.lane] = (int32_t)from.e0 + i + from.lane;
+      }
+  }
+  __device__ __forceinline__ void wait() const {
+    asm volatile("cp.async.wait_all;" ::: "memory");
+    __syncwarp();
+  }
+  __device__ __forceinline__ void put(int at, int64_t e, int64_t e0) {
+    list[at] = e - e0 < 64 ? first[e - e0] : (row_of ? __ldg(row_of + e) : (int32_t)e);
+  }
+  __device__ __forceinline__ int64_t operator[](int i) const { return list[i]; }
+};
+struct OwnRows {
+  __device__ __forceinline__ void put(int, int64_t, int64_t) {}
+};
+
+template <typename Rows, typename Body>
+__device__ __forceinline__ void for_edges_of_element(const SenderElements &from, int z, int32_t *list, Rows &rows, Body body) {
   const int lane = from.lane;
   int n = 0;
   for (int64_t eb = from.e0; eb < from.e1; eb += 32) {
@@ -398,7 +431,11 @@ __device__ __forceinline__ void for_edges_of_element(const SenderElements &from,
     else if (e < from.e1) of = __ldg(from.species + __ldg(from.sender + e));
     const bool hit = of == z;
     const unsigned m = __ballot_sync(0xffffffffu, hit);
-    if (hit) list[n + __popc(m & ((1u << lane) - 1u))] = (int32_t)e;
+    if (hit) {
+      const int at = n + __popc(m & ((1u << lane) - 1u));
+      list[at] = (int32_t)e;
+      rows.put(at, e, from.e0);
+    }
     n += __popc(m);
     if (n > SU_LIST - 32) {
       __syncwarp();
@@ -410,34 +447,6 @@ __device__ __forceinline__ void for_edges_of_element(const SenderElements &from,
   __syncwarp();
   if (n > 0) body(n);
 }
-
-// Rows of h and h' of a receiver's edges (EdgeRows; null: an edge's own).  Those of the first 64 wait in shared memory, where
-// asynchronous copies bring them: in registers they cost these kernels a block an SM.
-struct SharedRows {
-  const int32_t *__restrict__ row_of;
-  int32_t *first;
-  int32_t e0;
-  __device__ __forceinline__ SharedRows(const int32_t *__restrict__ row_of_, int32_t *first_, const SenderElements &from)
-      : row_of(row_of_), first(first_), e0((int32_t)from.e0) {
-#pragma unroll
-    for (int i = 0; i < 64; i += 32)
-      if (from.e0 + i + from.lane < from.e1) {
-        if (row_of)
-          asm volatile("cp.async.ca.shared.global [%0], [%1], 4;" ::"r"(smem_u32(first + i + from.lane)),
-                       "l"(row_of + from.e0 + i + from.lane)
-                       : "memory");
-        else
-          first[i + from.lane] = e0 + i + from.lane;
-      }
-  }
-  __device__ __forceinline__ void wait() const {
-    asm volatile("cp.async.wait_all;" ::: "memory");
-    __syncwarp();
-  }
-  __device__ __forceinline__ int64_t operator[](int32_t e) const {
-    return e - e0 < 64 ? first[e - e0] : (row_of ? __ldg(row_of + e) : e);
-  }
-};
 
 // 32 bytes of one lane in one store.  The lanes of a result tile hold 64 bytes of a row each: in 16-byte stores every
 // instruction half-fills 32 sectors, which L2 takes as 2.5 times the writes (10.2 million sectors for 131 MB).
@@ -512,7 +521,8 @@ __global__ void __launch_bounds__(SU_WARPS * 32)
 #pragma unroll
   for (int j = 0; j < 8; j++) acc[j][0] = acc[j][1] = acc[j][2] = acc[j][3] = 0.f;
   from.look_up();
-  for_edges_of_element(from, z, list, [&](int n) {
+  OwnRows rows;
+  for_edges_of_element(from, z, list, rows, [&](int n) {
     float4 hv[2][2];
     float yv[4];
     auto load = [&](int j0) {   // edges j0 + t and j0 + t + 4; past the end: the last edge with Y = 0
@@ -580,22 +590,24 @@ constexpr float SU_Y_SCALE = 256.f;
 __global__ void __launch_bounds__(SU_WARPS * 32)
     sums_f16_kernel(const uint4 *__restrict__ h, const float *__restrict__ Y, const int32_t *__restrict__ sender,
                     const int32_t *__restrict__ row_ptr, const int32_t *__restrict__ species,
-                    const int32_t *__restrict__ slot_of, int64_t nnodes, int elements, float factor,
+                    const int32_t *__restrict__ slot_of, const int32_t *__restrict__ row_of, int64_t nnodes, int elements, float factor,
                     float *__restrict__ A) {
   grid_begin();
-  __shared__ int32_t lists[SU_WARPS][SU_LIST];
+  __shared__ int32_t lists[SU_WARPS][SU_LIST], row_lists[SU_WARPS][64 + SU_LIST];
   const int lane = threadIdx.x & 31, w = threadIdx.x >> 5, g = lane >> 2, t = lane & 3;
   const int64_t pair = (int64_t)blockIdx.x * SU_WARPS + w;
   if (pair >= nnodes * elements) return;
   const int64_t node = pair / elements;
   const int z = (int)(pair - node * elements);
   SenderElements from(sender, species, row_ptr[node], row_ptr[node + 1], lane);
+  SharedRows rows(row_of, row_lists[w], from);
   int32_t *list = lists[w];
   float acc[8][4];
 #pragma unroll
   for (int j = 0; j < 8; j++) acc[j][0] = acc[j][1] = acc[j][2] = acc[j][3] = 0.f;
   from.look_up();
-  for_edges_of_element(from, z, list, [&](int n) {
+  rows.wait();
+  for_edges_of_element(from, z, list, rows, [&](int n) {
     for (int j0 = 0; j0 < n; j0 += 16) {
       uint4 hv[4], lv[4];
       uint32_t ah[4], al[4];
@@ -606,8 +618,9 @@ __global__ void __launch_bounds__(SU_WARPS * 32)
         for (int v = 0; v < 2; v++) {   // past the end: the last edge with Y = 0
           const int j = j0 + 8 * u + 2 * t + v;
           const int64_t e = list[j < n ? j : n - 1];
-          hv[2 * u + v] = __ldg(h + e * 16 + g);
-          lv[2 * u + v] = __ldg(h + e * 16 + 8 + g);
+          const int64_t row = rows[j < n ? j : n - 1];
+          hv[2 * u + v] = __ldg(h + row * 16 + g);
+          lv[2 * u + v] = __ldg(h + row * 16 + 8 + g);
           y[v][0] = j < n ? __ldg(Y + e * 16 + g) * SU_Y_SCALE : 0.f;
           y[v][1] = j < n ? __ldg(Y + e * 16 + g + 8) * SU_Y_SCALE : 0.f;
         }
@@ -641,11 +654,12 @@ __global__ void __launch_bounds__(SU_WARPS * 32)
 }
 
 int step_sums_half(const void *h, const float *Y, const int32_t *sender, const int32_t *row_ptr, const int32_t *species,
-                   const int32_t *slot_of, int64_t nnodes, int elements, float out_v, float *A, cudaStream_t st) {
+                   const int32_t *slot_of, const int32_t *row_of, int64_t nnodes, int elements, float out_v, float *A,
+                   cudaStream_t st) {
   const int64_t blocks = (nnodes * elements + SU_WARPS - 1) / SU_WARPS;
   if (blocks > 0)
     launch_chained(sums_f16_kernel, (unsigned)blocks, SU_WARPS * 32, 0, st, static_cast<const uint4 *>(h), Y, sender, row_ptr, species,
-                                                               slot_of, nnodes, elements, out_v / SU_Y_SCALE, A);
+                                                               slot_of, row_of, nnodes, elements, out_v / SU_Y_SCALE, A);
   return check_launch("cmace_step(sums)");
 }
 
@@ -659,27 +673,27 @@ __global__ void __launch_bounds__(SU_WARPS * 32)
                 const int32_t *__restrict__ slot_of, const int32_t *__restrict__ row_of, int64_t nnodes, int elements,
                 double *__restrict__ A) {
   grid_begin();
-  __shared__ int32_t lists[SU_WARPS][SU_LIST], first_rows[SU_WARPS][64];
+  __shared__ int32_t lists[SU_WARPS][SU_LIST], row_lists[SU_WARPS][64 + SU_LIST];
   const int lane = threadIdx.x & 31, w = threadIdx.x >> 5, g = lane >> 2, t = lane & 3;
   const int64_t pair = (int64_t)blockIdx.x * SU_WARPS + w;
   if (pair >= nnodes * elements) return;
   const int64_t node = pair / elements;
   const int z = (int)(pair - node * elements);
   SenderElements from(sender, species, row_ptr[node], row_ptr[node + 1], lane);
-  const SharedRows rows(row_of, first_rows[w], from);
+  SharedRows rows(row_of, row_lists[w], from);
   int32_t *list = lists[w];
   double acc[2][8][2];
 #pragma unroll
   for (int j = 0; j < 8; j++) acc[0][j][0] = acc[0][j][1] = acc[1][j][0] = acc[1][j][1] = 0.0;
   from.look_up();
   rows.wait();
-  for_edges_of_element(from, z, list, [&](int n) {
+  for_edges_of_element(from, z, list, rows, [&](int n) {
     double2 hv[4];
     double yv[2];
     auto load = [&](int j0) {   // edge j0 + t; past the end: the last edge with Y = 0
       const int j = j0 + t;
       const int64_t e = list[j < n ? j : n - 1];
-      const double2 *hp = reinterpret_cast<const double2 *>(h + rows[e] * ST_H + 8 * g);
+      const double2 *hp = reinterpret_cast<const double2 *>(h + rows[j < n ? j : n - 1] * ST_H + 8 * g);
 #pragma unroll
       for (int u = 0; u < 4; u++) hv[u] = __ldg(hp + u);
       yv[0] = j < n ? __ldg(Y + e * 16 + g) : 0.0;
@@ -798,7 +812,8 @@ __global__ void __launch_bounds__(SU_WARPS * 32, 3)
     }
   }
   from.look_up();
-  for_edges_of_element(from, z, list, [&](int n) {
+  OwnRows rows;
+  for_edges_of_element(from, z, list, rows, [&](int n) {
     for (int j0 = 0; j0 < n; j0 += 32) {
       const int nj = n - j0 < 32 ? n - j0 : 32;
       if (lane < nj) {   // what finish_edge reads
@@ -879,11 +894,11 @@ __global__ void __launch_bounds__(SU_WARPS * 32, 4)
     sums_bwd_f16_kernel(const float *__restrict__ gA, const uint4 *__restrict__ h, const uint4 *__restrict__ dh,
                         const float *__restrict__ Y, const int32_t *__restrict__ sender,
                         const int32_t *__restrict__ row_ptr, const int32_t *__restrict__ species,
-                        const int32_t *__restrict__ slot_of, const float *__restrict__ gY1,
+                        const int32_t *__restrict__ slot_of, const int32_t *__restrict__ row_of, const float *__restrict__ gY1,
                         const float *__restrict__ dr1, const Quad<float> *__restrict__ geo, int64_t nnodes, int elements,
                         float out_v, float out_t, float *__restrict__ gvec) {
   grid_begin();
-  __shared__ int32_t lists[SU_WARPS][SU_LIST];
+  __shared__ int32_t lists[SU_WARPS][SU_LIST], row_lists[SU_WARPS][64 + SU_LIST];
   __shared__ float stage[SU_WARPS][32 * 17];
   const int lane = threadIdx.x & 31, w = threadIdx.x >> 5, g = lane >> 2, t = lane & 3;
   const int64_t pair = (int64_t)blockIdx.x * SU_WARPS + w;
@@ -891,6 +906,7 @@ __global__ void __launch_bounds__(SU_WARPS * 32, 4)
   const int64_t node = pair / elements;
   const int z = (int)(pair - node * elements);
   SenderElements from(sender, species, row_ptr[node], row_ptr[node + 1], lane);
+  SharedRows rows(row_of, row_lists[w], from);
   int32_t *list = lists[w];
   float *st = stage[w];
   uint32_t ph[4][4], pl[4][4];   // A fragments of the 4 K steps
@@ -930,7 +946,8 @@ __global__ void __launch_bounds__(SU_WARPS * 32, 4)
           split_half2(mul2(pack2(v[i][r][u].z, v[i][r][u].w), sc2), ph[2 * i + u][2 + r], pl[2 * i + u][2 + r]);
         }
   }
-  for_edges_of_element(from, z, list, [&](int n) {
+  rows.wait();
+  for_edges_of_element(from, z, list, rows, [&](int n) {
     for (int j0 = 0; j0 < n; j0 += 32) {
       const int nj = n - j0 < 32 ? n - j0 : 32;
       if (lane < nj) {   // what finish_edge reads
@@ -940,7 +957,7 @@ __global__ void __launch_bounds__(SU_WARPS * 32, 4)
       uint4 hh[2], hl[2], dd[2], dl[2];
       auto load = [&](int j) {   // edge j0 + j + g, or the last one
         const int i = j0 + j + g;
-        const int64_t e = list[i < n ? i : n - 1];
+        const int64_t e = rows[i < n ? i : n - 1];
 #pragma unroll
         for (int q = 0; q < 2; q++) {
           hh[q] = __ldg(h + e * 16 + t + 4 * q);
@@ -996,13 +1013,13 @@ __global__ void __launch_bounds__(SU_WARPS * 32, 4)
 }
 
 int step_sums_bwd_half(const float *gA, const void *h, const void *dh, const float *Y, const int32_t *sender,
-                       const int32_t *row_ptr, const int32_t *species, const int32_t *slot_of, const float *gY1,
+                       const int32_t *row_ptr, const int32_t *species, const int32_t *slot_of, const int32_t *row_of, const float *gY1,
                        const float *dr1, const Quad<float> *geo, int64_t nnodes, int elements, float out_v, float out_t,
                        float *gvec, cudaStream_t st) {
   const int64_t blocks = (nnodes * elements + SU_WARPS - 1) / SU_WARPS;
   if (blocks > 0)
     launch_chained(sums_bwd_f16_kernel, (unsigned)blocks, SU_WARPS * 32, 0, st, 
-        gA, static_cast<const uint4 *>(h), static_cast<const uint4 *>(dh), Y, sender, row_ptr, species, slot_of, gY1, dr1,
+        gA, static_cast<const uint4 *>(h), static_cast<const uint4 *>(dh), Y, sender, row_ptr, species, slot_of, row_of, gY1, dr1,
         geo, nnodes, elements, out_v, out_t, gvec);
   return check_launch("cmace_step(sums_back)");
 }
@@ -1019,7 +1036,7 @@ __global__ void __launch_bounds__(SU_WARPS * 32, 3)
                     const Quad<double> *__restrict__ geo, int64_t nnodes, int64_t nedges, int elements,
                     double *__restrict__ gvec) {
   grid_begin();
-  __shared__ int32_t lists[SU_WARPS][SU_LIST], first_rows[SU_WARPS][64];
+  __shared__ int32_t lists[SU_WARPS][SU_LIST], row_lists[SU_WARPS][64 + SU_LIST];
   __shared__ double stage[SU_WARPS][32 * 17];
   const int lane = threadIdx.x & 31, w = threadIdx.x >> 5, g = lane >> 2, t = lane & 3;
   const int64_t pair = (int64_t)blockIdx.x * SU_WARPS + w;
@@ -1027,7 +1044,7 @@ __global__ void __launch_bounds__(SU_WARPS * 32, 3)
   const int64_t node = pair / elements;
   const int z = (int)(pair - node * elements);
   SenderElements from(sender, species, row_ptr[node], row_ptr[node + 1], lane);
-  const SharedRows rows(row_of, first_rows[w], from);
+  SharedRows rows(row_of, row_lists[w], from);
   int32_t *list = lists[w];
   double *st = stage[w];
   double2 P[2][8];
@@ -1041,7 +1058,7 @@ __global__ void __launch_bounds__(SU_WARPS * 32, 3)
   }
   from.look_up();
   rows.wait();
-  for_edges_of_element(from, z, list, [&](int n) {
+  for_edges_of_element(from, z, list, rows, [&](int n) {
     for (int j0 = 0; j0 < n; j0 += 32) {
       const int nj = n - j0 < 32 ? n - j0 : 32;
       if (lane < nj) {   // what finish_edge reads
@@ -1050,7 +1067,7 @@ __global__ void __launch_bounds__(SU_WARPS * 32, 3)
       }
       for (int j = 0; j < nj; j += 8) {
         const int i = j0 + j + g;   // this lane's row of h: that edge, or the last one
-        const int64_t e = rows[list[i < n ? i : n - 1]];
+        const int64_t e = rows[i < n ? i : n - 1];
         const double2 *hp = reinterpret_cast<const double2 *>(h + e * ST_H + 16 * t);
         const double2 *dp = reinterpret_cast<const double2 *>(dh + e * ST_H + 16 * t);
         double2 hv[8], dv[8];

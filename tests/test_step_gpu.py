@@ -163,12 +163,13 @@ def _images(n, side, seed):
 
 
 # An edge and its reverse share the rows of the radial perceptrons where both are in the list: a complete list, one with every
-# third edge missing (a reverse that is not there), one with edges twice and a row shuffled, one with ghost-like one-way edges.
-# Against the operators in float64, which know of no pairs: rounding over the chain, as in the tests above.
+# third edge missing (a reverse that is not there), one with edges twice and rows shuffled, one with one-way edges only.
+# Against the operators in float64, which know of no pairs: rounding over the chain, in float32 as in the tests above.
 @pytest.mark.parametrize("kind", ["complete", "missing", "twice", "one way"])
-@pytest.mark.parametrize("channels", [32, 64, 96])
-def test_edges_that_share_a_length(U, kind, channels):
-    pos, ei, sh = _images(130, 7.0, 3)
+@pytest.mark.parametrize("channels,dtype,tol", [(32, torch.float64, 1e-12), (64, torch.float64, 1e-12), (96, torch.float64, 1e-12),
+                                                (32, torch.float32, 1e-5), (64, torch.float32, 1e-5), (128, torch.float32, 1e-5)])
+def test_edges_that_share_a_length(U, kind, channels, dtype, tol):
+    pos, ei, sh = _images(170, 7.0, 3)
     rng = np.random.default_rng(4)
     keep = np.arange(ei.shape[1])
     if kind == "missing":
@@ -180,18 +181,19 @@ def test_edges_that_share_a_length(U, kind, channels):
         keep = rng.permutation(keep)
     keep = keep[np.argsort(ei[0][keep], kind="stable")]
     ei, sh = torch.from_numpy(ei[:, keep].astype(np.int32)).cuda(), torch.from_numpy(sh[keep]).cuda()
-    assert ei.shape[1] > 74 * 16 * 8
-    mace = model.InvariantMACE(systems.init_params(channels, 3, 7), U, dtype=torch.float64, device="cuda")
+    assert ei.shape[1] > 74 * 2 * 128   # where float32 looks for pairs; float64 does from 74 * 16 * 8
+    params = systems.init_params(channels, 3, 7)
+    mace = model.InvariantMACE(params, U, dtype=dtype, device="cuda")
     p = torch.from_numpy(pos).cuda()
     species = torch.from_numpy(rng.integers(0, 3, pos.shape[0]).astype(np.int32)).cuda()
     out = mace(dict(positions=p, species=species, edge_index=ei, shifts=sh))
     assert step.plan_of(mace) is not None
     p.requires_grad_(True)
-    energies = mace.node_energies(p, species, ei, sh)
+    energies = model.InvariantMACE(params, U, dtype=torch.float64, device="cuda").node_energies(p, species, ei, sh)
     (g,) = torch.autograd.grad(energies.sum(), p)
     energies = energies.detach()
-    assert abs(float(out["interaction_energy"] - energies.sum())) < 1e-12 * float(energies.abs().sum())
-    assert float((out["forces"] + g).abs().max()) < 1e-11 * float(g.abs().max())
+    assert abs(float(out["interaction_energy"] - energies.sum())) < tol * float(energies.abs().sum())
+    assert float((out["forces"] + g).abs().max()) < 10 * tol * float(g.abs().max())
 
 
 # below and above the 32 768 edges from which a new list's grouping by sender runs beside the step
