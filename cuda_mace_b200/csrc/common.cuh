@@ -109,6 +109,11 @@ __device__ __forceinline__ void store_vec_stream(T *p, const T (&src)[VEC]) {
 // writes are visible.  grid_release() lets the successor's blocks come once every block of this grid has called it: a
 // kernel with tensor memory calls it after its allocation, or a successor's block could take the columns that a block of
 // this grid on the same SM still needs, and wait for that block.  Worth about 2 us a kernel in a chain of small ones.
+//
+// A block's grid_release() comes after its own grid_wait().  So when a kernel's first block runs, everything before its predecessor has
+// completed: before grid_wait() it may read what is older than that (constant weights, the caller's list, what kernels before
+// the predecessor wrote) and set up barriers and tensor memory, and a chain of small kernels is mostly such beginnings.  Every
+// block waits on every path: a kernel that ended without having waited would let its successor overtake its predecessor.
 __device__ __forceinline__ void grid_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 __device__ __forceinline__ void grid_release() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 __device__ __forceinline__ void grid_begin() {

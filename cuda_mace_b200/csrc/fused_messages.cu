@@ -314,7 +314,6 @@ __global__ void __launch_bounds__(FusedShape<C>::THREADS, 1)
     }
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
   }
-  grid_wait();
   if (tid <= SETS) {
     const int64_t pieces = (int64_t)gridDim.x * SETS, b = (int64_t)blockIdx.x * SETS + tid;
     const int64_t per = (g.nedges + pieces - 1) / pieces;
@@ -324,12 +323,13 @@ __global__ void __launch_bounds__(FusedShape<C>::THREADS, 1)
   tc_fence_before();
   __syncthreads();
   tc_fence_after();
-  grid_release();   // after the allocation
   const uint32_t tmem = (uint32_t)uniform((int)tmem_base_slot), acc_t = tmem + 64u * S::BLOCKS + (uint32_t)(set * ACCS * S::BLOCKS * TILE);
   if (warp < 4) load_w_tmem<S::BLOCKS>(g.W, tmem, warp, lane);
   tc_fence_before();
   __syncthreads();
   tc_fence_after();
+  grid_wait();      // the list and the weights are older than the kernel before
+  grid_release();   // after the allocation
 
   const int64_t n0 = range_s[set], n1 = range_s[set + 1];
   const int64_t e0 = n0 < n1 ? g.row_ptr[n0] : 0, e1 = n0 < n1 ? g.row_ptr[n1] : 0;

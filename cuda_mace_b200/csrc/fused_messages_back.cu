@@ -239,12 +239,11 @@ __global__ void __launch_bounds__(EB_THREADS, 1)
     mbar_init(y_free, 8);
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
   }
-  grid_wait();
   if (warp == 8) tmem_alloc(smem_u32(&tmem_base_slot), 512);
   tc_fence_before();
   __syncthreads();
   tc_fence_after();
-  grid_release();   // after the allocation
+  // Of all that the block reads only G is the kernel before's: warp 12 waits for it and holds everybody else up with g_full.
   // h buffer b at 128 b: h, h', hi and lo 32 each; acc b at 256 + 128 b
   const uint32_t tmem = (uint32_t)uniform((int)tmem_base_slot);
   const int64_t ntiles = (g.nedges + EB_TILE - 1) / EB_TILE;
@@ -465,6 +464,10 @@ __global__ void __launch_bounds__(EB_THREADS, 1)
       const uint32_t hdst = sH + (uint32_t)sw64_offset(lane >> 2, lane & 3);
       bool ok = true;
       uint32_t k = 0;
+      if (warp == 12 && blockIdx.x >= ntiles) {   // nothing to do, but the block has to wait
+        grid_wait();
+        grid_release();
+      }
       int next[4];   // rows of h of this lane's edges in the next tile
       auto load_rows = [&](int64_t tile) {
 #pragma unroll
@@ -506,6 +509,10 @@ __global__ void __launch_bounds__(EB_THREADS, 1)
         };
         start(0);
         start(1);
+        if (warp == 12 && k == 0) {
+          grid_wait();
+          grid_release();   // after the allocation
+        }
         if (warp == 12 && elect_one()) {
           const int64_t last = base + EB_TILE - 1 < g.nedges ? base + EB_TILE - 1 : g.nedges - 1;
           const int first = __ldg(g.receiver + base);

@@ -140,8 +140,8 @@ __device__ __forceinline__ void build_problem_table(const GemmArgs &g, ProblemTa
   const int nprob = 4 * g.nelements;
   for (int p = threadIdx.x; p < nprob; p += blockDim.x) {
     const int l = p / g.nelements, z = p - l * g.nelements;
-    const int32_t b = g.elem_start ? g.elem_start[z] : 0;
-    const int64_t cnt = g.elem_start ? (int64_t)g.elem_start[z + 1] - b : g.M;
+    const int32_t b = g.elem_start ? __ldcg(g.elem_start + z) : 0;
+    const int64_t cnt = g.elem_start ? (int64_t)__ldcg(g.elem_start + z + 1) - b : g.M;
     const uint32_t rows = (uint32_t)(cnt * (2 * l + 1));   // fits 32 bits (checked on the host)
     tab->seg_begin[p] = b;
     tab->seg_rows[p] = (int32_t)rows;
@@ -293,7 +293,6 @@ __global__ void __launch_bounds__((GT_PRODUCER_WARPS + 1 + EW + 1) * 32, 1)
   __shared__ uint32_t tmem_base_slot;
   __shared__ int32_t tab_words[MODE == GT_MODE_LINEAR ? sizeof(ProblemTable) / 4 : 1];
   const ProblemTable *tab = reinterpret_cast<const ProblemTable *>(tab_words);
-  grid_wait();
   if (MODE == GT_MODE_LINEAR) build_problem_table(g, reinterpret_cast<ProblemTable *>(tab_words));
 
   // dynamic smem base rounded up to 1024 bytes (the swizzle pattern repeats every 1024 bytes)
@@ -335,6 +334,7 @@ __global__ void __launch_bounds__((GT_PRODUCER_WARPS + 1 + EW + 1) * 32, 1)
   __syncthreads();
   tc_fence_after();
   const uint32_t tmem_base = (uint32_t)uniform((int)tmem_base_slot);
+  grid_wait();      // the nodes' grouping is older than the kernel before
   grid_release();   // after the allocation
 
   const int k_blocks = g.k_blocks;

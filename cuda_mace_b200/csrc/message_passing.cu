@@ -543,18 +543,22 @@ __global__ void __launch_bounds__(SPLIT == 1 ? kWarpsPerBlock * 32 : SPLIT * 32)
     imp_bwd_node_kernel(const T *__restrict__ Tin, const int32_t *__restrict__ perm,
                         const int32_t *__restrict__ send_ptr, int64_t nnodes, int C,
                         T *__restrict__ gradX) {
-  grid_begin();
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const int64_t node = SPLIT == 1 ? (int64_t)blockIdx.x * kWarpsPerBlock + warp : blockIdx.x;
-  if (node >= nnodes) return;
+  if (node >= nnodes) {
+    grid_begin();
+    return;
+  }
   const int c0 = blockIdx.y * (32 * VEC) + lane * VEC;
-  const int64_t k1 = send_ptr[node + 1];
+  const int64_t k0 = send_ptr[node] + (SPLIT > 1 ? warp : 0), k1 = send_ptr[node + 1];
+  if (k0 + 32 * lane < k1) asm volatile("prefetch.global.L1 [%0];" ::"l"(perm + k0 + 32 * lane));
+  grid_begin();
   // 32 edges' indices in one load, then four rows in flight at a time
   constexpr int AHEAD = 4;
   T acc[2][VEC];
 #pragma unroll
   for (int v = 0; v < VEC; v++) acc[0][v] = acc[1][v] = T(0);
-  for (int64_t k = send_ptr[node] + (SPLIT > 1 ? warp : 0); k < k1; k += 32 * SPLIT) {
+  for (int64_t k = k0; k < k1; k += 32 * SPLIT) {
     const int64_t mine = k + (int64_t)SPLIT * lane;
     const int32_t e = mine < k1 ? perm[mine] : 0;
     const int n = (int)((k1 - k + SPLIT - 1) / SPLIT < 32 ? (k1 - k + SPLIT - 1) / SPLIT : 32);

@@ -72,12 +72,10 @@ __global__ void __launch_bounds__(RQ_THREADS, 1)
     for (int i = 0; i < 5; i++) mbar_init(wbar + 8u * i, 1);
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
   }
-  grid_wait();
   if (warp == 0) tmem_alloc(smem_u32(&tmem_base_slot), 512);
   tc_fence_before();
   __syncthreads();
   tc_fence_after();
-  grid_release();   // after the allocation
   const uint32_t tmem0 = (uint32_t)uniform((int)tmem_base_slot) + (uint32_t)group * 256u;   // operand o: + 128 o; hi at + 64, lo at + 96
 
   if (warp == 0 && elect_one()) {
@@ -89,6 +87,8 @@ __global__ void __launch_bounds__(RQ_THREADS, 1)
       bulk_copy_g2s(smem_base + (2u * i + 1u) * RQ_IMAGE, src + RQ_IMAGE, RQ_IMAGE, wbar);
     }
   }
+  grid_wait();
+  grid_release();   // after the allocation
   bool ok = warp_wait(wbar, 0, lane);
   if (!ok && lane == 0 && g.status) atomicCAS(g.status, 0, 31);
 

@@ -33,12 +33,11 @@ __global__ void __launch_bounds__(RO_THREADS, 1) radial_out_f64_kernel(const Rad
                  "r"(there ? 16 : 0)
                  : "memory");
   };
-  grid_wait();
-  grid_release();
   for (int i = tid; i < ST_H * RO_N / 2; i += RO_THREADS) {
     const int k = i / (RO_N / 2), c = 2 * (i % (RO_N / 2));
     copy(sB + k * RO_LDB + c, n0 + c < g.N ? g.W + (int64_t)k * g.N + n0 + c : g.W, n0 + c < g.N);
   }
+  grid_begin();
   const int64_t nrows = count_rows(g.rows, g.nedges), tiles = (nrows + TM - 1) / TM;
   const int64_t step = gridDim.x / (unsigned)slices;
   auto fetch = [&](int64_t t, double *dst) {

@@ -296,7 +296,6 @@ struct RadialPairArgs64 {
 };
 
 __global__ void __launch_bounds__(RD_WARPS * 32, 1) radial_pair_f64_kernel(const RadialPairArgs64 g) {
-  grid_begin();
   extern __shared__ __align__(16) double rd_smem[];
   __shared__ double etab[32];   // 2^(j/32)
   const int tid = threadIdx.x, warp = uniform(tid >> 5), lane = tid & 31;
@@ -310,6 +309,7 @@ __global__ void __launch_bounds__(RD_WARPS * 32, 1) radial_pair_f64_kernel(const
     sW3[(i >> 6) * RD_LD + (i & 63)] = (per ? g.w[1][2] : g.w[0][2])[i];
   }
   __syncthreads();
+  grid_begin();
   const int fr = lane >> 2, fk = lane & 3;
   double *const h_out = per ? g.h[1] : g.h[0], *const dh_out = per ? g.dh[1] : g.dh[0];
   resolve_rows(g.rows, g.E, (int64_t)blockIdx.x * (RD_WARPS * 32) + tid, (int64_t)gridDim.x * (RD_WARPS * 32));

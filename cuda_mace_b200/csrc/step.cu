@@ -251,7 +251,7 @@ static int run_step(const cmace_step_model &m, cmace_step_io &io, const Workspac
                                         st);
       return K::sums(w.h[0], w.Y, io.sender, io.row_ptr, w.species, w.slot_of, w.rows.row_of, n, Z, w.A, st);
     case S_FOLD: return linear_any(w.A, m.fold, start, Z, n, ST_H * Z, C, w.m0, io.status, st);
-    case S_CONTRACT0: return K::contract_fwd(w.m0, w.slot_type, static_cast<const T *>(m.weff[0]), n, C, w.b0, st);
+    case S_CONTRACT0: return K::contract_fwd(w.m0, w.slot_type, static_cast<const T *>(m.weff[0]), n, C, true, w.b0, st);
     case S_MID_FWD:
       return K::mid_fwd(w.b0, w.node_of, w.slot_type, static_cast<const T *>(m.up), static_cast<const T *>(m.extra), n, C,
                         io.up_local ? static_cast<T *>(io.up_local) : w.up, w.q0, st);
@@ -294,7 +294,7 @@ static int run_step(const cmace_step_model &m, cmace_step_io &io, const Workspac
       return K::mid_bwd(gup_owned, w.node_of, w.slot_type, w.dq, static_cast<const T *>(m.up_back),
                         static_cast<const T *>(m.extra_back), m.scale, n, C, w.gb0, st);
     case S_CONTRACT0_BACK:
-      return K::contract_bwd(w.m0, w.slot_type, static_cast<const T *>(m.weff[0]), w.gb0, n, C, w.gX0, st);
+      return K::contract_bwd(w.m0, w.slot_type, static_cast<const T *>(m.weff[0]), w.gb0, n, C, true, w.gX0, st);
     case S_FOLD_BACK:
       // float32: the blocks of two elements in one launch, which reads the rows from memory once
       if constexpr (!f64) {

@@ -107,8 +107,8 @@ struct StepKernels {
                        int32_t *slot_type, int32_t *elem_start, const int32_t *row_ptr, const EdgeRows &rows, cudaStream_t st);
   static int sums(const T *h, const T *Y, const int32_t *sender, const int32_t *row_ptr, const int32_t *species,
                   const int32_t *slot_of, const int32_t *row_of, int64_t nnodes, int elements, T *A, cudaStream_t st);
-  static int contract_fwd(const T *X, const int32_t *types, const T *weff, int64_t n, int C, T *b, cudaStream_t st);
-  static int contract_bwd(const T *X, const int32_t *types, const T *weff, const T *gb, int64_t n, int C, T *gX,
+  static int contract_fwd(const T *X, const int32_t *types, const T *weff, int64_t n, int C, bool early, T *b, cudaStream_t st);
+  static int contract_bwd(const T *X, const int32_t *types, const T *weff, const T *gb, int64_t n, int C, bool early, T *gX,
                           cudaStream_t st);
   static int contract_readout(const T *X, const int32_t *types, const T *weff, const T *wp1, const double *w2,
                               const T *q0, const double *atomic_e, double scale, double shift, int64_t n, int C, T *gX,
