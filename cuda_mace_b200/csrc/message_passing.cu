@@ -215,7 +215,7 @@ __global__ void __launch_bounds__(kWarpsPerBlock * 32)
 // own gY [E, 16].  Bound by bytes, as the pass that wrote the gradient: 848 -> 678 us at 8 000 atoms and 128 channels (805 with
 // 220 registers, two blocks an SM), 406 -> 363 at 64.
 template <int VEC>
-__global__ void __launch_bounds__(kWarpsPerBlock * 32, VEC == 1 ? 4 : 3)
+__global__ void __launch_bounds__(kWarpsPerBlock * 32, 3)
     imp_bwd_edge_pair_kernel(const double *__restrict__ X, const double *__restrict__ Y, const double *__restrict__ R,
                              const double *__restrict__ dR, const int32_t *__restrict__ row_of, const double *__restrict__ G,
                              const int32_t *__restrict__ sender, const int32_t *__restrict__ row_ptr, int64_t nnodes,
@@ -294,6 +294,309 @@ __global__ void __launch_bounds__(kWarpsPerBlock * 32, VEC == 1 ? 4 : 3)
       store_vec<double, VEC>(Tout + ee * C + c0, t);
       const double tot = warp_reduce16(p, lane);
       if ((lane & 1) == 0) gy[(lane >> 1) + ee * 16] = tot;
+    }
+  }
+}
+
+// ---- narrow rows: several edges a warp -----------------------------------------------------------------------------
+// With 32 or 64 channels a row does not fill a warp with 16-byte pieces, and what an edge costs beside its channels (harmonics
+// handed out, sums over channels, addresses) is what binds: 32 channels took 0.8 of 64 channels' time.  Here LANES lanes own an
+// edge, EPW = 32 / LANES edges are worked on side by side and AT of those one after the other, all of one receiver.  96 channels:
+// three a lane, 32 apart, in one pass instead of three chunks with a share of grad Y each.  us at 8 192 nodes of 30 edges, forward and
+// edge pass, before -> now: float32 50 -> 37 and 116 -> 72 with 32 channels, 71 -> 70 and 145 -> 125 with 64, 129 -> 83 and 352 -> 203
+// with 96; float64 86 -> 64 and 170 -> 139 with 32, 233 -> 167 and 538 -> 388 with 96 (64 channels fill a warp with 16-byte pieces).
+// In a float64 step of 8 000 atoms 138 -> 108 and 273 -> 216 with 32 channels, 366 -> 276 and 731 -> 631 with 96.
+template <typename T, int VEC>
+__device__ __forceinline__ void load_lane(T (&d)[VEC], const T *row, int sub, bool stream) {
+  if constexpr (VEC == 3) {
+#pragma unroll
+    for (int v = 0; v < 3; v++) d[v] = stream ? __ldcs(row + sub + 32 * v) : __ldg(row + sub + 32 * v);
+  } else {
+    if (stream) load_vec_stream<T, VEC>(d, row + sub * VEC);
+    else load_vec<T, VEC>(d, row + sub * VEC);
+  }
+}
+template <typename T, int VEC>
+__device__ __forceinline__ void store_lane(T *row, int sub, const T (&d)[VEC], bool stream) {
+  if constexpr (VEC == 3) {
+#pragma unroll
+    for (int v = 0; v < 3; v++) {
+      if (stream) __stcs(row + sub + 32 * v, d[v]);
+      else row[sub + 32 * v] = d[v];
+    }
+  } else {
+    if (stream) store_vec_stream<T, VEC>(row + sub * VEC, d);
+    else store_vec<T, VEC>(row + sub * VEC, d);
+  }
+}
+
+template <typename T, int EDGES>
+struct SlotHarmonics {
+  static constexpr int LD = 16 + 16 / (int)sizeof(T);   // an edge's 16 values; a piece more keeps eight edges in different banks
+  static constexpr int PER = (EDGES * 16 + 31) / 32;    // values a lane
+  // component and edge of a lane's value i, consecutive in memory for neighbouring lanes
+  static __device__ __forceinline__ bool at(int i, int lane, const ImpLayout &ys, int &edge, int &m) {
+    const int k = 32 * i + lane;
+    edge = ys.m == 1 ? k >> 4 : k % EDGES;
+    m = ys.m == 1 ? k & 15 : k / EDGES;
+    return k < EDGES * 16;
+  }
+};
+
+// Blocks an SM, as measured: float32 37 us with three at 32 channels (44 with four), 70 with four at 64 (81 with three); float64 of 32
+// channels 64 with three (76 with four), but 108 with four (166 with three) where rows are looked up.
+template <typename T, int VEC, int LANES, bool ROWS>
+constexpr int fwd_slots_blocks() {
+  if (VEC == 3) return sizeof(T) == 4 ? 5 : 2;
+  return (sizeof(T) == 4 ? LANES == 16 : ROWS) ? 4 : 3;
+}
+template <typename T, int VEC, int LANES, int SPLIT, bool ROWS>
+__global__ void __launch_bounds__(SPLIT == 1 ? kWarpsPerBlock * 32 : SPLIT * 32, SPLIT > 1 ? 1 : fwd_slots_blocks<T, VEC, LANES, ROWS>())
+    imp_fwd_slots_kernel(const T *__restrict__ X, const T *__restrict__ Y, const T *__restrict__ R, const int32_t *__restrict__ row_of,
+                         const int32_t *__restrict__ sender, const int32_t *__restrict__ row_ptr, int64_t nnodes, ImpLayout ys,
+                         T *__restrict__ out) {
+  grid_begin();
+  constexpr int EPW = 32 / LANES, AT = 2, EDGES = AT * EPW, C = VEC * LANES, KEPT = 16 / EPW;
+  using H = SlotHarmonics<T, EDGES>;
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, sub = lane % LANES, slot = lane / LANES;
+  const int64_t node = SPLIT == 1 ? (int64_t)blockIdx.x * kWarpsPerBlock + warp : blockIdx.x;
+  if (node >= nnodes) return;
+  const int64_t e0 = row_ptr[node], e1 = row_ptr[node + 1], begin = e0 + (SPLIT > 1 ? EDGES * warp : 0);
+  T acc[16][VEC];
+#pragma unroll
+  for (int m = 0; m < 16; m++)
+#pragma unroll
+    for (int v = 0; v < VEC; v++) acc[m][v] = T(0);
+  __shared__ __align__(16) T harmonics[SPLIT == 1 ? kWarpsPerBlock : SPLIT][2][EDGES * H::LD];
+  int turn = 0;
+  int32_t next[AT][2];   // senders and rows of this slot's next edges
+  auto look_up = [&](int64_t e) {
+#pragma unroll
+    for (int a = 0; a < AT; a++) {
+      const int64_t i = e + a * EPW + slot < e1 ? e + a * EPW + slot : e1 - 1;
+      next[a][0] = __ldg(sender + i);
+      next[a][1] = ROWS ? __ldg(row_of + i) : (int32_t)i;
+    }
+  };
+  if (begin < e1) look_up(begin);
+  for (int64_t e = begin; e < e1; e += EDGES * SPLIT, turn ^= 1) {
+    T yv[H::PER];
+#pragma unroll
+    for (int i = 0; i < H::PER; i++) {
+      int edge, m;
+      yv[i] = T(0);
+      if (H::at(i, lane, ys, edge, m) && e + edge < e1) yv[i] = __ldg(Y + m * ys.m + (e + edge) * ys.e);
+    }
+    T x[AT][VEC], r[AT][4][VEC];
+#pragma unroll
+    for (int a = 0; a < AT; a++) {
+      const bool there = e + a * EPW + slot < e1;   // beyond the receiver's edges: nothing is read or added
+#pragma unroll
+      for (int v = 0; v < VEC; v++) x[a][v] = r[a][0][v] = r[a][1][v] = r[a][2][v] = r[a][3][v] = T(0);
+      if (there) {
+        load_lane<T, VEC>(x[a], X + (int64_t)next[a][0] * C, sub, false);
+#pragma unroll
+        for (int l = 0; l < 4; l++) load_lane<T, VEC>(r[a][l], R + ((int64_t)next[a][1] * 4 + l) * C, sub, !ROWS);
+      }
+    }
+    look_up(e + EDGES * SPLIT);
+#pragma unroll
+    for (int a = 0; a < AT; a++)
+#pragma unroll
+      for (int l = 0; l < 4; l++)
+#pragma unroll
+        for (int v = 0; v < VEC; v++) r[a][l][v] *= x[a][v];
+    T *yp = harmonics[warp][turn];
+#pragma unroll
+    for (int i = 0; i < H::PER; i++) {
+      int edge, m;
+      if (H::at(i, lane, ys, edge, m)) yp[edge * H::LD + m] = yv[i];
+    }
+    __syncwarp();
+#pragma unroll
+    for (int a = 0; a < AT; a++) {
+      T y[16];
+      take16<T>(y, yp + (a * EPW + slot) * H::LD);
+#pragma unroll
+      for (int m = 0; m < 16; m++)
+#pragma unroll
+        for (int v = 0; v < VEC; v++) acc[m][v] = fma(y[m], r[a][l_of_lm(m)][v], acc[m][v]);
+    }
+  }
+  // the slots' sums: every slot ends up with KEPT components of all of them
+  if constexpr (EPW >= 2) {
+    const bool up = lane & 16;
+#pragma unroll
+    for (int m = 0; m < 8; m++)
+#pragma unroll
+      for (int v = 0; v < VEC; v++) {
+        const T send = up ? acc[m][v] : acc[m + 8][v], keep = up ? acc[m + 8][v] : acc[m][v];
+        acc[m][v] = keep + __shfl_xor_sync(0xffffffffu, send, 16);
+      }
+  }
+  if constexpr (EPW == 4) {
+    const bool up = lane & 8;
+#pragma unroll
+    for (int m = 0; m < 4; m++)
+#pragma unroll
+      for (int v = 0; v < VEC; v++) {
+        const T send = up ? acc[m][v] : acc[m + 4][v], keep = up ? acc[m + 4][v] : acc[m][v];
+        acc[m][v] = keep + __shfl_xor_sync(0xffffffffu, send, 8);
+      }
+  }
+  T *o = out + node * 16 * C;
+  if constexpr (SPLIT > 1) {
+    extern __shared__ __align__(16) unsigned char imp_smem[];
+    T *part = reinterpret_cast<T *>(imp_smem);   // [SPLIT][16][C]
+#pragma unroll
+    for (int m = 0; m < KEPT; m++) store_lane<T, VEC>(part + (warp * 16 + slot * KEPT + m) * C, sub, acc[m], false);
+    __syncthreads();
+    for (int i = threadIdx.x; i < 16 * C; i += SPLIT * 32) {
+      T sum = T(0);
+#pragma unroll
+      for (int w = 0; w < SPLIT; w++) sum += part[w * 16 * C + i];
+      o[i] = sum;
+    }
+  } else {
+#pragma unroll
+    for (int m = 0; m < KEPT; m++) store_lane<T, VEC>(o + (slot * KEPT + m) * C, sub, acc[m], false);
+  }
+}
+
+// Sums of p[m] over a slot's lanes: lane `sub` gets the components of `own` values from sub * own on (one of two lanes of 32 its
+// own: the other holds the same).
+template <typename T, int LANES>
+__device__ __forceinline__ void slot_reduce16(T (&p)[16], int lane) {
+  if constexpr (LANES == 32) {
+    p[0] = warp_reduce16(p, lane);
+  } else {
+    constexpr int STEPS = LANES == 16 ? 4 : 3;
+    int n = 16, off = LANES / 2;
+#pragma unroll
+    for (int k = 0; k < STEPS; k++, off >>= 1) {
+      n >>= 1;
+      const bool up = lane & off;
+#pragma unroll
+      for (int i = 0; i < 8; i++)
+        if (i < n) {
+          const T send = up ? p[i] : p[i + n], keep = up ? p[i + n] : p[i];
+          p[i] = keep + __shfl_xor_sync(0xffffffffu, send, off);
+        }
+    }
+  }
+}
+
+// PAIR: as imp_bwd_edge_pair_kernel (rows of R and R' by row_of, dE/dr in the place of grad Y_00); otherwise as imp_bwd_edge_kernel
+template <typename T, int VEC, int LANES, bool PAIR>
+__global__ void __launch_bounds__(kWarpsPerBlock * 32, VEC != 3 ? 3 : (sizeof(T) == 4 ? 4 : 2))
+    imp_bwd_edge_slots_kernel(const T *__restrict__ X, const T *__restrict__ Y, const T *__restrict__ R, const T *__restrict__ dR,
+                              const int32_t *__restrict__ row_of, const T *__restrict__ G, const int32_t *__restrict__ sender,
+                              const int32_t *__restrict__ row_ptr, int64_t nnodes, ImpLayout ys, int slices, T *__restrict__ gradR,
+                              T *__restrict__ gradY, T *__restrict__ Tout) {
+  grid_begin();
+  constexpr int EPW = 32 / LANES, AT = PAIR && VEC == 3 ? 1 : 2, EDGES = AT * EPW, C = VEC * LANES;
+  using H = SlotHarmonics<T, EDGES>;
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, sub = lane % LANES, slot = lane / LANES;
+  const int64_t item = (int64_t)blockIdx.x * kWarpsPerBlock + warp;
+  const int64_t node = slices == 1 ? item : item / slices;
+  const int slice = slices == 1 ? 0 : (int)(item - node * slices);
+  if (node >= nnodes) return;
+  const int64_t e1 = row_ptr[node + 1], begin = row_ptr[node] + EDGES * slice;
+  if (begin >= e1) return;
+  T g[16][VEC];
+#pragma unroll
+  for (int m = 0; m < 16; m++) load_lane<T, VEC>(g[m], G + (node * 16 + m) * C, sub, false);
+  __shared__ __align__(16) T harmonics[kWarpsPerBlock][2][EDGES * H::LD], sums[kWarpsPerBlock][EDGES * H::LD];
+  int turn = 0;
+  int32_t next[AT][2];
+  auto look_up = [&](int64_t e) {
+#pragma unroll
+    for (int a = 0; a < AT; a++) {
+      const int64_t i = e + a * EPW + slot < e1 ? e + a * EPW + slot : e1 - 1;
+      next[a][0] = __ldg(sender + i);
+      next[a][1] = PAIR && row_of ? __ldg(row_of + i) : (int32_t)i;
+    }
+  };
+  look_up(begin);
+  for (int64_t e = begin; e < e1; e += EDGES * slices, turn ^= 1) {
+    T yv[H::PER];
+#pragma unroll
+    for (int i = 0; i < H::PER; i++) {
+      int edge, m;
+      yv[i] = T(0);
+      if (H::at(i, lane, ys, edge, m) && e + edge < e1) yv[i] = __ldg(Y + m * ys.m + (e + edge) * ys.e);
+    }
+    T x[AT][VEC], r[AT][4][VEC], d[PAIR ? AT : 1][4][VEC];
+#pragma unroll
+    for (int a = 0; a < AT; a++) {   // an edge beyond the receiver's last is that one; it is not stored
+      load_lane<T, VEC>(x[a], X + (int64_t)next[a][0] * C, sub, false);
+#pragma unroll
+      for (int l = 0; l < 4; l++) {
+        load_lane<T, VEC>(r[a][l], R + ((int64_t)next[a][1] * 4 + l) * C, sub, !PAIR);
+        if constexpr (PAIR) load_lane<T, VEC>(d[a][l], dR + ((int64_t)next[a][1] * 4 + l) * C, sub, false);
+      }
+    }
+    look_up(e + EDGES * slices);
+    T *yp = harmonics[warp][turn];
+#pragma unroll
+    for (int i = 0; i < H::PER; i++) {
+      int edge, m;
+      if (H::at(i, lane, ys, edge, m)) yp[edge * H::LD + m] = yv[i];
+    }
+    __syncwarp();   // and everybody has read the sums of the edges before
+#pragma unroll
+    for (int a = 0; a < AT; a++) {
+      const int64_t ee = e + a * EPW + slot;
+      const bool there = ee < e1;
+      T y[16], p[16], t[VEC], w[VEC];
+      take16<T>(y, yp + (a * EPW + slot) * H::LD);
+#pragma unroll
+      for (int l = 0; l < 4; l++) {
+        T u[VEC], rx[VEC];
+#pragma unroll
+        for (int v = 0; v < VEC; v++) rx[v] = r[a][l][v] * x[a][v];
+#pragma unroll
+        for (int m = l * l; m < (l + 1) * (l + 1); m++) {
+          T pm = T(0);
+#pragma unroll
+          for (int v = 0; v < VEC; v++) {
+            u[v] = m == l * l ? y[m] * g[m][v] : fma(y[m], g[m][v], u[v]);
+            pm = fma(g[m][v], rx[v], pm);
+          }
+          p[m] = pm;
+        }
+        T gr[VEC];
+#pragma unroll
+        for (int v = 0; v < VEC; v++) {
+          t[v] = l == 0 ? u[v] * r[a][l][v] : fma(u[v], r[a][l][v], t[v]);
+          if constexpr (PAIR) w[v] = l == 0 ? u[v] * d[a][l][v] : fma(u[v], d[a][l][v], w[v]);
+          else gr[v] = x[a][v] * u[v];
+        }
+        if constexpr (!PAIR)
+          if (gradR != nullptr && there) store_lane<T, VEC>(gradR + (ee * 4 + l) * C, sub, gr, true);
+      }
+      if constexpr (PAIR) {
+        p[0] = T(0);
+#pragma unroll
+        for (int v = 0; v < VEC; v++) p[0] = fma(x[a][v], w[v], p[0]);
+      }
+      if (Tout != nullptr && there) store_lane<T, VEC>(Tout + ee * C, sub, t, false);
+      slot_reduce16<T, LANES>(p, lane);
+      T *q = sums[warp] + (a * EPW + slot) * H::LD;
+      if constexpr (LANES == 32) {
+        if ((lane & 1) == 0) q[lane >> 1] = p[0];
+      } else if constexpr (LANES == 16) {
+        q[sub] = p[0];
+      } else {
+        q[2 * sub] = p[0];
+        q[2 * sub + 1] = p[1];
+      }
+    }
+    __syncwarp();
+#pragma unroll
+    for (int i = 0; i < H::PER; i++) {
+      int edge, m;
+      if (H::at(i, lane, ys, edge, m) && e + edge < e1) gradY[m * ys.m + (e + edge) * ys.e] = sums[warp][edge * H::LD + m];
     }
   }
 }
@@ -549,7 +852,7 @@ __global__ void __launch_bounds__(SPLIT == 1 ? kWarpsPerBlock * 32 : SPLIT * 32)
     grid_begin();
     return;
   }
-  const int c0 = blockIdx.y * (32 * VEC) + lane * VEC;
+  const int chunk = blockIdx.y * (32 * VEC);
   const int64_t k0 = send_ptr[node] + (SPLIT > 1 ? warp : 0), k1 = send_ptr[node + 1];
   if (k0 + 32 * lane < k1) asm volatile("prefetch.global.L1 [%0];" ::"l"(perm + k0 + 32 * lane));
   grid_begin();
@@ -567,7 +870,7 @@ __global__ void __launch_bounds__(SPLIT == 1 ? kWarpsPerBlock * 32 : SPLIT * 32)
 #pragma unroll
       for (int u = 0; u < AHEAD; u++) {
         const int64_t row = __shfl_sync(0xffffffffu, e, (j + u) & 31);
-        if (j + u < n) load_vec<T, VEC>(a[u], Tin + row * C + c0);
+        if (j + u < n) load_lane<T, VEC>(a[u], Tin + row * C + chunk, lane, false);
       }
 #pragma unroll
       for (int u = 0; u < AHEAD; u++)
@@ -582,15 +885,15 @@ __global__ void __launch_bounds__(SPLIT == 1 ? kWarpsPerBlock * 32 : SPLIT * 32)
   if constexpr (SPLIT > 1) {
     __shared__ T part[SPLIT][32 * VEC];
 #pragma unroll
-    for (int v = 0; v < VEC; v++) part[warp][lane * VEC + v] = acc[0][v];
+    for (int v = 0; v < VEC; v++) part[warp][v * 32 + lane] = acc[0][v];
     __syncthreads();
     if (warp > 0) return;
 #pragma unroll
     for (int w = 1; w < SPLIT; w++)
 #pragma unroll
-      for (int v = 0; v < VEC; v++) acc[0][v] += part[w][lane * VEC + v];
+      for (int v = 0; v < VEC; v++) acc[0][v] += part[w][v * 32 + lane];
   }
-  store_vec<T, VEC>(gradX + node * C + c0, acc[0]);
+  store_lane<T, VEC>(gradX + node * C + chunk, lane, acc[0], false);
 }
 
 // ------------------------------------------------------------------------------------------
@@ -631,6 +934,46 @@ static void launch_fwd(const T *X, const T *Y, const T *R, const int32_t *row_of
                  out);
 }
 
+// whether rows of C channels go several edges (or 96 channels) to a warp
+template <typename T>
+static bool takes_slots(int C) {
+  return C == 32 || C == 96 || (sizeof(T) == 4 && C == 64);
+}
+template <typename T, int VEC, int LANES, bool ROWS>
+static void launch_fwd_slots(const T *X, const T *Y, const T *R, const int32_t *row_of, const int32_t *sender, const int32_t *row_ptr,
+                             int64_t nnodes, ImpLayout ys, T *out, cudaStream_t st) {
+  if (few_nodes(nnodes)) {
+    constexpr int smem = kSplit * 16 * VEC * LANES * (int)sizeof(T);
+    auto kernel = imp_fwd_slots_kernel<T, VEC, LANES, kSplit, ROWS>;
+    cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+    launch_chained(kernel, (unsigned)nnodes, kSplit * 32, smem, st, X, Y, R, row_of, sender, row_ptr, nnodes, ys, out);
+    return;
+  }
+  launch_chained(imp_fwd_slots_kernel<T, VEC, LANES, 1, ROWS>, (unsigned)((nnodes + kWarpsPerBlock - 1) / kWarpsPerBlock),
+                 kWarpsPerBlock * 32, 0, st, X, Y, R, row_of, sender, row_ptr, nnodes, ys, out);
+}
+template <typename T, bool ROWS>
+static void fwd_slots(const T *X, const T *Y, const T *R, const int32_t *row_of, const int32_t *sender, const int32_t *row_ptr,
+                      int64_t nnodes, ImpLayout ys, int C, T *out, cudaStream_t st) {
+  if (C == 96) launch_fwd_slots<T, 3, 32, ROWS>(X, Y, R, row_of, sender, row_ptr, nnodes, ys, out, st);
+  else if constexpr (sizeof(T) == 8) launch_fwd_slots<T, 2, 16, ROWS>(X, Y, R, row_of, sender, row_ptr, nnodes, ys, out, st);
+  else if (C == 64) launch_fwd_slots<T, 4, 16, ROWS>(X, Y, R, row_of, sender, row_ptr, nnodes, ys, out, st);
+  else launch_fwd_slots<T, 4, 8, ROWS>(X, Y, R, row_of, sender, row_ptr, nnodes, ys, out, st);
+}
+template <typename T, bool PAIR>
+static void bwd_edge_slots(const T *X, const T *Y, const T *R, const T *dR, const int32_t *row_of, const T *G, const int32_t *sender,
+                           const int32_t *row_ptr, int64_t nnodes, ImpLayout ys, int C, T *gradR, T *gY, T *Tout, cudaStream_t st) {
+  const int slices = few_nodes(nnodes) ? kSplit : 1;
+  auto launch = [&](auto kernel) {
+    launch_chained(kernel, (unsigned)((nnodes * slices + kWarpsPerBlock - 1) / kWarpsPerBlock), kWarpsPerBlock * 32, 0, st, X, Y, R, dR,
+                   row_of, G, sender, row_ptr, nnodes, ys, slices, gradR, gY, Tout);
+  };
+  if (C == 96) launch(imp_bwd_edge_slots_kernel<T, 3, 32, PAIR>);
+  else if constexpr (sizeof(T) == 8) launch(imp_bwd_edge_slots_kernel<T, 2, 16, PAIR>);
+  else if (C == 64) launch(imp_bwd_edge_slots_kernel<T, 4, 16, PAIR>);
+  else launch(imp_bwd_edge_slots_kernel<T, 4, 8, PAIR>);
+}
+
 template <typename T>
 int imp_fwd(const T *X, const T *Y, const T *R, const int32_t *sender, const int32_t *row_ptr,
             int64_t nnodes, int64_t nedges, ImpLayout ys, int C, T *out, cmace_stream_t stream) {
@@ -640,6 +983,10 @@ int imp_fwd(const T *X, const T *Y, const T *R, const int32_t *sender, const int
   if (!out || !row_ptr || (nedges > 0 && (!X || !R || !Y || !sender)))
     return fail(CMACE_ERR_ARG, "cmace_imp_fwd: null pointer");
   cudaStream_t st = (cudaStream_t)stream;
+  if (takes_slots<T>(C)) {
+    fwd_slots<T, false>(X, Y, R, nullptr, sender, row_ptr, nnodes, ys, C, out, st);
+    return check_launch("cmace_imp_fwd");
+  }
   switch (pick_vec<T>(C)) {
     case 4:
       if constexpr (sizeof(T) == 4) launch_fwd<T, 4>(X, Y, R, nullptr, sender, row_ptr, nnodes, ys, C, out, st);
@@ -664,21 +1011,24 @@ int imp_bwd_edge_pair_f64(const double *X, const double *Y, const double *R, con
                           const double *G, const int32_t *sender, const int32_t *row_ptr, int64_t nnodes, int64_t nedges, int C,
                           double *gY, double *T, cudaStream_t st) {
   if (nnodes == 0 || nedges == 0) return CMACE_OK;
+  if (takes_slots<double>(C)) {
+    bwd_edge_slots<double, true>(X, Y, R, dR, row_of, G, sender, row_ptr, nnodes, ImpLayout{1, 16}, C, nullptr, gY, T, st);
+    return check_launch("cmace_step(edges_back)");
+  }
   auto launch = [&](auto kernel, int chunks) {
     const int slices = few_nodes(nnodes * chunks) ? kSplit : 1;
     const dim3 grid((unsigned)((nnodes * slices + kWarpsPerBlock - 1) / kWarpsPerBlock), (unsigned)chunks);
     launch_chained(kernel, grid, kWarpsPerBlock * 32, 0, st, X, Y, R, dR, row_of, G, sender, row_ptr, nnodes, nedges, C, slices, gY, T);
   };
-  if (C % 64 == 0) launch(imp_bwd_edge_pair_kernel<2>, C / 64);
-  else launch(imp_bwd_edge_pair_kernel<1>, C / 32);
+  launch(imp_bwd_edge_pair_kernel<2>, C / 64);
   return check_launch("cmace_step(edges_back)");
 }
 int imp_fwd_rows_f64(const double *X, const double *Y, const double *R, const int32_t *row_of, const int32_t *sender,
                      const int32_t *row_ptr, int64_t nnodes, int64_t nedges, int C, double *out, cudaStream_t st) {
   if (nnodes == 0) return CMACE_OK;
   const ImpLayout ys{1, 16};
-  if (C % 64 == 0) launch_fwd<double, 2, true>(X, Y, R, row_of, sender, row_ptr, nnodes, ys, C, out, st);
-  else launch_fwd<double, 1, true>(X, Y, R, row_of, sender, row_ptr, nnodes, ys, C, out, st);
+  if (takes_slots<double>(C)) fwd_slots<double, true>(X, Y, R, row_of, sender, row_ptr, nnodes, ys, C, out, st);
+  else launch_fwd<double, 2, true>(X, Y, R, row_of, sender, row_ptr, nnodes, ys, C, out, st);
   return check_launch("cmace_step(messages)");
 }
 
@@ -711,6 +1061,10 @@ int imp_bwd_edge(const T *X, const T *Y, const T *R, const T *G, const int32_t *
     return fail(CMACE_ERR_ARG, "cmace_imp_bwd_edge: gradY_partial scratch required for %d chunks", nchunks);
   T *gy = nchunks > 1 ? partial : gradY;
   cudaStream_t st = (cudaStream_t)stream;
+  if (takes_slots<T>(C)) {
+    bwd_edge_slots<T, false>(X, Y, R, nullptr, nullptr, G, sender, row_ptr, nnodes, ys, C, gradR, gradY, Tout, st);
+    return check_launch("cmace_imp_bwd_edge");
+  }
   if constexpr (sizeof(T) == 4) {
     if (C == BS_C && aligned16(R) && aligned16(X) && aligned16(G)) {
       static int num_sms = 0;
@@ -780,6 +1134,10 @@ int imp_bwd_node(const T *Tin, const int32_t *perm, const int32_t *send_ptr, int
   if (nnodes == 0) return CMACE_OK;
   if (!send_ptr || !gradX) return fail(CMACE_ERR_ARG, "cmace_imp_bwd_node: null pointer");
   cudaStream_t st = (cudaStream_t)stream;
+  if (C == 96) {   // one pass over the rows instead of three
+    launch_bwd_node<T, 3>(Tin, perm, send_ptr, nnodes, nedges, C, gradX, st);
+    return check_launch("cmace_imp_bwd_node");
+  }
   switch (pick_vec<T>(C)) {
     case 4:
       if constexpr (sizeof(T) == 4) launch_bwd_node<T, 4>(Tin, perm, send_ptr, nnodes, nedges, C, gradX, st);

@@ -112,7 +112,7 @@ struct Workspace {
     take(rows.leaders, pairs ? E : 0);
     take(rows.count, pairs ? 1 : 0);
     if (!pairs) rows = EdgeRows{};
-    shares = sp ? spline_chunks<T>((int)C) : (f64 ? (int)C / (32 * pick_vec<T>((int)C)) : 1);
+    shares = sp ? spline_chunks<T>((int)C) : (f64 && C == 128 ? 2 : 1);   // float64: imp_bwd_edge_pair_f64's channel chunks
     take(gY0, sp ? shares * E * 16 : 0);
     take(dr0, sp ? shares * E : 0);
     take(Y, E * 16);

@@ -727,3 +727,27 @@ def test_float64_product_tiles(M, K, N):
                                      (40, 34, 128), (40, 45, 128), (3157, 45, 96), (3158, 45, 96)])
 def test_message_passing_around_the_split(dtype, N, deg, C, dev):
     test_message_passing(dtype, N, deg, C, None, 7, dev)
+
+
+# rows of fewer than 128 channels, several edges to a warp: fewer edges than a warp takes at a time, one more than that, a remainder,
+# with one warp a receiver and with eight (up to 1 184 receivers)
+@pytest.mark.parametrize("dtype", DTYPES)
+@pytest.mark.parametrize("N,deg,C", [(1300, 1, 32), (1300, 7, 32), (1300, 9, 32), (300, 3, 32), (300, 66, 32), (1300, 3, 64), (1300, 5, 64),
+                                     (300, 33, 64), (1300, 2, 96), (1300, 3, 96), (300, 17, 96)])
+def test_message_passing_of_narrow_rows(dtype, N, deg, C, dev):
+    test_message_passing(dtype, N, deg, C, None, 7, dev)
+
+
+# the same kernels: places of a warp that have no edge add nothing, not zero times what the receiver's last edge holds
+@pytest.mark.parametrize("dtype,C", [(torch.float64, 32), (torch.float64, 96), (torch.float32, 32), (torch.float32, 64),
+                                     (torch.float32, 96)])
+def test_an_infinite_weight_stays_infinite(dtype, C, dev):
+    from cuda_mace_b200 import ops
+
+    n, deg = 1300, 5
+    recv = torch.arange(n, dtype=torch.int32, device=dev).repeat_interleave(deg)
+    X, Y = torch.ones(n, C, dtype=dtype, device=dev), torch.ones(16, n * deg, dtype=dtype, device=dev)
+    R = torch.ones(n * deg, 4, C, dtype=dtype, device=dev)
+    R[deg - 1::deg] = float("inf")
+    out = ops.InvariantMessagePassingTP()(X, Y, R, recv.flip(0).contiguous(), recv, n)
+    assert bool((out == float("inf")).all())
