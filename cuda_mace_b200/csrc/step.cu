@@ -327,17 +327,20 @@ static int run_step(const cmace_step_model &m, cmace_step_io &io, const Workspac
 }
 
 // Programmatic launches while launch latency shows between the kernels, us a float32 step of 128 channels without and with them:
-// 150 -> 117 at 4 700 edges, 241 -> 213 at 52 000, 477 -> 456 at 156 000, 684 -> 670 at 260 000, 903 -> 897 at 364 000, the same
-// at 417 000, 1 265 -> 1 297 at 521 000.  A recorded step has smaller gaps: 130 -> 121 at 4 700, the same at 52 000, 300 -> 305 at
-// 78 000, 336 -> 344 at 99 000, 451 -> 462 at 156 000; its line is float64's, whose kernels are long by then (2 300 -> 2 333 at
-// 156 000), because chained kernels keep their predecessor's split between shared memory and L1.  Tabulated radial weights
-// live on L1: half the edges (516 -> 489 us at 94 000, 709 -> 700 at 157 000, the same at 261 000).
-constexpr int64_t kChainEdges = 98304, kChainEdgesLive = 393216;
+// 250 -> 199 at 52 000 edges, 347 -> 306 at 104 000, 454 -> 418 at 156 000, 756 -> 732 at 312 000, 952 -> 961 at 416 000, 1 793 -> 1 859
+// at 832 000 (64 channels: 692 -> 678 at 416 000, 1 233 -> 1 255 at 832 000).  A recorded step has smaller gaps: 324 -> 311 at
+// 104 000, 429 -> 424 at 156 000, the same at 208 000, 727 -> 740 at 312 000.  float64, whose kernels are long by then: 804 -> 779 at
+// 104 000 edges of 64 channels, 1 071 -> 1 123 at 156 000, 1 167 -> 1 211 at 104 000 of 128; recorded 437 -> 433 at 52 000, 775 -> 788
+// at 104 000: chained kernels keep their predecessor's split between shared memory and L1.  Tabulated radial weights live on L1:
+// half the edges (521 -> 501 us at 104 000, 720 -> 709 at 156 000, 911 -> 914 at 208 000; recorded 187 -> 183 at 26 000, 309 -> 313
+// at 52 000).
+constexpr int64_t kChainEdges = 98304, kChainEdgesRecorded = 196608, kChainEdgesLive = 393216;
 
 static bool chain_for(const cmace_step_model &m, int64_t edges, cudaStream_t st) {
   const int64_t e = is_spline(m) ? 2 * edges : edges;
   if (e <= kChainEdges) return true;
   if (m.is_f64 || e > kChainEdgesLive) return false;
+  if (!is_spline(m) && e <= kChainEdgesRecorded) return true;
   cudaStreamCaptureStatus status;
   return cudaStreamIsCapturing(st, &status) == cudaSuccess && status == cudaStreamCaptureStatusNone;
 }
