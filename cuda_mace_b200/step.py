@@ -352,19 +352,20 @@ def plan_of(model):
 
 
 # Z beyond a + b edges / atom: the operators are faster, {is_f64: {channels: (a, b)}}
-_MANY_ELEMENTS = {False: {32: (2.4, 0.255), 64: (2.3, 0.385), 96: (3.0, 0.65), 128: (8.0, 0.475)},
-                  True: {32: (1.7, 0.345), 64: (2.3, 0.405), 96: (3.0, 0.48), 128: (4.2, 0.42)}}
+_MANY_ELEMENTS = {False: {32: (2.35, 0.365), 64: (2.5, 0.58), 96: (6.3, 0.49), 128: (5.7, 0.72)},
+                  True: {32: (1.05, 0.55), 64: (1.55, 0.65), 96: (2.3, 0.6), 128: (3.2, 0.675)}}
 
 
 def pays(plan, atoms, edges, recorded=False):
     """Whether the sequence is the faster way for a system of this size; `recorded`: in a replayed graph.
 
     The first layer's sums and the products on them take 64 Z columns an atom whatever its edges are, the operators 4 C
-    radial weights an edge.  Native against operators, ms, one B200: 100 000 atoms of 10 edges, float32, 64 channels: 5.4; 6.4
-    at 4 elements, 6.8; 6.5 at 7, 8.1; 6.5 at 10, 10.8; 6.6 at 16; of 21 edges 10.2; 10.2 at 10; of 31 edges 13.7; 14.2 at
-    13; 128 channels, of 10 edges 11.65; 11.76 at 13, 12.05; 11.77
-    at 14; float64, 30 000 atoms of 10 edges, 128 channels: 8.4; 11.0 at 4, 10.5; 11.2 at 7, 12.6; 11.5 at 10.  The lines are
-    where both take the same; a condensed system (52 edges) stays native up to 15 elements.  The operators' launches take the
+    radial weights an edge.  Native against operators, ms, one B200, float32, 100 000 atoms of 10 edges: 32 channels 4.45; 4.43
+    at 6 elements, 64 6.20; 6.32 at 8 and 7.11; 6.30 at 10, 96 9.86; 9.45 at 12, 128 11.74; 11.68 at 13 (of 5 edges 8.90; 8.51 at 10);
+    50 000 atoms of 21 edges: 32 channels 3.87; 3.65 at 11, 64 5.04; 5.20 at 14 and 5.57; 5.22 at 16, 96 6.68; 6.90 at 16.  float64,
+    30 000 atoms of 10 edges: 32 channels 3.61; 4.21 at 5 and 4.42; 4.24 at 7, 64 5.91; 5.94 at 8, 96 8.55; 8.75 at 8 and 9.80; 8.87 at
+    10, 128 11.24; 11.17 at 10; 15 000 atoms of 21 edges: 32 4.10; 3.99 at 13, 64 5.43; 5.47 at 15, 96 7.65; 7.62 at 15, 128 9.02; 9.49
+    at 16.  The lines are where both take the same; a condensed system (52 edges) stays native at any number of elements.  The operators' launches take the
     host 2.1 ms, which small systems never need natively (20 000 atoms of 10 edges, 16 elements, float32, 32 channels: 1.98;
     2.07); recorded, both take the same at 3 000 atoms of 16 elements in float32 (0.39; 0.40) and 1 000 in float64."""
     m = plan.model
