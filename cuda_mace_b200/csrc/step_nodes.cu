@@ -31,28 +31,33 @@ __device__ __forceinline__ void prefetch_weff(const T *__restrict__ weff, int z,
   if (lane < ST_NW) asm volatile("prefetch.global.L1 [%0];" ::"l"(weff + ((int64_t)z * ST_NW + lane) * C + (c & ~31)));
 }
 
+// The value alone needs a third of the gradient's work (canon::value) and half its registers: forward 95 -> 58 us at 32 000 nodes of
+// 128 channels (278 MB: 43 us), 52 -> 35 at 16 000 in a step, 45 -> 29 in float64 at 8 000.  The backward is bound by its
+// arithmetic (about 500 instructions a node and channel: 57 us of its 140 by issue alone).
+//
 // early: whether types and weights are older than the kernel before (not where that kernel has laid the weights out)
 template <typename T, bool BWD>
-__global__ void __launch_bounds__(128, sizeof(T) == 4 ? 5 : 3)
+__global__ void __launch_bounds__(128, BWD ? (sizeof(T) == 4 ? 5 : 3) : (sizeof(T) == 4 ? 10 : 6))
     step_contract_kernel(const T *__restrict__ X, const int32_t *__restrict__ types, const T *__restrict__ weff,
                          const T *__restrict__ gb, int64_t nnodes, int C, bool early, T *__restrict__ out) {
   const int c = blockIdx.y * blockDim.x + threadIdx.x;
   if (early && nnodes <= gridDim.x) prefetch_weff(weff, __ldcg(types + blockIdx.x), C, c);
   grid_begin();
   for (int64_t node = blockIdx.x; node < nnodes; node += gridDim.x) {
-    T x[16], g[16], w3[canon::NCLASS3], w2[canon::NCLASS2], w1, value;
+    T x[16], w3[canon::NCLASS3], w2[canon::NCLASS2], w1;
     const T *xr = X + node * 16 * C + c;
 #pragma unroll
     for (int i = 0; i < 16; i++) x[i] = __ldcs(xr + i * C);
     load_weff(weff, types[node], C, c, w3, w2, w1);
-    const T go = BWD ? gb[node * C + c] : T(0);
-    canon::eval<T>(x, w3, w2, w1, g, value);
-    if (BWD) {
+    if constexpr (BWD) {
+      T g[16], value;
+      const T go = gb[node * C + c];
+      canon::eval<T>(x, w3, w2, w1, g, value);
       T *o = out + node * 16 * C + c;
 #pragma unroll
       for (int i = 0; i < 16; i++) __stcs(o + i * C, go * g[i]);
     } else {
-      out[node * C + c] = value;
+      out[node * C + c] = canon::value<T>(x, w3, w2, w1);
     }
   }
 }
@@ -65,9 +70,9 @@ static int channel_block(int C) {
   return 32;
 }
 
-// blocks, sized for 128 channels (four warps a block): at 32 channels 10 to 12 blocks are as many warps an SM
-static int64_t node_blocks(int64_t n, int per_sm) {
-  const int64_t cap = (int64_t)148 * per_sm;
+// blocks of ch threads: per_sm an SM of 128 threads, more of fewer
+static int64_t node_blocks(int64_t n, int per_sm, int ch) {
+  const int64_t cap = (int64_t)148 * per_sm * (128 / ch);
   return n < cap ? n : cap;
 }
 
@@ -76,7 +81,7 @@ int StepKernels<T>::contract_fwd(const T *X, const int32_t *types, const T *weff
                                  cudaStream_t st) {
   const int ch = channel_block(C);
   if (n > 0)
-    launch_chained(step_contract_kernel<T, false>, dim3((unsigned)node_blocks(n, 12), C / ch), ch, 0, st, X, types, weff, nullptr, n, C, early, b);
+    launch_chained(step_contract_kernel<T, false>, dim3((unsigned)node_blocks(n, 16, ch), C / ch), ch, 0, st, X, types, weff, nullptr, n, C, early, b);
   return check_launch("cmace_step(contract_fwd)");
 }
 template <typename T>
@@ -84,7 +89,7 @@ int StepKernels<T>::contract_bwd(const T *X, const int32_t *types, const T *weff
                                  cudaStream_t st) {
   const int ch = channel_block(C);
   if (n > 0)
-    launch_chained(step_contract_kernel<T, true>, dim3((unsigned)node_blocks(n, 12), C / ch), ch, 0, st, X, types, weff, gb, n, C, early, gX);
+    launch_chained(step_contract_kernel<T, true>, dim3((unsigned)node_blocks(n, 12, ch), C / ch), ch, 0, st, X, types, weff, gb, n, C, early, gX);
   return check_launch("cmace_step(contract_bwd)");
 }
 
@@ -159,7 +164,7 @@ int StepKernels<T>::contract_readout(const T *X, const int32_t *types, const T *
                                      const T *q0, const double *atomic_e, double scale, double shift, int64_t n, int C,
                                      T *gX, T *dq, double *inter, double *node_energy, cudaStream_t st) {
   if (n > 0)
-    launch_chained(contract_readout_kernel<T>, (unsigned)node_blocks(n, 10), C, 0, st, X, types, weff, wp1, w2, q0, atomic_e, scale,
+    launch_chained(contract_readout_kernel<T>, (unsigned)node_blocks(n, 10, C), C, 0, st, X, types, weff, wp1, w2, q0, atomic_e, scale,
                                                                           shift, n, C, gX, dq, inter, node_energy);
   return check_launch("cmace_step(contract_readout)");
 }
