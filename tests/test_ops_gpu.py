@@ -751,3 +751,18 @@ def test_an_infinite_weight_stays_infinite(dtype, C, dev):
     R[deg - 1::deg] = float("inf")
     out = ops.InvariantMessagePassingTP()(X, Y, R, recv.flip(0).contiguous(), recv, n)
     assert bool((out == float("inf")).all())
+
+
+# grouping by a key: one block's counting sort up to 8 192 entries of 1 600 keys, the radix sort beyond, against a stable sort; whole
+# and partial warps, pieces of one warp, keys that do not occur
+@pytest.mark.parametrize("n,nkeys", [(1, 1), (31, 7), (33, 40), (1024, 3), (1025, 1600), (5000, 1), (8192, 1600), (8192, 1601),
+                                     (8193, 600)])
+def test_grouping_by_key(n, nkeys, dev):
+    from cuda_mace_b200 import ops
+
+    g = torch.Generator().manual_seed(n + nkeys)
+    keys = torch.randint(0, max(1, nkeys - nkeys // 3), (n,), generator=g, dtype=torch.int32)
+    topo = ops.EdgeTopology(keys.to(dev), torch.zeros(n, dtype=torch.int32, device=dev), 1, nkeys)
+    perm, ptr = topo.sender_order()
+    assert torch.equal(perm.cpu().long(), torch.sort(keys, stable=True)[1])
+    assert torch.equal(ptr.cpu().long(), torch.searchsorted(torch.sort(keys)[0].long(), torch.arange(nkeys + 1)))
