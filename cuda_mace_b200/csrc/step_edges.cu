@@ -370,6 +370,17 @@ int StepKernels<T>::edge_prep(const double *pos, const int32_t *sender, const in
 constexpr int SU_WARPS = 4;
 constexpr int SU_LIST = 64;
 
+// Elements of a receiver that a warp takes one after the other (float32): its list, the senders' elements and the rows are looked up
+// once, which is most of a pair's chain of loads; while that leaves the chip about 24 warps an SM, in equal parts.  us, sums and
+// backward, one element a warp and this: 136, 183 -> 109, 166 at 16 000 atoms of 4 elements, 262, 289 -> 203, 264 of 10; 562, 735 ->
+// 414, 629 at 64 000; 33, 46 -> 29, 43 at 3 000 of 4 (all four: 31, 48).  In float64 the registers of the loop cost a block an SM:
+// 127, 260 -> 135, 260 at 8 000.
+static int elements_per_warp(int64_t nnodes, int elements) {
+  const int64_t fit = nnodes * elements / (148 * 24);
+  const int most = fit < 1 ? 1 : (fit > elements ? elements : (int)fit), chunks = (elements + most - 1) / most;
+  return (elements + chunks - 1) / chunks;
+}
+
 // In a chain of launches (EARLY) the look-up stands before grid_wait(), otherwise behind the loads that it would hold up: with one
 // order for both the sums of 16 000 atoms took 144 us instead of 135, their backward 191 instead of 183.
 struct SenderElements {
@@ -593,19 +604,20 @@ template <bool EARLY>
 __global__ void __launch_bounds__(SU_WARPS * 32)
     sums_f16_kernel(const uint4 *__restrict__ h, const float *__restrict__ Y, const int32_t *__restrict__ sender,
                     const int32_t *__restrict__ row_ptr, const int32_t *__restrict__ species,
-                    const int32_t *__restrict__ slot_of, const int32_t *__restrict__ row_of, int64_t nnodes, int elements,
+                    const int32_t *__restrict__ slot_of, const int32_t *__restrict__ row_of, int64_t nnodes, int elements, int per,
                     float factor,
                     float *__restrict__ A) {
   __shared__ int32_t lists[SU_WARPS][SU_LIST], row_lists[SU_WARPS][64 + SU_LIST];
   const int lane = threadIdx.x & 31, w = threadIdx.x >> 5, g = lane >> 2, t = lane & 3;
   const int64_t pair = (int64_t)blockIdx.x * SU_WARPS + w;
   if (!EARLY) grid_begin();
-  if (pair >= nnodes * elements) {
+  const int chunks = (elements + per - 1) / per;
+  if (pair >= nnodes * chunks) {
     if (EARLY) grid_begin();
     return;
   }
-  const int64_t node = pair / elements;
-  const int z = (int)(pair - node * elements);
+  const int64_t node = pair / chunks;
+  const int z0 = (int)(pair - node * chunks) * per, z1 = z0 + per < elements ? z0 + per : elements;
   SenderElements from(sender, species, row_ptr[node], row_ptr[node + 1], lane);
   if (EARLY) {
     from.look_up();
@@ -613,53 +625,57 @@ __global__ void __launch_bounds__(SU_WARPS * 32)
   }
   SharedRows rows(row_of, row_lists[w], from);
   int32_t *list = lists[w];
-  float acc[8][4];
-#pragma unroll
-  for (int j = 0; j < 8; j++) acc[j][0] = acc[j][1] = acc[j][2] = acc[j][3] = 0.f;
   if (!EARLY) from.look_up();
   rows.wait();
-  for_edges_of_element(from, z, list, rows, [&](int n) {
-    for (int j0 = 0; j0 < n; j0 += 16) {
-      uint4 hv[4], lv[4];
-      uint32_t ah[4], al[4];
+#pragma unroll 1
+  for (int z = z0; z < z1; z++) {
+    __syncwarp();   // the list of the element before has been read
+    float acc[8][4];
+#pragma unroll
+    for (int j = 0; j < 8; j++) acc[j][0] = acc[j][1] = acc[j][2] = acc[j][3] = 0.f;
+    for_edges_of_element(from, z, list, rows, [&](int n) {
+      for (int j0 = 0; j0 < n; j0 += 16) {
+        uint4 hv[4], lv[4];
+        uint32_t ah[4], al[4];
+#pragma unroll
+        for (int u = 0; u < 2; u++) {
+          float y[2][2];
+#pragma unroll
+          for (int v = 0; v < 2; v++) {   // past the end: the last edge with Y = 0
+            const int j = j0 + 8 * u + 2 * t + v;
+            const int64_t e = list[j < n ? j : n - 1];
+            const int64_t row = rows[j < n ? j : n - 1];
+            hv[2 * u + v] = __ldg(h + row * 16 + g);
+            lv[2 * u + v] = __ldg(h + row * 16 + 8 + g);
+            y[v][0] = j < n ? __ldg(Y + e * 16 + g) * SU_Y_SCALE : 0.f;
+            y[v][1] = j < n ? __ldg(Y + e * 16 + g + 8) * SU_Y_SCALE : 0.f;
+          }
+          split_half2(pack2(y[0][0], y[1][0]), ah[2 * u], al[2 * u]);
+          split_half2(pack2(y[0][1], y[1][1]), ah[2 * u + 1], al[2 * u + 1]);
+        }
+#pragma unroll
+        for (int j = 0; j < 8; j++) {
+          auto word = [&](const uint4 &x) { return (j >> 1) == 0 ? x.x : ((j >> 1) == 1 ? x.y : ((j >> 1) == 2 ? x.z : x.w)); };
+          const uint32_t sel = (j & 1) ? 0x7632u : 0x5410u;
+          const uint32_t h0 = __byte_perm(word(hv[0]), word(hv[1]), sel), h1 = __byte_perm(word(hv[2]), word(hv[3]), sel);
+          const uint32_t l0 = __byte_perm(word(lv[0]), word(lv[1]), sel), l1 = __byte_perm(word(lv[2]), word(lv[3]), sel);
+          mma_f16(acc[j], ah, h0, h1);
+          mma_f16(acc[j], ah, l0, l1);
+          mma_f16(acc[j], al, h0, h1);
+        }
+      }
+    });
+    const int width = elements * ST_H;
+    float *o = A + (int64_t)slot_of[node] * 16 * width + z * ST_H + 16 * t;
+#pragma unroll
+    for (int half = 0; half < 2; half++) {   // rows lm = g and g + 8
+      float *row = o + (int64_t)(g + 8 * half) * width;
 #pragma unroll
       for (int u = 0; u < 2; u++) {
-        float y[2][2];
-#pragma unroll
-        for (int v = 0; v < 2; v++) {   // past the end: the last edge with Y = 0
-          const int j = j0 + 8 * u + 2 * t + v;
-          const int64_t e = list[j < n ? j : n - 1];
-          const int64_t row = rows[j < n ? j : n - 1];
-          hv[2 * u + v] = __ldg(h + row * 16 + g);
-          lv[2 * u + v] = __ldg(h + row * 16 + 8 + g);
-          y[v][0] = j < n ? __ldg(Y + e * 16 + g) * SU_Y_SCALE : 0.f;
-          y[v][1] = j < n ? __ldg(Y + e * 16 + g + 8) * SU_Y_SCALE : 0.f;
-        }
-        split_half2(pack2(y[0][0], y[1][0]), ah[2 * u], al[2 * u]);
-        split_half2(pack2(y[0][1], y[1][1]), ah[2 * u + 1], al[2 * u + 1]);
+        const int c = 2 * half + u;
+        store32(row + 8 * u, acc[0][c] * factor, acc[1][c] * factor, acc[2][c] * factor, acc[3][c] * factor, acc[4][c] * factor,
+                acc[5][c] * factor, acc[6][c] * factor, acc[7][c] * factor);
       }
-#pragma unroll
-      for (int j = 0; j < 8; j++) {
-        auto word = [&](const uint4 &x) { return (j >> 1) == 0 ? x.x : ((j >> 1) == 1 ? x.y : ((j >> 1) == 2 ? x.z : x.w)); };
-        const uint32_t sel = (j & 1) ? 0x7632u : 0x5410u;
-        const uint32_t h0 = __byte_perm(word(hv[0]), word(hv[1]), sel), h1 = __byte_perm(word(hv[2]), word(hv[3]), sel);
-        const uint32_t l0 = __byte_perm(word(lv[0]), word(lv[1]), sel), l1 = __byte_perm(word(lv[2]), word(lv[3]), sel);
-        mma_f16(acc[j], ah, h0, h1);
-        mma_f16(acc[j], ah, l0, l1);
-        mma_f16(acc[j], al, h0, h1);
-      }
-    }
-  });
-  const int width = elements * ST_H;
-  float *o = A + (int64_t)slot_of[node] * 16 * width + z * ST_H + 16 * t;
-#pragma unroll
-  for (int half = 0; half < 2; half++) {   // rows lm = g and g + 8
-    float *row = o + (int64_t)(g + 8 * half) * width;
-#pragma unroll
-    for (int u = 0; u < 2; u++) {
-      const int c = 2 * half + u;
-      store32(row + 8 * u, acc[0][c] * factor, acc[1][c] * factor, acc[2][c] * factor, acc[3][c] * factor, acc[4][c] * factor,
-              acc[5][c] * factor, acc[6][c] * factor, acc[7][c] * factor);
     }
   }
 }
@@ -667,10 +683,11 @@ __global__ void __launch_bounds__(SU_WARPS * 32)
 int step_sums_half(const void *h, const float *Y, const int32_t *sender, const int32_t *row_ptr, const int32_t *species,
                    const int32_t *slot_of, const int32_t *row_of, int64_t nnodes, int elements, float out_v, float *A,
                    cudaStream_t st) {
-  const int64_t blocks = (nnodes * elements + SU_WARPS - 1) / SU_WARPS;
+  const int per = elements_per_warp(nnodes, elements);
+  const int64_t blocks = (nnodes * ((elements + per - 1) / per) + SU_WARPS - 1) / SU_WARPS;
   if (blocks > 0)
     launch_chained(chain_launches() ? sums_f16_kernel<true> : sums_f16_kernel<false>, (unsigned)blocks, SU_WARPS * 32, 0, st, static_cast<const uint4 *>(h), Y, sender, row_ptr, species,
-                                                               slot_of, row_of, nnodes, elements, out_v / SU_Y_SCALE, A);
+                                                               slot_of, row_of, nnodes, elements, per, out_v / SU_Y_SCALE, A);
   return check_launch("cmace_step(sums)");
 }
 
@@ -915,19 +932,20 @@ __global__ void __launch_bounds__(SU_WARPS * 32, 4)
                         const float *__restrict__ Y, const int32_t *__restrict__ sender,
                         const int32_t *__restrict__ row_ptr, const int32_t *__restrict__ species,
                         const int32_t *__restrict__ slot_of, const int32_t *__restrict__ row_of, const float *__restrict__ gY1,
-                        const float *__restrict__ dr1, const Quad<float> *__restrict__ geo, int64_t nnodes, int elements,
+                        const float *__restrict__ dr1, const Quad<float> *__restrict__ geo, int64_t nnodes, int elements, int per,
                         float out_v, float out_t, float *__restrict__ gvec) {
   __shared__ int32_t lists[SU_WARPS][SU_LIST], row_lists[SU_WARPS][64 + SU_LIST];
   __shared__ float stage[SU_WARPS][32 * 17];
   const int lane = threadIdx.x & 31, w = threadIdx.x >> 5, g = lane >> 2, t = lane & 3;
   const int64_t pair = (int64_t)blockIdx.x * SU_WARPS + w;
   if (!EARLY) grid_begin();
-  if (pair >= nnodes * elements) {
+  const int chunks = (elements + per - 1) / per;
+  if (pair >= nnodes * chunks) {
     if (EARLY) grid_begin();
     return;
   }
-  const int64_t node = pair / elements;
-  const int z = (int)(pair - node * elements);
+  const int64_t node = pair / chunks;
+  const int z0 = (int)(pair - node * chunks) * per, z1 = z0 + per < elements ? z0 + per : elements;
   SenderElements from(sender, species, row_ptr[node], row_ptr[node + 1], lane);
   SharedRows rows(row_of, row_lists[w], from);
   if (EARLY) {
@@ -936,118 +954,128 @@ __global__ void __launch_bounds__(SU_WARPS * 32, 4)
   }   // only the gradients of the sums are the kernel before's
   int32_t *list = lists[w];
   float *st = stage[w];
-  uint32_t ph[4][4], pl[4][4];   // A fragments of the 4 K steps
-  {
-    const int b = z >> 1, width = sums_block_width(elements, b);
-    const float *p = gA + (int64_t)b * nnodes * (16 * 128) + (int64_t)slot_of[node] * 16 * width + (z & 1) * ST_H + 8 * t;
-    float4 v[2][2][2];   // [piece][row g, g + 8][half of the piece]
-    float most = 0.f;
+#pragma unroll 1
+  for (int z = z0; z < z1; z++) {
+    __syncwarp();   // the list of the element before has been read
+    float sv, stt;
+    uint32_t ph[4][4], pl[4][4];   // A fragments of the 4 K steps
+    {
+      const int b = z >> 1, width = sums_block_width(elements, b);
+      const float *p = gA + (int64_t)b * nnodes * (16 * 128) + (int64_t)slot_of[node] * 16 * width + (z & 1) * ST_H + 8 * t;
+      float4 v[2][2][2];   // [piece][row g, g + 8][half of the piece]
+      float most = 0.f;
 #pragma unroll
-    for (int i = 0; i < 2; i++)
+      for (int i = 0; i < 2; i++)
 #pragma unroll
-      for (int r = 0; r < 2; r++) load32(p + (g + 8 * r) * width + 32 * i, v[i][r][0], v[i][r][1]);
-    if (!EARLY) from.look_up();
-#pragma unroll
-    for (int i = 0; i < 2; i++)
-#pragma unroll
-      for (int r = 0; r < 2; r++)
-#pragma unroll
-        for (int u = 0; u < 2; u++) {
-          most = fmaxf(most, fmaxf(fmaxf(fabsf(v[i][r][u].x), fabsf(v[i][r][u].y)), fmaxf(fabsf(v[i][r][u].z), fabsf(v[i][r][u].w))));
-        }
-#pragma unroll
-    for (int off = 16; off > 0; off >>= 1) most = fmaxf(most, __shfl_xor_sync(0xffffffffu, most, off));
-    int ex = 127 + 13 - ((int)((__float_as_uint(most) >> 23) & 255u) - 127);   // biased exponent of the scale
-    ex = ex < 1 ? 1 : (ex > 253 ? 253 : ex);
-    const float sc = __uint_as_float((uint32_t)ex << 23), inv = __uint_as_float((uint32_t)(254 - ex) << 23);
-    const unsigned long long sc2 = pack2(sc, sc);
-    out_v *= inv;
-    out_t *= inv;
-#pragma unroll
-    for (int i = 0; i < 2; i++)
-#pragma unroll
-      for (int u = 0; u < 2; u++)
-#pragma unroll
-        for (int r = 0; r < 2; r++) {
-          split_half2(mul2(pack2(v[i][r][u].x, v[i][r][u].y), sc2), ph[2 * i + u][r], pl[2 * i + u][r]);
-          split_half2(mul2(pack2(v[i][r][u].z, v[i][r][u].w), sc2), ph[2 * i + u][2 + r], pl[2 * i + u][2 + r]);
-        }
-  }
-  rows.wait();
-  for_edges_of_element(from, z, list, rows, [&](int n) {
-    for (int j0 = 0; j0 < n; j0 += 32) {
-      const int nj = n - j0 < 32 ? n - j0 : 32;
-      if (lane < nj) {   // what finish_edge reads
-        prefetch_l1(gY1 + (int64_t)list[j0 + lane] * 16);
-        prefetch_l1(geo + list[j0 + lane]);
+        for (int r = 0; r < 2; r++) load32(p + (g + 8 * r) * width + 32 * i, v[i][r][0], v[i][r][1]);
+      if (z + 1 < z1) {   // the next element's gradients on their way to L1: lane's half of a row of 64
+        const int nb = (z + 1) >> 1, nw = sums_block_width(elements, nb);
+        prefetch_l1(gA + (int64_t)nb * nnodes * (16 * 128) + ((int64_t)slot_of[node] * 16 + (lane >> 1)) * nw + ((z + 1) & 1) * ST_H + 32 * (lane & 1));
       }
-      uint4 hh[2], hl[2], dd[2], dl[2];
-      auto load = [&](int j) {   // edge j0 + j + g, or the last one
-        const int i = j0 + j + g;
-        const int64_t e = rows[i < n ? i : n - 1];
+      if (!EARLY && z == z0) from.look_up();
 #pragma unroll
-        for (int q = 0; q < 2; q++) {
-          hh[q] = __ldg(h + e * 16 + t + 4 * q);
-          hl[q] = __ldg(h + e * 16 + 8 + t + 4 * q);
-          dd[q] = __ldg(dh + e * 16 + t + 4 * q);
-          dl[q] = __ldg(dh + e * 16 + 8 + t + 4 * q);
-        }
-      };
-      load(0);
-      for (int j = 0; j < nj; j += 8) {
-        float ch[4] = {0.f, 0.f, 0.f, 0.f}, cd[4] = {0.f, 0.f, 0.f, 0.f};
-        const int i0 = j0 + j + 2 * t;   // this lane's result columns: edges 2 t and 2 t + 1 of the eight
-        const int64_t e0 = list[i0 < n ? i0 : n - 1], e1 = list[i0 + 1 < n ? i0 + 1 : n - 1];
-        const float y00 = __ldg(Y + e0 * 16 + g), y01 = __ldg(Y + e0 * 16 + g + 8);
-        const float y10 = __ldg(Y + e1 * 16 + g), y11 = __ldg(Y + e1 * 16 + g + 8);
+      for (int i = 0; i < 2; i++)
 #pragma unroll
-        for (int q = 0; q < 2; q++) {
-          mma_f16(ch, ph[2 * q], hh[q].x, hh[q].y);
-          mma_f16(cd, ph[2 * q], dd[q].x, dd[q].y);
-          mma_f16(ch, ph[2 * q], hl[q].x, hl[q].y);
-          mma_f16(cd, ph[2 * q], dl[q].x, dl[q].y);
-          mma_f16(ch, pl[2 * q], hh[q].x, hh[q].y);
-          mma_f16(cd, pl[2 * q], dd[q].x, dd[q].y);
-          mma_f16(ch, ph[2 * q + 1], hh[q].z, hh[q].w);
-          mma_f16(cd, ph[2 * q + 1], dd[q].z, dd[q].w);
-          mma_f16(ch, ph[2 * q + 1], hl[q].z, hl[q].w);
-          mma_f16(cd, ph[2 * q + 1], dl[q].z, dl[q].w);
-          mma_f16(ch, pl[2 * q + 1], hh[q].z, hh[q].w);
-          mma_f16(cd, pl[2 * q + 1], dd[q].z, dd[q].w);
-        }
-        if (j + 8 < nj) load(j + 8);
-        float *s0 = st + (j + 2 * t) * 17, *s1 = s0 + 17;
-        s0[g] = ch[0] * out_v;
-        s1[g] = ch[1] * out_v;
-        s0[g + 8] = ch[2] * out_v;
-        s1[g + 8] = ch[3] * out_v;
-        float r0 = fmaf(y00, cd[0], y01 * cd[2]), r1 = fmaf(y10, cd[1], y11 * cd[3]);
+        for (int r = 0; r < 2; r++)
 #pragma unroll
-        for (int off = 4; off < 32; off <<= 1) {
-          r0 += __shfl_xor_sync(0xffffffffu, r0, off);
-          r1 += __shfl_xor_sync(0xffffffffu, r1, off);
-        }
-        if (g == 0) {
-          s0[16] = r0 * out_t;
-          s1[16] = r1 * out_t;
-        }
-      }
-      __syncwarp();
-      if (lane < nj) finish_edge<float>(st + lane * 17, list[j0 + lane], gY1, dr1, geo, gvec);
-      __syncwarp();
+          for (int u = 0; u < 2; u++) {
+            most = fmaxf(most, fmaxf(fmaxf(fabsf(v[i][r][u].x), fabsf(v[i][r][u].y)), fmaxf(fabsf(v[i][r][u].z), fabsf(v[i][r][u].w))));
+          }
+#pragma unroll
+      for (int off = 16; off > 0; off >>= 1) most = fmaxf(most, __shfl_xor_sync(0xffffffffu, most, off));
+      int ex = 127 + 13 - ((int)((__float_as_uint(most) >> 23) & 255u) - 127);   // biased exponent of the scale
+      ex = ex < 1 ? 1 : (ex > 253 ? 253 : ex);
+      const float sc = __uint_as_float((uint32_t)ex << 23), inv = __uint_as_float((uint32_t)(254 - ex) << 23);
+      const unsigned long long sc2 = pack2(sc, sc);
+      sv = out_v * inv;
+      stt = out_t * inv;
+#pragma unroll
+      for (int i = 0; i < 2; i++)
+#pragma unroll
+        for (int u = 0; u < 2; u++)
+#pragma unroll
+          for (int r = 0; r < 2; r++) {
+            split_half2(mul2(pack2(v[i][r][u].x, v[i][r][u].y), sc2), ph[2 * i + u][r], pl[2 * i + u][r]);
+            split_half2(mul2(pack2(v[i][r][u].z, v[i][r][u].w), sc2), ph[2 * i + u][2 + r], pl[2 * i + u][2 + r]);
+          }
     }
-  });
+    if (z == z0) rows.wait();
+    for_edges_of_element(from, z, list, rows, [&](int n) {
+      for (int j0 = 0; j0 < n; j0 += 32) {
+        const int nj = n - j0 < 32 ? n - j0 : 32;
+        if (lane < nj) {   // what finish_edge reads
+          prefetch_l1(gY1 + (int64_t)list[j0 + lane] * 16);
+          prefetch_l1(geo + list[j0 + lane]);
+        }
+        uint4 hh[2], hl[2], dd[2], dl[2];
+        auto load = [&](int j) {   // edge j0 + j + g, or the last one
+          const int i = j0 + j + g;
+          const int64_t e = rows[i < n ? i : n - 1];
+#pragma unroll
+          for (int q = 0; q < 2; q++) {
+            hh[q] = __ldg(h + e * 16 + t + 4 * q);
+            hl[q] = __ldg(h + e * 16 + 8 + t + 4 * q);
+            dd[q] = __ldg(dh + e * 16 + t + 4 * q);
+            dl[q] = __ldg(dh + e * 16 + 8 + t + 4 * q);
+          }
+        };
+        load(0);
+        for (int j = 0; j < nj; j += 8) {
+          float ch[4] = {0.f, 0.f, 0.f, 0.f}, cd[4] = {0.f, 0.f, 0.f, 0.f};
+          const int i0 = j0 + j + 2 * t;   // this lane's result columns: edges 2 t and 2 t + 1 of the eight
+          const int64_t e0 = list[i0 < n ? i0 : n - 1], e1 = list[i0 + 1 < n ? i0 + 1 : n - 1];
+          const float y00 = __ldg(Y + e0 * 16 + g), y01 = __ldg(Y + e0 * 16 + g + 8);
+          const float y10 = __ldg(Y + e1 * 16 + g), y11 = __ldg(Y + e1 * 16 + g + 8);
+#pragma unroll
+          for (int q = 0; q < 2; q++) {
+            mma_f16(ch, ph[2 * q], hh[q].x, hh[q].y);
+            mma_f16(cd, ph[2 * q], dd[q].x, dd[q].y);
+            mma_f16(ch, ph[2 * q], hl[q].x, hl[q].y);
+            mma_f16(cd, ph[2 * q], dl[q].x, dl[q].y);
+            mma_f16(ch, pl[2 * q], hh[q].x, hh[q].y);
+            mma_f16(cd, pl[2 * q], dd[q].x, dd[q].y);
+            mma_f16(ch, ph[2 * q + 1], hh[q].z, hh[q].w);
+            mma_f16(cd, ph[2 * q + 1], dd[q].z, dd[q].w);
+            mma_f16(ch, ph[2 * q + 1], hl[q].z, hl[q].w);
+            mma_f16(cd, ph[2 * q + 1], dl[q].z, dl[q].w);
+            mma_f16(ch, pl[2 * q + 1], hh[q].z, hh[q].w);
+            mma_f16(cd, pl[2 * q + 1], dd[q].z, dd[q].w);
+          }
+          if (j + 8 < nj) load(j + 8);
+          float *s0 = st + (j + 2 * t) * 17, *s1 = s0 + 17;
+          s0[g] = ch[0] * sv;
+          s1[g] = ch[1] * sv;
+          s0[g + 8] = ch[2] * sv;
+          s1[g + 8] = ch[3] * sv;
+          float r0 = fmaf(y00, cd[0], y01 * cd[2]), r1 = fmaf(y10, cd[1], y11 * cd[3]);
+#pragma unroll
+          for (int off = 4; off < 32; off <<= 1) {
+            r0 += __shfl_xor_sync(0xffffffffu, r0, off);
+            r1 += __shfl_xor_sync(0xffffffffu, r1, off);
+          }
+          if (g == 0) {
+            s0[16] = r0 * stt;
+            s1[16] = r1 * stt;
+          }
+        }
+        __syncwarp();
+        if (lane < nj) finish_edge<float>(st + lane * 17, list[j0 + lane], gY1, dr1, geo, gvec);
+        __syncwarp();
+      }
+    });
+  }
 }
 
 int step_sums_bwd_half(const float *gA, const void *h, const void *dh, const float *Y, const int32_t *sender,
                        const int32_t *row_ptr, const int32_t *species, const int32_t *slot_of, const int32_t *row_of, const float *gY1,
                        const float *dr1, const Quad<float> *geo, int64_t nnodes, int elements, float out_v, float out_t,
                        float *gvec, cudaStream_t st) {
-  const int64_t blocks = (nnodes * elements + SU_WARPS - 1) / SU_WARPS;
+  const int per = elements_per_warp(nnodes, elements);
+  const int64_t blocks = (nnodes * ((elements + per - 1) / per) + SU_WARPS - 1) / SU_WARPS;
   if (blocks > 0)
     launch_chained(chain_launches() ? sums_bwd_f16_kernel<true> : sums_bwd_f16_kernel<false>, (unsigned)blocks, SU_WARPS * 32, 0, st, 
         gA, static_cast<const uint4 *>(h), static_cast<const uint4 *>(dh), Y, sender, row_ptr, species, slot_of, row_of, gY1, dr1,
-        geo, nnodes, elements, out_v, out_t, gvec);
+        geo, nnodes, elements, per, out_v, out_t, gvec);
   return check_launch("cmace_step(sums_back)");
 }
 
