@@ -10,18 +10,16 @@
 // yields Ahi*Bhi and Ahi*Blo from a single instruction (two column ranges of the accumulator, added in the
 // epilogue); with Alo*Bhi that is two instructions per K step instead of three.
 //
-// Structure (one CTA per SM, persistent over 128-row tiles, warp specialised, 18 warps):
+// Structure (one CTA per SM, persistent over 128-row tiles, warp specialised, 18 warps, LINEAR 21):
 //   warp 17    loader (PLAIN row map): per pipeline item one TMA tile load (128 rows x 32 columns of A,
 //              128-byte swizzle) straight into the stage's hi image (the tensor core ignores the low 13
 //              mantissa bits of a float32, so raw data is the hi operand) and one bulk copy of the matching
 //              pre-packed B block (hi and lo images, swizzled by the pack kernel).  Nothing waits in
-//              registers for HBM.
+//              registers for HBM.  LINEAR with gathered rows: warps 17-20 copy the row segments by cp.async.
 //   warps 0-7  converters (PLAIN): read the raw tile back from shared memory and store the residual image
 //              lo = tf32(a - trunc(a)) next to it -- or, where tensor memory has room beside the accumulators
 //              (kernel variant TS), into a ring of tensor-memory columns, from where the Alo*Bhi product
 //              takes its A operand.
-//              With the LINEAR row map (gathered rows) the same warps load the row segments into registers
-//              themselves, two items ahead, and convert from there.
 //   warp 8     MMA issuer: one elected thread issues tcgen05.mma kind::tf32 (M=128, N<=128, K=8),
 //              4 K-steps x 3 split terms per stage, and commits to the stage's "empty" barrier and,
 //              after the last K block of a tile, to the accumulator's "full" barrier.
@@ -55,14 +53,14 @@ constexpr int GT_MAX_STAGES = 8;
 constexpr int GT_TILE_M = 128;
 constexpr int GT_KBLOCK = 32;                       // floats per K block = one 128-byte swizzle row
 constexpr int GT_A_SLAB = GT_TILE_M * 128;          // bytes of one A image (hi or lo) per stage
-constexpr int GT_PRODUCER_WARPS = 8;                 // 8 measured best (4: 0.47 ms, 8: 0.36 ms, 16: 0.59 ms on the Linear case)
+constexpr int GT_PRODUCER_WARPS = 8;                // GRADR: they form A; otherwise: they convert
 constexpr int GT_ROWS_PER_THREAD = GT_TILE_M / (GT_PRODUCER_WARPS * 4);  // 8 threads cover one row segment
 constexpr int GT_ROW_STEP = GT_PRODUCER_WARPS * 4;                       // rows between a thread's row segments
 constexpr int GT_EPILOGUE_WARPS = 8;
+constexpr int GT_GATHER_WARPS = 4;                  // LINEAR: warps that copy gathered rows
 constexpr int GT_THREADS = (GT_PRODUCER_WARPS + 1 + GT_EPILOGUE_WARPS + 1) * 32;
 constexpr int GT_SMEM_BUDGET = 227 * 1024 - 2048;    // dynamic shared memory (the static barriers count against the same 227 KB)
 constexpr int GT_TMEM_COLS = 512;                   // two accumulators of 2 x 128 columns
-constexpr int GT_PREFETCH = 2;                      // K blocks of global loads in flight per producer thread
 constexpr int GT_EP_STRIDE = 20;                    // floats per row of an epilogue transpose buffer (16 + padding)
 constexpr int GT_EP_BYTES = 8 * 32 * GT_EP_STRIDE * 4;  // one buffer per epilogue warp, 20 KB in all
 constexpr int GT_EP_TMA_BYTES = 8 * 32 * 128;       // PLAIN with TMA stores: 32 rows x 128 bytes per epilogue warp
@@ -285,7 +283,7 @@ __device__ __forceinline__ void report(const GemmArgs &g, int code) {
 // its narrow output leaves the epilogue idle most of the time, and 14 warps instead of 18 give every thread 128
 // registers instead of 96, which is what its producer warps were short of (2.73 -> 2.35 ms).
 template <int MODE, bool TS = false, int CC = 0, int EW = GT_EPILOGUE_WARPS, bool OA = false>
-__global__ void __launch_bounds__((GT_PRODUCER_WARPS + 1 + EW + 1) * 32, 1)
+__global__ void __launch_bounds__((GT_PRODUCER_WARPS + 1 + EW + (MODE == GT_MODE_LINEAR ? GT_GATHER_WARPS : 1)) * 32, 1)
     gemm3x_tf32_kernel(const GemmArgs g, const __grid_constant__ CUtensorMap tmap,
                        const __grid_constant__ CUtensorMap tmap_out, const __grid_constant__ LinMaps lin_maps) {
   extern __shared__ __align__(1024) unsigned char smem[];
@@ -313,9 +311,10 @@ __global__ void __launch_bounds__((GT_PRODUCER_WARPS + 1 + EW + 1) * 32, 1)
 
   if (threadIdx.x == 0) {
     for (int s = 0; s < GT_STAGES; s++) {
-      // LINEAR, GRADR: one arrival per producer warp + the expect_tx arrival of the B copy; PLAIN: converters only
-      mbar_init(full_bar + 8 * s, GT_PRODUCER_WARPS + ((MODE == GT_MODE_PLAIN || g.lin_tma) ? 0 : 1));
-      mbar_init(tma_full + 8 * s, 1);         // the loader's expect_tx arrival (+ the copies' bytes)
+      // one arrival per producer or converter warp; GRADR: + the expect_tx arrival of the B copy
+      mbar_init(full_bar + 8 * s, GT_PRODUCER_WARPS + (MODE == GT_MODE_GRADR ? 1 : 0));
+      // the loader's expect_tx arrival (+ the copies' bytes); gathered rows: + one when each of its lanes' copies landed
+      mbar_init(tma_full + 8 * s, MODE == GT_MODE_LINEAR && !g.lin_tma ? 1 + 32 * GT_GATHER_WARPS : 1);
       mbar_init(empty_bar + 8 * s, 1);        // one tcgen05.commit
     }
     for (int a = 0; a < 2; a++) {
@@ -348,7 +347,7 @@ __global__ void __launch_bounds__((GT_PRODUCER_WARPS + 1 + EW + 1) * 32, 1)
   const uint32_t lo_ring = tmem_base + (ONE_ACC ? 2u : 4u) * (uint32_t)g.npad;
   const int items = k_blocks;                                     // pipeline items per tile
 
-  if (((MODE == GT_MODE_PLAIN && TS) || (MODE == GT_MODE_LINEAR && TS && g.lin_tma)) && warp < GT_PRODUCER_WARPS) {
+  if (((MODE == GT_MODE_PLAIN && TS) || MODE == GT_MODE_LINEAR) && warp < GT_PRODUCER_WARPS) {
     // ================================ converters, residual image to tensor memory ================================
     // A thread owns one row of the tile (the tensor-memory lane its warp may access) and 16 of the K block's 32
     // columns: four 16-byte shared-memory loads (conflict-free: the 128-byte swizzle puts the same logical chunk of
@@ -391,6 +390,7 @@ __global__ void __launch_bounds__((GT_PRODUCER_WARPS + 1 + EW + 1) * 32, 1)
         tmem_st16(t_lo + 32u * (uint32_t)stage, lo);
         tmem_st_wait();
         tc_fence_before();
+        if (MODE == GT_MODE_LINEAR && !g.lin_tma) fence_proxy_async();   // the raw image came by cp.async: generic proxy
         __syncwarp();
         if (lane == 0) mbar_arrive(full_bar + 8 * stage);
         if (++stage == GT_STAGES) {
@@ -610,117 +610,7 @@ __global__ void __launch_bounds__((GT_PRODUCER_WARPS + 1 + EW + 1) * 32, 1)
       if (lane == 0) mbar_arrive(g_empty + 8 * buf);
     }
     hand_over();
-  } else if (MODE == GT_MODE_LINEAR && warp < GT_PRODUCER_WARPS) {
-    // ================================ producers ================================
-    // Work items are (tile, K block) pairs in the order the MMA warp consumes them.  Loads run
-    // GT_PREFETCH items ahead of the conversion in a register ring, so that enough bytes are in flight
-    // per SM to cover HBM latency (about a microsecond) independently of the shared-memory ring depth.
-    // (LINEAR always runs as the TS variant.)  The residual image goes to tensor memory, which a warp reaches only
-    // for the 32 lanes (= rows) of its quarter: warp (q, hf) loads rows 32 q .. 32 q + 31, the 64-byte half hf of
-    // their 128-byte K-block segments (4 threads a row, rows (lane >> 2) + 8 i), writes the raw values to the
-    // shared-memory image, and then every lane reads ITS row's half back (all of it written by this warp) to form the
-    // residuals.
-    const int chunk = 4 * (warp >> 2) + (lane & 3);      // 16-byte chunk of the 128-byte row segment
-    const int rbase = 32 * (warp & 3) + (lane >> 2);     // rows rbase + row_step * i
-    constexpr int row_step = 8;
-    // head: the next (tile, K block) item whose loads have not been issued yet
-    struct Head {
-      Tile T;
-      int kb;
-      bool valid;
-      int64_t grow[GT_ROWS_PER_THREAD];
-    } head;
-    TileWalker<MODE> tiles(g, tab);
-    auto advance = [&]() {
-      if (++head.kb < k_blocks && head.valid) return;
-      head.kb = 0;
-      head.valid = tiles.next(head.T);
-      if (!head.valid) return;
-#pragma unroll
-      for (int i = 0; i < GT_ROWS_PER_THREAD; i++) head.grow[i] = global_row<MODE>(g, head.T, rbase + row_step * i);
-    };
-    // returns -1 when there is no item left (otherwise the index of the item's B block, which the loader warp copies)
-    auto issue = [&](float4 (&v)[GT_ROWS_PER_THREAD]) -> int64_t {
-      if (!head.valid) return -1;
-      const int k0 = head.kb * GT_KBLOCK + chunk * 4;
-#pragma unroll
-      for (int i = 0; i < GT_ROWS_PER_THREAD; i++) {
-        v[i] = make_float4(0.f, 0.f, 0.f, 0.f);
-        if (head.grow[i] >= 0 && k0 < g.K)
-          v[i] = __ldg(reinterpret_cast<const float4 *>(g.A + head.grow[i] * g.K + k0));
-      }
-      const int64_t bblock = (int64_t)(head.T.mat * g.n_tiles + head.T.ntile) * k_blocks + head.kb;
-      advance();
-      return bblock;
-    };
-    int stage = 0;
-    uint32_t phase = 0;
-    // returns false on a timed-out wait
-    auto commit = [&](const float4 (&v)[GT_ROWS_PER_THREAD]) -> bool {
-      // lane 0 polls the barrier for the warp
-      uint32_t got = 1;
-      if (lane == 0) got = mbar_wait(empty_bar + 8 * stage, phase ^ 1) ? 1u : 0u;
-      got = __shfl_sync(0xffffffffu, got, 0);
-      if (!got) {
-        report(g, 1);
-        return false;
-      }
-      const uint32_t sA = smem_base + stage * GT_STAGE_BYTES;
-      // (the B block of the item is copied by the loader warp into a ring of its own)
-#pragma unroll
-      for (int i = 0; i < GT_ROWS_PER_THREAD; i++) {
-        const uint32_t off = (uint32_t)sw128_offset(rbase + row_step * i, chunk);
-        asm volatile("st.shared.v4.f32 [%0], {%1, %2, %3, %4};" ::"r"(sA + off), "f"(v[i].x), "f"(v[i].y), "f"(v[i].z),
-                     "f"(v[i].w)
-                     : "memory");
-      }
-      __syncwarp();
-      const int q = warp & 3, hf = warp >> 2;
-      uint32_t lo[16];
-#pragma unroll
-      for (int c = 0; c < 4; c++) {
-        float4 a;
-        asm volatile("ld.shared.v4.f32 {%0, %1, %2, %3}, [%4];"
-                     : "=f"(a.x), "=f"(a.y), "=f"(a.z), "=f"(a.w)
-                     : "r"(sA + (uint32_t)sw128_offset(32 * q + lane, 4 * hf + c))
-                     : "memory");
-        lo[4 * c] = __float_as_uint(to_tf32(a.x - __uint_as_float(__float_as_uint(a.x) & 0xFFFFE000u)));
-        lo[4 * c + 1] = __float_as_uint(to_tf32(a.y - __uint_as_float(__float_as_uint(a.y) & 0xFFFFE000u)));
-        lo[4 * c + 2] = __float_as_uint(to_tf32(a.z - __uint_as_float(__float_as_uint(a.z) & 0xFFFFE000u)));
-        lo[4 * c + 3] = __float_as_uint(to_tf32(a.w - __uint_as_float(__float_as_uint(a.w) & 0xFFFFE000u)));
-      }
-      tmem_st16(lo_ring + 32u * (uint32_t)stage + ((uint32_t)(q * 32) << 16) + 16u * (uint32_t)hf, lo);
-      tmem_st_wait();
-      tc_fence_before();
-      fence_proxy_async();
-      __syncwarp();
-      if (lane == 0) mbar_arrive(full_bar + 8 * stage);
-      if (++stage == GT_STAGES) {
-        stage = 0;
-        phase ^= 1;
-      }
-      return true;
-    };
-
-    head.kb = k_blocks;  // forces advance() to step to the first tile
-    head.valid = false;
-    advance();
-    // register ring: GT_PREFETCH items of global loads in flight per thread
-    float4 buf[GT_PREFETCH][GT_ROWS_PER_THREAD];
-    int64_t inflight[GT_PREFETCH];
-#pragma unroll
-    for (int d = 0; d < GT_PREFETCH; d++) inflight[d] = issue(buf[d]);
-    for (bool run = true; run;) {
-#pragma unroll
-      for (int d = 0; d < GT_PREFETCH; d++) {
-        if (inflight[d] < 0 || !commit(buf[d])) {
-          run = false;
-          break;
-        }
-        inflight[d] = issue(buf[d]);
-      }
-    }
-  } else if (warp == GT_PRODUCER_WARPS + 1 + EW) {
+  } else if (warp >= GT_PRODUCER_WARPS + 1 + EW) {
     // ================================ loader ================================
     // PLAIN row map only.  Per pipeline item one thread starts two asynchronous copies that complete on the
     // stage's barrier: the TMA tile load of A (128 rows x 32 columns, 128-byte swizzle, zeros outside the
@@ -786,7 +676,7 @@ __global__ void __launch_bounds__((GT_PRODUCER_WARPS + 1 + EW + 1) * 32, 1)
         have = have_next;
       }
     }
-    if (MODE == GT_MODE_LINEAR && TS && g.lin_tma && elect_one()) {
+    if (MODE == GT_MODE_LINEAR && g.lin_tma && warp == GT_PRODUCER_WARPS + 1 + EW && elect_one()) {
       // Rows by TMA: per item four box loads (one per quarter of the tile: nq whole nodes x 2l+1 components x 32
       // columns land as consecutive 128-byte rows, swizzled, at the quarter's first row) and the B block, all on the
       // slot's tma_full barrier; the converter warps then add the residual image.  Boxes that reach past the last
@@ -820,34 +710,70 @@ __global__ void __launch_bounds__((GT_PRODUCER_WARPS + 1 + EW + 1) * 32, 1)
         }
       }
     }
-    if (MODE == GT_MODE_LINEAR && TS && !g.lin_tma && elect_one()) {
-      // Per item the B block of the tile's (l, element) problem into the ring of B blocks, same slot index and
-      // barriers as the A images: the copy starts as soon as the slot is released, while the producers still
-      // convert the items before it.
+    if (MODE == GT_MODE_LINEAR && !g.lin_tma) {
+      // Gathered rows: GT_GATHER_WARPS warps copy the 128 row segments of 128 bytes of an item into the slot's swizzled
+      // image, four rows an instruction (their 16-byte pieces fill whole bank rows), zeros behind the problem's last row
+      // and behind column K; one lane starts the B block.  The next tile's rows are looked up while this one's are copied.
+      // Before, the eight warps that convert loaded the segments into registers two items ahead (32 KB in flight an SM,
+      // and an exposed look-up a tile).  Forward and backward of 30 000 nodes,
+      // 4 elements: 328 -> 245 us with 128 channels (its bytes 150), 178 -> 141 with 64, 124 -> 115 with 32; 64 000
+      // nodes 690 -> 501, 3 000 51 -> 44.  One warp copying: 465, two 283, eight 243 (128 channels): its instructions
+      // cost about 110 cycles each in one warp.
+      constexpr int ROWS = GT_TILE_M / GT_GATHER_WARPS;   // of a warp
+      const int first = (warp - (GT_PRODUCER_WARPS + 1 + EW)) * ROWS;
       const uint32_t b_ring0 = smem_base + GT_STAGES * GT_STAGE_BYTES + (uint32_t)g.g_stage_bytes;
+      const int piece = lane & 7, sub = lane >> 3;
+      uint32_t dst[2];   // rows first + sub + 4 i: the swizzle repeats every eight rows
+      dst[0] = (uint32_t)sw128_offset(first + sub, piece);
+      dst[1] = (uint32_t)sw128_offset(first + sub + 4, piece);
       int slot = 0;
       uint32_t bphase = 0;
       bool ok = true;
       TileWalker<MODE> tiles(g, tab);
-      Tile T;
-      while (ok && tiles.next(T)) {
+      Tile T, Tn;
+      bool have = tiles.next(T);
+      int64_t next_row = have ? global_row<MODE>(g, T, first + (lane & (ROWS - 1))) : -1;
+      while (ok && have) {
         const unsigned char *bsrc = reinterpret_cast<const unsigned char *>(g.packed) +
                                     ((int64_t)(T.mat * g.n_tiles + T.ntile) * k_blocks) * (2 * (int64_t)b_image);
+        const float *src[ROWS / 4];   // null: a row of zeros
+#pragma unroll
+        for (int i = 0; i < ROWS / 4; i++) {
+          const int64_t row = __shfl_sync(0xffffffffu, next_row, 4 * i + sub);
+          src[i] = row >= 0 ? g.A + row * g.K + 4 * piece : nullptr;
+        }
+        have = tiles.next(Tn);   // its rows are looked up while this tile's are copied
+        if (have) next_row = global_row<MODE>(g, Tn, first + (lane & (ROWS - 1)));
         for (int kb = 0; kb < items; kb++) {
-          if (!mbar_wait(empty_bar + 8 * slot, bphase ^ 1)) {
+          uint32_t got = 1;
+          if (lane == 0) got = mbar_wait(empty_bar + 8 * slot, bphase ^ 1) ? 1u : 0u;
+          if (!__shfl_sync(0xffffffffu, got, 0)) {
             report(g, 9);
             ok = false;
             break;
           }
-          mbar_arrive_expect_tx(full_bar + 8 * slot, 2 * b_image);
-          bulk_copy_g2s(b_ring0 + (uint32_t)slot * 2u * b_image, bsrc + (int64_t)kb * (2 * (int64_t)b_image), 2 * b_image,
-                        full_bar + 8 * slot);
+          const uint32_t sA = smem_base + slot * GT_STAGE_BYTES, bar = tma_full + 8 * slot;
+          if (first == 0 && lane == 0) {
+            mbar_arrive_expect_tx(bar, 2 * b_image);
+            bulk_copy_g2s(b_ring0 + (uint32_t)slot * 2u * b_image, bsrc + (int64_t)kb * (2 * (int64_t)b_image), 2 * b_image, bar);
+          }
+          const bool in_k = kb * GT_KBLOCK + 4 * piece < g.K;
+#pragma unroll
+          for (int i = 0; i < ROWS / 4; i++) {
+            const bool in = in_k && src[i] != nullptr;
+            asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(sA + dst[i & 1] + 1024u * (uint32_t)(i >> 1)),
+                         "l"(in ? src[i] + kb * GT_KBLOCK : g.A), "r"(in ? 16 : 0)
+                         : "memory");
+          }
+          asm volatile("cp.async.mbarrier.arrive.noinc.shared::cta.b64 [%0];" ::"r"(bar) : "memory");
           if (++slot == GT_STAGES) {
             slot = 0;
             bphase ^= 1;
           }
         }
+        T = Tn;
       }
+      asm volatile("cp.async.wait_all;" ::: "memory");   // also where a wait gave up: no copy outlives the block
     }
     if (MODE == GT_MODE_PLAIN && elect_one()) {
       int stage = 0;
@@ -1517,7 +1443,9 @@ static int gemm_launch(GemmArgs &g, const char *what, cudaStream_t st) {
     g.total_tiles = ((row_tiles + per_col - 1) / per_col) * blocks;
   }
   if (blocks < 1) return CMACE_OK;
-  const int nthreads = g.mode == GT_MODE_GRADR ? (GT_PRODUCER_WARPS + 1 + 4 + 1) * 32 : GT_THREADS;
+  const int nthreads = g.mode == GT_MODE_GRADR    ? (GT_PRODUCER_WARPS + 1 + 4 + 1) * 32
+                       : g.mode == GT_MODE_LINEAR ? GT_THREADS + 32 * (GT_GATHER_WARPS - 1)
+                                                  : GT_THREADS;
   launch_chained(kern, (unsigned)blocks, nthreads, smem, st, g, tmap, tmap_out, lin_maps);
   return check_launch(what);
 }

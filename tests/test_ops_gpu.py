@@ -143,6 +143,31 @@ def test_elemental_linear(dtype, N, Z, K, dev):
     assert torch.equal(out2, out.detach())
 
 
+# one row; a tile's edge and one row past it; K of part of a block (8), of a block and a quarter (40), of three blocks;
+# several tiles a block of threads (2 x 16 x 9 001 rows are 2 251 tiles of 128 on 148), one element with most nodes
+@pytest.mark.parametrize("N,Z,K,Nout", [(2, 2, 8, 4), (128, 2, 40, 32), (129, 3, 96, 128), (257, 128, 32, 20), (9001, 5, 72, 64),
+                                        (9001, 2, 128, 128)])
+def test_elemental_linear_of_gathered_rows(N, Z, K, Nout, dev):
+    from cuda_mace_b200 import ops
+
+    g = torch.Generator().manual_seed(N + K)
+    X = torch.randn(N, 16, K, generator=g).to(dev)
+    W = torch.randn(Z, 4, K, Nout, generator=g).to(dev)
+    at = torch.randint(0, Z, (N,), generator=g)
+    at[::2] = 0
+    at[:2] = torch.tensor([Z - 1, 0])   # never stored in order
+    out = ops.elemental_linear_forward(X, W, W.transpose(-1, -2).contiguous(), at.to(torch.int32).to(dev))
+    ref, size = torch.empty(N, 16, Nout, dtype=torch.float64, device=dev), torch.empty(N, 16, Nout, device=dev, dtype=torch.float64)
+    for z in range(Z):
+        rows = (at == z).to(dev)
+        for l in range(4):
+            x, w = X[rows, l * l:(l + 1) ** 2].double(), W[z, l].double()
+            ref[rows, l * l:(l + 1) ** 2] = x @ w / K ** 0.5
+            size[rows, l * l:(l + 1) ** 2] = x.abs() @ w.abs() / K ** 0.5
+    # a product of the split operands is off by 2^-20 of itself; K sums in float32, three terms each
+    assert ((out.double() - ref).abs() <= (2 ** -19 + 3 * K * 2 ** -24) * size).all()
+
+
 @pytest.mark.parametrize("dtype", DTYPES)
 @pytest.mark.parametrize("N,Z,K", [(1000, 4, 128), (37, 10, 64), (333, 3, 32), (4, 2, 128)])
 def test_elemental_linear_on_nodes_stored_grouped_by_element(dtype, N, Z, K, dev):
