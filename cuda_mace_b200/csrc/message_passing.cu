@@ -841,8 +841,24 @@ __global__ void sum_partials_kernel(const T *__restrict__ partial, int nchunks, 
   out[i] = s;
 }
 
+// Gathers rows of T by the sender's list: bound by the latency of a row and the warps there are to wait.  What the compiler keeps in
+// flight follows the registers that it believes it has, so every width says for how many blocks an SM it is compiled (0: nothing said).
+// SPLIT warps a sender (few senders), five blocks, three doubles a lane four (48 registers would spill); with nothing said 29 -> 25 us
+// at 3 000 atoms of 128 channels in float32, 68 -> 58 at 8 000, 47 -> 37 in float64 at 3 000, 25 -> 21 with 96 channels.  (Six blocks:
+// 29 and 64; eight rows at a time instead of four: 31 and 68; two rows, eight blocks: 25 and 54, but 23 with 96 channels.)
+// One warp a sender, float32, at 16 000 atoms: 32 channels ten blocks 52 -> 44 (one 60, sixteen 64), 64 channels eight 70 -> 58 (one
+// 60, ten 60, twelve 80; 209 -> 183 at 64 000), 128 channels one 95 -> 88 (eight 91, ten 117; 330 -> 301 at 64 000), 96 channels
+// nothing said and the list's lines prefetched 81 (109 without the prefetch, which is no help to the others; one, six to nine 88, twelve
+// 130); float64 with 96 channels one 84 -> 76 at 8 000.
 template <typename T, int VEC, int SPLIT>
-__global__ void __launch_bounds__(SPLIT == 1 ? kWarpsPerBlock * 32 : SPLIT * 32)
+constexpr int node_blocks_an_sm() {
+  if (SPLIT > 1) return sizeof(T) * VEC <= 16 ? 5 : 4;
+  if (sizeof(T) == 8) return 1;
+  return VEC == 1 ? 10 : VEC == 2 ? 8 : VEC == 3 ? 0 : 1;
+}
+
+template <typename T, int VEC, int SPLIT>
+__global__ void __launch_bounds__(SPLIT == 1 ? kWarpsPerBlock * 32 : SPLIT * 32, node_blocks_an_sm<T, VEC, SPLIT>())
     imp_bwd_node_kernel(const T *__restrict__ Tin, const int32_t *__restrict__ perm,
                         const int32_t *__restrict__ send_ptr, int64_t nnodes, int C,
                         T *__restrict__ gradX) {
@@ -854,7 +870,7 @@ __global__ void __launch_bounds__(SPLIT == 1 ? kWarpsPerBlock * 32 : SPLIT * 32)
   }
   const int chunk = blockIdx.y * (32 * VEC);
   const int64_t k0 = send_ptr[node] + (SPLIT > 1 ? warp : 0), k1 = send_ptr[node + 1];
-  if (k0 + 32 * lane < k1) asm volatile("prefetch.global.L1 [%0];" ::"l"(perm + k0 + 32 * lane));
+  if (VEC == 3 && k0 + 32 * lane < k1) asm volatile("prefetch.global.L1 [%0];" ::"l"(perm + k0 + 32 * lane));
   grid_begin();
   // 32 edges' indices in one load, then four rows in flight at a time
   constexpr int AHEAD = 4;
@@ -883,15 +899,15 @@ __global__ void __launch_bounds__(SPLIT == 1 ? kWarpsPerBlock * 32 : SPLIT * 32)
 #pragma unroll
   for (int v = 0; v < VEC; v++) acc[0][v] += acc[1][v];
   if constexpr (SPLIT > 1) {
-    __shared__ T part[SPLIT][32 * VEC];
+    __shared__ __align__(16) T part[SPLIT][32 * VEC];
 #pragma unroll
-    for (int v = 0; v < VEC; v++) part[warp][v * 32 + lane] = acc[0][v];
+    for (int v = 0; v < VEC; v++) part[warp][lane * VEC + v] = acc[0][v];
     __syncthreads();
     if (warp > 0) return;
 #pragma unroll
     for (int w = 1; w < SPLIT; w++)
 #pragma unroll
-      for (int v = 0; v < VEC; v++) acc[0][v] += part[w][v * 32 + lane];
+      for (int v = 0; v < VEC; v++) acc[0][v] += part[w][lane * VEC + v];
   }
   store_lane<T, VEC>(gradX + node * C + chunk, lane, acc[0], false);
 }
