@@ -136,28 +136,30 @@ class ClockSampler:
 
 
 def algorithmic_bytes(name, s, N, Ns, E, C, Z):
-    """Bytes each step of the native sequence has to move when every tensor is read or written once (indices 4 B); the
-    float32 step at 128 channels forms the second layer's radial weights on chip, the others write them."""
+    """Bytes each step of the native sequence has to move (indices 4 B).  The two edges of a pair share a row of everything
+    that depends on the distance alone: it is written once and read by each of them.  The float32 step forms the second
+    layer's radial weights on chip, the float64 step writes them and their derivative."""
     if not name.startswith("step["):
         return {"cmace_receiver_csr": 4 * E + 4 * N, "cmace_nl_emit_f64": 35 * E + 48 * N}.get(name)
     row = 64 * s                              # one edge's hidden row (float32: an fp16 pair)
     m16, sums = 16 * N * C * s, 16 * N * 64 * Z * s
-    fused = s == 4 and C == 128
+    fused = s == 4
     R = 4 * C * s
+    P = E // 2                                # pairs of edges
     return {
         "edge_prep": 24 * Ns + E * (24 + 8 + 4 * s + 16 * s + 16 * s),
-        "radial": E * (16 * s + 4 * row),
+        "radial": P * (16 * s + 4 * row),
         "sums": E * (row + 16 * s + 4) + sums,
         "fold": sums + m16,
         "contract0": m16 + N * C * s,
         "mid_fwd": 2 * N * C * s,
-        "radial_out": 0 if fused else E * (row + R),
+        "radial_out": 0 if fused else P * (2 * row + 2 * R),
         "messages": E * ((row if fused else R) + 16 * s + 8) + Ns * C * s + m16,
         "linear": 2 * m16,
         "contract1": 2 * m16,
         "linear_back": 2 * m16,
         "edges_back": E * ((2 * row if fused else 2 * R) + 32 * s + C * s + 8) + Ns * C * s + m16,
-        "radial_back": 0 if fused else E * (R + row + s),
+        "radial_back": 0,                     # part of edges_back
         "senders": E * (C * s + 4) + Ns * C * s,
         "mid_back": 2 * N * C * s,
         "contract0_back": 2 * m16,
@@ -172,24 +174,24 @@ def algorithmic_bytes(name, s, N, Ns, E, C, Z):
 # moves this many bytes times its own E.
 _SRC = "profiles/step_sequence_8000_f32.txt"
 NCU_TRAFFIC_PER_EDGE = {
-    "step[edges_back]": (1240.0, _SRC),
-    "step[messages]": (434.0, _SRC),
-    "step[radial]": (943.0, _SRC),
-    "step[sums_back]": (996.0, _SRC),
+    "step[edges_back]": (1159.0, _SRC),
+    "step[messages]": (331.0, _SRC),
+    "step[radial]": (409.0, _SRC),
+    "step[sums_back]": (871.0, _SRC),
 }
 # warps a scheduler and issue slots used while active, from the same capture
 ISSUE_NOTE = {step: f", on {warps} warps a scheduler (issue slots {slots} % used in the ncu capture {_SRC})"
-              for step, warps, slots in (("step[edges_back]", 4, 59), ("step[messages]", 3, 43), ("step[radial]", 4, 51))}
+              for step, warps, slots in (("step[edges_back]", 4, 60), ("step[messages]", 3, 42), ("step[radial]", 4, 47))}
 
 
 def tensor_flops(name, s, E, C):
     """Tensor-core flops one launch executes, for the steps whose binding roof is the tensor pipe: float32 runs three
     fp16 terms of the product with the last radial layer ([E,64] x [64,4C]; the backward forms it for the derivative as
-    well) and of the hidden layers for values and derivatives of both perceptrons."""
+    well) and of the hidden layers for values and derivatives of both perceptrons, a row a pair of edges."""
     if s != 4 or C != 128:
         return None
     return {"step[messages]": 3 * 2 * E * 4 * C * 64, "step[edges_back]": 2 * 3 * 2 * E * 4 * C * 64,
-            "step[radial]": 2 * 2 * 3 * 2 * E * (16 * 64 + 2 * 64 * 64)}.get(name)
+            "step[radial]": 2 * 2 * 3 * 2 * (E // 2) * (16 * 64 + 2 * 64 * 64)}.get(name)
 
 
 def half_peak():
