@@ -393,33 +393,34 @@ __global__ void __launch_bounds__(256)
   }
 }
 
-// 8 nodes a tile while that leaves SMs idle, else 32 (four times the reuse of a weight); two blocks an SM in float32
-template <typename T, typename Kernel8, typename Kernel32, typename... Args>
-static int launch_mid(const char *what, int64_t n, int C, int threads, Kernel8 k8, Kernel32 k32, cudaStream_t st, Args... args) {
+// 8 nodes a tile while that leaves SMs idle, 16 while every block has one tile, else 32 (four times the reuse of a weight); two blocks
+// an SM in float32.  16 against 32, us forward and back, 128 channels: 1 500 nodes 14.6 + 12.7 against 16.8 + 14.8 (float64 25.6 + 23.0
+// against 29.1 + 25.0), 3 000 16.4 + 14.8 against 16.9 + 14.8 (float64, two tiles a block, 33.2 + 31.2 against 29.1 + 25.0), 6 000
+// 21.0 + 18.9 against 18.9 + 17.9; 32 channels, 3 000: 9.2 + 8.7 against 10.6 + 10.6.
+template <typename T, typename Kernel, typename... Args>
+static int launch_mid(const char *what, int64_t n, int C, int threads, Kernel k8, Kernel k16, Kernel k32, cudaStream_t st, Args... args) {
   if (n == 0) return CMACE_OK;
-  const bool small = n <= 8 * 148;
-  const int nodes = small ? 8 : 32;
+  const int64_t cap = 148 * (sizeof(T) == 4 ? 2 : 1);
+  const int nodes = n <= 8 * 148 ? 8 : (n <= 16 * cap ? 16 : 32);
+  const Kernel kernel = nodes == 8 ? k8 : (nodes == 16 ? k16 : k32);
   const size_t smem = sizeof(T) * ((size_t)C * (C + MID_PAD) + 2 * (size_t)nodes * (C + MID_PAD));   // forward: C + 4 a row
   int64_t blocks = (n + nodes - 1) / nodes;
-  const int64_t cap = 148 * (sizeof(T) == 4 ? 2 : 1);
   if (blocks > cap) blocks = cap;
-  cudaError_t e = small ? cudaFuncSetAttribute(k8, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem)
-                        : cudaFuncSetAttribute(k32, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+  cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
   if (e != cudaSuccess) return fail(CMACE_ERR_CUDA, "%s: %s", what, cudaGetErrorString(e));
-  if (small) launch_chained(k8, (unsigned)blocks, threads, smem, st, args...);
-  else launch_chained(k32, (unsigned)blocks, threads, smem, st, args...);
+  launch_chained(kernel, (unsigned)blocks, threads, smem, st, args...);
   return check_launch(what);
 }
 template <typename T>
 int StepKernels<T>::mid_fwd(const T *b, const int32_t *node_of, const int32_t *slot_type, const T *wu, const T *extra,
                             int64_t n, int C, T *up, T *q0, cudaStream_t st) {
-  return launch_mid<T>("cmace_step(mid_fwd)", n, C, 2 * C + 64, mid_fwd_kernel<T, 8>, mid_fwd_kernel<T, 32>, st, b, node_of, slot_type,
+  return launch_mid<T>("cmace_step(mid_fwd)", n, C, 2 * C + 64, mid_fwd_kernel<T, 8>, mid_fwd_kernel<T, 16>, mid_fwd_kernel<T, 32>, st, b, node_of, slot_type,
                        wu, extra, n, C, up, q0);
 }
 template <typename T>
 int StepKernels<T>::mid_bwd(const T *gup, const int32_t *node_of, const int32_t *slot_type, const T *dq, const T *wu_t,
                             const T *extra_t, double scale, int64_t n, int C, T *gb, cudaStream_t st) {
-  return launch_mid<T>("cmace_step(mid_bwd)", n, C, 2 * C, mid_bwd_kernel<T, 8>, mid_bwd_kernel<T, 32>, st, gup, node_of, slot_type,
+  return launch_mid<T>("cmace_step(mid_bwd)", n, C, 2 * C, mid_bwd_kernel<T, 8>, mid_bwd_kernel<T, 16>, mid_bwd_kernel<T, 32>, st, gup, node_of, slot_type,
                        dq, wu_t, extra_t, (T)scale, n, C, gb);
 }
 

@@ -72,6 +72,28 @@ def test_step_against_autograd(U, dtype, tol, n, C, Z, nb, radial):
     assert float((out["forces"] + g).abs().max()) < tol * float(g.abs().max())
 
 
+# tiles of 8 nodes up to 1 184 atoms, of 16 up to 2 368 in float64 and 4 736 in float32, of 32 beyond; one node past a tile and a
+# tile but one; every element's part of the matrices in turn within a tile.  Against the model's own autograd path, same bounds
+@pytest.mark.parametrize("dtype,tol,n", [(torch.float64, 1e-10, 1184), (torch.float64, 1e-10, 1185), (torch.float64, 1e-10, 2367),
+                                         (torch.float64, 1e-10, 2369), (torch.float32, 1e-4, 1185), (torch.float32, 1e-4, 4735),
+                                         (torch.float32, 1e-4, 4737)])
+def test_nodes_between_the_layers_at_tile_edges(U, dtype, tol, n):
+    C, Z = 64, 9
+    receiver, sender = torch.arange(n).repeat_interleave(2), torch.stack([torch.arange(n).roll(1), torch.arange(n).roll(-1)], 1).reshape(-1)
+    pos = torch.stack([1.3 * torch.arange(n), torch.arange(n) % 3, torch.arange(n) % 2], 1).double()   # a crooked closed chain
+    shifts = torch.zeros(2 * n, 3, dtype=torch.float64)
+    shifts[0, 0], shifts[-1, 0] = -1.3 * n, 1.3 * n
+    species = torch.randint(0, Z, (n,), generator=torch.Generator().manual_seed(n), dtype=torch.int32).cuda()
+    mace = model.InvariantMACE(systems.init_params(C, Z, 7), U, dtype=dtype, device="cuda")
+    plan = step.plan_of(mace)
+    assert plan is not None
+    p, edges, shifts = pos.cuda(), torch.stack([receiver, sender]).to(torch.int32).cuda(), shifts.cuda()
+    _, _, _, forces = step.energy_forces(plan, p, species, None, shifts, ops.EdgeTopology(edges[1], edges[0], n))
+    p.requires_grad_(True)
+    (g,) = torch.autograd.grad(mace.node_energies(p, species, edges, shifts).sum(), p)
+    assert float((forces + g).abs().max()) < tol * float(g.abs().max())
+
+
 def _list_of(receiver, n, seed, channels=128):
     """A model's weights and a list with these receivers; a shift an edge gives any distance up to the cutoff."""
     rng = np.random.default_rng(seed)
