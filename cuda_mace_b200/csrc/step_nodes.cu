@@ -31,6 +31,17 @@ __device__ __forceinline__ void prefetch_weff(const T *__restrict__ weff, int z,
   if (lane < ST_NW) asm volatile("prefetch.global.L1 [%0];" ::"l"(weff + ((int64_t)z * ST_NW + lane) * C + (c & ~31)));
 }
 
+// A block's next node on its way to L1, the lines of the warp's channels: the loads at the head of a node stall every warp of a block that
+// has little else resident.  us at 64 000 and 16 000 atoms of 128 channels: contract0 137 -> 130 and 37 -> 35, contract1 357 -> 349 and
+// 87 -> 84, contract0_back 261 -> 229 and 64 -> 58.  (The next node's element kept in a register as well: 146, 349, 251.)
+template <typename T>
+__device__ __forceinline__ void prefetch_node(const T *__restrict__ X, int64_t node, int64_t nnodes, int C, int c) {
+  constexpr int LINES = (int)sizeof(T) / 4;   // of 128 bytes, of a row of 32 channels
+  const int lane = threadIdx.x & 31;
+  if (node < nnodes && lane < 16 * LINES)
+    asm volatile("prefetch.global.L1 [%0];" ::"l"(X + (node * 16 + lane / LINES) * C + (c & ~31) + lane % LINES * 16));
+}
+
 // The value alone needs a third of the gradient's work (canon::value) and half its registers: forward 95 -> 58 us at 32 000 nodes of
 // 128 channels (278 MB: 43 us), 52 -> 35 at 16 000 in a step, 45 -> 29 in float64 at 8 000.  The backward is bound by its
 // arithmetic (about 500 instructions a node and channel: 57 us of its 140 by issue alone).
@@ -49,6 +60,7 @@ __global__ void __launch_bounds__(128, BWD ? (sizeof(T) == 4 ? 5 : 3) : (sizeof(
 #pragma unroll
     for (int i = 0; i < 16; i++) x[i] = __ldcs(xr + i * C);
     load_weff(weff, types[node], C, c, w3, w2, w1);
+    prefetch_node(X, node + gridDim.x, nnodes, C, c);
     if constexpr (BWD) {
       T g[16], value;
       const T go = gb[node * C + c];
@@ -119,6 +131,7 @@ __global__ void __launch_bounds__(128, sizeof(T) == 4 ? 5 : 3)
     for (int i = 0; i < 16; i++) x[i] = __ldcs(xr + i * C);
     const int z = types[node];
     load_weff(weff, z, C, c, w3, w2, w1);
+    prefetch_node(X, node + gridDim.x, nnodes, C, c);
     double qd = 0.0, e0 = 0.0;
     if (c < ST_RO) qd = (double)q0[node * (ST_RO + 1) + c];
     if (c == 0) e0 = (double)q0[node * (ST_RO + 1) + ST_RO];
