@@ -44,7 +44,7 @@ __device__ __forceinline__ void prefetch_node(const T *__restrict__ X, int64_t n
 
 // The value alone needs a third of the gradient's work (canon::value) and half its registers: forward 95 -> 58 us at 32 000 nodes of
 // 128 channels (278 MB: 43 us), 52 -> 35 at 16 000 in a step, 45 -> 29 in float64 at 8 000.  The backward is bound by its
-// arithmetic (about 500 instructions a node and channel: 57 us of its 140 by issue alone).
+// arithmetic (about 500 instructions a node and channel: 114 us of its 229 at 64 000 nodes by issue alone).
 //
 // early: whether types and weights are older than the kernel before (not where that kernel has laid the weights out)
 template <typename T, bool BWD>
