@@ -122,14 +122,17 @@ __device__ __forceinline__ void grid_begin() {
 }
 // It is off unless the caller has switched it on for this thread: blocks that arrive early keep the SM's split between
 // shared memory and L1 as the predecessor had it, which costs kernels that live on L1 more than 2 us once they are long.
-inline bool &chain_launches() {
-  static thread_local bool on = false;
-  return on;
+// from_second: on, but the next kernel waits for all that is before it in the stream (what its beginning reads may be the work of
+// a kernel right before it that is none of the chain's), the ones after it are chained to it.
+enum class Chain { off, from_second, on };
+inline Chain &chain_launches() {
+  static thread_local Chain chain = Chain::off;
+  return chain;
 }
 // on for a scope: the layout of the contraction's weights and the program that reads it
 struct ChainScope {
-  const bool before = chain_launches();
-  ChainScope() { chain_launches() = true; }
+  const Chain before = chain_launches();
+  ChainScope() { chain_launches() = Chain::on; }
   ~ChainScope() { chain_launches() = before; }
 };
 template <typename... Params, typename... Args>
@@ -143,7 +146,8 @@ inline void launch_chained(void (*kernel)(Params...), dim3 grid, dim3 block, siz
   cfg.dynamicSmemBytes = smem;
   cfg.stream = st;
   cfg.attrs = &attr;
-  cfg.numAttrs = chain_launches() ? 1 : 0;
+  cfg.numAttrs = chain_launches() == Chain::on ? 1 : 0;
+  if (chain_launches() == Chain::from_second) chain_launches() = Chain::on;
   cudaLaunchKernelEx(&cfg, kernel, Params(args)...);
 }
 

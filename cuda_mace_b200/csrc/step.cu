@@ -350,12 +350,12 @@ static int run_steps(const cmace_step_model &m, cmace_step_io &io, int first, in
   const Workspace<T> w(io.workspace, m, io.n_owned, io.n_local, io.nedges);
   if (io.workspace_bytes < w.bytes)
     return fail(CMACE_ERR_ARG, "cmace_step: workspace of %lld bytes, %lld needed", (long long)io.workspace_bytes, (long long)w.bytes);
-  // The first kernel of a range as well: the attribute relaxes the order after the kernel before it and nothing else, so a
-  // wait for another stream or a copy that the caller has put between still comes first.
-  chain_launches() = chain_for(m, io.nedges, st);
+  // The first kernel of a range beyond step 0 is not chained: its beginning may read the list or an exchanged row before its
+  // wait, and the caller may have put the kernel that makes them right before this call.  Step 0 begins with its wait.
+  chain_launches() = !chain_for(m, io.nedges, st) ? Chain::off : first > 0 ? Chain::from_second : Chain::on;
   int rc = CMACE_OK;
   for (int s = first; s < last && rc == CMACE_OK; s++) rc = run_step<T>(m, io, w, s, st);
-  chain_launches() = false;
+  chain_launches() = Chain::off;
   return rc;
 }
 

@@ -686,7 +686,7 @@ int step_sums_half(const void *h, const float *Y, const int32_t *sender, const i
   const int per = elements_per_warp(nnodes, elements);
   const int64_t blocks = (nnodes * ((elements + per - 1) / per) + SU_WARPS - 1) / SU_WARPS;
   if (blocks > 0)
-    launch_chained(chain_launches() ? sums_f16_kernel<true> : sums_f16_kernel<false>, (unsigned)blocks, SU_WARPS * 32, 0, st, static_cast<const uint4 *>(h), Y, sender, row_ptr, species,
+    launch_chained(chain_launches() == Chain::on ? sums_f16_kernel<true> : sums_f16_kernel<false>, (unsigned)blocks, SU_WARPS * 32, 0, st, static_cast<const uint4 *>(h), Y, sender, row_ptr, species,
                                                                slot_of, row_of, nnodes, elements, per, out_v / SU_Y_SCALE, A);
   return check_launch("cmace_step(sums)");
 }
@@ -773,7 +773,7 @@ int StepKernels<T>::sums(const T *h, const T *Y, const int32_t *sender, const in
     if constexpr (sizeof(T) == 4)
       launch_chained(sums_tf32_kernel, (unsigned)blocks, SU_WARPS * 32, 0, st, h, Y, sender, row_ptr, species, slot_of, nnodes, elements, A);
     else
-      launch_chained(chain_launches() ? sums_f64_kernel<true> : sums_f64_kernel<false>, (unsigned)blocks, SU_WARPS * 32, 0, st, h, Y, sender, row_ptr, species, slot_of,
+      launch_chained(chain_launches() == Chain::on ? sums_f64_kernel<true> : sums_f64_kernel<false>, (unsigned)blocks, SU_WARPS * 32, 0, st, h, Y, sender, row_ptr, species, slot_of,
                      row_of, nnodes, elements, A);
   }
   return check_launch("cmace_step(sums)");
@@ -1073,7 +1073,7 @@ int step_sums_bwd_half(const float *gA, const void *h, const void *dh, const flo
   const int per = elements_per_warp(nnodes, elements);
   const int64_t blocks = (nnodes * ((elements + per - 1) / per) + SU_WARPS - 1) / SU_WARPS;
   if (blocks > 0)
-    launch_chained(chain_launches() ? sums_bwd_f16_kernel<true> : sums_bwd_f16_kernel<false>, (unsigned)blocks, SU_WARPS * 32, 0, st, 
+    launch_chained(chain_launches() == Chain::on ? sums_bwd_f16_kernel<true> : sums_bwd_f16_kernel<false>, (unsigned)blocks, SU_WARPS * 32, 0, st, 
         gA, static_cast<const uint4 *>(h), static_cast<const uint4 *>(dh), Y, sender, row_ptr, species, slot_of, row_of, gY1, dr1,
         geo, nnodes, elements, per, out_v, out_t, gvec);
   return check_launch("cmace_step(sums_back)");
@@ -1186,7 +1186,7 @@ int StepKernels<T>::sums_bwd(const T *gA, const T *h, const T *dh, const T *Y, c
       launch_chained(sums_bwd_tf32_kernel, (unsigned)blocks, SU_WARPS * 32, 0, st, gA, h, dh, Y, sender, row_ptr, species, slot_of,
                                                                       gY1, dr1, geo, nnodes, elements, gvec);
     else
-      launch_chained(chain_launches() ? sums_bwd_f64_kernel<true> : sums_bwd_f64_kernel<false>, (unsigned)blocks, SU_WARPS * 32, 0, st, gA, h, dh, Y, sender, row_ptr, species, slot_of,
+      launch_chained(chain_launches() == Chain::on ? sums_bwd_f64_kernel<true> : sums_bwd_f64_kernel<false>, (unsigned)blocks, SU_WARPS * 32, 0, st, gA, h, dh, Y, sender, row_ptr, species, slot_of,
                      row_of, gY1, shares, geo, nnodes, nedges, elements, gvec);
   }
   return check_launch("cmace_step(sums_bwd)");

@@ -1,9 +1,11 @@
 """The whole-step sequence (cmace_step_run) against the float64 oracle at the sizes where its kernels can go wrong."""
+import ctypes
+
 import numpy as np
 import pytest
 import torch
 
-from cuda_mace_b200 import domain, evaluator, model, ops, step, systems
+from cuda_mace_b200 import _abi, domain, evaluator, model, ops, step, systems
 from oracle import model as omodel
 
 pytestmark = pytest.mark.gpu
@@ -568,6 +570,51 @@ def test_a_late_grouping_is_waited_for(U, monkeypatch):
     for _ in range(5):
         ev.set_neighbor_list(ev.species, ev.edge_index, ev.shifts)
         assert torch.equal(ev(p)[1], want)
+
+
+def _programmatic_edges(graph):
+    """(number of nodes, number of edges, of those programmatic) of a recorded graph"""
+    class Data(ctypes.Structure):   # cudaGraphEdgeData; type 1 is programmatic
+        _fields_ = [("from_port", ctypes.c_uint8), ("to_port", ctypes.c_uint8), ("type", ctypes.c_uint8),
+                    ("reserved", ctypes.c_uint8 * 5)]
+
+    cudart, raw = ctypes.CDLL("libcudart.so.12"), ctypes.c_void_p(graph.raw_cuda_graph())
+    nodes, count = ctypes.c_size_t(), ctypes.c_size_t()
+    assert cudart.cudaGraphGetNodes(raw, None, ctypes.byref(nodes)) == 0
+    assert cudart.cudaGraphGetEdges_v2(raw, None, None, None, ctypes.byref(count)) == 0
+    ends, data = (ctypes.c_void_p * (2 * count.value))(), (Data * count.value)()
+    assert cudart.cudaGraphGetEdges_v2(raw, ctypes.byref(ends), ctypes.byref(ends, count.value * ctypes.sizeof(ctypes.c_void_p)), data,
+                                       ctypes.byref(count)) == 0
+    return nodes.value, count.value, sum(d.type == 1 for d in data)
+
+
+# A caller that runs a range of steps, a kernel of its own and the other steps: the second range's first kernel, whatever step
+# launches it, comes after that kernel, the others are chained.  12: one that float32 steps leave out (radial_back)
+@pytest.mark.parametrize("split", [1, 2, 3, 5, 6, 7, 12, 13, 14, 16, 18])
+@pytest.mark.parametrize("dtype,C", [(torch.float32, 64), (torch.float64, 128)])
+def test_a_range_begins_after_what_its_caller_put_before_it(U, dtype, C, split, monkeypatch):
+    mace, data = _small(U, dtype, n=70, C=C)
+    want = mace(data)["forces"].clone()
+    run, counter, ranges = _abi.run_steps, torch.zeros(1, device="cuda"), []
+
+    def in_two(m, io, first, last, stream):
+        for a, b in ((first, split), (split, last)):
+            before = io.launches
+            run(m, io, a, b, stream)
+            ranges.append(io.launches - before)
+            if b == split:
+                counter.add_(1)
+
+    monkeypatch.setattr(_abi, "run_steps", in_two)
+    side, graph = torch.cuda.Stream(), torch.cuda.CUDAGraph(keep_graph=True)
+    side.wait_stream(torch.cuda.current_stream())
+    with torch.cuda.graph(graph, stream=side):
+        out = mace(data)
+    nodes, edges, chained = _programmatic_edges(graph)
+    assert nodes == sum(ranges) + 1 and edges == nodes - 1 and min(ranges) > 0
+    assert chained == sum(ranges) - 2
+    graph.replay()
+    assert torch.equal(out["forces"], want)
 
 
 def test_results_do_not_share_memory(U):
