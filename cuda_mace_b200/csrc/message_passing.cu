@@ -1071,16 +1071,16 @@ int imp_bwd_edge(const T *X, const T *Y, const T *R, const T *G, const int32_t *
     return fail(CMACE_ERR_ARG, "cmace_imp_bwd_edge: null pointer");
   if ((gradR && !aligned16(gradR)) || (Tout && !aligned16(Tout)))
     return fail(CMACE_ERR_ARG, "cmace_imp_bwd_edge: outputs must be 16-byte aligned");
+  cudaStream_t st = (cudaStream_t)stream;
+  if (takes_slots<T>(C)) {   // a whole row at a time: no partials
+    bwd_edge_slots<T, false>(X, Y, R, nullptr, nullptr, G, sender, row_ptr, nnodes, ys, C, gradR, gradY, Tout, st);
+    return check_launch("cmace_imp_bwd_edge");
+  }
   const int vec = pick_vec<T>(C);
   const int nchunks = C / (32 * vec);
   if (nchunks > 1 && !partial)
     return fail(CMACE_ERR_ARG, "cmace_imp_bwd_edge: gradY_partial scratch required for %d chunks", nchunks);
   T *gy = nchunks > 1 ? partial : gradY;
-  cudaStream_t st = (cudaStream_t)stream;
-  if (takes_slots<T>(C)) {
-    bwd_edge_slots<T, false>(X, Y, R, nullptr, nullptr, G, sender, row_ptr, nnodes, ys, C, gradR, gradY, Tout, st);
-    return check_launch("cmace_imp_bwd_edge");
-  }
   if constexpr (sizeof(T) == 4) {
     if (C == BS_C && aligned16(R) && aligned16(X) && aligned16(G)) {
       static int num_sms = 0;
@@ -1262,9 +1262,9 @@ int cmace_imp_bwd_edge_f64_noalloc(const double *X, const double *Y, const doubl
                 "(reduce the number of edges per call or use cmace_imp_bwd_edge_f64 with your own scratch)",
                 (long long)need, (long long)kStaticScratchElems);
   int err = 0;
-  double *scratch = need > 0 ? static_scratch_address(&err) : nullptr;
+  double *scratch = need > 0 && !takes_slots<double>(channels) ? static_scratch_address(&err) : nullptr;
   if (err) return fail(CMACE_ERR_CUDA, "cmace_imp_bwd_edge_f64_noalloc: cudaGetSymbolAddress failed");
-  if (need > 0) {
+  if (scratch) {
     // the array keeps the previous call's contents; the part this call sums over starts from zero
     cudaError_t e = cudaMemsetAsync(scratch, 0, (size_t)need * sizeof(double), (cudaStream_t)stream);
     if (e != cudaSuccess)

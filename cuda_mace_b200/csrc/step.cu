@@ -85,7 +85,7 @@ struct Workspace {
   EdgeRows rows;
   Quad<T> *geo;
   T *basis, *Y, *h[2], *dh[2], *A, *m0, *b0, *up, *R, *m1, *l1, *gX1, *gm1, *T_, *gY1, *dr1, *gup, *gb0, *gX0, *gA,
-      *gvec, *dR, *partial, *q0, *dq, *gY0, *dr0;
+      *gvec, *dR, *q0, *dq, *gY0, *dr0;
   int64_t bytes;
   int shares;   // of grad Y of the second layer, to be added up
 
@@ -138,7 +138,6 @@ struct Workspace {
     take(gX0, n * 16 * C);
     take(gvec, E * 4);
     take(dR, f64 && !sp ? E * 4 * C : 0);
-    take(partial, f64 || sp || is_fused(m) ? 0 : cmace_imp_bwd_scratch_elems(E, (int)C, 0));
     gm1 = m1;   // the messages are not read again after the Linear
     gA = A;     // nor the sums after their product
   }
@@ -282,7 +281,7 @@ static int run_step(const cmace_step_model &m, cmace_step_io &io, const Workspac
       if constexpr (f64)
         return imp_bwd_edge_pair_f64(up, w.Y, w.R, w.dR, w.rows.row_of, w.gm1, io.sender, io.row_ptr, n, E, C, w.gY1, w.T_, st);
       else
-        return imp_bwd_edge<T>(up, w.Y, w.R, w.gm1, io.sender, io.row_ptr, n, E, ys, C, nullptr, w.gY1, w.T_, w.partial, st);
+        return imp_bwd_edge<T>(up, w.Y, w.R, w.gm1, io.sender, io.row_ptr, n, E, ys, C, nullptr, w.gY1, w.T_, nullptr, st);
     case S_RADIAL_BACK:
       if constexpr (f64) return CMACE_OK;   // not reached
       else

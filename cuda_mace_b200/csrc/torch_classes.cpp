@@ -190,7 +190,7 @@ class IMPAutograd : public torch::autograd::Function<IMPAutograd> {
     const bool f64 = is_f64(X);
     Tensor gradR = torch::empty_like(radial), gradY = torch::empty_like(Y);
     Tensor T = torch::empty({std::max<int64_t>(E, 1), C}, X.options());
-    const int64_t nscratch = cmace_imp_bwd_scratch_elems(E, (int)C, f64 ? 1 : 0);
+    const int64_t nscratch = C == 96 ? 0 : cmace_imp_bwd_scratch_elems(E, (int)C, f64 ? 1 : 0);   // 96: none is read
     Tensor scratch = torch::empty({std::max<int64_t>(nscratch, 1)}, X.options());
     Tensor gradX = torch::empty_like(X);
     // The grouping by sender (a radix sort: six small kernels, 40 us at 250 000 edges) does not depend on the edge pass

@@ -381,6 +381,14 @@ def neighbor_list_rows(positions, box, pbc, r_cut, n_receivers=None, lo=(0.0, 0.
 # --------------------------------------------------------------------------------------
 # invariant message passing
 # --------------------------------------------------------------------------------------
+def _grad_y_scratch(X, nedges):
+    """Partials of grad Y, where a row of the edge pass goes in several chunks.  96 channels go in one, although the query still
+    names the scratch of the three that they were."""
+    C = X.shape[1]
+    n = 0 if C == 96 else _abi.call("cmace_imp_bwd_scratch_elems", nedges, C, int(X.dtype == torch.float64))
+    return torch.empty(n, dtype=X.dtype, device=X.device) if n > 0 else None
+
+
 class _IMPFunction(torch.autograd.Function):
     @staticmethod
     def forward(ctx, X, Y, radial, topo):
@@ -409,8 +417,7 @@ class _IMPFunction(torch.autograd.Function):
         gradR = torch.empty_like(radial)
         gradY = torch.empty_like(Y)
         T = torch.empty(E, C, dtype=X.dtype, device=X.device) if need_x else None
-        nscratch = _abi.call("cmace_imp_bwd_scratch_elems", E, C, 1 if X.dtype == torch.float64 else 0)
-        scratch = torch.empty(nscratch, dtype=X.dtype, device=X.device) if nscratch > 0 else None
+        scratch = _grad_y_scratch(X, E)
         _abi.call("cmace_imp_bwd_edge_" + _suffix(X), _ptr(X), _ptr(Y), _ptr(radial), _ptr(G),
                   _ptr(topo.sender), _ptr(topo.row_ptr), N, E, C, _ptr(gradR), _ptr(gradY), _ptr(T),
                   _ptr(scratch), _stream())
@@ -454,8 +461,7 @@ class _RadialIMPFunction(torch.autograd.Function):
         need_x = ctx.needs_input_grad[0]
         gradY = torch.empty_like(Y)
         T = torch.empty(E, C, dtype=X.dtype, device=X.device) if need_x else None
-        nscratch = _abi.call("cmace_imp_bwd_scratch_elems", E, C, 0)
-        scratch = torch.empty(nscratch, dtype=X.dtype, device=X.device) if nscratch > 0 else None
+        scratch = _grad_y_scratch(X, E)
         _abi.call("cmace_imp_bwd_edge_f32", _ptr(X), _ptr(Y), _ptr(R), _ptr(G), _ptr(topo.sender), _ptr(topo.row_ptr),
                   N, E, C, 0, _ptr(gradY), _ptr(T), _ptr(scratch), _stream(), tag="no gradR")
         gradX = None
@@ -545,8 +551,7 @@ class _FusedRadialIMPFunction(torch.autograd.Function):
         gradR = torch.empty_like(R)
         gradY = torch.empty_like(Y)
         T = torch.empty(E, C, dtype=X.dtype, device=X.device) if need_x else None
-        nscratch = _abi.call("cmace_imp_bwd_scratch_elems", E, C, 0)
-        scratch = torch.empty(nscratch, dtype=X.dtype, device=X.device) if nscratch > 0 else None
+        scratch = _grad_y_scratch(X, E)
         _abi.call("cmace_imp_bwd_edge_f32", _ptr(X), _ptr(Y), _ptr(R), _ptr(G), _ptr(topo.sender), _ptr(topo.row_ptr),
                   N, E, C, _ptr(gradR), _ptr(gradY), _ptr(T), _ptr(scratch), _stream())
         ctx.R = None

@@ -163,11 +163,12 @@ int cmace_spline_bwd_f64(const double *r, const double *r_knots, const double *c
  * (wrapper :157-284, kernels impl.cu:167-399).  The edge pass writes gradY [16,E], gradR [E,4,C] unless
  * gradR == NULL (a caller that forms the radial-weight gradient on the fly, cmace_gemm3x_gradr_f32),
  * and, when T != NULL, the per-edge sender contribution T [E,C]; the node pass sums T over each
- * sender's group into gradX [N,C].  A warp covers 32*VEC channels (VEC = 4, 2 or 1 scalars per
- * lane, the widest that divides C/32 within 16 bytes); when C needs several such chunks (e.g.
- * float64 with C = 128) each chunk writes its own partial of gradY into gradY_partial, a scratch
- * of cmace_imp_bwd_scratch_elems(...) scalars, and a second small kernel sums them.  Pass NULL
- * when that query returns 0. */
+ * sender's group into gradX [N,C].  32 and 96 channels, and 64 in float32, go a whole row at a time, several edges a
+ * warp where a row does not fill it.  Otherwise a warp covers 32*VEC channels (VEC = 4, 2 or 1 scalars per lane, the widest
+ * that divides C/32 within 16 bytes); when C needs several such chunks (e.g. float64 with C = 128) each chunk writes its own
+ * partial of gradY into gradY_partial, a scratch of cmace_imp_bwd_scratch_elems(...) scalars, and a second small kernel
+ * sums them.  Pass NULL when that query returns 0; with 96 channels NULL will do as well (the query answers what their three
+ * chunks needed, for callers that size by it; the array is not read). */
 int cmace_imp_fwd_f32(const float *X, const float *Y, const float *R, const int32_t *sender,
                       const int32_t *row_ptr, int64_t nnodes, int64_t nedges, int channels,
                       float *out, cmace_stream_t stream);

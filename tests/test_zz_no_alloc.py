@@ -68,3 +68,32 @@ def test_noalloc_rejects_sizes_beyond_the_built_in_array():
     rc = lib.cmace_imp_bwd_edge_f64_noalloc(None, None, None, None, None, None, 10, too_many_edges, 128, None, None,
                                             None, None)
     assert rc == 3 and b"built-in array" in lib.cmace_last_error()
+
+
+# a whole row at a time: no scratch is asked for or read, with or without an allocation by the caller
+@pytest.mark.parametrize("dtype", [torch.float32, torch.float64])
+def test_edge_pass_of_96_channels_needs_no_scratch(dtype):
+    from cuda_mace_b200 import _abi, ops
+
+    dev, N, C = torch.device("cuda:0"), 300, 96
+    send, recv = random_graph(5, N, 11, empty_every=6)
+    E = send.numel()
+    g = torch.Generator().manual_seed(5)
+    X, Y, R, G = (torch.randn(*shape, generator=g, dtype=torch.float64).to(dtype).to(dev)
+                  for shape in ((N, C), (16, E), (E, 4, C), (N, 16, C)))
+    topo = ops.EdgeTopology(send.to(dev), recv.to(dev), N)
+    args = [t.data_ptr() for t in (X, Y, R, G, topo.sender, topo.row_ptr)] + [N, E, C]
+    stream = torch.cuda.current_stream().cuda_stream
+    name = "cmace_imp_bwd_edge_" + ("f32" if dtype == torch.float32 else "f64")
+    results = []
+    for variant in ("scratch", "none", "noalloc")[:2 if dtype == torch.float32 else 3]:
+        outs = [torch.full_like(R, float("nan")), torch.full_like(Y, float("nan")), torch.full((E, C), float("nan"), dtype=dtype, device=dev)]
+        scratch = torch.full((3 * 16 * E,), 7.0, dtype=dtype, device=dev)
+        if variant == "noalloc":
+            _abi.call(name + "_noalloc", *args, *[t.data_ptr() for t in outs], stream)
+        else:
+            _abi.call(name, *args, *[t.data_ptr() for t in outs], scratch.data_ptr() if variant == "scratch" else None, stream)
+        assert bool((scratch == 7.0).all())
+        results.append(outs)
+    for other in results[1:]:
+        assert all(torch.equal(a, b) for a, b in zip(results[0], other))
