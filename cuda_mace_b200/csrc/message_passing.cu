@@ -16,6 +16,7 @@
 //   gradY[m, e]  = sum_c G[i, m, c] * R[e, l, c] * X[s, c]   (16-value warp transpose-reduce)
 // Backward, node pass: gradX[s, c] = sum over the edges sent by s of T[e, c], walking the
 // sender-grouped edge permutation; again one warp per node, no atomics.
+#include <atomic>
 #include <cstdlib>
 
 #include "common.cuh"
@@ -125,20 +126,22 @@ __global__ void __launch_bounds__(SPLIT == 1 ? kWarpsPerBlock * 32 : SPLIT * 32,
   for (int m = 0; m < 16; m++) store_vec<T, VEC>(o + m * C, acc[m]);
 }
 
-template <typename T, int VEC>
+// JOIN: a block's warps have the chunks from `chunk` on of one receiver and slice, and their shares of gradY are added up in shared
+// memory in order, from the second launch on to what the launch before has left; otherwise a warp has a receiver and slice.
+template <typename T, int VEC, bool JOIN = false>
 __global__ void __launch_bounds__(kWarpsPerBlock * 32)
     imp_bwd_edge_kernel(const T *__restrict__ X, const T *__restrict__ Y, const T *__restrict__ R,
                         const T *__restrict__ G, const int32_t *__restrict__ sender,
                         const int32_t *__restrict__ row_ptr, int64_t nnodes, int64_t nedges, ImpLayout ys, int C,
-                        int slices, T *__restrict__ gradR, T *__restrict__ gradY_out, T *__restrict__ Tout) {
+                        int slices, int chunk, T *__restrict__ gradR, T *__restrict__ gradY_out, T *__restrict__ Tout) {
   grid_begin();
   const int lane = threadIdx.x & 31;
   // everything written is per edge: `slices` warps share a receiver, each takes every slices-th pair of its edges
-  const int64_t item = (int64_t)blockIdx.x * kWarpsPerBlock + (threadIdx.x >> 5);
+  const int64_t item = JOIN ? (int64_t)blockIdx.x : (int64_t)blockIdx.x * kWarpsPerBlock + (threadIdx.x >> 5);
   const int64_t node = slices == 1 ? item : item / slices;
   const int slice = slices == 1 ? 0 : (int)(item - node * slices);
   if (node >= nnodes) return;
-  const int c0 = blockIdx.y * (32 * VEC) + lane * VEC;
+  const int c0 = (JOIN ? chunk + (int)(threadIdx.x >> 5) : (int)blockIdx.y) * (32 * VEC) + lane * VEC;
   const int64_t e0 = row_ptr[node], e1 = row_ptr[node + 1];
   if (e0 >= e1) return;
   // with several channel chunks each chunk writes its own [16, E] partial of gradY
@@ -149,6 +152,7 @@ __global__ void __launch_bounds__(kWarpsPerBlock * 32)
   for (int m = 0; m < 16; m++) load_vec<T, VEC>(g[m], G + (node * 16 + m) * C + c0);
 
   __shared__ __align__(16) PairHarmonics<T, kWarpsPerBlock> harmonics;
+  __shared__ T shares[JOIN ? 2 : 1][JOIN ? kWarpsPerBlock : 1][32];   // of a pair of edges
   int turn = 0;
   const int ylm = lane & 15, yedge = lane >> 4;
   for (int64_t e = e0 + 2 * slice; e < e1; e += 2 * slices, turn ^= 1) {
@@ -204,7 +208,19 @@ __global__ void __launch_bounds__(kWarpsPerBlock * 32)
       }
       if (Tout != nullptr) store_vec<T, VEC>(Tout + ee * C + c0, t);
       const T tot = warp_reduce16(p, lane);
-      if ((lane & 1) == 0) gy[(lane >> 1) * ys.m + ee * ys.e] = tot;
+      if ((lane & 1) == 0) {
+        if (JOIN) shares[turn][threadIdx.x >> 5][16 * h + (lane >> 1)] = tot;
+        else gy[(lane >> 1) * ys.m + ee * ys.e] = tot;
+      }
+    }
+    if constexpr (JOIN) {
+      __syncthreads();   // the buffer of the pair before has been read by then
+      const int warps = blockDim.x >> 5;
+      if ((int)(threadIdx.x >> 5) == turn % warps && (!yedge || e + 1 < e1)) {
+        T *dst = gy + ylm * ys.m + (yedge ? eb : e) * ys.e, sum = chunk ? *dst : T(0);
+        for (int w = 0; w < warps; w++) sum += shares[turn][w][lane];
+        *dst = sum;
+      }
     }
   }
 }
@@ -1020,7 +1036,25 @@ static void launch_bwd_edge(const T *X, const T *Y, const T *R, const T *G, cons
   const int slices = few_nodes(nnodes * (C / (32 * VEC))) ? kSplit : 1;
   dim3 grid((unsigned)((nnodes * slices + kWarpsPerBlock - 1) / kWarpsPerBlock), C / (32 * VEC));
   launch_chained(imp_bwd_edge_kernel<T, VEC>, grid, kWarpsPerBlock * 32, 0, st, X, Y, R, G, sender, row_ptr,
-                                                                     nnodes, nedges, ys, C, slices, gradR, gy, Tout);
+                                                                     nnodes, nedges, ys, C, slices, 0, gradR, gy, Tout);
+}
+// the same without partials (no edge is left undefined: gradY starts from zero)
+template <typename T, int VEC>
+static int launch_bwd_edge_joined(const T *X, const T *Y, const T *R, const T *G, const int32_t *sender, const int32_t *row_ptr,
+                                  int64_t nnodes, int64_t nedges, ImpLayout ys, int C, T *gradR, T *gradY, T *Tout,
+                                  const char *what, cudaStream_t st) {
+  cudaError_t e = cudaMemsetAsync(gradY, 0, (size_t)(16 * nedges) * sizeof(T), st);
+  if (e != cudaSuccess) return fail(CMACE_ERR_CUDA, "%s: %s", what, cudaGetErrorString(e));
+  // us with 1, 2, 4 and 8 slices at 128 channels: 300 receivers of 200 edges 222, 215, 178, 159; 800 of 80 194, 159, 163, 163; 2 000 of
+  // 30 158, 150, 156, 169; 6 000 of 10 156, 167, 194, 240 (partials in memory and a pass that sums them: 134, 146, 149, 146)
+  const int chunks = C / (32 * VEC), slices = few_nodes(2 * nnodes) ? 8 : (nnodes <= 4 * 148 * 8 ? 2 : 1);
+  if (nnodes * slices > 0x7fffffffLL) return fail(CMACE_ERR_UNSUPPORTED, "%s: too many nodes", what);
+  for (int chunk = 0; chunk < chunks; chunk += kWarpsPerBlock) {
+    const int warps = chunks - chunk < kWarpsPerBlock ? chunks - chunk : kWarpsPerBlock;
+    launch_chained(imp_bwd_edge_kernel<T, VEC, true>, (unsigned)(nnodes * slices), warps * 32, 0, st, X, Y, R, G, sender, row_ptr,
+                   nnodes, nedges, ys, C, slices, chunk, gradR, gradY, Tout);
+  }
+  return check_launch(what);
 }
 
 int imp_bwd_edge_pair_f64(const double *X, const double *Y, const double *R, const double *dR, const int32_t *row_of,
@@ -1050,27 +1084,33 @@ int imp_fwd_rows_f64(const double *X, const double *Y, const double *R, const in
 
 static __device__ int g_staged_stall;   // set when a bounded wait of the staged edge pass gave up
 int *staged_stall_flag() {
-  static int *per_device[64] = {nullptr};
+  static std::atomic<int *> per_device[64];
   int dev = 0;
   if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) return nullptr;
-  if (per_device[dev] == nullptr) {
-    int *p = nullptr;
-    if (cudaGetSymbolAddress(reinterpret_cast<void **>(&p), g_staged_stall) == cudaSuccess) per_device[dev] = p;
-  }
-  return per_device[dev];
+  int *p = per_device[dev].load(std::memory_order_relaxed);
+  if (p == nullptr && cudaGetSymbolAddress(reinterpret_cast<void **>(&p), g_staged_stall) == cudaSuccess)
+    per_device[dev].store(p, std::memory_order_relaxed);   // several threads: the same address
+  return p;
+}
+
+template <typename T>
+static int check_bwd_edge(const T *X, const T *Y, const T *R, const T *G, const int32_t *sender, const int32_t *row_ptr,
+                          int64_t nnodes, int64_t nedges, int C, const T *gradR, const T *gradY, const T *Tout) {
+  int rc = check_common<T>(X, R, G, nnodes, nedges, C, "cmace_imp_bwd_edge");
+  if (rc || nnodes == 0 || nedges == 0) return rc;
+  if (!X || !Y || !R || !G || !sender || !row_ptr || !gradY)
+    return fail(CMACE_ERR_ARG, "cmace_imp_bwd_edge: null pointer");
+  if ((gradR && !aligned16(gradR)) || (Tout && !aligned16(Tout)))
+    return fail(CMACE_ERR_ARG, "cmace_imp_bwd_edge: outputs must be 16-byte aligned");
+  return CMACE_OK;
 }
 
 template <typename T>
 int imp_bwd_edge(const T *X, const T *Y, const T *R, const T *G, const int32_t *sender,
                         const int32_t *row_ptr, int64_t nnodes, int64_t nedges, ImpLayout ys, int C, T *gradR,
                         T *gradY, T *Tout, T *partial, cmace_stream_t stream) {
-  int rc = check_common<T>(X, R, G, nnodes, nedges, C, "cmace_imp_bwd_edge");
-  if (rc) return rc;
-  if (nnodes == 0 || nedges == 0) return CMACE_OK;
-  if (!X || !Y || !R || !G || !sender || !row_ptr || !gradY)
-    return fail(CMACE_ERR_ARG, "cmace_imp_bwd_edge: null pointer");
-  if ((gradR && !aligned16(gradR)) || (Tout && !aligned16(Tout)))
-    return fail(CMACE_ERR_ARG, "cmace_imp_bwd_edge: outputs must be 16-byte aligned");
+  int rc = check_bwd_edge<T>(X, Y, R, G, sender, row_ptr, nnodes, nedges, C, gradR, gradY, Tout);
+  if (rc || nnodes == 0 || nedges == 0) return rc;
   cudaStream_t st = (cudaStream_t)stream;
   if (takes_slots<T>(C)) {   // a whole row at a time: no partials
     bwd_edge_slots<T, false>(X, Y, R, nullptr, nullptr, G, sender, row_ptr, nnodes, ys, C, gradR, gradY, Tout, st);
@@ -1177,33 +1217,8 @@ CMACE_IMP_LAUNCHERS(double)
 // Some callers cannot hand over scratch memory because they cannot allocate on the device at the point
 // of the call: a plugin running inside another framework's memory pool that is already sized, or a
 // host thread that must not call into an allocator while the device is busy.  For those, the float64
-// edge backward keeps its per-chunk gradY partials in a fixed array in the library image.
-constexpr int64_t kStaticScratchElems = 2 * 1024 * 1024;  // doubles: 16 MiB, e.g. 65 536 edges at C = 128
-static __device__ __align__(256) double g_static_gradY_partial[kStaticScratchElems];
-
-// device address of the array, looked up once per device (index = CUDA device ordinal)
-static double *static_scratch_address(int *err) {
-  static double *addr[64] = {nullptr};
-  int dev = 0;
-  cudaError_t e = cudaGetDevice(&dev);
-  if (e != cudaSuccess || dev < 0 || dev >= 64) {
-    *err = 1;
-    return nullptr;
-  }
-  if (addr[dev] == nullptr) {
-    // the array's name is a host-side handle, not a device pointer: ask the runtime for the address
-    // on the device that is current now
-    double *p = nullptr;
-    e = cudaGetSymbolAddress(reinterpret_cast<void **>(&p), g_static_gradY_partial);
-    if (e != cudaSuccess || p == nullptr) {
-      *err = 1;
-      return nullptr;
-    }
-    addr[dev] = p;
-  }
-  *err = 0;
-  return addr[dev];
-}
+// edge backward adds up the channel chunks' shares of gradY in its blocks; nothing is shared between calls.
+constexpr int64_t kNoallocElems = 2 * 1024 * 1024;  // scratch doubles a call would need otherwise, e.g. 65 536 edges at C = 128
 
 }  // namespace cmace
 
@@ -1250,28 +1265,27 @@ int cmace_imp_bwd_edge_f64(const double *X, const double *Y, const double *R, co
   return imp_bwd_edge<double>(X, Y, R, G, sender, row_ptr, nnodes, nedges, ImpLayout{nedges, 1}, channels, gradR, gradY, T,
                               gradY_partial, stream);
 }
-int64_t cmace_imp_bwd_edge_f64_noalloc_max_elems(void) { return kStaticScratchElems; }
+int64_t cmace_imp_bwd_edge_f64_noalloc_max_elems(void) { return kNoallocElems; }
 
 int cmace_imp_bwd_edge_f64_noalloc(const double *X, const double *Y, const double *R, const double *G,
                                    const int32_t *sender, const int32_t *row_ptr, int64_t nnodes, int64_t nedges,
                                    int channels, double *gradR, double *gradY, double *T, cmace_stream_t stream) {
   const int64_t need = cmace_imp_bwd_scratch_elems(nedges, channels, 1);
-  if (need > kStaticScratchElems)
+  const ImpLayout ys{nedges, 1};
+  if (need > kNoallocElems)
     return fail(CMACE_ERR_UNSUPPORTED,
-                "cmace_imp_bwd_edge_f64_noalloc: %lld scratch elements needed, the built-in array holds %lld "
-                "(reduce the number of edges per call or use cmace_imp_bwd_edge_f64 with your own scratch)",
-                (long long)need, (long long)kStaticScratchElems);
-  int err = 0;
-  double *scratch = need > 0 && !takes_slots<double>(channels) ? static_scratch_address(&err) : nullptr;
-  if (err) return fail(CMACE_ERR_CUDA, "cmace_imp_bwd_edge_f64_noalloc: cudaGetSymbolAddress failed");
-  if (scratch) {
-    // the array keeps the previous call's contents; the part this call sums over starts from zero
-    cudaError_t e = cudaMemsetAsync(scratch, 0, (size_t)need * sizeof(double), (cudaStream_t)stream);
-    if (e != cudaSuccess)
-      return fail(CMACE_ERR_CUDA, "cmace_imp_bwd_edge_f64_noalloc: %s", cudaGetErrorString(e));
-  }
-  return imp_bwd_edge<double>(X, Y, R, G, sender, row_ptr, nnodes, nedges, ImpLayout{nedges, 1}, channels, gradR, gradY, T, scratch,
-                              stream);
+                "cmace_imp_bwd_edge_f64_noalloc: %lld scratch elements needed, calls are limited to the %lld of its former "
+                "built-in array (reduce the number of edges per call or use cmace_imp_bwd_edge_f64 with your own scratch)",
+                (long long)need, (long long)kNoallocElems);
+  if (need == 0 || takes_slots<double>(channels))
+    return imp_bwd_edge<double>(X, Y, R, G, sender, row_ptr, nnodes, nedges, ys, channels, gradR, gradY, T, nullptr, stream);
+  const int rc = check_bwd_edge<double>(X, Y, R, G, sender, row_ptr, nnodes, nedges, channels, gradR, gradY, T);
+  if (rc || nnodes == 0 || nedges == 0) return rc;
+  auto run = [&](auto launch) {
+    return launch(X, Y, R, G, sender, row_ptr, nnodes, nedges, ys, channels, gradR, gradY, T, "cmace_imp_bwd_edge_f64_noalloc",
+                  (cudaStream_t)stream);
+  };
+  return pick_vec<double>(channels) == 2 ? run(launch_bwd_edge_joined<double, 2>) : run(launch_bwd_edge_joined<double, 1>);
 }
 
 int cmace_imp_bwd_node_f32(const float *T, const int32_t *perm, const int32_t *send_ptr, int64_t nnodes,

@@ -1,8 +1,7 @@
-"""The entry point for callers that cannot allocate device memory: cmace_imp_bwd_edge_f64_noalloc keeps
-its scratch in an array inside the library, so it is called with inputs and outputs only.  Checked through
-the C-ABI against cmace_imp_bwd_edge_f64 (caller-provided scratch) and against the oracle's gradients on two calls
-in a row, the second with different data, so stale contents of the shared array would show.  Collected last on
-purpose."""
+"""The entry point for callers that cannot allocate device memory: cmace_imp_bwd_edge_f64_noalloc is called with inputs
+and outputs only.  Checked through the C-ABI against cmace_imp_bwd_edge_f64 (caller-provided scratch) and against the
+oracle's gradients on two calls in a row with different data, and against the former in calls that overlap on several
+streams.  Collected last on purpose."""
 import pytest
 import torch
 
@@ -68,6 +67,40 @@ def test_noalloc_rejects_sizes_beyond_the_built_in_array():
     rc = lib.cmace_imp_bwd_edge_f64_noalloc(None, None, None, None, None, None, 10, too_many_edges, 128, None, None,
                                             None, None)
     assert rc == 3 and b"built-in array" in lib.cmace_last_error()
+
+
+# calls on streams of their own, each behind a pause of its own so that they overlap; the chunks of 64 channels (128, 192) or of 32
+# (160, in two launches) are added in the order in which the other entry sums its partials: the same bits
+@pytest.mark.parametrize("C", [128, 160, 192])
+def test_noalloc_calls_that_overlap(C):
+    from cuda_mace_b200 import _abi, ops
+
+    dev, calls = torch.device("cuda:0"), []
+    for k in range(4):
+        N, deg = 150 + 60 * k, 9 + k
+        send, recv = random_graph(k, N, deg, empty_every=6)
+        E = send.numel()
+        g = torch.Generator().manual_seed(k)
+        ins = [torch.randn(*shape, generator=g, dtype=torch.float64).to(dev) for shape in ((N, C), (16, E), (E, 4, C), (N, 16, C))]
+        topo = ops.EdgeTopology(send.to(dev), recv.to(dev), N)
+        args = [t.data_ptr() for t in ins] + [topo.sender.data_ptr(), topo.row_ptr.data_ptr(), N, E, C]
+        outs = [[torch.full_like(ins[2], float("nan")), torch.full_like(ins[1], float("nan")),
+                 torch.full((E, C), float("nan"), dtype=torch.float64, device=dev)] for _ in range(2)]
+        scratch = torch.empty(_abi.call("cmace_imp_bwd_scratch_elems", E, C, 1), dtype=torch.float64, device=dev)
+        _abi.call("cmace_imp_bwd_edge_f64", *args, *[t.data_ptr() for t in outs[0]], scratch.data_ptr(),
+                  torch.cuda.current_stream().cuda_stream)
+        calls.append((args, outs, ins, topo, torch.cuda.Stream()))
+    torch.cuda.synchronize()
+    for _ in range(5):
+        for args, (want, got), _, _, stream in calls:
+            with torch.cuda.stream(stream):
+                for t in got:
+                    t.fill_(float("nan"))
+                torch.cuda._sleep(200_000)
+                _abi.call("cmace_imp_bwd_edge_f64_noalloc", *args, *[t.data_ptr() for t in got], stream.cuda_stream)
+        torch.cuda.synchronize()
+        for _, (want, got), _, _, _ in calls:
+            assert all(torch.equal(a, b) for a, b in zip(want, got))
 
 
 # a whole row at a time: no scratch is asked for or read, with or without an allocation by the caller
