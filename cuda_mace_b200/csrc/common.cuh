@@ -112,8 +112,10 @@ __device__ __forceinline__ void store_vec_stream(T *p, const T (&src)[VEC]) {
 //
 // A block's grid_release() comes after its own grid_wait().  So when a kernel's first block runs, everything before its predecessor has
 // completed: before grid_wait() it may read what is older than that (constant weights, the caller's list, what kernels before
-// the predecessor wrote) and set up barriers and tensor memory, and a chain of small kernels is mostly such beginnings.  Every
-// block waits on every path: a kernel that ended without having waited would let its successor overtake its predecessor.
+// the predecessor wrote) and set up barriers and tensor memory, and a chain of small kernels is mostly such beginnings.  What the
+// chain itself has written (elements, groupings, rows of pairs) it reads from L2 there (__ldcg, cp.async.cg, bulk copies): the
+// order of the waits says that the writes have been performed, nothing says when an SM's L1 has let go of an older line.
+// Every block waits on every path: a kernel that ended without having waited would let its successor overtake its predecessor.
 __device__ __forceinline__ void grid_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 __device__ __forceinline__ void grid_release() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 __device__ __forceinline__ void grid_begin() {

@@ -473,7 +473,7 @@ __global__ void __launch_bounds__(EB_THREADS, 1)
 #pragma unroll
         for (int i = 0; i < 4; i++) {
           const int64_t e = tile * EB_TILE + eb_edge(r0 + 8 * i), c = e < g.nedges ? e : g.nedges - 1;
-          next[i] = g.row_of ? __ldg(g.row_of + c) : (int)c;
+          next[i] = g.row_of ? __ldcg(g.row_of + c) : (int)c;
         }
       };
       if (blockIdx.x < ntiles) load_rows(blockIdx.x);

@@ -394,9 +394,10 @@ struct SenderElements {
 #pragma unroll
     for (int c = 0; c < 2; c++) s[c] = e0 + 32 * c + lane < e1 ? __ldg(sender + e0 + 32 * c + lane) : -1;
   }
+  template <bool EARLY = false>
   __device__ __forceinline__ void look_up() {   // the elements in place of the senders
 #pragma unroll
-    for (int c = 0; c < 2; c++) s[c] = s[c] >= 0 ? __ldg(species + s[c]) : -1;
+    for (int c = 0; c < 2; c++) s[c] = s[c] >= 0 ? (EARLY ? __ldcg(species + s[c]) : __ldg(species + s[c])) : -1;
   }
 };
 
@@ -620,7 +621,7 @@ __global__ void __launch_bounds__(SU_WARPS * 32)
   const int z0 = (int)(pair - node * chunks) * per, z1 = z0 + per < elements ? z0 + per : elements;
   SenderElements from(sender, species, row_ptr[node], row_ptr[node + 1], lane);
   if (EARLY) {
-    from.look_up();
+    from.look_up<true>();
     grid_begin();
   }
   SharedRows rows(row_of, row_lists[w], from);
@@ -713,7 +714,7 @@ __global__ void __launch_bounds__(SU_WARPS * 32)
   const int z = (int)(pair - node * elements);
   SenderElements from(sender, species, row_ptr[node], row_ptr[node + 1], lane);
   if (EARLY) {
-    from.look_up();
+    from.look_up<true>();
     grid_begin();
   }
   SharedRows rows(row_of, row_lists[w], from);
@@ -947,11 +948,11 @@ __global__ void __launch_bounds__(SU_WARPS * 32, 4)
   const int64_t node = pair / chunks;
   const int z0 = (int)(pair - node * chunks) * per, z1 = z0 + per < elements ? z0 + per : elements;
   SenderElements from(sender, species, row_ptr[node], row_ptr[node + 1], lane);
-  SharedRows rows(row_of, row_lists[w], from);
   if (EARLY) {
-    from.look_up();
+    from.look_up<true>();
     grid_begin();
-  }   // only the gradients of the sums are the kernel before's
+  }
+  SharedRows rows(row_of, row_lists[w], from);
   int32_t *list = lists[w];
   float *st = stage[w];
 #pragma unroll 1
@@ -1103,8 +1104,8 @@ __global__ void __launch_bounds__(SU_WARPS * 32, 3)
   const int64_t node = pair / elements;
   const int z = (int)(pair - node * elements);
   SenderElements from(sender, species, row_ptr[node], row_ptr[node + 1], lane);
+  if (EARLY) grid_begin();
   SharedRows rows(row_of, row_lists[w], from);
-  if (EARLY) grid_begin();   // only the gradients of the sums are the kernel before's
   int32_t *list = lists[w];
   double *st = stage[w];
   double2 P[2][8];
