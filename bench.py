@@ -135,17 +135,26 @@ class ClockSampler:
                 "samples": len(sm)}
 
 
-def algorithmic_bytes(name, s, N, Ns, E, C, Z):
-    """Bytes each step of the native sequence has to move (indices 4 B).  The two edges of a pair share a row of everything
-    that depends on the distance alone: it is written once and read by each of them.  The float32 step forms the second
-    layer's radial weights on chip, the float64 step writes them and their derivative."""
+def radial_rows(s, N, senders):
+    """Rows of what depends on an edge's distance alone: one a pair of edges from a line on that csrc/step.cu draws by the number
+    of edges, one an edge below it and for an edge whose sender is a ghost (its reverse is on another rank)."""
+    E = len(senders)
+    if E <= (9472 if s == 8 else 18944):
+        return E
+    owned = int((np.asarray(senders) < N).sum())
+    return owned // 2 + E - owned
+
+
+def algorithmic_bytes(name, s, N, Ns, E, C, Z, P):
+    """Bytes each step of the native sequence has to move (indices 4 B); P: radial_rows(), each written once and read by the
+    edges that share it.  The float32 step forms the second layer's radial weights on chip, the float64 step writes them and
+    their derivative."""
     if not name.startswith("step["):
         return {"cmace_receiver_csr": 4 * E + 4 * N, "cmace_nl_emit_f64": 35 * E + 48 * N}.get(name)
     row = 64 * s                              # one edge's hidden row (float32: an fp16 pair)
     m16, sums = 16 * N * C * s, 16 * N * 64 * Z * s
     fused = s == 4
     R = 4 * C * s
-    P = E // 2                                # pairs of edges
     return {
         "edge_prep": 24 * Ns + E * (24 + 8 + 4 * s + 16 * s + 16 * s),
         "radial": P * (16 * s + 4 * row),
@@ -184,14 +193,16 @@ ISSUE_NOTE = {step: f", on {warps} warps a scheduler (issue slots {slots} % used
               for step, warps, slots in (("step[edges_back]", 4, 60), ("step[messages]", 3, 42), ("step[radial]", 4, 47))}
 
 
-def tensor_flops(name, s, E, C):
+def tensor_flops(name, s, E, C, P):
     """Tensor-core flops one launch executes, for the steps whose binding roof is the tensor pipe: float32 runs three
-    fp16 terms of the product with the last radial layer ([E,64] x [64,4C]; the backward forms it for the derivative as
-    well) and of the hidden layers for values and derivatives of both perceptrons, a row a pair of edges."""
-    if s != 4 or C != 128:
+    fp16 terms of the product with the last radial layer ([E,64] x [64,4C], 96 channels padded to 128 in the forward; the
+    backward forms it for the derivative as well) and of the hidden layers for values and derivatives of both perceptrons
+    (P: radial_rows())."""
+    if s != 4:
         return None
-    return {"step[messages]": 3 * 2 * E * 4 * C * 64, "step[edges_back]": 2 * 3 * 2 * E * 4 * C * 64,
-            "step[radial]": 2 * 2 * 3 * 2 * (E // 2) * (16 * 64 + 2 * 64 * 64)}.get(name)
+    padded = 128 if C == 96 else C
+    return {"step[messages]": 3 * 2 * E * 4 * padded * 64, "step[edges_back]": 2 * 3 * 2 * E * 4 * C * 64,
+            "step[radial]": 2 * 2 * 3 * 2 * P * (16 * 64 + 2 * 64 * 64)}.get(name)
 
 
 def half_peak():
@@ -532,9 +543,10 @@ def main():
     # ---- roofline of the dominant kernel --------------------------------------------------------
     peak, peak_src = peaks()
     per_kernel = {}
+    P = radial_rows(s_bytes, N, dom.edge_index[1])
     top, top_ms = None, -1.0
     for name, (calls, tot) in sorted(kernel_ms.items()):
-        b = algorithmic_bytes(name, s_bytes, N, Ns, E, 128, sysd["n_species"])
+        b = algorithmic_bytes(name, s_bytes, N, Ns, E, 128, sysd["n_species"], P)
         avg = tot / calls
         per_kernel[name] = {"calls_per_step": calls / kernel_steps, "avg_ms": avg,
                             "share_of_step": tot / (bracketed_ms * kernel_steps),
@@ -546,7 +558,7 @@ def main():
         per_edge = NCU_TRAFFIC_PER_EDGE.get(top)
         traffic = per_edge[0] * E if per_edge else None
         traffic_src = f"ncu capture of a smaller case scaled by edges, {per_edge[1]}" if per_edge else None
-        flops = tensor_flops(top, s_bytes, E, 128)
+        flops = tensor_flops(top, s_bytes, E, 128, P)
         if flops:
             # not HBM-bound (its operands are formed on chip): the tensor pipe is the roof that binds it
             tpeak, tsrc = half_peak()
@@ -561,10 +573,10 @@ def main():
             ach = per_kernel[top]["achieved_gbs"]
             roofline = {"kernel": top, "bound": "hbm", "achieved": ach, "peak": peak, "unit": "GB/s",
                         "frac": ach / peak, "traffic": traffic, "traffic_source": traffic_src, "peak_source": peak_src,
-                        "algorithmic_bytes_per_launch": algorithmic_bytes(top, s_bytes, N, Ns, E, 128, sysd["n_species"]),
+                        "algorithmic_bytes_per_launch": algorithmic_bytes(top, s_bytes, N, Ns, E, 128, sysd["n_species"], P),
                         "avg_launch_ms": per_kernel[top]["avg_ms"]}
         # the largest HBM-bound kernel beside it, for the fraction of the copy peak the streaming kernels reach
-        hbm = [(v["share_of_step"], k) for k, v in per_kernel.items() if v["achieved_gbs"] and not tensor_flops(k, s_bytes, E, 128)]
+        hbm = [(v["share_of_step"], k) for k, v in per_kernel.items() if v["achieved_gbs"] and not tensor_flops(k, s_bytes, E, 128, P)]
         if hbm:
             k = max(hbm)[1]
             roofline["largest_hbm_bound_kernel"] = {"kernel": k, "achieved": per_kernel[k]["achieved_gbs"], "peak": peak,

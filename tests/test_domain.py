@@ -86,6 +86,24 @@ def test_partition_bookkeeping():
         domain.partition_slabs(pos, species, box, 8, 5.0, 0)  # slabs thinner than the cutoff
 
 
+def test_rows_of_the_bench_are_the_lists():
+    """Rows that the step forms of what depends on a distance: edges whose reverse is in a rank's list share one."""
+    import bench
+
+    box = np.array([11.0, 12.0, 45.0])
+    pos = systems.random_box(800, box, 0.9, seed=3)
+    for world, rank in ((1, 0), (2, 1)):
+        dom = domain.partition_slabs(pos, np.zeros(800, dtype=np.int64), box, world, 5.0, rank)
+        recv, send = dom.edge_index
+        found = set(zip(recv.tolist(), send.tolist(), map(tuple, np.rint(dom.shifts / box).astype(int).tolist())))
+        twins = sum((j, i, tuple(-x for x in k)) in found for i, j, k in found)
+        assert len(found) == recv.size > 18944 and (twins < recv.size) == (world == 2)
+        for s in (4, 8):
+            assert bench.radial_rows(s, dom.n_owned, send) == recv.size - twins // 2
+    assert bench.radial_rows(4, 100, np.zeros(18944, dtype=np.int64)) == 18944
+    assert bench.radial_rows(8, 100, np.zeros(9474, dtype=np.int64)) == 4737
+
+
 def test_single_rank_is_plain_periodic():
     pos, species, box, _ = make_case()
     d = domain.partition_slabs(pos, species, box, 1, 5.0, 0)
