@@ -3,6 +3,8 @@ import ctypes
 import os
 import re
 
+import pytest
+
 from cuda_mace_b200 import _abi
 
 ROOT = os.path.dirname(os.path.dirname(os.path.abspath(__file__)))
@@ -46,6 +48,24 @@ def test_fused_layout_of_earlier_callers_is_not_read(built_library):
     fused = size()
     m.fused_layout = 0
     assert size() == fused + E * 4 * 128 * 4
+
+
+@pytest.mark.parametrize("channels", [32, 64, 96])
+def test_fused_layout_of_narrow_models_has_a_name_of_its_own(built_library, channels):
+    """As above: neither no name nor the one of 128 channels makes the library read what a narrow model's arrays hold, nor the
+    other way round."""
+    header = open(os.path.join(ROOT, "include", "cuda_mace_b200.h")).read()
+    assert int(re.search(r"#define CMACE_FUSED_LAYOUT_NARROW (\d+)", header).group(1)) == _abi.FUSED_LAYOUT_NARROW
+    E = 1024
+
+    def size(C, layout):
+        m = _abi.StepModel(channels=C, elements=2, nbessel=8, fused_w=1, fused_w_back=1, fused_layout=layout)
+        return _abi.call("cmace_step_workspace_bytes", ctypes.byref(m), 10, 10, E)
+
+    fused = size(channels, _abi.FUSED_LAYOUT_NARROW)
+    for layout in (0, 1, _abi.FUSED_LAYOUT):
+        assert size(channels, layout) == fused + E * 4 * channels * 4
+    assert size(128, _abi.FUSED_LAYOUT_NARROW) == size(128, 0)
 
 
 def test_argument_errors_are_reported_not_raised(built_library):

@@ -143,8 +143,8 @@ def test_elemental_linear(dtype, N, Z, K, dev):
     assert torch.equal(out2, out.detach())
 
 
-# one row; a tile's edge and one row past it; K of part of a block (8), of a block and a quarter (40), of three blocks;
-# several tiles a block of threads (2 x 16 x 9 001 rows are 2 251 tiles of 128 on 148), one element with most nodes
+# two nodes; a tile's edge and one row past it; K of part of a block (8), of a block and a quarter (40), of three blocks;
+# several tiles a block of threads (16 x 9 001 rows are 1 126 tiles of 128 and a few remainders on 148), one element with most nodes
 @pytest.mark.parametrize("N,Z,K,Nout", [(2, 2, 8, 4), (128, 2, 40, 32), (129, 3, 96, 128), (257, 128, 32, 20), (9001, 5, 72, 64),
                                         (9001, 2, 128, 128)])
 def test_elemental_linear_of_gathered_rows(N, Z, K, Nout, dev):

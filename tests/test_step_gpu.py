@@ -275,6 +275,32 @@ def test_a_layout_of_earlier_callers_gives_the_same_forces(U):
     assert abs(float(out["interaction_energy"] - ref["interaction_energy"])) < 1e-5 * abs(float(ref["interaction_energy"]))
 
 
+# The same for fewer channels, whose plans name their layout too: without that name the second layer's rows leave as float32 and
+# its radial weights are written.  300 edges and more than the 18 944 from which a named layout looks for pairs
+@pytest.mark.parametrize("channels,layout", [(32, 0), (64, 0), (96, 0), (64, 2), (128, 3)])
+def test_a_layout_without_its_name_writes_the_radial_weights(U, channels, layout):
+    params, pos, ei, sh, species = _list_of(np.arange(300) // 20, 16, channels, channels)
+    for many in (False, True):
+        if many:
+            pos, ei, sh = _images(170, 7.0, 3)
+            species = np.arange(170) % 3
+        data = dict(positions=torch.from_numpy(pos).cuda(), species=torch.from_numpy(species.astype(np.int32)).cuda(),
+                    edge_index=torch.from_numpy(ei).to(torch.int32).cuda(), shifts=torch.from_numpy(sh).cuda())
+        assert (ei.shape[1] > 74 * 2 * 128) == many
+        want = model.InvariantMACE(params, U, dtype=torch.float64, device="cuda")(data)
+        mace = model.InvariantMACE(params, U, dtype=torch.float32, device="cuda")
+        plan = step.plan_of(mace)
+        assert plan.model.fused_layout == (_abi.FUSED_LAYOUT if channels == 128 else _abi.FUSED_LAYOUT_NARROW)
+        size = lambda: _abi.call("cmace_step_workspace_bytes", ctypes.byref(plan.model), len(pos), len(pos), ei.shape[1])
+        named, plan.model.fused_layout = size(), layout
+        assert size() >= named + ei.shape[1] * (4 * channels * 4 - 8) - 512   # less the numbers of shared rows
+        out = mace(data)
+        assert step.plan_of(mace) is plan
+        scale = float(want["forces"].abs().max())
+        assert float((out["forces"] - want["forces"]).abs().max()) < 1e-4 * scale
+        assert abs(float(out["interaction_energy"] - want["interaction_energy"])) < 1e-5 * float(want["node_energy"].abs().sum())
+
+
 # nothing of these calls is launched: the checks come first
 @pytest.mark.parametrize("species,node_attrs", [
     (torch.zeros(12, dtype=torch.int32), None), (torch.zeros(11, dtype=torch.int32, device="meta"), None),
@@ -615,6 +641,35 @@ def test_a_range_begins_after_what_its_caller_put_before_it(U, dtype, C, split, 
     assert chained == sum(ranges) - 2
     graph.replay()
     assert torch.equal(out["forces"], want)
+
+
+# Recorded float32 steps are chained up to 196 608 edges, live ones too: the same kernels, so the same bits, also for positions that
+# the recording has not seen, several replays in a row (each begins while the one before may still run)
+@pytest.mark.parametrize("channels", [64, 128])
+def test_a_recorded_step_of_many_edges_is_chained_and_the_same(U, channels):
+    n = 2300
+    ev, p = _periodic(U, n, torch.float32, channels)
+    data = dict(positions=p.clone(), species=ev.species, edge_index=ev.edge_index, shifts=ev.shifts)
+    assert 98304 < ev.edge_index.shape[1] <= 196608
+    mace, moved = ev.model, [p + 0.001 * k * torch.sin(p + k) for k in range(3)]
+    want = []
+    for q in moved:
+        data["positions"].copy_(q)
+        out = mace(data)
+        want.append((out["energy"].clone(), out["forces"].clone()))
+    side, graph = torch.cuda.Stream(), torch.cuda.CUDAGraph(keep_graph=True)
+    side.wait_stream(torch.cuda.current_stream())
+    with torch.cuda.graph(graph, stream=side):
+        out = mace(data)
+    nodes, edges, chained = _programmatic_edges(graph)
+    assert edges == chained == nodes - 1
+    for _ in range(4):
+        got = []
+        for q in moved:
+            data["positions"].copy_(q)
+            graph.replay()
+            got.append((out["energy"].clone(), out["forces"].clone()))
+        assert all(torch.equal(a, b) for x, y in zip(got, want) for a, b in zip(x, y))
 
 
 def test_results_do_not_share_memory(U):
