@@ -19,7 +19,8 @@
 //   forces        position gradient and energies
 //
 // With tabulated radial weights (cubic splines) the first layer has no perceptron to sum against: `sums` is the
-// message passing on the element's constant feature row, with the table evaluated there (spline_messages.cu), `fold` the layer's element-dependent Linear, and the backward mirrors that.
+// message passing on the element's constant feature row, with the table evaluated there (spline_messages.cu), `fold` the
+// layer's element-dependent Linear, and the backward mirrors that.
 //
 // Nodes of the first layer are kept in element order (slots) between `sums` and `mid_fwd` and on the way back, so the
 // element-dependent products see consecutive rows whatever the caller's order is.
@@ -132,7 +133,7 @@ struct Workspace {
     take(dq, n * ST_RO);
     take(T_, E * C);
     take(gY1, shares * E * 16);
-    take(dr1, shares * E);
+    take(dr1, f64 && !sp ? 0 : shares * E);   // float64: in component 0 of gY1
     take(gup, nl * C);
     take(gb0, n * C);
     take(gX0, n * 16 * C);
@@ -283,10 +284,10 @@ static int run_step(const cmace_step_model &m, cmace_step_io &io, const Workspac
       else
         return imp_bwd_edge<T>(up, w.Y, w.R, w.gm1, io.sender, io.row_ptr, n, E, ys, C, nullptr, w.gY1, w.T_, nullptr, st);
     case S_RADIAL_BACK:
-      if constexpr (f64) return CMACE_OK;   // not reached
-      else
+      if constexpr (!f64)
         return gemm3x_gradr(up, w.gm1, w.Y, ys, io.sender, io.receiver, static_cast<const float *>(m.radial_back), E, C,
                             ST_H, w.dh[1], w.dr1, io.status, st);
+      break;
     case S_SENDERS:
       return imp_bwd_node<T>(w.T_, io.perm, io.send_ptr, nl, E, C, gup, st);
     case S_MID_BACK:
@@ -317,7 +318,7 @@ static int run_step(const cmace_step_model &m, cmace_step_io &io, const Workspac
           return step_sums_bwd_half(w.gA, w.h[0], w.dh[0], w.Y, io.sender, io.row_ptr, w.species, w.slot_of, w.rows.row_of, w.gY1,
                                     fused ? nullptr : w.dr1, w.geo, n, Z, scales[0].out_v, scales[0].out_t, w.gvec, st);
       return K::sums_bwd(w.gA, w.h[0], w.dh[0], w.Y, io.sender, io.row_ptr, w.species, w.slot_of, w.rows.row_of, w.gY1, w.shares,
-                         w.dr1, w.geo, n, E, Z, w.gvec, st);
+                         f64 ? nullptr : w.dr1, w.geo, n, E, Z, w.gvec, st);
     case S_FORCES:
       return K::forces(w.gvec, io.row_ptr, io.perm, io.send_ptr, n, nl, io.gradient_sign, io.gradient, io.species, Z,
                        io.interaction, io.node_energy, io.status, f64 ? nullptr : staged_stall_flag(), io.sums, st);
