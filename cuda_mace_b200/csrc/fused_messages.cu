@@ -529,7 +529,8 @@ int fused_messages(const float *X, const float *Y, const void *h, const void *W,
     cudaError_t e = cudaMemsetAsync(out, 0, (size_t)nnodes * 16 * C * sizeof(float), st);
     return e == cudaSuccess ? CMACE_OK : fail(CMACE_ERR_CUDA, "%s: %s", what, cudaGetErrorString(e));
   }
-  const FusedMessagesArgs g{X, Y, static_cast<const char *>(h), static_cast<const uint4 *>(W), sender, receiver, row_ptr, row_of, status, nnodes, nedges, factor, out};
+  const FusedMessagesArgs g{X, Y, static_cast<const char *>(h), static_cast<const uint4 *>(W), sender, receiver, row_ptr, row_of,
+                            status, nnodes, nedges, factor, out};
   switch (C) {
     case 32: return launch_fused_messages<32>(g, what, st);
     case 64: return launch_fused_messages<64>(g, what, st);

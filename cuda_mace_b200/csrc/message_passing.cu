@@ -360,7 +360,8 @@ struct SlotHarmonics {
 };
 
 // Blocks an SM, as measured: float32 37 us with three at 32 channels (44 with four), 70 with four at 64 (81 with three); float64 of 32
-// channels 64 with three (76 with four), but 108 with four (166 with three) where rows are looked up.
+// channels 64 with three (76 with four), but 108 with four (166 with three) where rows are looked up.  A block's 128 threads then have
+// 96 (five), 128 (four) or 168 registers each (three), 202 to 204 with two; none spills but 64 channels of float32 (16 bytes).
 template <typename T, int VEC, int LANES, bool ROWS>
 constexpr int fwd_slots_blocks() {
   if (VEC == 3) return sizeof(T) == 4 ? 5 : 2;
@@ -865,7 +866,8 @@ __global__ void sum_partials_kernel(const T *__restrict__ partial, int nchunks, 
 // One warp a sender, float32, at 16 000 atoms: 32 channels ten blocks 52 -> 44 (one 60, sixteen 64), 64 channels eight 70 -> 58 (one
 // 60, ten 60, twelve 80; 209 -> 183 at 64 000), 128 channels one 95 -> 88 (eight 91, ten 117; 330 -> 301 at 64 000), 96 channels
 // nothing said and the list's lines prefetched 81 (109 without the prefetch, which is no help to the others; one, six to nine 88, twelve
-// 130); float64 with 96 channels one 84 -> 76 at 8 000.
+// 130); float64 with 96 channels one 84 -> 76 at 8 000.  Registers that come of it: 48 of 256 threads (64 with three doubles a lane); of 128
+// threads in float32 48, 62, 48, 74 for one to four values a lane, in float64 64 or 80.  A compiler that arrives at others: measure again.
 template <typename T, int VEC, int SPLIT>
 constexpr int node_blocks_an_sm() {
   if (SPLIT > 1) return sizeof(T) * VEC <= 16 ? 5 : 4;

@@ -141,10 +141,10 @@ __device__ void group_nodes(int64_t first, int64_t end, int blocks, int block, b
 }
 
 // ---- edges that share a length ------------------------------------------------------------------------------------
-// An edge j -> i and its reverse i -> j have the same length bit for bit (their vectors are exact negatives), so both
-// perceptrons' rows h and h' are the same: they are formed once a pair.  In a complete list that is half of the radial work; an
-// edge whose reverse is missing (an incomplete list, a ghost sender) keeps a row of its own, and no row is shared on anything but
-// the equality of the vectors of this call.
+// The vectors of an edge j -> i and its reverse i -> j are exact negatives, so their lengths and both perceptrons' rows h and h' are
+// the same: they are formed once a pair.  In a complete list that is half of the radial work; an edge whose reverse is missing (an
+// incomplete list, a ghost sender) keeps a row of its own.  What is compared are the rounded unit vectors and 1/r of this call:
+// two edges between the same atoms that agree in these have the same length but for its rounding.
 //
 // Of a pair the edge with the lower receiver leads; the other looks for it in its sender's row of the list: a warp asks the rows
 // of eight of its edges at a time, lanes beside one another, the first edge that matches is the leader.  Leaders are numbered as
@@ -152,7 +152,10 @@ __device__ void group_nodes(int64_t first, int64_t end, int blocks, int block, b
 // leaders[k] is the edge of row k, row_of[e] the row of a leader, and ~leader for the other edge of a pair until the radial kernel
 // looks its row up (resolve_rows).  The search is a chain of four dependent loads in short lists and instruction issue in long ones:
 // 8 us for 9 900 edges, 14 for 416 000 in float64, 22 for 833 000 and 100 for 3.3 million in float32 (a quarter of the blocks'
-// additions to the counter: the same); with the vectors compared for four edges one after the other 20 and 39 in float64.
+// additions to the counter: the same); with the vectors compared for four edges one after the other 20 and 39 in float64.  A list
+// without reverses pays the search for nothing, us of a step: 3 to 4 for 20 600 edges, 7 for 42 000, 16 for 416 000, 60 for 1.7 million
+// where every edge looks (senders below their receivers), 3, 4, 4 and 18 where none does.  In a complete list the float32 radial kernel
+// alone saves 8 for 20 900 edges, 27 for 156 000, 140 for 833 000, 630 for 3.3 million.
 template <typename T>
 __device__ __forceinline__ void find_pairs(int64_t first, const int32_t *__restrict__ sender, const int32_t *__restrict__ receiver,
                                            const int32_t *__restrict__ row_ptr, const Quad<T> *__restrict__ geo, int64_t nedges,
@@ -687,8 +690,9 @@ int step_sums_half(const void *h, const float *Y, const int32_t *sender, const i
   const int per = elements_per_warp(nnodes, elements);
   const int64_t blocks = (nnodes * ((elements + per - 1) / per) + SU_WARPS - 1) / SU_WARPS;
   if (blocks > 0)
-    launch_chained(chain_launches() == Chain::on ? sums_f16_kernel<true> : sums_f16_kernel<false>, (unsigned)blocks, SU_WARPS * 32, 0, st, static_cast<const uint4 *>(h), Y, sender, row_ptr, species,
-                                                               slot_of, row_of, nnodes, elements, per, out_v / SU_Y_SCALE, A);
+    launch_chained(chain_launches() == Chain::on ? sums_f16_kernel<true> : sums_f16_kernel<false>, (unsigned)blocks, SU_WARPS * 32, 0,
+                   st, static_cast<const uint4 *>(h), Y, sender, row_ptr, species, slot_of, row_of, nnodes, elements, per,
+                   out_v / SU_Y_SCALE, A);
   return check_launch("cmace_step(sums)");
 }
 
@@ -772,10 +776,11 @@ int StepKernels<T>::sums(const T *h, const T *Y, const int32_t *sender, const in
   const int64_t blocks = (nnodes * elements + SU_WARPS - 1) / SU_WARPS;
   if (blocks > 0) {
     if constexpr (sizeof(T) == 4)
-      launch_chained(sums_tf32_kernel, (unsigned)blocks, SU_WARPS * 32, 0, st, h, Y, sender, row_ptr, species, slot_of, nnodes, elements, A);
+      launch_chained(sums_tf32_kernel, (unsigned)blocks, SU_WARPS * 32, 0, st, h, Y, sender, row_ptr, species, slot_of, nnodes,
+                     elements, A);
     else
-      launch_chained(chain_launches() == Chain::on ? sums_f64_kernel<true> : sums_f64_kernel<false>, (unsigned)blocks, SU_WARPS * 32, 0, st, h, Y, sender, row_ptr, species, slot_of,
-                     row_of, nnodes, elements, A);
+      launch_chained(chain_launches() == Chain::on ? sums_f64_kernel<true> : sums_f64_kernel<false>, (unsigned)blocks, SU_WARPS * 32,
+                     0, st, h, Y, sender, row_ptr, species, slot_of, row_of, nnodes, elements, A);
   }
   return check_launch("cmace_step(sums)");
 }
@@ -971,7 +976,8 @@ __global__ void __launch_bounds__(SU_WARPS * 32, 4)
         for (int r = 0; r < 2; r++) load32(p + (g + 8 * r) * width + 32 * i, v[i][r][0], v[i][r][1]);
       if (z + 1 < z1) {   // the next element's gradients on their way to L1: lane's half of a row of 64
         const int nb = (z + 1) >> 1, nw = sums_block_width(elements, nb);
-        prefetch_l1(gA + (int64_t)nb * nnodes * (16 * 128) + ((int64_t)slot_of[node] * 16 + (lane >> 1)) * nw + ((z + 1) & 1) * ST_H + 32 * (lane & 1));
+        const float *block = gA + (int64_t)nb * nnodes * (16 * 128) + (int64_t)slot_of[node] * 16 * nw;
+        prefetch_l1(block + (lane >> 1) * nw + ((z + 1) & 1) * ST_H + 32 * (lane & 1));
       }
       if (!EARLY && z == z0) from.look_up();
 #pragma unroll
@@ -1074,9 +1080,9 @@ int step_sums_bwd_half(const float *gA, const void *h, const void *dh, const flo
   const int per = elements_per_warp(nnodes, elements);
   const int64_t blocks = (nnodes * ((elements + per - 1) / per) + SU_WARPS - 1) / SU_WARPS;
   if (blocks > 0)
-    launch_chained(chain_launches() == Chain::on ? sums_bwd_f16_kernel<true> : sums_bwd_f16_kernel<false>, (unsigned)blocks, SU_WARPS * 32, 0, st, 
-        gA, static_cast<const uint4 *>(h), static_cast<const uint4 *>(dh), Y, sender, row_ptr, species, slot_of, row_of, gY1, dr1,
-        geo, nnodes, elements, per, out_v, out_t, gvec);
+    launch_chained(chain_launches() == Chain::on ? sums_bwd_f16_kernel<true> : sums_bwd_f16_kernel<false>, (unsigned)blocks,
+                   SU_WARPS * 32, 0, st, gA, static_cast<const uint4 *>(h), static_cast<const uint4 *>(dh), Y, sender, row_ptr, species,
+                   slot_of, row_of, gY1, dr1, geo, nnodes, elements, per, out_v, out_t, gvec);
   return check_launch("cmace_step(sums_back)");
 }
 
@@ -1187,8 +1193,9 @@ int StepKernels<T>::sums_bwd(const T *gA, const T *h, const T *dh, const T *Y, c
       launch_chained(sums_bwd_tf32_kernel, (unsigned)blocks, SU_WARPS * 32, 0, st, gA, h, dh, Y, sender, row_ptr, species, slot_of,
                                                                       gY1, dr1, geo, nnodes, elements, gvec);
     else
-      launch_chained(chain_launches() == Chain::on ? sums_bwd_f64_kernel<true> : sums_bwd_f64_kernel<false>, (unsigned)blocks, SU_WARPS * 32, 0, st, gA, h, dh, Y, sender, row_ptr, species, slot_of,
-                     row_of, gY1, shares, geo, nnodes, nedges, elements, gvec);
+      launch_chained(chain_launches() == Chain::on ? sums_bwd_f64_kernel<true> : sums_bwd_f64_kernel<false>, (unsigned)blocks,
+                     SU_WARPS * 32, 0, st, gA, h, dh, Y, sender, row_ptr, species, slot_of, row_of, gY1, shares, geo, nnodes, nedges,
+                     elements, gvec);
   }
   return check_launch("cmace_step(sums_bwd)");
 }

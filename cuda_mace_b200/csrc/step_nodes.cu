@@ -93,7 +93,8 @@ int StepKernels<T>::contract_fwd(const T *X, const int32_t *types, const T *weff
                                  cudaStream_t st) {
   const int ch = channel_block(C);
   if (n > 0)
-    launch_chained(step_contract_kernel<T, false>, dim3((unsigned)node_blocks(n, 16, ch), C / ch), ch, 0, st, X, types, weff, nullptr, n, C, early, b);
+    launch_chained(step_contract_kernel<T, false>, dim3((unsigned)node_blocks(n, 16, ch), C / ch), ch, 0, st, X, types, weff, nullptr, n,
+                   C, early, b);
   return check_launch("cmace_step(contract_fwd)");
 }
 template <typename T>
@@ -101,7 +102,8 @@ int StepKernels<T>::contract_bwd(const T *X, const int32_t *types, const T *weff
                                  cudaStream_t st) {
   const int ch = channel_block(C);
   if (n > 0)
-    launch_chained(step_contract_kernel<T, true>, dim3((unsigned)node_blocks(n, 12, ch), C / ch), ch, 0, st, X, types, weff, gb, n, C, early, gX);
+    launch_chained(step_contract_kernel<T, true>, dim3((unsigned)node_blocks(n, 12, ch), C / ch), ch, 0, st, X, types, weff, gb, n, C,
+                   early, gX);
   return check_launch("cmace_step(contract_bwd)");
 }
 
@@ -427,14 +429,14 @@ static int launch_mid(const char *what, int64_t n, int C, int threads, Kernel k8
 template <typename T>
 int StepKernels<T>::mid_fwd(const T *b, const int32_t *node_of, const int32_t *slot_type, const T *wu, const T *extra,
                             int64_t n, int C, T *up, T *q0, cudaStream_t st) {
-  return launch_mid<T>("cmace_step(mid_fwd)", n, C, 2 * C + 64, mid_fwd_kernel<T, 8>, mid_fwd_kernel<T, 16>, mid_fwd_kernel<T, 32>, st, b, node_of, slot_type,
-                       wu, extra, n, C, up, q0);
+  return launch_mid<T>("cmace_step(mid_fwd)", n, C, 2 * C + 64, mid_fwd_kernel<T, 8>, mid_fwd_kernel<T, 16>, mid_fwd_kernel<T, 32>, st,
+                       b, node_of, slot_type, wu, extra, n, C, up, q0);
 }
 template <typename T>
 int StepKernels<T>::mid_bwd(const T *gup, const int32_t *node_of, const int32_t *slot_type, const T *dq, const T *wu_t,
                             const T *extra_t, double scale, int64_t n, int C, T *gb, cudaStream_t st) {
-  return launch_mid<T>("cmace_step(mid_bwd)", n, C, 2 * C, mid_bwd_kernel<T, 8>, mid_bwd_kernel<T, 16>, mid_bwd_kernel<T, 32>, st, gup, node_of, slot_type,
-                       dq, wu_t, extra_t, (T)scale, n, C, gb);
+  return launch_mid<T>("cmace_step(mid_bwd)", n, C, 2 * C, mid_bwd_kernel<T, 8>, mid_bwd_kernel<T, 16>, mid_bwd_kernel<T, 32>, st, gup,
+                       node_of, slot_type, dq, wu_t, extra_t, (T)scale, n, C, gb);
 }
 
 #define CMACE_STEP_NODES(T)                                                                                          \

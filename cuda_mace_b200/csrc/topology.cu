@@ -35,7 +35,8 @@ __global__ void iota_kernel(int32_t *p, int64_t n) {
 // Short lists: a stable counting sort and its pointers by one block.  Every warp counts a contiguous piece, lanes with the same key
 // together (match); a key's places follow from the warps' counts in order, and a second walk over the piece writes them.  The radix
 // sort is eight launches and memsets around two passes; here one launch: 17 -> 7 us at 1 600 entries, 17 -> 11 at 3 000, 31 -> 26 at
-// 10 000, but 42 -> 48 at 20 000 (a match of 32 different keys costs 70 cycles of the one SM).  Keys outside 0 .. nkeys - 1 come last, as in the radix sort.
+// 10 000, but 42 -> 48 at 20 000 (a match of 32 different keys costs 70 cycles of the one SM).  Keys outside 0 .. nkeys - 1 come
+// last, as in the radix sort.
 constexpr int GS_THREADS = 1024, GS_WARPS = GS_THREADS / 32, GS_AHEAD = 4;
 constexpr int64_t GS_MOST = 8192;      // entries: the block's walk takes 2.4 us a thousand, the radix sort 17 to 30 us up to 10 000
 constexpr int64_t GS_MOST_KEYS = 1600; // 33 counts a key in shared memory

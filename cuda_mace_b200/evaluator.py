@@ -90,8 +90,9 @@ class EnergyForceEvaluator:
     def capture(self, positions_owned):
         """Records the whole energy+force step for the current neighbour list as a CUDA graph; later calls copy
         the positions into the graph's input and replay it, which takes the host's part (80 to 95 us a step) out
-        of a program that is short of it; the step itself is no faster (about 420 us either way at 3 000 atoms).  Single-rank domains only: the halo exchange of a multi-rank step is host-driven.  A new
-        neighbour list drops the recording, and so does a changed model."""
+        of a program that is short of it; the step itself is no faster (about 420 us either way at 3 000 atoms).  Single-rank
+        domains only: the halo exchange of a multi-rank step is host-driven.  A new neighbour list drops the recording, and so
+        does a changed model."""
         if self.dom.nranks != 1:
             raise RuntimeError("capture() needs a single-rank domain")
         self._graph, self._recording = None, True   # the warm-up takes the way that will be recorded

@@ -365,8 +365,8 @@ def pays(plan, atoms, edges, recorded=False):
     50 000 atoms of 21 edges: 32 channels 3.87; 3.65 at 11, 64 5.04; 5.20 at 14 and 5.57; 5.22 at 16, 96 6.68; 6.90 at 16.  float64,
     30 000 atoms of 10 edges: 32 channels 3.61; 4.21 at 5 and 4.42; 4.24 at 7, 64 5.91; 5.94 at 8, 96 8.55; 8.75 at 8 and 9.80; 8.87 at
     10, 128 11.24; 11.17 at 10; 15 000 atoms of 21 edges: 32 4.10; 3.99 at 13, 64 5.43; 5.47 at 15, 96 7.65; 7.62 at 15, 128 9.02; 9.49
-    at 16.  The lines are where both take the same; a condensed system (52 edges) stays native at any number of elements.  The operators' launches take the
-    host 2.1 ms, which small systems never need natively (20 000 atoms of 10 edges, 16 elements, float32, 32 channels: 1.98;
+    at 16.  The lines are where both take the same; a condensed system (52 edges) stays native at any number of elements.  The
+    operators' launches take the host 2.1 ms, which small systems never need natively (20 000 atoms of 10 edges, 16 elements, float32, 32 channels: 1.98;
     2.07); recorded, both take the same at 3 000 atoms of 16 elements in float32 (0.39; 0.40) and 1 000 in float64."""
     m = plan.model
     if plan.elements <= 4 or m.spline[0]:
