@@ -359,7 +359,9 @@ int cmace_symcon_effective_weights(const cmace_symcon_plan *plan, int is_f64, co
  * What OptimizedInvariantMACE.forward does with autograd (models/InvariantMACE.py:246-379), as one sequence of
  * kernel launches with its gradient written out: no autograd graph, no allocation, no synchronisation.  The caller
  * owns weights, workspace and outputs.  csrc/step.cu documents the sequence; steps can be run in ranges, which is
- * where a decomposed system exchanges node features (after "mid_fwd") and their gradients (after "senders"). */
+ * where a decomposed system exchanges node features (after "mid_fwd") and their gradients (after "senders").
+ * A range begins when what is before it on the stream is complete; within a range a kernel may read the list, the weights
+ * and exchanged rows while the kernel before it still runs. */
 #define CMACE_FUSED_LAYOUT 2 /* names the layouts of fused_w and fused_w_back below for 128 channels; changes with them */
 #define CMACE_FUSED_LAYOUT_NARROW 3 /* and those for 32, 64 and 96 channels */
 typedef struct cmace_step_model {
