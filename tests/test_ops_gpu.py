@@ -778,6 +778,21 @@ def test_an_infinite_weight_stays_infinite(dtype, C, dev):
     assert bool((out == float("inf")).all())
 
 
+# the same for every kernel of the forward, whole warps too: one warp a receiver and several, an odd number of edges
+@pytest.mark.parametrize("n", [100, 300, 600, 1300, 2500])
+@pytest.mark.parametrize("dtype,C", [(dtype, C) for dtype in DTYPES for C in (32, 64, 96, 128, 160)])
+def test_an_infinite_weight_stays_infinite_in_every_kernel(dtype, C, n, dev):
+    from cuda_mace_b200 import ops
+
+    deg = 5
+    recv = torch.arange(n, dtype=torch.int32, device=dev).repeat_interleave(deg)
+    X, Y = torch.ones(n, C, dtype=dtype, device=dev), torch.ones(16, n * deg, dtype=dtype, device=dev)
+    R = torch.ones(n * deg, 4, C, dtype=dtype, device=dev)
+    R[deg - 1::deg] = float("inf")
+    out = ops.InvariantMessagePassingTP()(X, Y, R, recv.flip(0).contiguous(), recv, n)
+    assert bool((out == float("inf")).all())
+
+
 # grouping by a key: one block's counting sort up to 8 192 entries of 1 600 keys, the radix sort beyond, against a stable sort; whole
 # and partial warps, pieces of one warp, keys that do not occur
 @pytest.mark.parametrize("n,nkeys", [(1, 1), (31, 7), (33, 40), (1024, 3), (1025, 1600), (5000, 1), (8192, 1600), (8192, 1601),
