@@ -384,8 +384,11 @@ static int elements_per_warp(int64_t nnodes, int elements) {
   return (elements + chunks - 1) / chunks;
 }
 
-// In a chain of launches (EARLY) the look-up stands before grid_wait(), otherwise behind the loads that it would hold up: with one
-// order for both the sums of 16 000 atoms took 144 us instead of 135, their backward 191 instead of 183.
+// In a chain of launches (EARLY) the list is read before grid_wait(), and while few warps ask (kSoonWarps) the senders' elements as well,
+// from L2: 91.9 -> 91.2 us a step of 192 atoms of 4 elements, but 106 -> 113 at 300 of 10, whose 3 000 warps meet at the ten lines of the
+// elements; those look them up behind the wait, through L1.  Otherwise the look-up stands behind the loads that it would hold up: with
+// one order for both the sums of 16 000 atoms took 144 us instead of 135, their backward 191 instead of 183.
+constexpr int64_t kSoonWarps = 148 * 8;
 struct SenderElements {
   const int32_t *__restrict__ sender, *__restrict__ species;
   int64_t e0, e1;
@@ -410,12 +413,16 @@ struct SenderElements {
 struct SharedRows {
   const int32_t *__restrict__ row_of;
   int32_t *first, *list;
-  __device__ __forceinline__ SharedRows(const int32_t *__restrict__ row_of_, int32_t (&buf)[64 + SU_LIST], const SenderElements &from)
+  // early: before grid_wait(), from L2
+  __device__ __forceinline__ SharedRows(const int32_t *__restrict__ row_of_, int32_t (&buf)[64 + SU_LIST], const SenderElements &from,
+                                        bool early = false)
       : row_of(row_of_), first(buf), list(buf + 64) {
 #pragma unroll
     for (int i = 0; i < 64; i += 32)
       if (from.e0 + i + from.lane < from.e1) {
-        if (row_of)
+        if (row_of && early)
+          first[i + from.lane] = __ldcg(row_of + from.e0 + i + from.lane);
+        else if (row_of)
           asm volatile("cp.async.ca.shared.global [%0], [%1], 4;" ::"r"(smem_u32(first + i + from.lane)),
                        "l"(row_of + from.e0 + i + from.lane)
                        : "memory");
@@ -620,12 +627,14 @@ __global__ void __launch_bounds__(SU_WARPS * 32)
     if (EARLY) grid_begin();
     return;
   }
+  const bool soon = nnodes * chunks <= kSoonWarps;
   const int64_t node = pair / chunks;
   const int z0 = (int)(pair - node * chunks) * per, z1 = z0 + per < elements ? z0 + per : elements;
   SenderElements from(sender, species, row_ptr[node], row_ptr[node + 1], lane);
   if (EARLY) {
-    from.look_up<true>();
+    if (soon) from.look_up<true>();
     grid_begin();
+    if (!soon) from.look_up();
   }
   SharedRows rows(row_of, row_lists[w], from);
   int32_t *list = lists[w];
@@ -714,12 +723,14 @@ __global__ void __launch_bounds__(SU_WARPS * 32)
     if (EARLY) grid_begin();
     return;
   }
+  const bool soon = nnodes * elements <= kSoonWarps;
   const int64_t node = pair / elements;
   const int z = (int)(pair - node * elements);
   SenderElements from(sender, species, row_ptr[node], row_ptr[node + 1], lane);
   if (EARLY) {
-    from.look_up<true>();
+    if (soon) from.look_up<true>();
     grid_begin();
+    if (!soon) from.look_up();
   }
   SharedRows rows(row_of, row_lists[w], from);
   int32_t *list = lists[w];
@@ -950,14 +961,16 @@ __global__ void __launch_bounds__(SU_WARPS * 32, 4)
     if (EARLY) grid_begin();
     return;
   }
+  const bool soon = nnodes * chunks <= kSoonWarps;
   const int64_t node = pair / chunks;
   const int z0 = (int)(pair - node * chunks) * per, z1 = z0 + per < elements ? z0 + per : elements;
   SenderElements from(sender, species, row_ptr[node], row_ptr[node + 1], lane);
+  SharedRows rows(row_of, row_lists[w], from, EARLY);
   if (EARLY) {
-    from.look_up<true>();
+    if (soon) from.look_up<true>();
     grid_begin();
-  }
-  SharedRows rows(row_of, row_lists[w], from);
+    if (!soon) from.look_up();
+  }   // only the gradients of the sums are the kernel before's
   int32_t *list = lists[w];
   float *st = stage[w];
 #pragma unroll 1
@@ -1110,8 +1123,8 @@ __global__ void __launch_bounds__(SU_WARPS * 32, 3)
   const int64_t node = pair / elements;
   const int z = (int)(pair - node * elements);
   SenderElements from(sender, species, row_ptr[node], row_ptr[node + 1], lane);
-  if (EARLY) grid_begin();
-  SharedRows rows(row_of, row_lists[w], from);
+  SharedRows rows(row_of, row_lists[w], from, EARLY);
+  if (EARLY) grid_begin();   // only the gradients of the sums are the kernel before's
   int32_t *list = lists[w];
   double *st = stage[w];
   double2 P[2][8];
