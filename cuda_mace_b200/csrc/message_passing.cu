@@ -18,6 +18,7 @@
 // sender-grouped edge permutation; again one warp per node, no atomics.
 #include <atomic>
 #include <cstdlib>
+#include <type_traits>
 
 #include "common.cuh"
 #include "step_common.cuh"
@@ -979,13 +980,20 @@ static bool takes_slots(int C) {
 template <typename T, int VEC, int LANES, bool ROWS>
 static void launch_fwd_slots(const T *X, const T *Y, const T *R, const int32_t *row_of, const int32_t *sender, const int32_t *row_ptr,
                              int64_t nnodes, ImpLayout ys, T *out, cudaStream_t st) {
-  if (few_nodes(nnodes)) {
-    constexpr int smem = kSplit * 16 * VEC * LANES * (int)sizeof(T);
-    auto kernel = imp_fwd_slots_kernel<T, VEC, LANES, kSplit, ROWS>;
+  // Warps a receiver while there are few: with 168 registers and more a thread an SM holds one or two blocks of eight warps.  us with one,
+  // two, four and eight (and of the kernel for whole warps), float32: 64 channels, 52 edges a receiver 14.4, 7.3, 6.2, 6.2 (6.2) at 64
+  // receivers, 16.5, 8.3, 6.2, 9.4 (8.3) at 300, 19.7, 10.3, 10.6, 14.4 (12.1) at 600, 23.6, 16.5, 16.4, 22.8 (16.7) at 1 150; 30 edges 14.6,
+  // 12.4, 12.4, 18.5 (13.3) at 1 150; 32 channels 8.3, 8.4, 10.2, 14.4 (10.4); 96 channels, 52 edges, float32 28.7, 16.4, 14.4, 14.5 (22.5) at
+  // 600, float64 29.1, 19.7, 14.4, 15.5 (22.6) at 300, 42.5, 40.2, 41.0, 47.7 (57.4) at 1 150.
+  auto split = [&](auto warps) {
+    constexpr int SPLIT = decltype(warps)::value, smem = SPLIT * 16 * VEC * LANES * (int)sizeof(T);
+    auto kernel = imp_fwd_slots_kernel<T, VEC, LANES, SPLIT, ROWS>;
     cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
-    launch_chained(kernel, (unsigned)nnodes, kSplit * 32, smem, st, X, Y, R, row_of, sender, row_ptr, nnodes, ys, out);
-    return;
-  }
+    launch_chained(kernel, (unsigned)nnodes, SPLIT * 32, smem, st, X, Y, R, row_of, sender, row_ptr, nnodes, ys, out);
+  };
+  if (nnodes <= (VEC == 3 ? 222 : 148)) return split(std::integral_constant<int, 8>{});
+  if (nnodes <= (VEC == 3 && sizeof(T) == 4 ? 800 : 444)) return split(std::integral_constant<int, 4>{});
+  if (few_nodes(nnodes)) return split(std::integral_constant<int, 2>{});
   launch_chained(imp_fwd_slots_kernel<T, VEC, LANES, 1, ROWS>, (unsigned)((nnodes + kWarpsPerBlock - 1) / kWarpsPerBlock),
                  kWarpsPerBlock * 32, 0, st, X, Y, R, row_of, sender, row_ptr, nnodes, ys, out);
 }
@@ -1020,7 +1028,11 @@ int imp_fwd(const T *X, const T *Y, const T *R, const int32_t *sender, const int
   if (!out || !row_ptr || (nedges > 0 && (!X || !R || !Y || !sender)))
     return fail(CMACE_ERR_ARG, "cmace_imp_fwd: null pointer");
   cudaStream_t st = (cudaStream_t)stream;
-  if (takes_slots<T>(C)) {
+  // Many receivers of few edges leave places of a warp empty, us of the two kernels, float32: 32 channels, 20 000 receivers of 2 edges 22.6
+  // against 16.5, of 4 26.7, 24.6, of 6 30.8, 30.7, of 8 35.0, 36.9; 64 channels, of 2 34.9, 31.1, of 8 63.6, 61.4, of 12 81.4, 79.8, 8 000 of
+  // 20 45.1, 45.1, of 30 61.8, 63.6.  At 1 300 receivers the places cost nothing; 96 channels and float64 gain at any number of edges.
+  const bool sparse = sizeof(T) == 4 && C <= 64 && nnodes >= 2000 && nedges < (C == 32 ? 6 : 20) * nnodes;
+  if (takes_slots<T>(C) && !sparse) {
     fwd_slots<T, false>(X, Y, R, nullptr, sender, row_ptr, nnodes, ys, C, out, st);
     return check_launch("cmace_imp_fwd");
   }

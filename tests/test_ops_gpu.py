@@ -763,6 +763,18 @@ def test_message_passing_of_narrow_rows(dtype, N, deg, C, dev):
     test_message_passing(dtype, N, deg, C, None, 7, dev)
 
 
+# where the number of warps a receiver changes (148, 222, 444, 700, 800, 1 184 receivers, 16 edges a receiver in the backward) and where
+# few edges go to the kernels for whole warps: 6 (32 channels) or 20 (64) a receiver from 2 000 on in the forward, 3 halves and 3 (from
+# 6 000) in the backward
+@pytest.mark.parametrize("dtype", DTYPES)
+@pytest.mark.parametrize("N,deg,C", [(148, 9, 32), (149, 9, 64), (222, 5, 96), (223, 7, 32), (444, 9, 64), (445, 17, 32), (445, 3, 96),
+                                     (700, 16, 32), (700, 15, 64), (701, 17, 32), (800, 3, 96), (801, 5, 96), (1184, 9, 32), (1185, 9, 64),
+                                     (2000, 1, 32), (2000, 2, 64), (1999, 1, 32), (2000, 5, 32), (2000, 6, 32), (2000, 19, 64), (2000, 20, 64),
+                                     (6000, 2, 32), (6000, 3, 64), (5999, 2, 64)])
+def test_message_passing_of_narrow_rows_where_the_kernel_changes(dtype, N, deg, C, dev):
+    test_message_passing(dtype, N, deg, C, None, 7, dev)
+
+
 # the same kernels: places of a warp that have no edge add nothing, not zero times what the receiver's last edge holds
 @pytest.mark.parametrize("dtype,C", [(torch.float64, 32), (torch.float64, 96), (torch.float32, 32), (torch.float32, 64),
                                      (torch.float32, 96)])
