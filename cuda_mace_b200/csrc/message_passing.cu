@@ -1007,8 +1007,12 @@ static void fwd_slots(const T *X, const T *Y, const T *R, const int32_t *row_of,
 }
 template <typename T, bool PAIR>
 static void bwd_edge_slots(const T *X, const T *Y, const T *R, const T *dR, const int32_t *row_of, const T *G, const int32_t *sender,
-                           const int32_t *row_ptr, int64_t nnodes, ImpLayout ys, int C, T *gradR, T *gY, T *Tout, cudaStream_t st) {
-  const int slices = few_nodes(nnodes) ? kSplit : 1;
+                           const int32_t *row_ptr, int64_t nnodes, int64_t nedges, ImpLayout ys, int C, T *gradR, T *gY, T *Tout,
+                           cudaStream_t st) {
+  // Warps a receiver while there are few: 444 blocks of four run at a time, and a warp takes four or eight edges.  us with four and eight,
+  // 52 edges a receiver, float32, 64 channels: 8.3, 6.2 at 64 receivers, 11.3, 12.4 at 300, 20.4, 18.5 at 600, 30.9, 30.8 at 1 150; 8 edges,
+  // 32 channels: 4.4, 6.2 at 300, 6.2, 6.3 at 600, 8.3, 10.0 at 1 150.  96 channels, two edges a warp, 52: 20.6, 16.4 at 300.
+  const int slices = !few_nodes(nnodes) ? 1 : (C == 96 || nnodes <= 222 || (nnodes <= 700 && nedges >= 16 * nnodes) ? 8 : 4);
   auto launch = [&](auto kernel) {
     launch_chained(kernel, (unsigned)((nnodes * slices + kWarpsPerBlock - 1) / kWarpsPerBlock), kWarpsPerBlock * 32, 0, st, X, Y, R, dR,
                    row_of, G, sender, row_ptr, nnodes, ys, slices, gradR, gY, Tout);
@@ -1079,7 +1083,7 @@ int imp_bwd_edge_pair_f64(const double *X, const double *Y, const double *R, con
                           double *gY, double *T, cudaStream_t st) {
   if (nnodes == 0 || nedges == 0) return CMACE_OK;
   if (takes_slots<double>(C)) {
-    bwd_edge_slots<double, true>(X, Y, R, dR, row_of, G, sender, row_ptr, nnodes, ImpLayout{1, 16}, C, nullptr, gY, T, st);
+    bwd_edge_slots<double, true>(X, Y, R, dR, row_of, G, sender, row_ptr, nnodes, nedges, ImpLayout{1, 16}, C, nullptr, gY, T, st);
     return check_launch("cmace_step(edges_back)");
   }
   auto launch = [&](auto kernel, int chunks) {
@@ -1129,8 +1133,11 @@ int imp_bwd_edge(const T *X, const T *Y, const T *R, const T *G, const int32_t *
   int rc = check_bwd_edge<T>(X, Y, R, G, sender, row_ptr, nnodes, nedges, C, gradR, gradY, Tout);
   if (rc || nnodes == 0 || nedges == 0) return rc;
   cudaStream_t st = (cudaStream_t)stream;
-  if (takes_slots<T>(C)) {   // a whole row at a time: no partials
-    bwd_edge_slots<T, false>(X, Y, R, nullptr, nullptr, G, sender, row_ptr, nnodes, ys, C, gradR, gradY, Tout, st);
+  // as in the forward, us of the two kernels: 20 000 receivers of 1 edge 28.7 against 20.5 (32 channels), 31.2, 25.7 (64), 36.9, 28.7 (32 in
+  // float64), of 2 edges 32.8, 28.7, 47.1, 44.9, 49.2, 46.7, of 3 39.0, 41.0, 55.3, 55.2, 61.3, 62.9; 3 000 of 1 edge 8.3, 6.2, of 2 8.3, 8.3
+  const bool sparse = C <= 64 && nnodes >= 2000 && 2 * nedges < (nnodes >= 6000 ? 6 : 3) * nnodes;
+  if (takes_slots<T>(C) && !sparse) {   // a whole row at a time: no partials
+    bwd_edge_slots<T, false>(X, Y, R, nullptr, nullptr, G, sender, row_ptr, nnodes, nedges, ys, C, gradR, gradY, Tout, st);
     return check_launch("cmace_imp_bwd_edge");
   }
   const int vec = pick_vec<T>(C);
