@@ -52,6 +52,7 @@ __global__ void __launch_bounds__(SPLIT == 1 ? kWarpsPerBlock * 32 : SPLIT * 32,
     for (int v = 0; v < VEC; v++) acc[m][v] = T(0);
 
   __shared__ __align__(16) PairHarmonics<T, SPLIT == 1 ? kWarpsPerBlock : SPLIT> harmonics;
+  constexpr bool BRANCH = sizeof(T) == 8 || SPLIT > 1;
   int turn = 0;
   const int ylm = lane & 15, yedge = lane >> 4;
   int32_t next[4];   // ROWS: senders and rows of the next pair, or the row of R would wait for its number
@@ -62,8 +63,9 @@ __global__ void __launch_bounds__(SPLIT == 1 ? kWarpsPerBlock * 32 : SPLIT * 32,
   if (ROWS && e0 < e1) look_up(e0 + (SPLIT > 1 ? 2 * warp : 0));
   for (int64_t e = e0 + (SPLIT > 1 ? 2 * warp : 0); e < e1; e += 2 * SPLIT, turn ^= 1) {
     // second edge of the pair: clamp to a valid edge, what it would add is zeroed below.  Zero harmonics alone would not do, the last edge's
-    // weights may be infinite (106.1 -> 106.6 us at 8 192 receivers of 30 edges, 128 channels, float64 223.4 -> 225.8; a branch, or the last
-    // edge behind the loop: 107, 280)
+    // weights may be infinite.  us at 8 192 receivers of 30 edges, 128 channels: 106.1 -> 106.6 by selects, 131 in a branch (registers), 132
+    // with a row of zeros, 107 with the last edge behind the loop; float64 223.3 -> 223.8 in a branch, 225.8 by selects, 280 with a row of
+    // zeros or behind the loop; eight warps a receiver, 800 of 52: 28.8 -> 28.8 in a branch, 30.8 by selects.
     const bool second = e + 1 < e1;
     const int64_t eb = second ? e + 1 : e;
     const int64_t ey = yedge ? eb : e;
@@ -90,8 +92,18 @@ __global__ void __launch_bounds__(SPLIT == 1 ? kWarpsPerBlock * 32 : SPLIT * 32,
 #pragma unroll
       for (int v = 0; v < VEC; v++) {
         ra[l][v] *= xa[v];
-        rb[l][v] = second ? rb[l][v] * xb[v] : T(0);
+        rb[l][v] *= xb[v];
+        if (!BRANCH && !second) rb[l][v] = T(0);
       }
+    if (BRANCH && !second) {   // volatile: it stays a branch
+#pragma unroll
+      for (int l = 0; l < 4; l++)
+#pragma unroll
+        for (int v = 0; v < VEC; v++) {
+          if constexpr (sizeof(T) == 8) asm volatile("mov.f64 %0, 0d0000000000000000;" : "=d"(rb[l][v]));
+          else asm volatile("mov.f32 %0, 0f00000000;" : "=f"(rb[l][v]));
+        }
+    }
     T *yp = harmonics.v[warp][turn];
     yp[lane] = yv;
     __syncwarp();
