@@ -62,10 +62,11 @@ __global__ void __launch_bounds__(SPLIT == 1 ? kWarpsPerBlock * 32 : SPLIT * 32,
   };
   if (ROWS && e0 < e1) look_up(e0 + (SPLIT > 1 ? 2 * warp : 0));
   for (int64_t e = e0 + (SPLIT > 1 ? 2 * warp : 0); e < e1; e += 2 * SPLIT, turn ^= 1) {
-    // second edge of the pair: clamp to a valid edge, what it would add is zeroed below.  Zero harmonics alone would not do, the last edge's
-    // weights may be infinite.  us at 8 192 receivers of 30 edges, 128 channels: 106.1 -> 106.6 by selects, 131 in a branch (registers), 132
-    // with a row of zeros, 107 with the last edge behind the loop; float64 223.3 -> 223.8 in a branch, 225.8 by selects, 280 with a row of
-    // zeros or behind the loop; eight warps a receiver, 800 of 52: 28.8 -> 28.8 in a branch, 30.8 by selects.
+    // second edge of the pair: clamp to a valid edge, what it would add is zeroed below.  Zero harmonics alone would not do, the last
+    // edge's weights may be infinite.  us at 8 192 receivers of 30 edges, 128 channels: 106.1 -> 106.6 by selects, 131 in a branch
+    // (registers), 132 with a row of zeros, 107 with the last edge behind the loop; float64 223.3 -> 223.8 in a branch, 225.8 by
+    // selects, 280 with a row of zeros or behind the loop; eight warps a receiver, 800 of 52: 28.8 -> 28.8 in a branch, 30.8 by
+    // selects.
     const bool second = e + 1 < e1;
     const int64_t eb = second ? e + 1 : e;
     const int64_t ey = yedge ? eb : e;
@@ -878,12 +879,12 @@ __global__ void sum_partials_kernel(const T *__restrict__ partial, int nchunks, 
 // flight follows the registers that it believes it has, so every width says for how many blocks an SM it is compiled (0: nothing said).
 // SPLIT warps a sender (few senders), five blocks, three doubles a lane four (48 registers would spill); with nothing said 29 -> 25 us
 // at 3 000 atoms of 128 channels in float32, 68 -> 58 at 8 000, 47 -> 37 in float64 at 3 000, 25 -> 21 with 96 channels.  (Six blocks:
-// 29 and 64; eight rows at a time instead of four: 31 and 68; two rows, eight blocks: 25 and 54, but 23 with 96 channels.)
-// One warp a sender, float32, at 16 000 atoms: 32 channels ten blocks 52 -> 44 (one 60, sixteen 64), 64 channels eight 70 -> 58 (one
-// 60, ten 60, twelve 80; 209 -> 183 at 64 000), 128 channels one 95 -> 88 (eight 91, ten 117; 330 -> 301 at 64 000), 96 channels
-// nothing said and the list's lines prefetched 81 (109 without the prefetch, which is no help to the others; one, six to nine 88, twelve
-// 130); float64 with 96 channels one 84 -> 76 at 8 000.  Registers that come of it: 48 of 256 threads (64 with three doubles a lane); of 128
-// threads in float32 48, 62, 48, 74 for one to four values a lane, in float64 64 or 80.  A compiler that arrives at others: measure again.
+// 29 and 64; eight rows at a time instead of four: 31 and 68; two rows, eight blocks: 25 and 54, but 23 with 96 channels.) One warp a
+// sender, float32, at 16 000 atoms: 32 channels ten blocks 52 -> 44 (one 60, sixteen 64), 64 channels eight 70 -> 58 (one 60, ten 60,
+// twelve 80; 209 -> 183 at 64 000), 128 channels one 95 -> 88 (eight 91, ten 117; 330 -> 301 at 64 000), 96 channels nothing said and
+// the list's lines prefetched 81 (109 without the prefetch, which is no help to the others; one, six to nine 88, twelve 130); float64
+// with 96 channels one 84 -> 76 at 8 000.  Registers that come of it: 48 of 256 threads (64 with three doubles a lane); of 128 threads
+// in float32 48, 62, 48, 74 for one to four values a lane, in float64 64 or 80.  A compiler that arrives at others: measure again.
 template <typename T, int VEC, int SPLIT>
 constexpr int node_blocks_an_sm() {
   if (SPLIT > 1) return sizeof(T) * VEC <= 16 ? 5 : 4;
@@ -992,11 +993,11 @@ static bool takes_slots(int C) {
 template <typename T, int VEC, int LANES, bool ROWS>
 static void launch_fwd_slots(const T *X, const T *Y, const T *R, const int32_t *row_of, const int32_t *sender, const int32_t *row_ptr,
                              int64_t nnodes, ImpLayout ys, T *out, cudaStream_t st) {
-  // Warps a receiver while there are few: with 168 registers and more a thread an SM holds one or two blocks of eight warps.  us with one,
-  // two, four and eight (and of the kernel for whole warps), float32: 64 channels, 52 edges a receiver 14.4, 7.3, 6.2, 6.2 (6.2) at 64
-  // receivers, 16.5, 8.3, 6.2, 9.4 (8.3) at 300, 19.7, 10.3, 10.6, 14.4 (12.1) at 600, 23.6, 16.5, 16.4, 22.8 (16.7) at 1 150; 30 edges 14.6,
-  // 12.4, 12.4, 18.5 (13.3) at 1 150; 32 channels 8.3, 8.4, 10.2, 14.4 (10.4); 96 channels, 52 edges, float32 28.7, 16.4, 14.4, 14.5 (22.5) at
-  // 600, float64 29.1, 19.7, 14.4, 15.5 (22.6) at 300, 42.5, 40.2, 41.0, 47.7 (57.4) at 1 150.
+  // Warps a receiver while there are few: with 168 registers and more a thread an SM holds one or two blocks of eight warps.  us with
+  // one, two, four and eight (and of the kernel for whole warps), float32: 64 channels, 52 edges a receiver 14.4, 7.3, 6.2, 6.2 (6.2)
+  // at 64 receivers, 16.5, 8.3, 6.2, 9.4 (8.3) at 300, 19.7, 10.3, 10.6, 14.4 (12.1) at 600, 23.6, 16.5, 16.4, 22.8 (16.7) at 1 150; 30
+  // edges 14.6, 12.4, 12.4, 18.5 (13.3) at 1 150; 32 channels 8.3, 8.4, 10.2, 14.4 (10.4); 96 channels, 52 edges, float32 28.7, 16.4,
+  // 14.4, 14.5 (22.5) at 600, float64 29.1, 19.7, 14.4, 15.5 (22.6) at 300, 42.5, 40.2, 41.0, 47.7 (57.4) at 1 150.
   auto split = [&](auto warps) {
     constexpr int SPLIT = decltype(warps)::value, smem = SPLIT * 16 * VEC * LANES * (int)sizeof(T);
     auto kernel = imp_fwd_slots_kernel<T, VEC, LANES, SPLIT, ROWS>;
@@ -1021,9 +1022,10 @@ template <typename T, bool PAIR>
 static void bwd_edge_slots(const T *X, const T *Y, const T *R, const T *dR, const int32_t *row_of, const T *G, const int32_t *sender,
                            const int32_t *row_ptr, int64_t nnodes, int64_t nedges, ImpLayout ys, int C, T *gradR, T *gY, T *Tout,
                            cudaStream_t st) {
-  // Warps a receiver while there are few: 444 blocks of four run at a time, and a warp takes four or eight edges.  us with four and eight,
-  // 52 edges a receiver, float32, 64 channels: 8.3, 6.2 at 64 receivers, 11.3, 12.4 at 300, 20.4, 18.5 at 600, 30.9, 30.8 at 1 150; 8 edges,
-  // 32 channels: 4.4, 6.2 at 300, 6.2, 6.3 at 600, 8.3, 10.0 at 1 150.  96 channels, two edges a warp, 52: 20.6, 16.4 at 300.
+  // Warps a receiver while there are few: 444 blocks of four run at a time, and a warp takes four or eight edges.  us with four and
+  // eight, 52 edges a receiver, float32, 64 channels: 8.3, 6.2 at 64 receivers, 11.3, 12.4 at 300, 20.4, 18.5 at 600, 30.9, 30.8
+  // at 1 150; 8 edges, 32 channels: 4.4, 6.2 at 300, 6.2, 6.3 at 600, 8.3, 10.0 at 1 150.  96 channels, two edges a warp, 52: 20.6,
+  // 16.4 at 300.
   const int slices = !few_nodes(nnodes) ? 1 : (C == 96 || nnodes <= 222 || (nnodes <= 700 && nedges >= 16 * nnodes) ? 8 : 4);
   auto launch = [&](auto kernel) {
     launch_chained(kernel, (unsigned)((nnodes * slices + kWarpsPerBlock - 1) / kWarpsPerBlock), kWarpsPerBlock * 32, 0, st, X, Y, R, dR,
@@ -1044,9 +1046,10 @@ int imp_fwd(const T *X, const T *Y, const T *R, const int32_t *sender, const int
   if (!out || !row_ptr || (nedges > 0 && (!X || !R || !Y || !sender)))
     return fail(CMACE_ERR_ARG, "cmace_imp_fwd: null pointer");
   cudaStream_t st = (cudaStream_t)stream;
-  // Many receivers of few edges leave places of a warp empty, us of the two kernels, float32: 32 channels, 20 000 receivers of 2 edges 22.6
-  // against 16.5, of 4 26.7, 24.6, of 6 30.8, 30.7, of 8 35.0, 36.9; 64 channels, of 2 34.9, 31.1, of 8 63.6, 61.4, of 12 81.4, 79.8, 8 000 of
-  // 20 45.1, 45.1, of 30 61.8, 63.6.  At 1 300 receivers the places cost nothing; 96 channels and float64 gain at any number of edges.
+  // Many receivers of few edges leave places of a warp empty, us of the two kernels, float32: 32 channels, 20 000 receivers of 2 edges
+  // 22.6 against 16.5, of 4 26.7, 24.6, of 6 30.8, 30.7, of 8 35.0, 36.9; 64 channels, of 2 34.9, 31.1, of 8 63.6, 61.4, of 12 81.4,
+  // 79.8, 8 000 of 20 45.1, 45.1, of 30 61.8, 63.6.  At 1 300 receivers the places cost nothing; 96 channels and float64 gain at any
+  // number of edges.
   const bool sparse = sizeof(T) == 4 && C <= 64 && nnodes >= 2000 && nedges < (C == 32 ? 6 : 20) * nnodes;
   if (takes_slots<T>(C) && !sparse) {
     fwd_slots<T, false>(X, Y, R, nullptr, sender, row_ptr, nnodes, ys, C, out, st);
@@ -1145,8 +1148,9 @@ int imp_bwd_edge(const T *X, const T *Y, const T *R, const T *G, const int32_t *
   int rc = check_bwd_edge<T>(X, Y, R, G, sender, row_ptr, nnodes, nedges, C, gradR, gradY, Tout);
   if (rc || nnodes == 0 || nedges == 0) return rc;
   cudaStream_t st = (cudaStream_t)stream;
-  // as in the forward, us of the two kernels: 20 000 receivers of 1 edge 28.7 against 20.5 (32 channels), 31.2, 25.7 (64), 36.9, 28.7 (32 in
-  // float64), of 2 edges 32.8, 28.7, 47.1, 44.9, 49.2, 46.7, of 3 39.0, 41.0, 55.3, 55.2, 61.3, 62.9; 3 000 of 1 edge 8.3, 6.2, of 2 8.3, 8.3
+  // as in the forward, us of the two kernels: 20 000 receivers of 1 edge 28.7 against 20.5 (32 channels), 31.2, 25.7 (64), 36.9, 28.7
+  // (32 in float64), of 2 edges 32.8, 28.7, 47.1, 44.9, 49.2, 46.7, of 3 39.0, 41.0, 55.3, 55.2, 61.3, 62.9; 3 000 of 1 edge 8.3, 6.2,
+  // of 2 8.3, 8.3
   const bool sparse = C <= 64 && nnodes >= 2000 && 2 * nedges < (nnodes >= 6000 ? 6 : 3) * nnodes;
   if (takes_slots<T>(C) && !sparse) {   // a whole row at a time: no partials
     bwd_edge_slots<T, false>(X, Y, R, nullptr, nullptr, G, sender, row_ptr, nnodes, nedges, ys, C, gradR, gradY, Tout, st);
